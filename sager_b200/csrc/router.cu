@@ -23,28 +23,183 @@ namespace sgr {
 
 namespace {
 
-constexpr int kRouterTok = 8;     // tokens per CTA of the logits kernel
-
-// grid (ceil(n_rows / warps), ceil(n_tokens / kRouterTok)); dynamic smem = nt*k fp16
-template <int TT>
+// ---- one token: a warp per expert row, straight from global memory ------------------
 __global__ void router_logits_kernel(const float* __restrict__ w, const uint16_t* __restrict__ x,
-                                     float* __restrict__ y, int n_rows, int k, int n_tokens) {
+                                     float* __restrict__ y, int n_rows, int k) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint16_t* xs = reinterpret_cast<uint16_t*>(smem);
-  const int tok0 = blockIdx.y * TT;
-  const int nt = min(TT, n_tokens - tok0);
-  for (int i = threadIdx.x; i < nt * k; i += blockDim.x) xs[i] = x[static_cast<size_t>(tok0) * k + i];
+  for (int i = threadIdx.x; i < k; i += blockDim.x) xs[i] = x[i];
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n_rows) return;
-  float out[TT];
-  router_row_dot<TT>(w + static_cast<size_t>(row) * k, xs, k, nt, lane, out);
-  if (lane == 0) {
+  float out[1];
+  router_row_dot<1>(w + static_cast<size_t>(row) * k, xs, k, 1, lane, out);
+  if (lane == 0) y[row] = out[0];
+}
+
+// ---- several tokens: a register-tiled fp32 product with the reference's sum order -----
+// A warp owns TR expert rows x TT tokens; lane l holds their chain l (k = l, l + 32, ...), so an
+// output's 32 partial sums live in the 32 lanes and every lane runs TR * TT independent FMA
+// chains from TR + TT shared-memory operands. Two tokens share a packed fp32x2 FMA (the same
+// rounding per component, half the issue slots). At the end the lanes exchange halves: in step
+// 16, 8, 4, 2, 1 a lane adds the partner's half of the outputs to its own, which is the pairing
+// of the reference's shuffle-down tree (addition commutes), in 31/32 of a shuffle per output
+// instead of five. Bound by the fp32 pipes and the issue slots around them (1.07 G FMAs for 2048
+// tokens x 256 rows x 2048: 29 us at 128 per clock and SM). Measured for 2048 / 777 / 96 tokens:
+// 81 / 41 / 10 us; a warp per (row, eight tokens) with the fp16 values converted at every use
+// took 534 / 212 / 33 us.
+__device__ __forceinline__ void fma2(unsigned long long& acc, float w, unsigned long long x) {
+  unsigned long long ww;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(ww), "l"(x));
+}
+// One step of the exchange: N outputs in, N / 2 out (the upper half in the lanes with `Bit` set), then the next.
+template <int N, int Bit>
+__device__ __forceinline__ void fold_lanes(float* f, int lane) {
+  if constexpr (Bit > 0) {
+    const bool up = (lane & Bit) != 0;
 #pragma unroll
-    for (int t = 0; t < TT; ++t)
-      if (t < nt) y[static_cast<size_t>(tok0 + t) * n_rows + row] = out[t];
+    for (int i = 0; i < N / 2; ++i) {
+      const float keep = up ? f[i + N / 2] : f[i];
+      const float send = up ? f[i] : f[i + N / 2];
+      f[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, Bit);
+    }
+    fold_lanes<N / 2, Bit / 2>(f, lane);
   }
+}
+
+// block: WR x WT warps; grid (row tiles, token tiles). KC columns per shared-memory stage, two
+// stages: the next one is on its way to registers while this one is used, so a stage has to last a
+// round trip to L2 (with 64 columns the trip showed: 124 us for 2048 tokens, 14 us for eight).
+template <int TR, int TT, int WR, int WT, int KC>
+__global__ void __launch_bounds__(WR* WT * 32)
+router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restrict__ x, float* __restrict__ y,
+                           int n_rows, int k, int n_tokens) {
+  constexpr int kWarps = WR * WT, kRows = TR * WR, kPairs = TT * WT / 2, kSteps = KC / 64;
+  constexpr int kRowsPerWarp = kRows / kWarps, kPairsPerWarp = kPairs / kWarps;
+  static_assert(kRows % kWarps == 0 && kPairs % kWarps == 0 && TR * TT >= 32 && KC % 64 == 0, "tile split");
+  // a stage: two k steps of a lane lie together, [row][step][lane][2 k] and [pair][step][lane][2 k][2 tokens], so
+  // that an operand is one 8- or 16-byte shared-memory access per two steps, without conflicts
+  extern __shared__ __align__(16) unsigned char smem[];
+  float2(*ws)[kRows][kSteps][32] = reinterpret_cast<float2(*)[kRows][kSteps][32]>(smem);
+  float4(*xs)[kPairs][kSteps][32] =
+      reinterpret_cast<float4(*)[kPairs][kSteps][32]>(smem + 2 * sizeof(float) * kRows * KC);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = blockIdx.x * kRows, tok0 = blockIdx.y * (TT * WT);
+  const int wr = warp % WR, wt = warp / WR;
+
+  // the stage this warp copies: rows warp, warp + kWarps, ... and token pairs likewise; rows and
+  // tokens past the end repeat the last one (never stored), columns past k are zero (add nothing)
+  const float* wp[kRowsPerWarp];
+  const uint16_t* xp[kPairsPerWarp][2];
+#pragma unroll
+  for (int i = 0; i < kRowsPerWarp; ++i)
+    wp[i] = w + static_cast<size_t>(min(row0 + warp + i * kWarps, n_rows - 1)) * k + lane;
+#pragma unroll
+  for (int i = 0; i < kPairsPerWarp; ++i)
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      xp[i][c] = x + static_cast<size_t>(min(tok0 + 2 * (warp + i * kWarps) + c, n_tokens - 1)) * k + lane;
+  float wreg[kRowsPerWarp][KC / 32];
+  uint16_t xreg[kPairsPerWarp][KC / 32][2];
+  auto fetch = [&](int k0) {
+    if (k0 + KC <= k) {
+#pragma unroll
+      for (int j = 0; j < KC / 32; ++j) {
+#pragma unroll
+        for (int i = 0; i < kRowsPerWarp; ++i) wreg[i][j] = __ldg(wp[i] + k0 + 32 * j);
+#pragma unroll
+        for (int i = 0; i < kPairsPerWarp; ++i)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) xreg[i][j][c] = __ldg(xp[i][c] + k0 + 32 * j);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < KC / 32; ++j) {
+        const bool in = k0 + 32 * j + lane < k;
+#pragma unroll
+        for (int i = 0; i < kRowsPerWarp; ++i) wreg[i][j] = in ? __ldg(wp[i] + k0 + 32 * j) : 0.f;
+#pragma unroll
+        for (int i = 0; i < kPairsPerWarp; ++i)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) xreg[i][j][c] = in ? __ldg(xp[i][c] + k0 + 32 * j) : static_cast<uint16_t>(0);
+      }
+    }
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int j = 0; j < kSteps; ++j) {
+#pragma unroll
+      for (int i = 0; i < kRowsPerWarp; ++i)
+        ws[buf][warp + i * kWarps][j][lane] = make_float2(wreg[i][2 * j], wreg[i][2 * j + 1]);
+#pragma unroll
+      for (int i = 0; i < kPairsPerWarp; ++i)
+        xs[buf][warp + i * kWarps][j][lane] = make_float4(h2f(xreg[i][2 * j][0]), h2f(xreg[i][2 * j][1]),
+                                                          h2f(xreg[i][2 * j + 1][0]), h2f(xreg[i][2 * j + 1][1]));
+    }
+  };
+
+  unsigned long long acc[TR][TT / 2];           // two packed fp32 sums each
+#pragma unroll
+  for (int r = 0; r < TR; ++r)
+#pragma unroll
+    for (int p = 0; p < TT / 2; ++p) acc[r][p] = 0ull;
+  fetch(0);
+  put(0);
+  __syncthreads();
+  for (int k0 = 0, buf = 0; k0 < k; k0 += KC, buf ^= 1) {
+    const bool more = k0 + KC < k;
+    if (more) fetch(k0 + KC);
+#pragma unroll
+    for (int j = 0; j < kSteps; ++j) {
+      float2 wv[TR];
+      ulonglong2 xv[TT / 2];
+#pragma unroll
+      for (int r = 0; r < TR; ++r) wv[r] = ws[buf][wr * TR + r][j][lane];
+#pragma unroll
+      for (int p = 0; p < TT / 2; ++p)
+        xv[p] = *reinterpret_cast<const ulonglong2*>(&xs[buf][wt * (TT / 2) + p][j][lane]);
+#pragma unroll
+      for (int r = 0; r < TR; ++r)
+#pragma unroll
+        for (int p = 0; p < TT / 2; ++p) fma2(acc[r][p], wv[r].x, xv[p].x);
+#pragma unroll
+      for (int r = 0; r < TR; ++r)
+#pragma unroll
+        for (int p = 0; p < TT / 2; ++p) fma2(acc[r][p], wv[r].y, xv[p].y);
+    }
+    if (more) put(buf ^ 1);       // the other buffer: every warp left it at the barrier below
+    __syncthreads();
+  }
+
+  // fold the 32 lanes: output o = r * TT + t; after the five exchanges lane l holds the outputs
+  // whose bits above log2(TR * TT / 32) spell l's bits from bit 4 down
+  float f[TR * TT];
+#pragma unroll
+  for (int r = 0; r < TR; ++r)
+#pragma unroll
+    for (int p = 0; p < TT / 2; ++p)
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(f[r * TT + 2 * p]), "=f"(f[r * TT + 2 * p + 1]) : "l"(acc[r][p]));
+  fold_lanes<TR * TT, 16>(f, lane);
+  constexpr int kLeft = TR * TT / 32;
+#pragma unroll
+  for (int i = 0; i < kLeft; ++i) {
+    const int o = i + kLeft * lane;           // step s split on output bit log2(TR*TT) - 1 - s and lane bit 4 - s
+    const int row = row0 + wr * TR + o / TT, tok = tok0 + wt * TT + o % TT;
+    if (row < n_rows && tok < n_tokens) y[static_cast<size_t>(tok) * n_rows + row] = f[i];
+  }
+}
+
+template <int TR, int TT, int WR, int WT, int KC>
+int launch_tiled(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens, cudaStream_t stream) {
+  constexpr int kSmem = 2 * KC * (TR * WR + TT * WT) * static_cast<int>(sizeof(float));
+  auto kern = router_logits_tiled_kernel<TR, TT, WR, WT, KC>;
+  if (kSmem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
+    return kErrLaunch;
+  const dim3 grid((n_rows + TR * WR - 1) / (TR * WR), (n_tokens + TT * WT - 1) / (TT * WT));
+  kern<<<grid, WR * WT * 32, kSmem, stream>>>(w, x, y, n_rows, k, n_tokens);
+  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
 int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens,
@@ -55,15 +210,13 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
     const int warps = 2;                           // 2 MB of W spread over >= 128 CTAs at E=256
     const size_t smem = static_cast<size_t>(k) * 2;
     if (smem > 48 * 1024) return kErrUnsupported;
-    router_logits_kernel<1><<<dim3((n_rows + warps - 1) / warps, 1), warps * 32, smem, stream>>>(
-        w, x, y, n_rows, k, 1);
+    router_logits_kernel<<<(n_rows + warps - 1) / warps, warps * 32, smem, stream>>>(w, x, y, n_rows, k);
+  } else if (static_cast<long long>(n_rows) * n_tokens >= 256LL * 592) {
+    // 8 x 16 outputs per warp keep the FMA pipes fullest; below one such CTA per SM the smaller tile has more
+    // warps to spread (at 256 x 592 the two take 41 and 38 us, and from there the larger one wins)
+    return launch_tiled<8, 16, 4, 2, 128>(w, x, y, n_rows, k, n_tokens, stream);
   } else {
-    const int warps = 4;
-    const size_t smem = static_cast<size_t>(kRouterTok) * k * 2;
-    if (smem > 48 * 1024) return kErrUnsupported;
-    router_logits_kernel<kRouterTok>
-        <<<dim3((n_rows + warps - 1) / warps, (n_tokens + kRouterTok - 1) / kRouterTok), warps * 32,
-           smem, stream>>>(w, x, y, n_rows, k, n_tokens);
+    return launch_tiled<4, 8, 4, 1, 256>(w, x, y, n_rows, k, n_tokens, stream);   // small: more warps to spread
   }
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
 }

@@ -45,6 +45,20 @@ def test_logits_odd_shapes(oracle):
     assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
 
 
+@pytest.mark.parametrize("rows,k,n_tok", [(256, 2048, 592), (250, 736, 611), (256, 2048, 591), (13, 96, 9), (1, 2048, 33),
+                                          (17, 32, 2)])
+def test_logits_tile_edges_bit_exact(oracle, rows, k, n_tok):
+    """Both tilings of the many-token kernel (the rule's line is rows x tokens = 256 x 592): ragged rows,
+    tokens and columns."""
+    w_np, w_dev = router_w(5, e=rows, h=k)
+    x_np, x_dev = make_x16(n_tok, k, 6)
+    y = torch.full((n_tok + 1, rows), 7.0, dtype=torch.float32, device=DEV)
+    ops.gemv_f32_out_f16x_mtok(w_dev, x_dev, y, rows, k, n_tok)
+    want = np.stack([oracle.router_logits(w_np, x_np[t]) for t in range(n_tok)])
+    assert np.array_equal(y.cpu().numpy()[:n_tok].view(np.uint32), want.view(np.uint32))
+    assert torch.all(y[n_tok] == 7.0)
+
+
 @pytest.mark.parametrize("seed", range(8))
 def test_topk_selection_exact(oracle, seed):
     rng = np.random.default_rng(seed)
