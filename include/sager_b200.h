@@ -351,13 +351,13 @@ typedef struct sgr_moe_prefill {
   int* meta;                /* [4] */
   int* mail;                /* [n_expert] */
   int* mail_n;              /* [1] */
-  void* xqg;                /* [R][hidden/256] Q8_K blocks, 16-byte aligned */
+  void* xqg;                /* [R][hidden/256] Q8_K blocks, 16-byte aligned; not used: rows are read through the plan */
   uint16_t* g;              /* [R][n_ff] */
   uint16_t* u;              /* [R][n_ff] */
   void* hq;                 /* [R][n_ff/256] Q8_K blocks, 16-byte aligned */
   uint16_t* y_grouped;      /* [R][hidden] */
-  uint16_t* expert_y;       /* [n_max][n_used+1][hidden] combine slab: used only when x_f16, y_grouped or sh_y is
-                               not 16-byte aligned - otherwise the combine reads the grouped rows in place */
+  uint16_t* expert_y;       /* [n_max][n_used+1][hidden] combine slab, 16-byte aligned: scratch for the GEMMs' operand
+                               rows; the combine itself uses it only when x_f16, y_grouped or sh_y is not 16-byte aligned */
   uint16_t* sh_g;           /* [n_max][n_ff] */
   uint16_t* sh_u;           /* [n_max][n_ff] */
   void* sh_q;               /* [n_max][n_ff/256] Q8_K blocks */

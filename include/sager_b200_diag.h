@@ -27,6 +27,11 @@ long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff, int n_
  * exercised without a GPU. */
 int sgr_residency_test_set_inflight(void* handle, int slot, int on);
 
+/* The expert stage (gate, up, SwiGLU, requantise, down) of a finished sgr_moe_layer_prefill call once more, on
+ * the plan and the operand rows that call left in its buffers. For timing. */
+struct sgr_moe_prefill;
+int sgr_moe_prefill_expert_stage(const struct sgr_moe_prefill* args, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "sager_b200.h"   // the public prototypes: definitions must agree with them
 #include "sager_b200_diag.h"
 
@@ -21,8 +23,66 @@ inline cudaStream_t as_stream(void* s) { return static_cast<cudaStream_t>(s); }
 // Device address of the library's status word on the current device.
 int* status_word();
 
-// One Q4_K matrix over n_tok Q8_K rows on the int8 tensor-core kernel of the grouped GEMM
-// (grouped_gemm_i8.cu): y[t][r], fp16. xq 16-byte aligned.
-int gemm_i8_dense(const void* w, const void* xq, uint16_t* y, int n_tok, int n_rows, int k, cudaStream_t stream);
+// SMs of the current device (0: none can be had), asked of the runtime once per device.
+int device_sms();
+
+// Opts kernel K in to `bytes` of dynamic shared memory on the current device, once per device.
+template <auto K>
+bool opt_in_smem(int bytes) {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> done[kMaxDevices];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+  if (done[dev].load(std::memory_order_relaxed) >= bytes) return true;
+  if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+  done[dev].store(bytes, std::memory_order_relaxed);
+  return true;
+}
+
+// Launch that may start while the kernel before it in the stream drains (programmatic dependent launch);
+// the kernel waits for that one's results itself.
+template <typename... KArgs, typename... Args>
+int launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? 0 : 4 /* kErrLaunch */;
+}
+
+// ---- tensor-core GEMM of Q4_K experts over their routed rows (grouped_gemm_i8.cu) ----
+// Operand rows: the quantised activations as the GEMM's fp16 tiles want them, kOpBlk bytes per 256 values -
+// 256 codes in K order (0, 2, 1, 3 of every four), eight low and eight high parts of the sub-block sums
+// (bsum = 64 * hi + lo), the fp32 scale, 12 bytes of padding. 16-byte aligned.
+constexpr int kOpBlk = 560;
+
+// One more expert (shared_w) that every row of its own slab visits may ride along.
+struct ExpertGemm {
+  const unsigned char* const* tab;
+  const int* off;
+  const int* rows;              // activation row of each grouped slot, or null: the slot itself
+  const unsigned char* xq;      // operand rows, or Q8_K rows (operand_rows false)
+  uint16_t* y;
+  int n_rows, k, n_expert;
+  bool operand_rows;
+  const void* shared_w;
+  const unsigned char* shared_xq;
+  uint16_t* shared_y;
+  int shared_rows;
+};
+int gemm_grouped(const ExpertGemm& g, cudaStream_t stream);
+// gate and up in one pass (g holds the gate side)
+int gemm_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, uint16_t* y_up, const void* shared_up,
+                 uint16_t* shared_y_up, cudaStream_t stream);
+// rows of k fp16 values (SwiGLU of x and u where u is given) -> operand rows; two slabs, the first of at most
+// *d_rows rows when that is given
+int quantize_operand(const uint16_t* x0, const uint16_t* u0, void* out0, long long rows0, const int* d_rows,
+                     const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, cudaStream_t stream);
 
 }  // namespace sgr

@@ -1,87 +1,135 @@
-// grouped_gemm_i8.cu - the prefill MoE grouped GEMM on the 5th-generation tensor
-// cores: tcgen05.mma kind::i8 with the accumulators in tensor memory.
+// grouped_gemm_i8.cu - the prefill MoE grouped GEMM on the 5th-generation tensor cores:
+// tcgen05.mma with the weights as the tensor-memory operand and the accumulators in tensor memory.
 //
 // It replaces the reference's prefill expert math for chunks of many tokens
 // (dequant_experts_q4_k_f16 + one cublasGemmEx per expert and matrix,
 // src/kernels/cuda/tc_gemm.cu:124-152, 209-240, driven from
 // src/core/session.cpp:2643-2760) but keeps the arithmetic of the reference's
 // Q4_K x Q8_K path (gemv_grouped_tab_q4_k_q8_f16out_mtok, q4_k.cu:765-836): Q8_K
-// activations, exact integer dots, fp32 scaling - so it is checked against that
+// activations, integer dots, fp32 scaling - so it is checked against that
 // path, not against the fp16 one.
 //
-// The kernel is persistent: one CTA per SM takes work items (expert, tile of 128 weight rows)
-// round-robin, so tensor memory, the barriers and the pipeline are set up once per SM and the
-// roles run on into the next item without draining. Inside an item the CTA walks that expert's
-// token rows in chunks of up to 64, two chunks per pass. The work of a pass is a list of jobs
-// (super-block, chunk); job j uses accumulator set j & 1 in tensor memory and is
-// finished by epilogue group j & 1, so with one chunk the two groups take alternate
-// super-blocks and with two chunks each group owns a chunk. Four roles run as a
-// pipeline over mbarriers:
-//   * unpack warps (one thread per weight row): the 144-byte block becomes seventeen
-//     int8 operand tiles per super-block. The 6-bit scale rides through the MMA: with
-//     sc = 8a + b the products b*q and a*q (<= 105) are two u8 tiles per sub-block, so a
-//     whole block accumulates exactly in int32 as D_b + 8*D_a; the eight min bytes are
-//     one more tile. Double-buffered.
-//   * stager warps: the activation codes of the job's chunk, copied asynchronously
-//     into the B tiles (three buffers in flight), the sub-block sums split as
-//     128*hi + lo into two more tiles (for the min term), the fp32 scales aside.
-//   * one elected thread issues the 18 MMAs of a job (M=128, N=chunk, K=32,
-//     tcgen05.mma kind::i8) and commits them to the barriers that release the
-//     accumulators to the epilogue and the operand buffers to their producers.
-//   * epilogue warps read their 32 lanes back (tcgen05.ld) and fold
-//     xd*(d*(D_b + 8*D_a) - dmin*(mlo + 128*mhi)) into per-token fp32 registers while the
-//     next job's MMAs run.
-// Operand tiles use the canonical K-major layout without swizzle: 8 rows x 16 bytes
-// per core matrix, the two K halves 128 bytes apart, 8-row groups 256 bytes apart.
+// The integers ride in fp16 operands (kind::f16, fp32 accumulators): sc * q <= 945 and an int8 code
+// are exact in fp16, their products are exact, and a super-block's sum is an integer that fp32 holds
+// exactly below 2^24 (rounded above, as the conversion of an int32 sum would be). One accumulator
+// takes the 256 products of a block; a second one takes the min term in a single K = 16 step,
+// mn x (bsum & 63) + (64 mn) x (bsum >> 6). Per output and block the epilogue then reads two fp32
+// values and spends three operations, where the int8 form of the same idea (6-bit scales split over
+// two u8 operand tiles, four int32 accumulators) spends about twenty, four of them conversions.
+//
+// The 128 weight rows of a tile are the M lanes of tensor memory, so a thread that owns a row
+// unpacks its block in registers and stores it with tcgen05.st: weights never cross shared memory
+// as operands (two bytes per weight written and read again there was the int8 form's limit).
+//
+// Persistent: one CTA per SM takes work units round-robin. A unit is one expert, one or several
+// tiles of 128 weight rows, and at most 80 of the expert's token rows; a job is one super-block
+// column of a tile. The roles run as a pipeline over mbarriers:
+//   * two producer warps copy the [128 rows][144 B] block columns into a ring (cp.async; plain loads
+//     where an expert's base is only 2-byte aligned);
+//   * eight unpack warps (thread = weight row; four warps take the even jobs, four the odd ones):
+//     nibbles -> sc * q as packed fp16 with one logic and one FMA instruction per two weights, in
+//     three half-block slots of tensor memory; the min operand and (d, dmin) go to shared memory;
+//   * the activation tiles of one block, two in flight: one warp copies them (cp.async) from rows
+//     that already are operands (kOpBlk bytes per block, written by quantize_operand: a prefill
+//     chunk), or eight warps make them from Q8_K rows (the plain entry, which has no scratch; they
+//     cost more instructions than everything else together). Rows of at most two blocks keep their
+//     tiles for all weight tiles of the unit;
+//   * one warp issues the 17 MMAs of a job (M = 128, N = tokens rounded up to 16, K = 16);
+//   * eight epilogue warps fold xd * (d * D0 - dmin * D1) into fp32 registers, each warp 32 rows of
+//     every second tile (gate / up alternate), while the next job's MMAs run into the other of two
+//     accumulator sets.
+// The gate and up projections run as one pass: their jobs alternate over the same activation tiles.
+// What runs per job is kept compact: with the five roles on a scheduler a loop that is unrolled over a
+// whole block waits for its instructions (a third of all stall cycles did).
+// The shared expert is one more expert whose rows are all the chunk's rows.
+//
+// Operand tiles in shared memory use the canonical K-major layout without swizzle: 8 rows x 16
+// bytes per core matrix, the two K halves 128 bytes apart, 8-row groups 256 bytes apart.
 // Every wait is bounded; on expiry the CTA raises the status word, frees its tensor
 // memory and returns.
+#include <algorithm>
+
 #include "api_util.cuh"
-#include "q4k_common.cuh"
+#include "quantize_dev.cuh"
 
 namespace sgr {
 namespace {
 
-constexpr int kGemmRows = 128;     // weight rows per CTA = MMA M
-constexpr int kGemmTok = 64;       // token rows per chunk = max MMA N
-constexpr int kTileA = kGemmRows * 32;            // bytes of one A tile (128 x 32 int8)
-constexpr int kTileB = kGemmTok * 32;             // bytes of one B tile (64 x 32 int8)
-constexpr int kATiles = 17;                       // 8 sub-blocks x {b*q, a*q} + the min tile
-constexpr int kBTiles = 10;                       // 8 code tiles + 2 split-sum tiles
-constexpr int kABufs = 2, kBBufs = 3, kDdRing = 4, kXdRing = 6;
-constexpr int kTmemCols = 512;                    // two sets of four 64-column accumulators
+constexpr int kGemmRows = 128;                    // weight rows per tile = MMA M = tensor-memory lanes
+constexpr int kGemmTok = 80;                      // token rows per unit = max MMA N
+constexpr int kStages = 7, kStageBytes = kGemmRows * kW4;     // 18,432
+constexpr int kBTile = kGemmTok * 32;             // one K = 16 step of the activations
+constexpr int kBBytes = 17 * kBTile;              // 16 code steps + the split sums
+constexpr int kMinBytes = kGemmRows * 32;         // the min operand of a job
+constexpr int kTmemCols = 512;                    // two accumulator sets of 2 x 80 columns, three half-block slots of 64
+constexpr int kColSet = 2 * kGemmTok, kColA = 2 * kColSet, kASlots = 3;
+static_assert(kColA + 64 * kASlots <= kTmemCols, "tensor memory");
 
-constexpr int kEpiWarps = 8, kUnpackWarps = 4, kStageWarps = 3;
-constexpr int kWarpUnpack0 = kEpiWarps, kWarpCtrl = kEpiWarps + kUnpackWarps, kWarpStage0 = kWarpCtrl + 1;
-constexpr int kGemmThreads = (kEpiWarps + kUnpackWarps + 1 + kStageWarps) * 32;    // 512
+// warps: epilogue | MMA, two producers, copying stager | unpack | converting stagers
+constexpr int kEpiWarps = 8, kWarpMma = kEpiWarps, kWarpProd0 = kEpiWarps + 1, kWarpUnpack0 = kEpiWarps + 4,
+              kUnpackGroups = 2, kWarpStage0 = kWarpUnpack0 + 4 * kUnpackGroups, kStageWarps = 8;
+// Threads and registers per thread of each role (setmaxnreg). The sum over the warpgroups is at most
+// what the launch holds.
+template <bool RAW>
+struct Cfg {
+  static constexpr int kThreads = (kWarpStage0 + (RAW ? kStageWarps : 0)) * 32;
+  static constexpr int kRegsLaunch = RAW ? 72 : 96, kRegsEpi = RAW ? 112 : 136, kRegsUnpack = RAW ? 56 : 72, kRegsCtrl = RAW ? 56 : 64,
+                       kRegsStage = 56;
+  static_assert(256 * (kRegsEpi + kRegsUnpack + (RAW ? kRegsStage : 0)) + 128 * kRegsCtrl <= kThreads * kRegsLaunch, "registers");
+};
 
 // shared-memory map (bytes)
-constexpr int kOffBar = 0;                                        // mbarriers, tmem base
-constexpr int kOffA = 1024;
-constexpr int kOffB = kOffA + kABufs * kATiles * kTileA;
-constexpr int kOffXd = kOffB + kBBufs * kBTiles * kTileB;         // [kXdRing][64] fp32 activation scales
-constexpr int kOffDd = kOffXd + kXdRing * kGemmTok * 4;           // [kDdRing][128] float2 (d, dmin)
-constexpr int kOffRed = kOffDd + kDdRing * kGemmRows * 8;         // [128][32] floats: one-chunk passes, group 1 -> group 0
-constexpr int kGemmSmem = kOffRed + kGemmRows * 32 * 4;
+constexpr int kOffW = 1024;
+constexpr int kOffB = kOffW + kStages * kStageBytes;
+constexpr int kOffMin = kOffB + 2 * kBBytes;                      // [2][128 rows][16 halfs] min operand
+constexpr int kOffDd = kOffMin + 2 * kMinBytes;                   // [4][128] float2 (d, dmin)
+constexpr int kOffXd = kOffDd + 4 * kGemmRows * 8;                // [4][80] fp32 activation scales
+constexpr int kGemmSmem = kOffXd + 4 * kGemmTok * 4;
 static_assert(kGemmSmem <= 227 * 1024, "shared memory");
 
-enum { kBarAFull = 0, kBarAEmpty = 2, kBarBFull = 4, kBarBEmpty = 7, kBarAccFull = 10, kBarAccEmpty = 12, kBarCount = 14 };
+enum { kBarWFull = 0, kBarWEmpty = kBarWFull + kStages, kBarAFull = kBarWEmpty + kStages, kBarAEmpty = kBarAFull + kASlots,
+       kBarBFull = kBarAEmpty + kASlots, kBarBEmpty = kBarBFull + 2, kBarAccFull = kBarBEmpty + 2,
+       kBarAccEmpty = kBarAccFull + 4,   // full: per epilogue group and set
+        kBarDrain = kBarAccEmpty + 2, kBarCount };
 
-__device__ __forceinline__ uint64_t umma_desc(const void* smem_tile) {
-  // K-major, no swizzle: start >> 4 | LBO (128 B) >> 4 << 16 | SBO (256 B) >> 4 << 32 | version 1 << 46
-  return static_cast<uint64_t>((smem_u32(smem_tile) & 0x3FFFFu) >> 4) | (static_cast<uint64_t>(8) << 16) |
-         (static_cast<uint64_t>(16) << 32) | (static_cast<uint64_t>(1) << 46);
+struct GemmArgs {
+  const unsigned char* const* tab0;    // [n_expert] gate (or the only matrix)
+  const unsigned char* const* tab1;    // [n_expert] up
+  const int* off;                      // [n_expert + 1] grouped slots of each expert
+  const int* rows;                     // activation row of a grouped slot; null: the slot itself
+  const unsigned char* xq;             // Q8_K rows (RAW) or operand rows
+  uint16_t *y, *y1;                    // [slots][n_rows] of tab0 / tab1
+  int n_rows, nb, n_expert;
+  int tiles, group, groups;            // row tiles per matrix, per unit, units per expert and pass
+  const unsigned char *sw0, *sw1, *sxq;   // one more expert over s_rows rows of its own (null: none)
+  uint16_t *sy, *sy1;
+  int s_rows, s_step, s_items;         // its rows, rows per unit, units
+  int n_items;
+  int* status;
+};
+
+// Operand descriptor (K-major, no swizzle) as two words: start >> 4 | LBO (128 B) >> 4 << 16, and
+// SBO (256 B) >> 4 | version 1 << 14. Only the first depends on the tile.
+__device__ __forceinline__ uint32_t umma_desc(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (8u << 16); }
+constexpr uint32_t kDescHi = 16u | (1u << 14);
+// D fp32, A and B fp16, both K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t umma_idesc(int n) {
+  return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(kGemmRows >> 4) << 24);
 }
-// D format s32, A unsigned 8-bit, B signed 8-bit, both K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t umma_idesc_i8(int n) {
-  return (2u << 4) | (0u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
-         (static_cast<uint32_t>(kGemmRows >> 4) << 24);
-}
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc,
-                                        uint32_t accumulate) {
+// A in tensor memory (lane = row, a column holds two consecutive K values) / A in shared memory
+// The whole warp runs the instruction stream, `lead` picks the lane that issues.
+__device__ __forceinline__ void umma_ts(uint32_t lead, uint32_t tmem_d, uint32_t tmem_a, uint32_t db, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u)
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 b, {%2, %5};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "r"(db), "r"(idesc), "r"(accumulate), "r"(kDescHi), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ss(uint32_t lead, uint32_t tmem_d, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(da), "r"(db), "r"(idesc), "r"(accumulate), "r"(kDescHi), "r"(lead)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -89,521 +137,703 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
                    smem_u32(bar))
                : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, int (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
-__device__ __forceinline__ void mbar_arrive_cta(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Bounded wait (as mbar_wait) in a handful of instructions per poll: polls return early whenever something
+// happens in the barrier unit, so with two dozen waiting warps their instructions count.
+__device__ __forceinline__ bool mbar_wait_tight(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b32 n;\n\tmov.b32 n, 0;\n"
+      "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
+      "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, %3;\n\t@q bra POLL;\n"
+      "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity), "r"(1u << 22)
+      : "memory");
+  return ok != 0;
+}
+template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
+// (x & mask) | bits in one instruction
+__device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t mask, uint32_t bits) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(x), "r"(mask), "r"(bits));
+  return d;
+}
+// two packed fp32: each component rounds as the scalar instruction
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(uint32_t lo, uint32_t hi) { f32x2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi)); return d; }
+__device__ __forceinline__ f32x2 splat2(float v) { return pack2(__float_as_uint(v), __float_as_uint(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
+__device__ __forceinline__ float part2(f32x2 v, int hi) {
+  uint32_t a, b;
+  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
+  return __uint_as_float(hi ? b : a);
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {    // one arrival when this thread's copies so far have landed
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // address of (row, 16-byte K half) inside a canonical tile
-__device__ __forceinline__ unsigned char* tile_at(unsigned char* tile, int row, int khalf) {
-  return tile + (row >> 3) * 256 + khalf * 128 + (row & 7) * 16;
-}
+__device__ __forceinline__ int tile_at(int row, int khalf) { return (row >> 3) * 256 + khalf * 128 + (row & 7) * 16; }
 
-// 16 bytes of a weight block: one 128-bit load when the expert's base is 16-byte
-// aligned (the normal case), 32-bit or 16-bit loads otherwise (the pointer-table
-// contract only promises the alignment of the block struct)
-__device__ __forceinline__ uint4 load16(const unsigned char* p, int align) {
-  if (align == 16) return __ldg(reinterpret_cast<const uint4*>(p));
-  uint32_t v[4];
-  if (align == 4) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(p) + i);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint16_t* h = reinterpret_cast<const uint16_t*>(p) + 2 * i;
-      v[i] = static_cast<uint32_t>(__ldg(h)) | (static_cast<uint32_t>(__ldg(h + 1)) << 16);
+// One work unit and the walk over a CTA's units; every role walks the same list on its own.
+struct Unit {
+  const unsigned char *w0, *w1;        // null: the expert is absent
+  const unsigned char* xq;
+  const int* rows;
+  uint16_t *y, *y1;
+  int tile0, n_tiles;                  // row tiles
+  int slot0, nt, n_mma;                // first slot, token rows, MMA N
+};
+struct Walk {
+  int it, m = 0, t0 = 0, step = 0, slot = 0;
+  const unsigned char *w0 = nullptr, *w1 = nullptr;
+  __device__ __forceinline__ explicit Walk(int first) : it(first) {}
+  template <bool DUAL>
+  __device__ __forceinline__ bool next(const GemmArgs& a, Unit& u) {
+    for (; it < a.n_items; it += gridDim.x) {
+      const bool shared = it < a.s_items;
+      const int i = shared ? it : it - a.s_items;
+      const int e = i / a.groups;                     // expert, or pass of the shared one
+      u.tile0 = (i - e * a.groups) * a.group;
+      u.n_tiles = min(a.group, a.tiles - u.tile0);
+      if (shared) {
+        u.w0 = a.sw0; u.w1 = a.sw1; u.xq = a.sxq; u.rows = nullptr; u.y = a.sy; u.y1 = a.sy1;
+        u.slot0 = e * a.s_step;
+        u.nt = min(a.s_step, a.s_rows - u.slot0);
+        it += gridDim.x;
+      } else {
+        if (m == 0) {
+          slot = __ldg(a.off + e);
+          m = __ldg(a.off + e + 1) - slot;
+          if (m <= 0) { m = 0; continue; }
+          w0 = a.tab0[e];
+          w1 = DUAL ? a.tab1[e] : w0;
+          if (w1 == nullptr) w0 = nullptr;
+          t0 = 0;
+          const int passes = (m + kGemmTok - 1) / kGemmTok;
+          step = ((m + passes - 1) / passes + 15) & ~15;
+        }
+        u.w0 = w0; u.w1 = w1; u.xq = a.xq; u.rows = a.rows; u.y = a.y; u.y1 = a.y1;
+        u.slot0 = slot + t0;
+        u.nt = min(step, m - t0);
+        t0 += step;
+        if (t0 >= m) { m = 0; it += gridDim.x; }
+      }
+      u.n_mma = (u.nt + 15) & ~15;
+      return true;
     }
+    return false;
   }
-  return make_uint4(v[0], v[1], v[2], v[3]);
+};
+// The jobs of a unit in order: f(tile, block, matrix, fill) -> false ends the walk. `fill` numbers the
+// activation tiles staged for the unit: one per block when they are shared by gate and up or stay for
+// all row tiles (at most two blocks), else one per (tile, block).
+template <bool DUAL, typename F>
+__device__ __forceinline__ bool for_jobs(const GemmArgs& a, const Unit& u, F f) {
+  int fill = 0;
+#pragma unroll 1
+  for (int t = 0; t < u.n_tiles; ++t) {
+    if (a.nb <= 2) fill = 0;
+#pragma unroll 1
+    for (int b = 0; b < a.nb; ++b, ++fill)
+#pragma unroll 1
+      for (int m = 0; m < (DUAL ? 2 : 1); ++m)
+        if (!f(t, b, m, fill)) return false;
+  }
+  return true;
 }
+__device__ __forceinline__ int fills_of(const GemmArgs& a, const Unit& u) { return a.nb <= 2 ? a.nb : u.n_tiles * a.nb; }
 
-// The jobs of a CTA in the order every role walks them.
-struct JobWalk {
-  int m_e, nb;
-  int pass, blk, ci, nc, j, abk;         // current pass, block column, chunk in pass, chunks in pass, job number, block number
-  __device__ __forceinline__ void start(int m_e_, int nb_) {
-    m_e = m_e_; nb = nb_; pass = 0; blk = 0; ci = 0; j = 0; abk = 0;
-    nc = min(2, (m_e + kGemmTok - 1) / kGemmTok);
-  }
-  __device__ __forceinline__ bool done() const { return pass * 2 * kGemmTok >= m_e; }
-  __device__ __forceinline__ int t0() const { return (2 * pass + ci) * kGemmTok; }
-  __device__ __forceinline__ int nt() const { return min(kGemmTok, m_e - t0()); }
-  __device__ __forceinline__ bool first_of_block() const { return ci == 0; }
-  __device__ __forceinline__ bool last_of_block() const { return ci == nc - 1; }
-  __device__ __forceinline__ void next() {
-    ++j;
-    if (++ci < nc) return;
-    ci = 0; ++abk;
-    if (++blk < nb) return;
-    blk = 0; ++pass;
-    nc = min(2, (m_e - pass * 2 * kGemmTok + kGemmTok - 1) / kGemmTok);
-  }
-};
-
-// One work item: 128 weight rows of one expert against that expert's token rows.
-struct Item {
-  int e, row0, row_off, m_e;
-  const unsigned char* w;
-};
-
-// grid: one CTA per SM (or per item when there are fewer); item i = expert i / tiles, row tile i % tiles.
-// With single_w the kernel serves ONE matrix over single_rows token rows (a dense projection, the shared
-// expert of a prefill chunk): item i = token pass i / tiles (128 rows each), row tile i % tiles.
-__global__ void __launch_bounds__(kGemmThreads, 1)
-grouped_gemm_i8_kernel(const unsigned char* const* __restrict__ w_tab, const int* __restrict__ off,
-                       const unsigned char* __restrict__ xq, uint16_t* __restrict__ y, int n_rows,
-                       int nb, int tiles, int n_items, const unsigned char* single_w, int single_rows,
-                       int* status) {
+template <bool DUAL, bool RAW>
+__global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(const GemmArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  auto item_at = [&](int it) {
-    Item r;
-    r.e = it / tiles;
-    r.row0 = (it - r.e * tiles) * kGemmRows;
-    if (single_w != nullptr) {                   // r.e is the token pass
-      r.row_off = r.e * 2 * kGemmTok;
-      r.m_e = min(2 * kGemmTok, single_rows - r.row_off);
-      r.w = single_w;
-      return r;
-    }
-    r.row_off = __ldg(off + r.e);
-    r.m_e = __ldg(off + r.e + 1) - r.row_off;
-    r.w = w_tab[r.e];
-    return r;
-  };
-  // first item at or after `it` (in this CTA's stride) that has token rows; with `need_w` also weights
-  auto next_item = [&](int it, bool need_w) {
-    for (; it < n_items; it += gridDim.x) {
-      const Item r = item_at(it);
-      if (r.m_e > 0 && (!need_w || r.w != nullptr)) break;
-    }
-    return it;
-  };
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kOffBar);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + kOffBar + 128);
-  int* fail = reinterpret_cast<int*>(smem + kOffBar + 136);
-  unsigned char* a_base = smem + kOffA;
-  unsigned char* b_base = smem + kOffB;
-  float* xd_sm = reinterpret_cast<float*>(smem + kOffXd);
-  float2* dd_sm = reinterpret_cast<float2*>(smem + kOffDd);
-  float* red = reinterpret_cast<float*>(smem + kOffRed);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 512);
+  volatile int* fail = reinterpret_cast<volatile int*>(smem + 516);
+  static_assert(kBarCount * 8 <= 512, "barriers");
 
   if (tid == 0) {
-    for (int i = 0; i < kABufs; ++i) { mbar_init(&bar[kBarAFull + i], kUnpackWarps * 32); mbar_init(&bar[kBarAEmpty + i], 1); }
-    for (int i = 0; i < kBBufs; ++i) { mbar_init(&bar[kBarBFull + i], 32); mbar_init(&bar[kBarBEmpty + i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&bar[kBarAccFull + i], 1); mbar_init(&bar[kBarAccEmpty + i], 4 * 32); }
+    for (int i = 0; i < kStages; ++i) { mbar_init(&bar[kBarWFull + i], 32); mbar_init(&bar[kBarWEmpty + i], 4); }
+    for (int i = 0; i < kASlots; ++i) { mbar_init(&bar[kBarAFull + i], 4); mbar_init(&bar[kBarAEmpty + i], 1); }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar[kBarBFull + i], RAW ? kStageWarps : 32); mbar_init(&bar[kBarBEmpty + i], 1);
+      mbar_init(&bar[kBarAccFull + i], 1); mbar_init(&bar[kBarAccFull + 2 + i], 1);
+      mbar_init(&bar[kBarAccEmpty + i], kEpiWarps / 2);
+    }
+    mbar_init(&bar[kBarDrain], 1);
     *fail = 0;
     fence_barrier_init();
   }
-  if (warp == 0) {
+  if (warp == kWarpMma) {
     __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                     smem_u32(tmem_slot)),
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(kTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  tc_fence_before();
   __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const size_t xrow_bytes = static_cast<size_t>(nb) * kX8;
-  JobWalk jw;
-  auto failed = [&]() { return *reinterpret_cast<volatile int*>(fail) != 0; };
-  // a wait that gives up: flag the CTA, every role leaves its loop at its next wait
-  auto wait = [&](int b, unsigned parity) {
-    if (*reinterpret_cast<volatile int*>(fail)) return false;
-    if (mbar_wait(&bar[b], parity)) return true;
-    *reinterpret_cast<volatile int*>(fail) = 1;
+  // a wait that gives up flags the CTA and ends its role; the others' waits then run out as well
+  auto wait_warp = [&](int b, unsigned parity) {
+    if (__all_sync(0xFFFFFFFFu, mbar_wait_tight(&bar[b], parity)) != 0) return true;
+    *fail = 1;
     return false;
   };
+  const int row_bytes = a.nb * kW4;
+  pdl_wait();                                        // plan and activations come from the kernels before this one
+  pdl_launch_dependents();
+  Walk wk(blockIdx.x);
+  Unit u;
 
-  if (warp >= kWarpUnpack0 && warp < kWarpCtrl) {
-    // ---------------- unpack: this thread's weight row -> operand tiles ----------------
-    const int r = tid - kWarpUnpack0 * 32;
-    auto row_ptr = [&](const Item& I) {
-      const int row = min(I.row0 + r, n_rows - 1);         // ragged last tile: duplicate, never stored
-      return I.w + static_cast<size_t>(row) * nb * kW4;
-    };
-    auto align_of = [](const unsigned char* w) {
-      const uintptr_t wa = reinterpret_cast<uintptr_t>(w);
-      return (wa & 15u) == 0 ? 16 : ((wa & 3u) == 0 ? 4 : 2);
-    };
-    // this thread's whole weight row of an item (nb blocks, contiguous) asked into L2: the loads that
-    // follow an item later find it there instead of waiting for DRAM one block column at a time
-    auto prefetch_row = [&](const unsigned char* p) {
-      const unsigned char* end = p + static_cast<size_t>(nb) * kW4;
-      for (const unsigned char* q = reinterpret_cast<const unsigned char*>(reinterpret_cast<uintptr_t>(p) & ~static_cast<uintptr_t>(127));
-           q < end; q += 128)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
-    };
-    int it = next_item(blockIdx.x, true);
-    uint4 cur[9];
-    if (it < n_items) {
-      const Item I0 = item_at(it);
-      const unsigned char* w0 = row_ptr(I0);
-      const int a0 = align_of(I0.w);
-      prefetch_row(w0);
+  if (warp < kEpiWarps) {
+    // ---------------- epilogue: this thread's weight row of every second tile ----------------
+    // (of the gate or of the up matrix when both run)
+    regs_inc<Cfg<RAW>::kRegsEpi>();
+    const unsigned grp = warp >> 2;
+    const int row = (warp & 3) * 32 + lane;                   // accumulator lane = weight row in the tile
+    const uint32_t lane_base = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const float2* dd_sm = reinterpret_cast<const float2*>(smem + kOffDd) + row;
+    const float* xd_sm = reinterpret_cast<const float*>(smem + kOffXd);
+    f32x2 acc[kGemmTok / 2];                                  // two token columns each
 #pragma unroll
-      for (int i = 0; i < 9; ++i) cur[i] = load16(w0 + 16 * i, a0);
-    }
-    int abk_base = 0;
-    while (it < n_items && !failed()) {
-      const Item I = item_at(it);
-      const unsigned char* wrow = row_ptr(I);
-      const int walign = align_of(I.w);
-      const int it_next = next_item(it + gridDim.x, true);
-      const unsigned char* wrow_next = nullptr;
-      int walign_next = 16;
-      if (it_next < n_items) {
-        const Item In = item_at(it_next);
-        wrow_next = row_ptr(In);
-        walign_next = align_of(In.w);
-        prefetch_row(wrow_next);
+    for (int c = 0; c < kGemmTok / 2; ++c) acc[c] = 0ull;
+    unsigned job = 0, fill0 = 0, tile_no = 0, seen = 0;        // seen: phase of each set's barrier
+    while (wk.next<DUAL>(a, u)) {
+      if (u.w0 == nullptr) {                                   // absent expert: zero rows
+        uint16_t* y = DUAL && grp ? u.y1 : u.y;
+        for (int t = 0; t < u.n_tiles; ++t) {
+          const int r = (u.tile0 + t) * kGemmRows + row;
+          if (r < a.n_rows)
+            for (int c = DUAL ? 0 : grp; c < u.nt; c += DUAL ? 1 : 2) y[static_cast<size_t>(u.slot0 + c) * a.n_rows + r] = 0;
+        }
+        continue;
       }
-      jw.start(I.m_e, nb);
-      int prev_abk = -1;
-      bool gave_up = false;
-      for (; !jw.done(); jw.next()) {
-      if (jw.abk == prev_abk) continue;                     // one unpack per block column
-      prev_abk = jw.abk;
-      const int abk = abk_base + jw.abk;
-      const int buf = abk % kABufs;
-      const unsigned ph = (abk / kABufs) & 1;
-      // the next block column in sequence is requested now: the next column of this row (column 0
-      // again for the next pass), or the first column of the next item's row
-      uint4 nxt[9];
-      {
-        const bool last_col = jw.blk + 1 == nb && (jw.pass + 1) * 2 * kGemmTok >= I.m_e;
-        const unsigned char* wn = last_col ? wrow_next : wrow + static_cast<size_t>(jw.blk + 1 < nb ? jw.blk + 1 : 0) * kW4;
-        const int an = last_col ? walign_next : walign;
-        if (wn != nullptr) {
+      const bool ok = for_jobs<DUAL>(a, u, [&](int t, int b, int m, int fill) {
+        const unsigned j = job++;
+        const int set = j & 1;
+        if ((DUAL ? m : (tile_no + t) & 1) != grp) return true;
+        if (!wait_warp(kBarAccFull + 2 * grp + set, (seen >> set) & 1)) return false;
+        seen ^= 1u << set;
+        tc_fence_after();
+        const float2 dd = dd_sm[(j & 3) * kGemmRows];
+        const f32x2 d2 = splat2(dd.x), nm2 = splat2(-dd.y);
+        const ulonglong2* xd = reinterpret_cast<const ulonglong2*>(xd_sm + ((fill0 + fill) & 3) * kGemmTok);
+        const uint32_t d0 = lane_base + set * kColSet;
 #pragma unroll
-          for (int i = 0; i < 9; ++i) nxt[i] = load16(wn + 16 * i, an);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 9; ++i) nxt[i] = make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-      if (!wait(kBarAEmpty + buf, ph ^ 1u)) { gave_up = true; break; }
-      unsigned char* a_tiles = a_base + static_cast<size_t>(buf) * kATiles * kTileA;
-      const uint4 hdr = cur[0];
-      const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x & 0xFFFFu)));
-      const float dmin = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x >> 16)));
-      const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const uint4 q0 = cur[1 + 2 * g], q1 = cur[2 + 2 * g];
-        const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const uint32_t sc_e = (s6.sc[g >> 1] >> (16 * (g & 1))) & 0xFFu;        // sub-block 2g
-        const uint32_t sc_o = (s6.sc[g >> 1] >> (16 * (g & 1) + 8)) & 0xFFu;    // sub-block 2g+1
-        const uint32_t be = sc_e & 7u, ae = sc_e >> 3, bo = sc_o & 7u, ao = sc_o >> 3;
-        uint32_t tb_e[8], ta_e[8], tb_o[8], ta_o[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t lo = raw[i] & 0x0F0F0F0Fu, hi = (raw[i] >> 4) & 0x0F0F0F0Fu;
-          tb_e[i] = lo * be; ta_e[i] = lo * ae;            // bytes <= 105: no carry between bytes
-          tb_o[i] = hi * bo; ta_o[i] = hi * ao;
-        }
-        unsigned char* t0p = a_tiles + (4 * g + 0) * kTileA;   // tile order: [sub-block][b part, a part]
-        unsigned char* t1p = a_tiles + (4 * g + 1) * kTileA;
-        unsigned char* t2p = a_tiles + (4 * g + 2) * kTileA;
-        unsigned char* t3p = a_tiles + (4 * g + 3) * kTileA;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          *reinterpret_cast<uint4*>(tile_at(t0p, r, h)) = make_uint4(tb_e[4 * h], tb_e[4 * h + 1], tb_e[4 * h + 2], tb_e[4 * h + 3]);
-          *reinterpret_cast<uint4*>(tile_at(t1p, r, h)) = make_uint4(ta_e[4 * h], ta_e[4 * h + 1], ta_e[4 * h + 2], ta_e[4 * h + 3]);
-          *reinterpret_cast<uint4*>(tile_at(t2p, r, h)) = make_uint4(tb_o[4 * h], tb_o[4 * h + 1], tb_o[4 * h + 2], tb_o[4 * h + 3]);
-          *reinterpret_cast<uint4*>(tile_at(t3p, r, h)) = make_uint4(ta_o[4 * h], ta_o[4 * h + 1], ta_o[4 * h + 2], ta_o[4 * h + 3]);
-        }
-      }
-      {  // min tile: the eight min bytes at k = 0..7, zeros elsewhere
-        unsigned char* t_mn = a_tiles + 16 * kTileA;
-        *reinterpret_cast<uint4*>(tile_at(t_mn, r, 0)) = make_uint4(s6.mn[0], s6.mn[1], 0u, 0u);
-        *reinterpret_cast<uint4*>(tile_at(t_mn, r, 1)) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      dd_sm[(abk % kDdRing) * kGemmRows + r] = make_float2(d, dmin);
-      fence_proxy_async();                                 // operand tiles -> visible to the tensor core
-      mbar_arrive_cta(&bar[kBarAFull + buf]);
-#pragma unroll
-      for (int i = 0; i < 9; ++i) cur[i] = nxt[i];
-      }   // block columns of the item
-      if (gave_up) break;
-      abk_base += jw.abk;
-      it = it_next;
-    }
-  } else if (warp >= kWarpStage0) {
-    // ---------------- stagers: activation codes, split sums and scales of a job's chunk ----------------
-    // Each of the three stager warps takes every third job; a lane owns token rows `lane` and
-    // `lane + 32` of the chunk. The 256 codes of a packed Q8_K block start 4 bytes into the
-    // 276-byte block, so their 16-byte pieces are not aligned: the lane reads the 17 aligned
-    // pieces that cover them and picks each operand piece out of two neighbours by whole words.
-    const int sg = warp - kWarpStage0;
-    int j_base = 0;
-    bool ok = true;
-    for (int it = next_item(blockIdx.x, true); it < n_items && !failed(); it = next_item(it + gridDim.x, true)) {
-    const Item I = item_at(it);
-    const int row_off = I.row_off;
-    jw.start(I.m_e, nb);
-    for (; !jw.done(); jw.next()) {
-      const int j = j_base + jw.j, buf = j % kBBufs;
-      if (j % kStageWarps != sg) continue;
-      const unsigned ph = (j / kBBufs) & 1;
-      const int t0 = jw.t0(), nt = jw.nt();
-      unsigned char* b_tiles = b_base + static_cast<size_t>(buf) * kBTiles * kTileB;
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        const int s = lane + 32 * half;                    // token row of the chunk
-        uint4 wv[17];
-        uint32_t pf[5] = {0u, 0u, 0u, 0u, 0u};             // scale, four words of sub-block sums
-        int sh = 0;
-        if (s < nt) {                                       // requested before the buffer is known to be free
-          const unsigned char* xb = xq + static_cast<size_t>(row_off + t0 + s) * xrow_bytes + static_cast<size_t>(jw.blk) * kX8;
-          const uintptr_t cs = reinterpret_cast<uintptr_t>(xb) + 4;
-          sh = static_cast<int>(cs & 15u) >> 2;
-          const uint4* a0 = reinterpret_cast<const uint4*>(cs & ~static_cast<uintptr_t>(15));
-#pragma unroll
-          for (int i = 0; i < 17; ++i) wv[i] = __ldg(a0 + i);
-          pf[0] = __ldg(reinterpret_cast<const uint32_t*>(xb));
-          const uint32_t* bs = reinterpret_cast<const uint32_t*>(xb + 260);       // 8 x int16
-          pf[1] = __ldg(bs); pf[2] = __ldg(bs + 1); pf[3] = __ldg(bs + 2); pf[4] = __ldg(bs + 3);
-        }
-        if (half == 0) {
-          ok = __all_sync(0xFFFFFFFFu, wait(kBarBEmpty + buf, ph ^ 1u));
-          if (!ok) break;
-        }
-        if (s < nt) {
-          auto put = [&](int c, uint32_t a, uint32_t b, uint32_t cc, uint32_t d) {
-            *reinterpret_cast<uint4*>(tile_at(b_tiles + (c >> 1) * kTileB, s, c & 1)) = make_uint4(a, b, cc, d);
-          };
-          if (sh == 0) {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) put(c, wv[c].x, wv[c].y, wv[c].z, wv[c].w);
-          } else if (sh == 1) {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) put(c, wv[c].y, wv[c].z, wv[c].w, wv[c + 1].x);
-          } else if (sh == 2) {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) put(c, wv[c].z, wv[c].w, wv[c + 1].x, wv[c + 1].y);
-          } else {
-#pragma unroll
-            for (int c = 0; c < 16; ++c) put(c, wv[c].w, wv[c + 1].x, wv[c + 1].y, wv[c + 1].z);
-          }
-        }
-        {                                                   // sums split as bsum = 128*hi + lo; rows beyond nt: zero scale
-          uint32_t lo01 = 0, lo23 = 0, hi01 = 0, hi23 = 0;
-          float xd = 0.f;
-          if (s < nt) {
-            xd = __uint_as_float(pf[0]);
-            lo01 = __byte_perm(pf[1] & 0x007F007Fu, pf[2] & 0x007F007Fu, 0x6420);
-            lo23 = __byte_perm(pf[3] & 0x007F007Fu, pf[4] & 0x007F007Fu, 0x6420);
-            hi01 = __byte_perm((pf[1] >> 7) & 0x00FF00FFu, (pf[2] >> 7) & 0x00FF00FFu, 0x6420);
-            hi23 = __byte_perm((pf[3] >> 7) & 0x00FF00FFu, (pf[4] >> 7) & 0x00FF00FFu, 0x6420);
-          }
-          xd_sm[(j % kXdRing) * kGemmTok + s] = xd;
-          *reinterpret_cast<uint4*>(tile_at(b_tiles + 8 * kTileB, s, 0)) = make_uint4(lo01, lo23, 0u, 0u);
-          *reinterpret_cast<uint4*>(tile_at(b_tiles + 8 * kTileB, s, 1)) = make_uint4(0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(tile_at(b_tiles + 9 * kTileB, s, 0)) = make_uint4(hi01, hi23, 0u, 0u);
-          *reinterpret_cast<uint4*>(tile_at(b_tiles + 9 * kTileB, s, 1)) = make_uint4(0u, 0u, 0u, 0u);
-        }
-      }
-      if (!ok) break;
-      fence_proxy_async();
-      mbar_arrive_cta(&bar[kBarBFull + buf]);
-    }
-    if (!ok) break;
-    j_base += jw.j;
-    }   // items
-  } else if (warp == kWarpCtrl) {
-    // ---------------- MMA issue: one elected thread ----------------
-    if (lane == 0) {
-      int j_base = 0, abk_base = 0;
-      unsigned use[2] = {0u, 0u};                           // jobs issued so far into each accumulator set
-      bool ok = true;
-      for (int it = next_item(blockIdx.x, true); it < n_items && ok; it = next_item(it + gridDim.x, true)) {
-      const Item I = item_at(it);
-      jw.start(I.m_e, nb);
-      for (; !jw.done(); jw.next()) {
-        const int j = j_base + jw.j, abk = abk_base + jw.abk;
-        const int abuf = abk % kABufs, bbuf = j % kBBufs, set = jw.j & 1;
-        ok = false;
-        if (jw.first_of_block() && !wait(kBarAFull + abuf, (abk / kABufs) & 1)) break;
-        if (!wait(kBarBFull + bbuf, (j / kBBufs) & 1)) break;
-        if (!wait(kBarAccEmpty + set, (use[set] & 1u) ^ 1u)) break;
-        ok = true;
-        ++use[set];
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // descriptors of consecutive tiles differ by the tile size in the address field
-        const uint64_t da0 = umma_desc(a_base + static_cast<size_t>(abuf) * kATiles * kTileA);
-        const uint64_t db0 = umma_desc(b_base + static_cast<size_t>(bbuf) * kBTiles * kTileB);
-        constexpr uint64_t kStepA = kTileA >> 4, kStepB = kTileB >> 4;
-        const int n_mma = (jw.nt() + 15) & ~15;             // MMA N: multiple of 16
-        const uint32_t idesc = umma_idesc_i8(n_mma);
-        const uint32_t acc = tmem + set * 4 * kGemmTok;
-        // D0 = sum (b*q) x, D1 = sum (a*q) x, D2 = min x sums_lo, D3 = min x sums_hi
-#pragma unroll
-        for (int sb = 0; sb < 8; ++sb) {
-          umma_i8(acc + 0 * kGemmTok, da0 + (2 * sb) * kStepA, db0 + sb * kStepB, idesc, sb > 0);
-          umma_i8(acc + 1 * kGemmTok, da0 + (2 * sb + 1) * kStepA, db0 + sb * kStepB, idesc, sb > 0);
-        }
-        umma_i8(acc + 2 * kGemmTok, da0 + 16 * kStepA, db0 + 8 * kStepB, idesc, 0u);
-        umma_i8(acc + 3 * kGemmTok, da0 + 16 * kStepA, db0 + 9 * kStepB, idesc, 0u);
-        umma_commit(&bar[kBarAccFull + set]);               // accumulators ready for the epilogue
-        umma_commit(&bar[kBarBEmpty + bbuf]);               // B tiles free
-        if (jw.last_of_block()) umma_commit(&bar[kBarAEmpty + abuf]);   // A tiles free
-      }
-      j_base += jw.j;
-      abk_base += jw.abk;
-      }   // items
-    }
-  } else {
-    // ---------------- epilogue: two groups of four warps; this thread's row, the job's tokens ----------------
-    const int grp = warp >> 2;
-    const int row = (warp & 3) * 32 + lane;                // accumulator lane = weight row in the tile
-    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    float acc[kGemmTok];
-#pragma unroll
-    for (int t = 0; t < kGemmTok; ++t) acc[t] = 0.f;
-    bool ok = true;
-    int j_base = 0, abk_base = 0;
-    unsigned use = 0u;                                     // jobs this group has finished (the phase of its accumulator set)
-    for (int it = next_item(blockIdx.x, false); it < n_items; it = next_item(it + gridDim.x, false)) {
-    const Item I = item_at(it);
-    const int row0 = I.row0, row_off = I.row_off, m_e = I.m_e;
-    if (I.w == nullptr) {                                    // absent expert: zero rows
-      for (int i = tid; i < m_e * kGemmRows; i += kEpiWarps * 32) {
-        const int t = i / kGemmRows, r = row0 + (i % kGemmRows);
-        if (r < n_rows) y[static_cast<size_t>(row_off + t) * n_rows + r] = 0;
-      }
-      continue;
-    }
-    jw.start(m_e, nb);
-    int pass_t0 = 0, pass_nc = jw.nc, pass_nt0 = 0, pass_nt1 = 0, cur_pass = 0;
-    auto flush = [&]() {
-      // end of a pass: one chunk -> group 1 hands its sums to group 0 through shared memory
-      // (two halves of 32 tokens); two chunks -> each group stores its own chunk
-      const bool valid = row0 + row < n_rows && ok && !failed();
-      if (pass_nc == 1) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          if (grp == 1) {
-#pragma unroll
-            for (int t = 0; t < 32; ++t) red[t * kGemmRows + row] = acc[32 * half + t];
-          }
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          if (grp == 0) {
-#pragma unroll
-            for (int t = 0; t < 32; ++t) acc[32 * half + t] += red[t * kGemmRows + row];
-          }
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-        }
-        if (grp == 0 && valid) {
-#pragma unroll
-          for (int t = 0; t < kGemmTok; ++t)
-            if (t < pass_nt0) y[static_cast<size_t>(row_off + pass_t0 + t) * n_rows + row0 + row] = f2h(acc[t]);
-        }
-      } else if (valid) {
-        const int nt = grp == 0 ? pass_nt0 : pass_nt1;
-        const int t0 = pass_t0 + grp * kGemmTok;
-#pragma unroll
-        for (int t = 0; t < kGemmTok; ++t)
-          if (t < nt) y[static_cast<size_t>(row_off + t0 + t) * n_rows + row0 + row] = f2h(acc[t]);
-      }
-#pragma unroll
-      for (int t = 0; t < kGemmTok; ++t) acc[t] = 0.f;
-    };
-    pass_nt0 = min(kGemmTok, m_e);
-    pass_nt1 = min(kGemmTok, max(0, m_e - kGemmTok));
-    for (; !jw.done(); jw.next()) {
-      if (jw.pass != cur_pass) {                            // both groups see the pass change at the same job
-        flush();
-        cur_pass = jw.pass;
-        pass_t0 = cur_pass * 2 * kGemmTok;
-        pass_nc = jw.nc;
-        pass_nt0 = min(kGemmTok, m_e - pass_t0);
-        pass_nt1 = min(kGemmTok, max(0, m_e - pass_t0 - kGemmTok));
-      }
-      if ((jw.j & 1) != grp || !ok) continue;              // (a group that gave up still walks the list: the
-                                                            //  barriers of the pass ends need both groups)
-      const int j = j_base + jw.j, abk = abk_base + jw.abk;
-      if (!__all_sync(0xFFFFFFFFu, wait(kBarAccFull + grp, use & 1u))) { ok = false; continue; }
-      ++use;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const float2 dd = dd_sm[(abk % kDdRing) * kGemmRows + row];
-      const float* xd = xd_sm + (j % kXdRing) * kGemmTok;
-      const int n_mma = (jw.nt() + 15) & ~15;
-      const uint32_t accp = tmem + lane_base + grp * 4 * kGemmTok;
-#pragma unroll
-      for (int c0 = 0; c0 < kGemmTok; c0 += 16) {
-        if (c0 < n_mma) {
-          int vb[16], va[16], mlo[16], mhi[16];
-          tmem_ld16(accp + 0 * kGemmTok + c0, vb);
-          tmem_ld16(accp + 1 * kGemmTok + c0, va);
-          tmem_ld16(accp + 2 * kGemmTok + c0, mlo);
-          tmem_ld16(accp + 3 * kGemmTok + c0, mhi);
+        for (int c = 0; c < kGemmTok; c += 8) {
+          if (c >= u.n_mma) break;
+          uint32_t v0[8], v1[8];
+          tmem_ld8(d0 + c, v0);
+          tmem_ld8(d0 + kGemmTok + c, v1);
+          const ulonglong2 xa = xd[c / 4], xb = xd[c / 4 + 1];
+          const f32x2 xv[4] = {xa.x, xa.y, xb.x, xb.y};
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            const int isum = vb[q] + 8 * va[q];
-            const int msum = mlo[q] + 128 * mhi[q];
-            acc[c0 + q] += xd[c0 + q] * (dd.x * static_cast<float>(isum) - dd.y * static_cast<float>(msum));
+          for (int q = 0; q < 4; ++q)           // acc += xd * (d * D0 - dmin * D1)
+            acc[c / 2 + q] = fma2(xv[q], fma2(nm2, pack2(v1[2 * q], v1[2 * q + 1]), mul2(d2, pack2(v0[2 * q], v0[2 * q + 1]))), acc[c / 2 + q]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_one(&bar[kBarAccEmpty + set]);
+        if (b + 1 == a.nb) {                                   // the tile is complete
+          const int r = (u.tile0 + t) * kGemmRows + row;
+          uint16_t* yp = (DUAL && grp ? u.y1 : u.y) + static_cast<size_t>(u.slot0) * a.n_rows + r;
+          const int n_left = r < a.n_rows ? u.nt : 0;
+#pragma unroll
+          for (int c = 0; c < kGemmTok; c += 8) {
+            if (c >= u.n_mma) break;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t h = h2_bits(__floats2half2_rn(part2(acc[c / 2 + q], 0), part2(acc[c / 2 + q], 1)));
+              if (c + 2 * q < n_left) yp[0] = static_cast<uint16_t>(h & 0xFFFFu);
+              if (c + 2 * q + 1 < n_left) yp[a.n_rows] = static_cast<uint16_t>(h >> 16);
+              yp += 2 * a.n_rows;
+              acc[c / 2 + q] = 0ull;
+            }
           }
         }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      mbar_arrive_cta(&bar[kBarAccEmpty + grp]);
+        return true;
+      });
+      if (!ok) break;
+      fill0 += fills_of(a, u);
+      tile_no += u.n_tiles;
     }
-    flush();
-    j_base += jw.j;
-    abk_base += jw.abk;
-    }   // items
+  } else if (warp >= kWarpUnpack0 && warp < kWarpStage0) {
+    // ---------------- unpack: this thread's weight row of a block -> tensor memory ----------------
+    // Group g of four warps takes jobs g, g + G, ... The halves of a job (sub-blocks 0-3 / 4-7) go round three
+    // slots of tensor memory: half 2j + h into slot (2j + h) mod 3. (Two groups are as far ahead of the
+    // tensor core as they can be: a third one's first wait could take a slot's phase for the one before it.)
+    regs_dec<Cfg<RAW>::kRegsUnpack>();
+    constexpr int G = kUnpackGroups;
+    const int grp = (warp - kWarpUnpack0) >> 2;
+    const int r = (warp & 3) * 32 + lane;
+    const uint32_t a_base = tmem + kColA + (static_cast<uint32_t>((warp & 3) * 32) << 16);
+    const __half2 k1024 = __float2half2_rn(1024.f), n1024 = __float2half2_rn(-1024.f), n64 = __float2half2_rn(-64.f);
+    const __half2 k16th = __float2half2_rn(0.0625f);
+    const uint32_t mlo = 0x000F000Fu, mhi = 0x00F000F0u, magic = 0x64006400u;
+    int to_mine = grp;                                           // jobs until this group's next one
+    unsigned job = grp;                                          // its number
+    int st = grp % kStages, slot = 2 * grp % kASlots;            // its ring stage and first slot
+    unsigned st_ph = 0, slot_ph = 1u ^ ((2 * grp / kASlots) & 1);
+    bool ok = true;
+    while (ok && wk.next<DUAL>(a, u)) {
+      if (u.w0 == nullptr) continue;
+      const int n_jobs = u.n_tiles * a.nb * (DUAL ? 2 : 1);
+#pragma unroll 1
+      for (; to_mine < n_jobs; to_mine += G) {
+        if (!(ok = wait_warp(kBarWFull + st, st_ph))) break;
+        const uint4* blk = reinterpret_cast<const uint4*>(smem + kOffW + st * kStageBytes + r * kW4);
+        const uint4 hdr = blk[0];
+        const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
+        uint32_t scw = s6.sc[0];
+#pragma unroll 1
+        for (int g = 0; g < 4; ++g) {
+          const uint4 q0 = blk[1], q1 = blk[2];
+          blk += 2;
+          const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+          // scales of the two sub-blocks of a 32-byte group, splat; nibbles enter as 1024 + q and 1024 + 16 q
+          const __half2 se = __hsub2(bits_h2(__byte_perm(scw, 0x64646464u, 0x4040)), k1024);
+          const __half2 so = __hsub2(bits_h2(__byte_perm(scw, 0x64646464u, 0x4141)), k1024);
+          const __half2 ce = __hmul2(se, n1024), so16 = __hmul2(so, k16th), co = __hmul2(so, n64);
+          scw = g == 1 ? s6.sc[1] : scw >> 16;
+          if ((g & 1) == 0) {
+            if (!(ok = wait_warp(kBarAEmpty + slot, slot_ph))) break;
+            tc_fence_after();
+          }
+          const uint32_t dst = a_base + slot * 64 + (g & 1) * 32;
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) {
+            uint32_t v[8], w[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t odd = raw[i + q] >> 8;
+              v[2 * q] = h2_bits(__hfma2(bits_h2(and_or(raw[i + q], mlo, magic)), se, ce));
+              v[2 * q + 1] = h2_bits(__hfma2(bits_h2(and_or(odd, mlo, magic)), se, ce));
+              w[2 * q] = h2_bits(__hfma2(bits_h2(and_or(raw[i + q], mhi, magic)), so16, co));
+              w[2 * q + 1] = h2_bits(__hfma2(bits_h2(and_or(odd, mhi, magic)), so16, co));
+            }
+            tmem_st8(dst + 2 * i, v);
+            tmem_st8(dst + 16 + 2 * i, w);
+          }
+          if (g == 0) {                                          // min operand and block scales of this job
+            uint32_t mn[4], mn64[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const __half2 p = __hsub2(bits_h2(__byte_perm(s6.mn[i >> 1], 0x64646464u, (i & 1) ? 0x4342 : 0x4140)), k1024);
+              mn[i] = h2_bits(p);
+              mn64[i] = h2_bits(__hmul2(p, __float2half2_rn(64.f)));
+            }
+            unsigned char* min_sm = smem + kOffMin + (job & 1) * kMinBytes;
+            *reinterpret_cast<uint4*>(min_sm + tile_at(r, 0)) = make_uint4(mn[0], mn[1], mn[2], mn[3]);
+            *reinterpret_cast<uint4*>(min_sm + tile_at(r, 1)) = make_uint4(mn64[0], mn64[1], mn64[2], mn64[3]);
+            reinterpret_cast<float2*>(smem + kOffDd)[(job & 3) * kGemmRows + r] =
+                make_float2(h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), h2f(static_cast<uint16_t>(hdr.x >> 16)));
+            fence_proxy_async();                                 // min operand -> visible to the tensor core
+          }
+          if (g & 1) {
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(&bar[kBarAFull + slot]);
+            if (g == 1 && ++slot == kASlots) { slot = 0; slot_ph ^= 1u; }
+          }
+        }
+        if (!ok) break;
+        if (lane == 0) mbar_arrive_one(&bar[kBarWEmpty + st]);         // the stage has been read
+        job += G;
+        st += G;
+        if (st >= kStages) { st -= kStages; st_ph ^= 1u; }
+        slot += 2 * G - 1;                                       // from the second half to the next job's first
+        while (slot >= kASlots) { slot -= kASlots; slot_ph ^= 1u; }
+      }
+      to_mine -= n_jobs;
+    }
+  } else if (warp < kWarpUnpack0) {
+    regs_dec<Cfg<RAW>::kRegsCtrl>();
+    if (warp == kWarpMma) {
+      // ---------------- MMA issue: the whole warp walks, one elected lane issues ----------------
+      // (operands computed by the whole warp stay in uniform registers: 15 to 41 cycles per MMA for N = 16 to 80,
+      // against 45 at least when a lone thread computes and issues)
+      unsigned job = 0, fill0 = 0, tile_no = 0;
+      int slot = 0;
+      unsigned slot_ph = 0;
+      const uint32_t d_min = umma_desc(smem_u32(smem + kOffMin)), d_b = umma_desc(smem_u32(smem + kOffB));
+      bool ok = true;
+      while (ok && wk.next<DUAL>(a, u)) {
+        if (u.w0 == nullptr) continue;
+        const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc(u.n_mma), 0);
+        ok = for_jobs<DUAL>(a, u, [&](int t, int, int m, int fill) {
+          const unsigned set = job & 1, f = fill0 + fill, buf = f & 1;
+          if (!DUAL || m == 0) {
+            if (!wait_warp(kBarBFull + buf, (f >> 1) & 1)) return false;
+            if (!RAW) fence_proxy_async();                       // copied tiles (cp.async is generic) -> the tensor core
+          }
+          if (!wait_warp(kBarAccEmpty + set, ((job >> 1) & 1) ^ 1u)) return false;
+          const uint32_t db = d_b + buf * (kBBytes >> 4), dm = d_min + set * (kMinBytes >> 4);
+          const uint32_t d0 = tmem + set * kColSet, d1 = d0 + kGemmTok;
+          // the activation tiles are free after their last job
+          const bool last_use = DUAL ? m == 1 : (a.nb > 2 || t + 1 == u.n_tiles);
+          uint32_t dk = db;
+#pragma unroll 1
+          for (int h = 0; h < 2; ++h) {
+            if (!wait_warp(kBarAFull + slot, slot_ph)) return false;
+            tc_fence_after();
+            uint32_t ta = tmem + kColA + slot * 64;
+            const uint32_t lead = elect_one();
+#pragma unroll 1
+            for (int k = 0; k < 8; k += 2) {
+              umma_ts(lead, d0, ta, dk, idesc, h | k);
+              umma_ts(lead, d0, ta + 8, dk + (kBTile >> 4), idesc, 1u);
+              ta += 16;
+              dk += 2 * (kBTile >> 4);
+            }
+            if (h == 1) umma_ss(lead, d1, dm, dk, idesc, 0u);
+            if (lead) {
+              umma_commit(&bar[kBarAEmpty + slot]);
+              if (h == 1) {
+                umma_commit(&bar[kBarAccFull + 2 * (DUAL ? m : (tile_no + t) & 1) + set]);
+                if (last_use) umma_commit(&bar[kBarBEmpty + buf]);
+              }
+            }
+            __syncwarp();
+            if (++slot == kASlots) { slot = 0; slot_ph ^= 1u; }
+          }
+          ++job;
+          return true;
+        });
+        fill0 += fills_of(a, u);
+        tile_no += u.n_tiles;
+      }
+      if (elect_one()) umma_commit(&bar[kBarDrain]);             // everything issued has finished before tensor memory goes back
+      mbar_wait_tight(&bar[kBarDrain], 0);
+    } else if (warp < kWarpProd0 + 2) {
+      // ---------------- producers: block columns of 128 rows into the ring, alternate jobs ----------------
+      // 16-byte piece p = 9 * row + c of a stage goes to lane p % 32; nine steps of 32 pieces are 32 rows, so a lane
+      // keeps the source offsets of nine steps.
+      const unsigned p = warp - kWarpProd0;
+      uint32_t offs[9];
+#pragma unroll
+      for (int q = 0; q < 9; ++q) offs[q] = (q * 32 + lane) / 9 * row_bytes + (q * 32 + lane) % 9 * 16;
+      unsigned job = 0, st = 0, st_ph = 1;
+      while (wk.next<DUAL>(a, u)) {
+        if (u.w0 == nullptr) continue;
+        const bool ok = for_jobs<DUAL>(a, u, [&](int t, int b, int m, int) {
+          const unsigned s = st, ph = st_ph;
+          if (++st == kStages) { st = 0; st_ph ^= 1u; }
+          if ((job++ & 1) != p) return true;
+          if (!wait_warp(kBarWEmpty + s, ph)) return false;
+          const unsigned char* base = m == 0 ? u.w0 : u.w1;
+          const int row0 = (u.tile0 + t) * kGemmRows;
+          const unsigned char* src = base + static_cast<size_t>(row0) * row_bytes + b * kW4;
+          const uint32_t dst = smem_u32(smem + kOffW + s * kStageBytes) + lane * 16;
+          if ((reinterpret_cast<uintptr_t>(base) & 15u) == 0 && row0 + kGemmRows <= a.n_rows) {
+#pragma unroll 1
+            for (int g = 0; g < 4; ++g) {
+#pragma unroll
+              for (int q = 0; q < 9; ++q) cp_async16(dst + (g * 9 + q) * 512, src + offs[q]);
+              src += 32 * row_bytes;
+            }
+            cp_async_arrive(&bar[kBarWFull + s]);
+          } else {                                               // ragged last tile, or a base off a 16-byte boundary
+            const int last = a.n_rows - 1 - row0;                // rows past the matrix repeat its last one: never stored
+            unsigned char* d = smem + kOffW + s * kStageBytes + lane * 16;
+#pragma unroll 1
+            for (int q = 0; q < kStageBytes / 512; ++q) {
+              const int pc = q * 32 + lane;
+              const uint16_t* x = reinterpret_cast<const uint16_t*>(src + min(pc / 9, last) * row_bytes + pc % 9 * 16);
+              uint32_t v[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) v[i] = static_cast<uint32_t>(__ldg(x + 2 * i)) | (static_cast<uint32_t>(__ldg(x + 2 * i + 1)) << 16);
+              *reinterpret_cast<uint4*>(d + q * 512) = make_uint4(v[0], v[1], v[2], v[3]);
+            }
+            mbar_arrive_one(&bar[kBarWFull + s]);
+          }
+          return true;
+        });
+        if (!ok) break;
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else if constexpr (!RAW) {
+      // ---------------- copying stager: operand rows of one block, 16 bytes per lane and step ----------------
+      // lane = (row of eight, one of four 16-byte pieces); a group of eight rows is 8.5 steps
+      const int r8 = lane & 7, pc = lane >> 3;
+      constexpr int kGroups = kGemmTok / 8, kGroups32 = (kGemmTok + 31) / 32;
+      const size_t xrow_bytes = static_cast<size_t>(a.nb) * kOpBlk;
+      const uint32_t lane_dst = smem_u32(smem + kOffB) + (pc >> 1) * kBTile + tile_at(r8, pc & 1);
+      const uint32_t xd_dst = smem_u32(smem + kOffXd) + lane * 4;
+      unsigned fill = 0;
+      while (wk.next<DUAL>(a, u)) {
+        if (u.w0 == nullptr) continue;
+        auto row_of = [&](int t) {
+          const int s = u.slot0 + min(t, u.nt - 1);             // columns past the last row repeat it; never stored
+          return u.rows != nullptr ? __ldg(u.rows + s) : s;
+        };
+          int row[kGroups32];                                     // of tokens lane, lane + 32, ...
+#pragma unroll
+        for (int g = 0; g < kGroups32; ++g) row[g] = row_of(g * 32 + lane);
+        const int n_fills = fills_of(a, u);
+        bool ok = true;
+        int blk = 0;
+#pragma unroll 1
+        for (int f = 0; f < n_fills; ++f, ++fill) {
+          const int buf = fill & 1;
+          ok = wait_warp(kBarBEmpty + buf, ((fill >> 1) & 1) ^ 1u);
+          if (!ok) break;
+          const unsigned char* src = u.xq + static_cast<size_t>(blk) * kOpBlk;
+          if (++blk == a.nb) blk = 0;
+          const uint32_t dst = lane_dst + buf * kBBytes;
+#pragma unroll
+          for (int g = 0; g < kGroups; ++g)
+            if (g * 8 < u.n_mma) {
+              const unsigned char* xb = src + __shfl_sync(0xFFFFFFFFu, row[g / 4], (g & 3) * 8 + r8) * xrow_bytes + pc * 16;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) cp_async16(dst + g * 256 + q * 2 * kBTile, xb + q * 64);
+              if (pc < 2) cp_async16(dst + g * 256 + 16 * kBTile, xb + 512);
+            }
+#pragma unroll
+          for (int g = 0; g < kGroups32; ++g)
+            if (g * 32 + lane < u.n_mma)
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(xd_dst + ((fill & 3) * kGemmTok + g * 32) * 4),
+                           "l"(src + row[g] * xrow_bytes + 544)
+                           : "memory");
+          cp_async_arrive(&bar[kBarBFull + buf]);
+        }
+        if (!ok) break;
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+  } else if constexpr (RAW) {
+    // ---------------- converting stagers: one block of the unit's Q8_K rows -> operand tiles ----------------
+    // Warp w takes 64 codes of every second group of eight rows, a lane 16 codes of one row of a group (blocks of
+    // 276 bytes start on 4-byte boundaries: word loads), and thread i the sums and the scale of row i. A fill's
+    // loads are issued before its buffer is awaited.
+    regs_dec<Cfg<RAW>::kRegsStage>();
+    const int w = (warp - kWarpStage0) & 3, gh = (warp - kWarpStage0) >> 2, i = tid - kWarpStage0 * 32;
+    const int r8 = lane & 7, pc = lane >> 3;
+    constexpr int kGroups = kGemmTok / 16;                      // row groups per warp
+    const size_t xrow_bytes = static_cast<size_t>(a.nb) * kX8;
+    float* xd_sm = reinterpret_cast<float*>(smem + kOffXd);
+    const __half2 m1152 = __float2half2_rn(-1152.f), m1024 = __float2half2_rn(-1024.f);
+    unsigned fill = 0;
+    while (wk.next<DUAL>(a, u)) {
+      if (u.w0 == nullptr) continue;
+      auto row_of = [&](int t) {
+        const int s = u.slot0 + min(t, u.nt - 1);               // columns past the last row repeat it; never stored
+        return u.rows != nullptr ? __ldg(u.rows + s) : s;
+      };
+      const int n_fills = fills_of(a, u);
+      int row[kGroups];
+#pragma unroll
+      for (int g = 0; g < kGroups; ++g) row[g] = row_of((2 * g + gh) * 8 + r8);
+      const int row_i = row_of(i);
+      bool ok = true;
+      int blk = 0;
+#pragma unroll 1
+      for (int f = 0; f < n_fills; ++f, ++fill) {
+        const int buf = fill & 1;
+        unsigned char* tiles = smem + kOffB + buf * kBBytes;
+        const unsigned char* xblk = u.xq + static_cast<size_t>(blk) * kX8;
+        if (++blk == a.nb) blk = 0;
+        uint32_t cw[kGroups][4];
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g)
+          if ((2 * g + gh) * 8 < u.n_mma) {
+            const uint32_t* xb = reinterpret_cast<const uint32_t*>(xblk + row[g] * xrow_bytes) + 1 + w * 16 + pc * 4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) cw[g][q] = __ldg(xb + q);
+          }
+        uint32_t sums[5] = {0u, 0u, 0u, 0u, 0u};                // scale, four words of sub-block sums
+        if (i < u.n_mma) {
+          const uint32_t* xb = reinterpret_cast<const uint32_t*>(xblk + row_i * xrow_bytes);
+          sums[0] = __ldg(xb);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) sums[1 + q] = __ldg(xb + 65 + q);
+        }
+        ok = wait_warp(kBarBEmpty + buf, ((fill >> 1) & 1) ^ 1u);
+        if (!ok) break;
+#pragma unroll
+        for (int g = 0; g < kGroups; ++g)
+          if ((2 * g + gh) * 8 < u.n_mma) {
+            uint32_t h[8];                                       // codes (0, 2), (1, 3) of every word, as the weights' nibbles
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t x = cw[g][q] ^ 0x80808080u;
+              h[2 * q] = h2_bits(__hadd2(bits_h2(and_or(x, 0x00FF00FFu, 0x64006400u)), m1152));
+              h[2 * q + 1] = h2_bits(__hadd2(bits_h2(__byte_perm(x, 0x64646464u, 0x4341)), m1152));
+            }
+            unsigned char* t = tiles + (w * 4 + pc) * kBTile;
+            *reinterpret_cast<uint4*>(t + tile_at((2 * g + gh) * 8 + r8, 0)) = make_uint4(h[0], h[1], h[2], h[3]);
+            *reinterpret_cast<uint4*>(t + tile_at((2 * g + gh) * 8 + r8, 1)) = make_uint4(h[4], h[5], h[6], h[7]);
+          }
+        if (i < u.n_mma) {
+          uint32_t lo[4], hi[4];                                 // bsum = 64 * hi + lo
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            lo[q] = h2_bits(__hadd2(bits_h2(and_or(sums[1 + q], 0x003F003Fu, 0x64006400u)), m1024));
+            const int s0 = static_cast<int16_t>(sums[1 + q] & 0xFFFFu) >> 6, s1 = static_cast<int16_t>(sums[1 + q] >> 16) >> 6;
+            hi[q] = h2_bits(__hadd2(bits_h2(static_cast<uint32_t>(s0 + 128) | (static_cast<uint32_t>(s1 + 128) << 16) | 0x64006400u), m1152));
+          }
+          unsigned char* t = tiles + 16 * kBTile;
+          *reinterpret_cast<uint4*>(t + tile_at(i, 0)) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          *reinterpret_cast<uint4*>(t + tile_at(i, 1)) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          xd_sm[(fill & 3) * kGemmTok + i] = __uint_as_float(sums[0]);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_one(&bar[kBarBFull + buf]);
+      }
+      if (!ok) break;
+    }
   }
 
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  tc_fence_before();
   __syncthreads();
-  if (tid == 0 && *fail && status != nullptr) atomicExch(status, 6);
-  if (warp == 0) {
+  if (tid == 0 && *fail && a.status != nullptr) atomicExch(a.status, 6);
+  if (warp == kWarpMma) {
     __syncwarp();
+    tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
   }
 }
 
+template <bool DUAL, bool RAW>
+int launch_gemm(GemmArgs a, cudaStream_t stream) {
+  a.status = status_word();
+  const int sms = device_sms();
+  if (a.status == nullptr || sms <= 0) return kErrLaunch;      // the kernel reports an expired wait through the word
+  a.tiles = (a.n_rows + kGemmRows - 1) / kGemmRows;
+  // Rows of at most two blocks keep their activation tiles for a unit's row tiles: four tiles per unit
+  // make the staging an eighth of the jobs' time and still leave about seven units per SM for 256 experts.
+  a.group = !DUAL && a.nb <= 2 ? std::min(4, a.tiles) : 1;
+  a.groups = (a.tiles + a.group - 1) / a.group;
+  if (a.sw0 != nullptr && a.s_rows > 0) {
+    const int passes = (a.s_rows + kGemmTok - 1) / kGemmTok;
+    a.s_step = ((a.s_rows + passes - 1) / passes + 15) & ~15;
+    a.s_items = a.groups * ((a.s_rows + a.s_step - 1) / a.s_step);
+  } else {
+    a.s_items = 0;
+  }
+  const long long n_items = static_cast<long long>(a.groups) * a.n_expert + a.s_items;
+  if (n_items > 0x7FFFFFFF - 1024) return kErrUnsupported;
+  a.n_items = static_cast<int>(n_items);
+  if (!opt_in_smem<grouped_gemm_kernel<DUAL, RAW>>(kGemmSmem)) return kErrLaunch;
+  return launch_pdl(grouped_gemm_kernel<DUAL, RAW>, dim3(std::min(a.n_items, sms)), Cfg<RAW>::kThreads, kGemmSmem, stream, a);
+}
+
+// Rows of fp16 values - or SwiGLU of two rows, rounded to fp16 as silu_mul_f16 does - -> operand rows
+// (api_util.cuh): the Q8_K quantiser of quantize_block_f16 with the codes, the split sums and the scale in
+// the form the GEMM copies. Two slabs in one launch, the first bounded by *d_rows on the device. One warp
+// per block.
+constexpr int kQuantWarps = 4;
+__global__ void __launch_bounds__(kQuantWarps * 32)
+quantize_operand_kernel(const uint16_t* __restrict__ x0, const uint16_t* __restrict__ u0,
+                        unsigned char* __restrict__ out0, long long n0, const int* __restrict__ d_rows,
+                        const uint16_t* __restrict__ x1, const uint16_t* __restrict__ u1,
+                        unsigned char* __restrict__ out1, long long n1, int nb) {
+  pdl_wait();
+  pdl_launch_dependents();
+  long long b = static_cast<long long>(blockIdx.x) * kQuantWarps + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  const uint16_t *x = x0, *u = u0;
+  unsigned char* out = out0;
+  if (b >= n0) {
+    b -= n0;
+    if (b >= n1) return;
+    x = x1;
+    u = u1;
+    out = out1;
+  } else if (d_rows != nullptr && b >= static_cast<long long>(*d_rows) * nb) {
+    return;
+  }
+  float v[8];
+  load_lane8(x + b * kQK, lane, v);
+  if (u != nullptr) {
+    float uv[8];
+    load_lane8(u + b * kQK, lane, uv);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = h2f(f2h(silu_mul(v[i], uv[i])));
+  }
+  int q[8], sum;
+  const float d = quantize_lane8(v, q, sum);
+  out += b * kOpBlk;
+  uint32_t h[4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    h[2 * i] = h2_bits(__floats2half2_rn(static_cast<float>(q[4 * i]), static_cast<float>(q[4 * i + 2])));
+    h[2 * i + 1] = h2_bits(__floats2half2_rn(static_cast<float>(q[4 * i + 1]), static_cast<float>(q[4 * i + 3])));
+  }
+  reinterpret_cast<uint4*>(out)[lane] = make_uint4(h[0], h[1], h[2], h[3]);
+  if ((lane & 3) == 0) {                                        // four lanes hold one sub-block: bsum = 64 * hi + lo
+    uint16_t* s = reinterpret_cast<uint16_t*>(out + 512) + (lane >> 2);
+    s[0] = f2h(static_cast<float>(sum & 63));
+    s[8] = f2h(static_cast<float>(sum >> 6));
+  }
+  if (lane == 0) *reinterpret_cast<float*>(out + 544) = d;
+}
+
+GemmArgs args_of(const ExpertGemm& g) {
+  GemmArgs a{};
+  a.tab0 = g.tab; a.off = g.off; a.rows = g.rows; a.xq = g.xq; a.y = g.y;
+  a.n_rows = g.n_rows; a.nb = g.k / kQK; a.n_expert = g.n_expert;
+  a.sw0 = a.sw1 = static_cast<const unsigned char*>(g.shared_w);
+  a.sxq = g.shared_xq; a.sy = g.shared_y; a.s_rows = g.shared_rows;
+  return a;
+}
+
 }  // namespace
+
+int gemm_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, uint16_t* y_up, const void* shared_up,
+                 uint16_t* shared_y_up, cudaStream_t stream) {
+  GemmArgs a = args_of(g);
+  a.tab1 = tab_up; a.y1 = y_up;
+  a.sw1 = static_cast<const unsigned char*>(shared_up); a.sy1 = shared_y_up;
+  return g.operand_rows ? launch_gemm<true, false>(a, stream) : launch_gemm<true, true>(a, stream);
+}
+int gemm_grouped(const ExpertGemm& g, cudaStream_t stream) {
+  return g.operand_rows ? launch_gemm<false, false>(args_of(g), stream) : launch_gemm<false, true>(args_of(g), stream);
+}
+int quantize_operand(const uint16_t* x0, const uint16_t* u0, void* out0, long long rows0, const int* d_rows,
+                     const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, cudaStream_t stream) {
+  const int nb = k / kQK;
+  const long long blocks = (rows0 + rows1) * nb;
+  if (blocks <= 0) return kOk;
+  return launch_pdl(quantize_operand_kernel, dim3(static_cast<unsigned>((blocks + kQuantWarps - 1) / kQuantWarps)),
+                    kQuantWarps * 32, 0, stream, x0, u0, static_cast<unsigned char*>(out0), rows0 * nb, d_rows, x1, u1,
+                    static_cast<unsigned char*>(out1), rows1 * nb, nb);
+}
+
 }  // namespace sgr
 
 using namespace sgr;
-
-// y[t][r] = W[r][:] . xq[t][:] for one matrix and n_tok token rows on the same tensor-core kernel
-// (the shared expert of a prefill chunk: one "expert" that every row visits).
-int sgr::gemm_i8_dense(const void* w, const void* xq, uint16_t* y, int n_tok, int n_rows, int k, cudaStream_t stream) {
-  if (n_tok <= 0 || n_rows <= 0) return kOk;
-  if (!w || !xq || !y || k <= 0 || k % kQK != 0) return kErrArg;
-  if (reinterpret_cast<uintptr_t>(xq) & 15u) return kErrAlign;
-  auto kern = grouped_gemm_i8_kernel;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem) != cudaSuccess)
-    return kErrLaunch;
-  int* status = status_word();
-  if (status == nullptr) return kErrLaunch;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return kErrLaunch;
-  const int tiles = (n_rows + kGemmRows - 1) / kGemmRows;
-  const long long n_items = static_cast<long long>(tiles) * ((n_tok + 2 * kGemmTok - 1) / (2 * kGemmTok));
-  if (n_items > 0x7FFFFFFF) return kErrUnsupported;
-  kern<<<static_cast<unsigned>(n_items < sms ? n_items : sms), kGemmThreads, kGemmSmem, stream>>>(
-      nullptr, nullptr, static_cast<const unsigned char*>(xq), y, n_rows, k / kQK, tiles, static_cast<int>(n_items),
-      static_cast<const unsigned char*>(w), n_tok, status);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
-}
 
 // y[off[e] + t][r] = W_e[r][:] . xq[off[e] + t][:] for every expert e and its rows
 // t < off[e+1] - off[e]; fp16 out, row length n_rows. w_tab[e] == null: zero rows.
@@ -611,23 +841,15 @@ SGR_API int sgr_moe_grouped_gemm_i8(const void* const* w_tab, const int* off, co
                                     uint16_t* y, int n_rows, int k, int n_expert, void* stream) {
   if (n_expert <= 0 || n_rows <= 0) return kOk;
   if (!w_tab || !off || !xq || !y || k <= 0 || k % kQK != 0) return kErrArg;
-  if (reinterpret_cast<uintptr_t>(xq) & 15u) return kErrAlign;   // rows are read in aligned 16-byte pieces
+  if (reinterpret_cast<uintptr_t>(xq) & 15u) return kErrAlign;
   if (n_expert > 65535) return kErrUnsupported;
-  auto kern = grouped_gemm_i8_kernel;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem) != cudaSuccess)
-    return kErrLaunch;
-  int* status = status_word();
-  if (status == nullptr) return kErrLaunch;       // the kernel reports an expired wait through it
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return kErrLaunch;
-  const int tiles = (n_rows + kGemmRows - 1) / kGemmRows;
-  const long long n_items = static_cast<long long>(tiles) * n_expert;
-  if (n_items > 0x7FFFFFFF) return kErrUnsupported;
-  kern<<<static_cast<unsigned>(n_items < sms ? n_items : sms), kGemmThreads, kGemmSmem, as_stream(stream)>>>(
-      reinterpret_cast<const unsigned char* const*>(w_tab), off, static_cast<const unsigned char*>(xq), y,
-      n_rows, k / kQK, tiles, static_cast<int>(n_items), nullptr, 0, status);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
+  ExpertGemm g{};
+  g.tab = reinterpret_cast<const unsigned char* const*>(w_tab);
+  g.off = off;
+  g.xq = static_cast<const unsigned char*>(xq);
+  g.y = y;
+  g.n_rows = n_rows;
+  g.k = k;
+  g.n_expert = n_expert;
+  return gemm_grouped(g, as_stream(stream));
 }
-

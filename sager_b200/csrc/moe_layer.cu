@@ -1240,23 +1240,12 @@ bool matrix_tmap(int row_bytes, int rows, const void* placeholder, uint32_t* out
 // Polls (64 ns apart) after which a kernel that waits for a peer's arrival words gives up.
 std::atomic<unsigned> g_wait_limit{1u << 22};
 
-template <typename Kern>
-int launch_pdl(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream,
-               const LayerDev& L) {
+template <auto K>
+int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const LayerDev& L) {
   if (smem > 32 * 1024 &&     // (static shared memory counts towards the 48 KB default limit)
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
+      !opt_in_smem<K>(static_cast<int>(smem)))
     return kErrLaunch;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, L) == cudaSuccess ? kOk : kErrLaunch;
+  return launch_pdl(K, grid, threads, smem, stream, L);
 }
 
 }  // namespace
@@ -1449,10 +1438,8 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
                    !matrix_tmap(L.nbf * kW4, L.H, a->workspace, L.tmap_dn)))
     return kErrUnsupported;
   {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      return kErrLaunch;
+    const int sms = device_sms();
+    if (sms <= 0) return kErrLaunch;
     L.grid = std::min(sms, kMaxGrid);
   }
   cudaStream_t s = as_stream(stream);
@@ -1466,7 +1453,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       a->workspace_bytes >= lay.items_total) {
     const tk::Geom g = tk::geom(tk::kMaxTok, L.H, L.FF, L.E, L.grid);
     if (g.total <= 227 * 1024 && g.rows_per_cta <= tk::kWarps)
-      return launch_pdl(tk::token_layer_kernel, dim3(L.grid), tk::kThreads, g.total, s, L);
+      return launch_layer<tk::token_layer_kernel>(dim3(L.grid), tk::kThreads, g.total, s, L);
   }
 
   int rc = kOk;
@@ -1477,21 +1464,21 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
         std::max<size_t>(static_cast<size_t>(kRouteTok + kRouteRows) * L.H * 4, static_cast<size_t>(kRouteTok) * L.E * 4),
         plan_smem(L.E, L.n_max, L.K));
     if (smem > 200 * 1024) return kErrUnsupported;
-    rc = launch_pdl(route_kernel, dim3((L.E + kRouteRows - 1) / kRouteRows, (L.n + kRouteTok - 1) / kRouteTok),
+    rc = launch_layer<route_kernel>(dim3((L.E + kRouteRows - 1) / kRouteRows, (L.n + kRouteTok - 1) / kRouteTok),
                     kRouteWarps * 32, smem, s, L);
   } else {
     if (!a->xq_in) return kErrArg;
-    rc = launch_pdl(plan_kernel, dim3(1), 256, plan_smem(L.E, L.n_max, L.K), s, L);
+    rc = launch_layer<plan_kernel>(dim3(1), 256, plan_smem(L.E, L.n_max, L.K), s, L);
   }
   if (rc != kOk) return rc;
 
   if ((stages & 6) && use_rows) {
     const int sms = L.grid;
     if (!(stages & 1) && !(stages & 128)) {
-      rc = launch_pdl(rearm_kernel, dim3(1), 256, 0, s, L);
+      rc = launch_layer<rearm_kernel>(dim3(1), 256, 0, s, L);
       if (rc != kOk) return rc;
     }
-    rc = launch_pdl(rs::expert_rows_kernel, dim3(sms), rs::kThreads, rs::kSmem, s, L);
+    rc = launch_layer<rs::expert_rows_kernel>(dim3(sms), rs::kThreads, rs::kSmem, s, L);
   } else if (stages & 6) {
     // geometry the consumer mapping was written for: a tile of rows is one 16-row
     // group, or at most eight (group, super-block) units
@@ -1500,15 +1487,12 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
     if (!units_ok(g.rows_gu, L.nbh) || !units_ok(g.rows_dn, L.nbf)) return kErrUnsupported;
     const size_t smem = stream_smem(L.H, L.FF);
     if (smem > 227 * 1024) return kErrUnsupported;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-      return kErrLaunch;
+    const int sms = device_sms();
     if (!(stages & 1)) {
-      rc = launch_pdl(rearm_kernel, dim3(1), 256, 0, s, L);
+      rc = launch_layer<rearm_kernel>(dim3(1), 256, 0, s, L);
       if (rc != kOk) return rc;
     }
-    rc = launch_pdl(expert_stream_kernel, dim3(sms), kStreamThreads, smem, s, L);
+    rc = launch_layer<expert_stream_kernel>(dim3(sms), kStreamThreads, smem, s, L);
   }
   return rc;
 }

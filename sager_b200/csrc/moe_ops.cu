@@ -202,8 +202,6 @@ __global__ void scatter_rows_generic_kernel(uint16_t* __restrict__ dst, const fl
 }
 
 // ---- SwiGLU and gates (norm_rotary.cu:133-183) ------------------------------------
-__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.f + expf(-g)) * u; }
-
 __global__ void silu_mul_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ g,
                                 const uint16_t* __restrict__ u, long long total,
                                 const int* __restrict__ d_rows, int n_ff) {

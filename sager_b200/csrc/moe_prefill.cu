@@ -6,14 +6,16 @@
 // silu_mul_f16_n -> quantize_q8_k_n -> down -> scatter_routed_f16 -> shared expert
 // (gemv2 mtok, silu_mul, quantize, gemv mtok, strided copy into slot K of the combine
 // slab) -> moe_combine_batched_f16, on the caller's scratch buffers
-// (src/core/session.cpp:207-257). The last three steps - scatter into the combine slab, the
-// shared rows' copy into its slot K, the combine over the slab - are one kernel here that reads
-// the grouped rows and the shared rows where they lie (same sums in the same order; the slab,
-// 75 MB written and read back for a 2048-row chunk, is not touched). The routed expert projections run on the int8
-// tensor-core grouped GEMM (grouped_gemm_i8.cu) where the reference dequantises to fp16
-// and calls a library GEMM per expert (src/core/session.cpp:2643-2760); every other
-// step is the launcher the reference calls. Stream-ordered, no host synchronisation,
-// nothing allocated: legal inside stream capture.
+// (src/core/session.cpp:207-257). What is joined here, with the same values in the same order:
+//   * gate, up and the shared expert's gate, up are one tensor-core launch (grouped_gemm_i8.cu) that
+//     reads its activation rows through the plan (no gather), down and the shared down another -
+//     where the reference dequantises to fp16 and calls a library GEMM per expert
+//     (src/core/session.cpp:2643-2760);
+//   * SwiGLU and the requantisation of both row sets are one launch, which writes the rows as ready
+//     GEMM operands; so does the input quantiser. They lie in the combine slab, unused otherwise;
+//   * scatter, strided copy and combine are one kernel that reads the grouped and the shared rows
+//     where they lie.
+// Stream-ordered, no host synchronisation, nothing allocated: legal inside stream capture.
 #include <algorithm>
 
 #include "api_util.cuh"
@@ -82,7 +84,59 @@ __global__ void combine_grouped_kernel(uint16_t* __restrict__ x, const uint16_t*
     reinterpret_cast<uint4*>(o)[j] = make_uint4(ow[0], ow[1], ow[2], ow[3]);
   }
 }
+
+// The rows the GEMMs read: ready operands in the combine slab's memory when they fit there (FFN up to about
+// 0.8 x hidden at top-8), otherwise Q8_K rows from which the GEMMs make their operands themselves.
+struct OperandRows {
+  bool ready;
+  unsigned char *x, *h, *s;       // layer input, routed h, shared expert's h
+};
+OperandRows operand_rows(const sgr_moe_prefill* a) {
+  const long long nbh = a->hidden / kQK, nbf = a->n_ff / kQK, x = a->n * nbh * kOpBlk,
+                  h = static_cast<long long>(a->n) * a->n_used * nbf * kOpBlk, s = a->n * nbf * kOpBlk;
+  unsigned char* slab = reinterpret_cast<unsigned char*>(a->expert_y);
+  if ((reinterpret_cast<uintptr_t>(slab) & 15u) == 0 &&
+      x + h + s <= static_cast<long long>(a->n_max) * (a->n_used + 1) * a->hidden * 2)
+    return {true, slab, slab + x, slab + x + h};
+  return {false, static_cast<unsigned char*>(a->xq), static_cast<unsigned char*>(a->hq), static_cast<unsigned char*>(a->sh_q)};
+}
+
+inline bool has_shared(const sgr_moe_prefill* a) { return a->shared_gate && a->shared_up && a->shared_down; }
+
+// gate / up, SwiGLU, requantise, down of the routed experts and of the shared one
+int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t stream) {
+  const int n = a->n, H = a->hidden, F = a->n_ff, E = a->n_expert, K = a->n_used;
+  const bool shared = has_shared(a);
+  const long long ts = a->tab_stride > 0 ? a->tab_stride : E, R = static_cast<long long>(a->n_max) * K;
+  auto tab = [&](int m) { return reinterpret_cast<const unsigned char* const*>(a->w_tab + m * ts); };
+  ExpertGemm up{};
+  up.tab = tab(0); up.off = a->off; up.rows = a->grows; up.xq = op.x; up.operand_rows = op.ready;
+  up.y = a->g; up.n_rows = F; up.k = H; up.n_expert = E;
+  ExpertGemm down{};
+  down.tab = tab(2); down.off = a->off; down.xq = op.h; down.operand_rows = op.ready;
+  down.y = a->y_grouped; down.n_rows = H; down.k = F; down.n_expert = E;
+  if (shared) {
+    up.shared_w = a->shared_gate; up.shared_xq = op.x; up.shared_y = a->sh_g; up.shared_rows = n;
+    down.shared_w = a->shared_down; down.shared_xq = op.s; down.shared_y = a->sh_y; down.shared_rows = n;
+  }
+  int rc = gemm_gate_up(up, tab(1), a->u, a->shared_up, a->sh_u, stream);
+  if (rc != kOk) return rc;
+  if (op.ready) {
+    rc = quantize_operand(a->g, a->u, op.h, static_cast<long long>(n) * K, a->meta, a->sh_g, a->sh_u, op.s, shared ? n : 0, F, stream);
+  } else {
+    rc = sgr_silu_mul_f16_n(a->g, a->g, a->u, a->meta, static_cast<int>(R), F, stream);
+    if (rc == kOk) rc = sgr_quantize_q8_k_n(a->g, a->hq, a->meta, F, static_cast<int>(R * (F / kQK)), stream);
+    if (rc == kOk && shared) rc = sgr_silu_mul_f16(a->sh_g, a->sh_g, a->sh_u, n, F, stream);
+    if (rc == kOk && shared) rc = sgr_quantize_q8_k(a->sh_g, a->sh_q, static_cast<long long>(n) * F, stream);
+  }
+  return rc == kOk ? gemm_grouped(down, stream) : rc;
+}
 }  // namespace
+
+// Diagnostics (sager_b200_diag.h): the expert stage of a finished call once more, for timing.
+SGR_API int sgr_moe_prefill_expert_stage(const sgr_moe_prefill* a, void* stream) {
+  return a == nullptr ? kErrArg : expert_stage(a, operand_rows(a), as_stream(stream));
+}
 
 SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
   if (a == nullptr) return kErrArg;
@@ -94,19 +148,18 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
       !a->y_grouped || !a->expert_y)
     return kErrArg;
   if (!a->logits_in && (!a->router_w || !a->logits)) return kErrArg;
-  const bool shared = a->shared_gate && a->shared_up && a->shared_down;
+  const bool shared = has_shared(a);
   if (shared && (!a->sh_g || !a->sh_u || !a->sh_q || !a->sh_y)) return kErrArg;
   const long long ts = a->tab_stride > 0 ? a->tab_stride : E;
   if (ts < E) return kErrArg;
   const int tok_per = a->tok_per > 0 ? a->tok_per : 16;
-  const void* const* tab_g = a->w_tab;
-  const void* const* tab_u = a->w_tab + ts;
-  const void* const* tab_d = a->w_tab + 2 * ts;
   const long long R = static_cast<long long>(a->n_max) * K;
   if (R > 0x7FFFFFFF / (F / kQK)) return kErrUnsupported;
   int rc;
 #define SGR_STEP(call) do { rc = (call); if (rc != kOk) return rc; } while (0)
-  SGR_STEP(sgr_quantize_q8_k(a->xn, a->xq, static_cast<long long>(n) * H, stream));
+  const OperandRows op = operand_rows(a);
+  if (op.ready) SGR_STEP(quantize_operand(a->xn, nullptr, op.x, n, nullptr, nullptr, nullptr, nullptr, 0, H, as_stream(stream)));
+  else SGR_STEP(sgr_quantize_q8_k(a->xn, a->xq, static_cast<long long>(n) * H, stream));
   const float* logits = a->logits_in;
   if (logits == nullptr) {
     SGR_STEP(sgr_gemv_f32_out_f16x_mtok(a->router_w, a->xn, a->logits, E, H, n, stream));
@@ -116,35 +169,13 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
                                    shared ? a->shared_w : 0.f, stream));
   SGR_STEP(sgr_moe_dispatch_scan(a->route_idx, a->route_w, a->gslot, a->grows, a->off, a->toff, a->meta,
                                  a->mail, a->mail_n, n, K, E, tok_per, stream));
-  SGR_STEP(sgr_gather_rows_q8_n(a->xqg, a->xq, a->grows, a->meta, static_cast<int>(R), H / kQK, stream));
-  SGR_STEP(sgr_moe_grouped_gemm_i8(tab_g, a->off, a->xqg, a->g, F, H, E, stream));
-  SGR_STEP(sgr_moe_grouped_gemm_i8(tab_u, a->off, a->xqg, a->u, F, H, E, stream));
-  SGR_STEP(sgr_silu_mul_f16_n(a->g, a->g, a->u, a->meta, static_cast<int>(R), F, stream));
-  SGR_STEP(sgr_quantize_q8_k_n(a->g, a->hq, a->meta, F, static_cast<int>(R * (F / kQK)), stream));
-  SGR_STEP(sgr_moe_grouped_gemm_i8(tab_d, a->off, a->hq, a->y_grouped, H, F, E, stream));
+  SGR_STEP(expert_stage(a, op, as_stream(stream)));
   // the combine reads the grouped rows in place when every buffer allows 16-byte accesses
   const bool direct = (H & 7) == 0 && K <= 1024 &&
                       ((reinterpret_cast<uintptr_t>(a->x_f16) | reinterpret_cast<uintptr_t>(a->y_grouped) |
                         (shared ? reinterpret_cast<uintptr_t>(a->sh_y) : 0)) & 15u) == 0;
   if (!direct) SGR_STEP(sgr_scatter_routed_f16(a->expert_y, a->y_grouped, a->gslot, n, K, H, stream));
   if (shared) {
-    // the shared expert is one expert that every row visits: the same tensor-core kernel as the routed
-    // ones when its row buffers allow 16-byte reads (the multi-token GEMV of the reference's sequence,
-    // gemv2_q4_k_q8_f16out_mtok, took 0.42 ms for gate and up of a 2048-row chunk)
-    const bool tc = ((reinterpret_cast<uintptr_t>(a->xq) | reinterpret_cast<uintptr_t>(a->sh_q)) & 15u) == 0;
-    if (tc) {
-      SGR_STEP(gemm_i8_dense(a->shared_gate, a->xq, a->sh_g, n, F, H, as_stream(stream)));
-      SGR_STEP(gemm_i8_dense(a->shared_up, a->xq, a->sh_u, n, F, H, as_stream(stream)));
-    } else {
-      SGR_STEP(sgr_gemv2_q4_k_q8_f16out_mtok(a->shared_gate, a->shared_up, a->xq, a->sh_g, a->sh_u, F, H, n, stream));
-    }
-    SGR_STEP(sgr_silu_mul_f16(a->sh_g, a->sh_g, a->sh_u, n, F, stream));
-    SGR_STEP(sgr_quantize_q8_k(a->sh_g, a->sh_q, static_cast<long long>(n) * F, stream));
-    if (tc) {
-      SGR_STEP(gemm_i8_dense(a->shared_down, a->sh_q, a->sh_y, n, H, F, as_stream(stream)));
-    } else {
-      SGR_STEP(sgr_gemv_q4_k_q8_f16out_mtok(a->shared_down, a->sh_q, a->sh_y, H, F, n, stream));
-    }
     if (a->shared_gate_w != nullptr) {           // scalar gate sigmoid(w_sg . x) on the shared rows (layer.cpp:128-134)
       if (a->sgate == nullptr) return kErrArg;
       SGR_STEP(sgr_gemv_f32_out_f16x_batched(a->shared_gate_w, a->xn, a->sgate, 1, H, n, stream));

@@ -39,6 +39,9 @@ __device__ __forceinline__ uint16_t f2h(float f) {
   return __half_as_ushort(__float2half(f));   // round to nearest even
 }
 
+// SwiGLU of one (gate, up) pair (norm_rotary.cu:133-141 of the reference)
+__device__ __forceinline__ float silu_mul(float g, float u) { return g / (1.f + expf(-g)) * u; }
+
 // ---- mbarrier + bulk copy (TMA without a tensor map, one CTA per copy) --------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -19,6 +19,16 @@ int* status_word() {
   }
   return g_status_addr[dev];
 }
+
+int device_sms() {
+  static std::atomic<int> sms[kMaxDevices];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  if ((n = sms[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 0;
+  sms[dev].store(n, std::memory_order_relaxed);
+  return n;
+}
 }  // namespace sgr
 
 // Reads (and clears when `clear` != 0) the status word of the current device.

@@ -167,15 +167,13 @@ class MoeStack:
 class PrefillLayer:
     """One MoE layer over a chunk of many token rows, as the reference's
     `Session::moe_dispatch_device` drives it for prefill (src/core/session.cpp:2482-3030),
-    call for call through the library's launchers - with the expert math on the int8
-    tensor-core grouped GEMM instead of the reference's fp16 cuBLAS path. Buffers follow
+    behind one call - with the expert math on the tensor-core grouped GEMM of the Q4_K x Q8_K
+    integers instead of the reference's fp16 cuBLAS path. Buffers follow
     the session's scratch (src/core/session.cpp:207-257)."""
 
     TOK_PER = 16
 
     def __init__(self, n_max, hidden, n_ff, n_expert, n_used, device):
-        from . import ops
-        self.ops = ops
         self.n_max, self.H, self.F, self.E, self.K = n_max, hidden, n_ff, n_expert, n_used
         d, u8, f16, i32, f32 = device, torch.uint8, torch.float16, torch.int32, torch.float32
         R = n_max * n_used
@@ -226,14 +224,6 @@ class PrefillLayer:
         """x [n][H] fp16 residual, combined in place: one call of sgr_moe_layer_prefill.
         `logits` replaces the router GEMV (the prefill benchmark draws them directly).
         experts_only re-issues the routed expert stage alone (gate, up, SwiGLU, requantise,
-        down) on the plan a full call left behind (timing)."""
-        o, H, F, E, K = self.ops, self.H, self.F, self.E, self.K
-        if not experts_only:
-            a = self.args(n, xn, x, weights, table, logits=logits, shared=shared)
-            lib().call("sgr_moe_layer_prefill", C.byref(a), stream_ptr())
-            return
-        o.moe_grouped_gemm_i8(table[0], self.off, self.xqg, self.g, F, H, E)
-        o.moe_grouped_gemm_i8(table[1], self.off, self.xqg, self.u, F, H, E)
-        o.silu_mul_f16_n(self.g, self.g, self.u, self.meta, n * K, F)
-        o.quantize_q8_k_n(self.g, self.hq, self.meta, F, n * K * (F // 256))
-        o.moe_grouped_gemm_i8(table[2], self.off, self.hq, self.yg, H, F, E)
+        down) on the plan and the operand rows a full call left behind (timing)."""
+        a = self.args(n, xn, x, weights, table, logits=logits, shared=shared and not experts_only)
+        lib().call("sgr_moe_prefill_expert_stage" if experts_only else "sgr_moe_layer_prefill", C.byref(a), stream_ptr())

@@ -68,6 +68,82 @@ def test_expert_shapes_match_device_plan_gemv(oracle, n_rows, k):
         f16_close(y.cpu().numpy(), y2.float().cpu().numpy())
 
 
+@pytest.mark.parametrize("n_rows,k,counts", [(128, 256, [16, 17, 80, 81, 160, 161]),   # edges of the token tiles
+                                             (640, 512, [1, 79, 96]),                   # two units of row tiles, the last short
+                                             (130, 768, [33, 2])])                      # three blocks: tiles staged per row tile
+def test_tile_edges(oracle, n_rows, k, counts):
+    run_case(oracle, n_rows, k, counts, seed=7, check_rows=12)
+    from sager_b200 import lib
+    assert lib().raw("sgr_status")(0) == 0
+
+
+@pytest.mark.parametrize("n_rows,k", [(128, 512), (512, 256)])
+def test_many_ragged_units_in_one_cta(oracle, n_rows, k):
+    """450 experts of 0 to 90 rows: a CTA walks several units of different sizes, nothing of one may be left for the next."""
+    rng = np.random.default_rng(8)
+    counts = rng.integers(0, 91, 450)
+    w_np, w_dev = make_q4k(n_rows, k, 78)
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    R = int(off[-1])
+    x_np, x_dev = make_x16(R, k, 6)
+    xq = quantize_dev(x_dev)
+    y = torch.zeros(R, n_rows, dtype=torch.float16, device=DEV)
+    ops.moe_grouped_gemm_i8(ops.ptr_table([w_dev] * 450, DEV), dev(off), xq, y, n_rows, k, 450)
+    y1 = torch.zeros_like(y)                       # the same rows through the batched GEMV family
+    ops.mmq_q4_k_q8_f16out(w_dev, xq, y1, n_rows, k, R)
+    assert f16_close(y.cpu().numpy(), y1.float().cpu().numpy())
+
+
+def test_weights_off_a_16_byte_boundary(oracle):
+    """Pointer tables only promise the block struct's 2-byte alignment."""
+    n_rows, k, counts = 256, 512, [5, 20]
+    E, off = 2, np.int32([0, 5, 25])
+    mats = [make_q4k(n_rows, k, 60 + e) for e in range(E)]
+    big = torch.empty(E, mats[0][1].numel() + 16, dtype=torch.uint8, device=DEV)
+    for e in range(E):
+        big[e, 2 + 2 * e:2 + 2 * e + mats[e][1].numel()] = mats[e][1].reshape(-1)
+    tab = torch.tensor([big[e].data_ptr() + 2 + 2 * e for e in range(E)], dtype=torch.int64, device=DEV)
+    xq = quantize_dev(make_x16(25, k, 3)[1])
+    y = torch.zeros(25, n_rows, dtype=torch.float16, device=DEV)
+    ops.moe_grouped_gemm_i8(tab, dev(off), xq, y, n_rows, k, E)
+    for r in range(25):
+        assert f16_close(y[r].cpu().numpy(), oracle.gemv(mats[0 if r < 5 else 1][0], xq.cpu().numpy()[r], n_rows, k)), r
+
+
+@pytest.mark.parametrize("H,F,E,K,n", [(512, 256, 16, 4, 70), (1024, 512, 8, 2, 333), (256, 512, 8, 4, 90)])
+def test_prefill_chunk_against_the_launchers_it_joins(oracle, H, F, E, K, n):
+    """The chunk's gate/up/down launches (operand rows, rows read through the plan, shared expert riding along) give the
+    values of the launchers they stand for - grouped GEMM on gathered rows, SwiGLU, quantiser. The sums of a GEMM are the
+    same integers and fp32 steps on both paths: equal to the bit. (256, 512): no room for operand rows in the slab."""
+    from sager_b200 import synth
+    from sager_b200.layer import PrefillLayer
+    w = synth.MoeWeights(H, F, E, DEV, seed=71, std=0.05)
+    x16 = synth.normal_fp16((n, H), 72, DEV)
+    L = PrefillLayer(n, H, F, E, K, DEV)
+    x = x16.clone()
+    t = w.table()
+    L.run(n, x16, x, w, t)
+    xq = quantize_dev(x16)
+    R = n * K
+    xqg = torch.zeros(R, H // 256 * 276, dtype=torch.uint8, device=DEV)
+    ops.gather_rows_q8(xqg, xq, L.grows, R, H // 256)
+    g, u, y = (torch.zeros(R, d, dtype=torch.float16, device=DEV) for d in (F, F, H))
+    ops.moe_grouped_gemm_i8(t[0].contiguous(), L.off, xqg, g, F, H, E)
+    ops.moe_grouped_gemm_i8(t[1].contiguous(), L.off, xqg, u, F, H, E)
+    ops.silu_mul_f16(g, g, u, R, F)
+    hq = quantize_dev(g)
+    ops.moe_grouped_gemm_i8(t[2].contiguous(), L.off, hq, y, H, F, E)
+    assert torch.equal(L.yg.view(torch.int16), y.view(torch.int16))
+    one = ops.ptr_table([w.matrix(E, 0)], DEV), ops.ptr_table([w.matrix(E, 1)], DEV), ops.ptr_table([w.matrix(E, 2)], DEV)
+    off = dev(np.int32([0, n]))
+    sg, su, sy = (torch.zeros(n, d, dtype=torch.float16, device=DEV) for d in (F, F, H))
+    ops.moe_grouped_gemm_i8(one[0], off, xq, sg, F, H, 1)
+    ops.moe_grouped_gemm_i8(one[1], off, xq, su, F, H, 1)
+    ops.silu_mul_f16(sg, sg, su, n, F)
+    ops.moe_grouped_gemm_i8(one[2], off, quantize_dev(sg), sy, H, F, 1)
+    assert torch.equal(L.sh_y.view(torch.int16), sy.view(torch.int16))
+
+
 def test_prefill_sized_plan(oracle):
     """2048 token rows, top-8 of 256 experts with uniform logits: 16384 routed rows, about 64
     per expert - the prefill configuration. Spot-checked against the oracle."""
