@@ -15,43 +15,58 @@ __device__ __forceinline__ bool aligned16(const void* p) {
 }
 
 // ---- dispatch plan (moe.cu:366-434) ---------------------------------------------
-// One CTA. hist -> exclusive prefixes off/toff -> grouped slots. Up to
-// kStableMax routes the slots inside an expert are filled in ascending
-// (row, kk) order (each expert's thread walks the id list in shared memory),
-// which makes the plan reproducible; larger plans use atomics like the
-// reference, whose consumers are all position-keyed.
+// One CTA. Every warp owns a contiguous piece of the route list and counts it per expert in a
+// shared-memory row of its own (lanes with the same expert meet by match_any); per expert a prefix
+// over the warps and one over the experts give each warp its first slots, and a second walk hands
+// the slots out. So the slots inside an expert are in ascending (row, kk) order whatever the size
+// and nothing is contended; what bounds it is the latency of the phases. Before: 16,384 routes over
+// 256 experts 24 us with atomics, 768 routes filled by one thread per expert 35 us.
 constexpr int kScanThreads = 1024;
-constexpr int kStableMax = 4096;
+constexpr int kScanCounters = 10240;       // [warps that share the list][n_expert] counters of 4 bytes
 
 __global__ void __launch_bounds__(kScanThreads)
 dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, int* __restrict__ gslot,
                      int* __restrict__ grows, int* __restrict__ off, int* __restrict__ toff,
                      int* __restrict__ meta, int* __restrict__ mail_n, int n_rows, int k,
-                     int n_expert, int tok_per) {
-  extern __shared__ int sm_i[];
-  int* hist = sm_i;                    // [n_expert]
-  int* fill = sm_i + n_expert;         // [n_expert]
-  int* ids = sm_i + 2 * n_expert;      // [total] when the stable path is taken
+                     int n_expert, int tok_per, int n_warps) {
+  extern __shared__ int cnt[];             // [n_warps][n_expert]: counts, then next slots
   __shared__ int bad_sh;
-  const int tid = threadIdx.x;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const int total = n_rows * k;
-  const bool stable = total <= kStableMax;
+  const int per = ((total + n_warps - 1) / n_warps + 31) & ~31;       // routes per warp
+  const int i0 = min(wp * per, total), i1 = wp < n_warps ? min(i0 + per, total) : i0;
   if (tid == 0) bad_sh = 0;
-  for (int e = tid; e < n_expert; e += kScanThreads) hist[e] = 0;
+  for (int e = tid; e < n_warps * n_expert; e += kScanThreads) cnt[e] = 0;
   __syncthreads();
-
-  for (int i = tid; i < total; i += kScanThreads) {
-    const int r = i / k, kk = i - r * k;
-    const int e = idx[static_cast<size_t>(r) * (k + 1) + kk];
-    const bool valid = e >= 0 && e < n_expert;
-    if (stable) ids[i] = valid ? e : -1;
-    if (!valid) {
-      // a corrupt id silences the whole row, shared-expert slot included
-      float* wr = weight + static_cast<size_t>(r) * (k + 1);
-      for (int q = 0; q <= k; ++q) wr[q] = 0.f;
-      atomicAdd(&bad_sh, 1);
-    } else {
-      atomicAdd(&hist[e], 1);
+  int* mine = cnt + static_cast<size_t>(min(wp, n_warps - 1)) * n_expert;
+  auto id_of = [&](int i) {
+    const int r = i / k;
+    const int e = __ldg(idx + static_cast<size_t>(r) * (k + 1) + (i - r * k));
+    return e >= 0 && e < n_expert ? e : -1;
+  };
+  // four groups of 32 routes requested together
+  for (int b = i0; b < i1; b += 128) {
+    int e4[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = b + 32 * q + lane;
+      e4[q] = i < i1 ? id_of(i) : -2;                                 // -2: past the end
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned same = __match_any_sync(0xFFFFFFFFu, e4[q]);
+      if (e4[q] >= 0 && lane == __ffs(same) - 1) mine[e4[q]] += __popc(same);
+      if (e4[q] == -1) {
+        // a corrupt id silences the whole row, shared-expert slot included
+        const int i = b + 32 * q + lane;
+        float* wr = weight + static_cast<size_t>(i / k) * (k + 1);
+        for (int j = 0; j <= k; ++j) wr[j] = 0.f;
+        gslot[i] = -1;
+        atomicAdd(&bad_sh, 1);
+      }
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -61,12 +76,18 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
   {
     __shared__ int wsum[2][kScanThreads / 32];
     __shared__ int carry[2];
-    const int lane = tid & 31, wp = tid >> 5;
     if (tid == 0) carry[0] = carry[1] = 0;
     __syncthreads();
     for (int base = 0; base < n_expert; base += kScanThreads) {
       const int e = base + tid;
-      const int c = e < n_expert ? hist[e] : 0;
+      int c = 0;
+      if (e < n_expert) {
+        for (int w = 0; w < n_warps; ++w) {                           // the expert's routes, warp after warp
+          const int v = cnt[static_cast<size_t>(w) * n_expert + e];
+          cnt[static_cast<size_t>(w) * n_expert + e] = c;
+          c += v;
+        }
+      }
       const int t = (c + tok_per - 1) / tok_per;
       int ic = c, it = t;
 #pragma unroll
@@ -79,9 +100,10 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
       int pc = carry[0], pt = carry[1];
       for (int w = 0; w < wp; ++w) { pc += wsum[0][w]; pt += wsum[1][w]; }
       if (e < n_expert) {
-        off[e] = pc + ic - c;
+        const int o0 = pc + ic - c;
+        off[e] = o0;
         toff[e] = pt + it - t;
-        fill[e] = pc + ic - c;
+        for (int w = 0; w < n_warps; ++w) cnt[static_cast<size_t>(w) * n_expert + e] += o0;
       }
       __syncthreads();
       if (tid == kScanThreads - 1) { carry[0] = pc + ic; carry[1] = pt + it; }
@@ -96,30 +118,30 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
       if (mail_n != nullptr) *mail_n = 0;
     }
   }
-  __syncthreads();
 
-  if (stable) {
-    for (int i = tid; i < total; i += kScanThreads)
-      if (ids[i] < 0) gslot[i] = -1;
-    for (int e = tid; e < n_expert; e += kScanThreads) {
-      if (hist[e] == 0) continue;
-      int pos = fill[e];
-      for (int i = 0; i < total; ++i) {
-        if (ids[i] == e) {
-          gslot[i] = pos;
-          grows[pos] = i / k;
-          ++pos;
-        }
-      }
+  for (int b = i0; b < i1; b += 128) {
+    int e4[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = b + 32 * q + lane;
+      e4[q] = i < i1 ? id_of(i) : -1;
     }
-  } else {
-    for (int i = tid; i < total; i += kScanThreads) {
-      const int r = i / k, kk = i - r * k;
-      const int e = idx[static_cast<size_t>(r) * (k + 1) + kk];
-      if (e < 0 || e >= n_expert) { gslot[i] = -1; continue; }
-      const int pos = atomicAdd(&fill[e], 1);
-      gslot[i] = pos;
-      grows[pos] = r;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const unsigned same = __match_any_sync(0xFFFFFFFFu, e4[q]);
+      const int first = __ffs(same) - 1;
+      int slot = 0;
+      if (e4[q] >= 0 && lane == first) {
+        slot = mine[e4[q]];
+        mine[e4[q]] = slot + __popc(same);
+      }
+      slot = __shfl_sync(0xFFFFFFFFu, slot, first) + __popc(same & ((1u << lane) - 1u));
+      if (e4[q] >= 0) {
+        const int i = b + 32 * q + lane;
+        gslot[i] = slot;
+        grows[slot] = i / k;
+      }
+      __syncwarp();
     }
   }
 }
@@ -328,12 +350,12 @@ SGR_API int sgr_moe_dispatch_scan(const int* idx, float* weight, int* gslot, int
   if (!idx || !weight || !gslot || !grows || !off || !toff || !meta || n_rows < 0 || k <= 0 ||
       n_expert <= 0 || tok_per <= 0)
     return kErrArg;
-  const long long total = static_cast<long long>(n_rows) * k;
-  const size_t smem = (2 * static_cast<size_t>(n_expert) + (total <= kStableMax ? total : 0)) * sizeof(int);
-  if (smem > 48 * 1024) return kErrUnsupported;
-  dispatch_scan_kernel<<<1, kScanThreads, smem, as_stream(stream)>>>(
-      idx, weight, gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per);
-  return ok_or_launch();
+  if (static_cast<long long>(n_rows) * k > 0x7FFFFF00) return kErrArg;
+  // the counters of as many warps as fit the default 48 KB; the former limit on experts, 6144, is within it
+  if (n_expert > 12000) return kErrUnsupported;
+  const int n_warps = std::max(1, std::min(kScanThreads / 32, kScanCounters / n_expert));
+  return launch_pdl(dispatch_scan_kernel, dim3(1), kScanThreads, static_cast<size_t>(n_warps) * n_expert * sizeof(int),
+                    as_stream(stream), idx, weight, gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, n_warps);
 }
 
 SGR_API int sgr_gather_rows_q8(void* dst, const void* src, const int* src_rows, int n_rows,

@@ -34,6 +34,8 @@ __global__ void combine_grouped_kernel(uint16_t* __restrict__ x, const uint16_t*
                                        const float* __restrict__ weight, int K, int H) {
   extern __shared__ float wsm[];       // [K+1] weights of this row, then [K] grouped slots
   int* slot_sm = reinterpret_cast<int*>(wsm + K + 1);
+  pdl_wait();
+  pdl_launch_dependents();
   const int row = blockIdx.x;
   for (int kk = threadIdx.x; kk <= K; kk += blockDim.x) {
     wsm[kk] = weight[static_cast<size_t>(row) * (K + 1) + kk];
@@ -47,16 +49,16 @@ __global__ void combine_grouped_kernel(uint16_t* __restrict__ x, const uint16_t*
     float acc[8];
 #pragma unroll
     for (int q = 0; q < 4; ++q) { acc[2 * q] = h2f(rw[q] & 0xFFFF); acc[2 * q + 1] = h2f(rw[q] >> 16); }
-    for (int k0 = 0; k0 < K; k0 += 4) {             // four routes' rows requested together
-      uint4 yv[4];
+    for (int k0 = 0; k0 < K; k0 += 8) {             // eight routes' rows requested together
+      uint4 yv[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 8; ++u) {
         const int gs = k0 + u < K ? slot_sm[k0 + u] : -1;
         yv[u] = gs >= 0 ? __ldg(reinterpret_cast<const uint4*>(y_grouped + static_cast<size_t>(gs) * H) + j)
                         : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 8; ++u) {
         if (k0 + u < K && slot_sm[k0 + u] >= 0) {
           const float w = wsm[k0 + u];
           const uint32_t yw[4] = {yv[u].x, yv[u].y, yv[u].z, yv[u].w};
@@ -188,10 +190,8 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
       return kErrLaunch;
   }
   if (direct) {
-    const int chunks = std::max(1, std::min((H / 8 + 127) / 128, (4 * 148 + n - 1) / n));
-    combine_grouped_kernel<<<dim3(n, chunks), 128, (2 * K + 1) * sizeof(float), as_stream(stream)>>>(
-        a->x_f16, a->y_grouped, a->gslot, shared ? a->sh_y : nullptr, a->route_w, K, H);
-    if (cudaPeekAtLastError() != cudaSuccess) return kErrLaunch;
+    SGR_STEP(launch_pdl(combine_grouped_kernel, dim3(n, (H / 8 + 127) / 128), 128, (2 * K + 1) * sizeof(float), as_stream(stream),
+                        a->x_f16, a->y_grouped, a->gslot, shared ? a->sh_y : nullptr, a->route_w, K, H));
   } else {
     SGR_STEP(sgr_moe_combine_batched_f16(a->x_f16, a->expert_y, a->route_w, K, H, n, stream));
   }

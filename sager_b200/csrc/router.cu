@@ -73,7 +73,7 @@ __device__ __forceinline__ void fold_lanes(float* f, int lane) {
 // stages: the next one is on its way to registers while this one is used, so a stage has to last a
 // round trip to L2 (with 64 columns the trip showed: 124 us for 2048 tokens, 14 us for eight).
 template <int TR, int TT, int WR, int WT, int KC>
-__global__ void __launch_bounds__(WR* WT * 32)
+__global__ void __launch_bounds__(WR* WT * 32, 8 / (WR * WT))
 router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restrict__ x, float* __restrict__ y,
                            int n_rows, int k, int n_tokens) {
   constexpr int kWarps = WR * WT, kRows = TR * WR, kPairs = TT * WT / 2, kSteps = KC / 64;
@@ -85,6 +85,8 @@ router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restri
   float2(*ws)[kRows][kSteps][32] = reinterpret_cast<float2(*)[kRows][kSteps][32]>(smem);
   float4(*xs)[kPairs][kSteps][32] =
       reinterpret_cast<float4(*)[kPairs][kSteps][32]>(smem + 2 * sizeof(float) * kRows * KC);
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * kRows, tok0 = blockIdx.y * (TT * WT);
   const int wr = warp % WR, wt = warp / WR;
@@ -127,6 +129,8 @@ router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restri
       }
     }
   };
+  // (the conversions are pinned here: moved up to the loads they would wait for them)
+  auto cvt = [](uint16_t h) { float f; asm volatile("cvt.f32.f16 %0, %1;" : "=f"(f) : "h"(h)); return f; };
   auto put = [&](int buf) {
 #pragma unroll
     for (int j = 0; j < kSteps; ++j) {
@@ -135,8 +139,8 @@ router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restri
         ws[buf][warp + i * kWarps][j][lane] = make_float2(wreg[i][2 * j], wreg[i][2 * j + 1]);
 #pragma unroll
       for (int i = 0; i < kPairsPerWarp; ++i)
-        xs[buf][warp + i * kWarps][j][lane] = make_float4(h2f(xreg[i][2 * j][0]), h2f(xreg[i][2 * j][1]),
-                                                          h2f(xreg[i][2 * j + 1][0]), h2f(xreg[i][2 * j + 1][1]));
+        xs[buf][warp + i * kWarps][j][lane] = make_float4(cvt(xreg[i][2 * j][0]), cvt(xreg[i][2 * j][1]),
+                                                          cvt(xreg[i][2 * j + 1][0]), cvt(xreg[i][2 * j + 1][1]));
     }
   };
 
@@ -194,12 +198,9 @@ router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restri
 template <int TR, int TT, int WR, int WT, int KC>
 int launch_tiled(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens, cudaStream_t stream) {
   constexpr int kSmem = 2 * KC * (TR * WR + TT * WT) * static_cast<int>(sizeof(float));
-  auto kern = router_logits_tiled_kernel<TR, TT, WR, WT, KC>;
-  if (kSmem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess)
-    return kErrLaunch;
+  if (kSmem > 48 * 1024 && !opt_in_smem<router_logits_tiled_kernel<TR, TT, WR, WT, KC>>(kSmem)) return kErrLaunch;
   const dim3 grid((n_rows + TR * WR - 1) / (TR * WR), (n_tokens + TT * WT - 1) / (TT * WT));
-  kern<<<grid, WR * WT * 32, kSmem, stream>>>(w, x, y, n_rows, k, n_tokens);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
+  return launch_pdl(router_logits_tiled_kernel<TR, TT, WR, WT, KC>, grid, WR * WT * 32, kSmem, stream, w, x, y, n_rows, k, n_tokens);
 }
 
 int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens,
@@ -214,7 +215,7 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
   } else if (static_cast<long long>(n_rows) * n_tokens >= 256LL * 592) {
     // 8 x 16 outputs per warp keep the FMA pipes fullest; below one such CTA per SM the smaller tile has more
     // warps to spread (at 256 x 592 the two take 41 and 38 us, and from there the larger one wins)
-    return launch_tiled<8, 16, 4, 2, 128>(w, x, y, n_rows, k, n_tokens, stream);
+    return launch_tiled<8, 16, 2, 2, 128>(w, x, y, n_rows, k, n_tokens, stream);
   } else {
     return launch_tiled<4, 8, 4, 1, 256>(w, x, y, n_rows, k, n_tokens, stream);   // small: more warps to spread
   }
@@ -227,6 +228,8 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int* __rest
                                    float* __restrict__ weight, int n_expert, int k, int stride,
                                    int n_rows, float shared_w) {
   extern __shared__ __align__(16) unsigned char smem[];
+  pdl_wait();
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * kTopkWarps + warp;
   if (row >= n_rows) return;
@@ -295,10 +298,8 @@ SGR_API int sgr_router_topk_batched(const float* logits, int* idx, float* weight
     return kErrArg;
   const size_t smem = static_cast<size_t>(kTopkWarps) * n_expert * sizeof(float);
   if (smem > 48 * 1024) return kErrUnsupported;
-  router_topk_kernel<<<(n_rows + kTopkWarps - 1) / kTopkWarps, kTopkWarps * 32, smem,
-                       as_stream(stream)>>>(logits, idx, weight, n_expert, n_expert_used,
-                                            idx_stride, n_rows, shared_w);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
+  return launch_pdl(router_topk_kernel, dim3((n_rows + kTopkWarps - 1) / kTopkWarps), kTopkWarps * 32, smem,
+                    as_stream(stream), logits, idx, weight, n_expert, n_expert_used, idx_stride, n_rows, shared_w);
 }
 
 SGR_API int sgr_router_topk(const float* logits, int* idx, float* weight, int n_expert,

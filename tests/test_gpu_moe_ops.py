@@ -48,6 +48,26 @@ def test_dispatch_scan_matches_oracle(oracle, n, k, e, tok):
     assert got["mail_n"][0] == 0                                      # the scan resets the mailbox
 
 
+@pytest.mark.parametrize("n,k,e", [(600, 8, 256), (2048, 8, 64), (129, 3, 5000), (33, 1, 1), (16, 8, 10241)])
+def test_dispatch_scan_is_stable_at_any_size(oracle, n, k, e):
+    """Pieces of the route list per warp: several groups, a ragged last one, fewer warps for many experts."""
+    rng = np.random.default_rng(n)
+    idx = np.zeros((n, k + 1), dtype=np.int32)
+    idx[:, :k] = np.stack([rng.choice(e, k, replace=False) for _ in range(n)])
+    idx[n // 2, 0] = -7
+    w = rng.random((n, k + 1)).astype(np.float32)
+    got, want = run_scan(idx, w, n, k, e, 16), oracle.dispatch_scan(idx, w, n, k, e, 16)
+    R = want["meta"][0]
+    assert np.array_equal(got["off"], want["off"]) and np.array_equal(got["toff"], want["toff"])
+    assert np.array_equal(got["weight"], want["weight"]) and np.array_equal(got["meta"][:3], want["meta"][:3])
+    # ascending (row, kk) inside every expert
+    flat = idx[:, :k].reshape(-1)
+    order = np.argsort(np.where((flat < 0) | (flat >= e), e, flat), kind="stable")[:R]
+    gslot = np.full(n * k, -1)
+    gslot[order] = np.arange(R)
+    assert np.array_equal(got["gslot"], gslot) and np.array_equal(got["grows"][:R], order // k)
+
+
 def test_dispatch_scan_large_plan_properties():
     n, k, e, tok = 2048, 8, 256, 16       # prefill-sized: atomic fill, order inside an expert free
     rng = np.random.default_rng(5)
