@@ -4,6 +4,8 @@
 // multi-token, pointer-table, host-plan grouped and device-plan grouped with
 // the null-pointer mailbox. One kernel template, four planners; all of them
 // end in tile_run (tile.cuh).
+#include <algorithm>
+
 #include "api_util.cuh"
 #include "tile.cuh"
 
@@ -189,35 +191,14 @@ __global__ void __launch_bounds__(kTileThreads) gemv_tile_kernel(const GemvArgs 
       a.status);
 }
 
-// Every launch of the family may start while the kernel before it in the stream drains
-// (programmatic dependent launch); the kernels wait for that kernel's results themselves,
-// just before they first read anything it could have written.
-template <typename Kern>
-int launch_dependent(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, const GemvArgs& a) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? kOk : kErrLaunch;
-}
-
 template <int NMAT, int TT, int MODE, bool F16>
 int launch_tile(const GemvArgs& a, dim3 grid, cudaStream_t stream) {
   const size_t smem = tile_smem(NMAT, a.nb, TT);
   if (smem > 200 * 1024) return kErrUnsupported;
-  auto kern = gemv_tile_kernel<NMAT, TT, MODE, F16>;
-  if (smem > 48 * 1024) {
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem)) != cudaSuccess)
-      return kErrLaunch;
-  }
-  return launch_dependent(kern, grid, kTileThreads, smem, stream, a);
+  if (smem > 48 * 1024 && !opt_in_smem<gemv_tile_kernel<NMAT, TT, MODE, F16>>(static_cast<int>(smem))) return kErrLaunch;
+  // (every launch of the family may start while the kernel before it drains; the kernels wait for that
+  // one's results themselves, just before they first read anything it could have written)
+  return launch_pdl(gemv_tile_kernel<NMAT, TT, MODE, F16>, grid, kTileThreads, smem, stream, a);
 }
 
 // ---- dense matrices far larger than the machine (the LM head): a persistent kernel ----------
@@ -320,146 +301,197 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
 template <int TT, bool F16>
 int launch_stream(const GemvArgs& a, int sms, cudaStream_t stream) {
   const size_t smem = stream_gemv_smem(a.nb, TT);
-  auto kern = gemv_stream_kernel<TT, F16>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-      cudaSuccess)
-    return kErrLaunch;
-  return launch_dependent(kern, dim3(sms), kStreamThreads, smem, stream, a);
+  if (!opt_in_smem<gemv_stream_kernel<TT, F16>>(static_cast<int>(smem))) return kErrLaunch;
+  return launch_pdl(gemv_stream_kernel<TT, F16>, dim3(sms), kStreamThreads, smem, stream, a);
 }
 
 // The persistent kernel pays off when every SM gets several stages.
 inline int stream_sms(const GemvArgs& a) {
   if (a.n_tokens > 4 || a.nb > 16 || (a.nb & (a.nb - 1)) != 0) return 0;
   if (reinterpret_cast<uintptr_t>(a.w[0]) & 15u) return 0;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return 0;
+  const int sms = device_sms();
+  if (sms <= 0) return 0;
   const long long stages = (static_cast<long long>(a.n_rows) * a.nb + kStreamBlocks - 1) / kStreamBlocks;
   return stages >= 8LL * sms ? sms : 0;
 }
 
-// ---- small dense matrices, two to four token rows (a verify window) ------------------------
-// Fewer tiles than SMs: latency decides, not bandwidth, and staging through shared memory
-// only adds to it. One lane per 32-byte nibble group (two sub-blocks) straight from global
-// memory, no barriers. The integer partial sums of a super-block meet exactly by shuffle
-// over its four lanes, its fp32 term is formed once, and the terms of a row are added in
-// the order of the tile kernels' shuffle tree.
-constexpr int kDirectThreads = 128;
+// ---- dense matrices below the streaming kernel's size, one to eight token rows -----------------
+// A launch of a few microseconds: latency decides. One lane per 32-byte nibble group (two sub-blocks)
+// straight from global memory, every weight byte of a warp requested before the previous kernel is
+// awaited; the token rows are laid out in shared memory once per CTA so that a lane's 64 codes, two
+// sums and scale are five conflict-free reads (a group is 80 bytes, a block 320) and serve R rows.
+// The integer partial sums of a super-block meet exactly by shuffle over its four lanes, its fp32
+// term is formed once, and the terms of a row are added in the order of the tile kernels' shuffle
+// tree. Up to three matrices of the same k in one launch, their rows one after another.
+constexpr int kDirectWarps = 8;
+constexpr int kDirectGroup = 80, kDirectBlock = 4 * kDirectGroup;
 
-template <int NMAT, int TT, bool F16>
-__global__ void __launch_bounds__(kDirectThreads) gemv_direct_kernel(const GemvArgs a) {
-  const int nb = a.nb;
-  const int groups = nb * 4;
-  const int lpr = groups < 32 ? groups : 32;               // lanes per row (a power of two >= 4)
-  const int lane = threadIdx.x & 31;
-  const int warp = blockIdx.x * (kDirectThreads / 32) + (threadIdx.x >> 5);
-  const int row_raw = warp * (32 / lpr) + lane / lpr;
-  const int row = min(row_raw, a.n_rows - 1);              // every lane runs the same loops
-  const int lr = lane & (lpr - 1);
-  const int nt = a.n_tokens;
-  float acc[NMAT][TT];
+struct DirectArgs {
+  const unsigned char* w[3];
+  void* y[3];
+  int rows_cum[3];                      // rows of matrices 0..m inclusive
+  const unsigned char* xq;
+  int nb, n_tokens;
+  uint16_t* res;                        // one token, fp16 out: residual row updated in place
+};
+
+// R row steps per warp (a step is 32 / lanes-per-row rows), NI groups of a row per lane
+template <int TT, int R, int NI, bool F16>
+__global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const DirectArgs a) {
+  extern __shared__ __align__(16) unsigned char xs[];
+  const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lpr = NI > 1 ? 32 : min(nb * 4, 32);           // lanes per row (a power of two >= 4)
+  const int lr = lane & (lpr - 1), g = lr & 3, blk0 = lr >> 2;
+  const int rows_step = 32 / lpr, total = a.rows_cum[2];
+  const int row0 = (blockIdx.x * kDirectWarps + warp) * R * rows_step + lane / lpr;
+  uint4 hdr[R][NI], q0[R][NI], q1[R][NI];
 #pragma unroll
-  for (int m = 0; m < NMAT; ++m)
+  for (int r = 0; r < R; ++r) {
+    const int row = min(row0 + r * rows_step, total - 1);  // every lane runs the same loops
+    const int m = row >= a.rows_cum[0] ? (row >= a.rows_cum[1] ? 2 : 1) : 0;
+    const unsigned char* wm = m == 0 ? a.w[0] : (m == 1 ? a.w[1] : a.w[2]);
+    const int lrow = row - (m == 0 ? 0 : (m == 1 ? a.rows_cum[0] : a.rows_cum[1]));
+    const unsigned char* wb = wm + (static_cast<size_t>(lrow) * nb + blk0) * kW4;
 #pragma unroll
-    for (int t = 0; t < TT; ++t) acc[m][t] = 0.f;
-  bool waited = false;                     // the previous kernel is awaited once the first weights are requested
-  for (int gi = lr; gi < groups; gi += lpr) {
-    const int blk = gi >> 2, g = gi & 3;
-    float d[NMAT], dmin[NMAT];
-    uint32_t lo[NMAT][8], hi[NMAT][8];
-    int sc_lo[NMAT], sc_hi[NMAT], mn_lo[NMAT], mn_hi[NMAT];
+    for (int i = 0; i < NI; ++i) {
+      hdr[r][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+      q0[r][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 16 + 32 * g));
+      q1[r][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 32 + 32 * g));
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int b = warp; b < a.n_tokens * nb; b += 4 * kDirectWarps) {      // four blocks' words requested together
+    uint32_t v[4][3];
 #pragma unroll
-    for (int m = 0; m < NMAT; ++m) {
-      const unsigned char* wb = a.w[m] + (static_cast<size_t>(row) * nb + blk) * kW4;
-      const uint4 hdr = __ldg(reinterpret_cast<const uint4*>(wb));
-      const uint4 q0 = __ldg(reinterpret_cast<const uint4*>(wb + 16 + 32 * g));
-      const uint4 q1 = __ldg(reinterpret_cast<const uint4*>(wb + 32 + 32 * g));
-      d[m] = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x & 0xFFFFu)));
-      dmin[m] = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x >> 16)));
-      const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-      const uint32_t scw = g < 2 ? s6.sc[0] : s6.sc[1], mnw = g < 2 ? s6.mn[0] : s6.mn[1];
-      sc_lo[m] = (scw >> (16 * (g & 1))) & 0xFF;
-      sc_hi[m] = (scw >> (16 * (g & 1) + 8)) & 0xFF;
-      mn_lo[m] = (mnw >> (16 * (g & 1))) & 0xFF;
-      mn_hi[m] = (mnw >> (16 * (g & 1) + 8)) & 0xFF;
-      const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        lo[m][i] = raw[i] & 0x0F0F0F0Fu;
-        hi[m][i] = (raw[i] >> 4) & 0x0F0F0F0Fu;
+    for (int u = 0; u < 4; ++u) {
+      const int bb = b + u * kDirectWarps;
+      if (bb < a.n_tokens * nb) {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(a.xq + static_cast<size_t>(bb) * kX8) + lane;
+        v[u][0] = __ldg(src);
+        v[u][1] = __ldg(src + 32);
+        if (lane < 5) v[u][2] = __ldg(src + 64);
       }
     }
-    if (!waited) {
-      pdl_wait();
-      pdl_launch_dependents();
-      waited = true;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int bb = b + u * kDirectWarps;
+      if (bb < a.n_tokens * nb) {
+        unsigned char* dst = xs + bb * kDirectBlock;       // word 0: scale; 1..64: codes; 65..68: sums
+        auto put = [&](int w, uint32_t x) { *reinterpret_cast<uint32_t*>(dst + (w >> 4) * kDirectGroup + (w & 15) * 4) = x; };
+        if (lane > 0) put(lane - 1, v[u][0]);
+        put(lane + 31, v[u][1]);
+        if (lane == 0) put(63, v[u][2]);
+        else if (lane < 5) *reinterpret_cast<uint32_t*>(dst + (lane - 1) * kDirectGroup + 64) = v[u][2];
+        const uint32_t d = __shfl_sync(0xFFFFFFFFu, v[u][0], 0);
+        if (lane < 4) *reinterpret_cast<uint32_t*>(dst + lane * kDirectGroup + 68) = d;
+      }
     }
+  }
+  __syncthreads();
+
+  constexpr int NA = NI > 1 ? 2 : 1;        // rows of 32 blocks: (t0 + t2) + (t1 + t3), the shuffle tree's order
+  float acc[R][TT][NA];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int t = 0; t < TT; ++t)
+#pragma unroll
+      for (int c = 0; c < NA; ++c) acc[r][t][c] = 0.f;
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
 #pragma unroll
     for (int t = 0; t < TT; ++t) {
-      if (t < nt) {
-        const unsigned char* xb = a.xq + (static_cast<size_t>(t) * nb + blk) * kX8;
-        const uint32_t* xc = reinterpret_cast<const uint32_t*>(xb + 4 + 64 * g);
-        uint32_t xv[16];
+      if (t < a.n_tokens) {
+        const unsigned char* xb = xs + (t * nb + blk0 + 8 * i) * kDirectBlock + g * kDirectGroup;
+        const uint4 x0 = *reinterpret_cast<const uint4*>(xb), x1 = *reinterpret_cast<const uint4*>(xb + 16);
+        const uint4 x2 = *reinterpret_cast<const uint4*>(xb + 32), x3 = *reinterpret_cast<const uint4*>(xb + 48);
+        const uint2 sd = *reinterpret_cast<const uint2*>(xb + 64);
+        const int bs_lo = static_cast<int16_t>(sd.x & 0xFFFFu), bs_hi = static_cast<int16_t>(sd.x >> 16);
+        const float xd = __uint_as_float(sd.y);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) xv[i] = __ldg(xc + i);
-        const uint32_t bs = __ldg(reinterpret_cast<const uint32_t*>(xb + 260 + 4 * g));   // two int16 sums
-        const float xd = __ldg(reinterpret_cast<const float*>(xb));
-        const int bs_lo = static_cast<int16_t>(bs & 0xFFFFu), bs_hi = static_cast<int16_t>(bs >> 16);
+        for (int r = 0; r < R; ++r) {
+          const Scales6 s6 = unpack_scales6(hdr[r][i].y, hdr[r][i].z, hdr[r][i].w);
+          const uint32_t scw = (g < 2 ? s6.sc[0] : s6.sc[1]) >> (16 * (g & 1)), mnw = (g < 2 ? s6.mn[0] : s6.mn[1]) >> (16 * (g & 1));
+          const uint32_t raw[8] = {q0[r][i].x, q0[r][i].y, q0[r][i].z, q0[r][i].w, q1[r][i].x, q1[r][i].y, q1[r][i].z, q1[r][i].w};
+          uint32_t lo[8], hi[8];
 #pragma unroll
-        for (int m = 0; m < NMAT; ++m) {
-          int dl = 0, dh = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            dl = __dp4a(static_cast<int>(lo[m][i]), static_cast<int>(xv[i]), dl);
-            dh = __dp4a(static_cast<int>(hi[m][i]), static_cast<int>(xv[8 + i]), dh);
+          for (int j = 0; j < 8; ++j) {
+            lo[j] = raw[j] & 0x0F0F0F0Fu;
+            hi[j] = (raw[j] >> 4) & 0x0F0F0F0Fu;
           }
-          int isum = sc_lo[m] * dl + sc_hi[m] * dh;
-          int msum = mn_lo[m] * bs_lo + mn_hi[m] * bs_hi;
+          int isum = static_cast<int>(scw & 0xFF) * dot8(lo, x0, x1) + static_cast<int>((scw >> 8) & 0xFF) * dot8(hi, x2, x3);
+          int msum = static_cast<int>(mnw & 0xFF) * bs_lo + static_cast<int>((mnw >> 8) & 0xFF) * bs_hi;
           isum += __shfl_xor_sync(0xFFFFFFFFu, isum, 1);
           msum += __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
           isum += __shfl_xor_sync(0xFFFFFFFFu, isum, 2);
           msum += __shfl_xor_sync(0xFFFFFFFFu, msum, 2);
-          if (g == 0) acc[m][t] += xd * (d[m] * static_cast<float>(isum) - dmin[m] * static_cast<float>(msum));
+          const float d = h2f(static_cast<uint16_t>(hdr[r][i].x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr[r][i].x >> 16));
+          acc[r][t][i % NA] += xd * (d * static_cast<float>(isum) - dmin * static_cast<float>(msum));
         }
       }
     }
   }
-  if (!waited) {
-    pdl_wait();
-    pdl_launch_dependents();
-  }
 #pragma unroll
-  for (int m = 0; m < NMAT; ++m)
+  for (int r = 0; r < R; ++r) {
+    const int row = row0 + r * rows_step;
+    const int m = row >= a.rows_cum[0] ? (row >= a.rows_cum[1] ? 2 : 1) : 0;
+    const int lo_row = m == 0 ? 0 : (m == 1 ? a.rows_cum[0] : a.rows_cum[1]);
+    const int m_rows = (m == 0 ? a.rows_cum[0] : (m == 1 ? a.rows_cum[1] : a.rows_cum[2])) - lo_row;
+    void* y = m == 0 ? a.y[0] : (m == 1 ? a.y[1] : a.y[2]);
 #pragma unroll
-    for (int t = 0; t < TT; ++t) acc[m][t] = reduce_lanes(acc[m][t], lpr);
-  if (lr == 0 && row_raw < a.n_rows) {
-#pragma unroll
-    for (int t = 0; t < TT; ++t)
-      if (t < nt) {
-#pragma unroll
-        for (int m = 0; m < NMAT; ++m)
-          store_out<F16>(a.y[m], static_cast<size_t>(t) * a.n_rows + row_raw, acc[m][t]);
+    for (int t = 0; t < TT; ++t) {
+      if (t >= a.n_tokens) break;
+      float v = acc[r][t][0];
+      if constexpr (NA > 1) v += acc[r][t][1];
+      for (int off = lpr >> 1; off >= 4; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, off);
+      if (lr != 0 || row >= total) continue;
+      if constexpr (F16 && TT == 1) {
+        if (a.res != nullptr) {
+          store_out_resadd(reinterpret_cast<uint16_t*>(y), a.res, static_cast<size_t>(row - lo_row), v);
+          continue;
+        }
       }
+      store_out<F16>(y, static_cast<size_t>(t) * m_rows + row - lo_row, v);
+    }
   }
 }
 
-template <int NMAT, bool F16>
-int launch_direct(const GemvArgs& a, cudaStream_t stream) {
-  const int lpr = a.nb * 4 < 32 ? a.nb * 4 : 32;
-  const int rows_per_cta = (kDirectThreads / 32) * (32 / lpr);
-  const int grid = (a.n_rows + rows_per_cta - 1) / rows_per_cta;
-  if (a.n_tokens == 2) return launch_dependent(gemv_direct_kernel<NMAT, 2, F16>, dim3(grid), kDirectThreads, 0, stream, a);
-  return launch_dependent(gemv_direct_kernel<NMAT, 4, F16>, dim3(grid), kDirectThreads, 0, stream, a);
+template <int TT, int R, int NI, bool F16>
+int launch_direct_as(const DirectArgs& a, cudaStream_t stream) {
+  const size_t smem = static_cast<size_t>(a.n_tokens) * a.nb * kDirectBlock;
+  if (smem > 48 * 1024 && !opt_in_smem<gemv_direct_kernel<TT, R, NI, F16>>(8 * 32 * kDirectBlock)) return kErrLaunch;
+  const int rows_cta = kDirectWarps * R * (NI > 1 ? 1 : std::max(1, 8 / a.nb));
+  return launch_pdl(gemv_direct_kernel<TT, R, NI, F16>, dim3((a.rows_cum[2] + rows_cta - 1) / rows_cta), kDirectWarps * 32, smem,
+                    stream, a);
 }
-
-// Two to four token rows over a matrix of at most a few tiles per SM, 16-byte aligned.
-template <int NMAT>
-inline bool direct_fits(const GemvArgs& a) {
-  if (a.n_tokens < 2 || a.n_tokens > 4 || (a.nb & (a.nb - 1)) != 0) return false;
-  for (int m = 0; m < NMAT; ++m)
+template <int TT, bool F16>
+int launch_direct_tt(const DirectArgs& a, cudaStream_t stream) {
+  // rows per warp: as many as registers hold while every SM still gets eight warps
+  const long long steps = a.nb >= 8 ? a.rows_cum[2] : (a.rows_cum[2] + 8 / a.nb - 1) / (8 / a.nb);
+  const long long per_sm = 148LL * kDirectWarps;
+  if (a.nb <= 8) {
+    if (steps >= 4 * per_sm) return launch_direct_as<TT, 4, 1, F16>(a, stream);
+    if (steps >= 2 * per_sm) return launch_direct_as<TT, 2, 1, F16>(a, stream);
+    return launch_direct_as<TT, 1, 1, F16>(a, stream);
+  }
+  if (a.nb == 16)
+    return steps >= 2 * per_sm ? launch_direct_as<TT, 2, 2, F16>(a, stream) : launch_direct_as<TT, 1, 2, F16>(a, stream);
+  return launch_direct_as<TT, 1, 4, F16>(a, stream);
+}
+// One to eight token rows, rows of a power of two of blocks up to 32, 16-byte aligned matrices.
+inline bool direct_fits(const DirectArgs& a) {
+  if (a.n_tokens < 1 || a.n_tokens > 8 || a.nb > 32 || (a.nb & (a.nb - 1)) != 0) return false;
+  for (int m = 0; m < 3; ++m)
     if (reinterpret_cast<uintptr_t>(a.w[m]) & 15u) return false;
-  return static_cast<long long>(a.n_rows) * a.nb <= 148LL * 4 * kStreamBlocks;
+  return true;
+}
+template <bool F16>
+int launch_direct(const DirectArgs& a, cudaStream_t stream) {
+  if (a.n_tokens == 1) return launch_direct_tt<1, F16>(a, stream);
+  if (a.n_tokens == 2) return launch_direct_tt<2, F16>(a, stream);
+  if (a.n_tokens <= 4) return launch_direct_tt<4, F16>(a, stream);
+  return launch_direct_tt<8, F16>(a, stream);
 }
 
 // tokens per CTA of the dense multi-token kernels (walked in sub-tiles of 8)
@@ -490,7 +522,10 @@ int launch_dense(const void* w0, const void* w1, const void* xq, void* y0, void*
       return launch_stream<4, F16>(a, sms, stream);
     }
   }
-  if (direct_fits<NMAT>(a)) return launch_direct<NMAT, F16>(a, stream);
+  {
+    DirectArgs d{{a.w[0], NMAT == 2 ? a.w[1] : nullptr, nullptr}, {y0, y1, nullptr}, {n_rows, NMAT * n_rows, NMAT * n_rows}, a.xq, a.nb, n_tokens, res};
+    if (NMAT * static_cast<long long>(n_rows) <= 0x7FFFFFFF && direct_fits(d)) return launch_direct<F16>(d, stream);
+  }
   if (n_tokens == 1) {
     a.tok_tile = 1;
     return launch_tile<NMAT, 1, kDense, F16>(a, dim3((n_rows + rc - 1) / rc, 1), stream);
@@ -613,6 +648,7 @@ int launch_multi(int nmat, const void* const (&w)[3], const void* xq, uint16_t* 
   if (reinterpret_cast<uintptr_t>(xq) & 3u) return kErrAlign;
   GemvArgs a{};
   int cum = 0, tiles = 0;
+  DirectArgs d{};
   a.nb = k / kQK;
   const int rc = tile_rows(a.nb);
   for (int m = 0; m < 3; ++m) {
@@ -621,6 +657,7 @@ int launch_multi(int nmat, const void* const (&w)[3], const void* xq, uint16_t* 
     a.ym[m] = m < nmat ? y[m] : nullptr;
     cum += r;
     a.rows_cum[m] = cum;
+    d.w[m] = a.wm[m]; d.y[m] = a.ym[m]; d.rows_cum[m] = cum;
     tiles += (r + rc - 1) / rc;
   }
   a.xq = static_cast<const unsigned char*>(xq);
@@ -628,6 +665,8 @@ int launch_multi(int nmat, const void* const (&w)[3], const void* xq, uint16_t* 
   a.n_tokens = 1;
   a.tok_tile = 1;
   a.status = status_word();
+  d.xq = a.xq; d.nb = a.nb; d.n_tokens = 1;
+  if (direct_fits(d)) return launch_direct<true>(d, stream);
   return launch_tile<1, 1, kMulti, true>(a, dim3(tiles, 1), stream);
 }
 }  // namespace

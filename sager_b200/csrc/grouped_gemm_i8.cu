@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
       int slot = 0;
       unsigned slot_ph = 0;
       const uint32_t d_min = umma_desc(smem_u32(smem + kOffMin)), d_b = umma_desc(smem_u32(smem + kOffB));
+      const uint32_t lead = elect_one();
       bool ok = true;
       while (ok && wk.next<DUAL>(a, u)) {
         if (u.w0 == nullptr) continue;
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
           for (int h = 0; h < 2; ++h) {
             if (!wait_warp(kBarAFull + slot, slot_ph)) return false;
             tc_fence_after();
-            const uint32_t ta = tmem + kColA + slot * 64, lead = elect_one();
+            const uint32_t ta = tmem + kColA + slot * 64;
 #pragma unroll
             for (int k = 0; k < 8; ++k) umma_ts(lead, d0, ta + k * 8, db + (h * 8 + k) * (kBTile >> 4), idesc, (h | k) != 0);
             if (h == 1) umma_ss(lead, d1, dm, db + 16 * (kBTile >> 4), idesc, 0u);

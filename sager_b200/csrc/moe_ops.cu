@@ -15,133 +15,127 @@ __device__ __forceinline__ bool aligned16(const void* p) {
 }
 
 // ---- dispatch plan (moe.cu:366-434) ---------------------------------------------
-// One CTA. Every warp owns a contiguous piece of the route list and counts it per expert in a
-// shared-memory row of its own (lanes with the same expert meet by match_any); per expert a prefix
-// over the warps and one over the experts give each warp its first slots, and a second walk hands
-// the slots out. So the slots inside an expert are in ascending (row, kk) order whatever the size
-// and nothing is contended; what bounds it is the latency of the phases. Before: 16,384 routes over
-// 256 experts 24 us with atomics, 768 routes filled by one thread per expert 35 us.
-constexpr int kScanThreads = 1024;
-constexpr int kScanCounters = 10240;       // [warps that share the list][n_expert] counters of 4 bytes
+// Every CTA reads the whole route list, counts it per expert and part of the list (shared-memory
+// atomics) and builds the prefixes for itself, so nothing is exchanged; each of its warps then walks
+// one part of the list for one expert of its own and hands the slots out by ballot. The slots inside
+// an expert are in ascending (row, kk) order whatever the size. Bound by the latency of the phases.
+// One CTA took 24 us for 16,384 routes over 256 experts (atomic fill) and 35 us for 768 (a thread per
+// expert walking the list); counting and ranking by match_any in one CTA 48 and 9 us.
+constexpr int kScanThreads = 512, kScanWarps = kScanThreads / 32;
+constexpr int kScanParts = 4;              // of the list, while [parts][n_expert] counters stay small
+constexpr int kScanPartExperts = 2048;
+constexpr int kScanStaged = 64 * 1024;     // routes whose ids are kept in shared memory, two bytes each
 
 __global__ void __launch_bounds__(kScanThreads)
 dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, int* __restrict__ gslot,
                      int* __restrict__ grows, int* __restrict__ off, int* __restrict__ toff,
                      int* __restrict__ meta, int* __restrict__ mail_n, int n_rows, int k,
-                     int n_expert, int tok_per, int n_warps) {
-  extern __shared__ int cnt[];             // [n_warps][n_expert]: counts, then next slots
+                     int n_expert, int tok_per, int parts, int staged) {
+  extern __shared__ __align__(16) int cnt[];             // [parts][n_expert] counts, then first slots; ids after them
+  uint16_t* ids = reinterpret_cast<uint16_t*>(cnt + static_cast<size_t>(parts) * n_expert);
   __shared__ int bad_sh;
+  __shared__ int wsum[2][kScanWarps];
+  __shared__ int carry[2];
   pdl_wait();
   pdl_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const int total = n_rows * k;
-  const int per = ((total + n_warps - 1) / n_warps + 31) & ~31;       // routes per warp
-  const int i0 = min(wp * per, total), i1 = wp < n_warps ? min(i0 + per, total) : i0;
-  if (tid == 0) bad_sh = 0;
-  for (int e = tid; e < n_warps * n_expert; e += kScanThreads) cnt[e] = 0;
+  const int per = ((total + parts - 1) / parts + 31) & ~31;           // routes per part
+  if (tid == 0) bad_sh = carry[0] = carry[1] = 0;
+  for (int e = tid; e < parts * n_expert; e += kScanThreads) cnt[e] = 0;
   __syncthreads();
-  int* mine = cnt + static_cast<size_t>(min(wp, n_warps - 1)) * n_expert;
   auto id_of = [&](int i) {
     const int r = i / k;
     const int e = __ldg(idx + static_cast<size_t>(r) * (k + 1) + (i - r * k));
-    return e >= 0 && e < n_expert ? e : -1;
+    return e >= 0 && e < n_expert ? e : 0xFFFF;
   };
-  // four groups of 32 routes requested together
-  for (int b = i0; b < i1; b += 128) {
-    int e4[4];
+  for (int b = tid; b < total; b += 8 * kScanThreads) {
+    int e8[8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int i = b + 32 * q + lane;
-      e4[q] = i < i1 ? id_of(i) : -2;                                 // -2: past the end
-    }
+    for (int q = 0; q < 8; ++q) e8[q] = b + q * kScanThreads < total ? id_of(b + q * kScanThreads) : -1;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const unsigned same = __match_any_sync(0xFFFFFFFFu, e4[q]);
-      if (e4[q] >= 0 && lane == __ffs(same) - 1) mine[e4[q]] += __popc(same);
-      if (e4[q] == -1) {
+    for (int q = 0; q < 8; ++q) {
+      const int i = b + q * kScanThreads;
+      if (e8[q] < 0) continue;
+      if (staged) ids[i] = static_cast<uint16_t>(e8[q]);
+      if (e8[q] != 0xFFFF) {
+        atomicAdd(cnt + static_cast<size_t>(i / per) * n_expert + e8[q], 1);
+      } else if (blockIdx.x == 0) {
         // a corrupt id silences the whole row, shared-expert slot included
-        const int i = b + 32 * q + lane;
         float* wr = weight + static_cast<size_t>(i / k) * (k + 1);
         for (int j = 0; j <= k; ++j) wr[j] = 0.f;
         gslot[i] = -1;
         atomicAdd(&bad_sh, 1);
       }
-      __syncwarp();
     }
   }
   __syncthreads();
 
   // exclusive prefixes of rows and of tiles over the experts: kScanThreads experts per round, scans
   // inside the warps, the warps' totals and the running totals through shared memory
-  {
-    __shared__ int wsum[2][kScanThreads / 32];
-    __shared__ int carry[2];
-    if (tid == 0) carry[0] = carry[1] = 0;
-    __syncthreads();
-    for (int base = 0; base < n_expert; base += kScanThreads) {
-      const int e = base + tid;
-      int c = 0;
-      if (e < n_expert) {
-        for (int w = 0; w < n_warps; ++w) {                           // the expert's routes, warp after warp
-          const int v = cnt[static_cast<size_t>(w) * n_expert + e];
-          cnt[static_cast<size_t>(w) * n_expert + e] = c;
-          c += v;
-        }
+  for (int base = 0; base < n_expert; base += kScanThreads) {
+    const int e = base + tid;
+    int c = 0;
+    if (e < n_expert) {
+      for (int w = 0; w < parts; ++w) {                               // the expert's routes, part after part
+        const int v = cnt[static_cast<size_t>(w) * n_expert + e];
+        cnt[static_cast<size_t>(w) * n_expert + e] = c;
+        c += v;
       }
-      const int t = (c + tok_per - 1) / tok_per;
-      int ic = c, it = t;
+    }
+    const int t = (c + tok_per - 1) / tok_per;
+    int ic = c, it = t;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int uc = __shfl_up_sync(0xFFFFFFFFu, ic, o), ut = __shfl_up_sync(0xFFFFFFFFu, it, o);
-        if (lane >= o) { ic += uc; it += ut; }
-      }
-      if (lane == 31) { wsum[0][wp] = ic; wsum[1][wp] = it; }
-      __syncthreads();
-      int pc = carry[0], pt = carry[1];
-      for (int w = 0; w < wp; ++w) { pc += wsum[0][w]; pt += wsum[1][w]; }
-      if (e < n_expert) {
-        const int o0 = pc + ic - c;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int uc = __shfl_up_sync(0xFFFFFFFFu, ic, o), ut = __shfl_up_sync(0xFFFFFFFFu, it, o);
+      if (lane >= o) { ic += uc; it += ut; }
+    }
+    if (lane == 31) { wsum[0][wp] = ic; wsum[1][wp] = it; }
+    __syncthreads();
+    int pc = carry[0], pt = carry[1];
+    for (int w = 0; w < wp; ++w) { pc += wsum[0][w]; pt += wsum[1][w]; }
+    if (e < n_expert) {
+      const int o0 = pc + ic - c;
+      if (blockIdx.x == 0) {
         off[e] = o0;
         toff[e] = pt + it - t;
-        for (int w = 0; w < n_warps; ++w) cnt[static_cast<size_t>(w) * n_expert + e] += o0;
       }
-      __syncthreads();
-      if (tid == kScanThreads - 1) { carry[0] = pc + ic; carry[1] = pt + it; }
-      __syncthreads();
+      for (int w = 0; w < parts; ++w) cnt[static_cast<size_t>(w) * n_expert + e] += o0;
     }
-    if (tid == 0) {
-      off[n_expert] = carry[0];
-      toff[n_expert] = carry[1];
-      meta[0] = carry[0];
-      meta[1] = carry[1];
-      meta[2] = bad_sh;
-      if (mail_n != nullptr) *mail_n = 0;
-    }
+    __syncthreads();
+    if (tid == kScanThreads - 1) { carry[0] = pc + ic; carry[1] = pt + it; }
+    __syncthreads();
+  }
+  if (blockIdx.x == 0 && tid == 0) {
+    off[n_expert] = carry[0];
+    toff[n_expert] = carry[1];
+    meta[0] = carry[0];
+    meta[1] = carry[1];
+    meta[2] = bad_sh;
+    if (mail_n != nullptr) *mail_n = 0;
   }
 
-  for (int b = i0; b < i1; b += 128) {
-    int e4[4];
+  const int e = blockIdx.x * (kScanWarps / parts) + wp / parts, part = wp % parts;
+  if (e >= n_expert) return;
+  int pos = cnt[static_cast<size_t>(part) * n_expert + e];
+  const int i1 = min((part + 1) * per, total);
+  for (int b = part * per; b < i1; b += 256) {
+    int e8[8];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < 8; ++q) {
       const int i = b + 32 * q + lane;
-      e4[q] = i < i1 ? id_of(i) : -1;
+      e8[q] = i < i1 ? (staged ? ids[i] : id_of(i)) : -1;
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const unsigned same = __match_any_sync(0xFFFFFFFFu, e4[q]);
-      const int first = __ffs(same) - 1;
-      int slot = 0;
-      if (e4[q] >= 0 && lane == first) {
-        slot = mine[e4[q]];
-        mine[e4[q]] = slot + __popc(same);
-      }
-      slot = __shfl_sync(0xFFFFFFFFu, slot, first) + __popc(same & ((1u << lane) - 1u));
-      if (e4[q] >= 0) {
-        const int i = b + 32 * q + lane;
+    for (int q = 0; q < 8; ++q) {
+      const unsigned hit = __ballot_sync(0xFFFFFFFFu, e8[q] == e);
+      if (hit == 0) continue;
+      if (e8[q] == e) {
+        const int i = b + 32 * q + lane, slot = pos + __popc(hit & ((1u << lane) - 1u));
         gslot[i] = slot;
         grows[slot] = i / k;
       }
-      __syncwarp();
+      pos += __popc(hit);
     }
   }
 }
@@ -351,11 +345,13 @@ SGR_API int sgr_moe_dispatch_scan(const int* idx, float* weight, int* gslot, int
       n_expert <= 0 || tok_per <= 0)
     return kErrArg;
   if (static_cast<long long>(n_rows) * k > 0x7FFFFF00) return kErrArg;
-  // the counters of as many warps as fit the default 48 KB; the former limit on experts, 6144, is within it
-  if (n_expert > 12000) return kErrUnsupported;
-  const int n_warps = std::max(1, std::min(kScanThreads / 32, kScanCounters / n_expert));
-  return launch_pdl(dispatch_scan_kernel, dim3(1), kScanThreads, static_cast<size_t>(n_warps) * n_expert * sizeof(int),
-                    as_stream(stream), idx, weight, gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, n_warps);
+  if (n_expert > 12 * 1024) return kErrUnsupported;
+  const int parts = n_expert <= kScanPartExperts ? kScanParts : 1, per_cta = kScanWarps / parts;
+  const int staged = n_rows * k <= kScanStaged;
+  const size_t smem = static_cast<size_t>(parts) * n_expert * sizeof(int) + (staged ? static_cast<size_t>(n_rows) * k * 2 : 0);
+  if (smem > 40 * 1024 && !opt_in_smem<dispatch_scan_kernel>(200 * 1024)) return kErrLaunch;
+  return launch_pdl(dispatch_scan_kernel, dim3((n_expert + per_cta - 1) / per_cta), kScanThreads, smem, as_stream(stream), idx, weight,
+                    gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, parts, staged);
 }
 
 SGR_API int sgr_gather_rows_q8(void* dst, const void* src, const int* src_rows, int n_rows,

@@ -17,6 +17,8 @@ constexpr int kQuantWarps = 4;
 __global__ void __launch_bounds__(kQuantWarps * 32)
 quantize_q8_k_kernel(const uint16_t* __restrict__ x, unsigned char* __restrict__ out,
                      long long n_blocks, const int* __restrict__ d_rows, int row_mult) {
+  pdl_wait();
+  pdl_launch_dependents();
   const long long b = static_cast<long long>(blockIdx.x) * kQuantWarps + (threadIdx.x >> 5);
   long long live = n_blocks;
   if (d_rows != nullptr) {
@@ -38,10 +40,8 @@ SGR_API int sgr_quantize_q8_k(const uint16_t* x_f16, void* out, long long n, voi
   if ((reinterpret_cast<uintptr_t>(out) & 3u) || (reinterpret_cast<uintptr_t>(x_f16) & 1u))
     return kErrAlign;
   const long long nblk = n / kQK;
-  quantize_q8_k_kernel<<<static_cast<unsigned>((nblk + kQuantWarps - 1) / kQuantWarps),
-                         kQuantWarps * 32, 0, as_stream(stream)>>>(
-      x_f16, static_cast<unsigned char*>(out), nblk, nullptr, 0);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
+  return launch_pdl(quantize_q8_k_kernel, dim3(static_cast<unsigned>((nblk + kQuantWarps - 1) / kQuantWarps)), kQuantWarps * 32, 0,
+                    as_stream(stream), x_f16, static_cast<unsigned char*>(out), nblk, static_cast<const int*>(nullptr), 0);
 }
 
 // Device-count variant (q4_k.cu:1869-1924 of the reference): the live element
@@ -53,8 +53,6 @@ SGR_API int sgr_quantize_q8_k_n(const uint16_t* x_f16, void* out, const int* d_r
   if (!x_f16 || !out || !d_rows || row_mult <= 0) return kErrArg;
   if ((reinterpret_cast<uintptr_t>(out) & 3u) || (reinterpret_cast<uintptr_t>(x_f16) & 1u))
     return kErrAlign;
-  quantize_q8_k_kernel<<<(n_max + kQuantWarps - 1) / kQuantWarps, kQuantWarps * 32, 0,
-                         as_stream(stream)>>>(x_f16, static_cast<unsigned char*>(out), n_max, d_rows,
-                                              row_mult);
-  return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
+  return launch_pdl(quantize_q8_k_kernel, dim3((n_max + kQuantWarps - 1) / kQuantWarps), kQuantWarps * 32, 0, as_stream(stream),
+                    x_f16, static_cast<unsigned char*>(out), static_cast<long long>(n_max), d_rows, row_mult);
 }

@@ -102,6 +102,7 @@ class MoeStack:
         self.idx = torch.zeros(len(layers), n_max, n_used + 1, dtype=torch.int32, device=device)
         self.w = torch.zeros(len(layers), n_max, n_used + 1, dtype=torch.float32, device=device)
         # one persistent launch per layer for up to three rows, else route + experts
+        self._args = {}
         self.launches_per_step = (1 if (kernel is None and n_max <= 3) else 2) * len(layers)
         # chain: layer l's input rows are RMSNorm(x) computed on the device by rmsnorm_quant_f16 (the
         # producer of the MoE half's rows in the reference's decode layer, src/core/session.cpp:1020-1032),
@@ -115,20 +116,29 @@ class MoeStack:
             self.launches_per_step += len(layers)
 
     def layer_args(self, li, n):
+        """The runner and the argument block of a layer. A step whose row count changes is issued call by call, so the
+        blocks are kept, one per (layer, row count), for as long as the addresses in them stay the same."""
         w = self.layers[li]
         r = self.runners[li % len(self.runners)]
         xn = self.xn if self.chain else self.x if self.inputs is None else self.inputs[li]
-        return r, r.args(n, xn, w.router, self.tables[li], w.shared_ptrs(), x_f16=self.x,
-                         bias=None if self.biases is None else self.biases[li],
-                         route_idx=self.idx[li], route_w=self.w[li])
+        bias = None if self.biases is None else self.biases[li]
+        key = tuple([t.data_ptr() for t in (xn, self.x, self.tables[li], w.router, w.blob, self.idx, self.w, r.ws)] +
+                    [bias.data_ptr() if bias is not None else 0])
+        kept = self._args.get((li, n))
+        if kept is None or kept[0] != key:
+            kept = (key, r.args(n, xn, w.router, self.tables[li], w.shared_ptrs(), x_f16=self.x, bias=bias,
+                                route_idx=self.idx[li], route_w=self.w[li]))
+            self._args[(li, n)] = kept
+        return r, kept[1]
 
     def _issue(self, n, stages=7):
+        stream = stream_ptr()
         for li in range(len(self.layers)):
             r, a = self.layer_args(li, n)
             if self.chain and (stages & 1):
                 lib().call("sgr_rmsnorm_quant_f16", _p(self.xn), _p(self.x), _p(self.norm_w[li]), _p(self.xq),
-                           self.layers[0].hidden, 1e-6, n, stream_ptr())
-            lib().call("sgr_moe_layer_decode_stages", C.byref(a), stages | self.kernel_bits, stream_ptr())
+                           self.layers[0].hidden, 1e-6, n, stream)
+            lib().call("sgr_moe_layer_decode_stages", C.byref(a), stages | self.kernel_bits, stream)
 
     def step_eager(self, n):
         self._issue(n)

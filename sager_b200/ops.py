@@ -8,41 +8,54 @@ torch's current stream. Nothing here computes: a missing library raises.
 from __future__ import annotations
 
 import ctypes as C
+import sys
 
 import torch
 
-from .capi import lib
+from .capi import SagerError, lib
 
 
-def _conv(a):
-    if a is None:
-        return None
-    if isinstance(a, torch.Tensor):
-        return C.c_void_p(a.data_ptr())
-    if isinstance(a, int) and a > 0x7FFFFFFF:
-        return C.c_void_p(a)                 # a raw device address
-    return a
+_raw_stream = torch._C._cuda_getCurrentRawStream
+_device = torch._C._cuda_getDevice
+
+
+def _stream() -> int:
+    """torch's current stream as an address (0 is the default stream), without building a Stream object."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return _raw_stream(_device())
 
 
 def stream_ptr():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(_stream())
+
+
+def _bind(name: str):
+    """The entry point as a Python function: tensors go as device addresses, the current stream last. A decode
+    step issues hundreds of these, so what does not depend on the arguments is looked up once."""
+    L = lib()
+    cfn = getattr(L.cdll, "sgr_" + name)
+    tensor, stream = torch.Tensor, _stream
+
+    def fn(*args):
+        rc = cfn(*[a.data_ptr() if isinstance(a, tensor) else a for a in args], stream())
+        if rc != 0:
+            raise SagerError("sgr_" + name, rc)
+
+    fn.__name__ = name
+    return fn
 
 
 def call(name: str, *args):
-    lib().call("sgr_" + name, *[_conv(a) for a in args], stream_ptr())
+    getattr(sys.modules[__name__], name)(*args)
 
 
 def __getattr__(name):
     if name.startswith("_"):
         raise AttributeError(name)
-    protos = lib().protos
-    if "sgr_" + name not in protos:
+    if "sgr_" + name not in lib().protos:
         raise AttributeError(f"no entry point sgr_{name}")
-
-    def fn(*args):
-        call(name, *args)
-
-    fn.__name__ = name
+    fn = globals()[name] = _bind(name)
     return fn
 
 

@@ -48,9 +48,9 @@ def test_dispatch_scan_matches_oracle(oracle, n, k, e, tok):
     assert got["mail_n"][0] == 0                                      # the scan resets the mailbox
 
 
-@pytest.mark.parametrize("n,k,e", [(600, 8, 256), (2048, 8, 64), (129, 3, 5000), (33, 1, 1), (16, 8, 10241)])
+@pytest.mark.parametrize("n,k,e", [(600, 8, 256), (2048, 8, 64), (129, 3, 5000), (33, 1, 1), (16, 8, 10241), (9000, 8, 256), (1, 1, 2048)])
 def test_dispatch_scan_is_stable_at_any_size(oracle, n, k, e):
-    """Pieces of the route list per warp: several groups, a ragged last one, fewer warps for many experts."""
+    """Parts of the route list: ragged ones, one part above 2048 experts, ids kept in shared memory or read again."""
     rng = np.random.default_rng(n)
     idx = np.zeros((n, k + 1), dtype=np.int32)
     idx[:, :k] = np.stack([rng.choice(e, k, replace=False) for _ in range(n)])

@@ -280,3 +280,21 @@ def test_grouped_device_plan_with_absent_experts(oracle, tok_per):
             assert f16_close(yd[r].cpu().numpy(), oracle.gemv(mats[e][2][0], hq_np[r], hidden, n_ff))
     n_mail = int(mail_n.item())
     assert sorted(mail.cpu().numpy()[:n_mail].tolist()) == sorted(mails_expected)
+
+
+@pytest.mark.parametrize("rows,k", [(1, 256), (37, 256), (67, 512), (129, 1024), (1187, 2048), (2371, 2048), (4737, 2048), (33, 4096),
+                                    (2373, 4096), (19, 8192)])
+@pytest.mark.parametrize("tok", [1, 2, 3, 4, 5, 8])
+def test_direct_kernel_edges(oracle, rows, k, tok):
+    """Every variant of the small-matrix kernel (lanes per row, rows per warp, groups per lane, token slots) at ragged row
+    counts; the line between one, two and four rows per warp lies at 1184 x 2 and x 4 rows."""
+    w_np, w_dev = make_q4k(rows, k, 5)
+    x_np, x_dev = make_x16(tok, k, 6)
+    xq = torch.zeros(tok, k // 256 * 276, dtype=torch.uint8, device=DEV)
+    ops.quantize_q8_k(x_dev, xq, tok * k)
+    y = torch.full((tok + 1, rows), 5.0, dtype=torch.float32, device=DEV)
+    ops.gemv_q4_k_q8_batched(w_dev, xq, y, rows, k, tok)
+    got = y.cpu().numpy()
+    for t in range(tok):
+        assert rel(got[t], oracle.gemv(w_np, xq.cpu().numpy()[t], rows, k)) <= GEMV_TOL
+    assert np.all(got[tok] == 5.0)
