@@ -316,15 +316,18 @@ inline int stream_sms(const GemvArgs& a) {
 }
 
 // ---- dense matrices below the streaming kernel's size, one to eight token rows -----------------
-// A launch of a few microseconds: latency decides. One lane per 32-byte nibble group (two sub-blocks)
-// straight from global memory, every weight byte of a warp requested before the previous kernel is
-// awaited; the token rows are laid out in shared memory once per CTA so that a lane's 64 codes, two
-// sums and scale are five conflict-free reads (a group is 80 bytes, a block 320) and serve R rows.
-// The integer partial sums of a super-block meet exactly by shuffle over its four lanes, its fp32
-// term is formed once, and the terms of a row are added in the order of the tile kernels' shuffle
-// tree. Up to three matrices of the same k in one launch, their rows one after another.
+// A launch of a few microseconds: latency decides. A warp owns sixteen rows and every eighth block
+// column (rows of fewer than eight blocks: the warps of a CTA take several row groups); each lane
+// loads its share of the weight bytes straight into MMA fragment order - the order of k inside a
+// sub-block is free as long as both operands use it - before the previous kernel is awaited, then its
+// share of that block of the token rows, and ten int8 MMAs leave the exact integer sums of sixteen
+// rows x eight tokens without a shuffle. The fp32 terms of a row's blocks meet in shared memory and
+// are added in the order of the tile kernels' shuffle tree. dp4a takes 2.2 cycles a warp and
+// scheduler for 128 products, this MMA 8 for 4096, a shuffle 4. One token fills an eighth of the MMA
+// and goes the dp4a way below (2048 -> 4096 + 512 + 512: 3.1 us against 4.0), several tokens this one
+// (2048 -> 4096 at 2 / 4 / 8 rows: 3.1 / 3.3 / 3.4 us, dp4a 3.8 / 5.2 / 8.9). Up to three matrices of the
+// same k in one launch, their rows one after another.
 constexpr int kDirectWarps = 8;
-constexpr int kDirectGroup = 80, kDirectBlock = 4 * kDirectGroup;
 
 struct DirectArgs {
   const unsigned char* w[3];
@@ -333,152 +336,203 @@ struct DirectArgs {
   const unsigned char* xq;
   int nb, n_tokens;
   uint16_t* res;                        // one token, fp16 out: residual row updated in place
+  __device__ __forceinline__ int matrix_of(int row) const { return row >= rows_cum[0] ? (row >= rows_cum[1] ? 2 : 1) : 0; }
+  __device__ __forceinline__ int first_row(int m) const { return m == 0 ? 0 : (m == 1 ? rows_cum[0] : rows_cum[1]); }
 };
 
-// R row steps per warp (a step is 32 / lanes-per-row rows), NI groups of a row per lane
-template <int TT, int R, int NI, bool F16>
+// NI: block columns per warp (1 for rows of up to eight blocks)
+template <int NI, bool F16>
 __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const DirectArgs a) {
-  extern __shared__ __align__(16) unsigned char xs[];
+  __shared__ float red[kDirectWarps][8][16];                // [warp][token][row]
   const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int lpr = NI > 1 ? 32 : min(nb * 4, 32);           // lanes per row (a power of two >= 4)
-  const int lr = lane & (lpr - 1), g = lr & 3, blk0 = lr >> 2;
-  const int rows_step = 32 / lpr, total = a.rows_cum[2];
-  const int row0 = (blockIdx.x * kDirectWarps + warp) * R * rows_step + lane / lpr;
-  uint4 hdr[R][NI], q0[R][NI], q1[R][NI];
+  const int gid = lane >> 2, tig = lane & 3;
+  const int wpg = NI > 1 ? kDirectWarps : min(nb, kDirectWarps);        // warps per row group
+  const int groups = kDirectWarps / wpg, total = a.rows_cum[2];
+  const int cta_row0 = blockIdx.x * groups * 16;
+  const int row0 = cta_row0 + warp / wpg * 16, blk0 = warp & (wpg - 1);
+  uint4 hdr[2][NI];
+  uint2 q[2][NI][4];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int row = min(row0 + r * rows_step, total - 1);  // every lane runs the same loops
-    const int m = row >= a.rows_cum[0] ? (row >= a.rows_cum[1] ? 2 : 1) : 0;
-    const unsigned char* wm = m == 0 ? a.w[0] : (m == 1 ? a.w[1] : a.w[2]);
-    const int lrow = row - (m == 0 ? 0 : (m == 1 ? a.rows_cum[0] : a.rows_cum[1]));
-    const unsigned char* wb = wm + (static_cast<size_t>(lrow) * nb + blk0) * kW4;
+  for (int h = 0; h < 2; ++h) {
+    const int row = min(row0 + gid + 8 * h, total - 1), m = a.matrix_of(row);
+    const unsigned char* wb = (m == 0 ? a.w[0] : (m == 1 ? a.w[1] : a.w[2])) +
+                              (static_cast<size_t>(row - a.first_row(m)) * nb + blk0) * kW4;
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
-      hdr[r][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
-      q0[r][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 16 + 32 * g));
-      q1[r][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 32 + 32 * g));
+      hdr[h][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+#pragma unroll
+      for (int g = 0; g < 4; ++g) q[h][i][g] = __ldg(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
     }
   }
   pdl_wait();
   pdl_launch_dependents();
-  for (int b = warp; b < a.n_tokens * nb; b += 4 * kDirectWarps) {      // four blocks' words requested together
-    uint32_t v[4][3];
+  constexpr int NA = NI > 2 ? 2 : 1;        // rows of 32 blocks: (t0 + t2) + (t1 + t3), the shuffle tree's order
+  float acc[NA][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int bb = b + u * kDirectWarps;
-      if (bb < a.n_tokens * nb) {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(a.xq + static_cast<size_t>(bb) * kX8) + lane;
-        v[u][0] = __ldg(src);
-        v[u][1] = __ldg(src + 32);
-        if (lane < 5) v[u][2] = __ldg(src + 64);
-      }
-    }
+  for (int c = 0; c < NA; ++c)
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int bb = b + u * kDirectWarps;
-      if (bb < a.n_tokens * nb) {
-        unsigned char* dst = xs + bb * kDirectBlock;       // word 0: scale; 1..64: codes; 65..68: sums
-        auto put = [&](int w, uint32_t x) { *reinterpret_cast<uint32_t*>(dst + (w >> 4) * kDirectGroup + (w & 15) * 4) = x; };
-        if (lane > 0) put(lane - 1, v[u][0]);
-        put(lane + 31, v[u][1]);
-        if (lane == 0) put(63, v[u][2]);
-        else if (lane < 5) *reinterpret_cast<uint32_t*>(dst + (lane - 1) * kDirectGroup + 64) = v[u][2];
-        const uint32_t d = __shfl_sync(0xFFFFFFFFu, v[u][0], 0);
-        if (lane < 4) *reinterpret_cast<uint32_t*>(dst + lane * kDirectGroup + 68) = d;
-      }
-    }
-  }
-  __syncthreads();
-
-  constexpr int NA = NI > 1 ? 2 : 1;        // rows of 32 blocks: (t0 + t2) + (t1 + t3), the shuffle tree's order
-  float acc[R][TT][NA];
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-#pragma unroll
-    for (int t = 0; t < TT; ++t)
-#pragma unroll
-      for (int c = 0; c < NA; ++c) acc[r][t][c] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[c][j] = 0.f;
+  const int zero[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
+    // token gid's codes in the weights' order of k, its sums 4 tig .. 4 tig + 3, the scales of tokens 2 tig, 2 tig + 1
+    uint32_t b[8][2] = {};
+    uint32_t s01 = 0u, s23 = 0u;
+    float xd[2] = {0.f, 0.f};
+    const int blk = blk0 + 8 * i;
+    if (gid < a.n_tokens) {
+      const uint32_t* xb = reinterpret_cast<const uint32_t*>(a.xq + (static_cast<size_t>(gid) * nb + blk) * kX8);
 #pragma unroll
-    for (int t = 0; t < TT; ++t) {
-      if (t < a.n_tokens) {
-        const unsigned char* xb = xs + (t * nb + blk0 + 8 * i) * kDirectBlock + g * kDirectGroup;
-        const uint4 x0 = *reinterpret_cast<const uint4*>(xb), x1 = *reinterpret_cast<const uint4*>(xb + 16);
-        const uint4 x2 = *reinterpret_cast<const uint4*>(xb + 32), x3 = *reinterpret_cast<const uint4*>(xb + 48);
-        const uint2 sd = *reinterpret_cast<const uint2*>(xb + 64);
-        const int bs_lo = static_cast<int16_t>(sd.x & 0xFFFFu), bs_hi = static_cast<int16_t>(sd.x >> 16);
-        const float xd = __uint_as_float(sd.y);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const Scales6 s6 = unpack_scales6(hdr[r][i].y, hdr[r][i].z, hdr[r][i].w);
-          const uint32_t scw = (g < 2 ? s6.sc[0] : s6.sc[1]) >> (16 * (g & 1)), mnw = (g < 2 ? s6.mn[0] : s6.mn[1]) >> (16 * (g & 1));
-          const uint32_t raw[8] = {q0[r][i].x, q0[r][i].y, q0[r][i].z, q0[r][i].w, q1[r][i].x, q1[r][i].y, q1[r][i].z, q1[r][i].w};
-          uint32_t lo[8], hi[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            lo[j] = raw[j] & 0x0F0F0F0Fu;
-            hi[j] = (raw[j] >> 4) & 0x0F0F0F0Fu;
-          }
-          int isum = static_cast<int>(scw & 0xFF) * dot8(lo, x0, x1) + static_cast<int>((scw >> 8) & 0xFF) * dot8(hi, x2, x3);
-          int msum = static_cast<int>(mnw & 0xFF) * bs_lo + static_cast<int>((mnw >> 8) & 0xFF) * bs_hi;
-          isum += __shfl_xor_sync(0xFFFFFFFFu, isum, 1);
-          msum += __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
-          isum += __shfl_xor_sync(0xFFFFFFFFu, isum, 2);
-          msum += __shfl_xor_sync(0xFFFFFFFFu, msum, 2);
-          const float d = h2f(static_cast<uint16_t>(hdr[r][i].x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr[r][i].x >> 16));
-          acc[r][t][i % NA] += xd * (d * static_cast<float>(isum) - dmin * static_cast<float>(msum));
-        }
+      for (int sb = 0; sb < 8; ++sb) {
+        b[sb][0] = __ldg(xb + 1 + 8 * sb + 2 * tig);
+        b[sb][1] = __ldg(xb + 2 + 8 * sb + 2 * tig);
       }
+      if (tig < 2) {
+        s01 = __ldg(xb + 65 + 2 * tig);
+        s23 = __ldg(xb + 66 + 2 * tig);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (2 * tig + j < a.n_tokens) xd[j] = __ldg(reinterpret_cast<const float*>(a.xq + (static_cast<size_t>(2 * tig + j) * nb + blk) * kX8));
+    const Scales6 sl = unpack_scales6(hdr[0][i].y, hdr[0][i].z, hdr[0][i].w), sh = unpack_scales6(hdr[1][i].y, hdr[1][i].z, hdr[1][i].w);
+    int isum[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const uint32_t raw[4] = {q[0][i][g].x, q[1][i][g].x, q[0][i][g].y, q[1][i][g].y};
+      uint32_t lo[4], hi[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        lo[j] = raw[j] & 0x0F0F0F0Fu;
+        hi[j] = raw[j] & 0xF0F0F0F0u;        // 16 q: the even sub-block's scale is taken 16-fold, d a sixteenth (exact)
+      }
+      const int shift = 16 * (g & 1);
+      const int sc0_lo = ((sl.sc[g >> 1] >> shift) & 0xFF) << 4, sc1_lo = (sl.sc[g >> 1] >> (shift + 8)) & 0xFF;
+      const int sc0_hi = ((sh.sc[g >> 1] >> shift) & 0xFF) << 4, sc1_hi = (sh.sc[g >> 1] >> (shift + 8)) & 0xFF;
+      int c0[4], c1[4];
+      mma_u8s8(c0, lo, b[2 * g][0], b[2 * g][1], zero);
+      mma_u8s8(c1, hi, b[2 * g + 1][0], b[2 * g + 1][1], zero);
+      isum[0] += sc0_lo * c0[0] + sc1_lo * c1[0];
+      isum[1] += sc0_lo * c0[1] + sc1_lo * c1[1];
+      isum[2] += sc0_hi * c0[2] + sc1_hi * c1[2];
+      isum[3] += sc0_hi * c0[3] + sc1_hi * c1[3];
+    }
+    // min term: the eight min bytes of a row are k = 0..7, the sums split as 128 * hi + lo
+    const uint32_t ma[4] = {tig == 0 ? sl.mn[0] : (tig == 1 ? sl.mn[1] : 0u), tig == 0 ? sh.mn[0] : (tig == 1 ? sh.mn[1] : 0u), 0u, 0u};
+    int dl[4], dh[4];
+    mma_u8s8(dl, ma, __byte_perm(s01 & 0x007F007Fu, s23 & 0x007F007Fu, 0x6420), 0u, zero);
+    mma_u8s8(dh, ma, __byte_perm((s01 >> 7) & 0x00FF00FFu, (s23 >> 7) & 0x00FF00FFu, 0x6420), 0u, zero);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint4& hd = hdr[j >> 1][i];
+      const float d = 0.0625f * h2f(static_cast<uint16_t>(hd.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hd.x >> 16));
+      acc[i % NA][j] += xd[j & 1] * (d * static_cast<float>(isum[j]) - dmin * static_cast<float>(dl[j] + 128 * dh[j]));
     }
   }
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int row = row0 + r * rows_step;
-    const int m = row >= a.rows_cum[0] ? (row >= a.rows_cum[1] ? 2 : 1) : 0;
-    const int lo_row = m == 0 ? 0 : (m == 1 ? a.rows_cum[0] : a.rows_cum[1]);
-    const int m_rows = (m == 0 ? a.rows_cum[0] : (m == 1 ? a.rows_cum[1] : a.rows_cum[2])) - lo_row;
-    void* y = m == 0 ? a.y[0] : (m == 1 ? a.y[1] : a.y[2]);
+  for (int j = 0; j < 4; ++j) {
+    float v = acc[0][j];
+    if constexpr (NA > 1) v += acc[1][j];
+    red[warp][2 * tig + (j & 1)][gid + 8 * (j >> 1)] = v;
+  }
+  __syncthreads();
+  for (int o = threadIdx.x; o < groups * 16 * a.n_tokens; o += kDirectWarps * 32) {
+    const int r = o & 15, t = (o >> 4) % a.n_tokens, grp = (o >> 4) / a.n_tokens;
+    const int row = cta_row0 + grp * 16 + r;
+    if (row >= total) continue;
+    float v[kDirectWarps];
 #pragma unroll
-    for (int t = 0; t < TT; ++t) {
-      if (t >= a.n_tokens) break;
-      float v = acc[r][t][0];
-      if constexpr (NA > 1) v += acc[r][t][1];
-      for (int off = lpr >> 1; off >= 4; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, off);
-      if (lr != 0 || row >= total) continue;
-      if constexpr (F16 && TT == 1) {
-        if (a.res != nullptr) {
-          store_out_resadd(reinterpret_cast<uint16_t*>(y), a.res, static_cast<size_t>(row - lo_row), v);
-          continue;
-        }
-      }
-      store_out<F16>(y, static_cast<size_t>(t) * m_rows + row - lo_row, v);
+    for (int w = 0; w < kDirectWarps; ++w) v[w] = w < wpg ? red[grp * wpg + w][t][r] : 0.f;
+    if (wpg == 8) {
+#pragma unroll
+      for (int w = 0; w < 4; ++w) v[w] += v[w + 4];
     }
+    if (wpg >= 4) { v[0] += v[2]; v[1] += v[3]; }
+    if (wpg >= 2) v[0] += v[1];
+    const int m = a.matrix_of(row), first = a.first_row(m);
+    void* y = m == 0 ? a.y[0] : (m == 1 ? a.y[1] : a.y[2]);
+    const int m_rows = (m == 0 ? a.rows_cum[0] : (m == 1 ? a.rows_cum[1] : a.rows_cum[2])) - first;
+    store_out<F16>(y, static_cast<size_t>(t) * m_rows + row - first, v[0]);
   }
 }
 
-template <int TT, int R, int NI, bool F16>
-int launch_direct_as(const DirectArgs& a, cudaStream_t stream) {
-  const size_t smem = static_cast<size_t>(a.n_tokens) * a.nb * kDirectBlock;
-  if (smem > 48 * 1024 && !opt_in_smem<gemv_direct_kernel<TT, R, NI, F16>>(8 * 32 * kDirectBlock)) return kErrLaunch;
-  const int rows_cta = kDirectWarps * R * (NI > 1 ? 1 : std::max(1, 8 / a.nb));
-  return launch_pdl(gemv_direct_kernel<TT, R, NI, F16>, dim3((a.rows_cum[2] + rows_cta - 1) / rows_cta), kDirectWarps * 32, smem,
-                    stream, a);
-}
-template <int TT, bool F16>
-int launch_direct_tt(const DirectArgs& a, cudaStream_t stream) {
-  // rows per warp: as many as registers hold while every SM still gets eight warps
-  const long long steps = a.nb >= 8 ? a.rows_cum[2] : (a.rows_cum[2] + 8 / a.nb - 1) / (8 / a.nb);
-  const long long per_sm = 148LL * kDirectWarps;
-  if (a.nb <= 8) {
-    if (steps >= 4 * per_sm) return launch_direct_as<TT, 4, 1, F16>(a, stream);
-    if (steps >= 2 * per_sm) return launch_direct_as<TT, 2, 1, F16>(a, stream);
-    return launch_direct_as<TT, 1, 1, F16>(a, stream);
+// One token: a warp per row (rows of fewer than eight blocks: several), one lane per 32-byte nibble group,
+// the token laid out in shared memory once per CTA so that a lane's 64 codes, two sums and scale are five
+// conflict-free reads (a group is 80 bytes, a block 320). The integer partial sums of a super-block meet
+// exactly by shuffle over its four lanes, the blocks' terms in the tile kernels' shuffle tree.
+constexpr int kDirectGroup = 80, kDirectBlock = 4 * kDirectGroup;
+
+template <int NI, bool F16>
+__global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct1_kernel(const DirectArgs a) {
+  __shared__ __align__(16) unsigned char xs[32 * kDirectBlock];
+  const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lpr = NI > 1 ? 32 : min(nb * 4, 32);           // lanes per row (a power of two >= 4)
+  const int lr = lane & (lpr - 1), g = lr & 3, blk0 = lr >> 2;
+  const int total = a.rows_cum[2];
+  const int row_raw = (blockIdx.x * kDirectWarps + warp) * (32 / lpr) + lane / lpr;
+  const int row = min(row_raw, total - 1), m = a.matrix_of(row), first = a.first_row(m);    // every lane runs the same loops
+  const unsigned char* wb = (m == 0 ? a.w[0] : (m == 1 ? a.w[1] : a.w[2])) + (static_cast<size_t>(row - first) * nb + blk0) * kW4;
+  uint4 hdr[NI], q0[NI], q1[NI];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    hdr[i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+    q0[i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 16 + 32 * g));
+    q1[i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 32 + 32 * g));
   }
-  if (a.nb == 16)
-    return steps >= 2 * per_sm ? launch_direct_as<TT, 2, 2, F16>(a, stream) : launch_direct_as<TT, 1, 2, F16>(a, stream);
-  return launch_direct_as<TT, 1, 4, F16>(a, stream);
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int b = warp; b < nb; b += kDirectWarps) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(a.xq + static_cast<size_t>(b) * kX8) + lane;
+    const uint32_t v0 = __ldg(src), v1 = __ldg(src + 32), v2 = lane < 5 ? __ldg(src + 64) : 0u;
+    unsigned char* dst = xs + b * kDirectBlock;            // word 0: scale; 1..64: codes; 65..68: sums
+    auto put = [&](int w, uint32_t x) { *reinterpret_cast<uint32_t*>(dst + (w >> 4) * kDirectGroup + (w & 15) * 4) = x; };
+    if (lane > 0) put(lane - 1, v0);
+    put(lane + 31, v1);
+    if (lane == 0) put(63, v2);
+    else if (lane < 5) *reinterpret_cast<uint32_t*>(dst + (lane - 1) * kDirectGroup + 64) = v2;
+    const uint32_t d = __shfl_sync(0xFFFFFFFFu, v0, 0);
+    if (lane < 4) *reinterpret_cast<uint32_t*>(dst + lane * kDirectGroup + 68) = d;
+  }
+  __syncthreads();
+  float acc[2] = {0.f, 0.f};                // rows of 32 blocks: (t0 + t2) + (t1 + t3), the shuffle tree's order
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const unsigned char* xb = xs + (blk0 + 8 * i) * kDirectBlock + g * kDirectGroup;
+    const uint4 x0 = *reinterpret_cast<const uint4*>(xb), x1 = *reinterpret_cast<const uint4*>(xb + 16);
+    const uint4 x2 = *reinterpret_cast<const uint4*>(xb + 32), x3 = *reinterpret_cast<const uint4*>(xb + 48);
+    const uint2 sd = *reinterpret_cast<const uint2*>(xb + 64);
+    const Scales6 s6 = unpack_scales6(hdr[i].y, hdr[i].z, hdr[i].w);
+    const uint32_t scw = (g < 2 ? s6.sc[0] : s6.sc[1]) >> (16 * (g & 1)), mnw = (g < 2 ? s6.mn[0] : s6.mn[1]) >> (16 * (g & 1));
+    const uint32_t raw[8] = {q0[i].x, q0[i].y, q0[i].z, q0[i].w, q1[i].x, q1[i].y, q1[i].z, q1[i].w};
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      lo[j] = raw[j] & 0x0F0F0F0Fu;
+      hi[j] = (raw[j] >> 4) & 0x0F0F0F0Fu;
+    }
+    int isum = static_cast<int>(scw & 0xFF) * dot8(lo, x0, x1) + static_cast<int>((scw >> 8) & 0xFF) * dot8(hi, x2, x3);
+    int msum = static_cast<int>(mnw & 0xFF) * static_cast<int16_t>(sd.x & 0xFFFFu) + static_cast<int>((mnw >> 8) & 0xFF) * static_cast<int16_t>(sd.x >> 16);
+    isum += __shfl_xor_sync(0xFFFFFFFFu, isum, 1);
+    msum += __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
+    isum += __shfl_xor_sync(0xFFFFFFFFu, isum, 2);
+    msum += __shfl_xor_sync(0xFFFFFFFFu, msum, 2);
+    const float d = h2f(static_cast<uint16_t>(hdr[i].x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr[i].x >> 16));
+    acc[i & 1] += __uint_as_float(sd.y) * (d * static_cast<float>(isum) - dmin * static_cast<float>(msum));
+  }
+  float v = acc[0];
+  if constexpr (NI > 1) v += acc[1];
+  for (int off = lpr >> 1; off >= 4; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, off);
+  if (lr != 0 || row_raw >= total) return;
+  void* y = m == 0 ? a.y[0] : (m == 1 ? a.y[1] : a.y[2]);
+  if constexpr (F16) {
+    if (a.res != nullptr) {
+      store_out_resadd(reinterpret_cast<uint16_t*>(y), a.res, static_cast<size_t>(row - first), v);
+      return;
+    }
+  }
+  store_out<F16>(y, static_cast<size_t>(row - first), v);
 }
+
 // One to eight token rows, rows of a power of two of blocks up to 32, 16-byte aligned matrices.
 inline bool direct_fits(const DirectArgs& a) {
   if (a.n_tokens < 1 || a.n_tokens > 8 || a.nb > 32 || (a.nb & (a.nb - 1)) != 0) return false;
@@ -488,10 +542,19 @@ inline bool direct_fits(const DirectArgs& a) {
 }
 template <bool F16>
 int launch_direct(const DirectArgs& a, cudaStream_t stream) {
-  if (a.n_tokens == 1) return launch_direct_tt<1, F16>(a, stream);
-  if (a.n_tokens == 2) return launch_direct_tt<2, F16>(a, stream);
-  if (a.n_tokens <= 4) return launch_direct_tt<4, F16>(a, stream);
-  return launch_direct_tt<8, F16>(a, stream);
+  const int threads = kDirectWarps * 32;
+  if (a.n_tokens == 1) {
+    const int rows_cta = kDirectWarps * std::max(1, 8 / a.nb);
+    const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
+    if (a.nb <= 8) return launch_pdl(gemv_direct1_kernel<1, F16>, grid, threads, 0, stream, a);
+    if (a.nb == 16) return launch_pdl(gemv_direct1_kernel<2, F16>, grid, threads, 0, stream, a);
+    return launch_pdl(gemv_direct1_kernel<4, F16>, grid, threads, 0, stream, a);
+  }
+  const int rows_cta = 16 * std::max(1, kDirectWarps / a.nb);
+  const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
+  if (a.nb <= 8) return launch_pdl(gemv_direct_kernel<1, F16>, grid, threads, 0, stream, a);
+  if (a.nb == 16) return launch_pdl(gemv_direct_kernel<2, F16>, grid, threads, 0, stream, a);
+  return launch_pdl(gemv_direct_kernel<4, F16>, grid, threads, 0, stream, a);
 }
 
 // tokens per CTA of the dense multi-token kernels (walked in sub-tiles of 8)
