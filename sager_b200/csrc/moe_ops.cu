@@ -18,19 +18,36 @@ __device__ __forceinline__ bool aligned16(const void* p) {
 // Every CTA reads the whole route list, counts it per expert and part of the list (shared-memory
 // atomics) and builds the prefixes for itself, so nothing is exchanged; each of its warps then walks
 // one part of the list for one expert of its own and hands the slots out by ballot. The slots inside
-// an expert are in ascending (row, kk) order whatever the size. Bound by the latency of the phases.
-// One CTA took 24 us for 16,384 routes over 256 experts (atomic fill) and 35 us for 768 (a thread per
-// expert walking the list); counting and ranking by match_any in one CTA 48 and 9 us.
+// an expert are in ascending (row, kk) order whatever the size. Bound by the latency of the phases:
+// 12 / 7 / 4 us for 16,384 / 6,216 / 768 routes over 256 experts. One CTA took 20 / 9.5 / 33 us (atomic fill
+// above 4096 routes, below a thread per expert walking the list); counting and ranking by match_any in
+// one CTA 48 us for the largest.
+// i / d for i below 2^31 by a multiplication (a division instruction sequence per route was half the time)
+struct FastDiv {
+  unsigned mul;
+  int shift;                               // < 0: d is 1
+  explicit FastDiv(unsigned d) : mul(0), shift(-1) {
+    if (d <= 1) return;
+    int l = 0;
+    while ((1u << l) < d && l < 31) ++l;
+    shift = l - 1;
+    mul = static_cast<unsigned>(((1ull << (31 + l)) + d - 1) / d);
+  }
+  __device__ __forceinline__ int operator()(int i) const {
+    return shift < 0 ? i : static_cast<int>(__umulhi(static_cast<unsigned>(i), mul) >> shift);
+  }
+};
+
 constexpr int kScanThreads = 512, kScanWarps = kScanThreads / 32;
-constexpr int kScanParts = 4;              // of the list, while [parts][n_expert] counters stay small
-constexpr int kScanPartExperts = 2048;
+constexpr int kScanParts = 8;              // of the list, while [parts][n_expert] counters stay small
+constexpr int kScanPartExperts = 1024;
 constexpr int kScanStaged = 64 * 1024;     // routes whose ids are kept in shared memory, two bytes each
 
 __global__ void __launch_bounds__(kScanThreads)
 dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, int* __restrict__ gslot,
                      int* __restrict__ grows, int* __restrict__ off, int* __restrict__ toff,
                      int* __restrict__ meta, int* __restrict__ mail_n, int n_rows, int k,
-                     int n_expert, int tok_per, int parts, int staged) {
+                     int n_expert, int tok_per, int parts, int per, FastDiv by_k, FastDiv by_per, int staged) {
   extern __shared__ __align__(16) int cnt[];             // [parts][n_expert] counts, then first slots; ids after them
   uint16_t* ids = reinterpret_cast<uint16_t*>(cnt + static_cast<size_t>(parts) * n_expert);
   __shared__ int bad_sh;
@@ -40,13 +57,11 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
   pdl_launch_dependents();
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   const int total = n_rows * k;
-  const int per = ((total + parts - 1) / parts + 31) & ~31;           // routes per part
   if (tid == 0) bad_sh = carry[0] = carry[1] = 0;
   for (int e = tid; e < parts * n_expert; e += kScanThreads) cnt[e] = 0;
   __syncthreads();
   auto id_of = [&](int i) {
-    const int r = i / k;
-    const int e = __ldg(idx + static_cast<size_t>(r) * (k + 1) + (i - r * k));
+    const int e = __ldg(idx + i + by_k(i));                           // rows of k + 1
     return e >= 0 && e < n_expert ? e : 0xFFFF;
   };
   for (int b = tid; b < total; b += 8 * kScanThreads) {
@@ -59,10 +74,10 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
       if (e8[q] < 0) continue;
       if (staged) ids[i] = static_cast<uint16_t>(e8[q]);
       if (e8[q] != 0xFFFF) {
-        atomicAdd(cnt + static_cast<size_t>(i / per) * n_expert + e8[q], 1);
+        atomicAdd(cnt + static_cast<size_t>(by_per(i)) * n_expert + e8[q], 1);
       } else if (blockIdx.x == 0) {
         // a corrupt id silences the whole row, shared-expert slot included
-        float* wr = weight + static_cast<size_t>(i / k) * (k + 1);
+        float* wr = weight + static_cast<size_t>(by_k(i)) * (k + 1);
         for (int j = 0; j <= k; ++j) wr[j] = 0.f;
         gslot[i] = -1;
         atomicAdd(&bad_sh, 1);
@@ -133,7 +148,7 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
       if (e8[q] == e) {
         const int i = b + 32 * q + lane, slot = pos + __popc(hit & ((1u << lane) - 1u));
         gslot[i] = slot;
-        grows[slot] = i / k;
+        grows[slot] = by_k(i);
       }
       pos += __popc(hit);
     }
@@ -347,11 +362,11 @@ SGR_API int sgr_moe_dispatch_scan(const int* idx, float* weight, int* gslot, int
   if (static_cast<long long>(n_rows) * k > 0x7FFFFF00) return kErrArg;
   if (n_expert > 12 * 1024) return kErrUnsupported;
   const int parts = n_expert <= kScanPartExperts ? kScanParts : 1, per_cta = kScanWarps / parts;
-  const int staged = n_rows * k <= kScanStaged;
+  const int staged = n_rows * k <= kScanStaged, per = ((n_rows * k + parts - 1) / parts + 31) / 32 * 32;       // routes per part
   const size_t smem = static_cast<size_t>(parts) * n_expert * sizeof(int) + (staged ? static_cast<size_t>(n_rows) * k * 2 : 0);
   if (smem > 40 * 1024 && !opt_in_smem<dispatch_scan_kernel>(200 * 1024)) return kErrLaunch;
   return launch_pdl(dispatch_scan_kernel, dim3((n_expert + per_cta - 1) / per_cta), kScanThreads, smem, as_stream(stream), idx, weight,
-                    gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, parts, staged);
+                    gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, parts, per, FastDiv(k), FastDiv(per), staged);
 }
 
 SGR_API int sgr_gather_rows_q8(void* dst, const void* src, const int* src_rows, int n_rows,
