@@ -291,12 +291,11 @@ int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStre
 // (larger value first, lower index first among equals) and an entry that never qualifies is the word
 // 0. A run is 64 words in descending order held by one warp; the 64 largest of two runs are a
 // lane-wise maximum against the reversed partner plus a six-step bitonic merge, all in shuffles.
-// Phase 1: a CTA of 32 warps per 2048-value segment, each warp sorts 64 values, five rounds of
-// pairwise selection leave the segment's best 64. Phase 2: one CTA does the same over the segments'
-// candidate lists (up to 128 segments). Values are read back from the logits by index, so what is
-// returned are the caller's own bits. (Selection by repeated arg-max - a warp per segment, k rounds
-// of two warp reductions and a rescan - is kept for more than 128 segments; it took 110 us for
-// 151,936 logits and k = 40, as slow as the reference's kernels.)
+// Phase 1: a CTA of 32 warps per 2048-value segment; phase 2: one CTA over the segments' candidate lists (up
+// to 128 segments). Both pick by threshold (topk_by_threshold) and fall back to the merges: each warp sorts 64
+// values, rounds of pairwise selection leave the best 64. Values are the caller's own bits. (Selection by
+// repeated arg-max - a warp per segment, k rounds of two warp reductions and a rescan - is kept for more than
+// 128 segments; it took 110 us for 151,936 logits and k = 40, the merges 14.6 us, the threshold 11.1 us.)
 constexpr float kTopkNone = -3.4e38f;
 constexpr int kTopkSeg = 2048;               // the reference's segment size: the caller's scratch is sized by it
 constexpr int kTopkPerLane = kTopkSeg / 32;
@@ -396,10 +395,73 @@ __device__ __forceinline__ void run_select(unsigned long long (&a)[2], const uns
   run_merge_desc(a, lane);
 }
 
-// grid: one CTA of 32 warps per segment. Every warp sorts 64 values, then five rounds halve the runs.
+// the value of a word; zeros are read back (the word does not know the sign of a zero)
+__device__ __forceinline__ float topk_value(unsigned long long w, const float* __restrict__ logits) {
+  if (w == 0ull) return kTopkNone;
+  const int key = static_cast<int>(static_cast<unsigned>(w >> 32) ^ 0x80000000u);
+  return key == 0 ? __ldg(logits + static_cast<int>(~static_cast<unsigned>(w))) : __int_as_float(key ^ ((key >> 31) & 0x7FFFFFFF));
+}
+
+// Selection by threshold (all 1024 threads): the k-th largest of a small pool of the words' keys bounds the k-th
+// largest of all from below, so only the words with keys at or above it can be picked; they are collected and each
+// counts how many are larger than itself, which is its place. Fills best[0..k) (0: nothing) and returns true, or false
+// when the pool bounds them badly and more than kTopkCand words are left (long runs of equal or nearly sorted values):
+// the caller then merges sorted runs, a dozen dependent rounds of shuffles and barriers.
+constexpr int kTopkCand = 256, kTopkPool = 192;
+struct TopkShared {
+  unsigned pool[kTopkPool];
+  unsigned threshold;
+  int count;
+  unsigned long long cand[kTopkCand];
+  unsigned long long best[64];
+};
+template <int PER>
+__device__ __forceinline__ bool topk_by_threshold(TopkShared& sh, const unsigned long long (&x)[PER], int n_pool, int k) {
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) sh.count = 0;
+  __syncthreads();                                 // the pool is complete
+  if (tid < n_pool) {
+    const unsigned mine = sh.pool[tid];
+    int above = 0;
+#pragma unroll 8
+    for (int i = 0; i < n_pool; ++i) {
+      const unsigned o = sh.pool[i];
+      above += (o > mine || (o == mine && i < tid)) ? 1 : 0;
+    }
+    if (above == k - 1) sh.threshold = mine;
+  }
+  __syncthreads();
+  const unsigned threshold = sh.threshold;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const bool in = x[j] != 0ull && static_cast<unsigned>(x[j] >> 32) >= threshold;
+    const unsigned who = __ballot_sync(0xFFFFFFFFu, in);
+    if (who == 0u) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&sh.count, __popc(who));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(who & ((1u << lane) - 1u));
+    if (in && at < kTopkCand) sh.cand[at] = x[j];
+  }
+  __syncthreads();
+  const int n = sh.count;
+  if (n > kTopkCand) return false;
+  if (tid < n) {
+    const unsigned long long mine = sh.cand[tid];
+    int above = 0;
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) above += sh.cand[i] > mine ? 1 : 0;
+    if (above < k) sh.best[above] = mine;
+  }
+  if (tid >= 512 && tid - 512 < k && tid - 512 >= n) sh.best[tid - 512] = 0ull;
+  __syncthreads();
+  return true;
+}
+
+// grid: one CTA of 32 warps per segment, 64 values a warp. The pool is the maximum of every 32 values.
 __global__ void __launch_bounds__(1024) topk_seg_sort_kernel(const float* __restrict__ logits, float* __restrict__ seg_v,
                                                             int* __restrict__ seg_i, int n, int k) {
   __shared__ unsigned long long runs[32][64];
+  __shared__ TopkShared sh;
   pdl_wait();
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -410,75 +472,94 @@ __global__ void __launch_bounds__(1024) topk_seg_sort_kernel(const float* __rest
     const int gi = base + lane + 32 * j;
     x[j] = gi < n ? topk_word(__ldg(logits + gi), gi) : 0ull;
   }
-  run_sort_desc(x, lane);
-  runs[warp][lane] = x[0];
-  runs[warp][lane + 32] = x[1];
-  for (int r = 0; r < 5; ++r) {
-    __syncthreads();
-    if (warp < (16 >> r)) {
-      const int sa = warp << (r + 1), sb = sa + (1 << r);
-      unsigned long long a[2] = {runs[sa][lane], runs[sa][lane + 32]};
-      const unsigned long long b[2] = {runs[sb][lane], runs[sb][lane + 32]};
-      run_select(a, b, lane);
-      runs[sa][lane] = a[0];
-      runs[sa][lane + 32] = a[1];
-    }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const unsigned top = __reduce_max_sync(0xFFFFFFFFu, static_cast<unsigned>(x[j] >> 32));
+    if (lane == 0) sh.pool[2 * warp + j] = top;
   }
-  __syncthreads();
+  const unsigned long long* best = sh.best;
+  if (!topk_by_threshold<2>(sh, x, 64, k)) {
+    run_sort_desc(x, lane);
+    runs[warp][lane] = x[0];
+    runs[warp][lane + 32] = x[1];
+    for (int r = 0; r < 5; ++r) {
+      __syncthreads();
+      if (warp < (16 >> r)) {
+        const int sa = warp << (r + 1), sb = sa + (1 << r);
+        unsigned long long a[2] = {runs[sa][lane], runs[sa][lane + 32]};
+        const unsigned long long b[2] = {runs[sb][lane], runs[sb][lane + 32]};
+        run_select(a, b, lane);
+        runs[sa][lane] = a[0];
+        runs[sa][lane + 32] = a[1];
+      }
+    }
+    __syncthreads();
+    best = runs[0];
+  }
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
-    const unsigned long long w = runs[0][j];
-    const int gi = w != 0ull ? static_cast<int>(~static_cast<unsigned>(w)) : -1;
-    seg_i[static_cast<size_t>(blockIdx.x) * k + j] = gi;
-    seg_v[static_cast<size_t>(blockIdx.x) * k + j] = gi >= 0 ? __ldg(logits + gi) : kTopkNone;
+    const unsigned long long w = best[j];
+    seg_i[static_cast<size_t>(blockIdx.x) * k + j] = w != 0ull ? static_cast<int>(~static_cast<unsigned>(w)) : -1;
+    seg_v[static_cast<size_t>(blockIdx.x) * k + j] = topk_value(w, logits);
   }
 }
 
 // One CTA merges the candidates of up to 128 segments: a segment's k candidates are a descending run
-// already. The first round reads pairs of runs from global memory, six more halve the 64 that remain.
+// already. The pool is the first few of every run, at least k in all.
 __global__ void __launch_bounds__(1024) topk_merge_sort_kernel(const float* __restrict__ logits,
                                                               const float* __restrict__ seg_v,
                                                               const int* __restrict__ seg_i, float* __restrict__ out_v,
                                                               int* __restrict__ out_i, int nseg, int k) {
   __shared__ unsigned long long runs[64][64];
+  __shared__ TopkShared sh;
   pdl_wait();
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  auto load_run = [&](int seg, unsigned long long (&x)[2]) {
+  unsigned long long x[8];                         // runs warp, warp + 32, ... : elements lane, lane + 32
+  float v[8];
+  int gi[8];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int e = lane + 32 * j;
-      x[j] = 0ull;
-      if (seg < nseg && e < k) {
-        const int gi = seg_i[static_cast<size_t>(seg) * k + e];
-        if (gi >= 0) x[j] = topk_word(seg_v[static_cast<size_t>(seg) * k + e], gi);
+  for (int j = 0; j < 8; ++j) {
+    const int seg = warp + 32 * (j >> 1), e = lane + 32 * (j & 1);
+    const bool in = seg < nseg && e < k;
+    gi[j] = in ? seg_i[static_cast<size_t>(seg) * k + e] : -1;
+    v[j] = in ? seg_v[static_cast<size_t>(seg) * k + e] : kTopkNone;
+  }
+  const int first = (k + nseg - 1) / nseg;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int seg = warp + 32 * (j >> 1), e = lane + 32 * (j & 1);
+    x[j] = gi[j] >= 0 ? topk_word(v[j], gi[j]) : 0ull;
+    if (seg < nseg && e < first) sh.pool[seg * first + e] = static_cast<unsigned>(x[j] >> 32);
+  }
+  const unsigned long long* best = sh.best;
+  if (!topk_by_threshold<8>(sh, x, nseg * first, k)) {
+    // runs warp and warp + 32 meet first, then warp + 64 and warp + 96, then six rounds halve the 64 that remain
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      unsigned long long a[2] = {x[4 * h], x[4 * h + 1]};
+      const unsigned long long b[2] = {x[4 * h + 2], x[4 * h + 3]};
+      run_select(a, b, lane);
+      runs[warp + 32 * h][lane] = a[0];
+      runs[warp + 32 * h][lane + 32] = a[1];
+    }
+    for (int r = 0; r < 6; ++r) {
+      __syncthreads();
+      if (warp < (32 >> r)) {
+        const int sa = warp << (r + 1), sb = sa + (1 << r);
+        unsigned long long a[2] = {runs[sa][lane], runs[sa][lane + 32]};
+        const unsigned long long b[2] = {runs[sb][lane], runs[sb][lane + 32]};
+        run_select(a, b, lane);
+        runs[sa][lane] = a[0];
+        runs[sa][lane + 32] = a[1];
       }
     }
-  };
-  for (int pr = warp; pr < 64; pr += 32) {
-    unsigned long long a[2], b[2];
-    load_run(2 * pr, a);
-    load_run(2 * pr + 1, b);
-    run_select(a, b, lane);
-    runs[pr][lane] = a[0];
-    runs[pr][lane + 32] = a[1];
-  }
-  for (int r = 0; r < 6; ++r) {
     __syncthreads();
-    if (warp < (32 >> r)) {
-      const int sa = warp << (r + 1), sb = sa + (1 << r);
-      unsigned long long a[2] = {runs[sa][lane], runs[sa][lane + 32]};
-      const unsigned long long b[2] = {runs[sb][lane], runs[sb][lane + 32]};
-      run_select(a, b, lane);
-      runs[sa][lane] = a[0];
-      runs[sa][lane + 32] = a[1];
-    }
+    best = runs[0];
   }
-  __syncthreads();
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
-    const unsigned long long w = runs[0][j];
-    const int gi = w != 0ull ? static_cast<int>(~static_cast<unsigned>(w)) : -1;
-    out_i[j] = gi;
-    out_v[j] = gi >= 0 ? __ldg(logits + gi) : kTopkNone;
+    const unsigned long long w = best[j];
+    out_i[j] = w != 0ull ? static_cast<int>(~static_cast<unsigned>(w)) : -1;
+    out_v[j] = topk_value(w, logits);
   }
 }
 

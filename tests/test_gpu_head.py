@@ -79,6 +79,34 @@ def _run_topk(o, logits, k):
     return out_v.cpu().numpy()[:kk], out_i.cpu().numpy()[:kk]
 
 
+@pytest.mark.parametrize("kind", ["normal", "ascending", "equal", "one_segment", "signed_zeros", "few"])
+@pytest.mark.parametrize("n,k", [(151936, 40), (262144, 64), (70000, 64), (2048, 1), (2049, 2)])
+def test_topk_threshold_and_merges(n, k, kind):
+    """What decides whether the threshold leaves few candidates: values spread over the segments, or in order, equal, all the
+    large ones in one segment, zeros of both signs, fewer values than k. Both ways must give the same picks and bits."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal(n).astype(np.float32)
+    if kind == "ascending":
+        x = np.sort(x)
+    elif kind == "equal":
+        x[:] = np.float32(-1.25)
+    elif kind == "one_segment":
+        x[:min(n, 2000)] += np.float32(100)
+    elif kind == "signed_zeros":
+        x = np.where(rng.random(n) < 0.5, np.float32(0.0), np.float32(-0.0)).astype(np.float32)
+    elif kind == "few":
+        x[:] = -np.inf
+        x[rng.integers(0, n, 5)] = rng.standard_normal(5)
+    slots = (n + 2047) // 2048 * k
+    xd = torch.from_numpy(x).to(DEV)
+    sv, si = torch.zeros(slots, device=DEV), torch.zeros(slots, dtype=torch.int32, device=DEV)
+    ov, oi = torch.zeros(k, device=DEV), torch.zeros(k, dtype=torch.int32, device=DEV)
+    ops.topk_select_f32_2p(xd, sv, si, slots, ov, oi, n, k)
+    want_v, want_i = topk_select(x, k)
+    assert np.array_equal(oi.cpu().numpy(), want_i)
+    assert np.array_equal(ov.cpu().numpy().view(np.uint32), np.asarray(want_v, dtype=np.float32).view(np.uint32))
+
+
 @pytest.mark.parametrize("n,k", [(151936, 32), (248320, 64), (2048, 8), (5000, 1), (100, 64), (40, 64)])
 def test_two_phase_topk_is_exact(n, k):
     rng = np.random.default_rng(n + k)
