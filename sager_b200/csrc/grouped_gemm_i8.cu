@@ -51,6 +51,7 @@
 
 #include "api_util.cuh"
 #include "quantize_dev.cuh"
+#include "umma.cuh"
 
 namespace sgr {
 namespace {
@@ -107,96 +108,6 @@ struct GemmArgs {
   int n_items;
   int* status;
 };
-
-// Operand descriptor (K-major, no swizzle) as two words: start >> 4 | LBO (128 B) >> 4 << 16, and
-// SBO (256 B) >> 4 | version 1 << 14. Only the first depends on the tile.
-__device__ __forceinline__ uint32_t umma_desc(uint32_t saddr) { return ((saddr & 0x3FFFFu) >> 4) | (8u << 16); }
-constexpr uint32_t kDescHi = 16u | (1u << 14);
-// D fp32, A and B fp16, both K-major, M = 128, N = n
-__device__ __forceinline__ uint32_t umma_idesc(int n) {
-  return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(kGemmRows >> 4) << 24);
-}
-// A in tensor memory (lane = row, a column holds two consecutive K values) / A in shared memory
-// The whole warp runs the instruction stream, `lead` picks the lane that issues.
-__device__ __forceinline__ void umma_ts(uint32_t lead, uint32_t tmem_d, uint32_t tmem_a, uint32_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 b, {%2, %5};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "r"(db), "r"(idesc), "r"(accumulate), "r"(kDescHi), "r"(lead)
-      : "memory");
-}
-__device__ __forceinline__ void umma_ss(uint32_t lead, uint32_t tmem_d, uint32_t da, uint32_t db, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %6, 0;\n\tmov.b64 a, {%1, %5};\n\tmov.b64 b, {%2, %5};\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(da), "r"(db), "r"(idesc), "r"(accumulate), "r"(kDescHi), "r"(lead)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
-  return p != 0;
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Bounded wait (as mbar_wait) in a handful of instructions per poll: polls return early whenever something
-// happens in the barrier unit, so with two dozen waiting warps their instructions count.
-__device__ __forceinline__ bool mbar_wait_tight(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t.reg .b32 n;\n\tmov.b32 n, 0;\n"
-      "POLL:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
-      "add.u32 n, n, 1;\n\tsetp.lt.u32 q, n, %3;\n\t@q bra POLL;\n"
-      "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(1u << 22)
-      : "memory");
-  return ok != 0;
-}
-template <int N> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
-
-__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
-__device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
-// (x & mask) | bits in one instruction
-__device__ __forceinline__ uint32_t and_or(uint32_t x, uint32_t mask, uint32_t bits) {
-  uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(x), "r"(mask), "r"(bits));
-  return d;
-}
-// two packed fp32: each component rounds as the scalar instruction
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(uint32_t lo, uint32_t hi) { f32x2 d; asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi)); return d; }
-__device__ __forceinline__ f32x2 splat2(float v) { return pack2(__float_as_uint(v), __float_as_uint(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 d; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b)); return d; }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 d; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c)); return d; }
-__device__ __forceinline__ float part2(f32x2 v, int hi) {
-  uint32_t a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
-  return __uint_as_float(hi ? b : a);
-}
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {    // one arrival when this thread's copies so far have landed
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // address of (row, 16-byte K half) inside a canonical tile
 __device__ __forceinline__ int tile_at(int row, int khalf) { return (row >> 3) * 256 + khalf * 128 + (row & 7) * 16; }
@@ -486,12 +397,12 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
       unsigned job = 0, fill0 = 0, tile_no = 0;
       int slot = 0;
       unsigned slot_ph = 0;
-      const uint32_t d_min = umma_desc(smem_u32(smem + kOffMin)), d_b = umma_desc(smem_u32(smem + kOffB));
+      const uint32_t d_min = umma_desc_core(smem_u32(smem + kOffMin)), d_b = umma_desc_core(smem_u32(smem + kOffB));
       const uint32_t lead = elect_one();
       bool ok = true;
       while (ok && wk.next<DUAL>(a, u)) {
         if (u.w0 == nullptr) continue;
-        const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc(u.n_mma), 0);
+        const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc_f16(u.n_mma), 0);
         ok = for_jobs<DUAL>(a, u, [&](int t, int, int m, int fill) {
           const unsigned set = job & 1, f = fill0 + fill, buf = f & 1;
           if (!DUAL || m == 0) {
@@ -509,8 +420,8 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
             tc_fence_after();
             const uint32_t ta = tmem + kColA + slot * 64;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) umma_ts(lead, d0, ta + k * 8, db + (h * 8 + k) * (kBTile >> 4), idesc, (h | k) != 0);
-            if (h == 1) umma_ss(lead, d1, dm, db + 16 * (kBTile >> 4), idesc, 0u);
+            for (int k = 0; k < 8; ++k) umma_ts(lead, d0, ta + k * 8, db + (h * 8 + k) * (kBTile >> 4), kDescCore, idesc, (h | k) != 0);
+            if (h == 1) umma_ss(lead, d1, dm, db + 16 * (kBTile >> 4), kDescCore, idesc, 0u);
             if (lead) {
               umma_commit(&bar[kBarAEmpty + slot]);
               if (h == 1) {

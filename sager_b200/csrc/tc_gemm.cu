@@ -21,8 +21,11 @@
 #include <atomic>
 #include <cstring>
 
+#include <algorithm>
+
 #include "api_util.cuh"
 #include "q4k_common.cuh"
+#include "umma.cuh"
 
 namespace sgr {
 namespace {
@@ -209,6 +212,223 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
   if (threadIdx.x == 0 && *fail != 0 && a.status != nullptr) atomicExch(a.status, 1);
 }
 
+// ---- Q4_K weights: the dequantisation inside the GEMM ------------------------------------------
+// A CTA owns 128 weight rows and up to 256 token rows. The 128 rows are the M lanes of tensor memory, so a thread
+// dequantises its row of a block in registers and stores it as the tensor-memory operand (tcgen05.st); only the
+// activations go through shared memory. Against a separate dequantisation and 128 x 128 tiles (7.5 + 64 us for
+// 4096 x 2048 over 2048 rows) that reads 36 bytes of weights per 64 k instead of 128 and half the activations: the
+// tiles' traffic from L2 was the bound. 43.7 us now, the MMAs' own time being 21. `scratch` still receives the dequantised rows (each token tile writes its share of the blocks).
+//   * warps 0-7: unpack, four to a block, even and odd blocks; then the epilogue
+//   * warp 8: activation tiles (TMA, 128-byte swizzle, 64 k a stage)
+//   * warp 9: block columns of the weights (cp.async), four in flight
+//   * warp 10: tensor memory and MMA issue
+constexpr int kQ4Threads = 352, kQ4WStages = 4, kQ4WBytes = 128 * kW4, kQ4Slots = 3;
+constexpr int kQ4BBytes = 128 * 1024;             // activation ring: 4 stages of 256 rows, 8 of 128 or fewer
+constexpr int kQ4Smem = 1024 + 1024 + kQ4BBytes + kQ4WStages * kQ4WBytes;
+enum { kQ4WFull = 0, kQ4WEmpty = 4, kQ4AFull = 8, kQ4AEmpty = 11, kQ4BFull = 14, kQ4BEmpty = 22, kQ4Acc = 30, kQ4Bars = 31 };
+
+struct Q4Args {
+  const unsigned char* w;
+  uint16_t *y, *scratch;
+  int n_rows, k, n_tokens;
+  int bn, stages;                                 // token rows per CTA, activation stages
+  int* status;
+};
+
+__global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_constant__ CUtensorMap map_x, const Q4Args a) {
+  extern __shared__ unsigned char tc_smem_raw[];
+  const uint32_t base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
+  unsigned char* smem = tc_smem_raw + (base - smem_u32(tc_smem_raw));
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + 512);
+  volatile int* fail = reinterpret_cast<volatile int*>(smem + 516);
+  unsigned char* w_sm = smem + 1024 + kQ4BBytes;
+  const uint32_t b_sm = base + 1024;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row0 = blockIdx.x * 128, tok0 = blockIdx.y * a.bn;
+  const int ntok = min(a.bn, a.n_tokens - tok0), nb = a.k / kQK;
+  const uint32_t b_bytes = static_cast<uint32_t>(a.bn) * 128;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kQ4WStages; ++i) { mbar_init(&bar[kQ4WFull + i], 32); mbar_init(&bar[kQ4WEmpty + i], 4); }
+    for (int i = 0; i < kQ4Slots; ++i) { mbar_init(&bar[kQ4AFull + i], 4); mbar_init(&bar[kQ4AEmpty + i], 1); }
+    for (int i = 0; i < 8; ++i) { mbar_init(&bar[kQ4BFull + i], 1); mbar_init(&bar[kQ4BEmpty + i], 1); }
+    mbar_init(&bar[kQ4Acc], 1);
+    *fail = 0;
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == 10) {
+    __syncwarp();
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot, tmem_a = tmem + 256;
+  auto wait_warp = [&](int b, unsigned parity) {
+    if (__all_sync(0xFFFFFFFFu, mbar_wait_tight(&bar[b], parity)) != 0) return true;
+    *fail = 1;
+    return false;
+  };
+
+  if (warp < 8) {
+    const int grp = warp >> 2, r = (warp & 3) * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    pdl_wait();                                   // scratch and y may still be read by the kernel before
+    pdl_launch_dependents();
+    const f32x2 magic = splat2(-8388608.f);
+    const int share = gridDim.y;                  // this token tile writes blocks blockIdx.y, + share, ... to scratch
+    uint16_t* row_out = a.scratch + static_cast<size_t>(min(row0 + r, a.n_rows - 1)) * a.k;
+    bool ok = true;
+    for (int job = grp; job < nb && ok; job += 2) {
+      const int st = job % kQ4WStages;
+      if (!(ok = wait_warp(kQ4WFull + st, (job / kQ4WStages) & 1))) break;
+      const uint4* blk = reinterpret_cast<const uint4*>(w_sm + st * kQ4WBytes + r * kW4);
+      const uint4 hdr = blk[0];
+      const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
+      const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
+      const bool keep = job % share == static_cast<int>(blockIdx.y) && row0 + r < a.n_rows;
+#pragma unroll 1
+      for (int g = 0; g < 4; ++g) {
+        const int x = 2 * job + (g >> 1), slot = x % kQ4Slots;
+        if ((g & 1) == 0) {
+          if (!(ok = wait_warp(kQ4AEmpty + slot, ((x / kQ4Slots) & 1) ^ 1u))) break;
+          tc_fence_after();
+        }
+        const uint4 q0 = blk[1 + 2 * g], q1 = blk[2 + 2 * g];
+        const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        const uint32_t scw = (g < 2 ? s6.sc[0] : s6.sc[1]) >> (16 * (g & 1)), mnw = (g < 2 ? s6.mn[0] : s6.mn[1]) >> (16 * (g & 1));
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {             // sub-block 2 g + h: value = fp16(fma(d * sc, q, -(dmin * mn)))
+          const f32x2 sd = splat2(d * static_cast<float>((scw >> (8 * h)) & 0xFFu));
+          const f32x2 sm = splat2(-(dmin * static_cast<float>((mnw >> (8 * h)) & 0xFFu)));
+          const uint32_t dst = tmem_a + lanes + slot * 64 + (g & 1) * 32 + h * 16;
+#pragma unroll
+          for (int i0 = 0; i0 < 8; i0 += 4) {
+            uint32_t v[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t nib = (raw[i0 + i] >> (4 * h)) & 0x0F0F0F0Fu;
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {       // 2^23 + q by byte insertion, - 2^23 exactly
+                const f32x2 q = add2(pack2(__byte_perm(nib, 0x4B000000u, 0x7440 + 2 * c), __byte_perm(nib, 0x4B000000u, 0x7441 + 2 * c)), magic);
+                const f32x2 f = fma2(sd, q, sm);
+                asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(v[2 * i + c]) : "f"(part2(f, 1)), "f"(part2(f, 0)));
+              }
+            }
+            tmem_st8(dst + 2 * i0, v);
+            if (keep) {
+              uint4* o = reinterpret_cast<uint4*>(row_out + job * kQK + (2 * g + h) * 32 + i0 * 4);
+              o[0] = make_uint4(v[0], v[1], v[2], v[3]);
+              o[1] = make_uint4(v[4], v[5], v[6], v[7]);
+            }
+          }
+        }
+        if (g & 1) {
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_one(&bar[kQ4AFull + slot]);
+        }
+      }
+      if (ok && lane == 0) mbar_arrive_one(&bar[kQ4WEmpty + st]);
+    }
+    // epilogue: this thread's weight row, half of the token columns; lane pairs exchange so that a store is two rows
+    ok = ok && wait_warp(kQ4Acc, 0);
+    if (ok && *fail == 0) {
+      tc_fence_after();
+      const int row = row0 + r, half = (a.bn >> 1);
+      const int c1 = min((grp + 1) * half, ntok);
+      const bool pairs = (a.n_rows & 1) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 3u) == 0;
+      const bool odd = lane & 1;
+#pragma unroll 1
+      for (int c = grp * half; c < c1; c += 8) {
+        uint32_t v[8];
+        tmem_ld8(tmem + lanes + c, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (pairs) {
+#pragma unroll
+          for (int q = 0; q < 8; q += 2) {
+            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[q] : v[q + 1], 1);
+            const float lo = __uint_as_float(odd ? got : v[q]), hi = __uint_as_float(odd ? v[q + 1] : got);
+            const int t = c + q + (odd ? 1 : 0);
+            if (t < c1 && row < a.n_rows)
+              *reinterpret_cast<uint32_t*>(a.y + static_cast<size_t>(tok0 + t) * a.n_rows + (row & ~1)) = h2_bits(__floats2half2_rn(lo, hi));
+          }
+        } else if (row < a.n_rows) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            if (c + q < c1) a.y[static_cast<size_t>(tok0 + c + q) * a.n_rows + row] = f2h(__uint_as_float(v[q]));
+        }
+      }
+    }
+  } else if (warp == 8) {
+    pdl_wait();
+    if (lane == 0) {
+      for (int kb = 0; kb < 4 * nb; ++kb) {
+        const int s = kb % a.stages;
+        if (!mbar_wait_tight(&bar[kQ4BEmpty + s], ((kb / a.stages) & 1) ^ 1u)) {
+          *fail = 1;
+          break;
+        }
+        mbar_expect_tx(&bar[kQ4BFull + s], b_bytes);
+        tc_tma_2d(b_sm + s * b_bytes, &map_x, kb * kBK, tok0, &bar[kQ4BFull + s]);
+      }
+    }
+  } else if (warp == 9) {
+    // (the weights do not depend on the kernel before) 16-byte piece p = 9 * row + c goes to lane p % 32; nine steps
+    // of 32 pieces are 32 rows. Rows past the matrix repeat its last one: never stored.
+    const int row_bytes = nb * kW4, last = a.n_rows - 1 - row0;
+    for (int job = 0; job < nb; ++job) {
+      const int st = job % kQ4WStages;
+      if (!wait_warp(kQ4WEmpty + st, ((job / kQ4WStages) & 1) ^ 1u)) break;
+      const unsigned char* src = a.w + static_cast<size_t>(row0) * row_bytes + job * kW4;
+      const uint32_t dst = smem_u32(w_sm + st * kQ4WBytes) + lane * 16;
+#pragma unroll 9
+      for (int q = 0; q < 36; ++q) {
+        const int piece = q * 32 + lane, row = piece / 9;
+        cp_async16(dst + q * 512, src + static_cast<size_t>(min(row, last)) * row_bytes + (piece - 9 * row) * 16);
+      }
+      cp_async_arrive(&bar[kQ4WFull + st]);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {
+    const uint32_t lead = elect_one();
+    const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc_f16(max(16, (ntok + 15) & ~15)), 0);
+    int slot = 0, s = 0;
+    unsigned slot_ph = 0, s_ph = 0;
+    bool ok = true;
+    for (int x = 0; x < 2 * nb && ok; ++x) {      // half-blocks
+      if (!(ok = wait_warp(kQ4AFull + slot, slot_ph))) break;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (!(ok = wait_warp(kQ4BFull + s, s_ph))) break;
+        tc_fence_after();
+        const uint32_t db = umma_desc_swizzled(b_sm + s * b_bytes), ta = tmem_a + slot * 64 + j * 32;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) umma_ts(lead, tmem, ta + kk * 8, db + kk * 2, kDescSwizzled, idesc, (x | j | kk) != 0);
+        if (lead) umma_commit(&bar[kQ4BEmpty + s]);
+        if (++s == a.stages) { s = 0; s_ph ^= 1u; }
+      }
+      if (!ok) break;
+      if (lead) umma_commit(&bar[kQ4AEmpty + slot]);
+      if (++slot == kQ4Slots) { slot = 0; slot_ph ^= 1u; }
+    }
+    if (lead) umma_commit(&bar[kQ4Acc]);          // arrives when everything issued so far has finished
+    mbar_wait_tight(&bar[kQ4Acc], 0);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 10) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+  if (threadIdx.x == 0 && *fail != 0 && a.status != nullptr) atomicExch(a.status, 1);
+}
+
 // ---- dequantisation ----------------------------------------------------------------------
 // Lane l of a warp owns weights 8l .. 8l+7 of one super-block: sub-block l/4, its
 // (l%4)-th octet. The warp's 32 stores are one contiguous 512-byte run.
@@ -368,6 +588,29 @@ int launch_dequant(const void* w, void* out16, long long n_blocks, cudaStream_t 
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
+int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratch, int n_rows, int k, int n_tokens, cudaStream_t s) {
+  if (reinterpret_cast<uintptr_t>(x) & 15u) return kErrAlign;
+  const int sms = device_sms(), row_tiles = (n_rows + 127) / 128;
+  if (sms <= 0) return kErrLaunch;
+  // Token rows per CTA: the fewest estimated cycles - waves of CTAs, each its blocks at the MMAs' rate (130 cycles
+  // per 256 columns and K = 16) or the unpacking's (about 1100 a block), and start-up and epilogue.
+  int bn = 64;
+  long long best = 0;
+  for (const int cand : {256, 128, 64}) {
+    const long long waves = (static_cast<long long>(row_tiles) * ((n_tokens + cand - 1) / cand) + sms - 1) / sms;
+    const long long cycles = waves * (static_cast<long long>(k / kQK) * std::max(2080 * cand / 256, 1100) + 4000 + 12 * cand);
+    if (best == 0 || cycles < best) {
+      best = cycles;
+      bn = cand;
+    }
+  }
+  CUtensorMap mx;
+  if (!operand_map(&mx, x, n_tokens, k, kLayoutSwizzled, bn)) return kErrUnsupported;
+  if (!opt_in_smem<tc_gemm_q4_kernel>(kQ4Smem)) return kErrLaunch;
+  Q4Args a{static_cast<const unsigned char*>(w), y, scratch, n_rows, k, n_tokens, bn, std::min(8, kQ4BBytes / (bn * 128)), status_word()};
+  return launch_pdl(tc_gemm_q4_kernel, dim3(row_tiles, (n_tokens + bn - 1) / bn), kQ4Threads, kQ4Smem, s, mx, a);
+}
+
 }  // namespace
 }  // namespace sgr
 
@@ -411,9 +654,7 @@ SGR_API int sgr_tc_gemm_q4_k_f16(const void* w, const uint16_t* x, uint16_t* y, 
   if (k < kQK || (k & (k - 1)) != 0) return kErrUnsupported;
   if (reinterpret_cast<uintptr_t>(w) & 15u) return kErrAlign;
   if (reinterpret_cast<uintptr_t>(scratch) & 15u) return kErrAlign;
-  const int rc = launch_dequant(w, scratch, static_cast<long long>(n_rows) * (k / kQK), as_stream(stream));
-  if (rc != kOk) return rc;
-  return launch_tc_gemm<false>(scratch, x, y, n_rows, k, n_tokens, as_stream(stream));
+  return launch_tc_q4(w, x, y, scratch, n_rows, k, n_tokens, as_stream(stream));
 }
 
 SGR_API int sgr_dequant_experts_q4_k_f16(const void* const* tab_a, const void* const* tab_b, const int* off,

@@ -154,6 +154,24 @@ def test_q4k_gemm_and_router(layout):
     assert rel(logits.cpu().numpy(), (x_dev.float() @ wr.t()).cpu().numpy()) < 2e-3
 
 
+@pytest.mark.parametrize("rows,k,tok", [(128, 256, 1), (100, 256, 17), (129, 512, 65), (1000, 2048, 129), (4096, 512, 300),
+                                        (333, 1024, 256), (4096, 2048, 1500)])
+def test_q4k_gemm_tile_edges(rows, k, tok):
+    """Ragged row and token tiles, odd row counts (no paired stores), the three token tile sizes."""
+    w_np, w_dev = make_q4k(rows, k, 13)
+    x_np, x_dev = make_x16(tok, k, 14)
+    scratch = torch.zeros(rows * k + 8, dtype=torch.float16, device=DEV)
+    y = torch.full((tok + 1, rows), 9.0, dtype=torch.float16, device=DEV)
+    ops.tc_gemm_q4_k_f16(w_dev, x_dev, y, scratch, rows, k, tok)
+    w16 = torch.zeros(rows, k, dtype=torch.float16, device=DEV)
+    ops.dequant_q4_k_f16(w_dev, w16, rows, k)
+    assert torch.equal(scratch[:rows * k].view(torch.int16), w16.view(-1).view(torch.int16)) and torch.all(scratch[rows * k:] == 0)
+    want = gemm_want(w16, x_dev)
+    # fp32 accumulation in another order, one rounding to fp16
+    assert rel(y[:tok].float().cpu().numpy(), want.cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
+    assert lib().raw("sgr_status")(0) == 0
+
+
 def test_refusals_launch_nothing():
     t = torch.zeros(4096, dtype=torch.float16, device=DEV)
     p = t.data_ptr()
