@@ -50,7 +50,10 @@ constexpr int kMaxRows = 64;       // token rows per call (row masks are 64-bit)
 constexpr int kTokTile = 8;        // token rows per tile of the item kernel (one MMA n-tile)
 constexpr int kMaxGrid = 192;            // most CTAs the expert kernels are launched with
 constexpr int kTmapSlots = 6;            // patched TMA descriptor sets per CTA of the row-streaming kernel
-constexpr int kTokenKernelMaxRows = 3;   // layers of up to this many token rows run as one persistent launch
+#ifndef SGR_TKR
+#define SGR_TKR 4
+#endif
+constexpr int kTokenKernelMaxRows = SGR_TKR;   // layers of up to this many token rows run as one persistent launch
                                          // (measured per layer, us: 26.6 / 36.1 / 44.7 against 30.1 / 39.6 / 47.3 for
                                          // route + expert kernel; at 4 rows 57 against 50)
 constexpr int kRowsKernelMinRows = 4;    // layers of at least this many token rows run the row-streaming kernel
@@ -1451,8 +1454,8 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       a->ep_dst == nullptr && a->ep_out == nullptr &&
       L.e_lo == 0 && L.e_hi == L.E && L.sh_lo == 0 && L.sh_hi == L.n && L.nbh <= 16 && L.nbf <= 16 &&
       a->workspace_bytes >= lay.items_total) {
-    const tk::Geom g = tk::geom(tk::kMaxTok, L.H, L.FF, L.E, L.grid);
-    if (g.total <= 227 * 1024 && g.rows_per_cta <= tk::kWarps)
+    const tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid);
+    if (g.total <= 227 * 1024 && g.rows_per_cta <= tk::kGroupWarps)
       return launch_layer<tk::token_layer_kernel>(dim3(L.grid), tk::kThreads, g.total, s, L);
   }
 

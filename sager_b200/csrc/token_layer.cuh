@@ -4,7 +4,7 @@
 // The single-token layer is latency-bound: 18 MB of weights are 3 us of HBM time, and
 // every dependent step around them - a launch, a global round trip, a grid-wide
 // barrier - costs about as much again. This kernel keeps the chain as short as the data
-// dependencies allow. One CTA per SM, eight consumer warps and a producer warp:
+// dependencies allow. One CTA per SM, sixteen consumer warps and a producer warp:
 //
 //   before the previous kernel's results are needed (programmatic dependent launch):
 //     the CTA's router rows and its share of the shared expert's gate / up / down rows
@@ -34,16 +34,27 @@
 namespace tk {
 
 constexpr int kMaxTok = 4;                 // token rows per call
-constexpr int kWarps = 8;                  // consumer warps
+constexpr int kWarps = 16;                 // consumer warps: four to a scheduler, the dots are chains of latencies
 constexpr int kConsumers = kWarps * 32;
+constexpr int kGroupWarps = 8;             // ring stages alternate between two groups of consumer warps
+constexpr int kGroupThreads = kGroupWarps * 32;
 constexpr int kThreads = kConsumers + 32;  // + producer warp
 constexpr int kPairsStage = 16;            // (gate, up) row pairs per ring stage
 constexpr int kRing = 2;
 constexpr int kDownTiles = 16;             // tiles whose down rows are resident at once
 constexpr int kMaxTiles = 33;              // n * K + 1 <= 33
-constexpr int kMaxHRows = 36;              // (tile, row) pairs: n * K + n <= 36
 constexpr int kHdr = 1024;
 constexpr int kTables = 4096;
+
+// Quantised rows laid out for lanes that each take half a block: a half is 128 codes, four int16 sums and the block's
+// scale in 192 bytes, a block 400, so that the eight lanes of a shared-memory access - four blocks x two halves of a
+// row, or two rows of two blocks - read sixteen bytes each from different banks.
+constexpr int kHalf = 192, kHBlk = 2 * kHalf + 16;
+struct HTile {
+  unsigned char* p;
+  int nb;
+  __device__ __forceinline__ unsigned char* blk(int row, int b) const { return p + static_cast<size_t>(row * nb + b) * kHBlk; }
+};
 
 struct Tables {                            // built after the selection, the same in every CTA
   int n_tiles;
@@ -56,8 +67,7 @@ struct Tables {                            // built after the selection, the sam
   int sel_idx[kMaxTok][kMaxTiles];         // [t][0..K]
   float sel_w[kMaxTok][kMaxTiles];
   int route_hrow[kMaxTok][kMaxTiles];      // [t][kk] -> h / y row of that route, -1 = absent; [t][K] = shared
-  XTile xt;                                // the quantised input rows
-  XTile hq;                                // the quantised h rows
+  float z[kMaxTok];                        // softmax denominators
 };
 static_assert(sizeof(Tables) <= kTables, "tables region");
 
@@ -73,33 +83,37 @@ struct Geom {
   size_t off_prob, off_ptab, off_xh, off_rw, off_xt, off_sh, off_ring, off_dn, off_y, total;
   int stage_bytes, slot_bytes;
 };
-__host__ __device__ inline Geom geom(int n_max, int H, int FF, int E, int grid) {
+__host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int grid) {
   Geom g;
   g.rows_per_cta = (E + grid - 1) / grid;
   g.nr_max = (H + grid - 1) / grid;
   g.sp_max = (FF + grid - 1) / grid;
   g.rb_h = (H / kQK) * kW4;
   g.rb_f = (FF / kQK) * kW4;
+  const int hrows = n * (K + 1);                            // (tile, row) pairs at most
   size_t p = kHdr + kTables;
   auto take = [&](size_t bytes) { const size_t at = p; p = (p + bytes + 127) & ~static_cast<size_t>(127); return at; };
-  g.off_prob = take(static_cast<size_t>(kMaxTok) * E * 4);
+  g.off_prob = take(static_cast<size_t>(n) * E * 4);
   g.off_ptab = take(static_cast<size_t>(3) * E * 8);        // the layer's pointer table, read once per CTA
   // x rows as fp16 and the router rows; later the same bytes hold the quantised h rows
-  const size_t a = static_cast<size_t>(kMaxTok) * H * 2 + 128 + static_cast<size_t>(g.rows_per_cta) * H * 4;
-  const size_t b = xtile_bytes(kMaxHRows, FF / kQK);
+  const size_t a = static_cast<size_t>(n) * H * 2 + 128 + static_cast<size_t>(g.rows_per_cta) * H * 4;
+  const size_t b = static_cast<size_t>(hrows) * (FF / kQK) * kHBlk;
   g.off_xh = take(a > b ? a : b);
-  g.off_rw = g.off_xh + ((static_cast<size_t>(kMaxTok) * H * 2 + 127) & ~static_cast<size_t>(127));
-  g.off_xt = take(xtile_bytes(kMaxTok, H / kQK));
+  g.off_rw = g.off_xh + ((static_cast<size_t>(n) * H * 2 + 127) & ~static_cast<size_t>(127));
+  g.off_xt = take(static_cast<size_t>(n) * (H / kQK) * kHBlk);
   g.off_sh = take(static_cast<size_t>(2) * g.sp_max * g.rb_h);
   g.stage_bytes = 2 * kPairsStage * g.rb_h;
   g.off_ring = take(static_cast<size_t>(kRing) * g.stage_bytes);
   g.slot_bytes = g.nr_max * g.rb_f;
-  g.off_dn = take(static_cast<size_t>(kDownTiles) * g.slot_bytes);
-  g.off_y = take(static_cast<size_t>(kMaxHRows) * g.nr_max * 4);
+  g.off_dn = take(static_cast<size_t>(hrows < kDownTiles ? hrows : kDownTiles) * g.slot_bytes);
+  g.off_y = take(static_cast<size_t>(hrows) * g.nr_max * 4);
   g.total = p;
   return g;
 }
 
+// Named barriers of the consumers: 6 all of them, 7 the warps with router rows, 5 the warps that quantise, 8 .. 11 the
+// two warps that select for a token row.
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 6, %0;" ::"n"(kConsumers) : "memory");
 }
@@ -124,11 +138,11 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // Grid-wide barrier on a 64-bit arrival counter that only ever grows: the k-th barrier of the
 // grid (over all launches on this workspace) completes when the counter reaches k * G. Waits are
 // bounded: false when the others did not arrive in time.
-// The grid barrier is driven by ONE thread per CTA that has no part in the work around it
-// (the last consumer thread): at kernel start it reads the counter - some multiple of the
-// grid size plus the arrivals of CTAs that are already further on, none of which can have
-// passed the first barrier - so barrier k of this launch completes at base + k * grid. An
-// arrival is a fence and a fire-and-forget add; nobody waits for the add's round trip.
+// The counter is read by the producer warp at kernel start - some multiple of the grid size plus the
+// arrivals of CTAs that are already further on, none of which can have passed the first barrier - so
+// barrier k of this launch completes at base + k * grid. An arrival is a fence and a fire-and-forget
+// add by the thread whose warp finishes the work; the producer warp polls and passes the word on
+// through an mbarrier, so no consumer waits for a round trip that it could work through.
 __device__ __forceinline__ unsigned long long grid_base(const unsigned long long* ctr, unsigned grid) {
   return ld_acquire_u64(ctr) / grid * grid;
 }
@@ -143,51 +157,41 @@ __device__ __forceinline__ bool grid_wait(const unsigned long long* ctr, unsigne
   return it < kSpinLimit;
 }
 
-// Q8_K-quantise `rows` fp32 rows of h (global memory, FF values each) into a staged tile, a warp
-// per 256-value block, four blocks' loads in flight per warp (arithmetic of stage_quantized_f32).
-__device__ __forceinline__ void quantize_h_rows(const XTile& xt, int rows, const float* src, int FF, int warp, int lane) {
-  const int jobs = rows * xt.nb;
-  for (int j0 = warp; j0 < jobs; j0 += 4 * kWarps) {
-    float4 a[4], b[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int job = min(j0 + u * kWarps, jobs - 1);
-      const int t = job / xt.nb, blk = job - t * xt.nb;
-      const float4* p = reinterpret_cast<const float4*>(src + static_cast<size_t>(t) * FF + blk * kQK) + lane * 2;
-      a[u] = __ldcg(p);
-      b[u] = __ldcg(p + 1);
+// One warp: eight values per lane of a 256-value block -> Q8_K codes, sums and scale in a tile
+// (arithmetic of src/kernels/cuda/q4_k.cu:94-130 in the reference).
+__device__ __forceinline__ void quantize_to_tile(unsigned char* blk, const float (&v)[8], int lane) {
+  int q[8], sum;
+  const float d = quantize_lane8(v, q, sum);
+  unsigned char* half = blk + (lane >> 4) * kHalf;
+  *reinterpret_cast<uint2*>(half + (lane & 15) * 8) =
+      make_uint2((q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) | (static_cast<uint32_t>(q[3] & 0xFF) << 24),
+                 (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) | (static_cast<uint32_t>(q[7] & 0xFF) << 24));
+  const int sum_next = __shfl_down_sync(0xFFFFFFFFu, sum, 4);
+  if ((lane & 7) == 0)
+    *reinterpret_cast<uint32_t*>(half + 128 + ((lane >> 3) & 1) * 4) =
+        (static_cast<uint32_t>(sum) & 0xFFFFu) | (static_cast<uint32_t>(sum_next) << 16);
+  if ((lane & 15) == 0) *reinterpret_cast<float*>(half + 136) = d;
+}
+
+// `rows` fp32 rows of h (global memory, FF values each) into a tile, a warp per 256-value block, two blocks' loads
+// in flight per warp.
+__device__ __forceinline__ void quantize_h_rows(const HTile& xt, int rows, const float* src, int warp, int lane) {
+  // (every CTA reads the same few KB: a load too many is 148 more requests to the same L2 lines)
+  const int jobs = rows * xt.nb;                   // blocks lie one after another in both places
+  for (int j0 = warp; j0 < jobs; j0 += 2 * kWarps) {
+    const float4* p = reinterpret_cast<const float4*>(src + static_cast<size_t>(j0) * kQK) + lane * 2;
+    float4 x = __ldcg(p), y = __ldcg(p + 1), x2, y2;
+    const bool two = j0 + kWarps < jobs;
+    if (two) {
+      x2 = __ldcg(p + kWarps * (kQK / 4));
+      y2 = __ldcg(p + kWarps * (kQK / 4) + 1);
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int job = j0 + u * kWarps;
-      if (job >= jobs) break;                    // warp-uniform
-      const int t = job / xt.nb, blk = job - t * xt.nb;
-      const float v[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
-      float m = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
-      const float amax = fmaxf(1e-30f, m);
-      const float d = amax / 127.f;
-      const float id = d > 0.f ? 1.f / d : 0.f;
-      int q[8], sum = 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        q[i] = max(-127, min(127, static_cast<int>(rintf(v[i] * id))));
-        sum += q[i];
-      }
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-      int8_t* qs = xt.qs + static_cast<size_t>(t) * xt.tok_stride + blk * kXqStride + lane * 8;
-      reinterpret_cast<uint32_t*>(qs)[0] = (q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) |
-                                           (static_cast<uint32_t>(q[3] & 0xFF) << 24);
-      reinterpret_cast<uint32_t*>(qs)[1] = (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) |
-                                           (static_cast<uint32_t>(q[7] & 0xFF) << 24);
-      const int sum_next = __shfl_down_sync(0xFFFFFFFFu, sum, 4);
-      if ((lane & 7) == 0)
-        xt.put_sum_pair(t, blk, lane >> 3, (static_cast<uint32_t>(sum) & 0xFFFFu) | (static_cast<uint32_t>(sum_next) << 16));
-      if (lane == 0) xt.d[t * xt.nb + blk] = d;
+#pragma unroll 1
+    for (int u = 0; u < (two ? 2 : 1); ++u) {      // warp-uniform
+      const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+      quantize_to_tile(xt.blk(0, j0 + u * kWarps), v, lane);
+      x = x2;
+      y = y2;
     }
   }
 }
@@ -201,131 +205,192 @@ struct RowSet {
 __device__ __forceinline__ RowSet rows_of(int mask, int base, bool by_bit) {
   RowSet r;
   r.n = __popc(mask);
-  r.r0 = base + (by_bit ? static_cast<int>(__fns(mask, 0, 1)) : 0);
-  r.r1 = base + (by_bit ? static_cast<int>(__fns(mask, 0, 2)) : 1);
-  r.r2 = base + (by_bit ? static_cast<int>(__fns(mask, 0, 3)) : 2);
-  r.r3 = base + (by_bit ? static_cast<int>(__fns(mask, 0, 4)) : 3);
+  r.r0 = base + (by_bit ? max(__ffs(mask) - 1, 0) : 0);
+  const int m1 = mask & (mask - 1), m2 = m1 & (m1 - 1), m3 = m2 & (m2 - 1);
+  r.r1 = base + (by_bit ? max(__ffs(m1) - 1, 0) : 1);
+  r.r2 = base + (by_bit ? max(__ffs(m2) - 1, 0) : 2);
+  r.r3 = base + (by_bit ? max(__ffs(m3) - 1, 0) : 3);
   return r;
 }
 
-// block_dot of q4k_common.cuh for one matrix and up to kMaxTok staged rows chosen by index.
-// Deliberately NOT inlined and NOT unrolled over rows or nibble groups: every phase of this kernel
-// runs once per CTA, so straight-line code is paid for in instruction fetch, not in issue slots
-// (measured: the unrolled form spent 2.5 us per call site fetching ~12 KB of code). One compact
-// loop serves the shared expert's gate / up, the routed gate / up and the down rows.
-__device__ __noinline__ float4 block_dot_rows(const uint4* wblk, const XTile* xtp, int blk, RowSet rs) {
-  const XTile& xt = *xtp;
-  const uint4 hdr = wblk[0];
-  const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x & 0xFFFFu)));
-  const float dmin = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x >> 16)));
-  const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-  float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-  for (int t = 0; t < rs.n; ++t) {
-    const int r = rs.at(t);
-    int isum = 0;
-#pragma unroll 1
-    for (int g = 0; g < 4; ++g) {
-      const uint4 q0 = wblk[1 + 2 * g], q1 = wblk[2 + 2 * g];
-      const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-      uint32_t lo[8], hi[8];
+// Half a super-block of NMAT weight rows against the rows of `rs` (a lane pair holds a block; the integer sums of the
+// halves meet before the one rounding, so the terms are block_dot's). Whole warps call it: `rows` is the warp's
+// largest row count. Not unrolled over rows: every phase of this kernel runs once per CTA, so straight-line code is
+// paid for in instruction fetch.
+template <int NMAT>
+__device__ __forceinline__ void half_dots(const unsigned char* const (&w)[NMAT], int half, const HTile& xt, int blk, const RowSet& rs,
+                                          int rows, float (&out)[NMAT][kMaxTok]) {
+  uint4 hdr[NMAT], wq[NMAT][4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        lo[i] = raw[i] & 0x0F0F0F0Fu;
-        hi[i] = (raw[i] >> 4) & 0x0F0F0F0Fu;
-      }
-      const uint32_t scw = (g & 2) ? s6.sc[1] : s6.sc[0];
-      const int sc_lo = (scw >> (16 * (g & 1))) & 0xFF;
-      const int sc_hi = (scw >> (16 * (g & 1) + 8)) & 0xFF;
-      const uint4* xa = xt.codes(r, blk, 2 * g);
-      const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
-      isum += sc_lo * dot8(lo, x0, x1) + sc_hi * dot8(hi, x2, x3);
-    }
-    const uint4 bs = xt.sums(r, blk);
-    int msum = __dp2a_lo(static_cast<int>(bs.x), static_cast<int>(s6.mn[0]), 0);
-    msum = __dp2a_hi(static_cast<int>(bs.y), static_cast<int>(s6.mn[0]), msum);
-    msum = __dp2a_lo(static_cast<int>(bs.z), static_cast<int>(s6.mn[1]), msum);
-    msum = __dp2a_hi(static_cast<int>(bs.w), static_cast<int>(s6.mn[1]), msum);
-    const float v = xt.scale(r, blk) * (d * static_cast<float>(isum) - dmin * static_cast<float>(msum));
-    if (t == 0) out.x = v;
-    else if (t == 1) out.y = v;
-    else if (t == 2) out.z = v;
-    else out.w = v;
+  for (int m = 0; m < NMAT; ++m) {
+    const uint4* p = reinterpret_cast<const uint4*>(w[m]);
+    hdr[m] = p[0];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) wq[m][i] = p[1 + 4 * half + i];
   }
-  return out;
+#pragma unroll
+  for (int m = 0; m < NMAT; ++m)
+#pragma unroll
+    for (int t = 0; t < kMaxTok; ++t) out[m][t] = 0.f;
+#pragma unroll 1
+  for (int t = 0; t < rows; ++t) {
+    const unsigned char* xb = xt.blk(rs.at(t < rs.n ? t : 0), blk) + half * kHalf;
+    int isum[NMAT];
+#pragma unroll
+    for (int m = 0; m < NMAT; ++m) isum[m] = 0;
+#pragma unroll
+    for (int gg = 0; gg < 2; ++gg) {
+      const uint4* xa = reinterpret_cast<const uint4*>(xb + 64 * gg);
+      const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
+#pragma unroll
+      for (int m = 0; m < NMAT; ++m) {
+        const uint4 q0 = wq[m][2 * gg], q1 = wq[m][2 * gg + 1];
+        const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+        uint32_t lo[8], hi[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          lo[i] = raw[i] & 0x0F0F0F0Fu;
+          hi[i] = (raw[i] >> 4) & 0x0F0F0F0Fu;
+        }
+        const Scales6 s6 = unpack_scales6(hdr[m].y, hdr[m].z, hdr[m].w);
+        const uint32_t scw = (half ? s6.sc[1] : s6.sc[0]) >> (16 * gg);
+        isum[m] += static_cast<int>(scw & 0xFF) * dot8(lo, x0, x1) + static_cast<int>((scw >> 8) & 0xFF) * dot8(hi, x2, x3);
+      }
+    }
+    const uint4 sd = *reinterpret_cast<const uint4*>(xb + 128);
+#pragma unroll
+    for (int m = 0; m < NMAT; ++m) {
+      const Scales6 s6 = unpack_scales6(hdr[m].y, hdr[m].z, hdr[m].w);
+      const uint32_t mnw = half ? s6.mn[1] : s6.mn[0];
+      int msum = __dp2a_lo(static_cast<int>(sd.x), static_cast<int>(mnw), 0);
+      msum = __dp2a_hi(static_cast<int>(sd.y), static_cast<int>(mnw), msum);
+      const int is = isum[m] + __shfl_xor_sync(0xFFFFFFFFu, isum[m], 1);
+      const int ms = msum + __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
+      const float d = h2f(static_cast<uint16_t>(hdr[m].x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr[m].x >> 16));
+      const float v = __uint_as_float(sd.z) * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
+      if (t == 0) out[m][0] = v;
+      else if (t == 1) out[m][1] = v;
+      else if (t == 2) out[m][2] = v;
+      else out[m][3] = v;
+    }
+  }
+}
+// sum over the blocks of a row, held by lane pairs `2 * lpr` lanes wide, in the order of reduce_lanes
+__device__ __forceinline__ float reduce_pairs(float v, int lpr) {
+  for (int off = lpr >> 1; off > 0; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, 2 * off);
+  return v;
 }
 
-// Gate / up of `np` pairs staged at st (gate rows, then up rows) for the rows `mask` of one tile:
-// thread = (pair, matrix, block lane); the lanes of a row add up with shuffles and the up row's
-// lanes sit `lpr` lanes above the gate row's. SwiGLU, fp32 h rows [hrow0 + slot][FF] to global
-// memory. One copy of this code serves the shared expert's stage and the ring stages.
-__device__ __noinline__ void gate_up_stage(const unsigned char* st, int np, int mask, int hrow0, int pair0,
-                                           const XTile* xt, float* hbuf, int FF, int nbh, int rb_h) {
-  const int tid = threadIdx.x;
-  const int lpr = next_pow2_cap32(nbh);
+// Gate / up of `np` pairs staged at st (gate rows, then up rows) for the rows `mask` of one tile by a group of eight
+// warps: thread = (pair, block, half), both matrices. SwiGLU, fp32 h rows [hrow0 + slot][FF] to global memory.
+// (Inlined at both of its uses: as a function it saved and restored 2,400 warp registers per CTA through local memory.)
+__device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, int mask, int hrow0, int pair0,
+                                           const HTile& xt, float* hbuf, int FF, int nbh, int rb_h) {
+  const int tid = threadIdx.x & (kGroupThreads - 1);
+  const int lpr = next_pow2_cap32(nbh), row_lanes = __ffs(2 * lpr) - 1;
   const RowSet rs = rows_of(mask, 0, true);
-  const int tasks = np * 2 * lpr;
+  const int tasks = np << row_lanes;
 #pragma unroll 1
-  for (int base = 0; base < tasks; base += kConsumers) {        // uniform trip count
+  for (int base = 0; base < tasks; base += kGroupThreads) {        // uniform trip count
     const int q = base + tid;
-    const int lr = q & (lpr - 1);
-    const int rm = q / lpr;
-    const int m = rm & 1, pair = rm >> 1;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (q < tasks) {
-      const unsigned char* row = st + static_cast<size_t>(m) * np * rb_h + static_cast<size_t>(pair) * rb_h;
-#pragma unroll 1
-      for (int blk = lr; blk < nbh; blk += lpr) {
-        const float4 v = block_dot_rows(reinterpret_cast<const uint4*>(row + blk * kW4), xt, blk, rs);
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-      }
-    }
-    const float av[kMaxTok] = {acc.x, acc.y, acc.z, acc.w};
+    const int half = q & 1, lr = (q >> 1) & (lpr - 1), pair = min(q >> row_lanes, np - 1), blk = min(lr, nbh - 1);
+    const unsigned char* row = st + static_cast<size_t>(pair) * rb_h + blk * kW4;
+    const unsigned char* const w[2] = {row, row + static_cast<size_t>(np) * rb_h};
+    float v[2][kMaxTok];
+    half_dots<2>(w, half, xt, blk, rs, rs.n, v);
 #pragma unroll
     for (int t = 0; t < kMaxTok; ++t) {
-      const float g = reduce_lanes(av[t], lpr);
-      const float u = __shfl_down_sync(0xFFFFFFFFu, g, lpr);
-      if (q < tasks && lr == 0 && m == 0 && t < rs.n)
-        hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = g / (1.f + expf(-g)) * u;
+      if (t >= rs.n) break;                        // uniform
+      const float g = reduce_pairs(lr < nbh ? v[0][t] : 0.f, lpr), u = reduce_pairs(lr < nbh ? v[1][t] : 0.f, lpr);
+      if (q < tasks && half == 0 && lr == 0) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(g, u);
     }
   }
 }
 
-// One warp: Q8_K-quantise 256 fp16 values (eight per lane, `raw`) into block `blk` of row t of
-// a staged tile (arithmetic of src/kernels/cuda/q4_k.cu:94-130 in the reference).
-__device__ __forceinline__ void quantize_f16_to_tile(const XTile& xt, int t, int blk, const uint4 raw, int lane) {
-  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  float v[8];
+__device__ __noinline__ void select_general(float* prob, int E, int K, int* idx, float* w, float shared_w, int lane) {
+  router_select_warp(prob, E, K, idx, w, shared_w, true, lane);
+}
+
+// Softmax and top-K of one token row by two warps (up to 256 experts, K < 32). The strictly serial sum of the
+// exponentials - the reference's order - is most of it, so one warp adds while the other picks the K + 1 largest
+// exponentials. Dividing by the sum keeps their order; only if it makes two of them equal, or something is not
+// finite, the order of the quotients could be another one, and the general selection on the quotients is run.
+__device__ __forceinline__ void select_pair(const float* logits, float* prob, Tables& tb, int t, bool adds, int E, int K, float shared_w,
+                                            int lane) {
+  float e[8];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    v[2 * i] = h2f(static_cast<uint16_t>(w[i] & 0xFFFFu));
-    v[2 * i + 1] = h2f(static_cast<uint16_t>(w[i] >> 16));
+  for (int j = 0; j < 8; ++j) e[j] = lane + 32 * j < E ? __ldcg(logits + lane + 32 * j) : -1e30f;
+  float mx = -1e30f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, e[j]);
+  {                                                // warp maximum through an order-preserving integer key
+    const int b = __float_as_int(mx);
+    const int mk = __reduce_max_sync(0xFFFFFFFFu, b ^ ((b >> 31) & 0x7FFFFFFF));
+    mx = __int_as_float(mk ^ ((mk >> 31) & 0x7FFFFFFF));
   }
-  float m = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
+  for (int j = 0; j < 8; ++j) e[j] = expf(e[j] - mx);
+  if (adds) {
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
-  const float amax = fmaxf(1e-30f, m);
-  const float d = amax / 127.f;
-  const float id = d > 0.f ? 1.f / d : 0.f;
-  int q[8], sum = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    q[i] = max(-127, min(127, static_cast<int>(rintf(v[i] * id))));
-    sum += q[i];
+    for (int j = 0; j < 8; ++j)
+      if (lane + 32 * j < E) prob[lane + 32 * j] = e[j];
+    __syncwarp();
+    if (lane == 0) {
+      float z = 0.f;
+      int i = 0;
+#pragma unroll 4
+      for (; i + 8 <= E; i += 8) {
+        const float4 a = *reinterpret_cast<const float4*>(prob + i), b = *reinterpret_cast<const float4*>(prob + i + 4);
+        z += a.x; z += a.y; z += a.z; z += a.w; z += b.x; z += b.y; z += b.z; z += b.w;
+      }
+      for (; i < E; ++i) z += prob[i];
+      tb.z[t] = z;
+    }
+    __syncwarp();
+    named_sync(8 + t, 64);
+    return;
   }
-  sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-  sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-  int8_t* qs = xt.qs + static_cast<size_t>(t) * xt.tok_stride + blk * kXqStride + lane * 8;
-  reinterpret_cast<uint32_t*>(qs)[0] = (q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) |
-                                       (static_cast<uint32_t>(q[3] & 0xFF) << 24);
-  reinterpret_cast<uint32_t*>(qs)[1] = (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) |
-                                       (static_cast<uint32_t>(q[7] & 0xFF) << 24);
-  const int sum_next = __shfl_down_sync(0xFFFFFFFFu, sum, 4);
-  if ((lane & 7) == 0)
-    xt.put_sum_pair(t, blk, lane >> 3, (static_cast<uint32_t>(sum) & 0xFFFFu) | (static_cast<uint32_t>(sum_next) << 16));
-  if (lane == 0) xt.d[t * xt.nb + blk] = d;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (lane + 32 * j >= E) e[j] = -1.f;
+  float my_e = -1.f;
+  int my_i = 0;
+#pragma unroll 1
+  for (int kk = 0; kk <= K; ++kk) {
+    float v[4];
+    int s[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { v[j] = fmaxf(e[2 * j], e[2 * j + 1]); s[j] = e[2 * j] >= e[2 * j + 1] ? 2 * j : 2 * j + 1; }
+    const int sa = v[0] >= v[1] ? s[0] : s[1], sb = v[2] >= v[3] ? s[2] : s[3];
+    const float va = fmaxf(v[0], v[1]), vb = fmaxf(v[2], v[3]), best = fmaxf(va, vb);
+    const int slot = va >= vb ? sa : sb;
+    const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(best));        // values are >= 0 or -1
+    const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(best) == top ? lane + 32 * slot : 0x7FFFFFFF);
+    if ((win & 31) == lane) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (j == (win >> 5)) e[j] = -1.f;
+    }
+    if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
+  }
+  named_sync(8 + t, 64);
+  const float z = tb.z[t];
+  const float p = my_e / z;
+  const float next = __shfl_down_sync(0xFFFFFFFFu, p, 1);
+  const bool fine = z > 0.f && z <= 3.4e38f && __all_sync(0xFFFFFFFFu, lane >= K || (my_e >= 0.f && p > next));
+  if (fine) {
+    float wsum = 0.f;
+    for (int kk = 0; kk < K; ++kk) wsum += __shfl_sync(0xFFFFFFFFu, p, kk);
+    if (lane < K) {
+      tb.sel_idx[t][lane] = my_i;
+      tb.sel_w[t][lane] = wsum > 0.f ? p / wsum : p;
+    }
+    if (lane == 0) tb.sel_w[t][K] = shared_w;
+  } else {
+    for (int i = lane; i < E; i += 32) prob[i] = __ldcg(logits + i);
+    __syncwarp();
+    select_general(prob, E, K, tb.sel_idx[t], tb.sel_w[t], shared_w, lane);
+  }
 }
 
 // Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned.
@@ -335,7 +400,7 @@ __device__ __forceinline__ void copy_plain(unsigned char* dst, const unsigned ch
 
 __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const Geom G = geom(kMaxTok, L.H, L.FF, L.E, gridDim.x);
+  const Geom G = geom(L.n, L.K, L.H, L.FF, L.E, gridDim.x);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);              // [kRing]
   uint64_t* empty = full + kRing;                                  // [kRing]
   uint64_t* sh_full = empty + kRing;                               // shared expert's gate / up pairs
@@ -343,6 +408,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   uint64_t* dn_full = shdn_full + 1;                               // routed tiles' down rows, one phase per round
   uint64_t* dn_empty = dn_full + 1;
   uint64_t* ready = dn_empty + 1;                                  // tables built
+  uint64_t* based = ready + 1;                                     // the grid counter has been read
+  uint64_t* passed = based + 1;                                    // grid barrier passed (or given up), one phase each
   StageDesc* desc = reinterpret_cast<StageDesc*>(smem + 128);      // [kRing]
   int* flag = reinterpret_cast<int*>(smem + 256);
   Tables& tb = *reinterpret_cast<Tables*>(smem + kHdr);
@@ -361,22 +428,23 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   unsigned long long* gctr = reinterpret_cast<unsigned long long*>(L.cnt + 12);
 
   // this CTA's shares: shared-expert pairs [sp0, sp1), output rows [r0, r1)
-  const int sp0 = static_cast<int>(static_cast<long long>(FF) * cta / grid);
-  const int sp1 = static_cast<int>(static_cast<long long>(FF) * (cta + 1) / grid);
-  const int r0 = static_cast<int>(static_cast<long long>(H) * cta / grid);
-  const int r1 = static_cast<int>(static_cast<long long>(H) * (cta + 1) / grid);
+  // (products stay below 2^31: at most 33 tiles x 8192 pairs x 192 CTAs)
+  auto share = [&](int total, int part) { return static_cast<int>(static_cast<unsigned>(total) * static_cast<unsigned>(part) / static_cast<unsigned>(grid)); };
+  const int sp0 = share(FF, cta), sp1 = share(FF, cta + 1), r0 = share(H, cta), r1 = share(H, cta + 1);
   const int nr = r1 - r0;
 
   if (tid == 0) {
     for (int s = 0; s < kRing; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], kWarps);
+      mbar_init(&empty[s], kGroupWarps);
     }
     mbar_init(sh_full, 1);
     mbar_init(shdn_full, 1);
     mbar_init(dn_full, 1);
     mbar_init(dn_empty, kWarps);
     mbar_init(ready, 1);
+    mbar_init(based, 1);
+    mbar_init(passed, 1);
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -418,16 +486,30 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         }
       }
     }
+    unsigned long long bar_base = 0;
+    if (lane == 0) {
+      bar_base = grid_base(gctr, grid);
+      mbar_arrive_one(based);
+    }
+    // barrier k of the grid: its outcome goes to flag[k - 1]
+    auto grid_poll = [&](int k) {
+      if (lane == 0) {
+        flag[k - 1] = grid_wait(gctr, bar_base + static_cast<unsigned long long>(k) * grid) ? 1 : 0;
+        __threadfence_block();
+        mbar_arrive_one(passed);
+      }
+      __syncwarp();
+    };
+    grid_poll(1);
     if (!mbar_wait(ready, 0)) {
-      if (lane == 0) atomicExch(L.status, 7);
+      if (lane == 0 && flag[0]) atomicExch(L.status, 7);
       return;
     }
     const int T = tb.n_tiles;
     const int t_first = has_shared ? 1 : 0;
     // routed gate / up pairs: a flat range of (tile, pair) per CTA
-    const long long P = static_cast<long long>(T - t_first) * FF;
-    const long long pa = P * cta / grid, pb = P * (cta + 1) / grid;
-    long long pos = pa;
+    const int P = (T - t_first) * FF, pb = share(P, cta + 1);
+    int pos = share(P, cta);
     int issued = 0;
     bool down_issued = false;
     int round = 0;
@@ -474,9 +556,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         if (lane == 0) atomicExch(L.status, 2);
         return;
       }
-      const int tile = t_first + static_cast<int>(pos / FF);
-      const int pair0 = static_cast<int>(pos - static_cast<long long>(tile - t_first) * FF);
-      const int np = static_cast<int>(min(static_cast<long long>(kPairsStage), min(static_cast<long long>(FF - pair0), pb - pos)));
+      const int tile = t_first + pos / FF, pair0 = pos - (tile - t_first) * FF;
+      const int np = min(kPairsStage, min(FF - pair0, pb - pos));
       const int mode = tb.tile_mode[tile];
       unsigned char* st = ring + static_cast<size_t>(s) * G.stage_bytes;
       if (lane == 0) {
@@ -507,6 +588,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       issue_down_round(0);
       round = 1;
     }
+    grid_poll(2);
     for (; round < rounds; ++round) {               // later rounds reuse the region
       if (!mbar_wait(dn_empty, (round - 1) & 1)) {
         if (lane == 0) atomicExch(L.status, 2);
@@ -518,68 +600,47 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   }
 
   // ---------------- consumers ----------------
-  const bool bar_thread = tid == kConsumers - 1;
-  unsigned long long bar_base = 0;
-  if (bar_thread) bar_base = grid_base(gctr, grid);
+  const int nl = G.rows_per_cta;                 // warps 0 .. nl - 1: a router row each; the others fetch and quantise x
   // router rows of this CTA's experts: fixed weights, on their way before the previous kernel is awaited
-  if (warp < G.rows_per_cta) {
-    const int e = cta + warp * grid;
-    if (e < E) {
-      const float* src = L.router_w + static_cast<size_t>(e) * H;
-      float* dst = rw + static_cast<size_t>(warp) * H;
-      if ((reinterpret_cast<uintptr_t>(L.router_w) & 15u) == 0) {
-        for (int c = lane * 4; c < H; c += 128)
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + c)), "l"(src + c) : "memory");
-      } else {
-        for (int c = lane; c < H; c += 32) dst[c] = __ldg(src + c);
-      }
+  for (int i = 0; i < nl; ++i) {
+    const int e = cta + i * grid;
+    if (e >= E) break;
+    const float* src = L.router_w + static_cast<size_t>(e) * H;
+    float* dst = rw + static_cast<size_t>(i) * H;
+    if ((reinterpret_cast<uintptr_t>(L.router_w) & 15u) == 0) {
+      for (int c = tid * 4; c < H; c += kConsumers * 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + c)), "l"(src + c) : "memory");
+    } else {
+      for (int c = tid; c < H; c += kConsumers) dst[c] = __ldg(src + c);
     }
   }
   pdl_wait();
   pdl_launch_dependents();
   if (cta == 0 && tid == 0 && L.mail_n != nullptr) *L.mail_n = 0;
 
-  // The layer's pointer table (3 x E pointers: after the selection the experts' addresses are then
-  // one shared-memory read away) and the x rows: a warp fetches a 256-value block (16 bytes per
-  // lane), keeps it as fp16 for the logits and quantises it from its registers; up to four blocks'
-  // loads are in flight per warp.
+  // The layer's pointer table (3 x E pointers: after the selection the experts' addresses are then one shared-memory
+  // read away) and the x rows as fp16, copied by all threads.
   for (int i = tid; i < 3 * E; i += kConsumers) {
-    const int m = i / E, e = i - m * E;
-    ptab[i] = L.tab[static_cast<size_t>(m) * L.tab_stride + e];
+    const int m = i >= 2 * E ? 2 : (i >= E ? 1 : 0);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(ptab + i)), "l"(L.tab + static_cast<size_t>(m) * L.tab_stride + (i - m * E))
+                 : "memory");
   }
-  const XTile xt = xtile_at(smem + G.off_xt, kMaxTok, L.nbh);
-  if (tid == 0) {
-    tb.xt = xt;
-    tb.hq = xtile_at(smem + G.off_xh, kMaxHRows, L.nbf);
-  }
-  {
-    const int jobs = n * L.nbh;
-    for (int j0 = warp; j0 < jobs; j0 += 4 * kWarps) {
-      uint4 raw[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int job = min(j0 + u * kWarps, jobs - 1);
-        raw[u] = __ldcg(reinterpret_cast<const uint4*>(L.xn) + static_cast<size_t>(job) * 32 + lane);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int job = j0 + u * kWarps;
-        if (job >= jobs) break;                  // warp-uniform
-        reinterpret_cast<uint4*>(xh)[static_cast<size_t>(job) * 32 + lane] = raw[u];
-        quantize_f16_to_tile(xt, job / L.nbh, job % L.nbh, raw[u], lane);
-      }
-    }
-  }
+  const int jobs = n * L.nbh, xw = warp - nl, n_xw = kWarps - nl;
+  for (int i = tid; i < jobs * 32; i += kConsumers)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xh + i * 8)), "l"(L.xn + static_cast<size_t>(i) * 8) : "memory");
+  const HTile xt = {smem + G.off_xt, L.nbh};
   asm volatile("cp.async.wait_all;" ::: "memory");
-  consumers_sync();                              // x rows (both forms), router rows and tables are in place
-  // logits: one warp per expert row; lane l adds k = l, l + 32, ... in ascending order with FMA and
-  // the lanes meet in a shuffle tree - the order of the reference's kernel (src/kernels/cuda/q4_k.cu:133-149).
-  // Eight steps of loads are issued ahead of their FMAs.
-  if (warp < G.rows_per_cta) {
+  consumers_sync();                              // fp16 x rows, router rows and the pointer table are in place
+  bool ok = true;
+  if (warp < nl) {
+    // logits: one warp per expert row; lane l adds k = l, l + 32, ... in ascending order with FMA and
+    // the lanes meet in a shuffle tree - the order of the reference's kernel (src/kernels/cuda/q4_k.cu:133-149).
+    // Eight steps of loads are issued ahead of their FMAs.
     const int e = cta + warp * grid;
     if (e < E) {
       const float* wr = rw + static_cast<size_t>(warp) * H;
       float acc[kMaxTok] = {0.f, 0.f, 0.f, 0.f};
+      const float b = L.bias != nullptr ? __ldg(L.bias + e) : 0.f;
       int k = lane;
       for (; k + 7 * 32 < H; k += 8 * 32) {
         float wv[8];
@@ -602,7 +663,6 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         for (int t = 0; t < kMaxTok; ++t)
           if (t < n) acc[t] = fmaf(wv, h2f(xh[static_cast<size_t>(t) * H + k]), acc[t]);
       }
-      const float b = L.bias != nullptr ? L.bias[e] : 0.f;
 #pragma unroll
       for (int t = 0; t < kMaxTok; ++t) {
         float a = acc[t];
@@ -611,32 +671,49 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         if (lane == 0 && t < n) L.logits[static_cast<size_t>(t) * E + e] = a + b;
       }
     }
-  }
-  consumers_sync();
-  if (bar_thread) grid_arrive(gctr);                       // arrive now; the wait comes after the shared expert's gate / up
-
-  bool ok = true;
-  // the shared expert does not depend on the routing: its gate / up share runs while the other
-  // CTAs arrive at the barrier (tile 0: every row, h rows 0 .. n-1)
-  if (has_shared && sp1 > sp0) {
-    if (!mbar_wait(sh_full, 0)) ok = false;
-    if (ok) gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, &tb.xt, L.hbuf, FF, L.nbh, G.rb_h);
-  }
-  if (bar_thread) flag[0] = grid_wait(gctr, bar_base + grid) ? 1 : 0;
-  consumers_sync();
-  if (!flag[0]) {
-    if (tid == 0) atomicExch(L.status, 5);
-    return;
+    if (nl > 1) named_sync(7, nl * 32);
+    if (tid == 0) {
+      mbar_wait(based, 0);                       // (set at kernel start)
+      grid_arrive(gctr);
+    }
+  } else {
+#pragma unroll 1
+    for (int job = xw; job < jobs; job += n_xw) {
+      float v[8];
+      load_lane8(xh + static_cast<size_t>(job) * kQK, lane, v);
+      quantize_to_tile(xt.blk(0, job), v, lane);
+    }
+    named_sync(5, n_xw * 32);
+    // the shared expert does not depend on the routing: its gate / up share runs in the second group while the CTAs
+    // meet at the barrier (tile 0: every row, h rows 0 .. n-1)
+    if (warp >= kGroupWarps && has_shared && sp1 > sp0) {
+      if (!mbar_wait(sh_full, 0)) ok = false;
+      if (__all_sync(0xFFFFFFFFu, ok))
+        gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h);
+    }
   }
 
   // ---- selection (every CTA, the same result) and the tile tables ----
-  if (warp < n) {
-    float* pr = prob + static_cast<size_t>(warp) * E;
-    for (int i = lane; i < E; i += 32) pr[i] = __ldcg(L.logits + static_cast<size_t>(warp) * E + i);
-    __syncwarp();
-    router_select_warp(pr, E, K, tb.sel_idx[warp], tb.sel_w[warp], L.shared_w, true, lane);
+  const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
+  if (warp < 2 * kMaxTok && (warp & (kMaxTok - 1)) < n) {
+    const int t = warp & (kMaxTok - 1);
+    const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
+    const float* lg = L.logits + static_cast<size_t>(t) * E;
+    float* pr = prob + static_cast<size_t>(t) * E;
+    if (!there) {
+      ok = false;
+    } else if (by_pairs) {
+      select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane);
+    } else if (warp < kMaxTok) {
+      for (int i = lane; i < E; i += 32) pr[i] = __ldcg(lg + i);
+      __syncwarp();
+      select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
+    }
   }
-  consumers_sync();
+  if (!consumers_all(ok)) {
+    if (tid == 0) atomicExch(L.status, 5);
+    return;
+  }
   if (cta == 0 && tid < n * (K + 1)) {
     const int t = tid / (K + 1), kk = tid - t * (K + 1);
     if (kk < K) L.idx[static_cast<size_t>(t) * L.rstride + kk] = tb.sel_idx[t][kk];
@@ -716,41 +793,37 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   consumers_sync();
   const int T = tb.n_tiles;
 
-  // ---- phase 3: gate / up of the routed tiles, SwiGLU ----
+  // ---- phase 3: gate / up of the routed tiles, SwiGLU; the groups take stages in turn ----
   {
-    const long long P = static_cast<long long>(T - t_first) * FF;
-    const long long pa = P * cta / grid, pb = P * (cta + 1) / grid;
-    long long pos = pa;
+    const int P = (T - t_first) * FF, pb = share(P, cta + 1);
+    const int group = warp / kGroupWarps;
+    int pos = share(P, cta), pair0 = pos % FF;
     for (int i = 0; pos < pb && ok; ++i) {
-      const int s = i % kRing;
-      const unsigned ph = (i / kRing) & 1;
-      if (!mbar_wait(&full[s], ph)) {
-        ok = false;
-        break;
-      }
+      const int s = i % kRing, np = min(kPairsStage, min(FF - pair0, pb - pos));    // as the producer cuts the range
+      pos += np;
+      pair0 = pair0 + np == FF ? 0 : pair0 + np;
+      if ((i & 1) != group) continue;
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], (i / kRing) & 1)) != 0;
+      if (!ok) break;
       const StageDesc d = desc[s];
       if (d.mode != 1)
         gate_up_stage(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
-                      d.pair0, &tb.xt, L.hbuf, FF, L.nbh, G.rb_h);
+                      d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h);
       __syncwarp();
       if (lane == 0) mbar_arrive_one(&empty[s]);
-      pos += d.np;
     }
   }
   ok = consumers_all(ok);                                   // (a wait that ran out in any thread ends the CTA's work)
-  if (bar_thread) {
-    grid_arrive(gctr);
-    flag[1] = grid_wait(gctr, bar_base + 2ull * grid) ? 1 : 0;
-  }
-  consumers_sync();
-  if (!flag[1] || !ok) {
+  if (tid == 0) grid_arrive(gctr);
+  const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
+  if (!consumers_all(met && ok)) {
     if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
     return;
   }
 
   // ---- phase 4: quantise h (all rows, from L2), down rows of this CTA, combine in place ----
-  const XTile hq = tb.hq;
-  quantize_h_rows(hq, tb.n_hrows, L.hbuf, FF, warp, lane);
+  const HTile hq = {smem + G.off_xh, L.nbf};
+  quantize_h_rows(hq, tb.n_hrows, L.hbuf, warp, lane);
   consumers_sync();
   const int lpf = next_pow2_cap32(L.nbf);
   const int rounds = (T + kDownTiles - 1) / kDownTiles;
@@ -758,32 +831,28 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int j0 = rd * kDownTiles, j1 = min(T, j0 + kDownTiles);
     if (rd == 0 && has_shared && !mbar_wait(shdn_full, 0)) ok = false;
     if (ok && !mbar_wait(dn_full, rd & 1)) ok = false;
+    ok = __all_sync(0xFFFFFFFFu, ok) != 0;
     if (!ok) break;
-    const int tasks = (j1 - j0) * nr * lpf;
+    const int tasks = (j1 - j0) * nr * lpf * 2, row_lanes = __ffs(2 * lpf) - 1;
 #pragma unroll 1
     for (int base = 0; base < tasks; base += kConsumers) {
       const int q = base + tid;
-      const int lr = q & (lpf - 1);
-      const int jr = q / lpf;
+      const int half = q & 1, lr = (q >> 1) & (lpf - 1), blk = min(lr, L.nbf - 1);
+      const int jr = q >> row_lanes;
       const int js = jr / max(nr, 1), r = jr - js * nr;
       const int tile = min(j0 + js, T - 1);
       const bool live = q < tasks && tb.tile_mode[tile] != 1;
       const int hrow0 = tb.tile_hrow0[tile];
-      const RowSet rs = rows_of(live ? tb.tile_mask[tile] : 0, hrow0, false);   // h rows are stored per tile
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live) {
-        const unsigned char* row = dn + static_cast<size_t>(js) * G.slot_bytes + static_cast<size_t>(r) * G.rb_f;
-#pragma unroll 1
-        for (int blk = lr; blk < L.nbf; blk += lpf) {
-          const float4 v = block_dot_rows(reinterpret_cast<const uint4*>(row + blk * kW4), &tb.hq, blk, rs);
-          acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-        }
-      }
-      const float av[kMaxTok] = {acc.x, acc.y, acc.z, acc.w};
+      const RowSet rs = rows_of(live ? tb.tile_mask[tile] : 0, live ? hrow0 : 0, false);   // h rows are stored per tile
+      const int rows = __reduce_max_sync(0xFFFFFFFFu, rs.n);
+      const unsigned char* const w[1] = {dn + (live ? static_cast<size_t>(js) * G.slot_bytes + static_cast<size_t>(r) * G.rb_f + blk * kW4 : 0)};
+      float v[1][kMaxTok];
+      half_dots<1>(w, half, hq, blk, rs, rows, v);
 #pragma unroll
       for (int t = 0; t < kMaxTok; ++t) {
-        const float y = reduce_lanes(av[t], lpf);
-        if (live && lr == 0 && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
+        if (t >= rows) break;                    // warp-uniform
+        const float y = reduce_pairs(lr < L.nbf ? v[0][t] : 0.f, lpf);
+        if (live && half == 0 && lr == 0 && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
       }
     }
     __syncwarp();
