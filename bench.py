@@ -920,7 +920,7 @@ def decode_leg(ws, inputs, x0, biases, n, args, device, e2e, chain=False):
     ex_bytes = sum((u + 1) * EXPERT_BYTES for u in uniq)
     step_bytes = sum((u + 1) * EXPERT_BYTES + ROUTER_BYTES for u in uniq)
     peak, peak_kind = load_peaks()
-    if args.kernel is None and n <= 3:
+    if args.kernel is None and n <= 4:
         # one persistent launch per layer does everything (router, selection, experts, combine): the
         # launch is the layer, timed inside the step; its algorithmic bytes include the router matrix
         gbs = step_bytes / (ms_step * 1e-3) / 1e9

@@ -36,6 +36,7 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "api_util.cuh"
 #include "quantize_dev.cuh"
@@ -50,12 +51,10 @@ constexpr int kMaxRows = 64;       // token rows per call (row masks are 64-bit)
 constexpr int kTokTile = 8;        // token rows per tile of the item kernel (one MMA n-tile)
 constexpr int kMaxGrid = 192;            // most CTAs the expert kernels are launched with
 constexpr int kTmapSlots = 6;            // patched TMA descriptor sets per CTA of the row-streaming kernel
-#ifndef SGR_TKR
-#define SGR_TKR 4
-#endif
-constexpr int kTokenKernelMaxRows = SGR_TKR;   // layers of up to this many token rows run as one persistent launch
-                                         // (measured per layer, us: 26.6 / 36.1 / 44.7 against 30.1 / 39.6 / 47.3 for
-                                         // route + expert kernel; at 4 rows 57 against 50)
+constexpr int kTokenKernelMaxRows = 4;   // layers of up to this many token rows run as one persistent launch: all that its
+                                         // row sets hold (us per layer at 1 / 2 / 3 / 4 rows, 256 experts, hidden 2048,
+                                         // n_ff 512: 18.4 / 27.1 / 36.2 / 46.2, route + expert kernel 47.3 at 4; 128
+                                         // experts, hidden 1024: 34.5 against 36.7 at 4)
 constexpr int kRowsKernelMinRows = 4;    // layers of at least this many token rows run the row-streaming kernel
                                          // (measured: 4 rows 8 % faster, 8 rows 16 %, 2 rows slower)
 constexpr int kRouteTok = 8;       // token rows per CTA of the route kernel

@@ -140,14 +140,13 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // bounded: false when the others did not arrive in time.
 // The counter is read by the producer warp at kernel start - some multiple of the grid size plus the
 // arrivals of CTAs that are already further on, none of which can have passed the first barrier - so
-// barrier k of this launch completes at base + k * grid. An arrival is a fence and a fire-and-forget
+// barrier k of this launch completes at base + k * grid. An arrival is a fire-and-forget releasing
 // add by the thread whose warp finishes the work; the producer warp polls and passes the word on
 // through an mbarrier, so no consumer waits for a round trip that it could work through.
 __device__ __forceinline__ unsigned long long grid_base(const unsigned long long* ctr, unsigned grid) {
   return ld_acquire_u64(ctr) / grid * grid;
 }
 __device__ __forceinline__ void grid_arrive(unsigned long long* ctr) {
-  __threadfence();
   asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(ctr) : "memory");
 }
 __device__ __forceinline__ bool grid_wait(const unsigned long long* ctr, unsigned long long target) {
@@ -217,9 +216,10 @@ __device__ __forceinline__ RowSet rows_of(int mask, int base, bool by_bit) {
 // halves meet before the one rounding, so the terms are block_dot's). Whole warps call it: `rows` is the warp's
 // largest row count. Not unrolled over rows: every phase of this kernel runs once per CTA, so straight-line code is
 // paid for in instruction fetch.
-template <int NMAT>
+// `loaded()` runs once the weight bytes are in registers.
+template <int NMAT, typename Loaded>
 __device__ __forceinline__ void half_dots(const unsigned char* const (&w)[NMAT], int half, const HTile& xt, int blk, const RowSet& rs,
-                                          int rows, float (&out)[NMAT][kMaxTok]) {
+                                          int rows, float (&out)[NMAT][kMaxTok], Loaded loaded) {
   uint4 hdr[NMAT], wq[NMAT][4];
 #pragma unroll
   for (int m = 0; m < NMAT; ++m) {
@@ -228,6 +228,7 @@ __device__ __forceinline__ void half_dots(const unsigned char* const (&w)[NMAT],
 #pragma unroll
     for (int i = 0; i < 4; ++i) wq[m][i] = p[1 + 4 * half + i];
   }
+  loaded();
 #pragma unroll
   for (int m = 0; m < NMAT; ++m)
 #pragma unroll
@@ -284,8 +285,10 @@ __device__ __forceinline__ float reduce_pairs(float v, int lpr) {
 // Gate / up of `np` pairs staged at st (gate rows, then up rows) for the rows `mask` of one tile by a group of eight
 // warps: thread = (pair, block, half), both matrices. SwiGLU, fp32 h rows [hrow0 + slot][FF] to global memory.
 // (Inlined at both of its uses: as a function it saved and restored 2,400 warp registers per CTA through local memory.)
+// A warp arrives at `empty` (if given) as soon as its weight bytes are in registers: the stage's refill, a DRAM round
+// trip, then runs under the arithmetic.
 __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, int mask, int hrow0, int pair0,
-                                           const HTile& xt, float* hbuf, int FF, int nbh, int rb_h) {
+                                           const HTile& xt, float* hbuf, int FF, int nbh, int rb_h, uint64_t* empty) {
   const int tid = threadIdx.x & (kGroupThreads - 1);
   const int lpr = next_pow2_cap32(nbh), row_lanes = __ffs(2 * lpr) - 1;
   const RowSet rs = rows_of(mask, 0, true);
@@ -297,7 +300,12 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
     const unsigned char* row = st + static_cast<size_t>(pair) * rb_h + blk * kW4;
     const unsigned char* const w[2] = {row, row + static_cast<size_t>(np) * rb_h};
     float v[2][kMaxTok];
-    half_dots<2>(w, half, xt, blk, rs, rs.n, v);
+    half_dots<2>(w, half, xt, blk, rs, rs.n, v, [&] {
+      if (empty != nullptr && base + kGroupThreads >= tasks) {
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive_one(empty);
+      }
+    });
 #pragma unroll
     for (int t = 0; t < kMaxTok; ++t) {
       if (t >= rs.n) break;                        // uniform
@@ -353,23 +361,31 @@ __device__ __forceinline__ void select_pair(const float* logits, float* prob, Ta
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     if (lane + 32 * j >= E) e[j] = -1.f;
+  // a lane's eight in descending order (Batcher's network), then the warp takes the largest head K + 1 times
+  int sl[8] = {0, 1, 2, 3, 4, 5, 6, 7};
+  auto ce = [&](int a, int b) {
+    const bool sw = e[b] > e[a];
+    const float x = fmaxf(e[a], e[b]), y = fminf(e[a], e[b]);
+    const int i = sw ? sl[b] : sl[a], j = sw ? sl[a] : sl[b];
+    e[a] = x; e[b] = y; sl[a] = i; sl[b] = j;
+  };
+  ce(0, 1); ce(2, 3); ce(4, 5); ce(6, 7);
+  ce(0, 2); ce(1, 3); ce(4, 6); ce(5, 7);
+  ce(1, 2); ce(5, 6); ce(0, 4); ce(3, 7);
+  ce(1, 5); ce(2, 6);
+  ce(1, 4); ce(3, 6);
+  ce(2, 4); ce(3, 5);
+  ce(3, 4);
   float my_e = -1.f;
   int my_i = 0;
 #pragma unroll 1
   for (int kk = 0; kk <= K; ++kk) {
-    float v[4];
-    int s[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) { v[j] = fmaxf(e[2 * j], e[2 * j + 1]); s[j] = e[2 * j] >= e[2 * j + 1] ? 2 * j : 2 * j + 1; }
-    const int sa = v[0] >= v[1] ? s[0] : s[1], sb = v[2] >= v[3] ? s[2] : s[3];
-    const float va = fmaxf(v[0], v[1]), vb = fmaxf(v[2], v[3]), best = fmaxf(va, vb);
-    const int slot = va >= vb ? sa : sb;
-    const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(best));        // values are >= 0 or -1
-    const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(best) == top ? lane + 32 * slot : 0x7FFFFFFF);
+    const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(e[0]));        // values are >= 0 or -1
+    const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(e[0]) == top ? lane + 32 * sl[0] : 0x7FFFFFFF);
     if ((win & 31) == lane) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (j == (win >> 5)) e[j] = -1.f;
+      for (int j = 0; j < 7; ++j) { e[j] = e[j + 1]; sl[j] = sl[j + 1]; }
+      e[7] = -1.f;
     }
     if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
   }
@@ -639,37 +655,45 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int e = cta + warp * grid;
     if (e < E) {
       const float* wr = rw + static_cast<size_t>(warp) * H;
-      float acc[kMaxTok] = {0.f, 0.f, 0.f, 0.f};
       const float b = L.bias != nullptr ? __ldg(L.bias + e) : 0.f;
-      int k = lane;
-      for (; k + 7 * 32 < H; k += 8 * 32) {
-        float wv[8];
-        uint16_t xv[kMaxTok][8];
+      auto run = [&](auto rows) {                // NT token slots: what is predicated off still takes its issue slots
+        constexpr int NT = decltype(rows)::value;
+        float acc[NT];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          wv[j] = wr[k + 32 * j];
+        for (int t = 0; t < NT; ++t) acc[t] = 0.f;
+        int k = lane;
+#pragma unroll 1
+        for (; k + 7 * 32 < H; k += 8 * 32) {
+          float wv[8];
+          uint16_t xv[NT][8];
 #pragma unroll
-          for (int t = 0; t < kMaxTok; ++t) xv[t][j] = t < n ? xh[static_cast<size_t>(t) * H + k + 32 * j] : static_cast<uint16_t>(0);
+          for (int j = 0; j < 8; ++j) {
+            wv[j] = wr[k + 32 * j];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) xv[t][j] = xh[static_cast<size_t>(t < n ? t : 0) * H + k + 32 * j];
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[t] = fmaf(wv[j], h2f(xv[t][j]), acc[t]);
+        }
+#pragma unroll 1
+        for (; k < H; k += 32) {
+          const float wv = wr[k];
+#pragma unroll
+          for (int t = 0; t < NT; ++t) acc[t] = fmaf(wv, h2f(xh[static_cast<size_t>(t < n ? t : 0) * H + k]), acc[t]);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int t = 0; t < NT; ++t) {
+          float a = acc[t];
 #pragma unroll
-          for (int t = 0; t < kMaxTok; ++t)
-            if (t < n) acc[t] = fmaf(wv[j], h2f(xv[t][j]), acc[t]);
-      }
-      for (; k < H; k += 32) {
-        const float wv = wr[k];
-#pragma unroll
-        for (int t = 0; t < kMaxTok; ++t)
-          if (t < n) acc[t] = fmaf(wv, h2f(xh[static_cast<size_t>(t) * H + k]), acc[t]);
-      }
-#pragma unroll
-      for (int t = 0; t < kMaxTok; ++t) {
-        float a = acc[t];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, off);
-        if (lane == 0 && t < n) L.logits[static_cast<size_t>(t) * E + e] = a + b;
-      }
+          for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, off);
+          if (lane == 0 && t < n) L.logits[static_cast<size_t>(t) * E + e] = a + b;
+        }
+      };
+      if (n == 1) run(std::integral_constant<int, 1>{});
+      else if (n == 2) run(std::integral_constant<int, 2>{});
+      else run(std::integral_constant<int, kMaxTok>{});
     }
     if (nl > 1) named_sync(7, nl * 32);
     if (tid == 0) {
@@ -689,7 +713,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     if (warp >= kGroupWarps && has_shared && sp1 > sp0) {
       if (!mbar_wait(sh_full, 0)) ok = false;
       if (__all_sync(0xFFFFFFFFu, ok))
-        gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h);
+        gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, nullptr);
     }
   }
 
@@ -808,9 +832,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       const StageDesc d = desc[s];
       if (d.mode != 1)
         gate_up_stage(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
-                      d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h);
-      __syncwarp();
-      if (lane == 0) mbar_arrive_one(&empty[s]);
+                      d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h, &empty[s]);
+      else if (lane == 0) mbar_arrive_one(&empty[s]);
     }
   }
   ok = consumers_all(ok);                                   // (a wait that ran out in any thread ends the CTA's work)
@@ -847,7 +870,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       const int rows = __reduce_max_sync(0xFFFFFFFFu, rs.n);
       const unsigned char* const w[1] = {dn + (live ? static_cast<size_t>(js) * G.slot_bytes + static_cast<size_t>(r) * G.rb_f + blk * kW4 : 0)};
       float v[1][kMaxTok];
-      half_dots<1>(w, half, hq, blk, rs, rows, v);
+      half_dots<1>(w, half, hq, blk, rs, rows, v, [] {});
 #pragma unroll
       for (int t = 0; t < kMaxTok; ++t) {
         if (t >= rows) break;                    // warp-uniform

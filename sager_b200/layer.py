@@ -21,7 +21,7 @@ def _p(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
-# None = the library's choice (one persistent launch for up to three rows, else route + the expert kernel
+# None = the library's choice (one persistent launch for up to four rows, else route + the expert kernel
 # picked by row count); "two_launch" = route + expert kernel by row count; "rows" / "items" force one of them
 KERNEL_BITS = {None: 0, "rows": 16, "items": 32, "two_launch": 64}
 
@@ -101,9 +101,9 @@ class MoeStack:
         # per-layer routing records, so a finished step can be inspected
         self.idx = torch.zeros(len(layers), n_max, n_used + 1, dtype=torch.int32, device=device)
         self.w = torch.zeros(len(layers), n_max, n_used + 1, dtype=torch.float32, device=device)
-        # one persistent launch per layer for up to three rows, else route + experts
+        # one persistent launch per layer for up to four rows, else route + experts
         self._args = {}
-        self.launches_per_step = (1 if (kernel is None and n_max <= 3) else 2) * len(layers)
+        self.launches_per_step = (1 if (kernel is None and n_max <= 4) else 2) * len(layers)
         # chain: layer l's input rows are RMSNorm(x) computed on the device by rmsnorm_quant_f16 (the
         # producer of the MoE half's rows in the reference's decode layer, src/core/session.cpp:1020-1032),
         # so every layer depends on the residual its predecessor wrote
