@@ -27,8 +27,8 @@ __device__ __forceinline__ float quantize_lane8(const float (&v)[8], int (&q)[8]
   float a = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) a = fmaxf(a, fabsf(v[i]));
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) a = fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, off));
+  // (a >= 0 and never NaN: its bits order as integers, and the warp maximum is one instruction)
+  a = __int_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_int(a)));
   const float amax = fmaxf(1e-30f, a);
   const float d = amax / 127.f;
   const float id = d > 0.f ? 1.f / d : 0.f;

@@ -39,7 +39,7 @@ constexpr int kConsumers = kWarps * 32;
 constexpr int kGroupWarps = 8;             // ring stages alternate between two groups of consumer warps
 constexpr int kGroupThreads = kGroupWarps * 32;
 constexpr int kThreads = kConsumers + 32;  // + producer warp
-constexpr int kPairsStage = 16;            // (gate, up) row pairs per ring stage
+constexpr int kPairsStage = 16;            // (gate, up) row pairs per ring stage, at least
 constexpr int kRing = 2;
 constexpr int kDownTiles = 16;             // tiles whose down rows are resident at once
 constexpr int kMaxTiles = 33;              // n * K + 1 <= 33
@@ -81,7 +81,7 @@ struct Geom {
   int sp_max;            // shared-expert pairs per CTA
   int rb_h, rb_f;        // bytes per gate/up row, per down row
   size_t off_prob, off_ptab, off_xh, off_rw, off_xt, off_sh, off_ring, off_dn, off_y, total;
-  int stage_bytes, slot_bytes;
+  int stage_pairs, stage_bytes, slot_bytes;
 };
 __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int grid) {
   Geom g;
@@ -102,7 +102,11 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
   g.off_rw = g.off_xh + ((static_cast<size_t>(n) * H * 2 + 127) & ~static_cast<size_t>(127));
   g.off_xt = take(static_cast<size_t>(n) * (H / kQK) * kHBlk);
   g.off_sh = take(static_cast<size_t>(2) * g.sp_max * g.rb_h);
-  g.stage_bytes = 2 * kPairsStage * g.rb_h;
+  // as many pairs as a group of warps takes at once (narrow rows take few lanes each)
+  const int nbh = H / kQK;
+  const int lanes = nbh <= 1 ? 2 : (nbh <= 2 ? 4 : (nbh <= 4 ? 8 : (nbh <= 8 ? 16 : 32)));
+  g.stage_pairs = kGroupThreads / lanes > kPairsStage ? kGroupThreads / lanes : kPairsStage;
+  g.stage_bytes = 2 * g.stage_pairs * g.rb_h;
   g.off_ring = take(static_cast<size_t>(kRing) * g.stage_bytes);
   g.slot_bytes = g.nr_max * g.rb_f;
   g.off_dn = take(static_cast<size_t>(hrows < kDownTiles ? hrows : kDownTiles) * g.slot_bytes);
@@ -112,7 +116,7 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
 }
 
 // Named barriers of the consumers: 6 all of them, 7 the warps with router rows, 5 the warps that quantise, 8 .. 11 the
-// two warps that select for a token row.
+// two warps that select for a token row, 12 the warps that pick.
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 6, %0;" ::"n"(kConsumers) : "memory");
@@ -180,17 +184,16 @@ __device__ __forceinline__ void quantize_h_rows(const HTile& xt, int rows, const
   for (int j0 = warp; j0 < jobs; j0 += 2 * kWarps) {
     const float4* p = reinterpret_cast<const float4*>(src + static_cast<size_t>(j0) * kQK) + lane * 2;
     float4 x = __ldcg(p), y = __ldcg(p + 1), x2, y2;
-    const bool two = j0 + kWarps < jobs;
+    const bool two = j0 + kWarps < jobs;           // warp-uniform
     if (two) {
       x2 = __ldcg(p + kWarps * (kQK / 4));
       y2 = __ldcg(p + kWarps * (kQK / 4) + 1);
     }
-#pragma unroll 1
-    for (int u = 0; u < (two ? 2 : 1); ++u) {      // warp-uniform
-      const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-      quantize_to_tile(xt.blk(0, j0 + u * kWarps), v, lane);
-      x = x2;
-      y = y2;
+    const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    quantize_to_tile(xt.blk(0, j0), v, lane);
+    if (two) {
+      const float v2[8] = {x2.x, x2.y, x2.z, x2.w, y2.x, y2.y, y2.z, y2.w};
+      quantize_to_tile(xt.blk(0, j0 + kWarps), v2, lane);
     }
   }
 }
@@ -212,68 +215,86 @@ __device__ __forceinline__ RowSet rows_of(int mask, int base, bool by_bit) {
   return r;
 }
 
-// Half a super-block of NMAT weight rows against the rows of `rs` (a lane pair holds a block; the integer sums of the
-// halves meet before the one rounding, so the terms are block_dot's). Whole warps call it: `rows` is the warp's
-// largest row count. Not unrolled over rows: every phase of this kernel runs once per CTA, so straight-line code is
-// paid for in instruction fetch.
-// `loaded()` runs once the weight bytes are in registers.
-template <int NMAT, typename Loaded>
-__device__ __forceinline__ void half_dots(const unsigned char* const (&w)[NMAT], int half, const HTile& xt, int blk, const RowSet& rs,
-                                          int rows, float (&out)[NMAT][kMaxTok], Loaded loaded) {
-  uint4 hdr[NMAT], wq[NMAT][4];
+// Half a super-block of NMAT weight rows in registers: nibbles, the half's four scales and mins, and the block scales of
+// the matrix whose value this lane will hold (with two matrices the even lane of a pair ends with the first one's).
+template <int NMAT>
+struct HalfW {
+  uint4 q[NMAT][4];
+  uint32_t sc[NMAT], mn[NMAT];
+  float d, dmin;
+};
+template <int NMAT>
+__device__ __forceinline__ void load_half(HalfW<NMAT>& W, const unsigned char* const (&w)[NMAT], int half) {
+  uint32_t dd = 0;
 #pragma unroll
   for (int m = 0; m < NMAT; ++m) {
     const uint4* p = reinterpret_cast<const uint4*>(w[m]);
-    hdr[m] = p[0];
+    const uint4 hdr = p[0];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) wq[m][i] = p[1 + 4 * half + i];
+    for (int i = 0; i < 4; ++i) W.q[m][i] = p[1 + 4 * half + i];
+    const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
+    W.sc[m] = half ? s6.sc[1] : s6.sc[0];
+    W.mn[m] = half ? s6.mn[1] : s6.mn[0];
+    if (m == 0 || half) dd = hdr.x;
   }
-  loaded();
+  W.d = h2f(static_cast<uint16_t>(dd & 0xFFFFu));
+  W.dmin = h2f(static_cast<uint16_t>(dd >> 16));
+}
+// unsigned codes in the high nibbles against signed bytes: sixteen times the dot, without a shift per word
+__device__ __forceinline__ int dot8_high(const uint32_t (&w)[8], const uint4& a, const uint4& b) {
+  const uint32_t x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  int acc = 0;
 #pragma unroll
-  for (int m = 0; m < NMAT; ++m)
+  for (int i = 0; i < 8; ++i) asm("dp4a.u32.s32 %0, %1, %2, %0;" : "+r"(acc) : "r"(w[i] & 0xF0F0F0F0u), "r"(x[i]));
+  return acc;
+}
+
+// The half blocks W against the rows of `rs` (a lane pair holds a block; the integer sums of the halves meet before the
+// one rounding, so the terms are block_dot's). Bound by the integer pipe: with two matrices each lane of the pair sends
+// the sum it does not keep and both finish one matrix, which halves the shuffles and the arithmetic after them. Whole
+// warps call it: `rows` is the warp's largest row count. Not unrolled over rows: every phase of this kernel runs once
+// per CTA, so straight-line code is paid for in instruction fetch.
+template <int NMAT>
+__device__ __forceinline__ void half_dots(const HalfW<NMAT>& W, int half, const HTile& xt, int blk, const RowSet& rs, int rows,
+                                          float (&out)[kMaxTok]) {
 #pragma unroll
-    for (int t = 0; t < kMaxTok; ++t) out[m][t] = 0.f;
+  for (int t = 0; t < kMaxTok; ++t) out[t] = 0.f;
 #pragma unroll 1
   for (int t = 0; t < rows; ++t) {
     const unsigned char* xb = xt.blk(rs.at(t < rs.n ? t : 0), blk) + half * kHalf;
-    int isum[NMAT];
+    int lo_sum[NMAT], hi_sum[NMAT], is[NMAT], ms[NMAT];              // hi_sum: sixteen-fold, below 2^29
 #pragma unroll
-    for (int m = 0; m < NMAT; ++m) isum[m] = 0;
+    for (int m = 0; m < NMAT; ++m) lo_sum[m] = hi_sum[m] = 0;
 #pragma unroll
     for (int gg = 0; gg < 2; ++gg) {
       const uint4* xa = reinterpret_cast<const uint4*>(xb + 64 * gg);
       const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
 #pragma unroll
       for (int m = 0; m < NMAT; ++m) {
-        const uint4 q0 = wq[m][2 * gg], q1 = wq[m][2 * gg + 1];
+        const uint4 q0 = W.q[m][2 * gg], q1 = W.q[m][2 * gg + 1];
         const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        uint32_t lo[8], hi[8];
+        uint32_t lo[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          lo[i] = raw[i] & 0x0F0F0F0Fu;
-          hi[i] = (raw[i] >> 4) & 0x0F0F0F0Fu;
-        }
-        const Scales6 s6 = unpack_scales6(hdr[m].y, hdr[m].z, hdr[m].w);
-        const uint32_t scw = (half ? s6.sc[1] : s6.sc[0]) >> (16 * gg);
-        isum[m] += static_cast<int>(scw & 0xFF) * dot8(lo, x0, x1) + static_cast<int>((scw >> 8) & 0xFF) * dot8(hi, x2, x3);
+        for (int i = 0; i < 8; ++i) lo[i] = raw[i] & 0x0F0F0F0Fu;
+        const uint32_t scw = W.sc[m] >> (16 * gg);
+        lo_sum[m] += static_cast<int>(scw & 0xFF) * dot8(lo, x0, x1);
+        hi_sum[m] += static_cast<int>((scw >> 8) & 0xFF) * dot8_high(raw, x2, x3);
       }
     }
     const uint4 sd = *reinterpret_cast<const uint4*>(xb + 128);
 #pragma unroll
     for (int m = 0; m < NMAT; ++m) {
-      const Scales6 s6 = unpack_scales6(hdr[m].y, hdr[m].z, hdr[m].w);
-      const uint32_t mnw = half ? s6.mn[1] : s6.mn[0];
-      int msum = __dp2a_lo(static_cast<int>(sd.x), static_cast<int>(mnw), 0);
-      msum = __dp2a_hi(static_cast<int>(sd.y), static_cast<int>(mnw), msum);
-      const int is = isum[m] + __shfl_xor_sync(0xFFFFFFFFu, isum[m], 1);
-      const int ms = msum + __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
-      const float d = h2f(static_cast<uint16_t>(hdr[m].x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr[m].x >> 16));
-      const float v = __uint_as_float(sd.z) * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
-      if (t == 0) out[m][0] = v;
-      else if (t == 1) out[m][1] = v;
-      else if (t == 2) out[m][2] = v;
-      else out[m][3] = v;
+      is[m] = lo_sum[m] + (hi_sum[m] >> 4);
+      ms[m] = __dp2a_hi(static_cast<int>(sd.y), static_cast<int>(W.mn[m]), __dp2a_lo(static_cast<int>(sd.x), static_cast<int>(W.mn[m]), 0));
     }
+    const int other_is = NMAT == 1 || !half ? is[NMAT - 1] : is[0], other_ms = NMAT == 1 || !half ? ms[NMAT - 1] : ms[0];
+    const int my_is = (half ? is[NMAT - 1] : is[0]) + __shfl_xor_sync(0xFFFFFFFFu, other_is, 1);
+    const int my_ms = (half ? ms[NMAT - 1] : ms[0]) + __shfl_xor_sync(0xFFFFFFFFu, other_ms, 1);
+    const float v = __uint_as_float(sd.z) * (W.d * static_cast<float>(my_is) - W.dmin * static_cast<float>(my_ms));
+    if (t == 0) out[0] = v;
+    else if (t == 1) out[1] = v;
+    else if (t == 2) out[2] = v;
+    else out[3] = v;
   }
 }
 // sum over the blocks of a row, held by lane pairs `2 * lpr` lanes wide, in the order of reduce_lanes
@@ -286,30 +307,36 @@ __device__ __forceinline__ float reduce_pairs(float v, int lpr) {
 // warps: thread = (pair, block, half), both matrices. SwiGLU, fp32 h rows [hrow0 + slot][FF] to global memory.
 // (Inlined at both of its uses: as a function it saved and restored 2,400 warp registers per CTA through local memory.)
 // A warp arrives at `empty` (if given) as soon as its weight bytes are in registers: the stage's refill, a DRAM round
-// trip, then runs under the arithmetic.
+// trip, then runs under the arithmetic. Warps without a pair only arrive.
 __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, int mask, int hrow0, int pair0,
-                                           const HTile& xt, float* hbuf, int FF, int nbh, int rb_h, uint64_t* empty) {
-  const int tid = threadIdx.x & (kGroupThreads - 1);
-  const int lpr = next_pow2_cap32(nbh), row_lanes = __ffs(2 * lpr) - 1;
+                                           const HTile& xt, float* hbuf, int FF, int nbh, int rb_h, int row_lanes, uint64_t* empty) {
+  const int tid = threadIdx.x & (kGroupThreads - 1), lane = tid & 31;
+  const int lpr = 1 << (row_lanes - 1);
   const RowSet rs = rows_of(mask, 0, true);
   const int tasks = np << row_lanes;
+  if ((tid & ~31) >= tasks) {
+    if (empty != nullptr && lane == 0) mbar_arrive_one(empty);
+    return;
+  }
+  const int half = tid & 1, lr = (tid >> 1) & (lpr - 1), blk = min(lr, nbh - 1);
 #pragma unroll 1
-  for (int base = 0; base < tasks; base += kGroupThreads) {        // uniform trip count
-    const int q = base + tid;
-    const int half = q & 1, lr = (q >> 1) & (lpr - 1), pair = min(q >> row_lanes, np - 1), blk = min(lr, nbh - 1);
-    const unsigned char* row = st + static_cast<size_t>(pair) * rb_h + blk * kW4;
-    const unsigned char* const w[2] = {row, row + static_cast<size_t>(np) * rb_h};
-    float v[2][kMaxTok];
-    half_dots<2>(w, half, xt, blk, rs, rs.n, v, [&] {
-      if (empty != nullptr && base + kGroupThreads >= tasks) {
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) mbar_arrive_one(empty);
-      }
-    });
+  for (int q = tid; (q & ~31) < tasks; q += kGroupThreads) {        // warp-uniform
+    const int pair = min(q >> row_lanes, np - 1);
+    const unsigned char* row = st + pair * rb_h + blk * kW4;
+    const unsigned char* const w[2] = {row, row + np * rb_h};
+    HalfW<2> W;
+    load_half<2>(W, w, half);
+    if (empty != nullptr && ((q + kGroupThreads) & ~31) >= tasks) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive_one(empty);
+    }
+    float v[kMaxTok];
+    half_dots<2>(W, half, xt, blk, rs, rs.n, v);
 #pragma unroll
     for (int t = 0; t < kMaxTok; ++t) {
       if (t >= rs.n) break;                        // uniform
-      const float g = reduce_pairs(lr < nbh ? v[0][t] : 0.f, lpr), u = reduce_pairs(lr < nbh ? v[1][t] : 0.f, lpr);
+      const float g = reduce_pairs(lr < nbh ? v[t] : 0.f, lpr);
+      const float u = __shfl_down_sync(0xFFFFFFFFu, g, 1);          // the odd lanes hold the up row
       if (q < tasks && half == 0 && lr == 0) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(g, u);
     }
   }
@@ -323,8 +350,10 @@ __device__ __noinline__ void select_general(float* prob, int E, int K, int* idx,
 // exponentials - the reference's order - is most of it, so one warp adds while the other picks the K + 1 largest
 // exponentials. Dividing by the sum keeps their order; only if it makes two of them equal, or something is not
 // finite, the order of the quotients could be another one, and the general selection on the quotients is run.
-__device__ __forceinline__ void select_pair(const float* logits, float* prob, Tables& tb, int t, bool adds, int E, int K, float shared_w,
-                                            int lane) {
+// `picked(lane's expert)` runs between the picks and the wait for the sum: they stand unless the function returns true.
+template <typename Picked>
+__device__ __forceinline__ bool select_pair(const float* logits, float* prob, Tables& tb, int t, bool adds, int E, int K, float shared_w,
+                                            int lane, Picked picked) {
   float e[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) e[j] = lane + 32 * j < E ? __ldcg(logits + lane + 32 * j) : -1e30f;
@@ -356,7 +385,7 @@ __device__ __forceinline__ void select_pair(const float* logits, float* prob, Ta
     }
     __syncwarp();
     named_sync(8 + t, 64);
-    return;
+    return false;
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j)
@@ -389,6 +418,9 @@ __device__ __forceinline__ void select_pair(const float* logits, float* prob, Ta
     }
     if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
   }
+  my_i = min(my_i, E - 1);                       // (with NaNs about, a lane's filler could be picked: not fine below)
+  if (lane < K) tb.sel_idx[t][lane] = my_i;
+  picked(my_i);
   named_sync(8 + t, 64);
   const float z = tb.z[t];
   const float p = my_e / z;
@@ -397,16 +429,14 @@ __device__ __forceinline__ void select_pair(const float* logits, float* prob, Ta
   if (fine) {
     float wsum = 0.f;
     for (int kk = 0; kk < K; ++kk) wsum += __shfl_sync(0xFFFFFFFFu, p, kk);
-    if (lane < K) {
-      tb.sel_idx[t][lane] = my_i;
-      tb.sel_w[t][lane] = wsum > 0.f ? p / wsum : p;
-    }
+    if (lane < K) tb.sel_w[t][lane] = wsum > 0.f ? p / wsum : p;
     if (lane == 0) tb.sel_w[t][K] = shared_w;
   } else {
     for (int i = lane; i < E; i += 32) prob[i] = __ldcg(logits + i);
     __syncwarp();
     select_general(prob, E, K, tb.sel_idx[t], tb.sel_w[t], shared_w, lane);
   }
+  return !fine;
 }
 
 // Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned.
@@ -461,6 +491,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     mbar_init(ready, 1);
     mbar_init(based, 1);
     mbar_init(passed, 1);
+    flag[2] = 0;                                 // a row's picks did not stand
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -526,6 +557,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     // routed gate / up pairs: a flat range of (tile, pair) per CTA
     const int P = (T - t_first) * FF, pb = share(P, cta + 1);
     int pos = share(P, cta);
+    const int cut = min(G.stage_pairs, (pb - pos + 1) / 2);          // both groups get work
     int issued = 0;
     bool down_issued = false;
     int round = 0;
@@ -573,7 +605,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         return;
       }
       const int tile = t_first + pos / FF, pair0 = pos - (tile - t_first) * FF;
-      const int np = min(kPairsStage, min(FF - pair0, pb - pos));
+      const int np = min(cut, min(FF - pair0, pb - pos));
       const int mode = tb.tile_mode[tile];
       unsigned char* st = ring + static_cast<size_t>(s) * G.stage_bytes;
       if (lane == 0) {
@@ -616,6 +648,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   }
 
   // ---------------- consumers ----------------
+  const int row_lanes = __ffs(2 * next_pow2_cap32(L.nbh)) - 1;
   const int nl = G.rows_per_cta;                 // warps 0 .. nl - 1: a router row each; the others fetch and quantise x
   // router rows of this CTA's experts: fixed weights, on their way before the previous kernel is awaited
   for (int i = 0; i < nl; ++i) {
@@ -713,38 +746,15 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     if (warp >= kGroupWarps && has_shared && sp1 > sp0) {
       if (!mbar_wait(sh_full, 0)) ok = false;
       if (__all_sync(0xFFFFFFFFu, ok))
-        gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, nullptr);
+        gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, nullptr);
     }
   }
 
   // ---- selection (every CTA, the same result) and the tile tables ----
-  const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
-  if (warp < 2 * kMaxTok && (warp & (kMaxTok - 1)) < n) {
-    const int t = warp & (kMaxTok - 1);
-    const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
-    const float* lg = L.logits + static_cast<size_t>(t) * E;
-    float* pr = prob + static_cast<size_t>(t) * E;
-    if (!there) {
-      ok = false;
-    } else if (by_pairs) {
-      select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane);
-    } else if (warp < kMaxTok) {
-      for (int i = lane; i < E; i += 32) pr[i] = __ldcg(lg + i);
-      __syncwarp();
-      select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
-    }
-  }
-  if (!consumers_all(ok)) {
-    if (tid == 0) atomicExch(L.status, 5);
-    return;
-  }
-  if (cta == 0 && tid < n * (K + 1)) {
-    const int t = tid / (K + 1), kk = tid - t * (K + 1);
-    if (kk < K) L.idx[static_cast<size_t>(t) * L.rstride + kk] = tb.sel_idx[t][kk];
-    L.w[static_cast<size_t>(t) * L.rstride + kk] = tb.sel_w[t][kk];
-  }
+  // The picks need no sum, so the tables and the fetch of the picked experts into L2 run while the other warps add. The
+  // rare row whose picks do not stand after the division has the tables built once more.
   const int t_first = has_shared ? 1 : 0;
-  if (warp == 0) {
+  auto build = [&] {
     // one lane per pick (n * K <= 32): picks of the same expert find each other with a match,
     // the lowest lane of a group founds the tile; tiles are numbered in pick order
     const int picks = n * K;
@@ -775,10 +785,6 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       tb.tile_mask[my_tile] = mask;
       tb.w[0][my_tile] = w0; tb.w[1][my_tile] = w1; tb.w[2][my_tile] = w2;
       tb.tile_mode[my_tile] = absent ? 1 : (aligned ? 0 : 2);
-      if (absent && cta == 0 && L.mail != nullptr) {
-        const int mi = atomicAdd(L.mail_n, 1);
-        if (mi < E) L.mail[mi] = e;
-      }
     }
     const int T = t_first + __popc(leaders);
     __syncwarp();
@@ -809,12 +815,58 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     }
     if (lane < n) tb.route_hrow[lane][K] = has_shared ? lane : -1;
     __syncwarp();
-    if (lane == 0) {
-      __threadfence_block();
-      mbar_arrive_one(ready);                   // the producer may issue every weight copy now
+  };
+  // this CTA's slice of the three matrices of a picked expert, whichever CTA reads it later
+  auto fetch = [&](int e) {
+    if (lane >= K) return;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const unsigned char* w = ptab[m * E + e];
+      const int units = m < 2 ? FF * (G.rb_h / 16) : H * (G.rb_f / 16);
+      const int u0 = share(units, cta), u1 = share(units, cta + 1);
+      if (w != nullptr && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && u1 > u0)
+        bulk_prefetch_l2(w + static_cast<size_t>(u0) * 16, static_cast<uint32_t>(u1 - u0) * 16);
+    }
+  };
+  const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
+  if (warp < 2 * kMaxTok && (warp & (kMaxTok - 1)) < n) {
+    const int t = warp & (kMaxTok - 1);
+    const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
+    const float* lg = L.logits + static_cast<size_t>(t) * E;
+    float* pr = prob + static_cast<size_t>(t) * E;
+    if (!there) ok = false;                      // (the named barriers below need every warp: it goes on with what is there)
+    if (by_pairs) {
+      const bool redo = select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane, [&](int e) {
+        fetch(e);
+        if (n > 1) named_sync(12, n * 32);       // every row's picks are in the tables
+        else __syncwarp();
+        if (warp == 0) build();
+      });
+      if (redo && lane == 0) *reinterpret_cast<volatile int*>(flag + 2) = 1;
+    } else if (warp < kMaxTok && there) {
+      for (int i = lane; i < E; i += 32) pr[i] = __ldcg(lg + i);
+      __syncwarp();
+      select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
     }
   }
-  consumers_sync();
+  if (!consumers_all(ok)) {
+    if (tid == 0) atomicExch(L.status, 5);
+    return;
+  }
+  if (!by_pairs || *reinterpret_cast<volatile int*>(flag + 2) != 0) {
+    if (warp == 0) build();
+    consumers_sync();
+  }
+  if (tid == 0) mbar_arrive_one(ready);          // the producer may issue every weight copy now
+  if (cta == 0 && tid < n * (K + 1)) {
+    const int t = tid / (K + 1), kk = tid - t * (K + 1);
+    if (kk < K) L.idx[static_cast<size_t>(t) * L.rstride + kk] = tb.sel_idx[t][kk];
+    L.w[static_cast<size_t>(t) * L.rstride + kk] = tb.sel_w[t][kk];
+  }
+  if (cta == 0 && L.mail != nullptr && tid >= t_first && tid < tb.n_tiles && tb.tile_mode[tid] == 1) {
+    const int mi = atomicAdd(L.mail_n, 1);
+    if (mi < E) L.mail[mi] = tb.tile_e[tid];
+  }
   const int T = tb.n_tiles;
 
   // ---- phase 3: gate / up of the routed tiles, SwiGLU; the groups take stages in turn ----
@@ -822,8 +874,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int P = (T - t_first) * FF, pb = share(P, cta + 1);
     const int group = warp / kGroupWarps;
     int pos = share(P, cta), pair0 = pos % FF;
+    const int cut = min(G.stage_pairs, (pb - pos + 1) / 2);
     for (int i = 0; pos < pb && ok; ++i) {
-      const int s = i % kRing, np = min(kPairsStage, min(FF - pair0, pb - pos));    // as the producer cuts the range
+      const int s = i % kRing, np = min(cut, min(FF - pair0, pb - pos));    // as the producer cuts the range
       pos += np;
       pair0 = pair0 + np == FF ? 0 : pair0 + np;
       if ((i & 1) != group) continue;
@@ -832,52 +885,61 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       const StageDesc d = desc[s];
       if (d.mode != 1)
         gate_up_stage(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
-                      d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h, &empty[s]);
+                      d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, &empty[s]);
       else if (lane == 0) mbar_arrive_one(&empty[s]);
     }
   }
   ok = consumers_all(ok);                                   // (a wait that ran out in any thread ends the CTA's work)
   if (tid == 0) grid_arrive(gctr);
-  const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
-  if (!consumers_all(met && ok)) {
-    if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
-    return;
-  }
 
   // ---- phase 4: quantise h (all rows, from L2), down rows of this CTA, combine in place ----
   const HTile hq = {smem + G.off_xh, L.nbf};
-  quantize_h_rows(hq, tb.n_hrows, L.hbuf, warp, lane);
-  consumers_sync();
-  const int lpf = next_pow2_cap32(L.nbf);
+  const int f_lanes = __ffs(2 * next_pow2_cap32(L.nbf)) - 1, lpf = 1 << (f_lanes - 1);
+  const int f_half = tid & 1, f_lr = (tid >> 1) & (lpf - 1), f_blk = min(f_lr, L.nbf - 1);
   const int rounds = (T + kDownTiles - 1) / kDownTiles;
+  bool first = true;
+#pragma unroll 1
   for (int rd = 0; rd < rounds && ok; ++rd) {
     const int j0 = rd * kDownTiles, j1 = min(T, j0 + kDownTiles);
     if (rd == 0 && has_shared && !mbar_wait(shdn_full, 0)) ok = false;
     if (ok && !mbar_wait(dn_full, rd & 1)) ok = false;
     ok = __all_sync(0xFFFFFFFFu, ok) != 0;
-    if (!ok) break;
-    const int tasks = (j1 - j0) * nr * lpf * 2, row_lanes = __ffs(2 * lpf) - 1;
+    const int tasks = (j1 - j0) * nr << f_lanes;
+    int base = 0;
 #pragma unroll 1
-    for (int base = 0; base < tasks; base += kConsumers) {
+    do {
+      // a task's weights go into registers first, at the first task while the other CTAs finish their gate / up
       const int q = base + tid;
-      const int half = q & 1, lr = (q >> 1) & (lpf - 1), blk = min(lr, L.nbf - 1);
-      const int jr = q >> row_lanes;
+      const int jr = q >> f_lanes;
       const int js = jr / max(nr, 1), r = jr - js * nr;
       const int tile = min(j0 + js, T - 1);
       const bool live = q < tasks && tb.tile_mode[tile] != 1;
       const int hrow0 = tb.tile_hrow0[tile];
       const RowSet rs = rows_of(live ? tb.tile_mask[tile] : 0, live ? hrow0 : 0, false);   // h rows are stored per tile
       const int rows = __reduce_max_sync(0xFFFFFFFFu, rs.n);
-      const unsigned char* const w[1] = {dn + (live ? static_cast<size_t>(js) * G.slot_bytes + static_cast<size_t>(r) * G.rb_f + blk * kW4 : 0)};
-      float v[1][kMaxTok];
-      half_dots<1>(w, half, hq, blk, rs, rows, v, [] {});
+      const unsigned char* const w[1] = {dn + (live ? js * G.slot_bytes + r * G.rb_f + f_blk * kW4 : 0)};
+      HalfW<1> W;
+      load_half<1>(W, w, f_half);
+      if (first) {
+        first = false;
+        const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
+        if (!consumers_all(met && ok)) {
+          if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
+          return;
+        }
+        quantize_h_rows(hq, tb.n_hrows, L.hbuf, warp, lane);
+        consumers_sync();
+      }
+      float v[kMaxTok];
+      half_dots<1>(W, f_half, hq, f_blk, rs, rows, v);
 #pragma unroll
       for (int t = 0; t < kMaxTok; ++t) {
         if (t >= rows) break;                    // warp-uniform
-        const float y = reduce_pairs(lr < L.nbf ? v[0][t] : 0.f, lpf);
-        if (live && half == 0 && lr == 0 && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
+        const float y = reduce_pairs(f_lr < L.nbf ? v[t] : 0.f, lpf);
+        if (live && f_half == 0 && f_lr == 0 && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
       }
-    }
+      base += kConsumers;
+    } while (base < tasks && ok);
     __syncwarp();
     if (lane == 0 && rd + 1 < rounds) mbar_arrive_one(dn_empty);
   }
