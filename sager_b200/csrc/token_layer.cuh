@@ -67,7 +67,7 @@ struct Tables {                            // built after the selection, the sam
   int sel_idx[kMaxTok][kMaxTiles];         // [t][0..K]
   float sel_w[kMaxTok][kMaxTiles];
   int route_hrow[kMaxTok][kMaxTiles];      // [t][kk] -> h / y row of that route, -1 = absent; [t][K] = shared
-  float z[kMaxTok];                        // softmax denominators
+  float pick_e[kMaxTok][32];               // the K + 1 largest exponentials
 };
 static_assert(sizeof(Tables) <= kTables, "tables region");
 
@@ -347,10 +347,10 @@ __device__ __noinline__ void select_general(float* prob, int E, int K, int* idx,
 }
 
 // Softmax and top-K of one token row by two warps (up to 256 experts, K < 32). The strictly serial sum of the
-// exponentials - the reference's order - is most of it, so one warp adds while the other picks the K + 1 largest
-// exponentials. Dividing by the sum keeps their order; only if it makes two of them equal, or something is not
-// finite, the order of the quotients could be another one, and the general selection on the quotients is run.
-// `picked(lane's expert)` runs between the picks and the wait for the sum: they stand unless the function returns true.
+// exponentials - the reference's order - is long, so one warp picks the K + 1 largest exponentials and goes on to build
+// the tables from them (`picked(lane's expert)`) while the other adds and makes the weights. Dividing by the sum keeps
+// the order; only if it makes two of them equal, or something is not finite, the order of the quotients could be another
+// one, and the adding warp runs the general selection on the quotients: it returns true, and the picks do not stand.
 template <typename Picked>
 __device__ __forceinline__ bool select_pair(const float* logits, float* prob, Tables& tb, int t, bool adds, int E, int K, float shared_w,
                                             int lane, Picked picked) {
@@ -367,62 +367,60 @@ __device__ __forceinline__ bool select_pair(const float* logits, float* prob, Ta
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) e[j] = expf(e[j] - mx);
-  if (adds) {
+  if (!adds) {
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-      if (lane + 32 * j < E) prob[lane + 32 * j] = e[j];
-    __syncwarp();
-    if (lane == 0) {
-      float z = 0.f;
-      int i = 0;
-#pragma unroll 4
-      for (; i + 8 <= E; i += 8) {
-        const float4 a = *reinterpret_cast<const float4*>(prob + i), b = *reinterpret_cast<const float4*>(prob + i + 4);
-        z += a.x; z += a.y; z += a.z; z += a.w; z += b.x; z += b.y; z += b.z; z += b.w;
+      if (lane + 32 * j >= E) e[j] = -1.f;
+    // a lane's eight in descending order (Batcher's network), then the warp takes the largest head K + 1 times
+    int sl[8] = {0, 1, 2, 3, 4, 5, 6, 7};
+    auto ce = [&](int a, int b) {
+      const bool sw = e[b] > e[a];
+      const float x = fmaxf(e[a], e[b]), y = fminf(e[a], e[b]);
+      const int i = sw ? sl[b] : sl[a], j = sw ? sl[a] : sl[b];
+      e[a] = x; e[b] = y; sl[a] = i; sl[b] = j;
+    };
+    ce(0, 1); ce(2, 3); ce(4, 5); ce(6, 7);
+    ce(0, 2); ce(1, 3); ce(4, 6); ce(5, 7);
+    ce(1, 2); ce(5, 6); ce(0, 4); ce(3, 7);
+    ce(1, 5); ce(2, 6);
+    ce(1, 4); ce(3, 6);
+    ce(2, 4); ce(3, 5);
+    ce(3, 4);
+    float my_e = -1.f;
+    int my_i = 0;
+#pragma unroll 1
+    for (int kk = 0; kk <= K; ++kk) {
+      const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(e[0]));        // values are >= 0 or -1
+      const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(e[0]) == top ? lane + 32 * sl[0] : 0x7FFFFFFF);
+      if ((win & 31) == lane) {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) { e[j] = e[j + 1]; sl[j] = sl[j + 1]; }
+        e[7] = -1.f;
       }
-      for (; i < E; ++i) z += prob[i];
-      tb.z[t] = z;
+      if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
     }
+    my_i = min(my_i, E - 1);                     // (with NaNs about, a lane's filler could be picked: not fine below)
+    if (lane < K) tb.sel_idx[t][lane] = my_i;
+    if (lane <= K) tb.pick_e[t][lane] = my_e;
     __syncwarp();
-    named_sync(8 + t, 64);
+    asm volatile("bar.arrive %0, 64;" ::"r"(8 + t) : "memory");
+    picked(my_i);
     return false;
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    if (lane + 32 * j >= E) e[j] = -1.f;
-  // a lane's eight in descending order (Batcher's network), then the warp takes the largest head K + 1 times
-  int sl[8] = {0, 1, 2, 3, 4, 5, 6, 7};
-  auto ce = [&](int a, int b) {
-    const bool sw = e[b] > e[a];
-    const float x = fmaxf(e[a], e[b]), y = fminf(e[a], e[b]);
-    const int i = sw ? sl[b] : sl[a], j = sw ? sl[a] : sl[b];
-    e[a] = x; e[b] = y; sl[a] = i; sl[b] = j;
-  };
-  ce(0, 1); ce(2, 3); ce(4, 5); ce(6, 7);
-  ce(0, 2); ce(1, 3); ce(4, 6); ce(5, 7);
-  ce(1, 2); ce(5, 6); ce(0, 4); ce(3, 7);
-  ce(1, 5); ce(2, 6);
-  ce(1, 4); ce(3, 6);
-  ce(2, 4); ce(3, 5);
-  ce(3, 4);
-  float my_e = -1.f;
-  int my_i = 0;
-#pragma unroll 1
-  for (int kk = 0; kk <= K; ++kk) {
-    const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(e[0]));        // values are >= 0 or -1
-    const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(e[0]) == top ? lane + 32 * sl[0] : 0x7FFFFFFF);
-    if ((win & 31) == lane) {
-#pragma unroll
-      for (int j = 0; j < 7; ++j) { e[j] = e[j + 1]; sl[j] = sl[j + 1]; }
-      e[7] = -1.f;
-    }
-    if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
+    if (lane + 32 * j < E) prob[lane + 32 * j] = e[j];
+  __syncwarp();
+  float z = 0.f;                                 // every lane adds: the same broadcast reads
+  int i = 0;
+#pragma unroll 4
+  for (; i + 8 <= E; i += 8) {
+    const float4 a = *reinterpret_cast<const float4*>(prob + i), b = *reinterpret_cast<const float4*>(prob + i + 4);
+    z += a.x; z += a.y; z += a.z; z += a.w; z += b.x; z += b.y; z += b.z; z += b.w;
   }
-  my_i = min(my_i, E - 1);                       // (with NaNs about, a lane's filler could be picked: not fine below)
-  if (lane < K) tb.sel_idx[t][lane] = my_i;
-  picked(my_i);
+  for (; i < E; ++i) z += prob[i];
   named_sync(8 + t, 64);
-  const float z = tb.z[t];
+  const float my_e = lane <= K ? tb.pick_e[t][lane] : -1.f;
   const float p = my_e / z;
   const float next = __shfl_down_sync(0xFFFFFFFFu, p, 1);
   const bool fine = z > 0.f && z <= 3.4e38f && __all_sync(0xFFFFFFFFu, lane >= K || (my_e >= 0.f && p > next));
@@ -432,7 +430,8 @@ __device__ __forceinline__ bool select_pair(const float* logits, float* prob, Ta
     if (lane < K) tb.sel_w[t][lane] = wsum > 0.f ? p / wsum : p;
     if (lane == 0) tb.sel_w[t][K] = shared_w;
   } else {
-    for (int i = lane; i < E; i += 32) prob[i] = __ldcg(logits + i);
+    __syncwarp();
+    for (int m = lane; m < E; m += 32) prob[m] = __ldcg(logits + m);
     __syncwarp();
     select_general(prob, E, K, tb.sel_idx[t], tb.sel_w[t], shared_w, lane);
   }
@@ -475,10 +474,15 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
 
   // this CTA's shares: shared-expert pairs [sp0, sp1), output rows [r0, r1)
   // (products stay below 2^31: at most 33 tiles x 8192 pairs x 192 CTAs)
-  auto share = [&](int total, int part) { return static_cast<int>(static_cast<unsigned>(total) * static_cast<unsigned>(part) / static_cast<unsigned>(grid)); };
+  const unsigned grid_inv = 0xFFFFFFFFu / static_cast<unsigned>(grid);
+  auto share = [&](int total, int part) {        // total * part / grid: the estimate is at most one short
+    const unsigned x = static_cast<unsigned>(total) * static_cast<unsigned>(part), q = __umulhi(x, grid_inv);
+    return static_cast<int>(q + (x - q * static_cast<unsigned>(grid) >= static_cast<unsigned>(grid) ? 1u : 0u));
+  };
   const int sp0 = share(FF, cta), sp1 = share(FF, cta + 1), r0 = share(H, cta), r1 = share(H, cta + 1);
   const int nr = r1 - r0;
 
+  const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
   if (tid == 0) {
     for (int s = 0; s < kRing; ++s) {
       mbar_init(&full[s], 1);
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     mbar_init(shdn_full, 1);
     mbar_init(dn_full, 1);
     mbar_init(dn_empty, kWarps);
-    mbar_init(ready, 1);
+    mbar_init(ready, by_pairs ? n + 1 : 1);      // tables built, and every row's picks found to stand (or not: flag[2])
     mbar_init(based, 1);
     mbar_init(passed, 1);
     flag[2] = 0;                                 // a row's picks did not stand
@@ -548,7 +552,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       __syncwarp();
     };
     grid_poll(1);
-    if (!mbar_wait(ready, 0)) {
+    bool built = mbar_wait(ready, 0);
+    if (built && by_pairs && *reinterpret_cast<volatile int*>(flag + 2) != 0) built = mbar_wait(ready, 1);
+    if (!built) {
       if (lane == 0 && flag[0]) atomicExch(L.status, 7);
       return;
     }
@@ -757,92 +763,86 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   auto build = [&] {
     // one lane per pick (n * K <= 32): picks of the same expert find each other with a match,
     // the lowest lane of a group founds the tile; tiles are numbered in pick order
-    const int picks = n * K;
-    const bool live = lane < picks;
-    const int pt = live ? lane / K : 0, pk = live ? lane - pt * K : 0;
+    const bool live = lane < n * K;
+    const int pt = live ? (lane >= K) + (lane >= 2 * K) + (lane >= 3 * K) : 0, pk = live ? lane - pt * K : 0;
     const int e = live ? tb.sel_idx[pt][pk] : -1 - lane;             // dead lanes match nobody
-    const unsigned same = __match_any_sync(0xFFFFFFFFu, e);
-    const bool leader = live && (__ffs(same) - 1 == lane);
+    const unsigned char *w0 = nullptr, *w1 = nullptr, *w2 = nullptr;
+    if (live) { w0 = ptab[e]; w1 = ptab[E + e]; w2 = ptab[2 * E + e]; }
+    const bool absent = w0 == nullptr || w1 == nullptr || w2 == nullptr;
+    const unsigned same = n == 1 ? 1u << lane : __match_any_sync(0xFFFFFFFFu, e);   // a row's picks are distinct
+    const int first = __ffs(same) - 1;
+    const bool leader = live && first == lane;
     const unsigned leaders = __ballot_sync(0xFFFFFFFFu, leader);
-    const int my_tile = t_first + __popc(leaders & ((1u << (__ffs(same) - 1)) - 1u));
-    // rows of the tile: the token of every lane in the group
-    int mask = 0;
-    for (unsigned m = same; m != 0; m &= m - 1) mask |= 1 << ((__ffs(m) - 1) / K);
-    if (has_shared && lane == 0) {
-      tb.tile_e[0] = E;
-      tb.tile_mask[0] = (1 << n) - 1;
-      tb.w[0][0] = L.sh[0]; tb.w[1][0] = L.sh[1]; tb.w[2][0] = L.sh[2];
-      tb.tile_mode[0] = ((reinterpret_cast<uintptr_t>(L.sh[0]) | reinterpret_cast<uintptr_t>(L.sh[1]) |
-                          reinterpret_cast<uintptr_t>(L.sh[2])) & 15u) == 0 ? 0 : 2;
-    }
-    bool absent = false;
-    if (leader) {
-      const unsigned char *w0 = ptab[e], *w1 = ptab[E + e], *w2 = ptab[2 * E + e];
-      absent = w0 == nullptr || w1 == nullptr || w2 == nullptr;
-      const bool aligned = ((reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1) |
-                             reinterpret_cast<uintptr_t>(w2)) & 15u) == 0;
-      tb.tile_e[my_tile] = e;
-      tb.tile_mask[my_tile] = mask;
-      tb.w[0][my_tile] = w0; tb.w[1][my_tile] = w1; tb.w[2][my_tile] = w2;
-      tb.tile_mode[my_tile] = absent ? 1 : (aligned ? 0 : 2);
-    }
-    const int T = t_first + __popc(leaders);
-    __syncwarp();
-    // first h / y row of every tile: prefix sum of the tiles' row counts (lane j = tile j, T <= 33:
-    // the last tile's start is the total minus its own rows)
-    const int cnt = lane < T ? __popc(tb.tile_mask[lane]) : 0;
+    const int my_tile = t_first + __popc(leaders & ((1u << first) - 1u));
+    int mask = 0;                                                    // rows of the tile: the token of every lane in the group
+    const unsigned row = K < 32 ? (1u << K) - 1u : 0xFFFFFFFFu;
+#pragma unroll
+    for (int t = 0; t < kMaxTok; ++t)
+      if (t < n && (same >> (t * K) & row) != 0) mask |= 1 << t;
+    // first h / y row of every tile: prefix sum of the founders' row counts
+    const int cnt = leader ? __popc(mask) : 0;
     int inc = cnt;
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
       const int v = __shfl_up_sync(0xFFFFFFFFu, inc, off);
       if (lane >= off) inc += v;
     }
-    if (lane < T) tb.tile_hrow0[lane] = inc - cnt;
-    const int total32 = __shfl_sync(0xFFFFFFFFu, inc, 31);
-    if (lane == 0) {
-      int hr = total32;
-      if (T > 32) {
-        tb.tile_hrow0[32] = hr;
-        hr += __popc(tb.tile_mask[32]);
-      }
-      tb.n_tiles = T;
-      tb.n_hrows = hr;
+    const int base = has_shared ? n : 0;
+    const int hrow0 = base + __shfl_sync(0xFFFFFFFFu, inc - cnt, first);
+    if (leader) {
+      const bool aligned = ((reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1) |
+                             reinterpret_cast<uintptr_t>(w2)) & 15u) == 0;
+      tb.tile_e[my_tile] = e;
+      tb.tile_mask[my_tile] = mask;
+      tb.tile_hrow0[my_tile] = hrow0;
+      tb.w[0][my_tile] = w0; tb.w[1][my_tile] = w1; tb.w[2][my_tile] = w2;
+      tb.tile_mode[my_tile] = absent ? 1 : (aligned ? 0 : 2);
     }
-    __syncwarp();
-    if (live) {
-      const bool gone = tb.tile_mode[my_tile] == 1;
-      tb.route_hrow[pt][pk] = gone ? -1 : tb.tile_hrow0[my_tile] + __popc(mask & ((1 << pt) - 1));
-    }
+    if (live) tb.route_hrow[pt][pk] = absent ? -1 : hrow0 + __popc(mask & ((1 << pt) - 1));
     if (lane < n) tb.route_hrow[lane][K] = has_shared ? lane : -1;
+    if (lane == 31) tb.n_hrows = base + inc;
+    if (lane == 0) {
+      tb.n_tiles = t_first + __popc(leaders);
+      if (has_shared) {
+        tb.tile_e[0] = E;
+        tb.tile_mask[0] = (1 << n) - 1;
+        tb.tile_hrow0[0] = 0;
+        tb.w[0][0] = L.sh[0]; tb.w[1][0] = L.sh[1]; tb.w[2][0] = L.sh[2];
+        tb.tile_mode[0] = ((reinterpret_cast<uintptr_t>(L.sh[0]) | reinterpret_cast<uintptr_t>(L.sh[1]) |
+                            reinterpret_cast<uintptr_t>(L.sh[2])) & 15u) == 0 ? 0 : 2;
+      }
+    }
     __syncwarp();
   };
   // this CTA's slice of the three matrices of a picked expert, whichever CTA reads it later
-  auto fetch = [&](int e) {
+  auto fetch = [&](int e, int g0, int g1, int d0, int d1) {
     if (lane >= K) return;
 #pragma unroll
     for (int m = 0; m < 3; ++m) {
       const unsigned char* w = ptab[m * E + e];
-      const int units = m < 2 ? FF * (G.rb_h / 16) : H * (G.rb_f / 16);
-      const int u0 = share(units, cta), u1 = share(units, cta + 1);
+      const int u0 = m < 2 ? g0 : d0, u1 = m < 2 ? g1 : d1;
       if (w != nullptr && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && u1 > u0)
         bulk_prefetch_l2(w + static_cast<size_t>(u0) * 16, static_cast<uint32_t>(u1 - u0) * 16);
     }
   };
-  const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
   if (warp < 2 * kMaxTok && (warp & (kMaxTok - 1)) < n) {
     const int t = warp & (kMaxTok - 1);
+    const int g0 = share(FF * (G.rb_h / 16), cta), g1 = share(FF * (G.rb_h / 16), cta + 1);
+    const int d0 = share(H * (G.rb_f / 16), cta), d1 = share(H * (G.rb_f / 16), cta + 1);
     const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
     const float* lg = L.logits + static_cast<size_t>(t) * E;
     float* pr = prob + static_cast<size_t>(t) * E;
     if (!there) ok = false;                      // (the named barriers below need every warp: it goes on with what is there)
     if (by_pairs) {
       const bool redo = select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane, [&](int e) {
-        fetch(e);
+        fetch(e, g0, g1, d0, d1);
         if (n > 1) named_sync(12, n * 32);       // every row's picks are in the tables
         else __syncwarp();
         if (warp == 0) build();
       });
       if (redo && lane == 0) *reinterpret_cast<volatile int*>(flag + 2) = 1;
+      __syncwarp();
+      if (there && lane == 0 && (warp == 0 || warp >= kMaxTok)) mbar_arrive_one(ready);
     } else if (warp < kMaxTok && there) {
       for (int i = lane; i < E; i += 32) pr[i] = __ldcg(lg + i);
       __syncwarp();
@@ -854,10 +854,13 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     return;
   }
   if (!by_pairs || *reinterpret_cast<volatile int*>(flag + 2) != 0) {
-    if (warp == 0) build();
+    if (warp == 0) {
+      build();
+      if (lane == 0)
+        for (int i = by_pairs ? n + 1 : 1; i > 0; --i) mbar_arrive_one(ready);
+    }
     consumers_sync();
   }
-  if (tid == 0) mbar_arrive_one(ready);          // the producer may issue every weight copy now
   if (cta == 0 && tid < n * (K + 1)) {
     const int t = tid / (K + 1), kk = tid - t * (K + 1);
     if (kk < K) L.idx[static_cast<size_t>(t) * L.rstride + kk] = tb.sel_idx[t][kk];
@@ -898,6 +901,11 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   const int f_half = tid & 1, f_lr = (tid >> 1) & (lpf - 1), f_blk = min(f_lr, L.nbf - 1);
   const int rounds = (T + kDownTiles - 1) / kDownTiles;
   bool first = true;
+  // this thread's output element (as a rule it has one), its residual fetched ahead of the barrier
+  const bool residual = L.add_residual && L.x_f16 != nullptr;
+  const int o_t = tid / max(nr, 1);
+  const size_t o_at = static_cast<size_t>(o_t) * H + r0 + (tid - o_t * nr);
+  const uint16_t res = residual && tid < n * nr ? L.x_f16[o_at] : 0;
 #pragma unroll 1
   for (int rd = 0; rd < rounds && ok; ++rd) {
     const int j0 = rd * kDownTiles, j1 = min(T, j0 + kDownTiles);
@@ -923,12 +931,11 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       if (first) {
         first = false;
         const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
+        quantize_h_rows(hq, tb.n_hrows, L.hbuf, warp, lane);
         if (!consumers_all(met && ok)) {
           if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
           return;
         }
-        quantize_h_rows(hq, tb.n_hrows, L.hbuf, warp, lane);
-        consumers_sync();
       }
       float v[kMaxTok];
       half_dots<1>(W, f_half, hq, f_blk, rs, rows, v);
@@ -950,13 +957,15 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   for (int i = tid; i < n * nr; i += kConsumers) {
     const int t = i / nr, rr = i - t * nr;
     const size_t o = static_cast<size_t>(t) * H + r0 + rr;
-    float acc = (L.add_residual && L.x_f16 != nullptr) ? h2f(L.x_f16[o]) : 0.f;
+    float acc = residual ? h2f(i == tid ? res : L.x_f16[o]) : 0.f;
+#pragma unroll 4
     for (int kk = 0; kk <= K; ++kk) {
       const int hr = tb.route_hrow[t][kk];
-      if (hr >= 0) acc += tb.sel_w[t][kk] * ysm[hr * G.nr_max + rr];
+      const float wk = tb.sel_w[t][kk], y = ysm[max(hr, 0) * G.nr_max + rr];
+      if (hr >= 0) acc += wk * y;
     }
     if (L.out_f32 != nullptr) L.out_f32[o] = acc;
-    if (L.x_f16 != nullptr && L.add_residual) L.x_f16[o] = f2h(acc);
+    if (residual) L.x_f16[o] = f2h(acc);
   }
 }
 
