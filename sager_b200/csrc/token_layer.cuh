@@ -116,7 +116,8 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
 }
 
 // Named barriers of the consumers: 6 all of them, 7 the warps with router rows, 5 the warps that quantise, 8 .. 11 the
-// two warps that select for a token row, 12 the warps that pick.
+// two warps that select for a token row, 12 the warps that pick,
+// 13 those and the second group.
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 6, %0;" ::"n"(kConsumers) : "memory");
@@ -348,7 +349,7 @@ __device__ __noinline__ void select_general(float* prob, int E, int K, int* idx,
 
 // Softmax and top-K of one token row by two warps (up to 256 experts, K < 32). The strictly serial sum of the
 // exponentials - the reference's order - is long, so one warp picks the K + 1 largest exponentials and goes on to build
-// the tables from them (`picked(lane's expert)`) while the other adds and makes the weights. Dividing by the sum keeps
+// the tables from them (`picked()`) while the other adds and makes the weights. Dividing by the sum keeps
 // the order; only if it makes two of them equal, or something is not finite, the order of the quotients could be another
 // one, and the adding warp runs the general selection on the quotients: it returns true, and the picks do not stand.
 template <typename Picked>
@@ -404,7 +405,7 @@ __device__ __forceinline__ bool select_pair(const float* logits, float* prob, Ta
     if (lane <= K) tb.pick_e[t][lane] = my_e;
     __syncwarp();
     asm volatile("bar.arrive %0, 64;" ::"r"(8 + t) : "memory");
-    picked(my_i);
+    picked();
     return false;
   }
 #pragma unroll
@@ -564,6 +565,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int P = (T - t_first) * FF, pb = share(P, cta + 1);
     int pos = share(P, cta);
     const int cut = min(G.stage_pairs, (pb - pos + 1) / 2);          // both groups get work
+    int tile = t_first + pos / FF, pair0 = pos - (tile - t_first) * FF;
     int issued = 0;
     bool down_issued = false;
     int round = 0;
@@ -571,13 +573,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     // down rows of the tiles of one round (tile 0 of round 0 is the shared expert's, fetched above)
     auto issue_down_round = [&](int rd) {
       const int j0 = rd * kDownTiles, j1 = min(T, j0 + kDownTiles);
-      uint32_t bytes = 0;
-      bool plain = false;
-      for (int j = j0; j < j1; ++j) {
-        if (j == 0 && has_shared) continue;
-        if (tb.tile_mode[j] == 0) bytes += static_cast<uint32_t>(nr * G.rb_f);
-        if (tb.tile_mode[j] == 2) plain = true;
-      }
+      const int md = j0 + lane < j1 && !(j0 + lane == 0 && has_shared) ? tb.tile_mode[j0 + lane] : 1;
+      const uint32_t bytes = static_cast<uint32_t>(__popc(__ballot_sync(0xFFFFFFFFu, md == 0)) * nr * G.rb_f);
+      const bool plain = __any_sync(0xFFFFFFFFu, md == 2);
       if (plain) {
         for (int j = j0; j < j1; ++j)
           if (!(j == 0 && has_shared) && tb.tile_mode[j] == 2)
@@ -587,16 +585,15 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         __syncwarp();
       }
       if (lane == 0) {
-        if (bytes > 0) {
-          mbar_expect_tx(dn_full, bytes);
-          for (int j = j0; j < j1; ++j)
-            if (!(j == 0 && has_shared) && tb.tile_mode[j] == 0)
-              bulk_g2s(dn + static_cast<size_t>(j - j0) * G.slot_bytes, tb.w[2][j] + static_cast<size_t>(r0) * G.rb_f,
-                       static_cast<uint32_t>(nr * G.rb_f), dn_full);
-        } else {
-          mbar_arrive_one(dn_full);
-        }
+        if (bytes > 0) mbar_expect_tx(dn_full, bytes);
+        else mbar_arrive_one(dn_full);
       }
+      __syncwarp();
+      const int jl = j0 + lane;                     // a lane per tile
+      if (bytes > 0 && md == 0)
+        bulk_g2s(dn + static_cast<size_t>(lane) * G.slot_bytes, tb.w[2][jl] + static_cast<size_t>(r0) * G.rb_f,
+                 static_cast<uint32_t>(nr * G.rb_f), dn_full);
+      __syncwarp();
     };
     while (pos < pb) {
       const int s = issued % kRing;
@@ -610,7 +607,6 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         if (lane == 0) atomicExch(L.status, 2);
         return;
       }
-      const int tile = t_first + pos / FF, pair0 = pos - (tile - t_first) * FF;
       const int np = min(cut, min(FF - pair0, pb - pos));
       const int mode = tb.tile_mode[tile];
       unsigned char* st = ring + static_cast<size_t>(s) * G.stage_bytes;
@@ -636,6 +632,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         }
       }
       pos += np;
+      pair0 += np;
+      if (pair0 == FF) { pair0 = 0; ++tile; }
       ++issued;
     }
     if (!down_issued) {
@@ -655,7 +653,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
 
   // ---------------- consumers ----------------
   const int row_lanes = __ffs(2 * next_pow2_cap32(L.nbh)) - 1;
-  const int nl = G.rows_per_cta;                 // warps 0 .. nl - 1: a router row each; the others fetch and quantise x
+  // warps 0 .. nlw - 1 take the logits, one (router row, token) at a time; the others quantise x
+  const int nl = G.rows_per_cta, nlw = min(nl * n, kGroupWarps);
   // router rows of this CTA's experts: fixed weights, on their way before the previous kernel is awaited
   for (int i = 0; i < nl; ++i) {
     const int e = cta + i * grid;
@@ -680,61 +679,43 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(ptab + i)), "l"(L.tab + static_cast<size_t>(m) * L.tab_stride + (i - m * E))
                  : "memory");
   }
-  const int jobs = n * L.nbh, xw = warp - nl, n_xw = kWarps - nl;
+  const int jobs = n * L.nbh, xw = warp - nlw, n_xw = kWarps - nlw;
   for (int i = tid; i < jobs * 32; i += kConsumers)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(xh + i * 8)), "l"(L.xn + static_cast<size_t>(i) * 8) : "memory");
   const HTile xt = {smem + G.off_xt, L.nbh};
   asm volatile("cp.async.wait_all;" ::: "memory");
   consumers_sync();                              // fp16 x rows, router rows and the pointer table are in place
   bool ok = true;
-  if (warp < nl) {
-    // logits: one warp per expert row; lane l adds k = l, l + 32, ... in ascending order with FMA and
-    // the lanes meet in a shuffle tree - the order of the reference's kernel (src/kernels/cuda/q4_k.cu:133-149).
-    // Eight steps of loads are issued ahead of their FMAs.
-    const int e = cta + warp * grid;
-    if (e < E) {
-      const float* wr = rw + static_cast<size_t>(warp) * H;
+  if (warp < nlw) {
+    // logits: lane l adds k = l, l + 32, ... in ascending order with FMA and the lanes meet in a shuffle tree - the
+    // order of the reference's kernel (src/kernels/cuda/q4_k.cu:133-149). Eight steps of loads are issued ahead of
+    // their FMAs.
+#pragma unroll 1
+    for (int item = warp; item < nl * n; item += nlw) {
+      const int t = (item >= nl) + (item >= 2 * nl) + (item >= 3 * nl), i = item - t * nl;
+      const int e = cta + i * grid;
+      if (e >= E) continue;
+      const float* wr = rw + static_cast<size_t>(i) * H;
+      const uint16_t* xr = xh + static_cast<size_t>(t) * H;
       const float b = L.bias != nullptr ? __ldg(L.bias + e) : 0.f;
-      auto run = [&](auto rows) {                // NT token slots: what is predicated off still takes its issue slots
-        constexpr int NT = decltype(rows)::value;
-        float acc[NT];
+      float acc = 0.f;
+      int k = lane;
+#pragma unroll 2
+      for (; k + 7 * 32 < H; k += 8 * 32) {
+        float wv[8];
+        uint16_t xv[8];
 #pragma unroll
-        for (int t = 0; t < NT; ++t) acc[t] = 0.f;
-        int k = lane;
+        for (int j = 0; j < 8; ++j) { wv[j] = wr[k + 32 * j]; xv[j] = xr[k + 32 * j]; }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc = fmaf(wv[j], h2f(xv[j]), acc);
+      }
 #pragma unroll 1
-        for (; k + 7 * 32 < H; k += 8 * 32) {
-          float wv[8];
-          uint16_t xv[NT][8];
+      for (; k < H; k += 32) acc = fmaf(wr[k], h2f(xr[k]), acc);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            wv[j] = wr[k + 32 * j];
-#pragma unroll
-            for (int t = 0; t < NT; ++t) xv[t][j] = xh[static_cast<size_t>(t < n ? t : 0) * H + k + 32 * j];
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-#pragma unroll
-            for (int t = 0; t < NT; ++t) acc[t] = fmaf(wv[j], h2f(xv[t][j]), acc[t]);
-        }
-#pragma unroll 1
-        for (; k < H; k += 32) {
-          const float wv = wr[k];
-#pragma unroll
-          for (int t = 0; t < NT; ++t) acc[t] = fmaf(wv, h2f(xh[static_cast<size_t>(t < n ? t : 0) * H + k]), acc[t]);
-        }
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-          float a = acc[t];
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, off);
-          if (lane == 0 && t < n) L.logits[static_cast<size_t>(t) * E + e] = a + b;
-        }
-      };
-      if (n == 1) run(std::integral_constant<int, 1>{});
-      else if (n == 2) run(std::integral_constant<int, 2>{});
-      else run(std::integral_constant<int, kMaxTok>{});
+      for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, off);
+      if (lane == 0) L.logits[static_cast<size_t>(t) * E + e] = acc + b;
     }
-    if (nl > 1) named_sync(7, nl * 32);
+    if (nlw > 1) named_sync(7, nlw * 32);
     if (tid == 0) {
       mbar_wait(based, 0);                       // (set at kernel start)
       grid_arrive(gctr);
@@ -782,13 +763,19 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     // first h / y row of every tile: prefix sum of the founders' row counts
     const int cnt = leader ? __popc(mask) : 0;
     int inc = cnt;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int v = __shfl_up_sync(0xFFFFFFFFu, inc, off);
-      if (lane >= off) inc += v;
-    }
     const int base = has_shared ? n : 0;
-    const int hrow0 = base + __shfl_sync(0xFFFFFFFFu, inc - cnt, first);
+    int hrow0;
+    if (n == 1) {                                                    // a tile per pick
+      hrow0 = base + lane;
+      inc = K;
+    } else {
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xFFFFFFFFu, inc, off);
+        if (lane >= off) inc += v;
+      }
+      hrow0 = base + __shfl_sync(0xFFFFFFFFu, inc - cnt, first);
+    }
     if (leader) {
       const bool aligned = ((reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1) |
                              reinterpret_cast<uintptr_t>(w2)) & 15u) == 0;
@@ -814,30 +801,16 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     }
     __syncwarp();
   };
-  // this CTA's slice of the three matrices of a picked expert, whichever CTA reads it later
-  auto fetch = [&](int e, int g0, int g1, int d0, int d1) {
-    if (lane >= K) return;
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      const unsigned char* w = ptab[m * E + e];
-      const int u0 = m < 2 ? g0 : d0, u1 = m < 2 ? g1 : d1;
-      if (w != nullptr && (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && u1 > u0)
-        bulk_prefetch_l2(w + static_cast<size_t>(u0) * 16, static_cast<uint32_t>(u1 - u0) * 16);
-    }
-  };
   if (warp < 2 * kMaxTok && (warp & (kMaxTok - 1)) < n) {
     const int t = warp & (kMaxTok - 1);
-    const int g0 = share(FF * (G.rb_h / 16), cta), g1 = share(FF * (G.rb_h / 16), cta + 1);
-    const int d0 = share(H * (G.rb_f / 16), cta), d1 = share(H * (G.rb_f / 16), cta + 1);
     const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
     const float* lg = L.logits + static_cast<size_t>(t) * E;
     float* pr = prob + static_cast<size_t>(t) * E;
     if (!there) ok = false;                      // (the named barriers below need every warp: it goes on with what is there)
     if (by_pairs) {
-      const bool redo = select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane, [&](int e) {
-        fetch(e, g0, g1, d0, d1);
+      const bool redo = select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane, [&] {
+        asm volatile("bar.arrive 13, %0;" ::"r"(n * 32 + kGroupThreads) : "memory");   // the second group fetches
         if (n > 1) named_sync(12, n * 32);       // every row's picks are in the tables
-        else __syncwarp();
         if (warp == 0) build();
       });
       if (redo && lane == 0) *reinterpret_cast<volatile int*>(flag + 2) = 1;
@@ -848,6 +821,25 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       __syncwarp();
       select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
     }
+  }
+  if (warp >= kGroupWarps && by_pairs) {
+    // The second group asks for this CTA's slice of the picked experts' matrices (whichever CTA reads it later) to be
+    // brought into L2 while warp 0 builds the tables. Line by line: in the copy engine's queue the requests would be
+    // ahead of the first stage's copies.
+    const int g0 = share(FF * (G.rb_h / 16), cta) * 16, g1 = share(FF * (G.rb_h / 16), cta + 1) * 16;
+    const int d0 = share(H * (G.rb_f / 16), cta) * 16, d1 = share(H * (G.rb_f / 16), cta + 1) * 16;
+    named_sync(13, n * 32 + kGroupThreads);
+    for (int t = 0; t < n; ++t)
+      for (int kk = warp - kGroupWarps; kk < K; kk += kGroupWarps) {
+        const int e = tb.sel_idx[t][kk];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          const unsigned char* w = ptab[m * E + e];
+          if (w == nullptr) continue;
+          for (int o = (m < 2 ? g0 : d0) + lane * 128; o < (m < 2 ? g1 : d1); o += 32 * 128)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(w + o) : "memory");
+        }
+      }
   }
   if (!consumers_all(ok)) {
     if (tid == 0) atomicExch(L.status, 5);
