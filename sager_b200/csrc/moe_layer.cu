@@ -1454,7 +1454,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       L.e_lo == 0 && L.e_hi == L.E && L.sh_lo == 0 && L.sh_hi == L.n && L.nbh <= 16 && L.nbf <= 16 &&
       a->workspace_bytes >= lay.items_total) {
     const tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid);
-    if (g.total <= 227 * 1024 && g.rows_per_cta <= tk::kGroupWarps)
+    if (g.total <= 227 * 1024 && g.down_tiles > 0 && g.rows_per_cta <= tk::kGroupWarps)
       return launch_layer<tk::token_layer_kernel>(dim3(L.grid), tk::kThreads, g.total, s, L);
   }
 

@@ -10,20 +10,27 @@
 //     the CTA's router rows and its share of the shared expert's gate / up / down rows
 //     are already on their way into shared memory - none of them depends on routing
 //   phase 1  Q8_K-quantise the rows (every CTA, redundantly: 4 KB per row), logits of the
-//            CTA's experts (one warp per expert row, the reference kernel's FMA order, so
-//            logits are bit-identical), grid barrier
-//   phase 2  every CTA selects redundantly from the n x E logits (one warp per row) and
-//            builds the same list of tiles (distinct experts, each with the set of rows
-//            routed to it). The producer warp then issues EVERY weight byte this CTA will
-//            need as bulk copies (TMA): its pairs of the routed gate / up rows AND its
-//            rows of the down matrices, so the down weights arrive while gate / up
-//            computes and the second half of the layer never waits for memory
+//            CTA's experts (a warp per expert row and token, the reference kernel's FMA order,
+//            so logits are bit-identical); arrive at the grid barrier; the shared expert's
+//            gate / up share while the others arrive
+//   phase 2  every CTA selects redundantly from the n x E logits: for each row one warp picks
+//            and one adds up the softmax; from the picks warp 0 builds the list of tiles
+//            (distinct experts, each with the set of rows routed to it). The producer warp
+//            then issues the weight copies (TMA): the CTA's pairs of the routed gate / up
+//            rows through a ring AND its rows of the down matrices, so the down weights
+//            arrive while gate / up computes
 //   phase 3  gate / up dots (dp4a, integer sub-block dots exact), SwiGLU, fp32 h rows to
-//            global memory, grid barrier
+//            global memory, grid barrier; the first down weights go into registers meanwhile
 //   phase 4  every CTA quantises the h rows it needs (all of them: a few KB from L2),
 //            runs the down dots for its H / grid output rows of EVERY tile, and - since
 //            all of a row's expert contributions are then in this CTA - adds
 //            residual + sum_k w_k * y_k + shared in place. No third barrier.
+//
+// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 15.9 us per
+// layer, of which 3.5 to the first barrier, 2 for picks and tables, 1.5 for the first bytes, 2 for
+// gate / up, 2 for the second barrier, 1 + 1 for h and the down rows; 26.6 with eight warps on whole
+// blocks and the selection in sequence), from two rows on the integer pipe and shared memory: 7 us
+// for every further row (23.0 / 30.1 / 36.6 us; 36.3 / 45.2 / 47.3 before).
 //
 // Work split: gate / up by pairs (a flat range of (tile, pair) per CTA), down by output
 // rows. Contracts are those of the two-launch path: null table entry = absent expert
@@ -41,7 +48,7 @@ constexpr int kGroupThreads = kGroupWarps * 32;
 constexpr int kThreads = kConsumers + 32;  // + producer warp
 constexpr int kPairsStage = 16;            // (gate, up) row pairs per ring stage, at least
 constexpr int kRing = 2;
-constexpr int kDownTiles = 16;             // tiles whose down rows are resident at once
+constexpr int kDownTiles = 16;             // tiles whose down rows are resident in their own region; as many again in the ring
 constexpr int kMaxTiles = 33;              // n * K + 1 <= 33
 constexpr int kHdr = 1024;
 constexpr int kTables = 4096;
@@ -81,7 +88,7 @@ struct Geom {
   int sp_max;            // shared-expert pairs per CTA
   int rb_h, rb_f;        // bytes per gate/up row, per down row
   size_t off_prob, off_ptab, off_xh, off_rw, off_xt, off_sh, off_ring, off_dn, off_y, total;
-  int stage_pairs, stage_bytes, slot_bytes;
+  int stage_pairs, stage_bytes, slot_bytes, down_tiles;
 };
 __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int grid) {
   Geom g;
@@ -109,7 +116,9 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
   g.stage_bytes = 2 * g.stage_pairs * g.rb_h;
   g.off_ring = take(static_cast<size_t>(kRing) * g.stage_bytes);
   g.slot_bytes = g.nr_max * g.rb_f;
-  g.off_dn = take(static_cast<size_t>(hrows < kDownTiles ? hrows : kDownTiles) * g.slot_bytes);
+  const int in_ring = kRing * g.stage_bytes / (g.slot_bytes > 0 ? g.slot_bytes : 1);
+  g.down_tiles = in_ring < kDownTiles ? in_ring : kDownTiles;      // (none: the caller takes another path)
+  g.off_dn = take(static_cast<size_t>(hrows < g.down_tiles ? hrows : g.down_tiles) * g.slot_bytes);
   g.off_y = take(static_cast<size_t>(hrows) * g.nr_max * 4);
   g.total = p;
   return g;
@@ -117,7 +126,7 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
 
 // Named barriers of the consumers: 6 all of them, 7 the warps with router rows, 5 the warps that quantise, 8 .. 11 the
 // two warps that select for a token row, 12 the warps that pick,
-// 13 those and the second group.
+// 13 the warp that picks the only row and the second group.
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 6, %0;" ::"n"(kConsumers) : "memory");
@@ -451,9 +460,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   uint64_t* empty = full + kRing;                                  // [kRing]
   uint64_t* sh_full = empty + kRing;                               // shared expert's gate / up pairs
   uint64_t* shdn_full = sh_full + 1;                               // shared expert's down rows (slot 0)
-  uint64_t* dn_full = shdn_full + 1;                               // routed tiles' down rows, one phase per round
-  uint64_t* dn_empty = dn_full + 1;
-  uint64_t* ready = dn_empty + 1;                                  // tables built
+  uint64_t* dn_full = shdn_full + 1;                               // [2] routed tiles' down rows, rounds in turn
+  uint64_t* dn_empty = dn_full + 2;                                // [2]
+  uint64_t* ready = dn_empty + 2;                                  // tables built
   uint64_t* based = ready + 1;                                     // the grid counter has been read
   uint64_t* passed = based + 1;                                    // grid barrier passed (or given up), one phase each
   StageDesc* desc = reinterpret_cast<StageDesc*>(smem + 128);      // [kRing]
@@ -491,8 +500,10 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     }
     mbar_init(sh_full, 1);
     mbar_init(shdn_full, 1);
-    mbar_init(dn_full, 1);
-    mbar_init(dn_empty, kWarps);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&dn_full[s], 1);
+      mbar_init(&dn_empty[s], kWarps);
+    }
     mbar_init(ready, by_pairs ? n + 1 : 1);      // tables built, and every row's picks found to stand (or not: flag[2])
     mbar_init(based, 1);
     mbar_init(passed, 1);
@@ -569,30 +580,32 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     int issued = 0;
     bool down_issued = false;
     int round = 0;
-    const int rounds = (T + kDownTiles - 1) / kDownTiles;
+    const int dt = G.down_tiles, rounds = (T + dt - 1) / dt;
     // down rows of the tiles of one round (tile 0 of round 0 is the shared expert's, fetched above)
     auto issue_down_round = [&](int rd) {
-      const int j0 = rd * kDownTiles, j1 = min(T, j0 + kDownTiles);
+      const int j0 = rd * dt, j1 = min(T, j0 + dt);
+      unsigned char* to = (rd & 1) ? ring : dn;
+      uint64_t* full_bar = &dn_full[rd & 1];
       const int md = j0 + lane < j1 && !(j0 + lane == 0 && has_shared) ? tb.tile_mode[j0 + lane] : 1;
       const uint32_t bytes = static_cast<uint32_t>(__popc(__ballot_sync(0xFFFFFFFFu, md == 0)) * nr * G.rb_f);
       const bool plain = __any_sync(0xFFFFFFFFu, md == 2);
       if (plain) {
         for (int j = j0; j < j1; ++j)
           if (!(j == 0 && has_shared) && tb.tile_mode[j] == 2)
-            copy_plain(dn + static_cast<size_t>(j - j0) * G.slot_bytes, tb.w[2][j] + static_cast<size_t>(r0) * G.rb_f,
+            copy_plain(to + static_cast<size_t>(j - j0) * G.slot_bytes, tb.w[2][j] + static_cast<size_t>(r0) * G.rb_f,
                        nr * G.rb_f, lane);
         fence_proxy_async();
         __syncwarp();
       }
       if (lane == 0) {
-        if (bytes > 0) mbar_expect_tx(dn_full, bytes);
-        else mbar_arrive_one(dn_full);
+        if (bytes > 0) mbar_expect_tx(full_bar, bytes);
+        else mbar_arrive_one(full_bar);
       }
       __syncwarp();
       const int jl = j0 + lane;                     // a lane per tile
       if (bytes > 0 && md == 0)
-        bulk_g2s(dn + static_cast<size_t>(lane) * G.slot_bytes, tb.w[2][jl] + static_cast<size_t>(r0) * G.rb_f,
-                 static_cast<uint32_t>(nr * G.rb_f), dn_full);
+        bulk_g2s(to + static_cast<size_t>(lane) * G.slot_bytes, tb.w[2][jl] + static_cast<size_t>(r0) * G.rb_f,
+                 static_cast<uint32_t>(nr * G.rb_f), full_bar);
       __syncwarp();
     };
     while (pos < pb) {
@@ -640,9 +653,19 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       issue_down_round(0);
       round = 1;
     }
+    if (round < rounds) {                           // the second round into the ring, once its last stages are in registers
+      for (int s = 0; s < kRing; ++s) {
+        const int used = (issued - s + kRing - 1) / kRing;
+        if (used > 0 && !mbar_wait(&empty[s], (used - 1) & 1)) {
+          if (lane == 0) atomicExch(L.status, 2);
+          return;
+        }
+      }
+      issue_down_round(round++);
+    }
     grid_poll(2);
-    for (; round < rounds; ++round) {               // later rounds reuse the region
-      if (!mbar_wait(dn_empty, (round - 1) & 1)) {
+    for (; round < rounds; ++round) {               // later rounds reuse the regions
+      if (!mbar_wait(&dn_empty[round & 1], (round / 2 - 1) & 1)) {
         if (lane == 0) atomicExch(L.status, 2);
         return;
       }
@@ -809,8 +832,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     if (!there) ok = false;                      // (the named barriers below need every warp: it goes on with what is there)
     if (by_pairs) {
       const bool redo = select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane, [&] {
-        asm volatile("bar.arrive 13, %0;" ::"r"(n * 32 + kGroupThreads) : "memory");   // the second group fetches
-        if (n > 1) named_sync(12, n * 32);       // every row's picks are in the tables
+        if (n == 1) asm volatile("bar.arrive 13, %0;" ::"n"(32 + kGroupThreads) : "memory");   // the second group fetches
+        else named_sync(12, n * 32);             // every row's picks are in the tables
         if (warp == 0) build();
       });
       if (redo && lane == 0) *reinterpret_cast<volatile int*>(flag + 2) = 1;
@@ -822,24 +845,24 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
     }
   }
-  if (warp >= kGroupWarps && by_pairs) {
-    // The second group asks for this CTA's slice of the picked experts' matrices (whichever CTA reads it later) to be
+  if (warp >= kGroupWarps && by_pairs && n == 1) {
+    // One row: the second group asks for this CTA's slice of the picked experts' matrices (whichever CTA reads it later) to be
     // brought into L2 while warp 0 builds the tables. Line by line: in the copy engine's queue the requests would be
-    // ahead of the first stage's copies.
+    // ahead of the first stage's copies. (16.3 -> 15.7 us; with more rows the other tiles' bytes only come ahead of the
+    // first stages' - 23.5 against 23.1, 31.7 against 30.9, 40.3 against 38.4 us at 2 / 3 / 4 rows.)
     const int g0 = share(FF * (G.rb_h / 16), cta) * 16, g1 = share(FF * (G.rb_h / 16), cta + 1) * 16;
     const int d0 = share(H * (G.rb_f / 16), cta) * 16, d1 = share(H * (G.rb_f / 16), cta + 1) * 16;
-    named_sync(13, n * 32 + kGroupThreads);
-    for (int t = 0; t < n; ++t)
-      for (int kk = warp - kGroupWarps; kk < K; kk += kGroupWarps) {
-        const int e = tb.sel_idx[t][kk];
+    named_sync(13, 32 + kGroupThreads);
+    for (int kk = warp - kGroupWarps; kk < K; kk += kGroupWarps) {
+      const int e = tb.sel_idx[0][kk];
 #pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          const unsigned char* w = ptab[m * E + e];
-          if (w == nullptr) continue;
-          for (int o = (m < 2 ? g0 : d0) + lane * 128; o < (m < 2 ? g1 : d1); o += 32 * 128)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(w + o) : "memory");
-        }
+      for (int m = 0; m < 3; ++m) {
+        const unsigned char* w = ptab[m * E + e];
+        if (w == nullptr) continue;
+        for (int o = (m < 2 ? g0 : d0) + lane * 128; o < (m < 2 ? g1 : d1); o += 32 * 128)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(w + o) : "memory");
       }
+    }
   }
   if (!consumers_all(ok)) {
     if (tid == 0) atomicExch(L.status, 5);
@@ -891,7 +914,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   const HTile hq = {smem + G.off_xh, L.nbf};
   const int f_lanes = __ffs(2 * next_pow2_cap32(L.nbf)) - 1, lpf = 1 << (f_lanes - 1);
   const int f_half = tid & 1, f_lr = (tid >> 1) & (lpf - 1), f_blk = min(f_lr, L.nbf - 1);
-  const int rounds = (T + kDownTiles - 1) / kDownTiles;
+  const int dt = G.down_tiles, rounds = (T + dt - 1) / dt;
   bool first = true;
   // this thread's output element (as a rule it has one), its residual fetched ahead of the barrier
   const bool residual = L.add_residual && L.x_f16 != nullptr;
@@ -900,9 +923,10 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   const uint16_t res = residual && tid < n * nr ? L.x_f16[o_at] : 0;
 #pragma unroll 1
   for (int rd = 0; rd < rounds && ok; ++rd) {
-    const int j0 = rd * kDownTiles, j1 = min(T, j0 + kDownTiles);
+    const int j0 = rd * dt, j1 = min(T, j0 + dt);
+    const unsigned char* from = (rd & 1) ? ring : dn;
     if (rd == 0 && has_shared && !mbar_wait(shdn_full, 0)) ok = false;
-    if (ok && !mbar_wait(dn_full, rd & 1)) ok = false;
+    if (ok && !mbar_wait(&dn_full[rd & 1], (rd >> 1) & 1)) ok = false;
     ok = __all_sync(0xFFFFFFFFu, ok) != 0;
     const int tasks = (j1 - j0) * nr << f_lanes;
     int base = 0;
@@ -917,7 +941,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       const int hrow0 = tb.tile_hrow0[tile];
       const RowSet rs = rows_of(live ? tb.tile_mask[tile] : 0, live ? hrow0 : 0, false);   // h rows are stored per tile
       const int rows = __reduce_max_sync(0xFFFFFFFFu, rs.n);
-      const unsigned char* const w[1] = {dn + (live ? js * G.slot_bytes + r * G.rb_f + f_blk * kW4 : 0)};
+      const unsigned char* const w[1] = {from + (live ? js * G.slot_bytes + r * G.rb_f + f_blk * kW4 : 0)};
       HalfW<1> W;
       load_half<1>(W, w, f_half);
       if (first) {
@@ -940,7 +964,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       base += kConsumers;
     } while (base < tasks && ok);
     __syncwarp();
-    if (lane == 0 && rd + 1 < rounds) mbar_arrive_one(dn_empty);
+    if (lane == 0 && rd + 2 < rounds) mbar_arrive_one(&dn_empty[rd & 1]);
   }
   if (!consumers_all(ok)) {
     if (tid == 0) atomicExch(L.status, 3);

@@ -478,6 +478,28 @@ def test_token_kernel_agrees_with_the_two_launch_path(full_w):
     assert lib().raw("sgr_status")(0) == 0
 
 
+@pytest.mark.parametrize("hidden,n_ff,E,k,n,ties", [
+    (1280, 1024, 48, 8, 4, False),     # eight tiles' down rows at a time: five rounds in two regions
+    (256, 256, 5, 4, 1, False),        # one block per row, fewer experts than lanes
+    (768, 512, 300, 3, 2, False),      # more experts than one selecting warp holds
+    (512, 256, 40, 4, 1, True),        # picks that do not stand: every logit twice, the lower expert goes first
+    (512, 256, 40, 4, 3, True),
+])
+def test_token_kernel_edges(hidden, n_ff, E, k, n, ties):
+    """The same routing and, to fp32 rounding of the same terms (1e-5), the same layer as route + expert kernel."""
+    w = synth.MoeWeights(hidden, n_ff, E, DEV, seed=88, std=0.05)
+    if ties:
+        w.router[E // 2:] = w.router[:E // 2]
+    x16 = synth.normal_fp16((n, hidden), 89, DEV)
+    r0, _, o0 = run_layer(w, n, k, x16)
+    r1, _, o1 = run_layer(w, n, k, x16, kernel="two_launch")
+    assert torch.equal(r0.route_idx[:n], r1.route_idx[:n]) and torch.equal(r0.route_w[:n], r1.route_w[:n])
+    assert rel(o0.cpu().numpy(), o1.cpu().numpy()) < 1e-5
+    if ties:
+        first = r0.route_idx[:n, 0].cpu().numpy()
+        assert (first < E // 2).all() and (r0.route_idx[:n, 1].cpu().numpy() == first + E // 2).all()
+
+
 @pytest.mark.parametrize("own_plan", [False, True])
 @pytest.mark.parametrize("tokens", [8, 64])
 def test_fused_exchange_entry_points_with_one_rank(full_w, tokens, own_plan):
