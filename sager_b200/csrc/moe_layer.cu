@@ -58,8 +58,8 @@ constexpr int kTokenKernelMaxRows = 4;   // layers of up to this many token rows
 constexpr int kRowsKernelMinRows = 4;    // layers of at least this many token rows run the row-streaming kernel
                                          // (measured: 4 rows 8 % faster, 8 rows 16 %, 2 rows slower)
 constexpr int kRouteTok = 8;       // token rows per CTA of the route kernel
-constexpr int kRouteWarps = 8;
-constexpr int kRouteRows = 2 * kRouteWarps;   // experts per CTA of the route kernel: two rows per warp
+constexpr int kRouteWarps = 16;    // warps of a route CTA: all stage, eight do the logits and eight quantise, pairs select
+constexpr int kRouteMaxRows = 16;  // most experts per route CTA
 
 constexpr int kTeams = 2;                         // consumer teams, items alternate between them
 constexpr int kTeamWarps = 8;
@@ -113,6 +113,7 @@ struct LayerDev {
   int xq16_stride;     // bytes between its rows (nbh * 288 in the workspace; the record stride for padded records)
   int xq_padded;       // the caller's xq_in / xq_out rows are in 288-byte blocks already
   int grid;            // CTAs of the expert kernel
+  int route_rows;      // experts per CTA of the route kernel: 2, 4, 8 or 16
   const unsigned* wait_flags;   // expert parallelism over peer memory: arrival words to wait for before planning
   const unsigned* wait_step;
   int wait_count, wait_mul, wait_add;
@@ -342,87 +343,48 @@ __device__ void build_plan(const LayerDev& L, unsigned char* smem) {
 inline size_t plan_smem(int E, int, int) { return static_cast<size_t>(E) * 12 + 3 * 128 * 4; }
 
 // ---- launch 1: route ------------------------------------------------------------------
-// grid (ceil(E / 16), ceil(n / 8)), 256 threads: a CTA computes the logits of sixteen
-// experts (two per warp) for a tile of up to eight token rows. The tile's activations are
-// staged in shared memory as fp32, k-major (see router_rows2_dot_kmajor), so that a
-// lane's values of one k for four rows are one vector load that serves both expert rows.
-// Dynamic smem: H * (8 + 16) floats (activations, router rows; the selection and the plan reuse it).
-template <int NT>
-__device__ __forceinline__ void route_tile_logits(const LayerDev& L, float* xs, const float* ws, int tok0, int nt,
+// grid (ceil(E / route_rows), ceil(n / 8)), 512 threads: a CTA computes the logits of 2, 4, 8 or 16
+// experts for a tile of up to eight token rows. The tile's activations are staged in shared memory as
+// fp16, k-major in groups of T rows, by all warps in one pass of loads; then eight warps do R x T
+// logits each while the other eight quantise, and the last CTA of the tile selects with two warps per
+// row. As few experts per CTA as one wave allows: the chain of phases bounds the launch, not its
+// bytes, and a lane's FMAs cannot be split (their order is the reference's). 64 rows, 256 experts,
+// hidden 2048: ROUTE_64; 8 rows: ROUTE_8 (one phase after the other with eight warps, fp32 activations and a
+// serial selection: 20.2 and 20.2).
+// Dynamic smem: route_rows * H floats, 8 * H halves (the selection and the plan reuse it).
+template <int R, int T>
+__device__ __forceinline__ void route_tile_logits(const LayerDev& L, const uint16_t* xs, const float* ws, int tok0, int nt,
                                                    int row0, int warp, int lane) {
-  // stage: lane = one k of a 32-wide chunk, all rows of the tile (rows beyond nt read as
-  // zero); four chunks per pass, so that all loads of a pass are in flight together
-  for (int c0 = warp; c0 < L.H / 32; c0 += 4 * kRouteWarps) {
-    uint16_t raw[4][NT];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = (c0 + u * kRouteWarps) * 32 + lane;
-#pragma unroll
-      for (int t = 0; t < NT; ++t)
-        raw[u][t] = (t < nt && k < L.H) ? L.xn[static_cast<size_t>(tok0 + t) * L.H + k] : static_cast<uint16_t>(0);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = (c0 + u * kRouteWarps) * 32 + lane;
-      if (k >= L.H) continue;
-      if (NT >= 4) {
-#pragma unroll
-        for (int p = 0; p < NT / 4; ++p)
-          *reinterpret_cast<float4*>(xs + static_cast<size_t>(p) * 4 * L.H + static_cast<size_t>(k) * 4) =
-              make_float4(h2f(raw[u][(4 * p) % NT]), h2f(raw[u][(4 * p + 1) % NT]), h2f(raw[u][(4 * p + 2) % NT]),
-                          h2f(raw[u][(4 * p + 3) % NT]));
-      } else if (NT == 2) {
-        *reinterpret_cast<float2*>(xs + static_cast<size_t>(k) * 2) = make_float2(h2f(raw[u][0]), h2f(raw[u][1 % NT]));
-      } else {
-        xs[k] = h2f(raw[u][0]);
-      }
-    }
-  }
-  asm volatile("cp.async.wait_all;" ::: "memory");     // this warp's two router rows have landed
-  __syncthreads();
-  float out[2][NT];
-  router_rows2_dot_kmajor<NT>(ws + static_cast<size_t>(2 * warp) * L.H, ws + static_cast<size_t>(2 * warp + 1) * L.H, xs,
-                              L.H, lane, out);
-  if (lane == 0) {
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      if (row0 + r < L.E) {
-        const float b = L.bias != nullptr ? L.bias[row0 + r] : 0.f;
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-          if (t < nt) L.logits[static_cast<size_t>(tok0 + t) * L.E + row0 + r] = out[r][t] + b;
-      }
-    }
-  }
+  constexpr int kGroups = kRouteTok / T;           // token groups; the warps take (row group, token group)
+  const int rg = warp / kGroups, tg = warp % kGroups;
+  const float v = router_tile_dot<R, T>(ws + static_cast<size_t>(rg) * R * L.H, xs + static_cast<size_t>(tg) * T * L.H, L.H, lane);
+  constexpr int kSpan = 32 / (R * T);
+  const int i = lane / kSpan, e = row0 + rg * R + i / T, t = tg * T + i % T;
+  if (lane % kSpan == 0 && e < L.E && t < nt)
+    L.logits[static_cast<size_t>(tok0 + t) * L.E + e] = v + (L.bias != nullptr ? __ldg(L.bias + e) : 0.f);
 }
 
 __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev L) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int last_sh;
-  float* xs = reinterpret_cast<float*>(smem);
+  __shared__ float pick_e[kRouteTok][32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tok0 = blockIdx.y * kRouteTok;
   const int nt = min(kRouteTok, L.n - tok0);
-  const int row0 = blockIdx.x * kRouteRows + 2 * warp;
+  const int rows = L.route_rows, row0 = blockIdx.x * rows;
+  float* ws = reinterpret_cast<float*>(smem);                                             // [rows][H]
+  uint16_t* xs = reinterpret_cast<uint16_t*>(ws + static_cast<size_t>(rows) * L.H);      // [8 / T][H][T]
 
-  // this warp's two router rows do not depend on the previous layer: they are on their
-  // way into shared memory (asynchronous copies) before the wait for that layer ends
-  float* ws = xs + static_cast<size_t>(kRouteTok) * L.H;              // [16 rows][H]
-  {
-    const float* w0 = L.router_w + static_cast<size_t>(min(row0, L.E - 1)) * L.H;
-    const float* w1 = L.router_w + static_cast<size_t>(min(row0 + 1, L.E - 1)) * L.H;
-    float* d0 = ws + static_cast<size_t>(2 * warp) * L.H;
-    float* d1 = d0 + L.H;
+  // the router rows do not depend on the previous layer: they are on their way into shared
+  // memory (asynchronous copies) before the wait for that layer ends
+  for (int r = 0; r < rows; ++r) {
+    const float* src = L.router_w + static_cast<size_t>(min(row0 + r, L.E - 1)) * L.H;
+    float* dst = ws + static_cast<size_t>(r) * L.H;
     if ((reinterpret_cast<uintptr_t>(L.router_w) & 15u) == 0) {
-      for (int c = lane * 4; c < L.H; c += 128) {
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d0 + c)), "l"(w0 + c) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(d1 + c)), "l"(w1 + c) : "memory");
-      }
+      for (int c = tid * 4; c < L.H; c += kRouteWarps * 128)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + c)), "l"(src + c) : "memory");
     } else {
-      for (int c = lane; c < L.H; c += 32) {
-        d0[c] = __ldg(w0 + c);
-        d1[c] = __ldg(w1 + c);
-      }
+      for (int c = tid; c < L.H; c += kRouteWarps * 32) dst[c] = __ldg(src + c);
     }
   }
   pdl_wait();
@@ -452,13 +414,50 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev 
     }
   }
 
-  // Q8_K rows of the tile (packed, and padded for the row-streaming kernel): block
-  // b of the tile goes to warp b / gridDim.x of CTA b % gridDim.x
-  if (L.xq_in != nullptr) {
-    if (blockIdx.x == 0 && L.tok_tile != kTokTile && !L.xq_padded) pad_xq_rows(L, tok0, nt, tid, blockDim.x);
+  // stage: lane = one k of a 32-wide chunk, all rows of the tile (rows beyond nt read as
+  // zero); four chunks per pass, so that all loads of a pass are in flight together
+  const int tsh = rows >= 16 ? 3 : (rows >= 4 ? 2 : 1);          // token rows per group: 8, 4 or 2
+  for (int c0 = warp; c0 < L.H / 32; c0 += 4 * kRouteWarps) {
+    uint16_t raw[4][kRouteTok];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = (c0 + u * kRouteWarps) * 32 + lane;
+#pragma unroll
+      for (int t = 0; t < kRouteTok; ++t)
+        raw[u][t] = (t < nt && k < L.H) ? L.xn[static_cast<size_t>(tok0 + t) * L.H + k] : static_cast<uint16_t>(0);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = (c0 + u * kRouteWarps) * 32 + lane;
+      if (k >= L.H) continue;
+      uint32_t q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) q[i] = raw[u][2 * i] | (static_cast<uint32_t>(raw[u][2 * i + 1]) << 16);
+      if (tsh == 3) {
+        *reinterpret_cast<uint4*>(xs + static_cast<size_t>(k) * 8) = make_uint4(q[0], q[1], q[2], q[3]);
+      } else if (tsh == 2) {
+        *reinterpret_cast<uint2*>(xs + static_cast<size_t>(k) * 4) = make_uint2(q[0], q[1]);
+        *reinterpret_cast<uint2*>(xs + static_cast<size_t>(L.H + k) * 4) = make_uint2(q[2], q[3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(xs + static_cast<size_t>(i * L.H + k) * 2) = q[i];
+      }
+    }
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  if (warp < kRouteWarps / 2) {
+    if (rows == 16) route_tile_logits<2, 8>(L, xs, ws, tok0, nt, row0, warp, lane);
+    else if (rows == 8) route_tile_logits<2, 4>(L, xs, ws, tok0, nt, row0, warp, lane);
+    else if (rows == 4) route_tile_logits<1, 4>(L, xs, ws, tok0, nt, row0, warp, lane);
+    else route_tile_logits<1, 2>(L, xs, ws, tok0, nt, row0, warp, lane);
+  } else if (L.xq_in != nullptr) {
+    // Q8_K rows of the tile (packed, and padded for the row-streaming kernel)
+    if (blockIdx.x == 0 && L.tok_tile != kTokTile && !L.xq_padded)
+      pad_xq_rows(L, tok0, nt, tid - kRouteWarps * 16, kRouteWarps * 16);
   } else {
-    const int b = warp * gridDim.x + blockIdx.x;
-    if (b < nt * L.nbh) {
+    // block b of the tile goes to quantising warp b / gridDim.x of CTA b % gridDim.x
+    for (int b = (warp - kRouteWarps / 2) * gridDim.x + blockIdx.x; b < nt * L.nbh; b += kRouteWarps / 2 * gridDim.x) {
       const int t = b / L.nbh, blk = b - t * L.nbh;
       quantize_block_f16(L.xn + static_cast<size_t>(tok0 + t) * L.H + blk * kQK,
                          L.xq + static_cast<size_t>(tok0 + t) * L.xq_stride + blk * kX8, lane,
@@ -466,20 +465,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev 
                              ? nullptr
                              : L.xq16 + static_cast<size_t>(tok0 + t) * L.xq16_stride + blk * 288);
     }
-    // more blocks than warps in the tile's CTAs (small expert counts): the rest in a loop
-    for (int b2 = b + kRouteWarps * gridDim.x; b2 < nt * L.nbh; b2 += kRouteWarps * gridDim.x) {
-      const int t = b2 / L.nbh, blk = b2 - t * L.nbh;
-      quantize_block_f16(L.xn + static_cast<size_t>(tok0 + t) * L.H + blk * kQK,
-                         L.xq + static_cast<size_t>(tok0 + t) * L.xq_stride + blk * kX8, lane,
-                         (L.tok_tile == kTokTile && !L.xq_padded)
-                             ? nullptr
-                             : L.xq16 + static_cast<size_t>(tok0 + t) * L.xq16_stride + blk * 288);
-    }
   }
-  if (nt > 4) route_tile_logits<8>(L, xs, ws, tok0, nt, row0, warp, lane);
-  else if (nt > 2) route_tile_logits<4>(L, xs, ws, tok0, nt, row0, warp, lane);
-  else if (nt > 1) route_tile_logits<2>(L, xs, ws, tok0, nt, row0, warp, lane);
-  else route_tile_logits<1>(L, xs, ws, tok0, nt, row0, warp, lane);
   // last CTA of this token tile selects (the counter's release covers the logits of all
   // warps, which the barrier ordered before it; its acquire covers the reads that follow)
   __syncthreads();
@@ -487,13 +473,19 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev 
   __syncthreads();
   if (!last_sh) return;
   if (tid == 0) L.cnt[blockIdx.y] = 0u;       // every CTA of the tile has counted in: ready for the next launch
-  float* prob = reinterpret_cast<float*>(smem) + static_cast<size_t>(warp % kRouteTok) * L.E;
-  for (int t = warp; t < nt; t += kRouteWarps) {
-    for (int i = lane; i < L.E; i += 32) prob[i] = __ldcg(L.logits + static_cast<size_t>(tok0 + t) * L.E + i);
-    __syncwarp();
-    router_select_warp(prob, L.E, L.K, L.idx + static_cast<size_t>(tok0 + t) * L.rstride,
-                       L.w + static_cast<size_t>(tok0 + t) * L.rstride, L.shared_w, true, lane);
-    __syncwarp();
+  {
+    const int t = warp % kRouteTok;              // warps t and t + 8 select for row t, or warp t alone
+    const float* lg = L.logits + static_cast<size_t>(tok0 + t) * L.E;
+    float* prob = reinterpret_cast<float*>(smem) + static_cast<size_t>(t) * ((L.E + 3) & ~3);     // rows at 16-byte steps
+    int* idx = L.idx + static_cast<size_t>(tok0 + t) * L.rstride;
+    float* w = L.w + static_cast<size_t>(tok0 + t) * L.rstride;
+    if (t < nt && L.E <= 256 && L.K < 32) {
+      router_select_pair(lg, prob, pick_e[t], idx, w, 1 + t, warp >= kRouteTok, L.E, L.K, L.shared_w, lane, [] {});
+    } else if (t < nt && warp < kRouteTok) {
+      for (int i = lane; i < L.E; i += 32) prob[i] = __ldcg(lg + i);
+      __syncwarp();
+      router_select_general(prob, L.E, L.K, idx, w, L.shared_w, lane);
+    }
   }
   if (L.skip_plan) {
     if (L.ep_dst == nullptr) return;
@@ -1462,11 +1454,16 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
   if (!(stages & 1)) {
     // plan, xq and routing are taken from the workspace as a previous call left them
   } else if (!a->routing_given) {
+    // as few experts per CTA as one wave of CTAs allows
+    const int tiles = (L.n + kRouteTok - 1) / kRouteTok;
+    L.route_rows = 2;
+    while (L.route_rows < kRouteMaxRows && (L.E + L.route_rows - 1) / L.route_rows * tiles > L.grid) L.route_rows *= 2;
     const size_t smem = std::max<size_t>(
-        std::max<size_t>(static_cast<size_t>(kRouteTok + kRouteRows) * L.H * 4, static_cast<size_t>(kRouteTok) * L.E * 4),
+        std::max<size_t>(static_cast<size_t>(L.route_rows) * L.H * 4 + static_cast<size_t>(kRouteTok) * L.H * 2,
+                         static_cast<size_t>(kRouteTok) * ((L.E + 3) & ~3) * 4),
         plan_smem(L.E, L.n_max, L.K));
     if (smem > 200 * 1024) return kErrUnsupported;
-    rc = launch_layer<route_kernel>(dim3((L.E + kRouteRows - 1) / kRouteRows, (L.n + kRouteTok - 1) / kRouteTok),
+    rc = launch_layer<route_kernel>(dim3((L.E + L.route_rows - 1) / L.route_rows, tiles),
                     kRouteWarps * 32, smem, s, L);
   } else {
     if (!a->xq_in) return kErrArg;

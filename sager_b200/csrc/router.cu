@@ -222,7 +222,7 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
-// one warp per row, 4 rows per CTA; dynamic smem = 4 * n_expert floats
+// one warp per row, 4 rows per CTA; dynamic smem = 4 rows of n_expert floats at 16-byte steps
 constexpr int kTopkWarps = 4;
 __global__ void router_topk_kernel(const float* __restrict__ logits, int* __restrict__ idx,
                                    float* __restrict__ weight, int n_expert, int k, int stride,
@@ -233,7 +233,7 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int* __rest
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * kTopkWarps + warp;
   if (row >= n_rows) return;
-  float* prob = reinterpret_cast<float*>(smem) + static_cast<size_t>(warp) * n_expert;
+  float* prob = reinterpret_cast<float*>(smem) + static_cast<size_t>(warp) * ((n_expert + 3) & ~3);
   for (int i = lane; i < n_expert; i += 32) prob[i] = logits[static_cast<size_t>(row) * n_expert + i];
   __syncwarp();
   router_select_warp(prob, n_expert, k, idx + static_cast<size_t>(row) * stride,
@@ -296,7 +296,7 @@ SGR_API int sgr_router_topk_batched(const float* logits, int* idx, float* weight
   if (!logits || !idx || !weight || n_expert <= 0 || n_expert_used <= 0 ||
       idx_stride < n_expert_used + 1)
     return kErrArg;
-  const size_t smem = static_cast<size_t>(kTopkWarps) * n_expert * sizeof(float);
+  const size_t smem = static_cast<size_t>(kTopkWarps) * ((n_expert + 3) & ~3) * sizeof(float);
   if (smem > 48 * 1024) return kErrUnsupported;
   return launch_pdl(router_topk_kernel, dim3((n_rows + kTopkWarps - 1) / kTopkWarps), kTopkWarps * 32, smem,
                     as_stream(stream), logits, idx, weight, n_expert, n_expert_used, idx_stride, n_rows, shared_w);

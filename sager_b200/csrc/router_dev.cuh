@@ -56,56 +56,50 @@ __device__ __forceinline__ void router_row_dot(const float* __restrict__ wrow,
   }
 }
 
-// The router dot of two expert rows (one warp) against NT token rows, everything in shared
-// memory as fp32: the rows' weights as they lie in global memory, the activations k-major
-// in planes of four token rows, xs[(t / 4) * 4 * k + kk * 4 + t % 4] (NT = 1, 2:
-// xs[kk * NT + t]). A lane's activations of one k are one 16-byte load per plane and serve
-// both rows. The loop is kept small on purpose: it runs once per CTA, and long unrolled
-// code would spend its time in instruction fetch. The FMAs of a (row, lane, token) chain
-// run in the same order as in router_row_dot, so the logits are bit-identical.
-template <int NT>
-__device__ __forceinline__ void router_fma_k2(float w0, float w1, const float* __restrict__ xs, int k, int kk,
-                                              float (&acc)[2][NT]) {
-  if (NT >= 4) {
+// The logits of R router rows and T token rows by one warp, rows in shared memory: weights [R][k] as they lie in global
+// memory, activations k-major fp16, xs[kk * T + t], so that a lane's T values of one k are one load. The FMAs of a (row,
+// lane, token) chain run in the same order as in router_row_dot, and the shuffle tree adds the same pairs - each step also
+// halves the number of sums a lane carries - so the logits are bit-identical. Lane l returns the sum of (row, token)
+// number l / (32 / (R * T)), row-major.
+template <int R, int T>
+__device__ __forceinline__ float router_tile_dot(const float* ws, const uint16_t* xs, int k, int lane) {
+  float v[R * T];
 #pragma unroll
-    for (int p = 0; p < NT / 4; ++p) {
-      const float4 a = *reinterpret_cast<const float4*>(xs + static_cast<size_t>(p) * 4 * k + static_cast<size_t>(kk) * 4);
-      const float v[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        acc[0][(4 * p + t) % NT] = fmaf(w0, v[t], acc[0][(4 * p + t) % NT]);
-        acc[1][(4 * p + t) % NT] = fmaf(w1, v[t], acc[1][(4 * p + t) % NT]);
-      }
-    }
-  } else if (NT == 2) {
-    const float2 a = *reinterpret_cast<const float2*>(xs + static_cast<size_t>(kk) * 2);
-    acc[0][0] = fmaf(w0, a.x, acc[0][0]); acc[0][1 % NT] = fmaf(w0, a.y, acc[0][1 % NT]);
-    acc[1][0] = fmaf(w1, a.x, acc[1][0]); acc[1][1 % NT] = fmaf(w1, a.y, acc[1][1 % NT]);
-  } else {
-    const float a = xs[kk];
-    acc[0][0] = fmaf(w0, a, acc[0][0]);
-    acc[1][0] = fmaf(w1, a, acc[1][0]);
-  }
-}
-
-template <int NT>
-__device__ __forceinline__ void router_rows2_dot_kmajor(const float* __restrict__ w0s, const float* __restrict__ w1s,
-                                                        const float* __restrict__ xs, int k, int lane,
-                                                        float (&out)[2][NT]) {
-  float acc[2][NT];
-#pragma unroll
-  for (int t = 0; t < NT; ++t) acc[0][t] = acc[1][t] = 0.f;
+  for (int i = 0; i < R * T; ++i) v[i] = 0.f;
 #pragma unroll 4
-  for (int kk = lane; kk < k; kk += 32) router_fma_k2<NT>(w0s[kk], w1s[kk], xs, k, kk, acc);
-#pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      float a = acc[r][t];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, off);
-      out[r][t] = a;
+  for (int kk = lane; kk < k; kk += 32) {
+    uint32_t raw[T / 2];
+    if constexpr (T == 8) {
+      const uint4 q = *reinterpret_cast<const uint4*>(xs + static_cast<size_t>(kk) * T);
+      raw[0] = q.x; raw[1] = q.y; raw[2] = q.z; raw[3] = q.w;
+    } else if constexpr (T == 4) {
+      const uint2 q = *reinterpret_cast<const uint2*>(xs + static_cast<size_t>(kk) * T);
+      raw[0] = q.x; raw[1] = q.y;
+    } else {
+      raw[0] = *reinterpret_cast<const uint32_t*>(xs + static_cast<size_t>(kk) * T);
     }
+    float w[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) w[r] = ws[static_cast<size_t>(r) * k + kk];
+#pragma unroll
+    for (int t = 0; t < T; ++t) {
+      const float x = h2f(static_cast<uint16_t>(raw[t / 2] >> (16 * (t & 1))));
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r * T + t] = fmaf(w[r], x, v[r * T + t]);
+    }
+  }
+  int off = 16;
+#pragma unroll
+  for (int m = R * T / 2; m > 0; m >>= 1, off >>= 1) {
+    const bool up = (lane & off) != 0;
+#pragma unroll
+    for (int i = 0; i < m; ++i) {
+      const float send = up ? v[i] : v[i + m], keep = up ? v[i + m] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, off);
+    }
+  }
+  for (; off > 0; off >>= 1) v[0] += __shfl_xor_sync(0xFFFFFFFFu, v[0], off);
+  return v[0];
 }
 
 // Softmax + top-k of one row by one warp. `prob` is n_expert floats of shared
@@ -263,6 +257,103 @@ __device__ __forceinline__ void router_select_warp(float* prob, int n_expert, in
     for (int kk = 0; kk < k; ++kk) out_w[kk] /= wsum;
   }
   if (lane == 0 && write_shared) out_w[k] = shared_w;
+}
+
+static __device__ __noinline__ void router_select_general(float* prob, int E, int K, int* idx, float* w, float shared_w, int lane) {
+  router_select_warp(prob, E, K, idx, w, shared_w, true, lane);
+}
+
+// Softmax and top-K of one token row by two warps (up to 256 experts, K < 32). The strictly serial sum of the
+// exponentials - the reference's order - is long, so one warp picks the K + 1 largest exponentials and goes on to build
+// what follows from them (`picked()`) while the other adds and makes the weights. Dividing by the sum keeps
+// the order; only if it makes two of them equal, or something is not finite, the order of the quotients could be another
+// one, and the adding warp runs the general selection on the quotients: it returns true, and the picks do not stand.
+// `logits` in global memory, `prob` (E) and `pick_e` (K + 1) in shared memory, `bar` a barrier of the two warps.
+template <typename Picked>
+__device__ __forceinline__ bool router_select_pair(const float* logits, float* prob, float* pick_e, int* idx, float* w, int bar, bool adds, int E,
+                                            int K, float shared_w, int lane, Picked picked) {
+  float e[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) e[j] = lane + 32 * j < E ? __ldcg(logits + lane + 32 * j) : -1e30f;
+  float mx = -1e30f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, e[j]);
+  {                                                // warp maximum through an order-preserving integer key
+    const int b = __float_as_int(mx);
+    const int mk = __reduce_max_sync(0xFFFFFFFFu, b ^ ((b >> 31) & 0x7FFFFFFF));
+    mx = __int_as_float(mk ^ ((mk >> 31) & 0x7FFFFFFF));
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) e[j] = expf(e[j] - mx);
+  if (!adds) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (lane + 32 * j >= E) e[j] = -1.f;
+    // a lane's eight in descending order (Batcher's network), then the warp takes the largest head K + 1 times
+    int sl[8] = {0, 1, 2, 3, 4, 5, 6, 7};
+    auto ce = [&](int a, int b) {
+      const bool sw = e[b] > e[a];
+      const float x = fmaxf(e[a], e[b]), y = fminf(e[a], e[b]);
+      const int i = sw ? sl[b] : sl[a], j = sw ? sl[a] : sl[b];
+      e[a] = x; e[b] = y; sl[a] = i; sl[b] = j;
+    };
+    ce(0, 1); ce(2, 3); ce(4, 5); ce(6, 7);
+    ce(0, 2); ce(1, 3); ce(4, 6); ce(5, 7);
+    ce(1, 2); ce(5, 6); ce(0, 4); ce(3, 7);
+    ce(1, 5); ce(2, 6);
+    ce(1, 4); ce(3, 6);
+    ce(2, 4); ce(3, 5);
+    ce(3, 4);
+    float my_e = -1.f;
+    int my_i = 0;
+#pragma unroll 1
+    for (int kk = 0; kk <= K; ++kk) {
+      const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(e[0]));        // values are >= 0 or -1
+      const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(e[0]) == top ? lane + 32 * sl[0] : 0x7FFFFFFF);
+      if ((win & 31) == lane) {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) { e[j] = e[j + 1]; sl[j] = sl[j + 1]; }
+        e[7] = -1.f;
+      }
+      if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
+    }
+    my_i = min(my_i, E - 1);                     // (with NaNs about, a lane's filler could be picked: not fine below)
+    if (lane < K) idx[lane] = my_i;
+    if (lane <= K) pick_e[lane] = my_e;
+    __syncwarp();
+    asm volatile("bar.arrive %0, 64;" ::"r"(bar) : "memory");
+    picked();
+    return false;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (lane + 32 * j < E) prob[lane + 32 * j] = e[j];
+  __syncwarp();
+  float z = 0.f;                                 // every lane adds: the same broadcast reads
+  int i = 0;
+#pragma unroll 4
+  for (; i + 8 <= E; i += 8) {
+    const float4 a = *reinterpret_cast<const float4*>(prob + i), b = *reinterpret_cast<const float4*>(prob + i + 4);
+    z += a.x; z += a.y; z += a.z; z += a.w; z += b.x; z += b.y; z += b.z; z += b.w;
+  }
+  for (; i < E; ++i) z += prob[i];
+  asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+  const float my_e = lane <= K ? pick_e[lane] : -1.f;
+  const float p = my_e / z;
+  const float next = __shfl_down_sync(0xFFFFFFFFu, p, 1);
+  const bool fine = z > 0.f && z <= 3.4e38f && __all_sync(0xFFFFFFFFu, lane >= K || (my_e >= 0.f && p > next));
+  if (fine) {
+    float wsum = 0.f;
+    for (int kk = 0; kk < K; ++kk) wsum += __shfl_sync(0xFFFFFFFFu, p, kk);
+    if (lane < K) w[lane] = wsum > 0.f ? p / wsum : p;
+    if (lane == 0) w[K] = shared_w;
+  } else {
+    __syncwarp();
+    for (int m = lane; m < E; m += 32) prob[m] = __ldcg(logits + m);
+    __syncwarp();
+    router_select_general(prob, E, K, idx, w, shared_w, lane);
+  }
+  return !fine;
 }
 
 }  // namespace sgr

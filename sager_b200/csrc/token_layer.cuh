@@ -100,7 +100,7 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
   const int hrows = n * (K + 1);                            // (tile, row) pairs at most
   size_t p = kHdr + kTables;
   auto take = [&](size_t bytes) { const size_t at = p; p = (p + bytes + 127) & ~static_cast<size_t>(127); return at; };
-  g.off_prob = take(static_cast<size_t>(n) * E * 4);
+  g.off_prob = take(static_cast<size_t>(n) * ((E + 3) & ~3) * 4);                // rows at 16-byte steps
   g.off_ptab = take(static_cast<size_t>(3) * E * 8);        // the layer's pointer table, read once per CTA
   // x rows as fp16 and the router rows; later the same bytes hold the quantised h rows
   const size_t a = static_cast<size_t>(n) * H * 2 + 128 + static_cast<size_t>(g.rows_per_cta) * H * 4;
@@ -350,102 +350,6 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
       if (q < tasks && half == 0 && lr == 0) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(g, u);
     }
   }
-}
-
-__device__ __noinline__ void select_general(float* prob, int E, int K, int* idx, float* w, float shared_w, int lane) {
-  router_select_warp(prob, E, K, idx, w, shared_w, true, lane);
-}
-
-// Softmax and top-K of one token row by two warps (up to 256 experts, K < 32). The strictly serial sum of the
-// exponentials - the reference's order - is long, so one warp picks the K + 1 largest exponentials and goes on to build
-// the tables from them (`picked()`) while the other adds and makes the weights. Dividing by the sum keeps
-// the order; only if it makes two of them equal, or something is not finite, the order of the quotients could be another
-// one, and the adding warp runs the general selection on the quotients: it returns true, and the picks do not stand.
-template <typename Picked>
-__device__ __forceinline__ bool select_pair(const float* logits, float* prob, Tables& tb, int t, bool adds, int E, int K, float shared_w,
-                                            int lane, Picked picked) {
-  float e[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) e[j] = lane + 32 * j < E ? __ldcg(logits + lane + 32 * j) : -1e30f;
-  float mx = -1e30f;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) mx = fmaxf(mx, e[j]);
-  {                                                // warp maximum through an order-preserving integer key
-    const int b = __float_as_int(mx);
-    const int mk = __reduce_max_sync(0xFFFFFFFFu, b ^ ((b >> 31) & 0x7FFFFFFF));
-    mx = __int_as_float(mk ^ ((mk >> 31) & 0x7FFFFFFF));
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) e[j] = expf(e[j] - mx);
-  if (!adds) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (lane + 32 * j >= E) e[j] = -1.f;
-    // a lane's eight in descending order (Batcher's network), then the warp takes the largest head K + 1 times
-    int sl[8] = {0, 1, 2, 3, 4, 5, 6, 7};
-    auto ce = [&](int a, int b) {
-      const bool sw = e[b] > e[a];
-      const float x = fmaxf(e[a], e[b]), y = fminf(e[a], e[b]);
-      const int i = sw ? sl[b] : sl[a], j = sw ? sl[a] : sl[b];
-      e[a] = x; e[b] = y; sl[a] = i; sl[b] = j;
-    };
-    ce(0, 1); ce(2, 3); ce(4, 5); ce(6, 7);
-    ce(0, 2); ce(1, 3); ce(4, 6); ce(5, 7);
-    ce(1, 2); ce(5, 6); ce(0, 4); ce(3, 7);
-    ce(1, 5); ce(2, 6);
-    ce(1, 4); ce(3, 6);
-    ce(2, 4); ce(3, 5);
-    ce(3, 4);
-    float my_e = -1.f;
-    int my_i = 0;
-#pragma unroll 1
-    for (int kk = 0; kk <= K; ++kk) {
-      const int top = __reduce_max_sync(0xFFFFFFFFu, __float_as_int(e[0]));        // values are >= 0 or -1
-      const int win = __reduce_min_sync(0xFFFFFFFFu, __float_as_int(e[0]) == top ? lane + 32 * sl[0] : 0x7FFFFFFF);
-      if ((win & 31) == lane) {
-#pragma unroll
-        for (int j = 0; j < 7; ++j) { e[j] = e[j + 1]; sl[j] = sl[j + 1]; }
-        e[7] = -1.f;
-      }
-      if (lane == kk) { my_e = __int_as_float(top); my_i = win; }
-    }
-    my_i = min(my_i, E - 1);                     // (with NaNs about, a lane's filler could be picked: not fine below)
-    if (lane < K) tb.sel_idx[t][lane] = my_i;
-    if (lane <= K) tb.pick_e[t][lane] = my_e;
-    __syncwarp();
-    asm volatile("bar.arrive %0, 64;" ::"r"(8 + t) : "memory");
-    picked();
-    return false;
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    if (lane + 32 * j < E) prob[lane + 32 * j] = e[j];
-  __syncwarp();
-  float z = 0.f;                                 // every lane adds: the same broadcast reads
-  int i = 0;
-#pragma unroll 4
-  for (; i + 8 <= E; i += 8) {
-    const float4 a = *reinterpret_cast<const float4*>(prob + i), b = *reinterpret_cast<const float4*>(prob + i + 4);
-    z += a.x; z += a.y; z += a.z; z += a.w; z += b.x; z += b.y; z += b.z; z += b.w;
-  }
-  for (; i < E; ++i) z += prob[i];
-  named_sync(8 + t, 64);
-  const float my_e = lane <= K ? tb.pick_e[t][lane] : -1.f;
-  const float p = my_e / z;
-  const float next = __shfl_down_sync(0xFFFFFFFFu, p, 1);
-  const bool fine = z > 0.f && z <= 3.4e38f && __all_sync(0xFFFFFFFFu, lane >= K || (my_e >= 0.f && p > next));
-  if (fine) {
-    float wsum = 0.f;
-    for (int kk = 0; kk < K; ++kk) wsum += __shfl_sync(0xFFFFFFFFu, p, kk);
-    if (lane < K) tb.sel_w[t][lane] = wsum > 0.f ? p / wsum : p;
-    if (lane == 0) tb.sel_w[t][K] = shared_w;
-  } else {
-    __syncwarp();
-    for (int m = lane; m < E; m += 32) prob[m] = __ldcg(logits + m);
-    __syncwarp();
-    select_general(prob, E, K, tb.sel_idx[t], tb.sel_w[t], shared_w, lane);
-  }
-  return !fine;
 }
 
 // Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned.
@@ -828,10 +732,10 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int t = warp & (kMaxTok - 1);
     const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
     const float* lg = L.logits + static_cast<size_t>(t) * E;
-    float* pr = prob + static_cast<size_t>(t) * E;
+    float* pr = prob + static_cast<size_t>(t) * ((E + 3) & ~3);
     if (!there) ok = false;                      // (the named barriers below need every warp: it goes on with what is there)
     if (by_pairs) {
-      const bool redo = select_pair(lg, pr, tb, t, warp >= kMaxTok, E, K, L.shared_w, lane, [&] {
+      const bool redo = router_select_pair(lg, pr, tb.pick_e[t], tb.sel_idx[t], tb.sel_w[t], 8 + t, warp >= kMaxTok, E, K, L.shared_w, lane, [&] {
         if (n == 1) asm volatile("bar.arrive 13, %0;" ::"n"(32 + kGroupThreads) : "memory");   // the second group fetches
         else named_sync(12, n * 32);             // every row's picks are in the tables
         if (warp == 0) build();
@@ -842,7 +746,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     } else if (warp < kMaxTok && there) {
       for (int i = lane; i < E; i += 32) pr[i] = __ldcg(lg + i);
       __syncwarp();
-      select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
+      router_select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
     }
   }
   if (warp >= kGroupWarps && by_pairs && n == 1) {

@@ -484,6 +484,7 @@ def test_token_kernel_agrees_with_the_two_launch_path(full_w):
     (768, 512, 300, 3, 2, False),      # more experts than one selecting warp holds
     (512, 256, 40, 4, 1, True),        # picks that do not stand: every logit twice, the lower expert goes first
     (512, 256, 40, 4, 3, True),
+    (512, 256, 10, 4, 3, False),       # rows of probabilities that are no multiple of sixteen bytes
 ])
 def test_token_kernel_edges(hidden, n_ff, E, k, n, ties):
     """The same routing and, to fp32 rounding of the same terms (1e-5), the same layer as route + expert kernel."""
@@ -498,6 +499,25 @@ def test_token_kernel_edges(hidden, n_ff, E, k, n, ties):
     if ties:
         first = r0.route_idx[:n, 0].cpu().numpy()
         assert (first < E // 2).all() and (r0.route_idx[:n, 1].cpu().numpy() == first + E // 2).all()
+
+
+@pytest.mark.parametrize("E,k,n", [
+    (10, 4, 9),        # two experts per route CTA, a token tile of one row
+    (40, 8, 33),       # two per CTA, five tiles
+    (80, 8, 40),       # four per CTA
+    (160, 6, 61),      # sixteen per CTA, a ragged last tile
+    (256, 8, 30),      # eight per CTA
+    (300, 3, 20),      # more experts than two selecting warps hold
+])
+def test_route_kernel_edges(oracle, E, k, n):
+    """Every split of the logits over CTAs and warps: the oracle's picks, weights to its fp32 rounding."""
+    w = synth.MoeWeights(512, 256, E, DEV, seed=90, std=0.05, distinct=4)
+    x16 = synth.normal_fp16((n, 512), 91 + E, DEV)
+    runner, _, _ = run_layer(w, n, k, x16, n_max=64, kernel="two_launch")
+    idx, wt = runner.route_idx.cpu().numpy(), runner.route_w.cpu().numpy()
+    for t in range(n):
+        i, v = oracle.router_topk(oracle.router_logits(w.router.cpu().numpy(), x16.cpu().numpy()[t]), k)
+        assert np.array_equal(idx[t, :k], i[:k]) and np.abs(wt[t, :k] - v[:k]).max() <= 1e-6
 
 
 @pytest.mark.parametrize("own_plan", [False, True])
