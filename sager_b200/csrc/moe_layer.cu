@@ -414,33 +414,37 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev 
     }
   }
 
-  // stage: lane = one k of a 32-wide chunk, all rows of the tile (rows beyond nt read as
-  // zero); four chunks per pass, so that all loads of a pass are in flight together
+  // stage: a lane takes two k of all rows of the tile (rows beyond nt read as zero), a warp 64; two such
+  // chunks per pass, so that all loads of a pass are in flight together
   const int tsh = rows >= 16 ? 3 : (rows >= 4 ? 2 : 1);          // token rows per group: 8, 4 or 2
-  for (int c0 = warp; c0 < L.H / 32; c0 += 4 * kRouteWarps) {
-    uint16_t raw[4][kRouteTok];
+  for (int c0 = warp; c0 < L.H / 64; c0 += 2 * kRouteWarps) {
+    uint32_t raw[2][kRouteTok];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = (c0 + u * kRouteWarps) * 32 + lane;
+    for (int u = 0; u < 2; ++u) {
+      const int k = (c0 + u * kRouteWarps) * 64 + 2 * lane;
 #pragma unroll
       for (int t = 0; t < kRouteTok; ++t)
-        raw[u][t] = (t < nt && k < L.H) ? L.xn[static_cast<size_t>(tok0 + t) * L.H + k] : static_cast<uint16_t>(0);
+        raw[u][t] = (t < nt && k < L.H) ? *reinterpret_cast<const uint32_t*>(L.xn + static_cast<size_t>(tok0 + t) * L.H + k) : 0u;
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = (c0 + u * kRouteWarps) * 32 + lane;
-      if (k >= L.H) continue;
-      uint32_t q[4];
+    for (int u = 0; u < 2; ++u) {
+      const int k0 = (c0 + u * kRouteWarps) * 64 + 2 * lane;
+      if (k0 >= L.H) continue;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = raw[u][2 * i] | (static_cast<uint32_t>(raw[u][2 * i + 1]) << 16);
-      if (tsh == 3) {
-        *reinterpret_cast<uint4*>(xs + static_cast<size_t>(k) * 8) = make_uint4(q[0], q[1], q[2], q[3]);
-      } else if (tsh == 2) {
-        *reinterpret_cast<uint2*>(xs + static_cast<size_t>(k) * 4) = make_uint2(q[0], q[1]);
-        *reinterpret_cast<uint2*>(xs + static_cast<size_t>(L.H + k) * 4) = make_uint2(q[2], q[3]);
-      } else {
+      for (int h = 0; h < 2; ++h) {
+        const int k = k0 + h;
+        uint32_t q[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(xs + static_cast<size_t>(i * L.H + k) * 2) = q[i];
+        for (int i = 0; i < 4; ++i) q[i] = __byte_perm(raw[u][2 * i], raw[u][2 * i + 1], h ? 0x7632 : 0x5410);
+        if (tsh == 3) {
+          *reinterpret_cast<uint4*>(xs + static_cast<size_t>(k) * 8) = make_uint4(q[0], q[1], q[2], q[3]);
+        } else if (tsh == 2) {
+          *reinterpret_cast<uint2*>(xs + static_cast<size_t>(k) * 4) = make_uint2(q[0], q[1]);
+          *reinterpret_cast<uint2*>(xs + static_cast<size_t>(L.H + k) * 4) = make_uint2(q[2], q[3]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(xs + static_cast<size_t>(i * L.H + k) * 2) = q[i];
+        }
       }
     }
   }

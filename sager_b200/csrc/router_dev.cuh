@@ -66,27 +66,44 @@ __device__ __forceinline__ float router_tile_dot(const float* ws, const uint16_t
   float v[R * T];
 #pragma unroll
   for (int i = 0; i < R * T; ++i) v[i] = 0.f;
-#pragma unroll 4
-  for (int kk = lane; kk < k; kk += 32) {
-    uint32_t raw[T / 2];
-    if constexpr (T == 8) {
-      const uint4 q = *reinterpret_cast<const uint4*>(xs + static_cast<size_t>(kk) * T);
-      raw[0] = q.x; raw[1] = q.y; raw[2] = q.z; raw[3] = q.w;
-    } else if constexpr (T == 4) {
-      const uint2 q = *reinterpret_cast<const uint2*>(xs + static_cast<size_t>(kk) * T);
-      raw[0] = q.x; raw[1] = q.y;
-    } else {
-      raw[0] = *reinterpret_cast<const uint32_t*>(xs + static_cast<size_t>(kk) * T);
+  // the loads of S steps are issued ahead of the FMAs of the S steps before (k is a multiple of 256: S divides the steps)
+  constexpr int S = T == 2 ? 8 : 4;
+  uint32_t raw[2][S][T / 2];
+  float w[2][S][R];
+  auto load = [&](int b, int kk) {
+#pragma unroll
+    for (int j = 0; j < S; ++j) {
+      const uint16_t* x = xs + static_cast<size_t>(kk + 32 * j) * T;
+      if constexpr (T == 8) {
+        const uint4 q = *reinterpret_cast<const uint4*>(x);
+        raw[b][j][0] = q.x; raw[b][j][1] = q.y; raw[b][j][2] = q.z; raw[b][j][3] = q.w;
+      } else if constexpr (T == 4) {
+        const uint2 q = *reinterpret_cast<const uint2*>(x);
+        raw[b][j][0] = q.x; raw[b][j][1] = q.y;
+      } else {
+        raw[b][j][0] = *reinterpret_cast<const uint32_t*>(x);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[b][j][r] = ws[static_cast<size_t>(r) * k + kk + 32 * j];
     }
-    float w[R];
+  };
+  auto add = [&](int b) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) w[r] = ws[static_cast<size_t>(r) * k + kk];
+    for (int j = 0; j < S; ++j)
 #pragma unroll
-    for (int t = 0; t < T; ++t) {
-      const float x = h2f(static_cast<uint16_t>(raw[t / 2] >> (16 * (t & 1))));
+      for (int t = 0; t < T; ++t) {
+        const float x = h2f(static_cast<uint16_t>(raw[b][j][t / 2] >> (16 * (t & 1))));
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[r * T + t] = fmaf(w[r], x, v[r * T + t]);
-    }
+        for (int r = 0; r < R; ++r) v[r * T + t] = fmaf(w[b][j][r], x, v[r * T + t]);
+      }
+  };
+  load(0, lane);
+#pragma unroll 1
+  for (int kk = lane; kk < k; kk += 2 * S * 32) {
+    if (kk + S * 32 < k) load(1, kk + S * 32);             // warp-uniform
+    add(0);
+    if (kk + 2 * S * 32 < k) load(0, kk + 2 * S * 32);
+    if (kk + S * 32 < k) add(1);
   }
   int off = 16;
 #pragma unroll
