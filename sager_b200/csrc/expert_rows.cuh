@@ -43,9 +43,10 @@ namespace rs {
 constexpr int kTok = 16;                        // token rows per tile
 constexpr int kConsumerWarps = 16;
 constexpr int kConsumers = kConsumerWarps * 32;
-constexpr int kXWarps = 3;                      // activation-row producers
+constexpr int kXWarps = 2;                      // activation-row producers
 constexpr int kXThreads = kXWarps * 32;
-constexpr int kThreads = kConsumers + 32 + kXThreads + 32;      // consumers, weight warp, activation warps, finisher warp
+constexpr int kPrepWarp = kConsumerWarps, kWeightWarp = kPrepWarp + 1, kFirstXWarp = kWeightWarp + 1, kFinishWarp = kFirstXWarp + kXWarps;
+constexpr int kThreads = (kFinishWarp + 1) * 32;
 constexpr int kStageCount = 5;
 constexpr int kHalfRows = 128;                  // a stage is two halves of 128 rows
 constexpr int kHalfBytes = kHalfRows * kW4;     // 18432
@@ -55,7 +56,7 @@ constexpr int kXCodes = kTok * kXqStride;
 constexpr int kXBytes = kXCodes + kTok * 16 + kTok * 16;
 constexpr int kStageBytes = (kWBytes + kXBytes + 127) & ~127;
 constexpr int kHq = 288;                        // padded Q8_K block of h: d | 12 bytes | 256 codes | 8 sums
-constexpr int kHdr = 4096;
+constexpr int kHdr = 4608;
 // The plan of a layer, built by every CTA for itself when the routing was made by this call's own
 // route kernel: row masks [E] | offsets [E + 1] | scan scratch | tile records | rows of the slots | slot
 // of every route. One round trip for the routing and a few barriers per CTA, all CTAs at once, instead
@@ -64,18 +65,19 @@ constexpr int kPlanExperts = 256, kPlanRoutes = 512;
 constexpr int kPlanTiles = kPlanExperts + kPlanRoutes / kTok + 8;     // a tile per expert, per further 16 rows, shared expert's
 constexpr int kPlanOffMask = 0, kPlanOffOff = kPlanExperts * 8, kPlanOffScan = kPlanOffOff + 1152;
 constexpr int kPlanOffRec = kPlanOffScan + 512, kPlanOffRows = kPlanOffRec + kPlanTiles * 16;
-constexpr int kPlanOffSlot = kPlanOffRows + kPlanRoutes * 4;
-constexpr int kPlanBytes = (kPlanOffSlot + kPlanRoutes * 4 + 127) & ~127;
+constexpr int kPlanOffSlot = kPlanOffRows + kPlanRoutes;               // (a source row is below 64: one byte)
+constexpr int kPlanOffTab = kPlanOffSlot + kPlanRoutes * 4;             // the layer's pointer table [3][E]
+constexpr int kPlanBytes = (kPlanOffTab + 3 * kPlanExperts * 8 + 127) & ~127;
 constexpr size_t kSmem = kHdr + kPlanBytes + static_cast<size_t>(kStageCount) * kStageBytes;
 constexpr int kGateUpPairs = 128;               // pairs per gate/up group
 constexpr int kDownRows = 256;                  // rows per down group
 constexpr int kFullArrivals = 1 + kXThreads;      // weight warp: one arrival; activation warps: a thread's copies landed
-constexpr int kMapRing = kStageCount + 1;        // descriptor slots per CTA: a slot is patched again only after every
-                                                 // stage that could still reference it has been refilled (a tile has at
-                                                 // least one stage, and at most kStageCount stages are in flight)
+constexpr int kAhead = AH;                        // stages of published groups that the weight warp is kept ahead with
+constexpr int kMapRing = kAhead + kStageCount + 2;   // descriptor slots per CTA: groups (of one stage at least) that are
+                                                 // published and not issued, in flight, and the one being patched
 
 static_assert(kSmem <= 227 * 1024, "ring exceeds shared memory");
-static_assert(kMapRing <= kTmapSlots, "the workspace holds kTmapSlots descriptor sets per CTA");
+static_assert(kMapRing <= kTmapSlots, "the workspace holds kTmapSlots descriptor pairs per CTA");
 
 struct Desc {     // one 16-byte shared-memory load per stage and warp
   int flags;     // bit 0 kind (0 gate/up, 1 down), bit 1 expert absent, bits 2-7 token rows,
@@ -166,64 +168,63 @@ struct Sched {
     return r;
   }
 };
-constexpr int kListSlots = 16;
+constexpr int kListSlots = 32;
 
-// One entry of a CTA's group list, published by the weight warp one group ahead of its copies,
-// with everything the other roles would otherwise fetch from global memory again.
-struct GEntry {
+// One entry of a CTA's group list, published by the preparing warp some stages ahead of the copies,
+// with everything the other roles would otherwise fetch from global memory again. A reader lags by at
+// most kAhead + kStageCount + 1 groups and the done queue's.
+struct alignas(16) GEntry {
   int id;          // global group number, -1 = end of this CTA's list
-  int absent;      // bit 0: the expert's pointers are null; bit 1 (down groups): the tile's h was already published
-                   // when the weight warp looked
+  int bits;        // bit 0: the expert's pointers are null; bit 1 (down groups): the tile's h was already published
+                   // when the preparing warp looked; bit 2: the pointers are 16-byte aligned
+  const unsigned char* maps;    // the group's descriptors
   int4 rc;         // the tile's record: expert, token rows, first h / y row, first entry of grows
-  int rows[kTok];  // gate/up groups: source row of the tile's token slot t in the quantised inputs
+  const unsigned char* w[3];    // the expert's matrices
+  unsigned char rows[kTok];     // gate/up groups: source row of the tile's token slot t in the quantised inputs
 };
+static_assert(kListSlots >= kAhead + kStageCount + 1 + kDoneSlots + 1, "a reader could be overtaken");
 static_assert(sizeof(GEntry) * kListSlots + 2048 <= kHdr, "group list exceeds the header");
 
 // One warp: Q8_K-quantise block `hb` of the fp32 h rows [hrow0, hrow0 + ntok) into the
 // padded rows of L.hq (arithmetic of src/kernels/cpu/q4_avx2.cpp:77-94 in the reference,
-// the same as stage_quantized_f32). Two rows per pass keep two sets of loads in flight.
-__device__ __forceinline__ void quantize_h_block(const LayerDev& L, int hrow0, int ntok, int hb, int lane) {
+// the same as stage_quantized_f32). The down groups of the tile wait for it, and beside sixteen
+// consumer warps a chain of instructions takes ten cycles each: R rows go through it side by side
+// (one after the other, a row took 0.85 us).
+template <int R>
+__device__ __forceinline__ void quantize_h_rows(const LayerDev& L, int hrow0, int ntok, int hb, int lane) {
   const size_t hq_stride = static_cast<size_t>(L.nbf) * kHq;
-  for (int t0 = 0; t0 < ntok; t0 += 2) {
-    float4 a[2], b[2];
+  float4 a[R], b[R];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int t = min(t0 + u, ntok - 1);
-      const float4* p = reinterpret_cast<const float4*>(L.hbuf + static_cast<size_t>(hrow0 + t) * L.FF + hb * kQK) + lane * 2;
-      a[u] = __ldcg(p);
-      b[u] = __ldcg(p + 1);
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int t = t0 + u;
-      if (t >= ntok) break;                      // warp-uniform
-      const float v[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
-      float m = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) m = fmaxf(m, fabsf(v[i]));
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
-      const float amax = fmaxf(1e-30f, m);
-      const float d = amax / 127.f;
-      const float id = d > 0.f ? 1.f / d : 0.f;
-      int q[8], sum = 0;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        q[i] = max(-127, min(127, static_cast<int>(rintf(v[i] * id))));
-        sum += q[i];
-      }
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 1);
-      sum += __shfl_xor_sync(0xFFFFFFFFu, sum, 2);
-      const int sum_next = __shfl_down_sync(0xFFFFFFFFu, sum, 4);
-      uint32_t* o32 = reinterpret_cast<uint32_t*>(L.hq + static_cast<size_t>(hrow0 + t) * hq_stride + hb * kHq);
-      if (lane == 0) o32[0] = __float_as_uint(d);
-      *reinterpret_cast<uint2*>(o32 + 4 + 2 * lane) =
-          make_uint2((q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) | (static_cast<uint32_t>(q[3] & 0xFF) << 24),
-                     (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) | (static_cast<uint32_t>(q[7] & 0xFF) << 24));
-      if ((lane & 7) == 0)
-        o32[68 + (lane >> 3)] = (static_cast<uint32_t>(sum) & 0xFFFFu) | (static_cast<uint32_t>(sum_next) << 16);
-    }
+  for (int u = 0; u < R; ++u) {
+    const float4* p = reinterpret_cast<const float4*>(L.hbuf + static_cast<size_t>(hrow0 + min(u, ntok - 1)) * L.FF + hb * kQK) + lane * 2;
+    a[u] = __ldcg(p);
+    b[u] = __ldcg(p + 1);
   }
+  uint32_t lo[R], hi[R], sums[R];
+  float d[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    const float v[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
+    int q[8], sum;
+    d[u] = quantize_lane8(v, q, sum);
+    lo[u] = (q[0] & 0xFF) | ((q[1] & 0xFF) << 8) | ((q[2] & 0xFF) << 16) | (static_cast<uint32_t>(q[3] & 0xFF) << 24);
+    hi[u] = (q[4] & 0xFF) | ((q[5] & 0xFF) << 8) | ((q[6] & 0xFF) << 16) | (static_cast<uint32_t>(q[7] & 0xFF) << 24);
+    sums[u] = (static_cast<uint32_t>(sum) & 0xFFFFu) | (static_cast<uint32_t>(__shfl_down_sync(0xFFFFFFFFu, sum, 4)) << 16);
+  }
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    if (u >= ntok) break;                        // warp-uniform
+    uint32_t* o32 = reinterpret_cast<uint32_t*>(L.hq + static_cast<size_t>(hrow0 + u) * hq_stride + hb * kHq);
+    if (lane == 0) o32[0] = __float_as_uint(d[u]);
+    *reinterpret_cast<uint2*>(o32 + 4 + 2 * lane) = make_uint2(lo[u], hi[u]);
+    if ((lane & 7) == 0) o32[68 + (lane >> 3)] = sums[u];
+  }
+}
+__device__ __forceinline__ void quantize_h_block(const LayerDev& L, int hrow0, int ntok, int hb, int lane) {
+  int t0 = 0;
+#pragma unroll 1
+  for (; ntok - t0 > 2; t0 += 4) quantize_h_rows<4>(L, hrow0 + t0, ntok - t0, hb, lane);
+  if (ntok - t0 > 0) quantize_h_rows<2>(L, hrow0 + t0, ntok - t0, hb, lane);
 }
 
 // Every thread of the CTA: the plan of build_plan (moe_layer.cu) in shared memory - same masks, same
@@ -235,11 +236,16 @@ __device__ __forceinline__ int build_plan_shared(const LayerDev& L, unsigned cha
   int* off_s = reinterpret_cast<int*>(ps + kPlanOffOff);
   int* scan = reinterpret_cast<int*>(ps + kPlanOffScan);          // [3][40]: warp totals of rows, tiles, heavy tiles; [120]: bad ids
   int4* rec_s = reinterpret_cast<int4*>(ps + kPlanOffRec);
-  int* rows_s = reinterpret_cast<int*>(ps + kPlanOffRows);
+  unsigned char* rows_s = ps + kPlanOffRows;
   int* slot_s = reinterpret_cast<int*>(ps + kPlanOffSlot);
   const int lane = tid & 31, wp = tid >> 5;
   const int total = L.n * L.K;
   // (the masks and the count of bad ids were cleared before the wait for the route kernel)
+  for (int i = tid; i < 3 * L.E; i += kThreads) {                 // the layer's pointer table, beside everything else
+    const int m = i >= 2 * L.E ? 2 : (i >= L.E ? 1 : 0);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(ps + kPlanOffTab + i * 8)),
+                 "l"(L.tab + static_cast<size_t>(m) * L.tab_stride + (i - m * L.E)) : "memory");
+  }
   int my_e = -1, my_r = 0;
   if (tid < total) {                            // kPlanRoutes <= kThreads: a route per thread
     my_r = tid / L.K;
@@ -303,7 +309,7 @@ __device__ __forceinline__ int build_plan_shared(const LayerDev& L, unsigned cha
     int pos = -1;
     if (my_e >= 0) {
       pos = off_s[my_e] + __popcll(mask[my_e] & ((1ull << my_r) - 1ull));
-      rows_s[pos] = my_r;
+      rows_s[pos] = static_cast<unsigned char>(my_r);
     }
     slot_s[tid] = pos;
   }
@@ -313,6 +319,7 @@ __device__ __forceinline__ int build_plan_shared(const LayerDev& L, unsigned cha
     L.meta[2] = scan[120];
     L.meta[3] = sh_tiles;
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   return tiles_total + sh_tiles;
 }
@@ -342,11 +349,21 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     *done_tail = 0u;
     *done_head = 0u;
     *reinterpret_cast<volatile unsigned*>(smem + 144) = 0u;
+    *reinterpret_cast<volatile unsigned*>(smem + 148) = 0u;
     fence_barrier_init();
   }
   if (L.plan_in_kernel) {           // shared memory of the plan that must start out clear
     for (int e = tid; e < kPlanExperts; e += kThreads) reinterpret_cast<unsigned long long*>(plan_s + kPlanOffMask)[e] = 0ull;
     if (tid == 0) reinterpret_cast<int*>(plan_s + kPlanOffScan)[120] = 0;
+  }
+  unsigned char* smaps = smem + 1024;                                 // three 128-byte descriptors being patched
+  uint32_t* tmpl = reinterpret_cast<uint32_t*>(smem + 1408);          // the two host-made descriptors
+  if (tid == kPrepWarp * 32) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {               // constant indices only (see LayerDev)
+      tmpl[i] = L.tmap_gu[i];
+      tmpl[32 + i] = L.tmap_dn[i];
+    }
   }
   __syncthreads();
   pdl_wait();                       // routing and quantised rows (and, without a plan of its own, the plan) come from the route kernel
@@ -373,7 +390,6 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   }
   const int n_tiles = plan_own ? build_plan_shared(L, plan_s, tid) : L.meta[1];
   const int4* rec_p = plan_own ? reinterpret_cast<const int4*>(plan_s + kPlanOffRec) : L.rec;
-  const int* rows_p = plan_own ? reinterpret_cast<const int*>(plan_s + kPlanOffRows) : L.grows;
   const int* slot_p = plan_own ? reinterpret_cast<const int*>(plan_s + kPlanOffSlot) : L.gslot;
   auto tile_rec = [&](int tile) { return plan_own ? rec_p[tile] : __ldcg(rec_p + tile); };
   sc.n_gu = n_tiles * sc.gpt_gu;
@@ -381,134 +397,139 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   const int rb_h = L.nbh * kW4, rb_f = L.nbf * kW4;
   GEntry* glist = reinterpret_cast<GEntry*>(smem + 2048);                       // [kListSlots] this CTA's groups
   volatile unsigned* g_pub = reinterpret_cast<volatile unsigned*>(smem + 144);  // entries of glist published
-  // a follower role's k-th group (bounded wait for the weight warp to publish it); an entry stays
-  // valid for kListSlots further groups, far longer than any role can lag behind the ring
+  volatile unsigned* issued = reinterpret_cast<volatile unsigned*>(smem + 148); // stages the weight warp has issued
+  // a follower role's k-th group (bounded wait for the preparing warp to publish it)
   auto follow = [&](int k, bool& ok) -> const GEntry* {
     unsigned it = 0;
     if (lane == 0)
-      while (*g_pub <= static_cast<unsigned>(k) && ++it < kSpinLimit) __nanosleep(40);
+      while (*g_pub <= static_cast<unsigned>(k) && ++it < kSpinLimit) __nanosleep(20);
     it = __shfl_sync(0xFFFFFFFFu, it, 0);
     ok = it < kSpinLimit;
     __threadfence_block();
     return glist + k % kListSlots;
   };
 
-  if (warp == kConsumerWarps) {
-    // ---------------- weight warp ----------------
-    // Streams group k while it prepares group k + 1: the tile's record is requested between two
-    // copies of group k, the expert's pointers (and the token slots' source rows) after its last copy,
-    // and the descriptors are patched once the group's copies are all issued - so these global round
-    // trips and the descriptor update overlap the stream. A group's number is drawn as late as that
-    // allows: a number drawn is a group that no other CTA can take, and a gate/up group that waits
-    // long for its CTA delays its tile's h, on which eight down groups elsewhere depend. So the next
-    // number is drawn four stages before the current group ends - or, when the group it follows is a
-    // short down group, as soon as that one's number is known.
-    unsigned char* smaps = smem + 1024;                                 // three 128-byte descriptors being patched
-    uint32_t* tmpl = reinterpret_cast<uint32_t*>(smem + 1408);          // the two host-made descriptors
-    unsigned char* gmaps = L.tmaps + static_cast<size_t>(blockIdx.x) * kMapRing * 3 * 128;
-    if (lane == 0) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {             // constant indices only (see LayerDev)
-        tmpl[i] = L.tmap_gu[i];
-        tmpl[32 + i] = L.tmap_dn[i];
-      }
-    }
-    __syncwarp();
-    struct Prep {
-      Group g;
-      int id;
-      int4 rc;
-      const unsigned char *w0, *w1, *w2;
-      const unsigned char* maps;
-      int row;            // this lane's entry of GEntry::rows
-      bool absent, aligned;
-      unsigned ready;     // down groups: quantised blocks of the tile's h published so far
-    };
+  if (warp == kPrepWarp) {
+    // ---------------- preparing warp ----------------
+    // Draws the CTA's groups and publishes each with its record, pointers and patched descriptors: three
+    // dependent round trips and the descriptor proxies' fences per group (2.5 us together), which the
+    // weight warp, when it did them between its copies, could not hide behind a down group's two stages.
+    // A number drawn is a group that no other CTA can take, and a gate/up group that waits long for its
+    // CTA delays its tile's h, on which the down groups elsewhere depend: so a number is drawn only when
+    // the weight warp has kAhead published stages or fewer left.
+    unsigned char* gmaps = L.tmaps + static_cast<size_t>(blockIdx.x) * kMapRing * 2 * 128;
+    const unsigned char* const* ptab = reinterpret_cast<const unsigned char* const*>(plan_s + kPlanOffTab);
+    unsigned planned = 0;                        // stages of the groups published so far
+    int drawn = blockIdx.x;                      // the first group is this CTA's own number
+    bool have = true;
     int map_seq = 0;
-    auto load_ptrs = [&](Prep& p) {
-      const bool shared = p.rc.x == L.E;
-      p.w0 = shared ? L.sh[0] : L.tab[p.rc.x];
-      p.w1 = shared ? L.sh[1] : L.tab[L.tab_stride + p.rc.x];
-      p.w2 = shared ? L.sh[2] : L.tab[2 * L.tab_stride + p.rc.x];
-      p.row = 0;
-      if (p.g.kind == 0 && lane < p.rc.y)
-        p.row = shared ? p.rc.w + lane : (plan_own ? rows_p[p.rc.w + lane] : __ldcg(rows_p + p.rc.w + lane));
-      // a down group's activation rows are the tile's quantised h: seen complete here (acquire), the
-      // activation warps need not look again (they run after this warp's publication of the entry)
-      p.ready = p.g.kind == 1 ? ld_acquire(L.ready + p.g.tile) : 0u;
-    };
-    // descriptors of the matrices this group reads (gate and up, or down), in the next slot of the
-    // CTA's ring: the ring keeps the descriptors of earlier groups intact while their copies fly
-    auto patch = [&](Prep& p) {
-      p.absent = p.w0 == nullptr || p.w1 == nullptr || p.w2 == nullptr;
-      p.aligned = ((reinterpret_cast<uintptr_t>(p.w0) | reinterpret_cast<uintptr_t>(p.w1) |
-                    reinterpret_cast<uintptr_t>(p.w2)) & 15u) == 0;
-      p.maps = nullptr;
-      if (p.absent || !p.aligned) return;
-      unsigned char* slot = gmaps + static_cast<size_t>(map_seq % kMapRing) * 3 * 128;
-      ++map_seq;
-      uint32_t* m = reinterpret_cast<uint32_t*>(smaps);
-      if (p.g.kind == 0) {
-        m[lane] = tmpl[lane];
-        m[32 + lane] = tmpl[lane];
-        __syncwarp();
-        if (lane == 0) {
-          tmap_replace_addr(smaps, p.w0);
-          tmap_replace_addr(smaps + 128, p.w1);
-        }
-        __syncwarp();
-        tmap_publish(slot, smaps);
-        tmap_publish(slot + 128, smaps + 128);
-        if (lane == 0) {
-          tmap_acquire(slot);
-          tmap_acquire(slot + 128);
-        }
-      } else {
-        m[64 + lane] = tmpl[32 + lane];
-        __syncwarp();
-        if (lane == 0) tmap_replace_addr(smaps + 256, p.w2);
-        __syncwarp();
-        tmap_publish(slot + 256, smaps + 256);
-        if (lane == 0) tmap_acquire(slot + 256);
-      }
-      __syncwarp();
-      p.maps = slot;
-    };
-    auto publish = [&](int k, const Prep& p) {
-      GEntry* e = glist + k % kListSlots;
-      if (lane < kTok) e->rows[lane] = p.row;
+    for (int k = 0;; ++k) {
+      unsigned it = 0;
       if (lane == 0) {
-        e->id = p.g.valid ? p.id : -1;
-        e->absent = (p.absent ? 1 : 0) | (p.ready >= static_cast<unsigned>(L.nbf) ? 2 : 0);
-        e->rc = p.rc;
+        while (planned - *issued > static_cast<unsigned>(kAhead) && ++it < kSpinLimit) __nanosleep(20);
+        if (!have) drawn = static_cast<int>(atomicAdd(&L.cnt[10], 1u));
+      }
+      it = __shfl_sync(0xFFFFFFFFu, it, 0);
+      if (it >= kSpinLimit) {
+        if (lane == 0) atomicExch(L.status, 2);
+        return;
+      }
+      const int id = __shfl_sync(0xFFFFFFFFu, drawn, 0);
+      const Group g = sc.decode(id);
+      int4 rc = make_int4(0, 0, 0, 0);
+      const unsigned char *w0 = nullptr, *w1 = nullptr, *w2 = nullptr, *maps = nullptr;
+      int row = 0;
+      unsigned ready = 0u;
+      bool absent = false, aligned = true;
+      have = false;
+      if (g.valid) {
+        rc = tile_rec(g.tile);
+        const bool shared = rc.x == L.E;
+        // a down group's activation rows are the tile's quantised h: seen complete here (acquire), the
+        // activation warps need not look again (they run after the publication of the entry)
+        if (g.kind == 1) {
+          ready = ld_acquire(L.ready + g.tile);
+          have = ready >= static_cast<unsigned>(L.nbf);     // a short group: its successor's number at hand when it starts
+          if (have && lane == 0) drawn = static_cast<int>(atomicAdd(&L.cnt[10], 1u));
+          have = __any_sync(0xFFFFFFFFu, have && lane == 0);
+        }
+        w0 = shared ? L.sh[0] : (plan_own ? ptab[rc.x] : L.tab[rc.x]);
+        w1 = shared ? L.sh[1] : (plan_own ? ptab[L.E + rc.x] : L.tab[L.tab_stride + rc.x]);
+        w2 = shared ? L.sh[2] : (plan_own ? ptab[2 * L.E + rc.x] : L.tab[2 * L.tab_stride + rc.x]);
+        if (g.kind == 0 && lane < rc.y)
+          row = shared ? rc.w + lane : (plan_own ? plan_s[kPlanOffRows + rc.w + lane] : __ldcg(L.grows + rc.w + lane));
+        absent = w0 == nullptr || w1 == nullptr || w2 == nullptr;
+        aligned = ((reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1) | reinterpret_cast<uintptr_t>(w2)) & 15u) == 0;
+        if (!absent && aligned) {
+          // descriptors of the matrices this group reads (gate and up, or down), in the next slot of the
+          // CTA's ring: the ring keeps the descriptors of earlier groups intact while their copies fly
+          unsigned char* slot = gmaps + static_cast<size_t>(map_seq % kMapRing) * 2 * 128;
+          ++map_seq;
+          uint32_t* m = reinterpret_cast<uint32_t*>(smaps);
+          if (g.kind == 0) {
+            m[lane] = tmpl[lane];
+            m[32 + lane] = tmpl[lane];
+            __syncwarp();
+            if (lane == 0) {
+              tmap_replace_addr(smaps, w0);
+              tmap_replace_addr(smaps + 128, w1);
+            }
+            __syncwarp();
+            tmap_publish(slot, smaps);
+            tmap_publish(slot + 128, smaps + 128);
+          } else {
+            m[64 + lane] = tmpl[32 + lane];
+            __syncwarp();
+            if (lane == 0) tmap_replace_addr(smaps + 256, w2);
+            __syncwarp();
+            tmap_publish(slot, smaps + 256);
+          }
+          __syncwarp();
+          maps = slot;
+        }
+      }
+      GEntry* e = glist + k % kListSlots;
+      if (lane < kTok) e->rows[lane] = static_cast<unsigned char>(row);
+      if (lane == 0) {
+        e->id = g.valid ? id : -1;
+        e->bits = (absent ? 1 : 0) | (ready >= static_cast<unsigned>(L.nbf) ? 2 : 0) | (aligned ? 4 : 0);
+        e->maps = maps;
+        e->rc = rc;
+        e->w[0] = w0; e->w[1] = w1; e->w[2] = w2;
       }
       __syncwarp();
       if (lane == 0) {
         __threadfence_block();
         *g_pub = static_cast<unsigned>(k) + 1u;
       }
-    };
-    Prep cur;
-    cur.id = blockIdx.x;                        // the first group is this CTA's own number
-    cur.g = sc.decode(cur.id);
-    cur.rc = make_int4(0, 0, 0, 0);
-    cur.w0 = cur.w1 = cur.w2 = nullptr;
-    cur.maps = nullptr;
-    cur.row = 0;
-    cur.absent = false;
-    cur.aligned = true;
-    cur.ready = 0u;
-    int drawn = 0;                               // lane 0: the number last drawn
-    bool id_ready = false;                       // ... which is that of the next group, not yet looked at
-    if (cur.g.valid) {
-      cur.rc = tile_rec(cur.g.tile);
-      load_ptrs(cur);
-      patch(cur);
+      if (!g.valid) return;
+      planned += static_cast<unsigned>(g.nb);
+      if (g.kind == 1 && !have && !absent) {
+        // its h is not there yet: no further groups until it is. (A CTA early to the down groups would otherwise
+        // fill its ring with them and keep them to itself, while the CTAs that make the h end up with none.)
+        it = 0;
+        if (lane == 0)
+          while (ld_acquire(L.ready + g.tile) < static_cast<unsigned>(L.nbf) && ++it < kSpinLimit) __nanosleep(20);
+        it = __shfl_sync(0xFFFFFFFFu, it, 0);
+        if (it >= kSpinLimit) {
+          if (lane == 0) atomicExch(L.status, 4);
+          return;
+        }
+      }
     }
-    publish(0, cur);
+  }
+
+  if (warp == kWeightWarp) {
+    // ---------------- weight warp: the copies of the published groups, stage by stage ----------------
     int q = 0;
     for (int k = 0;; ++k) {
-      const Group wk = cur.g;
+      bool got;
+      const GEntry* ge = follow(k, got);
+      if (!got) {
+        if (lane == 0) atomicExch(L.status, 7);
+        return;
+      }
+      const Group wk = sc.decode(ge->id);
       if (!wk.valid) {                           // end of the list: one last stage that only says so
         const int s = q % kStageCount;
         const unsigned ph = (q / kStageCount) & 1;
@@ -524,96 +545,75 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         }
         return;
       }
-      Prep nx;
-      nx.id = -1;
-      nx.g = sc.decode(-1);
-      nx.rc = make_int4(0, 0, 0, 0);
-      nx.w0 = nx.w1 = nx.w2 = nullptr;
-      nx.maps = nullptr;
-      nx.row = 0;
-      nx.absent = false;
-      nx.aligned = true;
-      nx.ready = 0u;
-      const int draw_at = id_ready ? -1 : max(0, wk.nb - 4);                   // stage after which the number is drawn
-      const int look_at = id_ready ? 0 : min(wk.nb - 1, draw_at + 1);          // ... and after which it is looked at
-      const int4 rc = cur.rc;
-      const bool absent = cur.absent, aligned = cur.aligned;
-      const unsigned char* maps = cur.maps;
+      const int4 rc = ge->rc;
+      const bool absent = (ge->bits & 1) != 0, aligned = (ge->bits & 4) != 0;
+      const unsigned char* maps = ge->maps;
+      if (!absent && aligned && lane == 0) {
+        if (wk.kind == 0) {
+          tmap_acquire(maps);
+          tmap_acquire(maps + 128);
+        } else {
+          tmap_acquire(maps);
+        }
+      }
       for (int blk = 0; blk < wk.nb; ++blk, ++q) {
-      const int s = q % kStageCount;
-      const unsigned ph = (q / kStageCount) & 1;
-      if (!mbar_wait(&wempty[s], ph ^ 1u)) {
-        if (lane == 0) atomicExch(L.status, 2);
-        return;
-      }
-      unsigned char* st = stages + static_cast<size_t>(s) * kStageBytes;
-      if (lane == 0) {
-        Desc d;
-        d.flags = wk.kind | (absent ? 2 : 0) | (rc.y << 2) | (blk << 8) | (blk == wk.nb - 1 ? 1 << 16 : 0) |
-                  ((k & 4095) << 20);
-        d.tile = wk.tile; d.hrow0 = rc.z;
-        d.row0 = wk.gi * (wk.kind == 0 ? kGateUpPairs : kDownRows);
-        desc[s] = d;
-      }
-      if (!absent && aligned) {
+        const int s = q % kStageCount;
+        const unsigned ph = (q / kStageCount) & 1;
+        if (!mbar_wait(&wempty[s], ph ^ 1u)) {
+          if (lane == 0) atomicExch(L.status, 2);
+          return;
+        }
+        unsigned char* st = stages + static_cast<size_t>(s) * kStageBytes;
         if (lane == 0) {
-          mbar_expect_tx(&full[s], kWBytes);      // this lane's arrival, with the bytes to come
-          if (wk.kind == 0) {
-            tma_load_box(st, maps, blk * kW4, wk.gi * kGateUpPairs, &full[s]);
-            tma_load_box(st + kHalfBytes, maps + 128, blk * kW4, wk.gi * kGateUpPairs, &full[s]);
-          } else {
-            tma_load_box(st, maps + 256, blk * kW4, wk.gi * kDownRows, &full[s]);
-            tma_load_box(st + kHalfBytes, maps + 256, blk * kW4, wk.gi * kDownRows + kHalfRows, &full[s]);
-          }
+          Desc d;
+          d.flags = wk.kind | (absent ? 2 : 0) | (rc.y << 2) | (blk << 8) | (blk == wk.nb - 1 ? 1 << 16 : 0) |
+                    ((k & 4095) << 20);
+          d.tile = wk.tile; d.hrow0 = rc.z;
+          d.row0 = wk.gi * (wk.kind == 0 ? kGateUpPairs : kDownRows);
+          desc[s] = d;
         }
-      } else {
-        if (!absent) {                           // sources without 16-byte alignment: plain loads
-          const unsigned char *b0, *b1;
-          int rb;
-          if (wk.kind == 0) {
-            rb = rb_h;
-            b0 = cur.w0 + static_cast<size_t>(wk.gi) * kGateUpPairs * rb_h + blk * kW4;
-            b1 = cur.w1 + static_cast<size_t>(wk.gi) * kGateUpPairs * rb_h + blk * kW4;
-          } else {
-            rb = rb_f;
-            b0 = cur.w2 + static_cast<size_t>(wk.gi) * kDownRows * rb_f + blk * kW4;
-            b1 = b0 + static_cast<size_t>(kHalfRows) * rb_f;
+        if (!absent && aligned) {
+          if (lane == 0) {
+            mbar_expect_tx(&full[s], kWBytes);      // this lane's arrival, with the bytes to come
+            if (wk.kind == 0) {
+              tma_load_box(st, maps, blk * kW4, wk.gi * kGateUpPairs, &full[s]);
+              tma_load_box(st + kHalfBytes, maps + 128, blk * kW4, wk.gi * kGateUpPairs, &full[s]);
+            } else {
+              tma_load_box(st, maps, blk * kW4, wk.gi * kDownRows, &full[s]);
+              tma_load_box(st + kHalfBytes, maps, blk * kW4, wk.gi * kDownRows + kHalfRows, &full[s]);
+            }
           }
-          for (int p = lane; p < kHalfBytes / 16; p += 32) {
-            const int r = p / 9, c = (p - r * 9) * 16;
-            copy16_any(st + p * 16, b0 + static_cast<size_t>(r) * rb + c);
-            copy16_any(st + kHalfBytes + p * 16, b1 + static_cast<size_t>(r) * rb + c);
+        } else {
+          if (!absent) {                           // sources without 16-byte alignment: plain loads
+            const unsigned char *b0, *b1;
+            int rb;
+            if (wk.kind == 0) {
+              rb = rb_h;
+              b0 = ge->w[0] + static_cast<size_t>(wk.gi) * kGateUpPairs * rb_h + blk * kW4;
+              b1 = ge->w[1] + static_cast<size_t>(wk.gi) * kGateUpPairs * rb_h + blk * kW4;
+            } else {
+              rb = rb_f;
+              b0 = ge->w[2] + static_cast<size_t>(wk.gi) * kDownRows * rb_f + blk * kW4;
+              b1 = b0 + static_cast<size_t>(kHalfRows) * rb_f;
+            }
+            for (int p = lane; p < kHalfBytes / 16; p += 32) {
+              const int r = p / 9, c = (p - r * 9) * 16;
+              copy16_any(st + p * 16, b0 + static_cast<size_t>(r) * rb + c);
+              copy16_any(st + kHalfBytes + p * 16, b1 + static_cast<size_t>(r) * rb + c);
+            }
+            fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
           }
-          fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
+          __syncwarp();                            // every lane's part of the stage (and of its descriptor) is written
+          if (lane == 0) mbar_arrive(&full[s]);
         }
-        __syncwarp();                            // every lane's part of the stage (and of its descriptor) is written
-        if (lane == 0) mbar_arrive(&full[s]);
+        if (lane == 0) *issued = static_cast<unsigned>(q) + 1u;
       }
-      // the next group's number and global reads, requested between this group's copies
-      if (blk == draw_at && lane == 0) drawn = static_cast<int>(atomicAdd(&L.cnt[10], 1u));
-      if (blk == look_at) {
-        nx.id = __shfl_sync(0xFFFFFFFFu, drawn, 0);
-        nx.g = sc.decode(nx.id);
-        id_ready = false;
-        if (nx.g.valid) {
-          nx.rc = tile_rec(nx.g.tile);
-          if (nx.g.kind == 1) {                  // a short group: have the number after it at hand when it starts
-            if (lane == 0) drawn = static_cast<int>(atomicAdd(&L.cnt[10], 1u));
-            id_ready = true;
-          }
-        }
-      }
-      if (blk == wk.nb - 1 && nx.g.valid) load_ptrs(nx);
-      }   // block columns of the group
-      if (nx.g.valid) patch(nx);
-      publish(k + 1, nx);
-      cur = nx;
     }
   }
 
-  if (warp > kConsumerWarps && warp <= kConsumerWarps + kXWarps) {
+  if (warp >= kFirstXWarp && warp < kFirstXWarp + kXWarps) {
     // ---------------- activation warps ----------------
-    const int xtid = tid - kConsumers - 32;
+    const int xtid = tid - kFirstXWarp * 32;
     int myoff = 0;                              // lane t < 16: byte offset of token slot t's row
     int q = 0;
     for (int k = 0;; ++k) {
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       }
       const Group wk = sc.decode(ge->id);
       const int4 rc = ge->rc;
-      const bool absent = (ge->absent & 1) != 0;
+      const bool absent = (ge->bits & 1) != 0;
       if (!wk.valid) {                           // end of the list: count in at the last stage and leave
         const int s = q % kStageCount;
         const unsigned ph = (q / kStageCount) & 1;
@@ -641,10 +641,10 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         if (lane < rc.y) myoff = ge->rows[lane] * L.xq16_stride;
       } else {
         if (lane < rc.y) myoff = (rc.z + lane) * L.nbf * kHq;
-        if (!absent && !(ge->absent & 2)) {     // the tile's h must be quantised and published
+        if (!absent && !(ge->bits & 2)) {     // the tile's h must be quantised and published
           unsigned it = 0;
           if (lane == 0)
-            while (ld_acquire(L.ready + wk.tile) < static_cast<unsigned>(L.nbf) && ++it < kSpinLimit) __nanosleep(64);
+            while (ld_acquire(L.ready + wk.tile) < static_cast<unsigned>(L.nbf) && ++it < kSpinLimit) __nanosleep(20);
           it = __shfl_sync(0xFFFFFFFFu, it, 0);
           if (it >= kSpinLimit) {
             if (lane == 0) atomicExch(L.status, 4);
@@ -684,7 +684,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     }
   }
 
-  if (warp == kConsumerWarps + 1 + kXWarps) {
+  if (warp == kFinishWarp) {
     // ---------------- finisher warp ----------------
     // Takes the finished gate/up groups of this CTA in order: counts the CTA in at the
     // group's block of h, and if that completes the block, quantises it for the tile's
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       if (!wk.valid || wk.kind == 1) return;     // a CTA's gate/up groups all come before its down groups
       unsigned it = 0;
       if (lane == 0)
-        while (*done_tail <= static_cast<unsigned>(g) && ++it < kSpinLimit) __nanosleep(100);
+        while (*done_tail <= static_cast<unsigned>(g) && ++it < kSpinLimit) __nanosleep(32);
       it = __shfl_sync(0xFFFFFFFFu, it, 0);
       if (it >= kSpinLimit) {
         if (lane == 0) atomicExch(L.status, 6);
@@ -711,16 +711,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       __syncwarp();
       if (lane == 0) *done_head = static_cast<unsigned>(g) + 1u;     // the slot may be reused
       if (r.ntok == 0) continue;
-      __threadfence();                         // cumulative: covers what the sixteen warps stored
-      unsigned old = 0;
-      if (lane == 0) old = atomicAdd(L.blk_cnt + r.tile * L.nbf + r.hb, 1u);
+      unsigned old = 0;                        // (the release is cumulative: covers what the sixteen warps stored)
+      if (lane == 0) old = atom_add_acq_rel(L.blk_cnt + r.tile * L.nbf + r.hb, 1u);
       old = __shfl_sync(0xFFFFFFFFu, old, 0);
+      __syncwarp();
       if (old == kQK / kGateUpPairs - 1) {
-        __threadfence();
         quantize_h_block(L, r.hrow0, r.ntok, r.hb, lane);
-        __threadfence();
         __syncwarp();
-        if (lane == 0) atomicAdd(L.ready + r.tile, 1u);
+        if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.ready + r.tile) : "memory");
       }
     }
     return;

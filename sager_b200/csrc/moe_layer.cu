@@ -49,8 +49,11 @@ namespace {
 
 constexpr int kMaxRows = 64;       // token rows per call (row masks are 64-bit)
 constexpr int kTokTile = 8;        // token rows per tile of the item kernel (one MMA n-tile)
-constexpr int kMaxGrid = 192;            // most CTAs the expert kernels are launched with
-constexpr int kTmapSlots = 6;            // patched TMA descriptor sets per CTA of the row-streaming kernel
+constexpr int kMaxGrid = 160;            // most CTAs the expert kernels are launched with
+#ifndef AH
+#define AH 3
+#endif
+constexpr int kTmapSlots = AH + 7;           // patched TMA descriptor pairs per CTA of the row-streaming kernel
 constexpr int kTokenKernelMaxRows = 4;   // layers of up to this many token rows run as one persistent launch: all that its
                                          // row sets hold (us per layer at 1 / 2 / 3 / 4 rows, 256 experts, hidden 2048,
                                          // n_ff 512: 18.4 / 27.1 / 36.2 / 46.2, route + expert kernel 47.3 at 4; 128
@@ -129,7 +132,7 @@ struct LayerDev {
   const unsigned char* ep_src;
   const unsigned* ep_step;
   int ep_world, ep_rec, ep_home, ep_mul, ep_add;
-  unsigned char* tmaps;   // [grid][kTmapSlots][3][128] row-streaming kernel: patched TMA descriptors
+  unsigned char* tmaps;   // [grid][kTmapSlots][2][128] row-streaming kernel: patched TMA descriptors
   // TMA descriptors (placeholder address) of a gate / up matrix and of a down matrix. Only ever
   // read with constant indices: a dynamic index would make every thread keep a local-memory
   // copy of the whole argument block.
@@ -170,7 +173,7 @@ inline WsLayout ws_layout(int n_max, int H, int FF, int E, int K) {
   l.items_total = p;
   l.hq = take(rows * (FF / kQK) * 288);     // padded Q8_K blocks (rs::kHq)
   l.xq16 = take(static_cast<size_t>(n_max) * (H / kQK) * 288);
-  l.tmaps = take(static_cast<size_t>(kMaxGrid) * kTmapSlots * 3 * 128);
+  l.tmaps = take(static_cast<size_t>(kMaxGrid) * kTmapSlots * 2 * 128);
   l.total = p;
   return l;
 }
