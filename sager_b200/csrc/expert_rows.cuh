@@ -46,8 +46,9 @@ constexpr int kConsumers = kConsumerWarps * 32;
 constexpr int kXWarps = 2;                      // activation-row producers
 constexpr int kXThreads = kXWarps * 32;
 constexpr int kPrepWarp = kConsumerWarps, kWeightWarp = kPrepWarp + 1, kFirstXWarp = kWeightWarp + 1, kFinishWarp = kFirstXWarp + kXWarps;
-constexpr int kThreads = (kFinishWarp + 1) * 32;
-constexpr int kStageCount = 5;
+constexpr int kFinishWarps = 2;
+constexpr int kThreads = (kFinishWarp + kFinishWarps) * 32;
+constexpr int kStageCount = 3;
 constexpr int kHalfRows = 128;                  // a stage is two halves of 128 rows
 constexpr int kHalfBytes = kHalfRows * kW4;     // 18432
 constexpr int kWBytes = 2 * kHalfBytes;
@@ -56,7 +57,7 @@ constexpr int kXCodes = kTok * kXqStride;
 constexpr int kXBytes = kXCodes + kTok * 16 + kTok * 16;
 constexpr int kStageBytes = (kWBytes + kXBytes + 127) & ~127;
 constexpr int kHq = 288;                        // padded Q8_K block of h: d | 12 bytes | 256 codes | 8 sums
-constexpr int kHdr = 4608;
+constexpr int kHdr = 4096;
 // The plan of a layer, built by every CTA for itself when the routing was made by this call's own
 // route kernel: row masks [E] | offsets [E + 1] | scan scratch | tile records | rows of the slots | slot
 // of every route. One round trip for the routing and a few barriers per CTA, all CTAs at once, instead
@@ -68,8 +69,12 @@ constexpr int kPlanOffRec = kPlanOffScan + 512, kPlanOffRows = kPlanOffRec + kPl
 constexpr int kPlanOffSlot = kPlanOffRows + kPlanRoutes;               // (a source row is below 64: one byte)
 constexpr int kPlanOffTab = kPlanOffSlot + kPlanRoutes * 4;             // the layer's pointer table [3][E]
 constexpr int kPlanBytes = (kPlanOffTab + 3 * kPlanExperts * 8 + 127) & ~127;
-constexpr size_t kSmem = kHdr + kPlanBytes + static_cast<size_t>(kStageCount) * kStageBytes;
-constexpr int kGateUpPairs = 128;               // pairs per gate/up group
+// h of a gate/up group, [16][256] fp32, two groups in turn (the padded row keeps the consumers' stores off one bank)
+constexpr int kHRow = 260;
+constexpr int kHBytes = kTok * kHRow * 4;
+constexpr size_t kSmem = kHdr + kPlanBytes + static_cast<size_t>(kStageCount) * kStageBytes + 2 * kHBytes;
+constexpr int kGateUpPairs = 256;               // pairs per gate/up group: one block of h, streamed as two halves of 128 pairs,
+                                                // or one of the halves where groups are few (Sched::split)
 constexpr int kDownRows = 256;                  // rows per down group
 constexpr int kFullArrivals = 1 + kXThreads;      // weight warp: one arrival; activation warps: a thread's copies landed
 constexpr int kAhead = AH;                        // stages of published groups that the weight warp is kept ahead with
@@ -81,8 +86,8 @@ static_assert(kMapRing <= kTmapSlots, "the workspace holds kTmapSlots descriptor
 
 struct Desc {     // one 16-byte shared-memory load per stage and warp
   int flags;     // bit 0 kind (0 gate/up, 1 down), bit 1 expert absent, bits 2-7 token rows,
-                 // bits 8-15 block column, bit 16 last column of the group, bit 17 end of this CTA's list,
-                 // bits 20-31 group number in this CTA
+                 // bits 8-15 block column, bit 16 last column, bit 17 end of this CTA's list,
+                 // bit 18 second half of a gate/up group, bits 20-31 group number in this CTA
   int tile;
   int hrow0;     // first h / y row of the tile
   int row0;      // first pair (gate/up) or first row (down) of the group
@@ -92,14 +97,9 @@ struct Desc {     // one 16-byte shared-memory load per stage and warp
   __device__ __forceinline__ int blk() const { return (flags >> 8) & 255; }
   __device__ __forceinline__ int last() const { return (flags >> 16) & 1; }
   __device__ __forceinline__ int end() const { return (flags >> 17) & 1; }     // no more stages for this CTA
+  __device__ __forceinline__ int half() const { return (flags >> 18) & 1; }
   __device__ __forceinline__ int seq() const { return (flags >> 20) & 4095; }
 };
-
-// A finished gate/up group, handed from the consumers to the finisher warp.
-struct Done {
-  int tile, hb, hrow0, ntok;     // ntok == 0: absent expert, nothing to count
-};
-constexpr int kDoneSlots = 8;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -151,11 +151,12 @@ __device__ __forceinline__ void copy16_any(unsigned char* dst, const unsigned ch
 // roles. Equal finishing times need no cost model this way, and a tile's down groups are
 // drawn long after its gate/up groups were (the whole gate/up list lies between).
 struct Group {
-  int kind, tile, gi, nb;        // 0 gate/up / 1 down, tile, group inside the tile, block columns
+  int kind, tile, gi, nb;        // 0 gate/up / 1 down, tile, group inside the tile, stages
   bool valid;
 };
 struct Sched {
   int n_gu, total, nbh, nbf, gpt_gu, gpt_dn;
+  int split;                     // 1: a gate/up group is half a block of h (bit 0 of gi tells which)
   __device__ __forceinline__ Group decode(int g) const {
     Group r;
     r.valid = g >= 0 && g < total;
@@ -164,41 +165,41 @@ struct Sched {
     const int gpt = r.kind ? gpt_dn : gpt_gu;
     r.tile = r.valid ? local / gpt : 0;
     r.gi = local - r.tile * gpt;
-    r.nb = r.kind ? nbf : nbh;
+    r.nb = r.kind ? nbf : (2 - split) * nbh;
     return r;
   }
 };
-constexpr int kListSlots = 32;
+constexpr int kListSlots = 16;
 
 // One entry of a CTA's group list, published by the preparing warp some stages ahead of the copies,
 // with everything the other roles would otherwise fetch from global memory again. A reader lags by at
-// most kAhead + kStageCount + 1 groups and the done queue's.
+// most kAhead + kStageCount + 1 groups and the two whose h waits for the finisher warp.
 struct alignas(16) GEntry {
   int id;          // global group number, -1 = end of this CTA's list
-  int bits;        // bit 0: the expert's pointers are null; bit 1 (down groups): the tile's h was already published
-                   // when the preparing warp looked; bit 2: the pointers are 16-byte aligned
+  int bits;        // bit 0: the expert's pointers are null; bit 1: they are 16-byte aligned
   const unsigned char* maps;    // the group's descriptors
   int4 rc;         // the tile's record: expert, token rows, first h / y row, first entry of grows
   const unsigned char* w[3];    // the expert's matrices
   unsigned char rows[kTok];     // gate/up groups: source row of the tile's token slot t in the quantised inputs
+  volatile int there;           // down groups: the tile's h has been seen complete
 };
-static_assert(kListSlots >= kAhead + kStageCount + 1 + kDoneSlots + 1, "a reader could be overtaken");
+static_assert(kListSlots > kAhead + kStageCount + 1 + 2, "a reader could be overtaken");
 static_assert(sizeof(GEntry) * kListSlots + 2048 <= kHdr, "group list exceeds the header");
 
-// One warp: Q8_K-quantise block `hb` of the fp32 h rows [hrow0, hrow0 + ntok) into the
-// padded rows of L.hq (arithmetic of src/kernels/cpu/q4_avx2.cpp:77-94 in the reference,
+// One warp: Q8_K-quantise block `hb` of h, rows `src` in shared memory, into the padded rows
+// [hrow0, hrow0 + ntok) of L.hq (arithmetic of src/kernels/cpu/q4_avx2.cpp:77-94 in the reference,
 // the same as stage_quantized_f32). The down groups of the tile wait for it, and beside sixteen
 // consumer warps a chain of instructions takes ten cycles each: R rows go through it side by side
 // (one after the other, a row took 0.85 us).
 template <int R>
-__device__ __forceinline__ void quantize_h_rows(const LayerDev& L, int hrow0, int ntok, int hb, int lane) {
+__device__ __forceinline__ void quantize_h_rows(const LayerDev& L, const float* src, int hrow0, int ntok, int hb, int lane) {
   const size_t hq_stride = static_cast<size_t>(L.nbf) * kHq;
   float4 a[R], b[R];
 #pragma unroll
   for (int u = 0; u < R; ++u) {
-    const float4* p = reinterpret_cast<const float4*>(L.hbuf + static_cast<size_t>(hrow0 + min(u, ntok - 1)) * L.FF + hb * kQK) + lane * 2;
-    a[u] = __ldcg(p);
-    b[u] = __ldcg(p + 1);
+    const float4* p = reinterpret_cast<const float4*>(src + min(u, ntok - 1) * kHRow) + lane * 2;
+    a[u] = p[0];
+    b[u] = p[1];
   }
   uint32_t lo[R], hi[R], sums[R];
   float d[R];
@@ -220,11 +221,13 @@ __device__ __forceinline__ void quantize_h_rows(const LayerDev& L, int hrow0, in
     if ((lane & 7) == 0) o32[68 + (lane >> 3)] = sums[u];
   }
 }
-__device__ __forceinline__ void quantize_h_block(const LayerDev& L, int hrow0, int ntok, int hb, int lane) {
-  int t0 = 0;
+// (batches of four rows in turn between the finisher warps, `f` is this one's number)
+__device__ __forceinline__ void quantize_h_block(const LayerDev& L, const float* src, int hrow0, int ntok, int hb, int f, int lane) {
 #pragma unroll 1
-  for (; ntok - t0 > 2; t0 += 4) quantize_h_rows<4>(L, hrow0 + t0, ntok - t0, hb, lane);
-  if (ntok - t0 > 0) quantize_h_rows<2>(L, hrow0 + t0, ntok - t0, hb, lane);
+  for (int t0 = 4 * f; t0 < ntok; t0 += 4 * kFinishWarps) {
+    if (ntok - t0 > 2) quantize_h_rows<4>(L, src + t0 * kHRow, hrow0 + t0, ntok - t0, hb, lane);
+    else quantize_h_rows<2>(L, src + t0 * kHRow, hrow0 + t0, ntok - t0, hb, lane);
+  }
 }
 
 // Every thread of the CTA: the plan of build_plan (moe_layer.cu) in shared memory - same masks, same
@@ -330,13 +333,12 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   uint64_t* empty = reinterpret_cast<uint64_t*>(smem + 64);      // a stage's activation part may be refilled
   uint64_t* wempty = reinterpret_cast<uint64_t*>(smem + 192);    // a stage's weight part may be refilled
   int* flag = reinterpret_cast<int*>(smem + 128);
-  unsigned* grp_cnt = reinterpret_cast<unsigned*>(smem + 256);      // [8] consumer warps done with a group
+  uint64_t* hfull = reinterpret_cast<uint64_t*>(smem + 160);     // [2] h of a gate/up group is in shared memory
+  uint64_t* hempty = reinterpret_cast<uint64_t*>(smem + 176);    // [2] ... and has been quantised
   Desc* desc = reinterpret_cast<Desc*>(smem + 384);
-  Done* done_q = reinterpret_cast<Done*>(smem + 640);               // [kDoneSlots]
-  volatile unsigned* done_tail = reinterpret_cast<volatile unsigned*>(smem + 136);   // groups handed over
-  volatile unsigned* done_head = reinterpret_cast<volatile unsigned*>(smem + 140);   // groups taken by the finisher
   unsigned char* plan_s = smem + kHdr;
   unsigned char* stages = smem + kHdr + kPlanBytes;
+  float* hs = reinterpret_cast<float*>(stages + static_cast<size_t>(kStageCount) * kStageBytes);   // [2][16][kHRow]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
@@ -345,9 +347,10 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       mbar_init(&empty[s], kConsumerWarps);
       mbar_init(&wempty[s], kConsumerWarps);
     }
-    for (int i = 0; i < 8; ++i) grp_cnt[i] = 0u;
-    *done_tail = 0u;
-    *done_head = 0u;
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&hfull[s], kConsumerWarps);
+      mbar_init(&hempty[s], kFinishWarps);
+    }
     *reinterpret_cast<volatile unsigned*>(smem + 144) = 0u;
     *reinterpret_cast<volatile unsigned*>(smem + 148) = 0u;
     fence_barrier_init();
@@ -370,7 +373,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   pdl_launch_dependents();
 
   Sched sc;
-  sc.gpt_gu = L.FF / kGateUpPairs; sc.gpt_dn = L.H / kDownRows;      // groups per tile
+  sc.gpt_dn = L.H / kDownRows;      // groups per tile
   sc.nbh = L.nbh; sc.nbf = L.nbf;
   // the plan: this CTA's own copy in shared memory, or the one a plan kernel left in the workspace
   const bool plan_own = L.plan_in_kernel != 0;
@@ -392,6 +395,11 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   const int4* rec_p = plan_own ? reinterpret_cast<const int4*>(plan_s + kPlanOffRec) : L.rec;
   const int* slot_p = plan_own ? reinterpret_cast<const int*>(plan_s + kPlanOffSlot) : L.gslot;
   auto tile_rec = [&](int tile) { return plan_own ? rec_p[tile] : __ldcg(rec_p + tile); };
+  // Groups of whole blocks quantise their h in the CTA; with fewer of them than two thirds of the CTAs, halves of a block
+  // and an exchange through global memory are faster (us per layer: hidden 2048, n_ff 512, 5 rows, 82 blocks: 44.6
+  // against 47.2, 8 rows, 118 blocks: 52.4 against 51.4).
+  sc.split = 3 * n_tiles * L.nbf < 2 * static_cast<int>(gridDim.x) ? 1 : 0;
+  sc.gpt_gu = L.nbf << sc.split;
   sc.n_gu = n_tiles * sc.gpt_gu;
   sc.total = sc.n_gu + n_tiles * sc.gpt_dn;
   const int rb_h = L.nbh * kW4, rb_f = L.nbf * kW4;
@@ -445,11 +453,10 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       if (g.valid) {
         rc = tile_rec(g.tile);
         const bool shared = rc.x == L.E;
-        // a down group's activation rows are the tile's quantised h: seen complete here (acquire), the
-        // activation warps need not look again (they run after the publication of the entry)
+        // a down group's activation rows are the tile's quantised h: seen complete here (acquire)
         if (g.kind == 1) {
           ready = ld_acquire(L.ready + g.tile);
-          have = ready >= static_cast<unsigned>(L.nbf);     // a short group: its successor's number at hand when it starts
+          have = ready >= static_cast<unsigned>(kFinishWarps * L.nbf);     // a short group: its successor's number at hand when it starts
           if (have && lane == 0) drawn = static_cast<int>(atomicAdd(&L.cnt[10], 1u));
           have = __any_sync(0xFFFFFFFFu, have && lane == 0);
         }
@@ -492,7 +499,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       if (lane < kTok) e->rows[lane] = static_cast<unsigned char>(row);
       if (lane == 0) {
         e->id = g.valid ? id : -1;
-        e->bits = (absent ? 1 : 0) | (ready >= static_cast<unsigned>(L.nbf) ? 2 : 0) | (aligned ? 4 : 0);
+        e->bits = (absent ? 1 : 0) | (aligned ? 2 : 0);
+        e->there = have ? 1 : 0;
         e->maps = maps;
         e->rc = rc;
         e->w[0] = w0; e->w[1] = w1; e->w[2] = w2;
@@ -508,8 +516,12 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         // its h is not there yet: no further groups until it is. (A CTA early to the down groups would otherwise
         // fill its ring with them and keep them to itself, while the CTAs that make the h end up with none.)
         it = 0;
-        if (lane == 0)
-          while (ld_acquire(L.ready + g.tile) < static_cast<unsigned>(L.nbf) && ++it < kSpinLimit) __nanosleep(20);
+        // (one poller per CTA, which tells the activation warps: more of them slowed the counters they wait for)
+        if (lane == 0) {
+          while (ld_acquire(L.ready + g.tile) < static_cast<unsigned>(kFinishWarps * L.nbf) && ++it < kSpinLimit) __nanosleep(50);
+          __threadfence_block();
+          if (it < kSpinLimit) e->there = 1;
+        }
         it = __shfl_sync(0xFFFFFFFFu, it, 0);
         if (it >= kSpinLimit) {
           if (lane == 0) atomicExch(L.status, 4);
@@ -546,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         return;
       }
       const int4 rc = ge->rc;
-      const bool absent = (ge->bits & 1) != 0, aligned = (ge->bits & 4) != 0;
+      const bool absent = (ge->bits & 1) != 0, aligned = (ge->bits & 2) != 0;
       const unsigned char* maps = ge->maps;
       if (!absent && aligned && lane == 0) {
         if (wk.kind == 0) {
@@ -556,7 +568,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           tmap_acquire(maps);
         }
       }
-      for (int blk = 0; blk < wk.nb; ++blk, ++q) {
+      const int cols = wk.kind == 0 ? L.nbh : L.nbf;
+      for (int i = 0; i < wk.nb; ++i, ++q) {
+        int half = 0, row0 = wk.gi * kDownRows, blk = i;
+        if (wk.kind == 0) {
+          half = sc.split ? wk.gi & 1 : (i >= cols ? 1 : 0);
+          row0 = (wk.gi >> sc.split) * kGateUpPairs + half * kHalfRows;
+          if (i >= cols) blk -= cols;
+        }
         const int s = q % kStageCount;
         const unsigned ph = (q / kStageCount) & 1;
         if (!mbar_wait(&wempty[s], ph ^ 1u)) {
@@ -566,21 +585,20 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         unsigned char* st = stages + static_cast<size_t>(s) * kStageBytes;
         if (lane == 0) {
           Desc d;
-          d.flags = wk.kind | (absent ? 2 : 0) | (rc.y << 2) | (blk << 8) | (blk == wk.nb - 1 ? 1 << 16 : 0) |
-                    ((k & 4095) << 20);
-          d.tile = wk.tile; d.hrow0 = rc.z;
-          d.row0 = wk.gi * (wk.kind == 0 ? kGateUpPairs : kDownRows);
+          d.flags = wk.kind | (absent ? 2 : 0) | (rc.y << 2) | (blk << 8) | (blk == cols - 1 ? 1 << 16 : 0) |
+                    (half << 18) | ((k & 4095) << 20);
+          d.tile = wk.tile; d.hrow0 = rc.z; d.row0 = row0;
           desc[s] = d;
         }
         if (!absent && aligned) {
           if (lane == 0) {
             mbar_expect_tx(&full[s], kWBytes);      // this lane's arrival, with the bytes to come
             if (wk.kind == 0) {
-              tma_load_box(st, maps, blk * kW4, wk.gi * kGateUpPairs, &full[s]);
-              tma_load_box(st + kHalfBytes, maps + 128, blk * kW4, wk.gi * kGateUpPairs, &full[s]);
+              tma_load_box(st, maps, blk * kW4, row0, &full[s]);
+              tma_load_box(st + kHalfBytes, maps + 128, blk * kW4, row0, &full[s]);
             } else {
-              tma_load_box(st, maps, blk * kW4, wk.gi * kDownRows, &full[s]);
-              tma_load_box(st + kHalfBytes, maps, blk * kW4, wk.gi * kDownRows + kHalfRows, &full[s]);
+              tma_load_box(st, maps, blk * kW4, row0, &full[s]);
+              tma_load_box(st + kHalfBytes, maps, blk * kW4, row0 + kHalfRows, &full[s]);
             }
           }
         } else {
@@ -589,11 +607,11 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
             int rb;
             if (wk.kind == 0) {
               rb = rb_h;
-              b0 = ge->w[0] + static_cast<size_t>(wk.gi) * kGateUpPairs * rb_h + blk * kW4;
-              b1 = ge->w[1] + static_cast<size_t>(wk.gi) * kGateUpPairs * rb_h + blk * kW4;
+              b0 = ge->w[0] + static_cast<size_t>(row0) * rb_h + blk * kW4;
+              b1 = ge->w[1] + static_cast<size_t>(row0) * rb_h + blk * kW4;
             } else {
               rb = rb_f;
-              b0 = ge->w[2] + static_cast<size_t>(wk.gi) * kDownRows * rb_f + blk * kW4;
+              b0 = ge->w[2] + static_cast<size_t>(row0) * rb_f + blk * kW4;
               b1 = b0 + static_cast<size_t>(kHalfRows) * rb_f;
             }
             for (int p = lane; p < kHalfBytes / 16; p += 32) {
@@ -641,18 +659,20 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         if (lane < rc.y) myoff = ge->rows[lane] * L.xq16_stride;
       } else {
         if (lane < rc.y) myoff = (rc.z + lane) * L.nbf * kHq;
-        if (!absent && !(ge->bits & 2)) {     // the tile's h must be quantised and published
+        if (!absent) {                        // the tile's h must be quantised and published
           unsigned it = 0;
           if (lane == 0)
-            while (ld_acquire(L.ready + wk.tile) < static_cast<unsigned>(L.nbf) && ++it < kSpinLimit) __nanosleep(20);
+            while (ge->there == 0 && ++it < kSpinLimit) __nanosleep(20);
           it = __shfl_sync(0xFFFFFFFFu, it, 0);
+          __threadfence_block();
           if (it >= kSpinLimit) {
             if (lane == 0) atomicExch(L.status, 4);
             return;
           }
         }
       }
-      for (int blk = 0; blk < wk.nb; ++blk, ++q) {
+      for (int i = 0; i < wk.nb; ++i, ++q) {
+      const int blk = wk.kind == 0 && i >= L.nbh ? i - L.nbh : i;
       const int s = q % kStageCount;
       const unsigned ph = (q / kStageCount) & 1;
       if (!mbar_wait(&empty[s], ph ^ 1u)) {
@@ -665,10 +685,10 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         const unsigned char* xsrc = (wk.kind == 0 ? L.xq16 : L.hq) + blk * kHq;
         const int total = rc.y * (kHq / 16);
         for (int base = 0; base < total; base += kXThreads) {      // warp-uniform trip count
-          const int i = base + xtid;
-          const bool valid = i < total;
-          const int t = valid ? i / (kHq / 16) : 0;
-          const int c = i - t * (kHq / 16);
+          const int p = base + xtid;
+          const bool valid = p < total;
+          const int t = valid ? p / (kHq / 16) : 0;
+          const int c = p - t * (kHq / 16);
           const int off = __shfl_sync(0xFFFFFFFFu, myoff, t);
           if (valid) {
             // scale | codes (second half of the block 16 bytes further on: see XTile::mid_pad) | sums
@@ -684,11 +704,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     }
   }
 
-  if (warp == kFinishWarp) {
-    // ---------------- finisher warp ----------------
-    // Takes the finished gate/up groups of this CTA in order: counts the CTA in at the
-    // group's block of h, and if that completes the block, quantises it for the tile's
-    // rows and publishes it. The consumers never wait for any of this.
+  if (warp >= kFinishWarp) {
+    // ---------------- finisher warps ----------------
+    // Take the finished gate/up groups of this CTA in order: quantise the group's block of h for the
+    // tile's rows from shared memory and publish it, each its own rows. A group of half a block leaves its
+    // half in global memory first; the CTA that comes second takes the other half from there and
+    // quantises. The consumers never wait for any of this, except for a buffer to be free again two
+    // groups later.
+    const int f = warp - kFinishWarp;
     for (int g = 0;; ++g) {
       bool got;
       const GEntry* ge = follow(g, got);
@@ -698,27 +721,47 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       }
       const Group wk = sc.decode(ge->id);
       if (!wk.valid || wk.kind == 1) return;     // a CTA's gate/up groups all come before its down groups
-      unsigned it = 0;
-      if (lane == 0)
-        while (*done_tail <= static_cast<unsigned>(g) && ++it < kSpinLimit) __nanosleep(32);
-      it = __shfl_sync(0xFFFFFFFFu, it, 0);
-      if (it >= kSpinLimit) {
+      const int4 rc = ge->rc;
+      const bool absent = (ge->bits & 1) != 0;
+      const int buf = g & 1;
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&hfull[buf], (g >> 1) & 1))) {
         if (lane == 0) atomicExch(L.status, 6);
         return;
       }
-      __threadfence_block();
-      const Done r = done_q[g % kDoneSlots];
-      __syncwarp();
-      if (lane == 0) *done_head = static_cast<unsigned>(g) + 1u;     // the slot may be reused
-      if (r.ntok == 0) continue;
-      unsigned old = 0;                        // (the release is cumulative: covers what the sixteen warps stored)
-      if (lane == 0) old = atom_add_acq_rel(L.blk_cnt + r.tile * L.nbf + r.hb, 1u);
-      old = __shfl_sync(0xFFFFFFFFu, old, 0);
-      __syncwarp();
-      if (old == kQK / kGateUpPairs - 1) {
-        quantize_h_block(L, r.hrow0, r.ntok, r.hb, lane);
+      float* hb = hs + buf * kTok * kHRow;
+      const int blk = wk.gi >> sc.split;
+      bool mine = !absent;
+      if (sc.split && !absent) {
+        const int half = wk.gi & 1;
+        float* own = L.hbuf + static_cast<size_t>(rc.z) * L.FF + blk * kQK + half * kHalfRows + lane * 4;
+        for (int t = 4 * f; t < rc.y; t = (t & 3) == 3 ? t + 1 + 4 * (kFinishWarps - 1) : t + 1)
+          *reinterpret_cast<float4*>(own + static_cast<size_t>(t) * L.FF) = *reinterpret_cast<const float4*>(hb + t * kHRow + half * kHalfRows + lane * 4);
         __syncwarp();
-        if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.ready + r.tile) : "memory");
+        unsigned old = 0;
+        if (lane == 0)
+          asm volatile("atom.acq_rel.gpu.global.or.b32 %0, [%1], %2;" : "=r"(old) : "l"(L.tile_cnt + 2 * wk.tile + f), "r"(1u << blk) : "memory");
+        mine = (__shfl_sync(0xFFFFFFFFu, old, 0) >> blk & 1u) != 0;
+        __syncwarp();
+        if (mine) {
+          const float* other = L.hbuf + static_cast<size_t>(rc.z) * L.FF + blk * kQK + (half ^ 1) * kHalfRows + lane * 4;
+          for (int t0 = 4 * f; t0 < rc.y; t0 += 4 * kFinishWarps) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              v[u] = __ldcg(reinterpret_cast<const float4*>(other + static_cast<size_t>(min(t0 + u, rc.y - 1)) * L.FF));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (t0 + u < rc.y) *reinterpret_cast<float4*>(hb + (t0 + u) * kHRow + (half ^ 1) * kHalfRows + lane * 4) = v[u];
+          }
+          __syncwarp();
+        }
+      }
+      if (mine) quantize_h_block(L, hb, rc.z, rc.y, blk, f, lane);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&hempty[buf]);
+        // (the release is cumulative: it covers the other lanes' stores, ordered before it by the warp barrier)
+        if (mine) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.ready + wk.tile) : "memory");
       }
     }
     return;
@@ -793,58 +836,46 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     // ---- the group is complete for this warp's rows ----
     const int gid = lane >> 2, tig = lane & 3;
     if (d_kind == 0) {
+      if ((sc.split || d.half() == 0) && !mbar_wait(&hempty[d_seq & 1], ((d_seq >> 1) & 1) ^ 1u)) {
+        if (lane == 0) atomicExch(L.status, 6);
+        ok = false;
+        break;
+      }
       if (d_mode == 1) {
-        if (d.row0 == 0 && warp == 0 && lane == 0 && L.mail != nullptr) {
+        if (d.row0 == 0 && d.half() == 0 && warp == 0 && lane == 0 && L.mail != nullptr) {
           const int e = tile_rec(d.tile).x;
           if (e != L.E) {
             const int mi = atomicAdd(L.mail_n, 1);
             if (mi < L.E) L.mail[mi] = e;
           }
         }
-      } else
-      if (d_ntok <= 2) {
-        const float u0 = __shfl_down_sync(0xFFFFFFFFu, acc[0][0], 16);
-        const float u1 = __shfl_down_sync(0xFFFFFFFFu, acc[0][1], 16);
-        if (lane < 16 && (lane & 1) == 0) {
-          const int col = d.row0 + 8 * warp + (lane >> 1);
-          const float g0 = acc[0][0], g1 = acc[0][1];
-          L.hbuf[static_cast<size_t>(d.hrow0) * L.FF + col] = g0 / (1.f + expf(-g0)) * u0;
-          if (d_ntok > 1) L.hbuf[static_cast<size_t>(d.hrow0 + 1) * L.FF + col] = g1 / (1.f + expf(-g1)) * u1;
-        }
       } else {
-        const int col = d.row0 + 8 * warp + gid;
+        float* hb = hs + (d_seq & 1) * kTok * kHRow + d.half() * kHalfRows + 8 * warp;
+        if (d_ntok <= 2) {
+          const float u0 = __shfl_down_sync(0xFFFFFFFFu, acc[0][0], 16);
+          const float u1 = __shfl_down_sync(0xFFFFFFFFu, acc[0][1], 16);
+          if (lane < 16 && (lane & 1) == 0) {
+            const float g0 = acc[0][0], g1 = acc[0][1];
+            hb[lane >> 1] = g0 / (1.f + expf(-g0)) * u0;
+            if (d_ntok > 1) hb[kHRow + (lane >> 1)] = g1 / (1.f + expf(-g1)) * u1;
+          }
+        } else {
 #pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          const int t0 = 8 * n + 2 * tig;
-          if (t0 < d_ntok) {
-            const float g = acc[n][0], u = acc[n][2];
-            L.hbuf[static_cast<size_t>(d.hrow0 + t0) * L.FF + col] = g / (1.f + expf(-g)) * u;
-          }
-          if (t0 + 1 < d_ntok) {
-            const float g = acc[n][1], u = acc[n][3];
-            L.hbuf[static_cast<size_t>(d.hrow0 + t0 + 1) * L.FF + col] = g / (1.f + expf(-g)) * u;
+          for (int n = 0; n < 2; ++n) {
+            const int t0 = 8 * n + 2 * tig;
+            if (t0 < d_ntok) {
+              const float g = acc[n][0], u = acc[n][2];
+              hb[t0 * kHRow + gid] = g / (1.f + expf(-g)) * u;
+            }
+            if (t0 + 1 < d_ntok) {
+              const float g = acc[n][1], u = acc[n][3];
+              hb[(t0 + 1) * kHRow + gid] = g / (1.f + expf(-g)) * u;
+            }
           }
         }
       }
-      // Count the warp in at the CTA's counter of this group (shared memory); the last
-      // warp hands the group to the finisher warp. Groups finish in order: a warp is at
-      // most a ring's depth of stages ahead of the slowest one.
-      __threadfence_block();
       __syncwarp();
-      if (lane == 0) {
-        if (atomicAdd(&grp_cnt[d_seq & 7], 1u) == kConsumerWarps - 1) {
-          grp_cnt[d_seq & 7] = 0u;
-          unsigned it = 0;                       // queue full: wait (bounded) for the finisher
-          while (static_cast<unsigned>(d_seq) - *done_head >= static_cast<unsigned>(kDoneSlots) && ++it < kSpinLimit)
-            __nanosleep(100);
-          if (it >= kSpinLimit) atomicExch(L.status, 6);
-          Done r;
-          r.tile = d.tile; r.hb = d.row0 / kQK; r.hrow0 = d.hrow0; r.ntok = d_mode == 1 ? 0 : d_ntok;
-          done_q[d_seq % kDoneSlots] = r;
-          __threadfence_block();
-          *done_tail = static_cast<unsigned>(d_seq) + 1u;
-        }
-      }
+      if ((sc.split || d.half() == 1) && lane == 0) mbar_arrive(&hfull[d_seq & 1]);
     } else {
       if (d_mode == 1) {
         for (int j = lane; j < 16 * d_ntok; j += 32)

@@ -79,7 +79,7 @@ struct LayerDev {
   int add_residual, routing_given, skip_plan;
   int plan_in_kernel;  // the row-streaming kernel builds the plan itself, in shared memory, from the routing
   // a second workspace whose counters this call's route stage re-arms (expert parallelism: the owner call that follows)
-  unsigned *rearm_cnt, *rearm_tile_cnt, *rearm_blk_cnt, *rearm_ready;
+  unsigned *rearm_cnt, *rearm_tile_cnt, *rearm_ready;
   int* rearm_mail_n;
   int rearm_tiles;
   int rstride;     // elements between consecutive rows of idx / w (K+1 when packed)
@@ -107,9 +107,9 @@ struct LayerDev {
   int* gslot;      // [n*K] grouped slot of a route, -1 = not computed here
   int* grows;      // [n*K] source row of a grouped slot
   unsigned* cnt;   // [0..7] route tiles, [8] route tiles done, [9] expert kernel grid barrier, [10] next group
-  unsigned* tile_cnt;  // [max_tiles] finished gate/up items per tile
-  unsigned* blk_cnt;   // [max_tiles][nbf] row-streaming kernel: warps done with a 256-wide block of h
-  unsigned* ready;     // [max_tiles] row-streaming kernel: quantised blocks of h published
+  unsigned* tile_cnt;  // [2][max_tiles] item kernel: finished gate/up items per tile; row-streaming kernel: [tile][finisher
+                       // warp] a bit per block of h whose first half is in global memory
+  unsigned* ready;     // [max_tiles] row-streaming kernel: finisher warps done with a quantised block of h
   unsigned char* hq;   // [(n_max*K + n_max)][nbf] Q8_K rows of h, 288-byte blocks (row-streaming kernel)
   int tok_tile;        // token rows per tile: 8 (item kernel) or 16 (row-streaming kernel)
   unsigned char* xq16; // the quantised rows once more in 288-byte blocks (row-streaming kernel)
@@ -148,7 +148,7 @@ struct LayerDev {
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct WsLayout {
-  size_t xq, logits, off, rec, meta, gslot, grows, cnt, tile_cnt, blk_cnt, ready, hbuf, ybuf, hq, xq16, tmaps, total;
+  size_t xq, logits, off, rec, meta, gslot, grows, cnt, tile_cnt, ready, hbuf, ybuf, hq, xq16, tmaps, total;
   size_t items_total;   // what the item kernel needs: everything up to and including ybuf
 };
 inline WsLayout ws_layout(int n_max, int H, int FF, int E, int K) {
@@ -165,8 +165,7 @@ inline WsLayout ws_layout(int n_max, int H, int FF, int E, int K) {
   l.gslot = take(static_cast<size_t>(n_max) * K * 4);
   l.grows = take(static_cast<size_t>(n_max) * K * 4);
   l.cnt = take((16 + static_cast<size_t>(H) / 16 + 1) * 4);
-  l.tile_cnt = take(tiles * 4);
-  l.blk_cnt = take(tiles * (FF / kQK) * 4);
+  l.tile_cnt = take(tiles * 2 * 4);
   l.ready = take(tiles * 4);
   l.hbuf = take(rows * FF * 4);
   l.ybuf = take(rows * H * 4);
@@ -202,11 +201,8 @@ __device__ __forceinline__ unsigned atom_add_acq_rel(unsigned* p, unsigned v) {
 
 __device__ __forceinline__ void reset_tile_counters(const LayerDev& L, int tid, int nthr) {
   const int tiles = L.n_max * L.K + L.n_max;
-  for (int i = tid; i < tiles; i += nthr) {
-    L.tile_cnt[i] = 0u;
-    L.ready[i] = 0u;
-  }
-  for (int i = tid; i < tiles * L.nbf; i += nthr) L.blk_cnt[i] = 0u;
+  for (int i = tid; i < 2 * tiles; i += nthr) L.tile_cnt[i] = 0u;
+  for (int i = tid; i < tiles; i += nthr) L.ready[i] = 0u;
 }
 
 // Rows [t0, t0 + nt) of caller-provided packed Q8_K rows, once more in 288-byte blocks.
@@ -406,10 +402,9 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev 
     // the owner call that follows this one on the stream plans inside its expert kernel: its
     // workspace is idle now (every earlier kernel of the stream has finished) and gets fresh counters
     for (int i = tid; i < L.rearm_tiles; i += blockDim.x) {
-      L.rearm_tile_cnt[i] = 0u;
+      L.rearm_tile_cnt[i] = L.rearm_tile_cnt[L.rearm_tiles + i] = 0u;
       L.rearm_ready[i] = 0u;
     }
-    for (int i = tid; i < L.rearm_tiles * L.nbf; i += blockDim.x) L.rearm_blk_cnt[i] = 0u;
     if (tid == 0) {
       L.rearm_cnt[9] = 0u;
       L.rearm_cnt[10] = static_cast<unsigned>(L.grid);
@@ -1343,7 +1338,6 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
   L.off = reinterpret_cast<int*>(ws + lay.off);
   L.rec = reinterpret_cast<int4*>(ws + lay.rec);
   L.tile_cnt = reinterpret_cast<unsigned*>(ws + lay.tile_cnt);
-  L.blk_cnt = reinterpret_cast<unsigned*>(ws + lay.blk_cnt);
   L.ready = reinterpret_cast<unsigned*>(ws + lay.ready);
   L.hq = ws + lay.hq;
   L.xq16 = ws + lay.xq16;
@@ -1430,7 +1424,6 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
     unsigned char* ws2 = static_cast<unsigned char*>(a->rearm_workspace);
     L.rearm_cnt = reinterpret_cast<unsigned*>(ws2 + lay2.cnt);
     L.rearm_tile_cnt = reinterpret_cast<unsigned*>(ws2 + lay2.tile_cnt);
-    L.rearm_blk_cnt = reinterpret_cast<unsigned*>(ws2 + lay2.blk_cnt);
     L.rearm_ready = reinterpret_cast<unsigned*>(ws2 + lay2.ready);
     L.rearm_tiles = a->rearm_n_max * a->n_used + a->rearm_n_max;
     L.rearm_mail_n = a->rearm_mail_n;
@@ -1604,7 +1597,7 @@ SGR_API int sgr_moe_layer_decode_static(const sgr_moe_layer* a, void* stream) {
   }
   unsigned char* ws = g_static_ws_addr[dev];
   // what must start at zero: the counters of the route and expert kernels, [cnt, hbuf) of the layout
-  // (cnt, tile_cnt, blk_cnt, ready are adjacent)
+  // (cnt, tile_cnt, ready are adjacent)
   if (cudaMemsetAsync(ws + lay.cnt, 0, lay.hbuf - lay.cnt, as_stream(stream)) != cudaSuccess)
     return kErrLaunch;
   sgr_moe_layer b = *a;
