@@ -324,11 +324,11 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
 #pragma unroll
   for (int g = 0; g < 4; ++g) ldmatrix_x4(raw[g], a_ptr + g * 32);
   loaded();
-  int isum[NT][4];
+  int isum[NT][4], hsum[NT][4];                  // even sub-blocks; odd ones, sixteen-fold
 #pragma unroll
   for (int n = 0; n < NT; ++n)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) isum[n][j] = 0;
+    for (int j = 0; j < 4; ++j) isum[n][j] = hsum[n][j] = 0;
   const int zero[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
@@ -341,20 +341,25 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
       lo[j] = raw[g][j] & 0x0F0F0F0Fu;
       hi[j] = raw[g][j] & 0xF0F0F0F0u;            // 16 * q: see warp_mma_rows
     }
-    const int sh = 16 * (g & 1);
-    const int sc0_lo = ((s_lo.sc[g >> 1] >> sh) & 0xFF) << 4, sc1_lo = (s_lo.sc[g >> 1] >> (sh + 8)) & 0xFF;
-    const int sc0_hi = ((s_hi.sc[g >> 1] >> sh) & 0xFF) << 4, sc1_hi = (s_hi.sc[g >> 1] >> (sh + 8)) & 0xFF;
+    const int sh = 2 * (g & 1);
+    const int sc0_lo = __byte_perm(s_lo.sc[g >> 1], 0, 0x4440 + sh), sc1_lo = __byte_perm(s_lo.sc[g >> 1], 0, 0x4441 + sh);
+    const int sc0_hi = __byte_perm(s_hi.sc[g >> 1], 0, 0x4440 + sh), sc1_hi = __byte_perm(s_hi.sc[g >> 1], 0, 0x4441 + sh);
 #pragma unroll
     for (int n = 0; n < NT; ++n) {
       int c0[4], c1[4];
       mma_u8s8(c0, lo, b[n][0], b[n][1], zero);
       mma_u8s8(c1, hi, b[n][2], b[n][3], zero);
-      isum[n][0] += sc0_lo * c0[0] + sc1_lo * c1[0];
-      isum[n][1] += sc0_lo * c0[1] + sc1_lo * c1[1];
-      isum[n][2] += sc0_hi * c0[2] + sc1_hi * c1[2];
-      isum[n][3] += sc0_hi * c0[3] + sc1_hi * c1[3];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        isum[n][j] += (j < 2 ? sc0_lo : sc0_hi) * c0[j];
+        hsum[n][j] += (j < 2 ? sc1_lo : sc1_hi) * c1[j];
+      }
     }
   }
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) isum[n][j] = 16 * isum[n][j] + hsum[n][j];
   const uint32_t a_lo = tig == 0 ? s_lo.mn[0] : (tig == 1 ? s_lo.mn[1] : 0u);
   const uint32_t a_hi = tig == 0 ? s_hi.mn[0] : (tig == 1 ? s_hi.mn[1] : 0u);
   const uint32_t ma[4] = {a_lo, a_hi, 0u, 0u};
@@ -391,9 +396,9 @@ __device__ __forceinline__ void half_block_dot_regs(const uint4 hdr, const uint4
   const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
   const uint32_t scw = half ? s6.sc[1] : s6.sc[0];
   const uint32_t mnw = half ? s6.mn[1] : s6.mn[0];
-  int isum[TT];
+  int isum[TT], hsum[TT];                       // hsum: sixteen-fold, below 2^29
 #pragma unroll
-  for (int t = 0; t < TT; ++t) isum[t] = 0;
+  for (int t = 0; t < TT; ++t) isum[t] = hsum[t] = 0;
 #pragma unroll
   for (int gg = 0; gg < 2; ++gg) {
     const int g = 2 * half + gg;
@@ -403,7 +408,7 @@ __device__ __forceinline__ void half_block_dot_regs(const uint4 hdr, const uint4
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       lo[i] = raw[i] & 0x0F0F0F0Fu;
-      hi[i] = (raw[i] >> 4) & 0x0F0F0F0Fu;
+      hi[i] = raw[i] & 0xF0F0F0F0u;
     }
     const int sc_lo = (scw >> (16 * gg)) & 0xFF, sc_hi = (scw >> (16 * gg + 8)) & 0xFF;
 #pragma unroll
@@ -411,7 +416,8 @@ __device__ __forceinline__ void half_block_dot_regs(const uint4 hdr, const uint4
       if (t < nt) {
         const uint4* xa = xt.codes(t, 0, 2 * g);
         const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
-        isum[t] += sc_lo * dot8(lo, x0, x1) + sc_hi * dot8(hi, x2, x3);
+        isum[t] += sc_lo * dot8(lo, x0, x1);
+        hsum[t] += sc_hi * dot8_high(hi, x2, x3);
       }
     }
   }
@@ -421,7 +427,8 @@ __device__ __forceinline__ void half_block_dot_regs(const uint4 hdr, const uint4
       const uint4 bs = xt.sums(t, 0);
       int msum = __dp2a_lo(static_cast<int>(half ? bs.z : bs.x), static_cast<int>(mnw), 0);
       msum = __dp2a_hi(static_cast<int>(half ? bs.w : bs.y), static_cast<int>(mnw), msum);
-      const int is = isum[t] + __shfl_xor_sync(0xFFFFFFFFu, isum[t], 1);
+      const int mine = isum[t] + (hsum[t] >> 4);
+      const int is = mine + __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
       const int ms = msum + __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
       acc[t] += xt.scale(t, 0) * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
     }

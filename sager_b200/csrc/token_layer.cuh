@@ -250,15 +250,6 @@ __device__ __forceinline__ void load_half(HalfW<NMAT>& W, const unsigned char* c
   W.d = h2f(static_cast<uint16_t>(dd & 0xFFFFu));
   W.dmin = h2f(static_cast<uint16_t>(dd >> 16));
 }
-// unsigned codes in the high nibbles against signed bytes: sixteen times the dot, without a shift per word
-__device__ __forceinline__ int dot8_high(const uint32_t (&w)[8], const uint4& a, const uint4& b) {
-  const uint32_t x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  int acc = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) asm("dp4a.u32.s32 %0, %1, %2, %0;" : "+r"(acc) : "r"(w[i] & 0xF0F0F0F0u), "r"(x[i]));
-  return acc;
-}
-
 // The half blocks W against the rows of `rs` (a lane pair holds a block; the integer sums of the halves meet before the
 // one rounding, so the terms are block_dot's). Bound by the integer pipe: with two matrices each lane of the pair sends
 // the sum it does not keep and both finish one matrix, which halves the shuffles and the arithmetic after them. Whole
