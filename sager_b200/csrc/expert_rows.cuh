@@ -907,12 +907,13 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   }
 
   // ---- all y rows written everywhere: blend ------------------------------------------------
-  __threadfence();
+  // (the barrier orders the other threads' stores before thread 0's release, which is cumulative)
   rs_consumers_sync();
   if (tid == 0) {
-    atomicAdd(&L.cnt[9], 1u);
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&L.cnt[9]) : "memory");
     unsigned it = 0;
-    while (ld_acquire(&L.cnt[9]) < gridDim.x && ++it < kSpinLimit) __nanosleep(32);
+    while (ld_acquire(&L.cnt[9]) < gridDim.x && ++it < kSpinLimit) {
+    }
     flag[0] = (it < kSpinLimit && ok) ? 1 : 0;
   }
   rs_consumers_sync();
