@@ -124,6 +124,14 @@ __device__ __forceinline__ void tma_load_box(void* dst, const void* gmem_map, in
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
+// The service warps' wait: they wait most of the time, and their polls took a fifth of the issue slots that the consumers need.
+__device__ __forceinline__ bool mbar_wait_idle(uint64_t* bar, uint32_t parity) {
+  for (int it = 0; it < (1 << 20); ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    __nanosleep(40);
+  }
+  return false;
+}
 __device__ __forceinline__ void rs_consumers_sync() {
   asm volatile("bar.sync 5, %0;" ::"n"(kConsumers) : "memory");
 }
@@ -227,6 +235,52 @@ __device__ __forceinline__ void quantize_h_block(const LayerDev& L, const float*
   for (int t0 = 4 * f; t0 < ntok; t0 += 4 * kFinishWarps) {
     if (ntok - t0 > 2) quantize_h_rows<4>(L, src + t0 * kHRow, hrow0 + t0, ntok - t0, hb, lane);
     else quantize_h_rows<2>(L, src + t0 * kHRow, hrow0 + t0, ntok - t0, hb, lane);
+  }
+}
+
+// Half a super-block (sub-blocks 4 * half .. 4 * half + 3) of one weight row against the up to two staged tokens, for a
+// pair of adjacent lanes that share the row: the integer sums of the two halves are added across the pair before the one
+// fp32 rounding, so the result equals block_dot's. `x` is the activation part of the stage. The consumers' integer pipe
+// bounds the stage: odd sub-blocks stay sixteen-fold and the lane's addresses are made once.
+__device__ __forceinline__ void half_dot(const uint4& hdr, const uint4 (&wq)[4], int half, const unsigned char* x, int ntok, float (&acc)[4]) {
+  const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
+  const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
+  const uint32_t scw = half ? s6.sc[1] : s6.sc[0], mnw = half ? s6.mn[1] : s6.mn[0];
+  const unsigned char* codes = x + half * 144;                 // (the second half of a block lies 16 bytes further on)
+  const unsigned char* sums = x + kXCodes + half * 8;
+  int isum[2] = {0, 0}, hsum[2] = {0, 0};                      // hsum: sixteen-fold, below 2^29
+#pragma unroll
+  for (int gg = 0; gg < 2; ++gg) {
+    const uint4 q0 = wq[2 * gg], q1 = wq[2 * gg + 1];
+    const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      lo[i] = raw[i] & 0x0F0F0F0Fu;
+      hi[i] = raw[i] & 0xF0F0F0F0u;
+    }
+    const int sc_lo = __byte_perm(scw, 0, 0x4440 + 2 * gg), sc_hi = __byte_perm(scw, 0, 0x4441 + 2 * gg);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (t < ntok) {                             // warp-uniform
+        const uint4* xa = reinterpret_cast<const uint4*>(codes + t * kXqStride + 64 * gg);
+        const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
+        isum[t] += sc_lo * dot8(lo, x0, x1);
+        hsum[t] += sc_hi * dot8_high(hi, x2, x3);
+      }
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    if (t < ntok) {                               // warp-uniform: the shuffles stay converged
+      const uint2 bs = *reinterpret_cast<const uint2*>(sums + t * 16);
+      const int min_sum = __dp2a_hi(static_cast<int>(bs.y), static_cast<int>(mnw), __dp2a_lo(static_cast<int>(bs.x), static_cast<int>(mnw), 0));
+      const int mine = isum[t] + (hsum[t] >> 4);
+      const int is = mine + __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
+      const int ms = min_sum + __shfl_xor_sync(0xFFFFFFFFu, min_sum, 1);
+      const float scale = *reinterpret_cast<const float*>(x + kXCodes + kTok * 16 + t * 16);
+      acc[t] += scale * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
+    }
   }
 }
 
@@ -533,7 +587,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
 
   if (warp == kWeightWarp) {
     // ---------------- weight warp: the copies of the published groups, stage by stage ----------------
-    int q = 0;
+    int q = 0, s = 0;
+    unsigned ph = 0;
     for (int k = 0;; ++k) {
       bool got;
       const GEntry* ge = follow(k, got);
@@ -543,9 +598,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       }
       const Group wk = sc.decode(ge->id);
       if (!wk.valid) {                           // end of the list: one last stage that only says so
-        const int s = q % kStageCount;
-        const unsigned ph = (q / kStageCount) & 1;
-        if (!mbar_wait(&wempty[s], ph ^ 1u)) {
+        if (!mbar_wait_idle(&wempty[s], ph ^ 1u)) {
           if (lane == 0) atomicExch(L.status, 2);
           return;
         }
@@ -569,16 +622,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         }
       }
       const int cols = wk.kind == 0 ? L.nbh : L.nbf;
-      for (int i = 0; i < wk.nb; ++i, ++q) {
+      for (int i = 0; i < wk.nb; ++i) {
         int half = 0, row0 = wk.gi * kDownRows, blk = i;
         if (wk.kind == 0) {
           half = sc.split ? wk.gi & 1 : (i >= cols ? 1 : 0);
           row0 = (wk.gi >> sc.split) * kGateUpPairs + half * kHalfRows;
           if (i >= cols) blk -= cols;
         }
-        const int s = q % kStageCount;
-        const unsigned ph = (q / kStageCount) & 1;
-        if (!mbar_wait(&wempty[s], ph ^ 1u)) {
+        if (!mbar_wait_idle(&wempty[s], ph ^ 1u)) {
           if (lane == 0) atomicExch(L.status, 2);
           return;
         }
@@ -624,7 +675,9 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           __syncwarp();                            // every lane's part of the stage (and of its descriptor) is written
           if (lane == 0) mbar_arrive(&full[s]);
         }
-        if (lane == 0) *issued = static_cast<unsigned>(q) + 1u;
+        ++q;
+        if (lane == 0) *issued = static_cast<unsigned>(q);
+        if (++s == kStageCount) { s = 0; ph ^= 1u; }
       }
     }
   }
@@ -633,7 +686,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     // ---------------- activation warps ----------------
     const int xtid = tid - kFirstXWarp * 32;
     int myoff = 0;                              // lane t < 16: byte offset of token slot t's row
-    int q = 0;
+    int s = 0;                                  // ring position and its phase
+    unsigned ph = 0;
     for (int k = 0;; ++k) {
       bool got;
       const GEntry* ge = follow(k, got);
@@ -645,9 +699,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       const int4 rc = ge->rc;
       const bool absent = (ge->bits & 1) != 0;
       if (!wk.valid) {                           // end of the list: count in at the last stage and leave
-        const int s = q % kStageCount;
-        const unsigned ph = (q / kStageCount) & 1;
-        if (!mbar_wait(&empty[s], ph ^ 1u)) {
+        if (!mbar_wait_idle(&empty[s], ph ^ 1u)) {
           if (lane == 0) atomicExch(L.status, 2);
           return;
         }
@@ -671,11 +723,9 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           }
         }
       }
-      for (int i = 0; i < wk.nb; ++i, ++q) {
+      for (int i = 0; i < wk.nb; ++i) {
       const int blk = wk.kind == 0 && i >= L.nbh ? i - L.nbh : i;
-      const int s = q % kStageCount;
-      const unsigned ph = (q / kStageCount) & 1;
-      if (!mbar_wait(&empty[s], ph ^ 1u)) {
+      if (!mbar_wait_idle(&empty[s], ph ^ 1u)) {
         if (lane == 0) atomicExch(L.status, 2);
         return;
       }
@@ -700,6 +750,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         }
       }
       cp_async_arrive(&full[s]);
+      if (++s == kStageCount) { s = 0; ph ^= 1u; }
       }   // block columns of the group
     }
   }
@@ -724,7 +775,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       const int4 rc = ge->rc;
       const bool absent = (ge->bits & 1) != 0;
       const int buf = g & 1;
-      if (!__all_sync(0xFFFFFFFFu, mbar_wait(&hfull[buf], (g >> 1) & 1))) {
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait_idle(&hfull[buf], (g >> 1) & 1))) {
         if (lane == 0) atomicExch(L.status, 6);
         return;
       }
@@ -768,11 +819,14 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   }
 
   // ---------------- consumers ----------------
-  float acc[2][4];
+  float acc[2][4];                               // (up to two token rows: acc[0][0], acc[0][1])
   bool ok = true;
-  for (int q = 0;; ++q) {
-    const int s = q % kStageCount;
-    const unsigned ph = (q / kStageCount) & 1;
+  // offsets in a stage, set when a group's half or a down group starts: this lane's half-block row, or its ldmatrix row and
+  // the rows gid and gid + 8 that it owns results of
+  int w_off = 0, own_lo = 0, own_hi = 0;
+  int s = 0;
+  unsigned ph = 0;
+  for (;; ph ^= s == kStageCount - 1 ? 1u : 0u, s = s == kStageCount - 1 ? 0 : s + 1) {
     if (!mbar_wait(&full[s], ph)) {
       if (lane == 0) atomicExch(L.status, 3);
       ok = false;
@@ -785,9 +839,33 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     if (d_blk == 0) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[0][j] = acc[1][j] = 0.f;
+      // unit u of the warp's sixteen: gate rows 0 .. 7 and the up rows of the same pairs, or sixteen down rows
+      auto row_at = [&](int u) {
+        return d_kind == 0 ? ((u & 7) + 8 * warp) * kW4 + (u >> 3) * kHalfBytes : (16 * warp + u) * kW4;
+      };
+      if (d_ntok <= 2) {
+        w_off = row_at(lane >> 1);
+      } else {
+        w_off = row_at((lane & 7) + ((lane >> 3) & 1) * 8) + 16 + (lane >> 4) * 16;
+        own_lo = row_at(lane >> 2);
+        own_hi = row_at((lane >> 2) + 8);
+      }
     }
     bool w_released = false;
-    if (d_mode == 0) {
+    if (d_mode == 0 && d_ntok <= 2) {
+      // the lane's half block goes to registers and the weight part of the stage back to the
+      // weight warp before the arithmetic: its refill is the long round trip of the ring
+      const uint4* wrow = reinterpret_cast<const uint4*>(st + w_off);
+      const int half = lane & 1;
+      const uint4 hdr = wrow[0];
+      uint4 wq[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) wq[i] = wrow[1 + 4 * half + i];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&wempty[s]);
+      w_released = true;
+      half_dot(hdr, wq, half, st + kWBytes, d_ntok, acc[0]);
+    } else if (d_mode == 0) {
       XTile xt;
       xt.qs = reinterpret_cast<int8_t*>(st + kWBytes);
       xt.bs = reinterpret_cast<int16_t*>(st + kWBytes + kXCodes);
@@ -797,34 +875,13 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       xt.tok_stride = kXqStride;
       xt.d_step = 4;
       xt.mid_pad = 16;
-      // unit row u of this warp -> byte offset of its block in the stage
-      auto row_at = [&](int u) {
-        return d_kind == 0 ? ((u & 7) + 8 * warp) * kW4 + (u >> 3) * kHalfBytes : (16 * warp + u) * kW4;
-      };
-      if (d_ntok <= 2) {
-        // the lane's half block goes to registers and the weight part of the stage back to the
-        // weight warp before the arithmetic: its refill is the long round trip of the ring
-        float a2[2] = {acc[0][0], acc[0][1]};
-        uint4 hdr, wq[4];
-        half_block_load(reinterpret_cast<const uint4*>(st + row_at(lane >> 1)), lane & 1, hdr, wq);
+      auto loaded = [&]() {
         __syncwarp();
         if (lane == 0) mbar_arrive(&wempty[s]);
-        w_released = true;
-        half_block_dot_regs<2>(hdr, wq, lane & 1, xt, d_ntok, a2);
-        acc[0][0] = a2[0];
-        acc[0][1] = a2[1];
-      } else {
-        const unsigned char* a_ptr = st + row_at((lane & 7) + ((lane >> 3) & 1) * 8) + 16 + (lane >> 4) * 16;
-        const unsigned char* h_lo = st + row_at(lane >> 2);
-        const unsigned char* h_hi = st + row_at((lane >> 2) + 8);
-        auto loaded = [&]() {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&wempty[s]);
-        };
-        w_released = true;
-        if (d_ntok <= 8) warp_mma_block<1>(a_ptr, h_lo, h_hi, xt, acc, loaded);
-        else warp_mma_block<2>(a_ptr, h_lo, h_hi, xt, acc, loaded);
-      }
+      };
+      w_released = true;
+      if (d_ntok <= 8) warp_mma_block<1>(st + w_off, st + own_lo, st + own_hi, xt, acc, loaded);
+      else warp_mma_block<2>(st + w_off, st + own_lo, st + own_hi, xt, acc, loaded);
     }
     __syncwarp();
     if (lane == 0) {                             // this warp no longer reads the stage

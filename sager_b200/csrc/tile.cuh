@@ -384,72 +384,6 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
   }
 }
 
-// Half a super-block (sub-blocks 4*half .. 4*half+3) of one weight row against up to
-// TT staged tokens (block 0 of a tile staged with nb == 1), for a pair of adjacent
-// lanes that share the row: the integer sums of the two halves are added across
-// the pair before the one fp32 rounding, so the result equals block_dot's.
-template <int TT>
-__device__ __forceinline__ void half_block_dot_regs(const uint4 hdr, const uint4 (&wq)[4], int half, const XTile& xt,
-                                                    int nt, float (&acc)[TT]) {
-  const float d = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x & 0xFFFFu)));
-  const float dmin = __half2float(__ushort_as_half(static_cast<uint16_t>(hdr.x >> 16)));
-  const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-  const uint32_t scw = half ? s6.sc[1] : s6.sc[0];
-  const uint32_t mnw = half ? s6.mn[1] : s6.mn[0];
-  int isum[TT], hsum[TT];                       // hsum: sixteen-fold, below 2^29
-#pragma unroll
-  for (int t = 0; t < TT; ++t) isum[t] = hsum[t] = 0;
-#pragma unroll
-  for (int gg = 0; gg < 2; ++gg) {
-    const int g = 2 * half + gg;
-    const uint4 q0 = wq[2 * gg], q1 = wq[2 * gg + 1];
-    const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    uint32_t lo[8], hi[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      lo[i] = raw[i] & 0x0F0F0F0Fu;
-      hi[i] = raw[i] & 0xF0F0F0F0u;
-    }
-    const int sc_lo = (scw >> (16 * gg)) & 0xFF, sc_hi = (scw >> (16 * gg + 8)) & 0xFF;
-#pragma unroll
-    for (int t = 0; t < TT; ++t) {
-      if (t < nt) {
-        const uint4* xa = xt.codes(t, 0, 2 * g);
-        const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
-        isum[t] += sc_lo * dot8(lo, x0, x1);
-        hsum[t] += sc_hi * dot8_high(hi, x2, x3);
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < TT; ++t) {
-    if (t < nt) {                               // nt is warp-uniform: the shuffles stay converged
-      const uint4 bs = xt.sums(t, 0);
-      int msum = __dp2a_lo(static_cast<int>(half ? bs.z : bs.x), static_cast<int>(mnw), 0);
-      msum = __dp2a_hi(static_cast<int>(half ? bs.w : bs.y), static_cast<int>(mnw), msum);
-      const int mine = isum[t] + (hsum[t] >> 4);
-      const int is = mine + __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
-      const int ms = msum + __shfl_xor_sync(0xFFFFFFFFu, msum, 1);
-      acc[t] += xt.scale(t, 0) * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
-    }
-  }
-}
-
-// The same from shared memory: the lane's half of the block is read first, so a caller that wants
-// to hand the weight bytes back before the arithmetic can use the two steps separately.
-__device__ __forceinline__ void half_block_load(const uint4* wrow, int half, uint4& hdr, uint4 (&wq)[4]) {
-  hdr = wrow[0];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) wq[i] = wrow[1 + 4 * half + i];
-}
-template <int TT>
-__device__ __forceinline__ void half_block_dot(const uint4* wrow, int half, const XTile& xt, int nt,
-                                               float (&acc)[TT]) {
-  uint4 hdr, wq[4];
-  half_block_load(wrow, half, hdr, wq);
-  half_block_dot_regs<TT>(hdr, wq, half, xt, nt, acc);
-}
-
 // Four warps cover the tile: with at least four 16-row groups each warp takes
 // groups w, w+4, ...; with fewer, the warps of a group split the super-blocks and
 // their partial sums meet in shared memory (fixed order, so results are
