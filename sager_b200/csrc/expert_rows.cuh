@@ -1,14 +1,14 @@
 // expert_rows.cuh - the expert kernel for layers with many token rows (part of
 // moe_layer.cu, which defines LayerDev and the plan before including this file).
 //
-// A persistent kernel, one CTA per SM: 16 consumer warps, a weight warp, three
-// activation warps and a finisher warp.
-// Work is cut into groups: 128 (gate, up) row pairs of one tile (up to 16 token
-// rows of one expert), or 256 rows of its down matrix. A group is streamed through
-// a ring of shared-memory stages one super-block column at a time: a stage holds
-// the 144-byte blocks of the group's 256 weight rows for one block index, plus
+// A persistent kernel, one CTA per SM: 16 consumer warps, a preparing warp, a weight warp,
+// two activation warps and two finisher warps.
+// Work is cut into groups: the 256 (gate, up) row pairs of one block of h of one tile (up to 16
+// token rows of one expert) - or half of them where groups are few -, or 256 rows of its down
+// matrix. A group is streamed through a ring of three shared-memory stages one super-block column
+// at a time: a stage holds the 144-byte blocks of 256 weight rows for one block index, plus
 // that block of the tile's activation rows, re-laid for the dot engine. Every
-// consumer warp owns sixteen of the rows for the whole group - eight gate rows
+// consumer warp owns sixteen of the rows - eight gate rows
 // and the eight up rows of the same indices, so SwiGLU needs no exchange - and
 // keeps its sums in registers from the first column to the last: no partial sums
 // in shared memory, no barrier between the warps; the only synchronisation is
@@ -16,26 +16,30 @@
 //
 // The weight part of a stage arrives by TMA: two tiled copies per stage (boxes of
 // 144 bytes x 128 rows) through 2-D tensor maps over [rows][row bytes]. The maps
-// are made on the host for a placeholder address; the weight warp patches a group's
-// descriptors while the group before it streams: the expert's base addresses go into shared-memory copies
-// (tensormap.replace), publishes them to a per-CTA ring of descriptors in global
-// memory (tensormap.cp_fenceproxy) and acquires them before use. (16-byte cp.async
+// are made on the host for a placeholder address; the preparing warp patches a group's
+// descriptors some stages ahead of its copies: the expert's base addresses go into shared-memory
+// copies (tensormap.replace), are published to a per-CTA ring of descriptors in global
+// memory (tensormap.cp_fenceproxy) and acquired by the weight warp before use. (16-byte cp.async
 // copies reach the same HBM rate on their own, but every one of them passes through
 // the load/store pipe that the consumers' shared-memory loads need; bulk copies of
-// 144 bytes are issue-bound at roughly one per 60 cycles and warp.) Three more
-// producer warps copy the stage's block of the tile's activation rows with
+// 144 bytes are issue-bound at roughly one per 60 cycles and warp.) The activation
+// warps copy the stage's block of the tile's activation rows with
 // cp.async. The two roles walk the same list of stages independently, so the
 // weight stream never waits for an activation row that is not ready yet. Experts
 // whose pointers are not 16-byte aligned cannot go through TMA: the weight warp
 // copies them with plain loads.
 //
-// Gate/up groups write fp32 h. The last warp of a CTA to finish a group counts
-// the CTA in at the group's 256-wide block of h (global counter); the CTA that
-// completes the block quantises it for the tile's rows to Q8_K (padded 288-byte
-// blocks, 16-byte copyable) and publishes it; the activation warp waits
-// (bounded) for a tile's blocks before it copies them for a down group.
+// Gate/up groups leave h in shared memory, where the finisher warps quantise it to Q8_K (padded
+// 288-byte blocks, 16-byte copyable) and publish the block; half groups exchange their halves through
+// global memory first. A down group's activations are copied once its tile's blocks are all
+// published; the preparing warp watches for that (bounded) and draws no further group meanwhile.
 // Down groups write fp32 y; after a grid-wide barrier the CTAs add
-// residual + sum_k w_k * y_k + shared expert (combine_rows).
+// residual + sum_k w_k * y_k + shared expert (combine_flat).
+//
+// What bounds it at 64 rows over 256 experts (hidden 2048, n_ff 512, 160 distinct experts under the
+// benchmark's skew: 284 MB, 44 us of HBM): 90 us per layer with the route kernel, of which 28 until the
+// first stage is there, 65 of streaming - 49 without the arithmetic, whose integer instructions hold the
+// stages back -, 7 of barrier and blend (101 with five stages, one finisher and blocks of h shared by two CTAs).
 #pragma once
 
 namespace rs {

@@ -1,19 +1,16 @@
-// moe_layer.cu - one MoE layer of a decode step (1..64 token rows) in two
-// launches chained with programmatic dependent launch:
+// moe_layer.cu - one MoE layer of a decode step (1..64 token rows): for up to four rows one
+// persistent launch (token_layer.cuh), else two launches chained with programmatic dependent launch:
 //
-//   route   : Q8_K-quantise the rows, router logits, softmax/top-k, and - in the
-//             last CTA to finish - the expert-major plan of the layer (tiles of up
-//             to 16 rows per expert)
-//   experts : a persistent kernel, one CTA per SM. Work items are (tile, row chunk)
-//             pairs: first every gate/up item (16 rows of gate and of up for one
-//             tile: SwiGLU, fp32 h rows), then every down item (64 rows of the down
-//             matrix: Q8_K-quantise h, fp32 y rows). A producer warp streams the
-//             weight rows of the CTA's items through a ring of shared-memory
-//             stages with TMA bulk copies, several items ahead of the eight
-//             consumer warps, which run int8 tensor-core MMAs on them. Down items
-//             wait (bounded) for the gate/up items of their tile; their weights are
-//             already in flight by then. The last CTA to finish a 64-row chunk of
-//             the output adds residual + sum_k w_k * y_k + shared expert.
+//   route   : Q8_K-quantise the rows, router logits, softmax/top-k, and - where the expert
+//             kernel does not make it itself - in the last CTA to finish the expert-major plan
+//             of the layer (tiles of up to 16 rows per expert)
+//   experts : a persistent kernel, one CTA per SM: expert_rows.cuh streams groups of weight
+//             rows by super-block columns; the item kernel below (selectable, and where the former
+//             does not apply) takes (tile, row chunk) items - first every gate/up item (16 rows of
+//             gate and of up for one tile: SwiGLU, fp32 h rows), then every down item (64 rows of
+//             the down matrix: Q8_K-quantise h, fp32 y rows) - through a ring of shared-memory
+//             stages with TMA bulk copies. Down work waits (bounded) for the gate/up work of its
+//             tile. At the end residual + sum_k w_k * y_k + shared expert is added.
 //
 // It replaces the launch sequence of the reference's device-dispatch path
 // (Session::moe_dispatch_device, src/core/session.cpp:2482-3030: quantize_q8_k,
@@ -28,8 +25,7 @@
 // AVX2 path more closely than the reference's fp16-staged device path does.
 //
 // Every weight byte is read once, and the weight stream never stops at the
-// gate/up -> down dependency. The route kernel prefetches the router matrix into
-// L2 before it waits for the previous layer.
+// gate/up -> down dependency.
 #include <cuda.h>
 
 #include <algorithm>
@@ -347,9 +343,10 @@ inline size_t plan_smem(int E, int, int) { return static_cast<size_t>(E) * 12 + 
 // fp16, k-major in groups of T rows, by all warps in one pass of loads; then eight warps do R x T
 // logits each while the other eight quantise, and the last CTA of the tile selects with two warps per
 // row. As few experts per CTA as one wave allows: the chain of phases bounds the launch, not its
-// bytes, and a lane's FMAs cannot be split (their order is the reference's). 64 rows, 256 experts,
-// hidden 2048: ROUTE_64; 8 rows: ROUTE_8 (one phase after the other with eight warps, fp32 activations and a
-// serial selection: 20.2 and 20.2).
+// bytes, and a lane's FMAs cannot be split (their order is the reference's). To the end of the
+// selection at 256 experts, hidden 2048: 11.3 us for 8 rows, 17.6 for 64 (20.2 both with one phase after
+// the other in eight warps, sixteen experts per CTA and one warp per selected row); at 64 rows six
+// of them are 160 KB per CTA on their way out of L2, two the logits, three the selection.
 // Dynamic smem: route_rows * H floats, 8 * H halves (the selection and the plan reuse it).
 template <int R, int T>
 __device__ __forceinline__ void route_tile_logits(const LayerDev& L, const uint16_t* xs, const float* ws, int tok0, int nt,
