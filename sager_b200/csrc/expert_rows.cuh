@@ -242,50 +242,35 @@ __device__ __forceinline__ void quantize_h_block(const LayerDev& L, const float*
   }
 }
 
-// Half a super-block (sub-blocks 4 * half .. 4 * half + 3) of one weight row against the up to two staged tokens, for a
-// pair of adjacent lanes that share the row: the integer sums of the two halves are added across the pair before the one
-// fp32 rounding, so the result equals block_dot's. `x` is the activation part of the stage. The consumers' integer pipe
-// bounds the stage: odd sub-blocks stay sixteen-fold and the lane's addresses are made once.
-__device__ __forceinline__ void half_dot(const uint4& hdr, const uint4 (&wq)[4], int half, const unsigned char* x, int ntok, float (&acc)[4]) {
-  const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
+// Half a super-block (sub-blocks 4 * half .. 4 * half + 3) of one weight row against a tile's only token row, for a
+// pair of adjacent lanes that share the weight row: the integer sums of the two halves are added across the pair before
+// the one fp32 rounding, so the result equals block_dot's. `x` is the activation part of the stage. The consumers'
+// integer pipe bounds the stage: odd sub-blocks stay sixteen-fold. (From two rows on the MMA below costs less: 64 rows
+// over 256 experts 90.4 -> 88.8 us per layer, 8 rows 50.8 -> 49.6; at one row it loses, 93.6 and 55.2.)
+__device__ __forceinline__ float half_dot(const uint4& hdr, const uint4 (&wq)[4], int half, const unsigned char* x) {
   const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
   const uint32_t scw = half ? s6.sc[1] : s6.sc[0], mnw = half ? s6.mn[1] : s6.mn[0];
   const unsigned char* codes = x + half * 144;                 // (the second half of a block lies 16 bytes further on)
-  const unsigned char* sums = x + kXCodes + half * 8;
-  int isum[2] = {0, 0}, hsum[2] = {0, 0};                      // hsum: sixteen-fold, below 2^29
+  int isum = 0, hsum = 0;                                      // hsum: sixteen-fold, below 2^29
 #pragma unroll
   for (int gg = 0; gg < 2; ++gg) {
     const uint4 q0 = wq[2 * gg], q1 = wq[2 * gg + 1];
     const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    uint32_t lo[8], hi[8];
+    uint32_t lo[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      lo[i] = raw[i] & 0x0F0F0F0Fu;
-      hi[i] = raw[i] & 0xF0F0F0F0u;
-    }
-    const int sc_lo = __byte_perm(scw, 0, 0x4440 + 2 * gg), sc_hi = __byte_perm(scw, 0, 0x4441 + 2 * gg);
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      if (t < ntok) {                             // warp-uniform
-        const uint4* xa = reinterpret_cast<const uint4*>(codes + t * kXqStride + 64 * gg);
-        const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
-        isum[t] += sc_lo * dot8(lo, x0, x1);
-        hsum[t] += sc_hi * dot8_high(hi, x2, x3);
-      }
-    }
+    for (int i = 0; i < 8; ++i) lo[i] = raw[i] & 0x0F0F0F0Fu;
+    const uint4* xa = reinterpret_cast<const uint4*>(codes + 64 * gg);
+    const uint4 x0 = xa[0], x1 = xa[1], x2 = xa[2], x3 = xa[3];
+    isum += static_cast<int>(__byte_perm(scw, 0, 0x4440 + 2 * gg)) * dot8(lo, x0, x1);
+    hsum += static_cast<int>(__byte_perm(scw, 0, 0x4441 + 2 * gg)) * dot8_high(raw, x2, x3);
   }
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    if (t < ntok) {                               // warp-uniform: the shuffles stay converged
-      const uint2 bs = *reinterpret_cast<const uint2*>(sums + t * 16);
-      const int min_sum = __dp2a_hi(static_cast<int>(bs.y), static_cast<int>(mnw), __dp2a_lo(static_cast<int>(bs.x), static_cast<int>(mnw), 0));
-      const int mine = isum[t] + (hsum[t] >> 4);
-      const int is = mine + __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
-      const int ms = min_sum + __shfl_xor_sync(0xFFFFFFFFu, min_sum, 1);
-      const float scale = *reinterpret_cast<const float*>(x + kXCodes + kTok * 16 + t * 16);
-      acc[t] += scale * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
-    }
-  }
+  const uint2 bs = *reinterpret_cast<const uint2*>(x + kXCodes + half * 8);
+  const int min_sum = __dp2a_hi(static_cast<int>(bs.y), static_cast<int>(mnw), __dp2a_lo(static_cast<int>(bs.x), static_cast<int>(mnw), 0));
+  const int mine = isum + (hsum >> 4);
+  const int is = mine + __shfl_xor_sync(0xFFFFFFFFu, mine, 1);
+  const int ms = min_sum + __shfl_xor_sync(0xFFFFFFFFu, min_sum, 1);
+  const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
+  return *reinterpret_cast<const float*>(x + kXCodes + kTok * 16) * (d * static_cast<float>(is) - dmin * static_cast<float>(ms));
 }
 
 // Every thread of the CTA: the plan of build_plan (moe_layer.cu) in shared memory - same masks, same
@@ -823,7 +808,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
   }
 
   // ---------------- consumers ----------------
-  float acc[2][4];                               // (up to two token rows: acc[0][0], acc[0][1])
+  float acc[2][4];                               // (one token row: acc[0][0])
   bool ok = true;
   // offsets in a stage, set when a group's half or a down group starts: this lane's half-block row, or its ldmatrix row and
   // the rows gid and gid + 8 that it owns results of
@@ -847,7 +832,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       auto row_at = [&](int u) {
         return d_kind == 0 ? ((u & 7) + 8 * warp) * kW4 + (u >> 3) * kHalfBytes : (16 * warp + u) * kW4;
       };
-      if (d_ntok <= 2) {
+      if (d_ntok == 1) {
         w_off = row_at(lane >> 1);
       } else {
         w_off = row_at((lane & 7) + ((lane >> 3) & 1) * 8) + 16 + (lane >> 4) * 16;
@@ -856,7 +841,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       }
     }
     bool w_released = false;
-    if (d_mode == 0 && d_ntok <= 2) {
+    if (d_mode == 0 && d_ntok == 1) {
       // the lane's half block goes to registers and the weight part of the stage back to the
       // weight warp before the arithmetic: its refill is the long round trip of the ring
       const uint4* wrow = reinterpret_cast<const uint4*>(st + w_off);
@@ -868,7 +853,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       __syncwarp();
       if (lane == 0) mbar_arrive(&wempty[s]);
       w_released = true;
-      half_dot(hdr, wq, half, st + kWBytes, d_ntok, acc[0]);
+      acc[0][0] += half_dot(hdr, wq, half, st + kWBytes);
     } else if (d_mode == 0) {
       XTile xt;
       xt.qs = reinterpret_cast<int8_t*>(st + kWBytes);
@@ -912,14 +897,9 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         }
       } else {
         float* hb = hs + (d_seq & 1) * kTok * kHRow + d.half() * kHalfRows + 8 * warp;
-        if (d_ntok <= 2) {
-          const float u0 = __shfl_down_sync(0xFFFFFFFFu, acc[0][0], 16);
-          const float u1 = __shfl_down_sync(0xFFFFFFFFu, acc[0][1], 16);
-          if (lane < 16 && (lane & 1) == 0) {
-            const float g0 = acc[0][0], g1 = acc[0][1];
-            hb[lane >> 1] = g0 / (1.f + expf(-g0)) * u0;
-            if (d_ntok > 1) hb[kHRow + (lane >> 1)] = g1 / (1.f + expf(-g1)) * u1;
-          }
+        if (d_ntok == 1) {
+          const float g = acc[0][0], u = __shfl_down_sync(0xFFFFFFFFu, g, 16);
+          if (lane < 16 && (lane & 1) == 0) hb[lane >> 1] = g / (1.f + expf(-g)) * u;
         } else {
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
@@ -943,12 +923,8 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           L.ybuf[static_cast<size_t>(d.hrow0 + j / 16) * L.H + d.row0 + 16 * warp + (j & 15)] = 0.f;
         continue;
       }
-      if (d_ntok <= 2) {
-        if ((lane & 1) == 0) {
-          const int col = d.row0 + 16 * warp + (lane >> 1);
-          L.ybuf[static_cast<size_t>(d.hrow0) * L.H + col] = acc[0][0];
-          if (d_ntok > 1) L.ybuf[static_cast<size_t>(d.hrow0 + 1) * L.H + col] = acc[0][1];
-        }
+      if (d_ntok == 1) {
+        if ((lane & 1) == 0) L.ybuf[static_cast<size_t>(d.hrow0) * L.H + d.row0 + 16 * warp + (lane >> 1)] = acc[0][0];
       } else {
         const int col = d.row0 + 16 * warp + gid;
 #pragma unroll
