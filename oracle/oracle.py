@@ -35,7 +35,7 @@ def build(ref_root: str | None = None) -> None:
     reference's own CPU sources."""
     ref_root = ref_root or reference_root()
     subprocess.check_call(["make", "-s", "-C", HERE, "oracle"])
-    if os.path.isdir(ref_root):
+    if os.path.isdir(os.path.join(ref_root, "src")):          # (an empty directory is no tree)
         subprocess.check_call(["make", "-s", "-C", HERE, "ref", f"REF={ref_root}"],
                               stderr=subprocess.DEVNULL)
         subprocess.check_call(["make", "-s", "-C", HERE, "refcuda", f"REF={ref_root}"],
