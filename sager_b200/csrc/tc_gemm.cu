@@ -212,12 +212,44 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const __grid_consta
   if (threadIdx.x == 0 && *fail != 0 && a.status != nullptr) atomicExch(a.status, 1);
 }
 
+// ---- dequantisation ----------------------------------------------------------------------
+// Lane l of a warp owns weights 8l .. 8l+7 of one super-block: sub-block l/4, its
+// (l%4)-th octet. The warp's 32 stores are one contiguous 512-byte run.
+// value = fp16( fma(d*sc, q, -(dmin*m)) ): one rounding to fp32, one to fp16
+// (src/kernels/cuda/tc_gemm.cu:58-95 of the reference).
+__device__ __forceinline__ uint4 dequant_octet(const unsigned char* blk, int lane) {
+  const uint32_t dm = __ldg(reinterpret_cast<const uint32_t*>(blk));
+  const Scales6 s6 = unpack_scales6(__ldg(reinterpret_cast<const uint32_t*>(blk + 4)),
+                                    __ldg(reinterpret_cast<const uint32_t*>(blk + 8)),
+                                    __ldg(reinterpret_cast<const uint32_t*>(blk + 12)));
+  const int sb = lane >> 2, q = lane & 3;
+  const float sd = h2f(static_cast<uint16_t>(dm & 0xFFFFu)) *
+                   static_cast<float>(((sb < 4 ? s6.sc[0] : s6.sc[1]) >> (8 * (sb & 3))) & 0xFFu);
+  const float sm = h2f(static_cast<uint16_t>(dm >> 16)) *
+                   static_cast<float>(((sb < 4 ? s6.mn[0] : s6.mn[1]) >> (8 * (sb & 3))) & 0xFFu);
+  const uint32_t* qp = reinterpret_cast<const uint32_t*>(blk + 16 + (sb >> 1) * 32 + q * 8);
+  const uint2 w = make_uint2(__ldg(qp), __ldg(qp + 1));
+  const int shift = (sb & 1) * 4;
+  auto half_of = [&](uint32_t word, int byte) -> uint32_t {
+    const uint32_t nib = (word >> (8 * byte + shift)) & 0xFu;
+    return f2h(__fmaf_rn(sd, static_cast<float>(nib), -sm));
+  };
+  uint4 o;
+  o.x = half_of(w.x, 0) | (half_of(w.x, 1) << 16);
+  o.y = half_of(w.x, 2) | (half_of(w.x, 3) << 16);
+  o.z = half_of(w.y, 0) | (half_of(w.y, 1) << 16);
+  o.w = half_of(w.y, 2) | (half_of(w.y, 3) << 16);
+  return o;
+}
+
 // ---- Q4_K weights: the dequantisation inside the GEMM ------------------------------------------
 // A CTA owns 128 weight rows and up to 256 token rows. The 128 rows are the M lanes of tensor memory, so a thread
 // dequantises its row of a block in registers and stores it as the tensor-memory operand (tcgen05.st); only the
 // activations go through shared memory. Against a separate dequantisation and 128 x 128 tiles (7.5 + 64 us for
 // 4096 x 2048 over 2048 rows) that reads 36 bytes of weights per 64 k instead of 128 and half the activations: the
-// tiles' traffic from L2 was the bound. 43.7 us now, the MMAs' own time being 21. `scratch` still receives the dequantised rows (each token tile writes its share of the blocks).
+// tiles' traffic from L2 was the bound. 43.7 us now, the MMAs' own time being 21. `scratch` still receives the dequantised
+// rows: with few tiles by CTAs of their own on the SMs left over (a thread's 16-byte pieces of its row take longer than its
+// block: 1000 x 4096 over 75 rows 33.8 -> 22.6 us, over 64 rows 54.5 -> 22.5), else each token tile writes its share of the blocks.
 //   * warps 0-7: unpack, four to a block, even and odd blocks; then the epilogue
 //   * warp 8: activation tiles (TMA, 128-byte swizzle, 64 k a stage)
 //   * warp 9: block columns of the weights (cp.async), four in flight
@@ -231,7 +263,7 @@ struct Q4Args {
   const unsigned char* w;
   uint16_t *y, *scratch;
   int n_rows, k, n_tokens;
-  int bn, stages;                                 // token rows per CTA, activation stages
+  int bn, stages, tiles;                          // token rows per CTA, activation stages, token tiles (grid.y beyond: scratch)
   int* status;
 };
 
@@ -247,6 +279,23 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * 128, tok0 = blockIdx.y * a.bn;
   const int ntok = min(a.bn, a.n_tokens - tok0), nb = a.k / kQK;
+  if (static_cast<int>(blockIdx.y) >= a.tiles) {  // writes the row tile's dequantised blocks, a warp per block
+    pdl_wait();
+    pdl_launch_dependents();
+    const int blocks = min(128, a.n_rows - row0) * nb, part = blockIdx.y - a.tiles, parts = gridDim.y - a.tiles;
+    const unsigned char* w = a.w + static_cast<size_t>(row0) * nb * kW4;
+    uint4* out = reinterpret_cast<uint4*>(a.scratch + static_cast<size_t>(row0) * a.k);
+    const int stride = parts * (kQ4Threads / 32);
+    for (int b = part * (kQ4Threads / 32) + warp; b < blocks; b += 4 * stride) {
+      uint4 v[4];                                 // four blocks' loads in flight
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = dequant_octet(w + static_cast<size_t>(min(b + u * stride, blocks - 1)) * kW4, lane);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (b + u * stride < blocks) out[static_cast<size_t>(b + u * stride) * 32 + lane] = v[u];
+    }
+    return;
+  }
   const uint32_t b_bytes = static_cast<uint32_t>(a.bn) * 128;
 
   if (threadIdx.x == 0) {
@@ -279,7 +328,8 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     pdl_wait();                                   // scratch and y may still be read by the kernel before
     pdl_launch_dependents();
     const f32x2 magic = splat2(-8388608.f);
-    const int share = gridDim.y;                  // this token tile writes blocks blockIdx.y, + share, ... to scratch
+    const int share = a.tiles;                    // this token tile writes blocks blockIdx.y, + share, ... to scratch
+    const bool writes = static_cast<int>(gridDim.y) == a.tiles;
     uint16_t* row_out = a.scratch + static_cast<size_t>(min(row0 + r, a.n_rows - 1)) * a.k;
     bool ok = true;
     for (int job = grp; job < nb && ok; job += 2) {
@@ -289,7 +339,7 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
       const uint4 hdr = blk[0];
       const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
       const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-      const bool keep = job % share == static_cast<int>(blockIdx.y) && row0 + r < a.n_rows;
+      const bool keep = writes && job % share == static_cast<int>(blockIdx.y) && row0 + r < a.n_rows;
 #pragma unroll 1
       for (int g = 0; g < 4; ++g) {
         const int x = 2 * job + (g >> 1), slot = x % kQ4Slots;
@@ -427,36 +477,6 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
   if (threadIdx.x == 0 && *fail != 0 && a.status != nullptr) atomicExch(a.status, 1);
-}
-
-// ---- dequantisation ----------------------------------------------------------------------
-// Lane l of a warp owns weights 8l .. 8l+7 of one super-block: sub-block l/4, its
-// (l%4)-th octet. The warp's 32 stores are one contiguous 512-byte run.
-// value = fp16( fma(d*sc, q, -(dmin*m)) ): one rounding to fp32, one to fp16
-// (src/kernels/cuda/tc_gemm.cu:58-95 of the reference).
-__device__ __forceinline__ uint4 dequant_octet(const unsigned char* blk, int lane) {
-  const uint32_t dm = __ldg(reinterpret_cast<const uint32_t*>(blk));
-  const Scales6 s6 = unpack_scales6(__ldg(reinterpret_cast<const uint32_t*>(blk + 4)),
-                                    __ldg(reinterpret_cast<const uint32_t*>(blk + 8)),
-                                    __ldg(reinterpret_cast<const uint32_t*>(blk + 12)));
-  const int sb = lane >> 2, q = lane & 3;
-  const float sd = h2f(static_cast<uint16_t>(dm & 0xFFFFu)) *
-                   static_cast<float>(((sb < 4 ? s6.sc[0] : s6.sc[1]) >> (8 * (sb & 3))) & 0xFFu);
-  const float sm = h2f(static_cast<uint16_t>(dm >> 16)) *
-                   static_cast<float>(((sb < 4 ? s6.mn[0] : s6.mn[1]) >> (8 * (sb & 3))) & 0xFFu);
-  const uint32_t* qp = reinterpret_cast<const uint32_t*>(blk + 16 + (sb >> 1) * 32 + q * 8);
-  const uint2 w = make_uint2(__ldg(qp), __ldg(qp + 1));
-  const int shift = (sb & 1) * 4;
-  auto half_of = [&](uint32_t word, int byte) -> uint32_t {
-    const uint32_t nib = (word >> (8 * byte + shift)) & 0xFu;
-    return f2h(__fmaf_rn(sd, static_cast<float>(nib), -sm));
-  };
-  uint4 o;
-  o.x = half_of(w.x, 0) | (half_of(w.x, 1) << 16);
-  o.y = half_of(w.x, 2) | (half_of(w.x, 3) << 16);
-  o.z = half_of(w.y, 0) | (half_of(w.y, 1) << 16);
-  o.w = half_of(w.y, 2) | (half_of(w.y, 3) << 16);
-  return o;
 }
 
 __global__ void __launch_bounds__(256) dequant_rows_kernel(const unsigned char* __restrict__ w,
@@ -607,8 +627,12 @@ int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratc
   CUtensorMap mx;
   if (!operand_map(&mx, x, n_tokens, k, kLayoutSwizzled, bn)) return kErrUnsupported;
   if (!opt_in_smem<tc_gemm_q4_kernel>(kQ4Smem)) return kErrLaunch;
-  Q4Args a{static_cast<const unsigned char*>(w), y, scratch, n_rows, k, n_tokens, bn, std::min(8, kQ4BBytes / (bn * 128)), status_word()};
-  return launch_pdl(tc_gemm_q4_kernel, dim3(row_tiles, (n_tokens + bn - 1) / bn), kQ4Threads, kQ4Smem, s, mx, a);
+  Q4Args a{static_cast<const unsigned char*>(w), y, scratch, n_rows, k, n_tokens, bn, std::min(8, kQ4BBytes / (bn * 128)), (n_tokens + bn - 1) / bn, status_word()};
+  // SMs that the tiles leave idle, by whole columns of row tiles, write the scratch, unless that takes longer than the
+  // tiles do with their shares: us per block and row tile, 3.2 / spare against 1.3 + 2 / tiles (measured).
+  int spare = std::max(0, std::min(k / kQK, sms / row_tiles - a.tiles));
+  if (32 * a.tiles >= spare * (13 * a.tiles + 20)) spare = 0;
+  return launch_pdl(tc_gemm_q4_kernel, dim3(row_tiles, a.tiles + spare), kQ4Threads, kQ4Smem, s, mx, a);
 }
 
 }  // namespace

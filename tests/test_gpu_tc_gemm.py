@@ -155,9 +155,10 @@ def test_q4k_gemm_and_router(layout):
 
 
 @pytest.mark.parametrize("rows,k,tok", [(128, 256, 1), (100, 256, 17), (129, 512, 65), (1000, 2048, 129), (4096, 512, 300),
-                                        (333, 1024, 256), (4096, 2048, 1500)])
+                                        (333, 1024, 256), (4096, 2048, 1500), (4096, 512, 75), (1000, 512, 1024)])
 def test_q4k_gemm_tile_edges(rows, k, tok):
-    """Ragged row and token tiles, odd row counts (no paired stores), the three token tile sizes."""
+    """Ragged row and token tiles, odd row counts (no paired stores), the three token tile sizes, the scratch written by
+    the tiles and by CTAs of their own."""
     w_np, w_dev = make_q4k(rows, k, 13)
     x_np, x_dev = make_x16(tok, k, 14)
     scratch = torch.zeros(rows * k + 8, dtype=torch.float16, device=DEV)
