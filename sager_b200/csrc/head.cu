@@ -31,8 +31,7 @@ constexpr int kQ6 = 210;                     // bytes per Q6_K super-block
 constexpr int kHeadWarps = 8;
 constexpr int kHeadRows = 4;                  // rows a warp works on at once
 constexpr int kHeadThreads = kHeadWarps * 32 + 32;
-constexpr int kHeadStages = 4;
-constexpr int kHeadStageBytes = 54 * 1024;   // whole rows, at most this many bytes per stage (and at most 32 rows)
+constexpr int kHeadStages = 4;                // at most
 
 struct HeadArgs {
   const unsigned char* w;
@@ -46,6 +45,8 @@ struct HeadArgs {
 // staged activations: codes [nb][256] int8, 16-column sums [nb][16] int32, scales [nb] fp32
 __host__ __device__ inline size_t head_x_bytes(int nb) { return static_cast<size_t>(nb) * (256 + 64 + 4); }
 
+// G lanes to a row: 32, or 16 for rows of up to four blocks; S stages
+template <int G, int S>
 __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const HeadArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -54,14 +55,14 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
   const int nb = a.nb;
   const int row_bytes = nb * kQ6;
   const int stage_bytes = (a.rows_per_stage * row_bytes + 127) & ~127;
-  int8_t* xs = reinterpret_cast<int8_t*>(ring + static_cast<size_t>(kHeadStages) * stage_bytes);
+  int8_t* xs = reinterpret_cast<int8_t*>(ring + static_cast<size_t>(S) * stage_bytes);
   int* xsum = reinterpret_cast<int*>(xs + static_cast<size_t>(nb) * 256);
   float* xd = reinterpret_cast<float*>(xsum + nb * 16);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_stages = (a.n_rows + a.rows_per_stage - 1) / a.rows_per_stage;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kHeadStages; ++i) {
+    for (int i = 0; i < S; ++i) {
       mbar_init(full + i, 1);
       mbar_init(empty + i, kHeadWarps);
     }
@@ -75,8 +76,8 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
     if (lane == 0) {
       int it = 0;
       for (int st = blockIdx.x; st < n_stages; st += gridDim.x, ++it) {
-        const int s = it % kHeadStages;
-        if (it >= kHeadStages && !mbar_wait(empty + s, ((it / kHeadStages) - 1) & 1)) {
+        const int s = it % S;
+        if (it >= S && !mbar_wait(empty + s, ((it / S) - 1) & 1)) {
           ok = false;
           break;
         }
@@ -117,8 +118,8 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
     // as five aligned words each and realigned with a funnel shift (by 0 or 16 bits).
     int it = 0;
     for (int st = blockIdx.x; st < n_stages && ok; st += gridDim.x, ++it) {
-      const int s = it % kHeadStages;
-      ok = mbar_wait(full + s, (it / kHeadStages) & 1);
+      const int s = it % S;
+      ok = mbar_wait(full + s, (it / S) & 1);
       if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
       const int r0 = st * a.rows_per_stage;
       const int nr = min(a.rows_per_stage, a.n_rows - r0);
@@ -126,15 +127,15 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
       // four rows of the stage per warp and pass (rows warp, warp + 8, ...): their loads are in flight
       // together, the activation words are fetched once for the four, and one transposing reduction
       // (six shuffles) replaces four of five
-      for (int rb = warp; rb < nr; rb += kHeadWarps * kHeadRows) {
+      for (int rb = warp; rb < nr; rb += kHeadWarps * kHeadRows * (32 / G)) {
         const unsigned char* roww[kHeadRows];
 #pragma unroll
         for (int i = 0; i < kHeadRows; ++i)
-          roww[i] = stage + static_cast<size_t>(min(rb + i * kHeadWarps, nr - 1)) * row_bytes;
+          roww[i] = stage + static_cast<size_t>(min(rb + (i * (32 / G) + lane / G) * kHeadWarps, nr - 1)) * row_bytes;
         float acc[kHeadRows];
 #pragma unroll
         for (int i = 0; i < kHeadRows; ++i) acc[i] = 0.f;
-        for (int u = lane; u < nb * 4; u += 32) {
+        for (int u = lane % G; u < nb * 4; u += G) {
           const int blk = u >> 2, n_half = (u >> 1) & 1, is = u & 1;
           const int off0 = blk * kQ6 + n_half * 64 + is * 16, offh = blk * kQ6 + 128 + n_half * 32 + is * 16;
           const int8_t* xcol = xs + blk * 256 + n_half * 128 + is * 16;
@@ -181,18 +182,17 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
           }
         }
         static_assert(kHeadRows == 4, "the reduction below transposes four rows");
-        // lanes 0-15 take rows 0 and 1, lanes 16-31 rows 2 and 3; then lanes with bit 3 clear the first of the two
-        const bool hi16 = (lane & 16) != 0, hi8 = (lane & 8) != 0;
-        float s0 = hi16 ? acc[2] : acc[0], s1 = hi16 ? acc[3] : acc[1];
-        s0 += __shfl_xor_sync(0xFFFFFFFFu, hi16 ? acc[0] : acc[2], 16);
-        s1 += __shfl_xor_sync(0xFFFFFFFFu, hi16 ? acc[1] : acc[3], 16);
-        float t = hi8 ? s1 : s0;
-        t += __shfl_xor_sync(0xFFFFFFFFu, hi8 ? s0 : s1, 8);
-        t += __shfl_xor_sync(0xFFFFFFFFu, t, 4);
-        t += __shfl_xor_sync(0xFFFFFFFFu, t, 2);
-        t += __shfl_xor_sync(0xFFFFFFFFu, t, 1);
-        const int row = rb + (lane >> 3) * kHeadWarps;          // lanes 8i .. 8i+7 hold row i of the pass
-        if ((lane & 7) == 0 && row < nr) a.y[r0 + row] = t;
+        // of a row's G lanes the lower half takes rows 0 and 1, the upper 2 and 3; then the lower quarter the first of the two
+        const bool hi2 = (lane & (G / 2)) != 0, hi1 = (lane & (G / 4)) != 0;
+        float s0 = hi2 ? acc[2] : acc[0], s1 = hi2 ? acc[3] : acc[1];
+        s0 += __shfl_xor_sync(0xFFFFFFFFu, hi2 ? acc[0] : acc[2], G / 2);
+        s1 += __shfl_xor_sync(0xFFFFFFFFu, hi2 ? acc[1] : acc[3], G / 2);
+        float t = hi1 ? s1 : s0;
+        t += __shfl_xor_sync(0xFFFFFFFFu, hi1 ? s0 : s1, G / 4);
+#pragma unroll
+        for (int off = G / 8; off > 0; off >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, off);
+        const int row = rb + (((lane % G) / (G / 4)) * (32 / G) + lane / G) * kHeadWarps;
+        if (lane % (G / 4) == 0 && row < nr) a.y[r0 + row] = t;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive_one(empty + s);
@@ -266,18 +266,26 @@ int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStre
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
     return kErrLaunch;
-  // bulk copies need 16-byte aligned sources of 16-byte multiples: whole rows when the row is one
-  const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && row_bytes % 16 == 0 &&
-                          row_bytes <= kHeadStageBytes && n_rows >= 4 * sms;
+  // A stage is what a pass of the eight warps takes - 32 rows, or 64 of up to four blocks, which two half-warps share (k =
+  // 1024: a lane in two had nothing to do) - as long as two fit; half a pass costs as much as a whole one (k = 4096 with
+  // 54 KB stages, 248,320 rows: 261 us with norm and top-k, now 150; k = 1024, by the plain kernel before: 194, now 63). Bulk copies need 16-byte multiples: all stages are, and the last one has to be.
+  const bool narrow = a.nb <= 4;
+  const size_t fixed = 128 + head_x_bytes(a.nb), room = fixed < 227 * 1024 ? 227 * 1024 - fixed : 0;
+  a.rows_per_stage = kHeadWarps * kHeadRows * (narrow ? 2 : 1);
+  const int fit = static_cast<int>((room / 2 < 128 ? 0 : room / 2 - 127) / row_bytes);
+  if (fit < a.rows_per_stage) a.rows_per_stage = fit >= 8 ? fit & ~7 : fit;
+  const size_t stage_bytes = (static_cast<size_t>(a.rows_per_stage) * row_bytes + 127) & ~size_t(127);
+  const int stages = a.rows_per_stage > 0 ? static_cast<int>(std::min<size_t>(kHeadStages, room / stage_bytes)) : 0;
+  const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && stages >= 2 && n_rows >= 4 * sms &&
+                          static_cast<long long>(a.rows_per_stage) * row_bytes % 16 == 0 &&
+                          static_cast<long long>(n_rows % a.rows_per_stage) * row_bytes % 16 == 0;
   if (!streamable) return launch_head(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);
-  a.rows_per_stage = std::min(kHeadWarps * kHeadRows, kHeadStageBytes / row_bytes);
-  const int stage_bytes = (a.rows_per_stage * row_bytes + 127) & ~127;
-  const size_t smem = 128 + static_cast<size_t>(kHeadStages) * stage_bytes + head_x_bytes(a.nb);
-  if (smem > 227 * 1024) return launch_head(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);
-  if (cudaFuncSetAttribute(gemv_q6_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) !=
-      cudaSuccess)
+  const size_t smem = fixed + stages * stage_bytes;
+  auto kern = narrow ? gemv_q6_stream_kernel<16, 4>
+                     : (stages == 4 ? gemv_q6_stream_kernel<32, 4> : (stages == 3 ? gemv_q6_stream_kernel<32, 3> : gemv_q6_stream_kernel<32, 2>));
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
     return kErrLaunch;
-  return launch_head(gemv_q6_stream_kernel, dim3(sms), kHeadThreads, smem, stream, a);
+  return launch_head(kern, dim3(sms), kHeadThreads, smem, stream, a);
 }
 
 // ---- two-phase top-k ---------------------------------------------------------------------
