@@ -305,9 +305,11 @@ int launch_stream(const GemvArgs& a, int sms, cudaStream_t stream) {
   return launch_pdl(gemv_stream_kernel<TT, F16>, dim3(sms), kStreamThreads, smem, stream, a);
 }
 
-// The persistent kernel pays off when every SM gets several stages.
+// The persistent kernel pays off when every SM gets several stages and its dp4a dots keep up: one token row, and two of
+// more than eight blocks (248,320 rows of 16 blocks, with norm and top-k: 176 us against 195 by the MMA kernel below; of
+// eight blocks 103 against 99; four rows 288 against 231 and 169 against 125).
 inline int stream_sms(const GemvArgs& a) {
-  if (a.n_tokens > 4 || a.nb > 16 || (a.nb & (a.nb - 1)) != 0) return 0;
+  if (a.n_tokens > 2 || (a.n_tokens == 2 && a.nb <= 8) || a.nb > 16 || (a.nb & (a.nb - 1)) != 0) return 0;
   if (reinterpret_cast<uintptr_t>(a.w[0]) & 15u) return 0;
   const int sms = device_sms();
   if (sms <= 0) return 0;
@@ -581,8 +583,7 @@ int launch_dense(const void* w0, const void* w1, const void* xq, void* y0, void*
   if constexpr (NMAT == 1) {
     if (const int sms = stream_sms(a)) {
       if (n_tokens == 1) return launch_stream<1, F16>(a, sms, stream);
-      if (n_tokens == 2) return launch_stream<2, F16>(a, sms, stream);
-      return launch_stream<4, F16>(a, sms, stream);
+      return launch_stream<2, F16>(a, sms, stream);
     }
   }
   {
