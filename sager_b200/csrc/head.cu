@@ -43,7 +43,7 @@ struct HeadArgs {
 };
 
 // staged activations: codes [nb][256] int8, 16-column sums [nb][16] int32, scales [nb] fp32
-__host__ __device__ inline size_t head_x_bytes(int nb) { return static_cast<size_t>(nb) * (256 + 64 + 4); }
+__host__ __device__ constexpr size_t head_x_bytes(int nb) { return static_cast<size_t>(nb) * (256 + 64 + 4); }
 
 // G lanes to a row: 32, or 16 for rows of up to four blocks; S stages
 template <int G, int S>
@@ -281,6 +281,8 @@ int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStre
                           static_cast<long long>(n_rows % a.rows_per_stage) * row_bytes % 16 == 0;
   if (!streamable) return launch_head(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);
   const size_t smem = fixed + stages * stage_bytes;
+  static_assert(kHeadStages == 4 && 128 + head_x_bytes(4) + 4 * ((kHeadWarps * kHeadRows * 2 * 4 * kQ6 + 127) / 128 * 128) <= 227 * 1024,
+                "four stages of narrow rows fit, and so do those of fewer blocks");
   auto kern = narrow ? gemv_q6_stream_kernel<16, 4>
                      : (stages == 4 ? gemv_q6_stream_kernel<32, 4> : (stages == 3 ? gemv_q6_stream_kernel<32, 3> : gemv_q6_stream_kernel<32, 2>));
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
