@@ -50,12 +50,14 @@ constexpr int kMaxGrid = 160;            // most CTAs the expert kernels are lau
 #define AH 3
 #endif
 constexpr int kTmapSlots = AH + 7;           // patched TMA descriptor pairs per CTA of the row-streaming kernel
-constexpr int kTokenKernelMaxRows = 4;   // layers of up to this many token rows run as one persistent launch: all that its
-                                         // row sets hold (us per layer at 1 / 2 / 3 / 4 rows, 256 experts, hidden 2048,
-                                         // n_ff 512: 18.4 / 27.1 / 36.2 / 46.2, route + expert kernel 47.3 at 4; 128
-                                         // experts, hidden 1024: 34.5 against 36.7 at 4)
-constexpr int kRowsKernelMinRows = 4;    // layers of at least this many token rows run the row-streaming kernel
-                                         // (measured: 4 rows 8 % faster, 8 rows 16 %, 2 rows slower)
+// Layers of up to this many token rows run as one persistent launch: all that its row sets hold (us per layer at 1 / 2 /
+// 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 15.7 / 22.1 / 29.7 / 36.4, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
+// 128 experts, hidden 1024: 13.6 / 17.9 / 20.3 / 22.6 against 23.6 / 25.7 / 31.3 / 29.6).
+constexpr int kTokenKernelMaxRows = 4;
+// Layers of at least this many token rows have the row-streaming kernel's order of the sums (block after block), and of the
+// two expert kernels run that one (us per layer with the route kernel, 256 experts: 37.7 against 46.5 for the item kernel at
+// 4 rows, 50.3 against 66.7 at 8; at 1 row 29.4 against 26.9).
+constexpr int kRowsKernelMinRows = 4;
 constexpr int kRouteTok = 8;       // token rows per CTA of the route kernel
 constexpr int kRouteWarps = 16;    // warps of a route CTA: all stage, eight do the logits and eight quantise, pairs select
 constexpr int kRouteMaxRows = 16;  // most experts per route CTA
@@ -1438,13 +1440,15 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
   // A few token rows, whole layer on this device, all stages in one call: the single
   // persistent launch (token_layer.cuh). Bit 6 of `stages` keeps the two-launch path.
   if ((stages & 7) == 7 && !(stages & (8 | 16 | 32 | 64)) && a->n <= kTokenKernelMaxRows && a->n * a->n_used <= 32 &&
+      (a->n < kRowsKernelMinRows || use_rows) &&      // (a workspace for the item kernel: that kernel's order of the sums)
       !a->routing_given && a->xq_in == nullptr && a->xq_out == nullptr && a->wait_flags == nullptr &&
       a->ep_dst == nullptr && a->ep_out == nullptr &&
       L.e_lo == 0 && L.e_hi == L.E && L.sh_lo == 0 && L.sh_hi == L.n && L.nbh <= 16 && L.nbf <= 16 &&
       a->workspace_bytes >= lay.items_total) {
     const tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid);
     if (g.total <= 227 * 1024 && g.down_tiles > 0 && g.rows_per_cta <= tk::kGroupWarps)
-      return launch_layer<tk::token_layer_kernel>(dim3(L.grid), tk::kThreads, g.total, s, L);
+      return a->n < kRowsKernelMinRows ? launch_layer<tk::token_layer_kernel<false>>(dim3(L.grid), tk::kThreads, g.total, s, L)
+                                       : launch_layer<tk::token_layer_kernel<true>>(dim3(L.grid), tk::kThreads, g.total, s, L);
   }
 
   int rc = kOk;

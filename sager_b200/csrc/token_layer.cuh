@@ -26,11 +26,11 @@
 //            all of a row's expert contributions are then in this CTA - adds
 //            residual + sum_k w_k * y_k + shared in place. No third barrier.
 //
-// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 15.9 us per
+// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 15.7 us per
 // layer, of which 3.5 to the first barrier, 2 for picks and tables, 1.5 for the first bytes, 2 for
 // gate / up, 2 for the second barrier, 1 + 1 for h and the down rows; 26.6 with eight warps on whole
-// blocks and the selection in sequence), from two rows on the integer pipe and shared memory: 7 us
-// for every further row (23.0 / 30.1 / 36.6 us; 36.3 / 45.2 / 47.3 before).
+// blocks and the selection in sequence). A further row costs 7 us - 22.1 / 29.7 / 36.4 us at 2 / 3 / 4 rows -,
+// where its bytes cost 2.2.
 //
 // Work split: gate / up by pairs (a flat range of (tile, pair) per CTA), down by output
 // rows. Contracts are those of the two-launch path: null table entry = absent expert
@@ -255,9 +255,12 @@ __device__ __forceinline__ void load_half(HalfW<NMAT>& W, const unsigned char* c
 // the sum it does not keep and both finish one matrix, which halves the shuffles and the arithmetic after them. Whole
 // warps call it: `rows` is the warp's largest row count. Not unrolled over rows: every phase of this kernel runs once
 // per CTA, so straight-line code is paid for in instruction fetch.
-template <int NMAT>
-__device__ __forceinline__ void half_dots(const HalfW<NMAT>& W, int half, const HTile& xt, int blk, const RowSet& rs, int rows,
-                                          float (&out)[kMaxTok]) {
+// `out`: this lane's block terms. CHAIN: the sums over the row's `nb` blocks instead, valid in the lanes of the last
+// block (lr == nb - 1, `lr` this lane's position in the row), added block after block - the order of the row-streaming
+// kernel's consumers, so that layers of four rows and more have the same bits whichever kernel runs them.
+template <int NMAT, bool CHAIN>
+__device__ __forceinline__ void half_dots(const HalfW<NMAT>& W, int half, const HTile& xt, int blk, int lr, int nb, const RowSet& rs,
+                                          int rows, float (&out)[kMaxTok]) {
 #pragma unroll
   for (int t = 0; t < kMaxTok; ++t) out[t] = 0.f;
 #pragma unroll 1
@@ -291,14 +294,25 @@ __device__ __forceinline__ void half_dots(const HalfW<NMAT>& W, int half, const 
     const int other_is = NMAT == 1 || !half ? is[NMAT - 1] : is[0], other_ms = NMAT == 1 || !half ? ms[NMAT - 1] : ms[0];
     const int my_is = (half ? is[NMAT - 1] : is[0]) + __shfl_xor_sync(0xFFFFFFFFu, other_is, 1);
     const int my_ms = (half ? ms[NMAT - 1] : ms[0]) + __shfl_xor_sync(0xFFFFFFFFu, other_ms, 1);
-    const float v = __uint_as_float(sd.z) * (W.d * static_cast<float>(my_is) - W.dmin * static_cast<float>(my_ms));
+    float v = W.d * static_cast<float>(my_is) - W.dmin * static_cast<float>(my_ms);
+    if constexpr (CHAIN) {
+      const float term = v;
+      v = fmaf(__uint_as_float(sd.z), term, 0.f);
+#pragma unroll 1
+      for (int b = 1; b < nb; ++b) {
+        const float before = __shfl_up_sync(0xFFFFFFFFu, v, 2);
+        if (lr == b) v = fmaf(__uint_as_float(sd.z), term, before);
+      }
+    } else {
+      v = __uint_as_float(sd.z) * v;
+    }
     if (t == 0) out[0] = v;
     else if (t == 1) out[1] = v;
     else if (t == 2) out[2] = v;
     else out[3] = v;
   }
 }
-// sum over the blocks of a row, held by lane pairs `2 * lpr` lanes wide, in the order of reduce_lanes
+// Sum over the blocks of a row, held by lane pairs `2 * lpr` lanes wide, in the order of reduce_lanes, at block 0's lanes.
 __device__ __forceinline__ float reduce_pairs(float v, int lpr) {
   for (int off = lpr >> 1; off > 0; off >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, 2 * off);
   return v;
@@ -309,6 +323,7 @@ __device__ __forceinline__ float reduce_pairs(float v, int lpr) {
 // (Inlined at both of its uses: as a function it saved and restored 2,400 warp registers per CTA through local memory.)
 // A warp arrives at `empty` (if given) as soon as its weight bytes are in registers: the stage's refill, a DRAM round
 // trip, then runs under the arithmetic. Warps without a pair only arrive.
+template <bool CHAIN>
 __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, int mask, int hrow0, int pair0,
                                            const HTile& xt, float* hbuf, int FF, int nbh, int rb_h, int row_lanes, uint64_t* empty) {
   const int tid = threadIdx.x & (kGroupThreads - 1), lane = tid & 31;
@@ -332,13 +347,13 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
       if (lane == 0) mbar_arrive_one(empty);
     }
     float v[kMaxTok];
-    half_dots<2>(W, half, xt, blk, rs, rs.n, v);
+    half_dots<2, CHAIN>(W, half, xt, blk, lr, nbh, rs, rs.n, v);
+    const int at = CHAIN ? nbh - 1 : 0;
 #pragma unroll
     for (int t = 0; t < kMaxTok; ++t) {
       if (t >= rs.n) break;                        // uniform
-      const float g = reduce_pairs(lr < nbh ? v[t] : 0.f, lpr);
-      const float u = __shfl_down_sync(0xFFFFFFFFu, g, 1);          // the odd lanes hold the up row
-      if (q < tasks && half == 0 && lr == 0) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(g, u);
+      const float g = CHAIN ? v[t] : reduce_pairs(lr < nbh ? v[t] : 0.f, lpr), u = __shfl_down_sync(0xFFFFFFFFu, g, 1);          // the odd lanes hold the up row
+      if (q < tasks && half == 0 && lr == at) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(g, u);
     }
   }
 }
@@ -348,6 +363,8 @@ __device__ __forceinline__ void copy_plain(unsigned char* dst, const unsigned ch
   for (int p = lane; p < bytes / 16; p += 32) rs::copy16_any(dst + p * 16, src + static_cast<size_t>(p) * 16);
 }
 
+// CHAIN: layers of four token rows (see half_dots)
+template <bool CHAIN>
 __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
   const Geom G = geom(L.n, L.K, L.H, L.FF, L.E, gridDim.x);
@@ -651,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     if (warp >= kGroupWarps && has_shared && sp1 > sp0) {
       if (!mbar_wait(sh_full, 0)) ok = false;
       if (__all_sync(0xFFFFFFFFu, ok))
-        gate_up_stage(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, nullptr);
+        gate_up_stage<CHAIN>(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, nullptr);
     }
   }
 
@@ -797,7 +814,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       if (!ok) break;
       const StageDesc d = desc[s];
       if (d.mode != 1)
-        gate_up_stage(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
+        gate_up_stage<CHAIN>(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
                       d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, &empty[s]);
       else if (lane == 0) mbar_arrive_one(&empty[s]);
     }
@@ -849,12 +866,13 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         }
       }
       float v[kMaxTok];
-      half_dots<1>(W, f_half, hq, f_blk, rs, rows, v);
+      half_dots<1, CHAIN>(W, f_half, hq, f_blk, f_lr, L.nbf, rs, rows, v);
+      const int at = CHAIN ? L.nbf - 1 : 0;
 #pragma unroll
       for (int t = 0; t < kMaxTok; ++t) {
         if (t >= rows) break;                    // warp-uniform
-        const float y = reduce_pairs(f_lr < L.nbf ? v[t] : 0.f, lpf);
-        if (live && f_half == 0 && f_lr == 0 && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
+        const float y = CHAIN ? v[t] : reduce_pairs(f_lr < L.nbf ? v[t] : 0.f, lpf);
+        if (live && f_half == 0 && f_lr == at && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
       }
       base += kConsumers;
     } while (base < tasks && ok);

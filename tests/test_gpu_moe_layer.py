@@ -501,6 +501,38 @@ def test_token_kernel_edges(hidden, n_ff, E, k, n, ties):
         assert (first < E // 2).all() and (r0.route_idx[:n, 1].cpu().numpy() == first + E // 2).all()
 
 
+@pytest.mark.parametrize("hidden,n_ff,E,k", [
+    (2048, 512, 256, 8), (1024, 512, 128, 8), (2048, 256, 64, 8), (512, 256, 16, 4),      # 8, 4 and 2 block columns, down rows of 2 and 1
+    (256, 256, 5, 4), (768, 768, 12, 3), (1280, 1024, 48, 8), (4096, 256, 20, 2),          # 1, 3, 5 and 16; 3 and 4
+])
+def test_four_rows_have_the_bits_of_the_row_streaming_kernel(hidden, n_ff, E, k):
+    """From four rows on a layer's sums run block after block, whichever kernel takes it: no bit changes when a batch of four
+    moves between the one-launch and the two-launch path. Hot experts (tiles of several rows), null experts, no shared one."""
+    w = synth.MoeWeights(hidden, n_ff, E, DEV, seed=87, std=0.05)
+    for i, (absent, use_shared) in enumerate((((), True), ((0, E - 1), True), ((), False))):
+        x16 = synth.normal_fp16((4, hidden), 860 + i, DEV)
+        x16[1:3] = x16[0] + 0.05 * x16[1:3]               # three rows that pick much the same experts
+        r0, x0, o0 = run_layer(w, 4, k, x16, absent=absent, use_shared=use_shared)
+        r1, x1, o1 = run_layer(w, 4, k, x16, absent=absent, use_shared=use_shared, kernel="two_launch")
+        assert torch.equal(r0.route_idx, r1.route_idx) and torch.equal(r0.route_w, r1.route_w)
+        assert torch.equal(o0.view(torch.int32), o1.view(torch.int32)) and torch.equal(x0.view(torch.int16), x1.view(torch.int16))
+
+
+def test_four_rows_on_a_workspace_for_the_item_kernel(full_w):
+    """A workspace too small for the row-streaming kernel keeps four rows on the item kernel and its order of the sums."""
+    x16 = synth.normal_fp16((4, full_w.hidden), 870, DEV)
+    outs = []
+    for kernel in (None, "items"):
+        runner = MoeLayerRunner(4, full_w.hidden, full_w.n_ff, full_w.n_expert, 8, DEV)
+        out = torch.zeros(4, full_w.hidden, dtype=torch.float32, device=DEV)
+        a = runner.args(4, x16, full_w.router, full_w.table(), full_w.shared_ptrs(), x_f16=x16.clone(), out_f32=out)
+        a.workspace_bytes -= 256                  # one alignment step short of the whole layout
+        runner.run(a, kernel=kernel)
+        torch.cuda.synchronize()
+        outs.append(out)
+    assert torch.equal(outs[0].view(torch.int32), outs[1].view(torch.int32))
+
+
 @pytest.mark.parametrize("E,k,n", [
     (10, 4, 9),        # two experts per route CTA, a token tile of one row
     (40, 8, 33),       # two per CTA, five tiles
