@@ -9,8 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <atomic>
-
+#include "opt_in.cuh"
 #include "sager_b200.h"   // the public prototypes: definitions must agree with them
 #include "sager_b200_diag.h"
 
@@ -26,17 +25,14 @@ int* status_word();
 // SMs of the current device (0: none can be had), asked of the runtime once per device.
 int device_sms();
 
-// Opts kernel K in to `bytes` of dynamic shared memory on the current device, once per device.
+// Opts kernel K in to `bytes` of dynamic shared memory on the current device; a call to the runtime only when it grows.
 template <auto K>
 bool opt_in_smem(int bytes) {
-  constexpr int kMaxDevices = 64;
-  static std::atomic<int> done[kMaxDevices];
+  static SmemGrant grant;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
-  if (done[dev].load(std::memory_order_relaxed) >= bytes) return true;
-  if (cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
-  done[dev].store(bytes, std::memory_order_relaxed);
-  return true;
+  return cudaGetDevice(&dev) == cudaSuccess && grant.ensure(dev, bytes, [](int n) {
+           return cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, n) == cudaSuccess;
+         });
 }
 
 // Launch that may start while the kernel before it in the stream drains (programmatic dependent launch);

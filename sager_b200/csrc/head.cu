@@ -235,19 +235,10 @@ __global__ void gemv_q6_direct_kernel(const HeadArgs a) {
   if (lane == 0) a.y[row] = acc;
 }
 
-template <typename Kern>
-int launch_head(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, const HeadArgs& a) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess ? kOk : kErrLaunch;
+template <int G, int S>
+int launch_stream(const HeadArgs& a, int sms, size_t smem, cudaStream_t stream) {
+  if (!opt_in_smem<gemv_q6_stream_kernel<G, S>>(static_cast<int>(smem))) return kErrLaunch;
+  return launch_pdl(gemv_q6_stream_kernel<G, S>, dim3(sms), kHeadThreads, smem, stream, a);
 }
 
 int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStream_t stream) {
@@ -279,15 +270,13 @@ int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStre
   const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && stages >= 2 && n_rows >= 4 * sms &&
                           static_cast<long long>(a.rows_per_stage) * row_bytes % 16 == 0 &&
                           static_cast<long long>(n_rows % a.rows_per_stage) * row_bytes % 16 == 0;
-  if (!streamable) return launch_head(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);
+  if (!streamable) return launch_pdl(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);
   const size_t smem = fixed + stages * stage_bytes;
   static_assert(kHeadStages == 4 && 128 + head_x_bytes(4) + 4 * ((kHeadWarps * kHeadRows * 2 * 4 * kQ6 + 127) / 128 * 128) <= 227 * 1024,
                 "four stages of narrow rows fit, and so do those of fewer blocks");
-  auto kern = narrow ? gemv_q6_stream_kernel<16, 4>
-                     : (stages == 4 ? gemv_q6_stream_kernel<32, 4> : (stages == 3 ? gemv_q6_stream_kernel<32, 3> : gemv_q6_stream_kernel<32, 2>));
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess)
-    return kErrLaunch;
-  return launch_head(kern, dim3(sms), kHeadThreads, smem, stream, a);
+  if (narrow) return launch_stream<16, 4>(a, sms, smem, stream);
+  if (stages == 4) return launch_stream<32, 4>(a, sms, smem, stream);
+  return stages == 3 ? launch_stream<32, 3>(a, sms, smem, stream) : launch_stream<32, 2>(a, sms, smem, stream);
 }
 
 // ---- two-phase top-k ---------------------------------------------------------------------

@@ -1,4 +1,6 @@
 // status.cu - the library's device status word and version query.
+#include <atomic>
+
 #include "api_util.cuh"
 #include "q4k_common.cuh"
 
