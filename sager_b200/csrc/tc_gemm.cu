@@ -609,7 +609,7 @@ int launch_dequant(const void* w, void* out16, long long n_blocks, cudaStream_t 
 }
 
 int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratch, int n_rows, int k, int n_tokens, cudaStream_t s) {
-  if (reinterpret_cast<uintptr_t>(x) & 15u) return kErrAlign;
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(y) & 1u)) return kErrAlign;
   const int sms = device_sms(), row_tiles = (n_rows + 127) / 128;
   if (sms <= 0) return kErrLaunch;
   // Token rows per CTA: the fewest estimated cycles - waves of CTAs, each its blocks at the MMAs' rate (130 cycles

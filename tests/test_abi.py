@@ -33,6 +33,7 @@ def test_argument_validation_needs_no_gpu():
     assert lib.raw("sgr_tc_gemm_f16_raw")(16, 16, 16, 8, 100, 4, None) == 3          # k % 64 != 0
     assert lib.raw("sgr_tc_gemm_f16_raw")(18, 16, 16, 8, 64, 4, None) == 2           # operand not 16-byte aligned
     assert lib.raw("sgr_tc_gemm_q4_k_f16")(16, 16, 16, 16, 8, 768, 4, None) == 3     # k not a power of two
+    assert lib.raw("sgr_tc_gemm_q4_k_f16")(16, 16, 17, 16, 8, 512, 4, None) == 2     # output not 2-byte aligned
     assert lib.raw("sgr_tc_scratch_elems")(512, 2048) == 512 * 2048
 
 
