@@ -157,6 +157,11 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
   const int tok_per = a->tok_per > 0 ? a->tok_per : 16;
   const long long R = static_cast<long long>(a->n_max) * K;
   if (R > 0x7FFFFFFF / (F / kQK)) return kErrUnsupported;
+  // as the launchers of the sequence refuse them
+  auto off_by = [](const void* p, unsigned mask) { return (reinterpret_cast<uintptr_t>(p) & mask) != 0; };
+  if (off_by(a->xn, 1) || off_by(a->xq, 3) || off_by(a->xqg, 15) || off_by(a->hq, 15) || off_by(a->g, 1) ||
+      (shared && (off_by(a->sh_g, 1) || off_by(a->sh_q, 3))))
+    return kErrAlign;
   int rc;
 #define SGR_STEP(call) do { rc = (call); if (rc != kOk) return rc; } while (0)
   const OperandRows op = operand_rows(a);

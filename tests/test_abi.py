@@ -1,5 +1,6 @@
 """CPU checks of the C boundary: the library builds for sm_100a, loads without a
 GPU and exports every symbol the header declares; the shim header compiles."""
+import ctypes as C
 import os
 import subprocess
 
@@ -35,6 +36,26 @@ def test_argument_validation_needs_no_gpu():
     assert lib.raw("sgr_tc_gemm_q4_k_f16")(16, 16, 16, 16, 8, 768, 4, None) == 3     # k not a power of two
     assert lib.raw("sgr_tc_gemm_q4_k_f16")(16, 16, 17, 16, 8, 512, 4, None) == 2     # output not 2-byte aligned
     assert lib.raw("sgr_tc_scratch_elems")(512, 2048) == 512 * 2048
+
+
+def test_prefill_chunk_refuses_unaligned_buffers():
+    """What the launchers of the sequence refuse, the one call refuses, and before anything is launched."""
+    lib = capi.lib()
+
+    def call(**moved):
+        a = capi.MoePrefillArgs()
+        a.n, a.n_max, a.hidden, a.n_ff, a.n_expert, a.n_used = 4, 4, 512, 256, 8, 2
+        for name, kind in capi.MoePrefillArgs._fields_:
+            if kind is C.c_void_p:
+                setattr(a, name, 4096)
+        a.shared_gate_w = a.sgate = None
+        for name, by in moved.items():
+            setattr(a, name, 4096 + by if by is not None else None)
+        return lib.raw("sgr_moe_layer_prefill")(C.byref(a), None)
+
+    for name, by in (("xn", 1), ("xq", 2), ("xqg", 8), ("hq", 4), ("g", 1), ("sh_g", 1), ("sh_q", 2)):
+        assert call(**{name: by}) == 2, name
+    assert call(xn=None) == 1
 
 
 def test_shim_header_compiles_against_c_abi():
