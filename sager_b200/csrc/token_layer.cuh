@@ -152,9 +152,10 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // Grid-wide barrier on a 64-bit arrival counter that only ever grows: the k-th barrier of the
 // grid (over all launches on this workspace) completes when the counter reaches k * G. Waits are
 // bounded: false when the others did not arrive in time.
-// The counter is read by the producer warp at kernel start - some multiple of the grid size plus the
-// arrivals of CTAs that are already further on, none of which can have passed the first barrier - so
-// barrier k of this launch completes at base + k * grid. An arrival is a fire-and-forget releasing
+// The counter is read by the producer warp when the kernels before this one have finished - some multiple of
+// the grid size plus the arrivals of this launch's CTAs that are already further on, none of which can have passed
+// the first barrier - so barrier k of this launch completes at base + k * grid. (Read at kernel start, it could lie
+// between the barriers of a launch before on the same workspace, wherever two CTAs fit on one SM.) An arrival is a fire-and-forget releasing
 // add by the thread whose warp finishes the work; the producer warp polls and passes the word on
 // through an mbarrier, so no consumer waits for a round trip that it could work through.
 __device__ __forceinline__ unsigned long long grid_base(const unsigned long long* ctr, unsigned grid) {
@@ -461,6 +462,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         }
       }
     }
+    // (an earlier launch on this workspace may still be between its two barriers until now)
+    pdl_wait();
     unsigned long long bar_base = 0;
     if (lane == 0) {
       bar_base = grid_base(gctr, grid);
@@ -652,7 +655,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     }
     if (nlw > 1) named_sync(7, nlw * 32);
     if (tid == 0) {
-      mbar_wait(based, 0);                       // (set at kernel start)
+      mbar_wait(based, 0);                       // (set when the kernels before this one have finished)
       grid_arrive(gctr);
     }
   } else {

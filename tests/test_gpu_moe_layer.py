@@ -518,6 +518,32 @@ def test_four_rows_have_the_bits_of_the_row_streaming_kernel(hidden, n_ff, E, k)
         assert torch.equal(o0.view(torch.int32), o1.view(torch.int32)) and torch.equal(x0.view(torch.int16), x1.view(torch.int16))
 
 
+@pytest.mark.parametrize("hidden,n_ff,E,k", [(512, 256, 16, 4), (256, 256, 5, 4), (2048, 512, 32, 8)])
+def test_one_launch_layers_back_to_back_on_one_workspace(hidden, n_ff, E, k):
+    """The layers of a step share a workspace and its barrier counter, and each may start while the one before it drains:
+    the bits of the same layers with a device synchronisation between them."""
+    layers = [synth.MoeWeights(hidden, n_ff, E, DEV, seed=880 + i, std=0.05) for i in range(6)]
+    for n in (1, 2, 4):
+        x0 = synth.normal_fp16((n, hidden), 890 + n, DEV)
+        ins = [synth.normal_fp16((n, hidden), 891 + 10 * n + i, DEV) for i in range(6)]
+        st = MoeStack(layers, n, k, DEV, inputs=ins)
+        st.x.copy_(x0)
+        for li in range(6):
+            r, a = st.layer_args(li, n)
+            r.run(a)
+            torch.cuda.synchronize()
+        want, idx = st.x.clone(), st.idx.clone()
+        st.capture(n)
+        for _ in range(50):
+            st.x.copy_(x0)
+            st.replay()
+            st.x.copy_(x0)
+            st.step_eager(n)
+        torch.cuda.synchronize()
+        assert torch.equal(st.x.view(torch.int16), want.view(torch.int16)) and torch.equal(st.idx, idx)
+    assert lib().raw("sgr_status")(0) == 0
+
+
 def test_four_rows_on_a_workspace_for_the_item_kernel(full_w):
     """A workspace too small for the row-streaming kernel keeps four rows on the item kernel and its order of the sums."""
     x16 = synth.normal_fp16((4, full_w.hidden), 870, DEV)
