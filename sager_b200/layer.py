@@ -102,7 +102,6 @@ class MoeStack:
         self.idx = torch.zeros(len(layers), n_max, n_used + 1, dtype=torch.int32, device=device)
         self.w = torch.zeros(len(layers), n_max, n_used + 1, dtype=torch.float32, device=device)
         # one persistent launch per layer for up to four rows, else route + experts
-        self._args = {}
         self.launches_per_step = (1 if (kernel is None and n_max <= 4) else 2) * len(layers)
         # chain: layer l's input rows are RMSNorm(x) computed on the device by rmsnorm_quant_f16 (the
         # producer of the MoE half's rows in the reference's decode layer, src/core/session.cpp:1020-1032),
@@ -116,20 +115,12 @@ class MoeStack:
             self.launches_per_step += len(layers)
 
     def layer_args(self, li, n):
-        """The runner and the argument block of a layer. A step whose row count changes is issued call by call, so the
-        blocks are kept, one per (layer, row count), for as long as the addresses in them stay the same."""
         w = self.layers[li]
         r = self.runners[li % len(self.runners)]
         xn = self.xn if self.chain else self.x if self.inputs is None else self.inputs[li]
-        bias = None if self.biases is None else self.biases[li]
-        key = tuple([t.data_ptr() for t in (xn, self.x, self.tables[li], w.router, w.blob, self.idx, self.w, r.ws)] +
-                    [bias.data_ptr() if bias is not None else 0])
-        kept = self._args.get((li, n))
-        if kept is None or kept[0] != key:
-            kept = (key, r.args(n, xn, w.router, self.tables[li], w.shared_ptrs(), x_f16=self.x, bias=bias,
-                                route_idx=self.idx[li], route_w=self.w[li]))
-            self._args[(li, n)] = kept
-        return r, kept[1]
+        return r, r.args(n, xn, w.router, self.tables[li], w.shared_ptrs(), x_f16=self.x,
+                         bias=None if self.biases is None else self.biases[li],
+                         route_idx=self.idx[li], route_w=self.w[li])
 
     def _issue(self, n, stages=7):
         stream = stream_ptr()

@@ -193,6 +193,36 @@ def test_expert_ranges_partition_the_layer(full_w):
     assert rel(total.cpu().numpy(), out_full.cpu().numpy()) < 1e-6
 
 
+def test_stack_argument_blocks_belong_to_the_caller():
+    """A block from layer_args may be changed without touching the stack's own steps, follows what the weights object says
+    now, and asks no more of that object than its router, table and shared pointers."""
+    class Weights:
+        def __init__(self, w):
+            self.hidden, self.n_ff, self.n_expert, self.router, self.w, self.shared = w.hidden, w.n_ff, w.n_expert, w.router, w, True
+
+        def table(self):
+            return self.w.table()
+
+        def shared_ptrs(self):
+            return self.w.shared_ptrs() if self.shared else None
+
+    w = Weights(synth.MoeWeights(512, 256, 16, DEV, seed=230, std=0.05))
+    x0 = synth.normal_fp16((2, 512), 231, DEV)
+    st = MoeStack([w], 2, 4, DEV)
+
+    def step():
+        st.x.copy_(x0)
+        st.step_eager(2)
+        return st.x.clone()
+
+    first = step()
+    _, a = st.layer_args(0, 2)
+    a.no_residual, a.x_f16 = 1, None
+    assert torch.equal(step(), first)
+    w.shared = False
+    assert not torch.equal(step(), first)
+
+
 def test_stack_graph_replay_is_deterministic(oracle):
     layers = [synth.MoeWeights(512, 256, 16, DEV, seed=200 + i, std=0.05) for i in range(3)]
     n, k = 4, 4
