@@ -140,22 +140,6 @@ __device__ __forceinline__ void rs_consumers_sync() {
   asm volatile("bar.sync 5, %0;" ::"n"(kConsumers) : "memory");
 }
 
-// 16 bytes from a source that is only 2- or 4-byte aligned
-__device__ __forceinline__ void copy16_any(unsigned char* dst, const unsigned char* src) {
-  uint32_t v[4];
-  if ((reinterpret_cast<uintptr_t>(src) & 3u) == 0) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(src) + i);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint16_t* h = reinterpret_cast<const uint16_t*>(src) + 2 * i;
-      v[i] = static_cast<uint32_t>(__ldg(h)) | (static_cast<uint32_t>(__ldg(h + 1)) << 16);
-    }
-  }
-  *reinterpret_cast<uint4*>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
-}
-
 // Groups are handed out dynamically, in one global order: every gate/up group of the
 // layer (tile-major), then every down group. A CTA starts with group blockIdx.x and takes
 // further ones from a global counter; its weight warp draws the next number while it
@@ -654,11 +638,12 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
               b0 = ge->w[2] + static_cast<size_t>(row0) * rb_f + blk * kW4;
               b1 = b0 + static_cast<size_t>(kHalfRows) * rb_f;
             }
-            for (int p = lane; p < kHalfBytes / 16; p += 32) {
-              const int r = p / 9, c = (p - r * 9) * 16;
-              copy16_any(st + p * 16, b0 + static_cast<size_t>(r) * rb + c);
-              copy16_any(st + kHalfBytes + p * 16, b1 + static_cast<size_t>(r) * rb + c);
-            }
+            const uintptr_t align = reinterpret_cast<uintptr_t>(b0) | reinterpret_cast<uintptr_t>(b1);
+            copy_unaligned(st, 2 * kHalfBytes / 16, lane, align, [&](int p) {
+              const int r = p / 9, h = r / kHalfRows;
+              return (h ? b1 : b0) + static_cast<size_t>(r - h * kHalfRows) * rb + (p - r * 9) * 16;
+            });
+            asm volatile("cp.async.wait_all;" ::: "memory");
             fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
           }
           __syncwarp();                            // every lane's part of the stage (and of its descriptor) is written

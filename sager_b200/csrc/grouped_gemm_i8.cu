@@ -459,8 +459,10 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
           const unsigned char* base = m == 0 ? u.w0 : u.w1;
           const int row0 = (u.tile0 + t) * kGemmRows;
           const unsigned char* src = base + static_cast<size_t>(row0) * row_bytes + b * kW4;
-          const uint32_t dst = smem_u32(smem + kOffW + s * kStageBytes) + lane * 16;
-          if ((reinterpret_cast<uintptr_t>(base) & 15u) == 0 && row0 + kGemmRows <= a.n_rows) {
+          unsigned char* stage = smem + kOffW + s * kStageBytes;
+          const uintptr_t align = reinterpret_cast<uintptr_t>(base) & 15u;
+          if (align == 0 && row0 + kGemmRows <= a.n_rows) {
+            const uint32_t dst = smem_u32(stage) + lane * 16;
 #pragma unroll 1
             for (int g = 0; g < 4; ++g) {
 #pragma unroll
@@ -470,17 +472,16 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
             cp_async_arrive(&bar[kBarWFull + s]);
           } else {                                               // ragged last tile, or a base off a 16-byte boundary
             const int last = a.n_rows - 1 - row0;                // rows past the matrix repeat its last one: never stored
-            unsigned char* d = smem + kOffW + s * kStageBytes + lane * 16;
-#pragma unroll 1
-            for (int q = 0; q < kStageBytes / 512; ++q) {
-              const int pc = q * 32 + lane;
-              const uint16_t* x = reinterpret_cast<const uint16_t*>(src + min(pc / 9, last) * row_bytes + pc % 9 * 16);
-              uint32_t v[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i) v[i] = static_cast<uint32_t>(__ldg(x + 2 * i)) | (static_cast<uint32_t>(__ldg(x + 2 * i + 1)) << 16);
-              *reinterpret_cast<uint4*>(d + q * 512) = make_uint4(v[0], v[1], v[2], v[3]);
+            auto piece = [&](int p) { return src + min(p / 9, last) * row_bytes + p % 9 * 16; };
+            if (align == 0) {
+#pragma unroll 4
+              for (int q = lane; q < kStageBytes / 16; q += 32) cp_async16(smem_u32(stage) + q * 16, piece(q));
+              cp_async_arrive(&bar[kBarWFull + s]);
+            } else if (copy_unaligned(stage, kStageBytes / 16, lane, align, piece)) {
+              mbar_arrive_one(&bar[kBarWFull + s]);
+            } else {
+              cp_async_arrive(&bar[kBarWFull + s]);
             }
-            mbar_arrive_one(&bar[kBarWFull + s]);
           }
           return true;
         });

@@ -359,9 +359,13 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
   }
 }
 
-// Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned.
+// Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned; plain_done() ends a row of them.
 __device__ __forceinline__ void copy_plain(unsigned char* dst, const unsigned char* src, int bytes, int lane) {
-  for (int p = lane; p < bytes / 16; p += 32) rs::copy16_any(dst + p * 16, src + static_cast<size_t>(p) * 16);
+  copy_unaligned(dst, bytes / 16, lane, reinterpret_cast<uintptr_t>(src), [&](int p) { return src + static_cast<size_t>(p) * 16; });
+}
+__device__ __forceinline__ void plain_done() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  fence_proxy_async();
 }
 
 // CHAIN: layers of four token rows (see half_dots)
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         copy_plain(sh_stage, L.sh[0] + static_cast<size_t>(sp0) * G.rb_h, np * G.rb_h, lane);
         copy_plain(sh_stage + static_cast<size_t>(np) * G.rb_h, L.sh[1] + static_cast<size_t>(sp0) * G.rb_h, np * G.rb_h, lane);
         copy_plain(dn, L.sh[2] + static_cast<size_t>(r0) * G.rb_f, nr * G.rb_f, lane);
-        fence_proxy_async();
+        plain_done();
         __syncwarp();
         if (lane == 0) {
           mbar_arrive_one(sh_full);
@@ -509,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
           if (!(j == 0 && has_shared) && tb.tile_mode[j] == 2)
             copy_plain(to + static_cast<size_t>(j - j0) * G.slot_bytes, tb.w[2][j] + static_cast<size_t>(r0) * G.rb_f,
                        nr * G.rb_f, lane);
-        fence_proxy_async();
+        plain_done();
         __syncwarp();
       }
       if (lane == 0) {
@@ -546,7 +550,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       if (mode == 2) {
         copy_plain(st, tb.w[0][tile] + static_cast<size_t>(pair0) * G.rb_h, np * G.rb_h, lane);
         copy_plain(st + static_cast<size_t>(np) * G.rb_h, tb.w[1][tile] + static_cast<size_t>(pair0) * G.rb_h, np * G.rb_h, lane);
-        fence_proxy_async();
+        plain_done();
       }
       __syncwarp();
       if (lane == 0) {
