@@ -639,7 +639,10 @@ int launch_gemm(GemmArgs a, cudaStream_t stream) {
   a.tiles = (a.n_rows + kGemmRows - 1) / kGemmRows;
   // Rows of at most two blocks keep their activation tiles for a unit's row tiles: four tiles per unit
   // make the staging an eighth of the jobs' time and still leave about seven units per SM for 256 experts.
+  // With fewer units than SMs the other SMs would have nothing to do: then smaller units (8 experts of 2048 x 512 over 64 /
+  // 300 rows each: 10.8 / 26.7 us, with units of four tiles 17.8 / 62.5).
   a.group = !DUAL && a.nb <= 2 ? std::min(4, a.tiles) : 1;
+  while (a.group > 1 && static_cast<long long>((a.tiles + a.group - 1) / a.group) * a.n_expert < sms) a.group /= 2;
   a.groups = (a.tiles + a.group - 1) / a.group;
   if (a.sw0 != nullptr && a.s_rows > 0) {
     const int passes = (a.s_rows + kGemmTok - 1) / kGemmTok;

@@ -94,6 +94,26 @@ def test_many_ragged_units_in_one_cta(oracle, n_rows, k):
     assert f16_close(y.cpu().numpy(), y1.float().cpu().numpy())
 
 
+@pytest.mark.parametrize("E", [80, 60, 20])              # units of four row tiles (the last of one), of two, of one
+@pytest.mark.parametrize("k", [256, 512])
+def test_row_tiles_per_unit(E, k):
+    """Few experts take smaller units, so that every SM has one: 640 rows are five tiles."""
+    n_rows = 640
+    rng = np.random.default_rng(E)
+    counts = rng.integers(0, 100, E)
+    mats = [make_q4k(n_rows, k, 300 + e)[1] for e in range(3)]
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    R = int(off[-1])
+    xq = quantize_dev(make_x16(R, k, 7)[1])
+    y = torch.zeros(R, n_rows, dtype=torch.float16, device=DEV)
+    ops.moe_grouped_gemm_i8(ops.ptr_table([mats[e % 3] for e in range(E)], DEV), dev(off), xq, y, n_rows, k, E)
+    want = torch.zeros_like(y)
+    for e in range(E):
+        if counts[e]:
+            ops.mmq_q4_k_q8_f16out(mats[e % 3], xq[off[e]:off[e + 1]].contiguous(), want[off[e]:off[e + 1]], n_rows, k, int(counts[e]))
+    assert f16_close(y.cpu().numpy(), want.float().cpu().numpy())
+
+
 def test_weights_off_a_16_byte_boundary(oracle):
     """Pointer tables only promise the block struct's 2-byte alignment."""
     n_rows, k, counts = 256, 512, [5, 20]
