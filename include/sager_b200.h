@@ -314,7 +314,7 @@ int sgr_moe_layer_decode_stages(const sgr_moe_layer* args, int stages, void* str
  * expert and matrix) with the contract of gemv_grouped_tab_q4_k_q8_f16out_mtok (cuda_ops.hpp:247):
  * xq is the expert-major slab of Q8_K rows, off[n_expert+1] the row prefix of the device plan,
  * y[off[e]+t][r] = W_e[r] . xq[off[e]+t] in fp16; a null table entry gives zero rows. The integer
- * arithmetic is that of the Q4_K x Q8_K path (exact sub-block dots), not of the fp16 GEMM. */
+ * arithmetic is that of the Q4_K x Q8_K path (integer block sums, exact below 2^24), not of the fp16 GEMM. */
 int sgr_moe_grouped_gemm_i8(const void* const* w_tab, const int* off, const void* xq, uint16_t* y,
                             int n_rows, int k, int n_expert, void* stream);
 

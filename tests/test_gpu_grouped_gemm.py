@@ -1,4 +1,4 @@
-"""GPU parity of the tcgen05 int8 grouped GEMM (sgr_moe_grouped_gemm_i8) against the
+"""GPU parity of the tcgen05 grouped GEMM (sgr_moe_grouped_gemm_i8) against the
 oracle's Q4_K x Q8_K row dot and against the library's own device-plan grouped GEMV,
 which implements the reference's batched Q4_K path (q4_k.cu:765-836). Same integers
 on every path, so fp16 outputs agree to one fp16 step."""
@@ -92,6 +92,41 @@ def test_many_ragged_units_in_one_cta(oracle, n_rows, k):
     y1 = torch.zeros_like(y)                       # the same rows through the batched GEMV family
     ops.mmq_q4_k_q8_f16out(w_dev, xq, y1, n_rows, k, R)
     assert f16_close(y.cpu().numpy(), y1.float().cpu().numpy())
+
+
+def saturated_blocks(rows, nb, d, dmin):
+    """Q4_K rows with every code 15, every scale and min 63."""
+    w = np.zeros((rows, nb, 144), np.uint8)
+    w[..., 0:2], w[..., 2:4] = (np.frombuffer(np.float16(v).tobytes(), np.uint8) for v in (d, dmin))
+    w[..., 4:] = 0xFF
+    return w.reshape(rows, -1)
+
+
+@pytest.mark.parametrize("mins", [0, 14, 15])               # min term: none, all but a fifteenth cancels, everything cancels
+@pytest.mark.parametrize("nb,lo", [(1, 127), (1, 90), (2, 100), (8, 64)])
+def test_block_sums_past_2_to_the_24(nb, lo, mins):
+    """Codes near 127 against 15 x 63: block sums of 16 to 31 million, which the fp32 accumulator no longer holds exactly. Half of
+    the sixteen steps of a block can lie past 2^24, where one step rounds to a multiple of two: 16 units at most."""
+    rows, n, d = 128, 64, 2.0 ** -10
+    rng = np.random.default_rng(nb * 1000 + lo)
+    codes = rng.integers(lo, 128, (n, nb, 256))
+    codes[n // 2:] *= -1
+    xq = np.zeros((n, nb, 276), np.uint8)
+    xq[..., 0:4] = np.frombuffer(np.float32(1.0).tobytes(), np.uint8)
+    xq[..., 4:260] = codes.astype(np.int8).view(np.uint8)
+    sums = codes.reshape(n, nb, 8, 32).sum(3)
+    xq[..., 260:] = sums.astype(np.int16).view(np.uint8).reshape(n, nb, 16)
+    w = dev(saturated_blocks(rows, nb, d, mins * d))
+    x = dev(xq.reshape(n, -1))
+    y = torch.zeros(n, rows, dtype=torch.float16, device=DEV)
+    ops.moe_grouped_gemm_i8(ops.ptr_table([w], DEV), dev(np.int32([0, n])), x, y, rows, nb * 256, 1)
+    units = 63 * (15 - mins) * sums.reshape(n, -1).sum(1)    # exact result over d
+    got = y.double().cpu().numpy() / d
+    half_step = np.spacing(np.minimum(np.abs(units * d), 60000).astype(np.float16)).astype(np.float64) / d / 2
+    fp32 = nb * 2.0 ** -23 * 63 * 15 * 127 * 256             # roundings of the block terms and their sum
+    assert (np.abs(units * d) < 60000).all() or mins == 0
+    keep = np.abs(units * d) < 60000                         # (beyond that fp16 has no value)
+    assert (np.abs(got - units[:, None]) <= (16 * nb + fp32 + half_step)[:, None])[keep].all()
 
 
 @pytest.mark.parametrize("E", [80, 60, 20])              # units of four row tiles (the last of one), of two, of one
