@@ -473,11 +473,11 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
             }
             cp_async_arrive(&bar[kBarWFull + s]);
           } else {                                               // ragged last tile, or a base off a 16-byte boundary
-            const int last = a.n_rows - 1 - row0;                // rows past the matrix repeat its last one: never stored
+            const int last = a.n_rows - 1 - row0;                // rows past the matrix (never stored): zero, or its last one
             auto piece = [&](int p) { return src + min(p / 9, last) * row_bytes + p % 9 * 16; };
             if (align == 0) {
 #pragma unroll 4
-              for (int q = lane; q < kStageBytes / 16; q += 32) cp_async16(smem_u32(stage) + q * 16, piece(q));
+              for (int q = lane; q < kStageBytes / 16; q += 32) cp_async16_or_zero(smem_u32(stage) + q * 16, piece(q), q / 9 <= last);
               cp_async_arrive(&bar[kBarWFull + s]);
             } else if (copy_unaligned(stage, kStageBytes / 16, lane, align, piece)) {
               mbar_arrive_one(&bar[kBarWFull + s]);

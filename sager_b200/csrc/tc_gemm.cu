@@ -429,7 +429,8 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     }
   } else if (warp == 9) {
     // (the weights do not depend on the kernel before) 16-byte piece p = 9 * row + c goes to lane p % 32; nine steps
-    // of 32 pieces are 32 rows. Rows past the matrix repeat its last one: never stored.
+    // of 32 pieces are 32 rows. Rows past the matrix are zero: never stored. (Repeating its last row, hundreds of warps
+    // asked for the same lines: 32 rows over 2048 tokens of 2048 columns 32 us.)
     const int row_bytes = nb * kW4, last = a.n_rows - 1 - row0;
     for (int job = 0; job < nb; ++job) {
       const int st = job % kQ4WStages;
@@ -439,7 +440,7 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
 #pragma unroll 9
       for (int q = 0; q < 36; ++q) {
         const int piece = q * 32 + lane, row = piece / 9;
-        cp_async16(dst + q * 512, src + static_cast<size_t>(min(row, last)) * row_bytes + (piece - 9 * row) * 16);
+        cp_async16_or_zero(dst + q * 512, src + static_cast<size_t>(min(row, last)) * row_bytes + (piece - 9 * row) * 16, row <= last);
       }
       cp_async_arrive(&bar[kQ4WFull + st]);
     }

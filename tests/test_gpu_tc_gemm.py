@@ -173,6 +173,22 @@ def test_q4k_gemm_tile_edges(rows, k, tok):
     assert lib().raw("sgr_status")(0) == 0
 
 
+@pytest.mark.parametrize("rows", [1, 32, 127, 200])
+def test_q4k_gemm_few_rows_past_a_tile(rows):
+    """A last row tile of few rows under many token tiles: nothing of the rows past the matrix reaches the output."""
+    k, tok = 512, 2100
+    w_np, w_dev = make_q4k(rows, k, 23)
+    x_np, x_dev = make_x16(tok, k, 24)
+    scratch = torch.zeros(rows * k, dtype=torch.float16, device=DEV)
+    y = torch.full((tok + 1, rows), 9.0, dtype=torch.float16, device=DEV)
+    ops.tc_gemm_q4_k_f16(w_dev, x_dev, y, scratch, rows, k, tok)
+    w16 = torch.zeros(rows, k, dtype=torch.float16, device=DEV)
+    ops.dequant_q4_k_f16(w_dev, w16, rows, k)
+    assert torch.equal(scratch.view(torch.int16), w16.view(-1).view(torch.int16))
+    assert rel(y[:tok].float().cpu().numpy(), gemm_want(w16, x_dev).cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
+    # (fp32 accumulation in another order, one rounding to fp16)
+
+
 def test_refusals_launch_nothing():
     t = torch.zeros(4096, dtype=torch.float16, device=DEV)
     p = t.data_ptr()
