@@ -264,6 +264,7 @@ struct Q4Args {
   uint16_t *y, *scratch;
   int n_rows, k, n_tokens;
   int bn, stages, tiles;                          // token rows per CTA, activation stages, token tiles (grid.y beyond: scratch)
+  int tiles_write;                                // the token tiles write the scratch
   int* status;
 };
 
@@ -329,7 +330,6 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     pdl_launch_dependents();
     const f32x2 magic = splat2(-8388608.f);
     const int share = a.tiles;                    // this token tile writes blocks blockIdx.y, + share, ... to scratch
-    const bool writes = static_cast<int>(gridDim.y) == a.tiles;
     uint16_t* row_out = a.scratch + static_cast<size_t>(min(row0 + r, a.n_rows - 1)) * a.k;
     bool ok = true;
     for (int job = grp; job < nb && ok; job += 2) {
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
       const uint4 hdr = blk[0];
       const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
       const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-      const bool keep = writes && job % share == static_cast<int>(blockIdx.y) && row0 + r < a.n_rows;
+      const bool keep = a.tiles_write && job % share == static_cast<int>(blockIdx.y) && row0 + r < a.n_rows;
 #pragma unroll 1
       for (int g = 0; g < 4; ++g) {
         const int x = 2 * job + (g >> 1), slot = x % kQ4Slots;
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
   } else if (warp == 9) {
     // (the weights do not depend on the kernel before) 16-byte piece p = 9 * row + c goes to lane p % 32; nine steps
     // of 32 pieces are 32 rows. Rows past the matrix are zero: never stored. (Repeating its last row, hundreds of warps
-    // asked for the same lines: 32 rows over 2048 tokens of 2048 columns 32 us.)
+    // asked for the same lines: 32 rows over 2048 tokens of 2048 columns 32.3 us, now 13.6.)
     const int row_bytes = nb * kW4, last = a.n_rows - 1 - row0;
     for (int job = 0; job < nb; ++job) {
       const int st = job % kQ4WStages;
@@ -628,11 +628,21 @@ int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratc
   CUtensorMap mx;
   if (!operand_map(&mx, x, n_tokens, k, kLayoutSwizzled, bn)) return kErrUnsupported;
   if (!opt_in_smem<tc_gemm_q4_kernel>(kQ4Smem)) return kErrLaunch;
-  Q4Args a{static_cast<const unsigned char*>(w), y, scratch, n_rows, k, n_tokens, bn, std::min(8, kQ4BBytes / (bn * 128)), (n_tokens + bn - 1) / bn, status_word()};
-  // SMs that the tiles leave idle, by whole columns of row tiles, write the scratch, unless that takes longer than the
-  // tiles do with their shares: us per block and row tile, 3.2 / spare against 1.3 + 2 / tiles (measured).
+  Q4Args a{static_cast<const unsigned char*>(w), y, scratch, n_rows, k, n_tokens, bn, std::min(8, kQ4BBytes / (bn * 128)), (n_tokens + bn - 1) / bn, 0, status_word()};
+  // Who writes the scratch, by us per block of a row tile (measured): SMs that the tiles leave idle, in whole columns of row
+  // tiles, 3.2 / spare beside the tiles' 1.3; the tiles themselves, 2 / tiles on top of it; or the dequantisation kernel
+  // ahead of the GEMM, 2.5 us and the bytes at 5 TB/s. Few tokens over many rows leave few SMs and few tiles: 8192 x 4096
+  // over 64 tokens takes 53 us by one spare column, 43 by the kernel ahead.
   int spare = std::max(0, std::min(k / kQK, sms / row_tiles - a.tiles));
   if (32 * a.tiles >= spare * (13 * a.tiles + 20)) spare = 0;
+  const double added = k / kQK * (spare > 0 ? std::max(0.0, 3.2 / spare - 1.3) : 2.0 / a.tiles);
+  const bool ahead = added > 2.5 + static_cast<double>(n_rows) * k * 2.5625 / 5e6;
+  if (ahead) {
+    const int rc = launch_dequant(w, scratch, static_cast<long long>(n_rows) * (k / kQK), s);
+    if (rc != kOk) return rc;
+    spare = 0;
+  }
+  a.tiles_write = spare == 0 && !ahead;
   return launch_pdl(tc_gemm_q4_kernel, dim3(row_tiles, a.tiles + spare), kQ4Threads, kQ4Smem, s, mx, a);
 }
 

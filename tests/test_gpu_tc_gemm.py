@@ -185,8 +185,23 @@ def test_q4k_gemm_few_rows_past_a_tile(rows):
     w16 = torch.zeros(rows, k, dtype=torch.float16, device=DEV)
     ops.dequant_q4_k_f16(w_dev, w16, rows, k)
     assert torch.equal(scratch.view(torch.int16), w16.view(-1).view(torch.int16))
+    # fp32 accumulation in another order, one rounding to fp16
     assert rel(y[:tok].float().cpu().numpy(), gemm_want(w16, x_dev).cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
-    # (fp32 accumulation in another order, one rounding to fp16)
+
+
+@pytest.mark.parametrize("rows,k,tok", [(8192, 4096, 64), (8200, 4096, 3), (12288, 4096, 17)])
+def test_q4k_gemm_dequantised_ahead(rows, k, tok):
+    """Few tokens over many rows: the scratch is written by the dequantisation kernel ahead of the GEMM."""
+    w_np, w_dev = make_q4k(rows, k, 25)
+    x_np, x_dev = make_x16(tok, k, 26)
+    scratch = torch.zeros(rows * k + 8, dtype=torch.float16, device=DEV)
+    y = torch.full((tok + 1, rows), 9.0, dtype=torch.float16, device=DEV)
+    ops.tc_gemm_q4_k_f16(w_dev, x_dev, y, scratch, rows, k, tok)
+    w16 = torch.zeros(rows, k, dtype=torch.float16, device=DEV)
+    ops.dequant_q4_k_f16(w_dev, w16, rows, k)
+    assert torch.equal(scratch[:rows * k].view(torch.int16), w16.view(-1).view(torch.int16)) and torch.all(scratch[rows * k:] == 0)
+    # fp32 accumulation in another order, one rounding to fp16
+    assert rel(y[:tok].float().cpu().numpy(), gemm_want(w16, x_dev).cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
 
 
 def test_refusals_launch_nothing():
