@@ -22,10 +22,12 @@
 namespace sgr {
 namespace {
 
-// PER values per thread kept in registers (0: any number, read twice). One row is a chain of latencies -
-// load, warp fold, the warp sums in order, normalise, quantise: the norm weights are requested before the
-// previous kernel is awaited, and every thread adds the warp sums itself instead of waiting for one to do
-// it (one barrier and about a microsecond less).
+// PER values per thread kept in registers (0: any number, read twice). Few rows are a chain of latencies -
+// load, warp fold, the warp sums in order, normalise, quantise -, and the PER variants shorten it: the norm weights are
+// requested before the previous kernel is awaited, and every thread adds the warp sums itself instead of waiting for one to
+// do it (one barrier and about a microsecond less). With two CTAs on an SM, or rows of many values, the issue slots
+// decide, and 32 warps that add 32 sums each cost more than the barrier: one thread adds (512 rows of 4096: 8.2 us, by
+// all threads 9.9; one row of 8192: 4.35 / 4.61).
 template <int PER>
 __global__ void __launch_bounds__(1024) rmsnorm_quant_kernel(uint16_t* __restrict__ out, const uint16_t* __restrict__ x,
                                                             const uint16_t* __restrict__ w,
@@ -59,17 +61,28 @@ __global__ void __launch_bounds__(1024) rmsnorm_quant_kernel(uint16_t* __restric
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, off);
   if (lane == 0) red[warp] = acc;
   __syncthreads();
-  float s = 0.f;
   const int nw = blockDim.x >> 5;
+  float scale;
+  if constexpr (PER > 0) {
+    float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < 32; i += 4) {
-    const float4 r = *reinterpret_cast<const float4*>(red + i);
-    if (i < nw) s += r.x;
-    if (i + 1 < nw) s += r.y;
-    if (i + 2 < nw) s += r.z;
-    if (i + 3 < nw) s += r.w;
+    for (int i = 0; i < 32; i += 4) {
+      const float4 r = *reinterpret_cast<const float4*>(red + i);
+      if (i < nw) s += r.x;
+      if (i + 1 < nw) s += r.y;
+      if (i + 2 < nw) s += r.z;
+      if (i + 3 < nw) s += r.w;
+    }
+    scale = rsqrtf(s / static_cast<float>(n) + eps);
+  } else {
+    if (tid == 0) {
+      float s = 0.f;
+      for (int i = 0; i < nw; ++i) s += red[i];
+      red[0] = rsqrtf(s / static_cast<float>(n) + eps);
+    }
+    __syncthreads();
+    scale = red[0];
   }
-  const float scale = rsqrtf(s / static_cast<float>(n) + eps);
   if constexpr (PER > 0) {
 #pragma unroll
     for (int j = 0; j < N; ++j)
@@ -110,8 +123,10 @@ SGR_API int sgr_rmsnorm_quant_f16(uint16_t* out, const uint16_t* x, const uint16
   auto launch = [&](auto kern) {
     return launch_pdl(kern, dim3(n_rows), b, smem, as_stream(stream), out, x, w, static_cast<unsigned char*>(xq), n, eps);
   };
-  if (n <= b) return launch(rmsnorm_quant_kernel<1>);
-  if (n <= 2 * b) return launch(rmsnorm_quant_kernel<2>);
-  if (n <= 4 * b) return launch(rmsnorm_quant_kernel<4>);
+  if (n_rows <= device_sms()) {                 // one CTA per SM at most
+    if (n <= b) return launch(rmsnorm_quant_kernel<1>);
+    if (n <= 2 * b) return launch(rmsnorm_quant_kernel<2>);
+    if (n <= 4 * b) return launch(rmsnorm_quant_kernel<4>);
+  }
   return launch(rmsnorm_quant_kernel<0>);
 }

@@ -24,6 +24,24 @@ def _norm_inputs(rows, n, seed):
     return x, w
 
 
+@pytest.mark.parametrize("n", [256, 768, 1024, 1280, 2048, 3072, 4096, 4352, 8192, 16384])
+def test_rmsnorm_quant_rows_do_not_depend_on_their_number(n):
+    """Up to one row per SM the row is held in registers and every thread adds the warp sums, beyond that one thread does; rows of
+    more than 4096 values always go the second way: the same bits."""
+    rows = torch.cuda.get_device_properties(0).multi_processor_count + 1
+    x, w = _norm_inputs(rows, n, 5)
+    xd, wd = x.to(DEV), w.to(DEV)
+    res = []
+    for parts in ((rows,), (1, rows - 1)):
+        out, xq = torch.zeros_like(xd), torch.zeros(rows, n // 256 * 276, dtype=torch.uint8, device=DEV)
+        r0 = 0
+        for m in parts:
+            ops.rmsnorm_quant_f16(out[r0:], xd[r0:], wd, xq[r0:], n, 1e-6, m)
+            r0 += m
+        res.append((out, xq))
+    assert torch.equal(res[0][0].view(torch.int16), res[1][0].view(torch.int16)) and torch.equal(res[0][1], res[1][1])
+
+
 @pytest.mark.parametrize("rows,n", [(1, 2048), (4, 2048), (64, 2048), (3, 512), (2, 4096), (5, 256)])
 def test_rmsnorm_quant_blocks_are_those_of_its_own_output(oracle, rows, n):
     x, w = _norm_inputs(rows, n, 10 + rows)
