@@ -30,6 +30,19 @@ def test_quantize_q8_k_bit_exact(oracle, golden):
     assert np.array_equal(quantize_dev(dev(ex)).cpu().numpy(), golden["q8_edge_q"])
 
 
+@pytest.mark.parametrize("blocks", [1, 5, 12287, 12288, 12289, 30001])
+def test_quantize_q8_k_both_launch_forms(oracle, blocks):
+    """12,288 blocks is the line between the launch that overlaps the kernel before it and the plain one."""
+    x_np, x_dev = make_x16(blocks, 256, blocks)
+    xq = torch.zeros(blocks + 1, 276, dtype=torch.uint8, device=DEV)
+    ops.quantize_q8_k(x_dev, xq, blocks * 256)
+    assert np.array_equal(xq[:blocks].cpu().numpy(), oracle.quantize_q8k_f16(x_np)) and not xq[blocks].any()
+    d_rows = dev(np.int32([blocks - 1]))
+    xq.zero_()
+    ops.quantize_q8_k_n(x_dev, xq, d_rows, 256, blocks)
+    assert np.array_equal(xq[:blocks - 1].cpu().numpy(), oracle.quantize_q8k_f16(x_np)[:blocks - 1]) and not xq[blocks - 1].any()
+
+
 def test_quantize_q8_k_unaligned_input(oracle):
     x_np, x_dev = make_x16(1, 1024 + 8, 7)
     view = x_dev.reshape(-1)[3:3 + 1024]                 # 6-byte offset: scalar load path
