@@ -267,7 +267,10 @@ int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStre
   if (fit < a.rows_per_stage) a.rows_per_stage = fit >= 8 ? fit & ~7 : fit;
   const size_t stage_bytes = (static_cast<size_t>(a.rows_per_stage) * row_bytes + 127) & ~size_t(127);
   const int stages = a.rows_per_stage > 0 ? static_cast<int>(std::min<size_t>(kHeadStages, room / stage_bytes)) : 0;
-  const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && stages >= 2 && n_rows >= 4 * sms &&
+  // Rows per SM from which the ring pays (us, plain kernel / ring: one block 2,500 rows 2.8 / 2.8, 1,000 rows 2.3 / 2.9; two
+  // blocks 2,500 rows 2.8 / 3.1, 3,000 rows 3.4 / 3.2; four blocks 1,000 rows 3.1 / 3.4, 1,500 rows 3.5 / 3.4).
+  const int least = a.nb <= 2 ? 18 : (narrow ? 8 : 4);
+  const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && stages >= 2 && n_rows >= least * sms &&
                           static_cast<long long>(a.rows_per_stage) * row_bytes % 16 == 0 &&
                           static_cast<long long>(n_rows % a.rows_per_stage) * row_bytes % 16 == 0;
   if (!streamable) return launch_pdl(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);

@@ -21,7 +21,8 @@ def _q8(x_dev, k):
 
 
 @pytest.mark.parametrize("rows,k", [(1000, 2048), (37, 512), (151936, 2048), (4096, 4096),
-                                    (5000, 1024), (4098, 1024), (4999, 1024), (1001, 256), (3007, 1536), (1000, 16384), (600, 65536)])
+                                    (5000, 1024), (4098, 1024), (4999, 1024), (1001, 256), (3007, 1536), (1000, 16384), (600, 65536),
+                                    (2600, 512), (2700, 512), (2672, 256), (1183, 1024), (1192, 768)])     # about where the ring starts to pay
 def test_q6k_head_gemv(oracle, rows, k):
     rng = np.random.default_rng(rows + k)
     w_np = make_q6k(rng, rows, k)
