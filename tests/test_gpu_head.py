@@ -81,7 +81,7 @@ def _run_topk(o, logits, k):
     return out_v.cpu().numpy()[:kk], out_i.cpu().numpy()[:kk]
 
 
-@pytest.mark.parametrize("kind", ["normal", "ascending", "equal", "one_segment", "signed_zeros", "few"])
+@pytest.mark.parametrize("kind", ["normal", "ascending", "equal", "one_segment", "signed_zeros", "few", "masked", "masked_tail", "two_values"])
 @pytest.mark.parametrize("n,k", [(151936, 40), (262144, 64), (70000, 64), (2048, 1), (2049, 2)])
 def test_topk_threshold_and_merges(n, k, kind):
     """What decides whether the threshold leaves few candidates: values spread over the segments, or in order, equal, all the
@@ -96,6 +96,12 @@ def test_topk_threshold_and_merges(n, k, kind):
         x[:min(n, 2000)] += np.float32(100)
     elif kind == "signed_zeros":
         x = np.where(rng.random(n) < 0.5, np.float32(0.0), np.float32(-0.0)).astype(np.float32)
+    elif kind == "masked":                        # fewer values than k, or about as many, above a floor of equal ones
+        x[rng.random(n) >= 20 / n] = -1e9
+    elif kind == "masked_tail":
+        x[:n // 2] = np.float32(-3e38)
+    elif kind == "two_values":                    # hundreds of the larger one
+        x = np.where(rng.random(n) < 0.004, np.float32(2.0), np.float32(1.0)).astype(np.float32)
     elif kind == "few":
         x[:] = -np.inf
         x[rng.integers(0, n, 5)] = rng.standard_normal(5)
