@@ -19,9 +19,8 @@ __device__ __forceinline__ bool aligned16(const void* p) {
 // atomics) and builds the prefixes for itself, so nothing is exchanged; each of its warps then walks
 // one part of the list for one expert of its own and hands the slots out by ballot. The slots inside
 // an expert are in ascending (row, kk) order whatever the size. Bound by the latency of the phases:
-// 12 / 7 / 4 us for 16,384 / 6,216 / 768 routes over 256 experts. One CTA took 20 / 9.5 / 33 us (atomic fill
-// above 4096 routes, below a thread per expert walking the list); counting and ranking by match_any in
-// one CTA 48 us for the largest.
+// 3.9 us for 512 routes over 256 experts, 5.1 for 4,096. One CTA took 23 / 157 us (a thread per expert walking the
+// list); counting and ranking by match_any in one CTA 48 us for 16,384.
 // i / d for i below 2^31 by a multiplication (a division instruction sequence per route was half the time)
 struct FastDiv {
   unsigned mul;
@@ -39,15 +38,17 @@ struct FastDiv {
 };
 
 constexpr int kScanThreads = 512, kScanWarps = kScanThreads / 32;
-constexpr int kScanParts = 8;              // of the list, while [parts][n_expert] counters stay small
-constexpr int kScanPartExperts = 1024;
-constexpr int kScanStaged = 64 * 1024;     // routes whose ids are kept in shared memory, two bytes each
+constexpr int kScanParts = 8;              // of the list
+// With more experts or routes than this dispatch_scan_many_kernel (us for 256 experts, this kernel / that one: 4,096 routes 5.1 /
+// 5.9, 6,216 7.2 / 6.1, 16,384 12.3 / 8.0; for 288 experts a single row 4.2 / 3.5, 512 experts 2,048 routes 6.2 / 6.0).
+constexpr int kScanExperts = 256, kScanRoutes = 4096;
 
 __global__ void __launch_bounds__(kScanThreads)
 dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, int* __restrict__ gslot,
                      int* __restrict__ grows, int* __restrict__ off, int* __restrict__ toff,
                      int* __restrict__ meta, int* __restrict__ mail_n, int n_rows, int k,
-                     int n_expert, int tok_per, int parts, int per, FastDiv by_k, FastDiv by_per, int staged) {
+                     int n_expert, int tok_per, int per, FastDiv by_k, FastDiv by_per) {
+  constexpr int parts = kScanParts;
   extern __shared__ __align__(16) int cnt[];             // [parts][n_expert] counts, then first slots; ids after them
   uint16_t* ids = reinterpret_cast<uint16_t*>(cnt + static_cast<size_t>(parts) * n_expert);
   __shared__ int bad_sh;
@@ -72,7 +73,7 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
     for (int q = 0; q < 8; ++q) {
       const int i = b + q * kScanThreads;
       if (e8[q] < 0) continue;
-      if (staged) ids[i] = static_cast<uint16_t>(e8[q]);
+      ids[i] = static_cast<uint16_t>(e8[q]);
       if (e8[q] != 0xFFFF) {
         atomicAdd(cnt + static_cast<size_t>(by_per(i)) * n_expert + e8[q], 1);
       } else if (blockIdx.x == 0) {
@@ -139,7 +140,7 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int i = b + 32 * q + lane;
-      e8[q] = i < i1 ? (staged ? ids[i] : id_of(i)) : -1;
+      e8[q] = i < i1 ? ids[i] : -1;
     }
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
@@ -151,6 +152,110 @@ dispatch_scan_kernel(const int* __restrict__ idx, float* __restrict__ weight, in
         grows[slot] = by_k(i);
       }
       pos += __popc(hit);
+    }
+  }
+}
+
+// More experts or routes: what every CTA does per expert (clear, prefix) and per route (its warps' walks) would be repeated by
+// too many CTAs. Here a CTA takes a part of the route list: it counts the whole list, what lies before its part apart from
+// the rest, builds the prefixes - a thread takes a run of experts -, and one warp hands out the part's slots 32 routes at a time,
+// equal ids by match. Bound by the counting of the whole list, a shared-memory atomic per route: 16,384 routes 8.0 us over 256
+// experts, 12.0 over 5,000; 131,072 routes 37.6 (one CTA 20 / 26 / 135).
+constexpr int kManyThreads = 1024, kManyWarps = kManyThreads / 32;
+
+__global__ void __launch_bounds__(kManyThreads)
+dispatch_scan_many_kernel(const int* __restrict__ idx, float* __restrict__ weight, int* __restrict__ gslot,
+                          int* __restrict__ grows, int* __restrict__ off, int* __restrict__ toff,
+                          int* __restrict__ meta, int* __restrict__ mail_n, int n_rows, int k,
+                          int n_expert, int tok_per, int per, FastDiv by_k) {
+  extern __shared__ __align__(16) int before[];          // [n_expert] routes before this CTA's part, then its next slots
+  int* rest = before + n_expert;                         // [n_expert] the other routes
+  __shared__ int bad_sh;
+  __shared__ int wsum[2][kManyWarps];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+  const int total = n_rows * k, first = blockIdx.x * per, last = min(first + per, total);
+  if (tid == 0) bad_sh = 0;
+  for (int e = tid; e < 2 * n_expert; e += kManyThreads) before[e] = 0;
+  __syncthreads();
+  auto id_of = [&](int i) {
+    const int e = __ldg(idx + i + by_k(i));              // rows of k + 1
+    return e >= 0 && e < n_expert ? e : -1;
+  };
+  for (int b = tid; b < total; b += 8 * kManyThreads) {
+    int e8[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e8[q] = b + q * kManyThreads < total ? id_of(b + q * kManyThreads) : -2;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int i = b + q * kManyThreads;
+      if (e8[q] >= 0) {
+        atomicAdd((i < first ? before : rest) + e8[q], 1);
+      } else if (e8[q] == -1 && blockIdx.x == 0) {
+        // a corrupt id silences the whole row, shared-expert slot included
+        float* wr = weight + static_cast<size_t>(by_k(i)) * (k + 1);
+        for (int j = 0; j <= k; ++j) wr[j] = 0.f;
+        gslot[i] = -1;
+        atomicAdd(&bad_sh, 1);
+      }
+    }
+  }
+  __syncthreads();
+
+  // exclusive prefixes of rows and of tiles: a thread takes a run of experts
+  const int span = (n_expert + kManyThreads - 1) / kManyThreads, e0 = min(tid * span, n_expert), e1 = min(e0 + span, n_expert);
+  int c = 0, t = 0;
+  for (int e = e0; e < e1; ++e) {
+    const int v = before[e] + rest[e];
+    c += v;
+    t += (v + tok_per - 1) / tok_per;
+  }
+  int ic = c, it = t;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int uc = __shfl_up_sync(0xFFFFFFFFu, ic, o), ut = __shfl_up_sync(0xFFFFFFFFu, it, o);
+    if (lane >= o) { ic += uc; it += ut; }
+  }
+  if (lane == 31) { wsum[0][wp] = ic; wsum[1][wp] = it; }
+  __syncthreads();
+  int pc = ic - c + __reduce_add_sync(0xFFFFFFFFu, lane < wp ? wsum[0][lane] : 0);
+  int pt = it - t + __reduce_add_sync(0xFFFFFFFFu, lane < wp ? wsum[1][lane] : 0);
+  for (int e = e0; e < e1; ++e) {
+    const int v = before[e] + rest[e];
+    if (blockIdx.x == 0) { off[e] = pc; toff[e] = pt; }
+    before[e] += pc;
+    pc += v;
+    pt += (v + tok_per - 1) / tok_per;
+  }
+  if (blockIdx.x == 0 && tid == kManyThreads - 1) {
+    off[n_expert] = pc;
+    toff[n_expert] = pt;
+    meta[0] = pc;
+    meta[1] = pt;
+    meta[2] = bad_sh;
+    if (mail_n != nullptr) *mail_n = 0;
+  }
+  __syncthreads();
+
+  if (wp != 0) return;
+  for (int b = first; b < last; b += 256) {
+    int e8[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e8[q] = b + 32 * q + lane < last ? id_of(b + 32 * q + lane) : -1;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = e8[q], i = b + 32 * q + lane;
+      const unsigned same = __match_any_sync(0xFFFFFFFFu, e);
+      const int rank = __popc(same & ((1u << lane) - 1u));
+      if (e >= 0) {
+        const int slot = before[e] + rank;
+        gslot[i] = slot;
+        grows[slot] = by_k(i);
+      }
+      __syncwarp();
+      if (e >= 0 && rank == 0) before[e] += __popc(same);
+      __syncwarp();
     }
   }
 }
@@ -361,12 +466,22 @@ SGR_API int sgr_moe_dispatch_scan(const int* idx, float* weight, int* gslot, int
     return kErrArg;
   if (static_cast<long long>(n_rows) * k > 0x7FFFFF00) return kErrArg;
   if (n_expert > 12 * 1024) return kErrUnsupported;
-  const int parts = n_expert <= kScanPartExperts ? kScanParts : 1, per_cta = kScanWarps / parts;
-  const int staged = n_rows * k <= kScanStaged, per = ((n_rows * k + parts - 1) / parts + 31) / 32 * 32;       // routes per part
-  const size_t smem = static_cast<size_t>(parts) * n_expert * sizeof(int) + (staged ? static_cast<size_t>(n_rows) * k * 2 : 0);
-  if (smem > 40 * 1024 && !opt_in_smem<dispatch_scan_kernel>(200 * 1024)) return kErrLaunch;
-  return launch_pdl(dispatch_scan_kernel, dim3((n_expert + per_cta - 1) / per_cta), kScanThreads, smem, as_stream(stream), idx, weight,
-                    gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, parts, per, FastDiv(k), FastDiv(per), staged);
+  const int total = n_rows * k;
+  cudaStream_t st = as_stream(stream);
+  if (n_expert > kScanExperts || total > kScanRoutes) {
+    const int sms = device_sms();
+    if (sms <= 0) return kErrLaunch;
+    const int per = std::max(256, (total + sms - 1) / sms);
+    const size_t smem = 2 * static_cast<size_t>(n_expert) * sizeof(int);
+    if (smem > 40 * 1024 && !opt_in_smem<dispatch_scan_many_kernel>(static_cast<int>(smem))) return kErrLaunch;
+    return launch_pdl(dispatch_scan_many_kernel, dim3(std::max(1, (total + per - 1) / per)), kManyThreads, smem, st, idx, weight, gslot, grows,
+                      off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, per, FastDiv(k));
+  }
+  const int per = ((total + kScanParts - 1) / kScanParts + 31) / 32 * 32;       // routes per part
+  const size_t smem = static_cast<size_t>(kScanParts) * n_expert * sizeof(int) + static_cast<size_t>(total) * 2;
+  constexpr int per_cta = kScanWarps / kScanParts;
+  return launch_pdl(dispatch_scan_kernel, dim3((n_expert + per_cta - 1) / per_cta), kScanThreads, smem, st, idx, weight,
+                    gslot, grows, off, toff, meta, mail_n, n_rows, k, n_expert, tok_per, per, FastDiv(k), FastDiv(per));
 }
 
 SGR_API int sgr_gather_rows_q8(void* dst, const void* src, const int* src_rows, int n_rows,

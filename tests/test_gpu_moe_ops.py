@@ -48,9 +48,10 @@ def test_dispatch_scan_matches_oracle(oracle, n, k, e, tok):
     assert got["mail_n"][0] == 0                                      # the scan resets the mailbox
 
 
-@pytest.mark.parametrize("n,k,e", [(600, 8, 256), (2048, 8, 64), (129, 3, 5000), (33, 1, 1), (16, 8, 10241), (9000, 8, 256), (1, 1, 2048)])
+@pytest.mark.parametrize("n,k,e", [(600, 8, 256), (2048, 8, 64), (129, 3, 5000), (33, 1, 1), (16, 8, 10241), (9000, 8, 256), (1, 1, 2048),
+                                   (512, 8, 256), (513, 8, 256), (3, 1, 257), (4097, 1, 9), (40000, 8, 300), (37, 5, 12288)])
 def test_dispatch_scan_is_stable_at_any_size(oracle, n, k, e):
-    """Parts of the route list: ragged ones, one part above 2048 experts, ids kept in shared memory or read again."""
+    """Parts of the route list, ragged ones among them, and the line between the two kernels at 256 experts and 4,096 routes."""
     rng = np.random.default_rng(n)
     idx = np.zeros((n, k + 1), dtype=np.int32)
     idx[:, :k] = np.stack([rng.choice(e, k, replace=False) for _ in range(n)])
