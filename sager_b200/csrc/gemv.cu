@@ -342,38 +342,10 @@ struct DirectArgs {
   __device__ __forceinline__ int first_row(int m) const { return m == 0 ? 0 : (m == 1 ? rows_cum[0] : rows_cum[1]); }
 };
 
-// NI: block columns per warp (1 for rows of up to eight blocks)
-template <int NI, bool F16>
-__global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const DirectArgs a) {
-  __shared__ float red[kDirectWarps][8][16];                // [warp][token][row]
-  const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gid = lane >> 2, tig = lane & 3;
-  const int wpg = NI > 1 ? kDirectWarps : min(nb, kDirectWarps);        // warps per row group
-  const int groups = kDirectWarps / wpg, total = a.rows_cum[2];
-  const int cta_row0 = blockIdx.x * groups * 16;
-  const int row0 = cta_row0 + warp / wpg * 16, blk0 = warp & (wpg - 1);
-  uint4 hdr[2][NI];
-  uint2 q[2][NI][4];
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int row = min(row0 + gid + 8 * h, total - 1), m = a.matrix_of(row);
-    const unsigned char* wb = (m == 0 ? a.w[0] : (m == 1 ? a.w[1] : a.w[2])) +
-                              (static_cast<size_t>(row - a.first_row(m)) * nb + blk0) * kW4;
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      hdr[h][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
-#pragma unroll
-      for (int g = 0; g < 4; ++g) q[h][i][g] = __ldg(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
-    }
-  }
-  pdl_wait();
-  pdl_launch_dependents();
-  constexpr int NA = NI > 2 ? 2 : 1;        // rows of 32 blocks: (t0 + t2) + (t1 + t3), the shuffle tree's order
-  float acc[NA][4];
-#pragma unroll
-  for (int c = 0; c < NA; ++c)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[c][j] = 0.f;
+// The terms of the NI block columns blk0, blk0 + 8, ... that are in registers: sixteen rows x eight tokens.
+template <int NI, int NA>
+__device__ __forceinline__ void direct_blocks(const DirectArgs& a, const uint4 (&hdr)[2][NI], const uint2 (&q)[2][NI][4], int blk0,
+                                              int gid, int tig, float (&acc)[NA][4]) {
   const int zero[4] = {0, 0, 0, 0};
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
@@ -383,7 +355,7 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
     float xd[2] = {0.f, 0.f};
     const int blk = blk0 + 8 * i;
     if (gid < a.n_tokens) {
-      const uint32_t* xb = reinterpret_cast<const uint32_t*>(a.xq + (static_cast<size_t>(gid) * nb + blk) * kX8);
+      const uint32_t* xb = reinterpret_cast<const uint32_t*>(a.xq + (static_cast<size_t>(gid) * a.nb + blk) * kX8);
 #pragma unroll
       for (int sb = 0; sb < 8; ++sb) {
         b[sb][0] = __ldg(xb + 1 + 8 * sb + 2 * tig);
@@ -396,7 +368,7 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j)
-      if (2 * tig + j < a.n_tokens) xd[j] = __ldg(reinterpret_cast<const float*>(a.xq + (static_cast<size_t>(2 * tig + j) * nb + blk) * kX8));
+      if (2 * tig + j < a.n_tokens) xd[j] = __ldg(reinterpret_cast<const float*>(a.xq + (static_cast<size_t>(2 * tig + j) * a.nb + blk) * kX8));
     const Scales6 sl = unpack_scales6(hdr[0][i].y, hdr[0][i].z, hdr[0][i].w), sh = unpack_scales6(hdr[1][i].y, hdr[1][i].z, hdr[1][i].w);
     int isum[4] = {0, 0, 0, 0};
 #pragma unroll
@@ -411,13 +383,13 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
       const int shift = 16 * (g & 1);
       const int sc0_lo = ((sl.sc[g >> 1] >> shift) & 0xFF) << 4, sc1_lo = (sl.sc[g >> 1] >> (shift + 8)) & 0xFF;
       const int sc0_hi = ((sh.sc[g >> 1] >> shift) & 0xFF) << 4, sc1_hi = (sh.sc[g >> 1] >> (shift + 8)) & 0xFF;
-      int c0[4], c1[4];
-      mma_u8s8(c0, lo, b[2 * g][0], b[2 * g][1], zero);
-      mma_u8s8(c1, hi, b[2 * g + 1][0], b[2 * g + 1][1], zero);
-      isum[0] += sc0_lo * c0[0] + sc1_lo * c1[0];
-      isum[1] += sc0_lo * c0[1] + sc1_lo * c1[1];
-      isum[2] += sc0_hi * c0[2] + sc1_hi * c1[2];
-      isum[3] += sc0_hi * c0[3] + sc1_hi * c1[3];
+      int e0[4], e1[4];
+      mma_u8s8(e0, lo, b[2 * g][0], b[2 * g][1], zero);
+      mma_u8s8(e1, hi, b[2 * g + 1][0], b[2 * g + 1][1], zero);
+      isum[0] += sc0_lo * e0[0] + sc1_lo * e1[0];
+      isum[1] += sc0_lo * e0[1] + sc1_lo * e1[1];
+      isum[2] += sc0_hi * e0[2] + sc1_hi * e1[2];
+      isum[3] += sc0_hi * e0[3] + sc1_hi * e1[3];
     }
     // min term: the eight min bytes of a row are k = 0..7, the sums split as 128 * hi + lo
     const uint32_t ma[4] = {tig == 0 ? sl.mn[0] : (tig == 1 ? sl.mn[1] : 0u), tig == 0 ? sh.mn[0] : (tig == 1 ? sh.mn[1] : 0u), 0u, 0u};
@@ -429,6 +401,50 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
       const uint4& hd = hdr[j >> 1][i];
       const float d = 0.0625f * h2f(static_cast<uint16_t>(hd.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hd.x >> 16));
       acc[i % NA][j] += xd[j & 1] * (d * static_cast<float>(isum[j]) - dmin * static_cast<float>(dl[j] + 128 * dh[j]));
+    }
+  }
+}
+
+// NI: block columns per warp (1 for rows of up to eight blocks); LONG: rows of more than 32 blocks, 32 at a time
+template <int NI, bool F16, bool LONG = false>
+__global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const DirectArgs a) {
+  __shared__ float red[kDirectWarps][8][16];                // [warp][token][row]
+  const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gid = lane >> 2, tig = lane & 3;
+  const int wpg = NI > 1 ? kDirectWarps : min(nb, kDirectWarps);        // warps per row group
+  const int groups = kDirectWarps / wpg, total = a.rows_cum[2];
+  const int cta_row0 = blockIdx.x * groups * 16;
+  const int row0 = cta_row0 + warp / wpg * 16, blk0 = warp & (wpg - 1);
+  uint4 hdr[2][NI];
+  uint2 q[2][NI][4];
+  auto fetch = [&](int c0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int row = min(row0 + gid + 8 * h, total - 1), m = a.matrix_of(row);
+      const unsigned char* wb = (m == 0 ? a.w[0] : (m == 1 ? a.w[1] : a.w[2])) +
+                                (static_cast<size_t>(row - a.first_row(m)) * nb + blk0 + c0) * kW4;
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        hdr[h][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+#pragma unroll
+        for (int g = 0; g < 4; ++g) q[h][i][g] = __ldg(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
+      }
+    }
+  };
+  fetch(0);
+  pdl_wait();
+  pdl_launch_dependents();
+  constexpr int NA = NI > 2 ? 2 : 1;        // rows of 32 blocks: (t0 + t2) + (t1 + t3), the shuffle tree's order
+  float acc[NA][4];
+#pragma unroll
+  for (int c = 0; c < NA; ++c)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[c][j] = 0.f;
+  direct_blocks<NI, NA>(a, hdr, q, blk0, gid, tig, acc);
+  if constexpr (LONG) {
+    for (int c0 = 8 * NI; c0 < nb; c0 += 8 * NI) {
+      fetch(c0);
+      direct_blocks<NI, NA>(a, hdr, q, blk0 + c0, gid, tig, acc);
     }
   }
 #pragma unroll
@@ -535,9 +551,9 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct1_kernel(const D
   store_out<F16>(y, static_cast<size_t>(row - first), v);
 }
 
-// One to eight token rows, rows of a power of two of blocks up to 32, 16-byte aligned matrices.
+// One to eight token rows, rows of a power of two of blocks (one token: up to 32), 16-byte aligned matrices.
 inline bool direct_fits(const DirectArgs& a) {
-  if (a.n_tokens < 1 || a.n_tokens > 8 || a.nb > 32 || (a.nb & (a.nb - 1)) != 0) return false;
+  if (a.n_tokens < 1 || a.n_tokens > 8 || (a.n_tokens == 1 && a.nb > 32) || (a.nb & (a.nb - 1)) != 0) return false;
   for (int m = 0; m < 3; ++m)
     if (reinterpret_cast<uintptr_t>(a.w[m]) & 15u) return false;
   return true;
@@ -556,7 +572,8 @@ int launch_direct(const DirectArgs& a, cudaStream_t stream) {
   const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
   if (a.nb <= 8) return launch_pdl(gemv_direct_kernel<1, F16>, grid, threads, 0, stream, a);
   if (a.nb == 16) return launch_pdl(gemv_direct_kernel<2, F16>, grid, threads, 0, stream, a);
-  return launch_pdl(gemv_direct_kernel<4, F16>, grid, threads, 0, stream, a);
+  if (a.nb == 32) return launch_pdl(gemv_direct_kernel<4, F16>, grid, threads, 0, stream, a);
+  return launch_pdl(gemv_direct_kernel<4, F16, true>, grid, threads, 0, stream, a);
 }
 
 // tokens per CTA of the dense multi-token kernels (walked in sub-tiles of 8)

@@ -295,6 +295,20 @@ def test_grouped_device_plan_with_absent_experts(oracle, tok_per):
     assert sorted(mail.cpu().numpy()[:n_mail].tolist()) == sorted(mails_expected)
 
 
+@pytest.mark.parametrize("rows,k,tok", [(33, 16384, 2), (33, 16384, 8), (2049, 16384, 4), (5, 32768, 3), (16, 65536, 5)])
+def test_direct_kernel_long_rows(oracle, rows, k, tok):
+    """Rows of more than 32 blocks, 32 at a time."""
+    w_np, w_dev = make_q4k(rows, k, 5)
+    x_np, x_dev = make_x16(tok, k, 6)
+    xq = torch.zeros(tok, k // 256 * 276, dtype=torch.uint8, device=DEV)
+    ops.quantize_q8_k(x_dev, xq, tok * k)
+    y = torch.full((tok + 1, rows), 5.0, dtype=torch.float32, device=DEV)
+    ops.gemv_q4_k_q8_batched(w_dev, xq, y, rows, k, tok)
+    for t in range(tok):
+        assert rel(y[t].cpu().numpy(), oracle.gemv(w_np, xq.cpu().numpy()[t], rows, k)) <= GEMV_TOL
+    assert torch.all(y[tok] == 5.0)
+
+
 @pytest.mark.parametrize("rows,k", [(1, 256), (37, 256), (67, 512), (129, 1024), (1187, 2048), (2371, 2048), (4737, 2048), (33, 4096),
                                     (2373, 4096), (19, 8192)])
 @pytest.mark.parametrize("tok", [1, 2, 3, 4, 5, 8])
