@@ -576,6 +576,19 @@ int launch_direct(const DirectArgs& a, cudaStream_t stream) {
   return launch_pdl(gemv_direct_kernel<4, F16, true>, grid, threads, 0, stream, a);
 }
 
+// Where the tile kernel's CTAs, which copy their rows by one bulk copy each, are faster than the direct ones (us, direct / tile):
+// many rows of one or two blocks, whose lanes have little else in flight (one token, 24,000 / 60,000 rows of one block
+// 2.3 / 2.6, 3.5 / 3.1; 32,000 / 100,000 of two 3.8 / 3.5, 8.0 / 6.0; five to eight tokens 60,000 rows of one block 5.7 / 5.0), and
+// one token's rows of four or eight blocks that fill most of a single wave of them (20,000 of eight blocks 7.5 / 7.2, 16,000 6.5 /
+// 7.0, 24,000 - a second wave - 8.9 / 10.0; 40,000 of four 7.0 / 6.4, 60,000 9.6 / 10.5).
+inline bool tile_wins(const GemvArgs& a) {
+  if (a.nb > 8 || (a.n_tokens != 1 && (a.nb > 1 || a.n_tokens < 5))) return false;
+  const long long sms = device_sms(), rows = a.n_rows;
+  if (a.nb <= 2) return rows > 190 * sms;
+  const long long resident = 227 * 1024 / static_cast<long long>(tile_smem(1, a.nb, 1) + 1024), wave = sms * resident * tile_rows(a.nb);
+  return rows <= wave && 100 * rows > 72 * wave;
+}
+
 // tokens per CTA of the dense multi-token kernels (walked in sub-tiles of 8)
 constexpr int kDenseTokTile = 16;
 
@@ -603,7 +616,7 @@ int launch_dense(const void* w0, const void* w1, const void* xq, void* y0, void*
       return launch_stream<2, F16>(a, sms, stream);
     }
   }
-  {
+  if (NMAT == 2 || !tile_wins(a)) {
     DirectArgs d{{a.w[0], NMAT == 2 ? a.w[1] : nullptr, nullptr}, {y0, y1, nullptr}, {n_rows, NMAT * n_rows, NMAT * n_rows}, a.xq, a.nb, n_tokens, res};
     if (NMAT * static_cast<long long>(n_rows) <= 0x7FFFFFFF && direct_fits(d)) return launch_direct<F16>(d, stream);
   }

@@ -309,6 +309,20 @@ def test_direct_kernel_long_rows(oracle, rows, k, tok):
     assert torch.all(y[tok] == 5.0)
 
 
+@pytest.mark.parametrize("rows,k,tok", [(28119, 256, 1), (28121, 256, 1), (28121, 512, 1), (37800, 1024, 1), (52097, 1024, 1),
+                                        (17103, 2048, 1), (23681, 2048, 1), (28121, 256, 5), (28119, 256, 8)])
+def test_line_between_direct_and_tile_kernel(oracle, rows, k, tok):
+    w_np, w_dev = make_q4k(rows, k, 5)
+    x_np, x_dev = make_x16(tok, k, 6)
+    xq = torch.zeros(tok, k // 256 * 276, dtype=torch.uint8, device=DEV)
+    ops.quantize_q8_k(x_dev, xq, tok * k)
+    y = torch.full((tok + 1, rows), 5.0, dtype=torch.float32, device=DEV)
+    ops.gemv_q4_k_q8_batched(w_dev, xq, y, rows, k, tok)
+    for t in (0, tok - 1):
+        assert rel(y[t].cpu().numpy(), oracle.gemv(w_np, xq.cpu().numpy()[t], rows, k)) <= GEMV_TOL
+    assert torch.all(y[tok] == 5.0)
+
+
 @pytest.mark.parametrize("rows,k", [(1, 256), (37, 256), (67, 512), (129, 1024), (1187, 2048), (2371, 2048), (4737, 2048), (33, 4096),
                                     (2373, 4096), (19, 8192)])
 @pytest.mark.parametrize("tok", [1, 2, 3, 4, 5, 8])
