@@ -81,7 +81,7 @@ constexpr int kGateUpPairs = 256;               // pairs per gate/up group: one 
                                                 // or one of the halves where groups are few (Sched::split)
 constexpr int kDownRows = 256;                  // rows per down group
 constexpr int kFullArrivals = 1 + kXThreads;      // weight warp: one arrival; activation warps: a thread's copies landed
-constexpr int kAhead = AH;                        // stages of published groups that the weight warp is kept ahead with
+constexpr int kAhead = kAheadStages;
 constexpr int kMapRing = kAhead + kStageCount + 2;   // descriptor slots per CTA: groups (of one stage at least) that are
                                                  // published and not issued, in flight, and the one being patched
 

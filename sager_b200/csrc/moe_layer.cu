@@ -46,10 +46,8 @@ namespace {
 constexpr int kMaxRows = 64;       // token rows per call (row masks are 64-bit)
 constexpr int kTokTile = 8;        // token rows per tile of the item kernel (one MMA n-tile)
 constexpr int kMaxGrid = 160;            // most CTAs the expert kernels are launched with
-#ifndef AH
-#define AH 3
-#endif
-constexpr int kTmapSlots = AH + 7;           // patched TMA descriptor pairs per CTA of the row-streaming kernel
+constexpr int kAheadStages = 3;          // stages of published groups that the row-streaming kernel's weight warp is kept ahead with
+constexpr int kTmapSlots = kAheadStages + 7;      // patched TMA descriptor pairs per CTA of that kernel
 // Layers of up to this many token rows run as one persistent launch: all that its row sets hold (us per layer at 1 / 2 /
 // 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 15.7 / 22.1 / 29.7 / 36.4, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
 // 128 experts, hidden 1024: 13.6 / 17.9 / 20.3 / 22.6 against 23.6 / 25.7 / 31.3 / 29.6).
