@@ -105,6 +105,13 @@ OperandRows operand_rows(const sgr_moe_prefill* a) {
 
 inline bool has_shared(const sgr_moe_prefill* a) { return a->shared_gate && a->shared_up && a->shared_down; }
 
+// the combine reads the grouped rows in place when every buffer allows 16-byte accesses
+bool combines_in_place(const sgr_moe_prefill* a) {
+  return (a->hidden & 7) == 0 && a->n_used <= 1024 &&
+         ((reinterpret_cast<uintptr_t>(a->x_f16) | reinterpret_cast<uintptr_t>(a->y_grouped) |
+           (has_shared(a) ? reinterpret_cast<uintptr_t>(a->sh_y) : 0)) & 15u) == 0;
+}
+
 // gate / up, SwiGLU, requantise, down of the routed experts and of the shared one
 int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t stream) {
   const int n = a->n, H = a->hidden, F = a->n_ff, E = a->n_expert, K = a->n_used;
@@ -137,7 +144,10 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
 
 // Diagnostics (sager_b200_diag.h): the expert stage of a finished call once more, for timing.
 SGR_API int sgr_moe_prefill_expert_stage(const sgr_moe_prefill* a, void* stream) {
-  return a == nullptr ? kErrArg : expert_stage(a, operand_rows(a), as_stream(stream));
+  if (a == nullptr) return kErrArg;
+  const OperandRows op = operand_rows(a);
+  if (op.ready && !combines_in_place(a)) return kErrUnsupported;      // the combine's slab lies where the operand rows were
+  return expert_stage(a, op, as_stream(stream));
 }
 
 SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
@@ -177,10 +187,7 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
   SGR_STEP(sgr_moe_dispatch_scan(a->route_idx, a->route_w, a->gslot, a->grows, a->off, a->toff, a->meta,
                                  a->mail, a->mail_n, n, K, E, tok_per, stream));
   SGR_STEP(expert_stage(a, op, as_stream(stream)));
-  // the combine reads the grouped rows in place when every buffer allows 16-byte accesses
-  const bool direct = (H & 7) == 0 && K <= 1024 &&
-                      ((reinterpret_cast<uintptr_t>(a->x_f16) | reinterpret_cast<uintptr_t>(a->y_grouped) |
-                        (shared ? reinterpret_cast<uintptr_t>(a->sh_y) : 0)) & 15u) == 0;
+  const bool direct = combines_in_place(a);
   if (!direct) SGR_STEP(sgr_scatter_routed_f16(a->expert_y, a->y_grouped, a->gslot, n, K, H, stream));
   if (shared) {
     if (a->shared_gate_w != nullptr) {           // scalar gate sigmoid(w_sg . x) on the shared rows (layer.cpp:128-134)

@@ -56,6 +56,14 @@ def test_prefill_chunk_refuses_unaligned_buffers():
     for name, by in (("xn", 1), ("xq", 2), ("xqg", 8), ("hq", 4), ("g", 1), ("sh_g", 1), ("sh_q", 2)):
         assert call(**{name: by}) == 2, name
     assert call(xn=None) == 1
+    # the expert stage is not repeated on operand rows that the combine has overwritten
+    a = capi.MoePrefillArgs()
+    a.n, a.n_max, a.hidden, a.n_ff, a.n_expert, a.n_used = 4, 4, 512, 256, 8, 2
+    for name, kind in capi.MoePrefillArgs._fields_:
+        if kind is C.c_void_p:
+            setattr(a, name, 4096)
+    a.x_f16 = 4096 + 2
+    assert lib.raw("sgr_moe_prefill_expert_stage")(C.byref(a), None) == 3
 
 
 def test_shim_header_compiles_against_c_abi():
