@@ -109,10 +109,11 @@ def test_gemv_sweep_vs_oracle(oracle, rows, k, batch):
     assert f16_close(y16.cpu().numpy(), want)
 
 
-@pytest.mark.parametrize("rows,k,batch", [(40005, 2048, 3), (160001, 512, 2), (20003, 4096, 1), (20003, 4096, 2)])
+@pytest.mark.parametrize("rows,k,batch", [(40005, 2048, 3), (160001, 512, 2), (20003, 4096, 1), (20003, 4096, 2),
+                                          (40005, 2048, 1), (160001, 512, 1), (80003, 1024, 1), (310001, 256, 1)])
 def test_large_dense_gemv_persistent_kernel(oracle, rows, k, batch):
-    """Matrices of several stages per SM take the persistent streaming kernel; ragged last
-    stage, every supported row length (2, 8, 16 super-blocks) and token count."""
+    """Matrices of several stages per SM: one token, and two of more than eight super-blocks, take the persistent streaming
+    kernel (rows of 1, 2, 4, 8 and 16 super-blocks, ragged last stage), more tokens the MMA kernel at that size."""
     w_np, w_dev = make_q4k(rows, k, 41)
     x_np, x_dev = make_x16(batch, k, 42)
     xq = quantize_dev(x_dev)
@@ -328,7 +329,7 @@ def test_line_between_direct_and_tile_kernel(oracle, rows, k, tok):
 @pytest.mark.parametrize("tok", [1, 2, 3, 4, 5, 8])
 def test_direct_kernel_edges(oracle, rows, k, tok):
     """Every variant of the small-matrix kernel (lanes per row, rows per warp, groups per lane, token slots) at ragged row
-    counts; the line between one, two and four rows per warp lies at 1184 x 2 and x 4 rows."""
+    counts."""
     w_np, w_dev = make_q4k(rows, k, 5)
     x_np, x_dev = make_x16(tok, k, 6)
     xq = torch.zeros(tok, k // 256 * 276, dtype=torch.uint8, device=DEV)
