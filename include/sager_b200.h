@@ -309,7 +309,7 @@ int sgr_moe_layer_decode(const sgr_moe_layer* args, void* stream);
  * at a time and for the home side of an expert-parallel layer. */
 int sgr_moe_layer_decode_stages(const sgr_moe_layer* args, int stages, void* stream);
 
-/* Prefill grouped GEMM on int8 tensor cores (tcgen05, accumulators in tensor memory).
+/* Prefill grouped GEMM on the tensor cores (tcgen05, accumulators in tensor memory; _i8: of the quantised integers).
  * Replaces dequant_experts_q4_k_f16 + tc_gemm_f16_raw (cuda_ops.hpp:125-131, one cuBLAS GEMM per
  * expert and matrix) with the contract of gemv_grouped_tab_q4_k_q8_f16out_mtok (cuda_ops.hpp:247):
  * xq is the expert-major slab of Q8_K rows, off[n_expert+1] the row prefix of the device plan,
@@ -323,8 +323,9 @@ int sgr_moe_grouped_gemm_i8(const void* const* w_tab, const int* off, const void
  * (src/core/session.cpp:2482-3030 of the reference) on the session's own scratch buffers
  * (src/core/session.cpp:207-257; shapes below with R = n_max * n_used): quantise, router logits,
  * top-k, device plan, gather, gate / up, SwiGLU, requantise, down, scatter, shared expert,
- * combine into x_f16. The routed projections run on sgr_moe_grouped_gemm_i8; every other step is
- * the library's launcher of the same name. Stream-ordered, allocates nothing. */
+ * combine into x_f16, in seven launches: the projections of the routed and of the shared expert are two
+ * launches of the grouped GEMM, with the rows read through the plan. What the launchers of the sequence refuse is
+ * refused before anything is launched. Stream-ordered, allocates nothing. */
 typedef struct sgr_moe_prefill {
   int n, n_max;             /* token rows of this chunk / rows the buffers were sized for */
   int hidden, n_ff, n_expert, n_used;

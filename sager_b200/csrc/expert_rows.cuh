@@ -11,8 +11,8 @@
 // consumer warp owns sixteen of the rows - eight gate rows
 // and the eight up rows of the same indices, so SwiGLU needs no exchange - and
 // keeps its sums in registers from the first column to the last: no partial sums
-// in shared memory, no barrier between the warps; the only synchronisation is
-// the full/empty mbarrier pair of each stage.
+// in shared memory, no barrier between the warps; they synchronise by the stages' mbarriers
+// (full; weight part free; activation part free) and, once per block of h, by those of its buffer.
 //
 // The weight part of a stage arrives by TMA: two tiled copies per stage (boxes of
 // 144 bytes x 128 rows) through 2-D tensor maps over [rows][row bytes]. The maps

@@ -2,8 +2,8 @@
 // (src/kernels/cuda/q4_k.cu:1534-1562, 1660-1849, 1926-1985 and
 // src/kernels/cuda/mmq.cu:368-378 of the reference): dense single-row and
 // multi-token, pointer-table, host-plan grouped and device-plan grouped with
-// the null-pointer mailbox. One kernel template, four planners; all of them
-// end in tile_run (tile.cuh).
+// the null-pointer mailbox. One kernel template, four planners, all of which end in
+// tile_run_staged (tile.cuh); dense matrices of up to eight tokens have kernels of their own.
 #include <algorithm>
 
 #include "api_util.cuh"
@@ -206,7 +206,7 @@ int launch_tile(const GemvArgs& a, dim3 grid, cudaStream_t stream) {
 // whole number of rows when nb divides 256), each stage one bulk copy into a five-deep
 // ring issued by a producer warp. Thread t of the eight consumer warps owns block t of the
 // stage: a quarter-warp reads eight consecutive 144-byte blocks, 16 bytes per lane per
-// load, which spreads over all 32 banks without padding. The activations (at most four
+// load, which spreads over all 32 banks without padding. The activations (at most two
 // token rows) are staged once per CTA. The nb lanes of a row meet by shuffle.
 constexpr int kStreamBlocks = 256;                       // super-blocks per stage = consumer threads
 constexpr int kStreamStageBytes = kStreamBlocks * kW4;   // 36,864
@@ -624,7 +624,7 @@ int launch_dense(const void* w0, const void* w1, const void* xq, void* y0, void*
     a.tok_tile = 1;
     return launch_tile<NMAT, 1, kDense, F16>(a, dim3((n_rows + rc - 1) / rc, 1), stream);
   }
-  if (n_tokens <= 4) {              // a verify window: dp4a over four token slots beats the MMA fragment set-up
+  if (n_tokens <= 4) {              // (block counts that are no power of two, matrices off a 16-byte boundary)
     a.tok_tile = 4;
     return launch_tile<NMAT, 4, kDense, F16>(a, dim3((n_rows + rc - 1) / rc, 1), stream);
   }

@@ -16,7 +16,7 @@
 // The head is the largest matrix of a step (151,936 x 2048: 255 MB), so the GEMV is a
 // persistent kernel: one CTA per SM, a producer warp streaming stages of whole rows (1680
 // contiguous bytes each at k = 2048) into a shared-memory ring with bulk copies, eight
-// eight consumer warps of four rows each. A lane owns a quarter of a block (64 weights, four sub-groups): two
+// consumer warps of four rows each. A lane owns a quarter of a block (64 weights, four sub-groups): two
 // 16-byte runs of ql and one of qh, read as words (blocks start on 2-byte boundaries only: odd
 // blocks are realigned with a funnel shift), each ql word giving two packed words of 6-bit values
 // and each qh word serving four of them, fed to dp4a; a row of k = 2048 is one pass of a warp.

@@ -480,18 +480,4 @@ __device__ __forceinline__ void tile_run_staged(unsigned char* smem,
   if (!ok && threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
 }
 
-// Same, with the activations taken from packed Q8_K rows in global memory:
-//   xrow(t) -> pointer to the row of token slot t (0 <= t < ntok)
-template <int NMAT, int TT, typename XRow, typename Emit>
-__device__ __forceinline__ void tile_run(unsigned char* smem,
-                                         const unsigned char* const (&wsrc)[NMAT], int nrows,
-                                         int nb, int ntok, XRow xrow, Emit emit, int* status) {
-  tile_run_staged<NMAT, TT>(
-      smem, wsrc, nrows, nb, ntok, [] {},
-      [&](const XTile& xt, int t0, int nt) {
-        xtile_stage(xt, nt, [&](int t) { return xrow(t0 + t); }, threadIdx.x, kTileThreads);
-      },
-      emit, status);
-}
-
 }  // namespace sgr

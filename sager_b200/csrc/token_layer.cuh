@@ -252,7 +252,7 @@ __device__ __forceinline__ void load_half(HalfW<NMAT>& W, const unsigned char* c
   W.dmin = h2f(static_cast<uint16_t>(dd >> 16));
 }
 // The half blocks W against the rows of `rs` (a lane pair holds a block; the integer sums of the halves meet before the
-// one rounding, so the terms are block_dot's). Bound by the integer pipe: with two matrices each lane of the pair sends
+// one rounding, so the terms are block_dot's). Mostly integer instructions: with two matrices each lane of the pair sends
 // the sum it does not keep and both finish one matrix, which halves the shuffles and the arithmetic after them. Whole
 // warps call it: `rows` is the warp's largest row count. Not unrolled over rows: every phase of this kernel runs once
 // per CTA, so straight-line code is paid for in instruction fetch.
