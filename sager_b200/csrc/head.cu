@@ -422,8 +422,66 @@ struct TopkShared {
   int ties[256];                                   // words equal to the threshold, 32 at a time, then of all before them
 };
 template <int PER>
+struct TopkWords {
+  unsigned long long v[PER];
+};
+// The words for which wanted(j) holds into sh.cand, in any order; returns their number.
+template <int PER, typename Wanted>
+__device__ __forceinline__ int topk_collect(TopkShared& sh, const unsigned long long (&x)[PER], Wanted wanted) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const bool in = wanted(j);
+    const unsigned who = __ballot_sync(0xFFFFFFFFu, in);
+    if (who == 0u) continue;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(&sh.count, __popc(who));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(who & ((1u << lane) - 1u));
+    if (in && at < kTopkCand) sh.cand[at] = x[j];
+  }
+  __syncthreads();
+  return sh.count;
+}
+// `n` words reach the threshold, too many: collect them without all but the first k that equal it; more than kTopkCand
+// when that does not help. (A function: the common case does not fetch its instructions.)
+template <int PER>
+__device__ __noinline__ int topk_drop_ties(TopkShared& sh, TopkWords<PER> x, unsigned threshold, int n, int k) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto tie = [&](int j) { return x.v[j] != 0ull && static_cast<unsigned>(x.v[j] >> 32) == threshold; };
+  auto slot = [&](int j) { return 2 * (warp + 32 * (j >> 1)) + (j & 1); };
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const unsigned who = __ballot_sync(0xFFFFFFFFu, tie(j));
+    if (lane == 0) sh.ties[slot(j)] = __popc(who);
+  }
+  __syncthreads();
+  if (warp == 0) {                                 // their prefix sums, PER per lane
+    int own[PER], sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) { own[i] = sum; sum += sh.ties[lane * PER + i]; }
+    int before = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xFFFFFFFFu, before, o);
+      if (lane >= o) before += v;
+    }
+    if (lane == 31) sh.n_ties = before;
+    if (lane == 0) sh.count = 0;
+    before -= sum;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) sh.ties[lane * PER + i] = before + own[i];
+  }
+  __syncthreads();
+  if (n - sh.n_ties + k > kTopkCand) return kTopkCand + 1;
+  return topk_collect<PER>(sh, x.v, [&](int j) {
+    const bool t = tie(j);
+    const int rank = sh.ties[slot(j)] + __popc(__ballot_sync(0xFFFFFFFFu, t) & ((1u << lane) - 1u));
+    return t ? rank < k : x.v[j] != 0ull && static_cast<unsigned>(x.v[j] >> 32) > threshold;
+  });
+}
+template <int PER>
 __device__ __forceinline__ bool topk_by_threshold(TopkShared& sh, const unsigned long long (&x)[PER], int n_pool, int k) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   if (tid == 0) sh.count = 0;
   __syncthreads();                                 // the pool is complete
   if (tid < n_pool) {
@@ -438,53 +496,13 @@ __device__ __forceinline__ bool topk_by_threshold(TopkShared& sh, const unsigned
   }
   __syncthreads();
   const unsigned threshold = sh.threshold;
-  auto collect = [&](auto wanted) {
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const bool in = wanted(j);
-      const unsigned who = __ballot_sync(0xFFFFFFFFu, in);
-      if (who == 0u) continue;
-      int at = 0;
-      if (lane == 0) at = atomicAdd(&sh.count, __popc(who));
-      at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(who & ((1u << lane) - 1u));
-      if (in && at < kTopkCand) sh.cand[at] = x[j];
-    }
-    __syncthreads();
-    return sh.count;
-  };
-  int n = collect([&](int j) { return x[j] != 0ull && static_cast<unsigned>(x[j] >> 32) >= threshold; });
+  int n = topk_collect<PER>(sh, x, [&](int j) { return x[j] != 0ull && static_cast<unsigned>(x[j] >> 32) >= threshold; });
   if (n > kTopkCand) {
-    auto tie = [&](int j) { return x[j] != 0ull && static_cast<unsigned>(x[j] >> 32) == threshold; };
-    auto slot = [&](int j) { return 2 * (warp + 32 * (j >> 1)) + (j & 1); };
+    TopkWords<PER> w;
 #pragma unroll
-    for (int j = 0; j < PER; ++j) {
-      const unsigned who = __ballot_sync(0xFFFFFFFFu, tie(j));
-      if (lane == 0) sh.ties[slot(j)] = __popc(who);
-    }
-    __syncthreads();
-    if (warp == 0) {                               // their prefix sums, PER per lane
-      int own[PER], sum = 0;
-#pragma unroll
-      for (int i = 0; i < PER; ++i) { own[i] = sum; sum += sh.ties[lane * PER + i]; }
-      int before = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xFFFFFFFFu, before, o);
-        if (lane >= o) before += v;
-      }
-      if (lane == 31) sh.n_ties = before;
-      if (lane == 0) sh.count = 0;
-      before -= sum;
-#pragma unroll
-      for (int i = 0; i < PER; ++i) sh.ties[lane * PER + i] = before + own[i];
-    }
-    __syncthreads();
-    if (n - sh.n_ties + k > kTopkCand) return false;
-    n = collect([&](int j) {
-      const bool t = tie(j);
-      const int rank = sh.ties[slot(j)] + __popc(__ballot_sync(0xFFFFFFFFu, t) & ((1u << lane) - 1u));
-      return t ? rank < k : x[j] != 0ull && static_cast<unsigned>(x[j] >> 32) > threshold;
-    });
+    for (int j = 0; j < PER; ++j) w.v[j] = x[j];
+    n = topk_drop_ties<PER>(sh, w, threshold, n, k);
+    if (n > kTopkCand) return false;
   }
   if (tid < n) {
     const unsigned long long mine = sh.cand[tid];

@@ -437,10 +437,18 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
       if (!wait_warp(kQ4WEmpty + st, ((job / kQ4WStages) & 1) ^ 1u)) break;
       const unsigned char* src = a.w + static_cast<size_t>(row0) * row_bytes + job * kW4;
       const uint32_t dst = smem_u32(w_sm + st * kQ4WBytes) + lane * 16;
+      if (last >= 127) {
 #pragma unroll 9
-      for (int q = 0; q < 36; ++q) {
-        const int piece = q * 32 + lane, row = piece / 9;
-        cp_async16_or_zero(dst + q * 512, src + static_cast<size_t>(min(row, last)) * row_bytes + (piece - 9 * row) * 16, row <= last);
+        for (int q = 0; q < 36; ++q) {
+          const int piece = q * 32 + lane, row = piece / 9;
+          cp_async16(dst + q * 512, src + static_cast<size_t>(row) * row_bytes + (piece - 9 * row) * 16);
+        }
+      } else {
+#pragma unroll 1
+        for (int q = 0; q < 36; ++q) {
+          const int piece = q * 32 + lane, row = piece / 9;
+          cp_async16_or_zero(dst + q * 512, src + static_cast<size_t>(min(row, last)) * row_bytes + (piece - 9 * row) * 16, row <= last);
+        }
       }
       cp_async_arrive(&bar[kQ4WFull + st]);
     }
