@@ -639,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
               b1 = b0 + static_cast<size_t>(kHalfRows) * rb_f;
             }
             const uintptr_t align = reinterpret_cast<uintptr_t>(b0) | reinterpret_cast<uintptr_t>(b1);
-            copy_unaligned(st, 2 * kHalfBytes / 16, lane, align, [&](int p) {
+            warp_copy_unaligned(st, 2 * kHalfBytes / 16, lane, align, [&](int p) {
               const int r = p / 9, h = r / kHalfRows;
               return (h ? b1 : b0) + static_cast<size_t>(r - h * kHalfRows) * rb + (p - r * 9) * 16;
             });

@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
 #pragma unroll 4
               for (int q = lane; q < kStageBytes / 16; q += 32) cp_async16_or_zero(smem_u32(stage) + q * 16, piece(q), q / 9 <= last);
               cp_async_arrive(&bar[kBarWFull + s]);
-            } else if (copy_unaligned(stage, kStageBytes / 16, lane, align, piece)) {
+            } else if (warp_copy_unaligned(stage, kStageBytes / 16, lane, align, piece)) {
               mbar_arrive_one(&bar[kBarWFull + s]);
             } else {
               cp_async_arrive(&bar[kBarWFull + s]);

@@ -102,7 +102,7 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes
 // over 256 experts 8 / 2 bytes off takes 367 / 1230 us, with a piece's half words one piece at a time 2059 / 2060; a
 // three-row layer of the one-launch kernel 40 / 96 us, 178 / 178 before.
 template <typename Src>
-__device__ __forceinline__ bool copy_unaligned(unsigned char* dst, int pieces, int lane, uintptr_t align, Src src_of) {
+__device__ __forceinline__ bool warp_copy_unaligned(unsigned char* dst, int pieces, int lane, uintptr_t align, Src src_of) {
   if ((align & 3u) == 0) {
     const bool by8 = (align & 7u) == 0;
 #pragma unroll 4
