@@ -73,6 +73,26 @@ struct ExpertGemm {
   int shared_rows;
 };
 int gemm_grouped(const ExpertGemm& g, cudaStream_t stream);
+// ---- the same for few token rows per expert (grouped_gemm_rows.cu) ----
+// Its activation rows: kRowBlk bytes per 256 values - fp32 scale, 12 bytes of padding, 256 codes, and the sub-block sums as
+// bsum = 128 * hi + lo: lo of sub-blocks 0-3, hi of 0-3, lo of 4-7, hi of 4-7, a byte each. 16-byte aligned.
+constexpr int kRowBlk = 288;
+// maps: [n_expert + 1][3] descriptors of 128 bytes (gate, up, down; the shared expert's last) and 16 bytes of counters, made and
+// cleared by quantize_rows. n_rows and k multiples of 256, outputs 4-byte aligned.
+struct ExpertMaps {
+  const unsigned char* const* tab;     // [3][stride]
+  long long stride;
+  void* maps;                          // 128-byte aligned
+  const void* shared[3];
+  int n_expert, hidden, n_ff;
+};
+// gate, up and SwiGLU: y receives h
+int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, const void* maps, cudaStream_t stream);
+int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream);
+// rows of k fp16 values -> such rows; two slabs, the first of at most *d_rows rows when that is given.
+// Clears the counters of the two GEMM launches; with make_maps the descriptors are made as well.
+int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_rows, const uint16_t* x1, void* out1, long long rows1,
+                  int k, const ExpertMaps& em, bool make_maps, cudaStream_t stream);
 // gate and up in one pass (g holds the gate side)
 int gemm_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, uint16_t* y_up, const void* shared_up,
                  uint16_t* shared_y_up, cudaStream_t stream);

@@ -112,22 +112,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void tmap_replace_addr(void* smem_map, const void* gaddr) {
-  asm volatile("tensormap.replace.tile.global_address.shared::cta.b1024.b64 [%0], %1;" ::"r"(smem_u32(smem_map)), "l"(gaddr) : "memory");
-}
-// whole warp: copy the patched 128-byte descriptor to global memory for the TMA unit
-__device__ __forceinline__ void tmap_publish(void* gmem_map, void* smem_map) {
-  asm volatile("tensormap.cp_fenceproxy.global.shared::cta.tensormap::generic.release.gpu.sync.aligned [%0], [%1], 128;"
-               ::"l"(gmem_map), "r"(smem_u32(smem_map)) : "memory");
-}
-__device__ __forceinline__ void tmap_acquire(const void* gmem_map) {
-  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(gmem_map) : "memory");
-}
-// box (144 bytes x 128 rows) at byte column x, row y; dst 128-byte aligned, x a multiple of 16
-__device__ __forceinline__ void tma_load_box(void* dst, const void* gmem_map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
 // The service warps' wait: they wait most of the time, and their polls took a fifth of the issue slots that the consumers need.
 __device__ __forceinline__ bool mbar_wait_idle(uint64_t* bar, uint32_t parity) {
   for (int it = 0; it < (1 << 20); ++it) {

@@ -1,0 +1,489 @@
+// grouped_gemm_rows.cu - the prefill MoE grouped GEMM for chunks that leave an expert few token rows.
+//
+// Same contract and same values as the tcgen05 form (grouped_gemm_i8.cu; both replace the reference's prefill expert math,
+// src/kernels/cuda/tc_gemm.cu:124-152, 209-240): Q8_K activations, exact integer sums per super-block, and per block
+//     acc = fma(xd, fma(-dmin, M, d * S), acc)
+// in block order, so the two agree to the bit (while S stays below 2^24, which the tensor-memory accumulator holds
+// exactly). That form unpacks every weight to fp16 and passes a block column through five roles whatever the number of
+// token rows: 1,800 cycles per 128 rows x 256 weights at 16 rows, 2,500 at 64, where HBM needs 800. Here a consumer warp
+// keeps sixteen weight rows and their sums from the first block column to the last (as the decode layer's row-streaming
+// kernel, expert_rows.cuh): nibbles go into mma.sync m16n8k32 with one logic instruction per four, the sub-block scales
+// are applied to the int32 results.
+//
+// Persistent, one CTA per SM. A unit is 128 (gate, up) row pairs, or 256 rows, of one expert and at most 32 of its
+// token rows; its block columns stream through a ring of four stages (256 blocks of 144 bytes by two TMA copies, and
+// that block of the token rows by one bulk copy each). Sixteen consumer warps, one weight warp, two activation warps; a
+// consumer returns its share of the weight bytes as soon as they are in registers. Gate and up rows of the same index meet
+// in a warp, so SwiGLU happens on the accumulators (rounded to fp16 first, as the reference's staged rows are). Waits are
+// bounded; an expiry raises the status word.
+#include <algorithm>
+
+#include "api_util.cuh"
+#include "quantize_dev.cuh"
+#include "tile.cuh"
+#include "tmap_dev.cuh"
+
+namespace sgr {
+namespace {
+
+constexpr int kTok = 32;                                     // token rows per unit
+constexpr int kConsumerWarps = 16, kWeightWarp = kConsumerWarps, kFirstXWarp = kWeightWarp + 1, kXWarps = 2;
+constexpr int kThreads = (kFirstXWarp + kXWarps) * 32;
+constexpr int kStages = 4;
+constexpr int kHalfBytes = 128 * kW4, kWBytes = 2 * kHalfBytes;
+// activation part of a stage: a 288-byte block (kRowBlk, api_util.cuh) per token row; rows 76 words apart, so
+// that eight rows' 16 bytes lie in different banks
+constexpr int kXRow = 304, kXCodes = 16, kXSums = 272, kXBytes = kTok * kXRow;
+static_assert(kRowBlk <= kXRow && kXSums + 16 == kRowBlk, "block layout");
+constexpr int kStageBytes = (kWBytes + kXBytes + 127) & ~127;
+constexpr int kHdr = 1024;
+constexpr int kSmem = kHdr + kStages * kStageBytes;
+static_assert(kSmem <= 227 * 1024, "shared memory");
+
+struct RowsArgs {
+  const unsigned char* const* tab0;    // [E] gate (or the only matrix)
+  const unsigned char* const* tab1;    // [E] up
+  const unsigned char* maps;           // [E + 1][3] descriptors; the matrix of tab0 is map0
+  int map0;
+  const int* off;                      // [E + 1] grouped slots of each expert
+  const int* rows;                     // source row of a grouped slot; null: the slot itself
+  const unsigned char *xq, *sxq;       // activation rows in 288-byte blocks; the shared expert's
+  uint16_t *y, *sy;                    // [slots][n_rows]
+  const unsigned char *sw0, *sw1;      // the shared expert (null: none)
+  int n_rows, nb, n_expert, groups;    // row groups per matrix
+  int s_rows, s_step, s_items, n_items;
+  unsigned* next;                      // items handed out beyond the first of every CTA
+  int* status;
+};
+
+// One unit, as the weight warp publishes it in shared memory for the activation warps.
+struct alignas(16) Unit {
+  int slot0, nt, flags;                // first slot, token rows (0: end of the list), 1 shared / 2 absent
+  int pad;
+};
+constexpr int kListSlots = 8;          // units published ahead: at most one per stage, and the one being read
+static_assert(kListSlots >= kStages + 3, "a reader could be overtaken");
+
+struct Desc {      // one 16-byte load per stage and warp
+  int flags;       // bits 0-7 token rows, 8 first column, 9 last, 10 absent, 11 shared, 12 end of the list
+  int slot0, group;
+  int pad;
+};
+
+// (as one instruction: sums of products are otherwise regrouped into a multiplication, a multiply-add and an addition)
+__device__ __forceinline__ int imad(int a, int b, int c) {
+  int d;
+  asm("mad.lo.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+// One super-block of a warp's sixteen rows against NT groups of eight token rows; as warp_mma_block (tile.cuh) with the
+// fp32 steps spelled out, and with the even sub-blocks' scales taken sixteen-fold instead of their sums.
+template <int NT, typename Loaded>
+__device__ __forceinline__ void rows_block(const unsigned char* a_ptr, const unsigned char* h_lo, const unsigned char* h_hi,
+                                           const unsigned char* xs, float (&acc)[4][4], int lane, Loaded loaded) {
+  const int gid = lane >> 2, tig = lane & 3;
+  const uint4 h0 = *reinterpret_cast<const uint4*>(h_lo);
+  const uint4 h1 = *reinterpret_cast<const uint4*>(h_hi);
+  uint32_t raw[4][4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) ldmatrix_x4(raw[g], a_ptr + g * 32);
+  loaded();
+  const float d_lo = 0.0625f * h2f(static_cast<uint16_t>(h0.x & 0xFFFFu)), m_lo = -h2f(static_cast<uint16_t>(h0.x >> 16));
+  const float d_hi = 0.0625f * h2f(static_cast<uint16_t>(h1.x & 0xFFFFu)), m_hi = -h2f(static_cast<uint16_t>(h1.x >> 16));
+  const Scales6 s_lo = unpack_scales6(h0.y, h0.z, h0.w), s_hi = unpack_scales6(h1.y, h1.z, h1.w);
+  int isum[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) isum[n][j] = 0;
+  const int zero[4] = {0, 0, 0, 0};
+  // matrices of an activation load: (tokens, k 0-15 / 16-31) of sub-block 2g, then of 2g + 1
+  const unsigned char* b_ptr = xs + (lane & 7) * kXRow + kXCodes + (lane >> 3) * 16;
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    uint32_t lo[4], hi[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      lo[j] = raw[g][j] & 0x0F0F0F0Fu;
+      hi[j] = raw[g][j] & 0xF0F0F0F0u;            // sixteen-fold
+    }
+    const int sh = 2 * (g & 1);
+    const int sc0_lo = __byte_perm(s_lo.sc[g >> 1], 0, 0x4440 + sh) << 4, sc1_lo = __byte_perm(s_lo.sc[g >> 1], 0, 0x4441 + sh);
+    const int sc0_hi = __byte_perm(s_hi.sc[g >> 1], 0, 0x4440 + sh) << 4, sc1_hi = __byte_perm(s_hi.sc[g >> 1], 0, 0x4441 + sh);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      uint32_t b[4];
+      ldmatrix_x4(b, b_ptr + n * 8 * kXRow + g * 64);
+      int c0[4], c1[4];
+      mma_u8s8(c0, lo, b[0], b[1], zero);
+      mma_u8s8(c1, hi, b[2], b[3], zero);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        isum[n][j] = imad(j < 2 ? sc0_lo : sc0_hi, c0[j], isum[n][j]);
+        isum[n][j] = imad(j < 2 ? sc1_lo : sc1_hi, c1[j], isum[n][j]);
+      }
+    }
+  }
+  const uint32_t ma[4] = {tig == 0 ? s_lo.mn[0] : (tig == 1 ? s_lo.mn[1] : 0u), tig == 0 ? s_hi.mn[0] : (tig == 1 ? s_hi.mn[1] : 0u), 0u, 0u};
+#pragma unroll
+  for (int n = 0; n < NT; ++n) {
+    // parts of the sub-block sums 4 tig .. 4 tig + 3 of token 8 n + gid (lanes whose mins are zero read another's)
+    const uint2 sv = *reinterpret_cast<const uint2*>(xs + (8 * n + gid) * kXRow + kXSums + 8 * (tig & 1));
+    int dl[4], dh[4];
+    mma_u8s8(dl, ma, sv.x, 0u, zero);
+    mma_u8s8(dh, ma, sv.y, 0u, zero);
+    const float* xd = reinterpret_cast<const float*>(xs + (8 * n + 2 * tig) * kXRow);
+    const float xd0 = xd[0], xd1 = xd[kXRow / 4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float s = __fmul_rn(j < 2 ? d_lo : d_hi, static_cast<float>(isum[n][j]));
+      acc[n][j] = __fmaf_rn(j & 1 ? xd1 : xd0, __fmaf_rn(j < 2 ? m_lo : m_hi, static_cast<float>(imad(dh[j], 128, dl[j])), s), acc[n][j]);
+    }
+  }
+}
+
+template <bool DUAL>
+__global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const RowsArgs a) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem);            // [kStages] copies landed
+  uint64_t* wempty = full + kStages;                             // weight part may be refilled
+  uint64_t* xempty = wempty + kStages;                           // activation part may be refilled
+  volatile unsigned* published = reinterpret_cast<volatile unsigned*>(smem + 132);
+  Desc* desc = reinterpret_cast<Desc*>(smem + 256);
+  Unit* list = reinterpret_cast<Unit*>(smem + 512);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&full[s], 1 + kXWarps);
+      mbar_init(&wempty[s], kConsumerWarps);
+      mbar_init(&xempty[s], kConsumerWarps);
+    }
+    *published = 0;
+    fence_barrier_init();
+  }
+  __syncthreads();
+  pdl_wait();                                        // plan, descriptors and activations come from the kernels before this one
+  pdl_launch_dependents();
+  auto wait = [&](uint64_t* b, unsigned parity) {
+    if (__all_sync(0xFFFFFFFFu, mbar_wait(b, parity)) != 0) return true;
+    if (lane == 0) atomicExch(a.status, 6);
+    return false;
+  };
+  int s = 0;
+  unsigned ph = 0;
+  auto advance = [&] { if (++s == kStages) { s = 0; ph ^= 1u; } };
+
+  if (warp == kWeightWarp) {
+    // ---------------- weights ----------------
+    // Items are handed out as CTAs come to want them: with rounds of fixed length the slowest CTA had 293,000 cycles of
+    // 241,000 on average (777 rows over 256 experts). The three round trips of a new item hide behind four full stages.
+    const int row_bytes = a.nb * kW4;
+    unsigned k = 0;                                  // units published
+    auto publish = [&](int slot0, int nt, int flags) {
+      if (lane == 0) {
+        Unit* e = list + k % kListSlots;
+        e->slot0 = slot0; e->nt = nt; e->flags = flags;
+        __threadfence_block();
+        *published = k + 1;
+      }
+      ++k;
+    };
+    unsigned item = blockIdx.x;
+    while (item < static_cast<unsigned>(a.n_items)) {
+      unsigned later = 0;
+      if (lane == 0) later = atomicAdd(a.next, 1u);
+      const bool shared = item < static_cast<unsigned>(a.s_items);
+      const int i = static_cast<int>(shared ? item : item - a.s_items), e = i / a.groups, group = i - e * a.groups;
+      int slot = e * a.s_step, m = min(a.s_step, a.s_rows - slot);
+      const unsigned char *w0 = a.sw0, *w1 = a.sw1;
+      if (!shared) {
+        slot = __ldg(a.off + e);
+        m = __ldg(a.off + e + 1) - slot;
+        w0 = a.tab0[e];
+        w1 = DUAL ? a.tab1[e] : w0;
+      }
+      const uintptr_t align = (reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1)) & 15u;
+      const bool absent = w0 == nullptr || w1 == nullptr;
+      const unsigned char* map0 = a.maps + (static_cast<size_t>(shared ? a.n_expert : e) * 3 + a.map0) * 128;
+      const int row0 = group * (DUAL ? 128 : 256);
+      if (m > 0 && !absent && align == 0 && lane == 0) {
+        tmap_acquire(map0);
+        if (DUAL) tmap_acquire(map0 + 128);
+      }
+      const int passes = (m + kTok - 1) / kTok, step = m > kTok ? ((m + passes - 1) / passes + 7) & ~7 : kTok;
+#pragma unroll 1
+      for (; m > 0; m -= step, slot += step) {
+        const int nt = min(step, m);
+        publish(slot, nt, (shared ? 1 : 0) | (absent ? 2 : 0));
+#pragma unroll 1
+        for (int b = 0; b < a.nb; ++b) {
+          if (!wait(&wempty[s], ph ^ 1u)) return;
+          unsigned char* st = smem + kHdr + s * kStageBytes;
+          if (lane == 0) {
+            Desc d;
+            d.flags = nt | (b == 0 ? 1 << 8 : 0) | (b + 1 == a.nb ? 1 << 9 : 0) | (absent ? 1 << 10 : 0) | (shared ? 1 << 11 : 0);
+            d.slot0 = slot; d.group = group; d.pad = 0;
+            desc[s] = d;
+          }
+          if (!absent && align == 0) {
+            if (lane == 0) {
+              mbar_expect_tx(&full[s], kWBytes);
+              tma_load_box(st, map0, b * kW4, row0, &full[s]);
+              tma_load_box(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
+            }
+          } else {
+            if (!absent) {                           // a base off a 16-byte boundary: plain copies
+              const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
+              const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
+              warp_copy_unaligned(st, kWBytes / 16, lane, align, [&](int p) {
+                const int r = p / 9, h = r >> 7;
+                return (h ? b1 : b0) + static_cast<size_t>(r & 127) * row_bytes + (p - r * 9) * 16;
+              });
+              asm volatile("cp.async.wait_all;" ::: "memory");
+              fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(&full[s]);
+          }
+          advance();
+        }
+      }
+      item = __shfl_sync(0xFFFFFFFFu, later, 0) + gridDim.x;
+    }
+    publish(0, 0, 0);
+    if (!wait(&wempty[s], ph ^ 1u)) return;
+    if (lane == 0) {                                 // one last stage that only says that the list is at its end
+      Desc d;
+      d.flags = 1 << 12; d.slot0 = d.group = d.pad = 0;
+      desc[s] = d;
+      mbar_arrive_one(&full[s]);
+    }
+  } else if (warp >= kFirstXWarp) {
+    // ---------------- activations: one bulk copy of 288 bytes per token row and block ----------------
+    const int x = warp - kFirstXWarp, t = kXWarps * lane + x;      // this lane's token row
+    const size_t xrow = static_cast<size_t>(a.nb) * kRowBlk;
+    for (unsigned k = 0;; ++k) {
+      unsigned it = 0;
+      if (lane == 0)
+        while (*published <= k && ++it < (1u << 24)) __nanosleep(20);
+      if (__shfl_sync(0xFFFFFFFFu, it, 0) >= (1u << 24)) {
+        if (lane == 0) atomicExch(a.status, 6);
+        return;
+      }
+      __threadfence_block();
+      const Unit u = list[k % kListSlots];
+      if (u.nt == 0) break;
+      const bool shared = u.flags & 1, copies = !(u.flags & 2) && t < u.nt;
+      int row = u.slot0 + t;
+      if (copies && !shared && a.rows != nullptr) row = __ldg(a.rows + row);
+      const unsigned char* src = (shared ? a.sxq : a.xq) + static_cast<size_t>(row) * xrow;
+      const int mine = u.flags & 2 ? 0 : (u.nt - x + kXWarps - 1) / kXWarps;     // rows of this warp
+#pragma unroll 1
+      for (int b = 0; b < a.nb; ++b, src += kRowBlk) {
+        if (!wait(&xempty[s], ph ^ 1u)) return;
+        if (lane == 0) {
+          if (mine > 0) mbar_expect_tx(&full[s], mine * kRowBlk);
+          else mbar_arrive_one(&full[s]);
+        }
+        __syncwarp();
+        if (copies) bulk_g2s(smem + kHdr + s * kStageBytes + kWBytes + t * kXRow, src, kRowBlk, &full[s]);
+        advance();
+      }
+    }
+    if (!wait(&xempty[s], ph ^ 1u)) return;
+    if (lane == 0) mbar_arrive_one(&full[s]);
+  } else {
+    // ---------------- consumers: sixteen rows each ----------------
+    float acc[4][4];
+    const int gid = lane >> 2, tig = lane & 3;
+    // unit u of the sixteen: gate rows 0 .. 7 and the up rows of the same indices, or sixteen adjacent rows
+    auto row_at = [&](int u) { return DUAL ? ((u & 7) + 8 * warp) * kW4 + (u >> 3) * kHalfBytes : (16 * warp + u) * kW4; };
+    const int w_off = row_at((lane & 7) + ((lane >> 3) & 1) * 8) + 16 + (lane >> 4) * 16, own_lo = row_at(gid), own_hi = row_at(gid + 8);
+    for (;; advance()) {
+      if (!wait(&full[s], ph)) return;
+      const Desc d = desc[s];
+      if (d.flags >> 12 & 1) break;
+      const int nt = d.flags & 255;
+      unsigned char* st = smem + kHdr + s * kStageBytes;
+      if (d.flags >> 8 & 1) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[n][j] = 0.f;
+      }
+      auto loaded = [&] {
+        __syncwarp();
+        if (lane == 0) mbar_arrive_one(&wempty[s]);
+      };
+      if (d.flags >> 10 & 1) loaded();
+      else if (nt <= 8) rows_block<1>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
+      else if (nt <= 16) rows_block<2>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
+      else if (nt <= 24) rows_block<3>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
+      else rows_block<4>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
+      __syncwarp();
+      if (lane == 0) mbar_arrive_one(&xempty[s]);
+      if (!(d.flags >> 9 & 1)) continue;
+      // ---- the unit is complete for this warp's rows: the lanes of two neighbouring rows trade halves, so that a
+      // store is two rows of one token ----
+      uint16_t* y = (d.flags >> 11 & 1) ? a.sy : a.y;
+      const int odd = gid & 1;
+      const uint32_t sel = odd ? 0x3276u : 0x5410u;
+      const int row = d.group * (DUAL ? 128 : 256) + (DUAL ? 8 : 16) * warp + gid - odd;
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        if (8 * n >= nt) break;
+        const int t = 8 * n + 2 * tig + odd;
+        uint16_t* o = y + static_cast<size_t>(d.slot0 + t) * a.n_rows + row;
+        const __half2 lo = __floats2half2_rn(acc[n][0], acc[n][1]), hi = __floats2half2_rn(acc[n][2], acc[n][3]);
+        auto trade = [&](__half2 v) {
+          const uint32_t mine = *reinterpret_cast<const uint32_t*>(&v);
+          return __byte_perm(mine, __shfl_xor_sync(0xFFFFFFFFu, mine, 4), sel);
+        };
+        if (DUAL) {
+          const uint32_t h = trade(__floats2half2_rn(silu_mul(__low2float(lo), __low2float(hi)), silu_mul(__high2float(lo), __high2float(hi))));
+          if (t < nt) *reinterpret_cast<uint32_t*>(o) = h;
+        } else {
+          const uint32_t v0 = trade(lo), v1 = trade(hi);
+          if (t < nt) {
+            *reinterpret_cast<uint32_t*>(o) = v0;
+            *reinterpret_cast<uint32_t*>(o + 8) = v1;
+          }
+        }
+      }
+    }
+  }
+}
+
+template <bool DUAL>
+int launch_rows(RowsArgs a, cudaStream_t stream) {
+  a.status = status_word();
+  const int sms = device_sms();
+  if (a.status == nullptr || sms <= 0) return kErrLaunch;
+  a.groups = a.n_rows / (DUAL ? 128 : 256);
+  a.s_items = 0;
+  if (a.sw0 != nullptr && a.s_rows > 0) {
+    const int passes = (a.s_rows + kTok - 1) / kTok;
+    a.s_step = ((a.s_rows + passes - 1) / passes + 7) & ~7;
+    a.s_items = a.groups * ((a.s_rows + a.s_step - 1) / a.s_step);
+  }
+  const long long n_items = static_cast<long long>(a.groups) * a.n_expert + a.s_items;
+  if (n_items > 0x7FFFFFFF) return kErrUnsupported;
+  a.n_items = static_cast<int>(n_items);
+  if (!opt_in_smem<grouped_gemm_rows_kernel<DUAL>>(kSmem)) return kErrLaunch;
+  return launch_pdl(grouped_gemm_rows_kernel<DUAL>, dim3(std::min(a.n_items, sms)), kThreads, kSmem, stream, a);
+}
+
+// Rows of fp16 values -> Q8_K rows in blocks of kRowBlk bytes, two slabs
+// in one launch, the first bounded by *d_rows on the device; and, in CTAs of their own (map_ctas of them), the descriptors of every
+// expert's three matrices. One warp per block or expert.
+constexpr int kQuantWarps = 4;
+struct MapArgs {
+  unsigned* counters;                  // of the GEMM launches, cleared
+  const unsigned char* const* tab;     // [3][stride]
+  long long stride;
+  unsigned char* maps;
+  const unsigned char* shared[3];
+  int n_expert;
+  alignas(16) uint32_t up[32], down[32];
+};
+__global__ void __launch_bounds__(kQuantWarps * 32)
+quantize_rows_kernel(const uint16_t* __restrict__ x0, unsigned char* __restrict__ out0, long long n0, const int* __restrict__ d_rows,
+                     const uint16_t* __restrict__ x1, unsigned char* __restrict__ out1, long long n1, int nb, unsigned map_ctas,
+                     const __grid_constant__ MapArgs m) {
+  __shared__ __align__(128) unsigned char patch[kQuantWarps][3][128];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && threadIdx.x < 4) m.counters[threadIdx.x] = 0u;
+  if (blockIdx.x < map_ctas) {
+    const int e = blockIdx.x * kQuantWarps + warp;
+    if (e > m.n_expert) return;
+    const unsigned char* w[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      w[i] = e == m.n_expert ? m.shared[i] : m.tab[i * m.stride + e];
+      reinterpret_cast<uint32_t*>(patch[warp][i])[lane] = i < 2 ? m.up[lane] : m.down[lane];
+    }
+    __syncwarp();
+    // (a base that is absent or off a 16-byte boundary keeps the placeholder: its descriptor is not used)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (lane == i && w[i] != nullptr && (reinterpret_cast<uintptr_t>(w[i]) & 15u) == 0) tmap_replace_addr(patch[warp][i], w[i]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 3; ++i) tmap_publish(m.maps + (static_cast<size_t>(e) * 3 + i) * 128, patch[warp][i]);
+    return;
+  }
+  long long b = static_cast<long long>(blockIdx.x - map_ctas) * kQuantWarps + warp;
+  const uint16_t* x = x0;
+  unsigned char* out = out0;
+  if (b >= n0) {
+    b -= n0;
+    if (b >= n1) return;
+    x = x1;
+    out = out1;
+  } else if (d_rows != nullptr && b >= static_cast<long long>(*d_rows) * nb) {
+    return;
+  }
+  float v[8];
+  load_lane8(x + b * kQK, lane, v);
+  int q[8], sum;
+  const float d = quantize_lane8(v, q, sum);
+  uint32_t* o32 = reinterpret_cast<uint32_t*>(out + b * kRowBlk);
+  auto pack = [&](int i) {
+    return (q[i] & 0xFF) | ((q[i + 1] & 0xFF) << 8) | ((q[i + 2] & 0xFF) << 16) | (static_cast<uint32_t>(q[i + 3] & 0xFF) << 24);
+  };
+  if (lane == 0) o32[0] = __float_as_uint(d);
+  *reinterpret_cast<uint2*>(o32 + 4 + 2 * lane) = make_uint2(pack(0), pack(4));
+  if ((lane & 3) == 0) {                           // sub-block lane / 4
+    unsigned char* parts = reinterpret_cast<unsigned char*>(o32 + 68) + (lane >> 4) * 8 + ((lane >> 2) & 3);
+    parts[0] = static_cast<unsigned char>(sum & 127);
+    parts[4] = static_cast<unsigned char>((sum >> 7) & 0xFF);
+  }
+}
+
+unsigned* counters_of(const void* maps, int n_expert) {
+  return reinterpret_cast<unsigned*>(static_cast<unsigned char*>(const_cast<void*>(maps)) + (n_expert + 1LL) * 384);
+}
+RowsArgs args_of(const ExpertGemm& g, const void* maps, int map0) {
+  RowsArgs a{};
+  a.maps = static_cast<const unsigned char*>(maps);
+  a.next = counters_of(maps, g.n_expert) + map0;
+  a.tab0 = g.tab; a.map0 = map0; a.off = g.off; a.rows = g.rows; a.xq = g.xq; a.y = g.y;
+  a.n_rows = g.n_rows; a.nb = g.k / kQK; a.n_expert = g.n_expert;
+  a.sw0 = a.sw1 = static_cast<const unsigned char*>(g.shared_w);
+  a.sxq = g.shared_xq; a.sy = g.shared_y; a.s_rows = g.shared_rows;
+  return a;
+}
+
+}  // namespace
+
+int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, const void* maps, cudaStream_t stream) {
+  RowsArgs a = args_of(g, maps, 0);
+  a.tab1 = tab_up;
+  a.sw1 = static_cast<const unsigned char*>(shared_up);
+  return launch_rows<true>(a, stream);
+}
+int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream) { return launch_rows<false>(args_of(g, maps, 2), stream); }
+
+int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_rows, const uint16_t* x1, void* out1, long long rows1,
+                  int k, const ExpertMaps& em, bool make_maps, cudaStream_t stream) {
+  const int nb = k / kQK;
+  const long long ctas = ((rows0 + rows1) * nb + kQuantWarps - 1) / kQuantWarps;
+  MapArgs m{};
+  unsigned map_ctas = 0;
+  m.counters = counters_of(em.maps, em.n_expert);
+  if (make_maps) {
+    m.tab = em.tab; m.stride = em.stride; m.maps = static_cast<unsigned char*>(em.maps); m.n_expert = em.n_expert;
+    for (int i = 0; i < 3; ++i) m.shared[i] = static_cast<const unsigned char*>(em.shared[i]);
+    if (!matrix_tmap(em.hidden / kQK * kW4, em.n_ff, em.maps, m.up) || !matrix_tmap(em.n_ff / kQK * kW4, em.hidden, em.maps, m.down))
+      return kErrUnsupported;
+    map_ctas = static_cast<unsigned>(em.n_expert / kQuantWarps + 1);
+  }
+  if (ctas + map_ctas > 0x7FFFFFFF) return kErrUnsupported;
+  if (ctas + map_ctas == 0) return kOk;
+  return launch_pdl(quantize_rows_kernel, dim3(static_cast<unsigned>(ctas + map_ctas)), kQuantWarps * 32, 0, stream, x0,
+                    static_cast<unsigned char*>(out0), rows0 * nb, d_rows, x1, static_cast<unsigned char*>(out1), rows1 * nb, nb, map_ctas, m);
+}
+
+}  // namespace sgr

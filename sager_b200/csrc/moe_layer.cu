@@ -38,6 +38,7 @@
 #include "quantize_dev.cuh"
 #include "router_dev.cuh"
 #include "tile.cuh"
+#include "tmap_dev.cuh"
 
 namespace sgr {
 
@@ -1183,10 +1184,20 @@ __global__ void ep_step_kernel(unsigned* step) {
 }
 
 
-// A 2-D TMA descriptor over a Q4_K matrix seen as bytes, [rows][row_bytes], with boxes of
-// one super-block column (144 bytes) x 128 rows, encoded for a placeholder address: the
-// expert kernel patches the real base address in on the device. Encoded once per
-// geometry (cuTensorMapEncodeTiled, reached through the runtime's driver entry point).
+// Polls (64 ns apart) after which a kernel that waits for a peer's arrival words gives up.
+std::atomic<unsigned> g_wait_limit{1u << 22};
+
+template <auto K>
+int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const LayerDev& L) {
+  if (smem > 32 * 1024 &&     // (static shared memory counts towards the 48 KB default limit)
+      !opt_in_smem<K>(static_cast<int>(smem)))
+    return kErrLaunch;
+  return launch_pdl(K, grid, threads, smem, stream, L);
+}
+
+}  // namespace
+
+// (tmap_dev.cuh; cuTensorMapEncodeTiled is reached through the runtime's driver entry point)
 bool matrix_tmap(int row_bytes, int rows, const void* placeholder, uint32_t* out128) {
   struct Entry { int row_bytes, rows; unsigned char bytes[128]; };
   static std::mutex mu;
@@ -1229,19 +1240,6 @@ bool matrix_tmap(int row_bytes, int rows, const void* placeholder, uint32_t* out
   }
   return true;
 }
-
-// Polls (64 ns apart) after which a kernel that waits for a peer's arrival words gives up.
-std::atomic<unsigned> g_wait_limit{1u << 22};
-
-template <auto K>
-int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const LayerDev& L) {
-  if (smem > 32 * 1024 &&     // (static shared memory counts towards the 48 KB default limit)
-      !opt_in_smem<K>(static_cast<int>(smem)))
-    return kErrLaunch;
-  return launch_pdl(K, grid, threads, smem, stream, L);
-}
-
-}  // namespace
 }  // namespace sgr
 
 using namespace sgr;

@@ -24,6 +24,10 @@
 using namespace sgr;
 
 namespace {
+// Up to this many routed rows per expert on average the row-streaming GEMM takes the expert stage: its work grows with the rows,
+// the tcgen05 form's with the weights. Two layers of 2048 / 512 / 256 experts, us: 3 rows per expert 255 against 405 for the
+// tcgen05 form, 8 314 / 464, 16 423 / 532, 24 553 / 579, 28 625 / 611; of 1024 / 512 / 128: 16 170 / 190, 24 200 / 204.
+constexpr int kFewRows = 24;
 // x[row] += sum_k w[row][k] * y_grouped[gslot[row][k]] (k = 0 .. K-1, in this order; a route that was
 // not computed, gslot < 0, adds nothing) + w[row][K] * sh_y[row] (when there is a shared expert):
 // scatter_routed_f16 + the strided copy + moe_combine_batched_f16 of the reference's sequence
@@ -87,29 +91,49 @@ __global__ void combine_grouped_kernel(uint16_t* __restrict__ x, const uint16_t*
   }
 }
 
-// The rows the GEMMs read: ready operands in the combine slab's memory when they fit there (FFN up to about
-// 0.8 x hidden at top-8), otherwise Q8_K rows from which the GEMMs make their operands themselves.
+inline bool has_shared(const sgr_moe_prefill* a) { return a->shared_gate && a->shared_up && a->shared_down; }
+
+// The rows the GEMMs read lie in the combine slab's memory when they fit there: Q8_K rows in padded blocks and the expert
+// descriptors for the kernel of few token rows per expert, ready operands for the tcgen05 one (FFN up to about 0.8 x hidden
+// at top-8); otherwise Q8_K rows from which the tcgen05 GEMMs make their operands themselves.
+enum class Rows { kPadded, kOperands, kPacked };
 struct OperandRows {
-  bool ready;
+  Rows form;
   unsigned char *x, *h, *s;       // layer input, routed h, shared expert's h
+  unsigned char* maps;
 };
 OperandRows operand_rows(const sgr_moe_prefill* a) {
-  const long long nbh = a->hidden / kQK, nbf = a->n_ff / kQK, x = a->n * nbh * kOpBlk,
-                  h = static_cast<long long>(a->n) * a->n_used * nbf * kOpBlk, s = a->n * nbf * kOpBlk;
+  const long long nbh = a->hidden / kQK, nbf = a->n_ff / kQK, room = static_cast<long long>(a->n_max) * (a->n_used + 1) * a->hidden * 2;
   unsigned char* slab = reinterpret_cast<unsigned char*>(a->expert_y);
-  if ((reinterpret_cast<uintptr_t>(slab) & 15u) == 0 &&
-      x + h + s <= static_cast<long long>(a->n_max) * (a->n_used + 1) * a->hidden * 2)
-    return {true, slab, slab + x, slab + x + h};
-  return {false, static_cast<unsigned char*>(a->xq), static_cast<unsigned char*>(a->hq), static_cast<unsigned char*>(a->sh_q)};
+  const uintptr_t at = reinterpret_cast<uintptr_t>(slab);
+  auto laid = [&](Rows form, long long blk, long long front) {
+    const long long x = a->n * nbh * blk, h = static_cast<long long>(a->n) * a->n_used * nbf * blk, s = a->n * nbf * blk;
+    unsigned char* base = slab + front;
+    return OperandRows{front + x + h + s <= room ? form : Rows::kPacked, base, base + x, base + x + h, slab + (-at & 127u)};
+  };
+  const uintptr_t outs = reinterpret_cast<uintptr_t>(a->g) | reinterpret_cast<uintptr_t>(a->y_grouped) |
+                         reinterpret_cast<uintptr_t>(a->sh_g) | reinterpret_cast<uintptr_t>(a->sh_y);
+  if ((at & 15u) == 0 && (outs & 3u) == 0 && static_cast<long long>(a->n) * a->n_used <= static_cast<long long>(kFewRows) * a->n_expert) {
+    const OperandRows r = laid(Rows::kPadded, kRowBlk, (-at & 127u) + (a->n_expert + 1LL) * 384 + 16);
+    if (r.form == Rows::kPadded) return r;
+  }
+  if ((at & 15u) == 0) {
+    const OperandRows r = laid(Rows::kOperands, kOpBlk, 0);
+    if (r.form == Rows::kOperands) return r;
+  }
+  return {Rows::kPacked, static_cast<unsigned char*>(a->xq), static_cast<unsigned char*>(a->hq), static_cast<unsigned char*>(a->sh_q), nullptr};
 }
-
-inline bool has_shared(const sgr_moe_prefill* a) { return a->shared_gate && a->shared_up && a->shared_down; }
 
 // the combine reads the grouped rows in place when every buffer allows 16-byte accesses
 bool combines_in_place(const sgr_moe_prefill* a) {
   return (a->hidden & 7) == 0 && a->n_used <= 1024 &&
          ((reinterpret_cast<uintptr_t>(a->x_f16) | reinterpret_cast<uintptr_t>(a->y_grouped) |
            (has_shared(a) ? reinterpret_cast<uintptr_t>(a->sh_y) : 0)) & 15u) == 0;
+}
+
+ExpertMaps expert_maps(const sgr_moe_prefill* a, const OperandRows& op) {
+  return {reinterpret_cast<const unsigned char* const*>(a->w_tab), a->tab_stride > 0 ? a->tab_stride : a->n_expert, op.maps,
+          {a->shared_gate, a->shared_up, a->shared_down}, a->n_expert, a->hidden, a->n_ff};
 }
 
 // gate / up, SwiGLU, requantise, down of the routed experts and of the shared one
@@ -119,18 +143,25 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   const long long ts = a->tab_stride > 0 ? a->tab_stride : E, R = static_cast<long long>(a->n_max) * K;
   auto tab = [&](int m) { return reinterpret_cast<const unsigned char* const*>(a->w_tab + m * ts); };
   ExpertGemm up{};
-  up.tab = tab(0); up.off = a->off; up.rows = a->grows; up.xq = op.x; up.operand_rows = op.ready;
+  up.tab = tab(0); up.off = a->off; up.rows = a->grows; up.xq = op.x; up.operand_rows = op.form == Rows::kOperands;
   up.y = a->g; up.n_rows = F; up.k = H; up.n_expert = E;
   ExpertGemm down{};
-  down.tab = tab(2); down.off = a->off; down.xq = op.h; down.operand_rows = op.ready;
+  down.tab = tab(2); down.off = a->off; down.xq = op.h; down.operand_rows = up.operand_rows;
   down.y = a->y_grouped; down.n_rows = H; down.k = F; down.n_expert = E;
   if (shared) {
     up.shared_w = a->shared_gate; up.shared_xq = op.x; up.shared_y = a->sh_g; up.shared_rows = n;
     down.shared_w = a->shared_down; down.shared_xq = op.s; down.shared_y = a->sh_y; down.shared_rows = n;
   }
-  int rc = gemm_gate_up(up, tab(1), a->u, a->shared_up, a->sh_u, stream);
+  int rc;
+  if (op.form == Rows::kPadded) {              // SwiGLU happens in the GEMM
+    rc = gemm_rows_gate_up(up, tab(1), a->shared_up, op.maps, stream);
+    if (rc == kOk)
+      rc = quantize_rows(a->g, op.h, static_cast<long long>(n) * K, a->meta, a->sh_g, op.s, shared ? n : 0, F, expert_maps(a, op), false, stream);
+    return rc == kOk ? gemm_rows_down(down, op.maps, stream) : rc;
+  }
+  rc = gemm_gate_up(up, tab(1), a->u, a->shared_up, a->sh_u, stream);
   if (rc != kOk) return rc;
-  if (op.ready) {
+  if (op.form == Rows::kOperands) {
     rc = quantize_operand(a->g, a->u, op.h, static_cast<long long>(n) * K, a->meta, a->sh_g, a->sh_u, op.s, shared ? n : 0, F, stream);
   } else {
     rc = sgr_silu_mul_f16_n(a->g, a->g, a->u, a->meta, static_cast<int>(R), F, stream);
@@ -146,7 +177,7 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
 SGR_API int sgr_moe_prefill_expert_stage(const sgr_moe_prefill* a, void* stream) {
   if (a == nullptr) return kErrArg;
   const OperandRows op = operand_rows(a);
-  if (op.ready && !combines_in_place(a)) return kErrUnsupported;      // the combine's slab lies where the operand rows were
+  if (op.form != Rows::kPacked && !combines_in_place(a)) return kErrUnsupported;      // the combine's slab lies where the operand rows were
   return expert_stage(a, op, as_stream(stream));
 }
 
@@ -175,7 +206,9 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
   int rc;
 #define SGR_STEP(call) do { rc = (call); if (rc != kOk) return rc; } while (0)
   const OperandRows op = operand_rows(a);
-  if (op.ready) SGR_STEP(quantize_operand(a->xn, nullptr, op.x, n, nullptr, nullptr, nullptr, nullptr, 0, H, as_stream(stream)));
+  if (op.form == Rows::kPadded) {
+    SGR_STEP(quantize_rows(a->xn, op.x, n, nullptr, nullptr, nullptr, 0, H, expert_maps(a, op), true, as_stream(stream)));
+  } else if (op.form == Rows::kOperands) SGR_STEP(quantize_operand(a->xn, nullptr, op.x, n, nullptr, nullptr, nullptr, nullptr, 0, H, as_stream(stream)));
   else SGR_STEP(sgr_quantize_q8_k(a->xn, a->xq, static_cast<long long>(n) * H, stream));
   const float* logits = a->logits_in;
   if (logits == nullptr) {

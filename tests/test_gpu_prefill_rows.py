@@ -1,0 +1,118 @@
+"""The prefill chunk's expert stage for few token rows per expert (row-streaming GEMM) against the launchers it joins: grouped
+GEMM on gathered rows, SwiGLU, quantiser. Integer sums and fp32 steps are the same on both paths: equal to the bit."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from sager_b200 import lib, ops, synth
+from sager_b200.ops import stream_ptr
+from sager_b200.layer import PrefillLayer
+from tests.util import DEV, dev
+
+pytestmark = pytest.mark.gpu
+
+
+def quantize_dev(x16):
+    n, k = x16.shape
+    out = torch.zeros(n, k // 256 * 276, dtype=torch.uint8, device=DEV)
+    ops.quantize_q8_k(x16, out, n * k)
+    return out
+
+
+def launchers(tabs, off, grows, x16, R, H, F, E):
+    """y of the routed rows through the separate launchers; tabs: three [E] pointer tables."""
+    xqg = torch.zeros(R, H // 256 * 276, dtype=torch.uint8, device=DEV)
+    ops.gather_rows_q8(xqg, quantize_dev(x16), grows, R, H // 256)
+    g, u, y = (torch.zeros(R, d, dtype=torch.float16, device=DEV) for d in (F, F, H))
+    ops.moe_grouped_gemm_i8(tabs[0], off, xqg, g, F, H, E)
+    ops.moe_grouped_gemm_i8(tabs[1], off, xqg, u, F, H, E)
+    ops.silu_mul_f16(g, g, u, R, F)
+    ops.moe_grouped_gemm_i8(tabs[2], off, quantize_dev(g), y, H, F, E)
+    return y
+
+
+def chosen_logits(counts, n, seed):
+    """Router logits (top-1) that give expert e counts[e] of the rows, in shuffled order."""
+    e = np.repeat(np.arange(len(counts)), counts)
+    assert len(e) == n
+    np.random.default_rng(seed).shuffle(e)
+    logits = np.zeros((n, len(counts)), np.float32)
+    logits[np.arange(n), e] = 5.0
+    return dev(logits)
+
+
+# rows per expert at the edges of the token groups (8, 16, 24, 32), of the passes, none at all
+EDGES = [1, 8, 9, 16, 17, 24, 25, 32, 33, 40, 0, 65, 2, 3, 0, 31]
+
+
+@pytest.mark.parametrize("H,F", [(512, 256), (256, 512), (2048, 512), (512, 768)])
+@pytest.mark.parametrize("shift", [0, 2, 4])
+def test_rows_per_expert(H, F, shift):
+    """shift: bytes by which the experts' blobs lie off a 16-byte boundary."""
+    E, K, n = len(EDGES), 1, sum(EDGES)
+    n_max = n * (1 + 2 * F // H)                # room for the rows and the descriptors
+    w = synth.MoeWeights(H, F, E, DEV, seed=81, std=0.05)
+    big = torch.empty(w.blob.numel() + 16, dtype=torch.uint8, device=DEV)
+    big[shift:shift + w.blob.numel()] = w.blob.reshape(-1)
+    w.blob = big[shift:shift + w.blob.numel()].view(w.n_slots, -1)
+    x16 = synth.normal_fp16((n, H), 82, DEV)
+    L = PrefillLayer(n_max, H, F, E, K, DEV)
+    x = x16.clone()
+    absent = (3,)
+    t = w.table(absent)
+    L.run(n, x16, x, w, t, logits=chosen_logits(EDGES, n, 5))
+    off = L.off.cpu().numpy()
+    assert np.array_equal(np.diff(off), EDGES)
+    y = launchers([t[m].contiguous() for m in range(3)], L.off, L.grows, x16, n, H, F, E)
+    assert torch.equal(L.yg[:n].view(torch.int16), y.view(torch.int16))
+    assert (L.yg[off[3]:off[4]] == 0).all()
+    one = [ops.ptr_table([w.matrix(E, m)], DEV) for m in range(3)]
+    sy = launchers(one, dev(np.int32([0, n])), dev(np.arange(n, dtype=np.int32)), x16, n, H, F, 1)
+    assert torch.equal(L.sh_y[:n].view(torch.int16), sy.view(torch.int16))
+    assert lib().raw("sgr_status")(0) == 0
+    # the expert stage once more on what the call left behind (the hand-out counters start anew)
+    want = L.yg.clone()
+    L.yg.zero_()
+    a = L.args(n, x16, x, w, t, logits=None)
+    lib().call("sgr_moe_prefill_expert_stage", C.byref(a), stream_ptr())
+    assert torch.equal(L.yg[:n].view(torch.int16), want[:n].view(torch.int16))
+
+
+@pytest.mark.parametrize("E,K,n", [(300, 2, 77), (1, 1, 20), (257, 8, 65)])
+def test_many_units(E, K, n):
+    """More experts than a CTA's first round, one expert, no shared expert."""
+    H, F = 512, 256
+    w = synth.MoeWeights(H, F, E, DEV, seed=83, std=0.05, distinct=9)
+    x16 = synth.normal_fp16((n, H), 84, DEV)
+    L = PrefillLayer(4 * n, H, F, E, K, DEV)
+    t = w.table()
+    for shared in (True, False):
+        x = x16.clone()
+        L.run(n, x16, x, w, t, shared=shared)
+        y = launchers([t[m].contiguous() for m in range(3)], L.off, L.grows, x16, n * K, H, F, E)
+        assert torch.equal(L.yg[:n * K].view(torch.int16), y.view(torch.int16)), shared
+    assert lib().raw("sgr_status")(0) == 0
+
+
+def test_saturated_codes():
+    """Codes, scales and nibbles near their largest: block sums beyond 2^24 stay exact integers here (one rounding to fp32 each),
+    so the result is within the fp16 step of the exact one."""
+    H, F, E, K, n = 512, 256, 4, 1, 40
+    rng = np.random.default_rng(3)
+    x = torch.from_numpy(rng.choice([-1.0, 1.0], (n, 1)) * rng.uniform(0.9, 1.0, (n, H))).half().to(DEV)
+    w = synth.MoeWeights(H, F, E, DEV, seed=85, std=0.05)
+    blob = w.blob.view(w.n_slots, -1, 144)
+    blob[:, :, 0:4] = dev(np.frombuffer(np.float16([2.0 ** -14, 0.0]).tobytes(), np.uint8).copy())
+    blob[:, :, 4:] = 0xFF
+    L = PrefillLayer(4 * n, H, F, E, K, DEV)
+    L.run(n, x, x.clone(), w, w.table(), logits=chosen_logits([10] * 4, n, 6))
+    xq = quantize_dev(x).cpu().numpy().reshape(n, H // 256, 276)
+    d = xq[..., 0:4].copy().view(np.float32)[..., 0].astype(np.float64)
+    codes = xq[..., 4:260].view(np.int8).astype(np.int64)
+    g = (d * codes.sum(2) * 63 * 15 * 2.0 ** -14).sum(1)         # gate and up alike, every row
+    h = (g / (1 + np.exp(-g)) * g)
+    got = L.g[:n].double().cpu().numpy()[np.argsort(L.grows[:n].cpu().numpy())]
+    # g to fp16 (2^-11), h = silu(g) g: its relative error is at most (2 + |g|) times that of g, and rounded itself
+    assert (np.abs(got - h[:, None]) <= (np.abs(h) * (3 + np.abs(g)) * 2.0 ** -11 + 1e-6)[:, None]).all()
