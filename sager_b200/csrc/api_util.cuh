@@ -58,6 +58,16 @@ int launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cuda
 // (bsum = 64 * hi + lo), the fp32 scale, 12 bytes of padding. 16-byte aligned.
 constexpr int kOpBlk = 560;
 
+// TMA descriptors of a layer's experts, which quantize_operand or quantize_rows makes: [n_expert + 1][3] of 128 bytes (gate, up,
+// down; the shared expert's last), then 16 bytes of counters.
+struct ExpertMaps {
+  const unsigned char* const* tab;     // [3][stride]
+  long long stride;
+  void* maps;                          // 128-byte aligned
+  const void* shared[3];
+  int n_expert, hidden, n_ff;
+};
+
 // One more expert (shared_w) that every row of its own slab visits may ride along.
 struct ExpertGemm {
   const unsigned char* const* tab;
@@ -67,6 +77,7 @@ struct ExpertGemm {
   uint16_t* y;
   int n_rows, k, n_expert;
   bool operand_rows;
+  const void* maps;             // with operand rows: the descriptors; n_rows is then a multiple of 128
   const void* shared_w;
   const unsigned char* shared_xq;
   uint16_t* shared_y;
@@ -77,15 +88,7 @@ int gemm_grouped(const ExpertGemm& g, cudaStream_t stream);
 // Its activation rows: kRowBlk bytes per 256 values - fp32 scale, 12 bytes of padding, 256 codes, and the sub-block sums as
 // bsum = 128 * hi + lo: lo of sub-blocks 0-3, hi of 0-3, lo of 4-7, hi of 4-7, a byte each. 16-byte aligned.
 constexpr int kRowBlk = 288;
-// maps: [n_expert + 1][3] descriptors of 128 bytes (gate, up, down; the shared expert's last) and 16 bytes of counters, made and
-// cleared by quantize_rows. n_rows and k multiples of 256, outputs 4-byte aligned.
-struct ExpertMaps {
-  const unsigned char* const* tab;     // [3][stride]
-  long long stride;
-  void* maps;                          // 128-byte aligned
-  const void* shared[3];
-  int n_expert, hidden, n_ff;
-};
+// n_rows and k multiples of 256, outputs 4-byte aligned.
 // gate, up and SwiGLU: y receives h
 int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, const void* maps, cudaStream_t stream);
 int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream);
@@ -97,8 +100,9 @@ int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_
 int gemm_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, uint16_t* y_up, const void* shared_up,
                  uint16_t* shared_y_up, cudaStream_t stream);
 // rows of k fp16 values (SwiGLU of x and u where u is given) -> operand rows; two slabs, the first of at most
-// *d_rows rows when that is given
+// *d_rows rows when that is given; with make_maps the descriptors are made as well
 int quantize_operand(const uint16_t* x0, const uint16_t* u0, void* out0, long long rows0, const int* d_rows,
-                     const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, cudaStream_t stream);
+                     const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, const ExpertMaps& em, bool make_maps,
+                     cudaStream_t stream);
 
 }  // namespace sgr

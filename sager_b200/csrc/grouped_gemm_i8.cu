@@ -26,12 +26,13 @@
 // Persistent: one CTA per SM takes work units round-robin. A unit is one expert, one or several
 // tiles of 128 weight rows, and at most 80 of the expert's token rows; a job is one super-block
 // column of a tile. The roles run as a pipeline over mbarriers:
-//   * two producer warps copy the [128 rows][144 B] block columns into a ring (cp.async; plain loads
-//     where an expert's base is only 2-byte aligned);
+//   * a producer warp brings the [128 rows][144 B] block columns into a ring, one TMA copy each through the expert's
+//     descriptor (made by the quantiser's launch); the plain entry, which has no memory for descriptors, uses two warps and
+//     cp.async. Plain loads where an expert's base is only 2-byte aligned;
 //   * eight unpack warps (thread = weight row; four warps take the even jobs, four the odd ones):
 //     nibbles -> sc * q as packed fp16 with one logic and one FMA instruction per two weights, in
 //     three half-block slots of tensor memory; the min operand and (d, dmin) go to shared memory;
-//   * the activation tiles of one block, two in flight: one warp copies them (cp.async) from rows
+//   * the activation tiles of one block, two in flight: two warps copy them (cp.async) from rows
 //     that already are operands (kOpBlk bytes per block, written by quantize_operand: a prefill
 //     chunk), or eight warps make them from Q8_K rows (the plain entry, which has no scratch; they
 //     cost more instructions than everything else together). Rows of at most two blocks keep their
@@ -53,6 +54,7 @@
 
 #include "api_util.cuh"
 #include "quantize_dev.cuh"
+#include "tmap_dev.cuh"
 #include "umma.cuh"
 
 namespace sgr {
@@ -60,7 +62,9 @@ namespace {
 
 constexpr int kGemmRows = 128;                    // weight rows per tile = MMA M = tensor-memory lanes
 constexpr int kGemmTok = 80;                      // token rows per unit = max MMA N
-constexpr int kStages = 7, kStageBytes = kGemmRows * kW4;     // 18,432
+// (Four stages: a fifth to seventh hides nothing more, and what shared memory does not take is L1 cache - 2048 rows, two layers:
+// 892 us with seven, 876 with four. With two producers on cp.async and one stager it was 913.)
+constexpr int kStages = 4, kStageBytes = kGemmRows * kW4;     // 18,432
 constexpr int kBTile = kGemmTok * 32;             // one K = 16 step of the activations
 constexpr int kBBytes = 17 * kBTile;              // 16 code steps + the split sums
 constexpr int kMinBytes = kGemmRows * 32;         // the min operand of a job
@@ -68,8 +72,8 @@ constexpr int kTmemCols = 512;                    // two accumulator sets of 2 x
 constexpr int kColSet = 2 * kGemmTok, kColA = 2 * kColSet, kASlots = 3;
 static_assert(kColA + 64 * kASlots <= kTmemCols, "tensor memory");
 
-// warps: epilogue | MMA, two producers, copying stager | unpack | converting stagers
-constexpr int kEpiWarps = 8, kWarpMma = kEpiWarps, kWarpProd0 = kEpiWarps + 1, kWarpUnpack0 = kEpiWarps + 4,
+// warps: epilogue | MMA, and three that copy: two producers (RAW) or one producer and two stagers | unpack | converting stagers
+constexpr int kEpiWarps = 8, kWarpMma = kEpiWarps, kWarpProd0 = kEpiWarps + 1, kCopyStagers = 2, kWarpUnpack0 = kEpiWarps + 4,
               kUnpackGroups = 2, kWarpStage0 = kWarpUnpack0 + 4 * kUnpackGroups, kStageWarps = 8;
 // Threads and registers per thread of each role (setmaxnreg). The sum over the warpgroups is at most
 // what the launch holds.
@@ -108,6 +112,8 @@ struct GemmArgs {
   uint16_t *sy, *sy1;
   int s_rows, s_step, s_items;         // its rows, rows per unit, units
   int n_items;
+  const unsigned char* maps;           // (operand rows) [n_expert + 1][3] descriptors; the matrix of tab0 is map0
+  int map0;
   int* status;
 };
 
@@ -121,6 +127,7 @@ struct Unit {
   const int* rows;
   uint16_t *y, *y1;
   int tile0, n_tiles;                  // row tiles
+  int expert;
   int slot0, nt, n_mma;                // first slot, token rows, MMA N
 };
 struct Walk {
@@ -136,7 +143,7 @@ struct Walk {
       u.tile0 = (i - e * a.groups) * a.group;
       u.n_tiles = min(a.group, a.tiles - u.tile0);
       if (shared) {
-        u.w0 = a.sw0; u.w1 = a.sw1; u.xq = a.sxq; u.rows = nullptr; u.y = a.sy; u.y1 = a.sy1;
+        u.w0 = a.sw0; u.w1 = a.sw1; u.xq = a.sxq; u.rows = nullptr; u.y = a.sy; u.y1 = a.sy1; u.expert = a.n_expert;
         u.slot0 = e * a.s_step;
         u.nt = min(a.s_step, a.s_rows - u.slot0);
         it += gridDim.x;
@@ -152,7 +159,7 @@ struct Walk {
           const int passes = (m + kGemmTok - 1) / kGemmTok;
           step = ((m + passes - 1) / passes + 15) & ~15;
         }
-        u.w0 = w0; u.w1 = w1; u.xq = a.xq; u.rows = a.rows; u.y = a.y; u.y1 = a.y1;
+        u.w0 = w0; u.w1 = w1; u.xq = a.xq; u.rows = a.rows; u.y = a.y; u.y1 = a.y1; u.expert = e;
         u.slot0 = slot + t0;
         u.nt = min(step, m - t0);
         t0 += step;
@@ -193,10 +200,10 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
   static_assert(kBarCount * 8 <= 512, "barriers");
 
   if (tid == 0) {
-    for (int i = 0; i < kStages; ++i) { mbar_init(&bar[kBarWFull + i], 32); mbar_init(&bar[kBarWEmpty + i], 4); }
+    for (int i = 0; i < kStages; ++i) { mbar_init(&bar[kBarWFull + i], RAW ? 32 : 1); mbar_init(&bar[kBarWEmpty + i], 4); }
     for (int i = 0; i < kASlots; ++i) { mbar_init(&bar[kBarAFull + i], 4); mbar_init(&bar[kBarAEmpty + i], 1); }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(&bar[kBarBFull + i], RAW ? kStageWarps : 32); mbar_init(&bar[kBarBEmpty + i], 1);
+      mbar_init(&bar[kBarBFull + i], RAW ? kStageWarps : 32 * kCopyStagers); mbar_init(&bar[kBarBEmpty + i], 1);
       mbar_init(&bar[kBarAccFull + i], 1); mbar_init(&bar[kBarAccFull + 2 + i], 1);
       mbar_init(&bar[kBarAccEmpty + i], kEpiWarps / 2);
     }
@@ -442,7 +449,42 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
       }
       if (elect_one()) umma_commit(&bar[kBarDrain]);             // everything issued has finished before tensor memory goes back
       mbar_wait_tight(&bar[kBarDrain], 0);
-    } else if (warp < kWarpProd0 + 2) {
+    } else if (!RAW && warp == kWarpProd0) {
+      // ---------------- producer: a block column of 128 rows is one TMA copy ----------------
+      unsigned st = 0, st_ph = 1;
+      while (wk.next<DUAL>(a, u)) {
+        if (u.w0 == nullptr) continue;
+        const uintptr_t align = (reinterpret_cast<uintptr_t>(u.w0) | reinterpret_cast<uintptr_t>(u.w1)) & 15u;
+        const unsigned char* map = a.maps + (static_cast<size_t>(u.expert) * 3 + a.map0) * 128;
+        if (align == 0 && lane == 0) {
+          tmap_acquire(map);
+          if (DUAL) tmap_acquire(map + 128);
+        }
+        const bool ok = for_jobs<DUAL>(a, u, [&](int t, int b, int m, int) {
+          const unsigned s = st;
+          if (!wait_warp(kBarWEmpty + s, st_ph)) return false;
+          if (++st == kStages) { st = 0; st_ph ^= 1u; }
+          unsigned char* stage = smem + kOffW + s * kStageBytes;
+          const int row0 = (u.tile0 + t) * kGemmRows;
+          if (align == 0) {
+            if (lane == 0) {
+              mbar_expect_tx(&bar[kBarWFull + s], kStageBytes);
+              tma_load_box(stage, map + 128 * m, b * kW4, row0, &bar[kBarWFull + s]);
+            }
+          } else {                                               // a base off a 16-byte boundary
+            const unsigned char* src = (m == 0 ? u.w0 : u.w1) + static_cast<size_t>(row0) * row_bytes + b * kW4;
+            warp_copy_unaligned(stage, kStageBytes / 16, lane, align, [&](int p) { return src + p / 9 * row_bytes + p % 9 * 16; });
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            fence_proxy_async();                                 // the next fill of the stage may be a TMA copy
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(&bar[kBarWFull + s]);
+          }
+          __syncwarp();
+          return true;
+        });
+        if (!ok) break;
+      }
+    } else if (RAW && warp < kWarpProd0 + 2) {
       // ---------------- producers: block columns of 128 rows into the ring, alternate jobs ----------------
       // 16-byte piece p = 9 * row + c of a stage goes to lane p % 32; nine steps of 32 pieces are 32 rows, so a lane
       // keeps the source offsets of nine steps.
@@ -491,12 +533,13 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
       }
       asm volatile("cp.async.wait_all;" ::: "memory");
     } else if constexpr (!RAW) {
-      // ---------------- copying stager: operand rows of one block, 16 bytes per lane and step ----------------
-      // lane = (row of eight, one of four 16-byte pieces); a group of eight rows is 8.5 steps
-      const int r8 = lane & 7, pc = lane >> 3;
+      // ---------------- copying stagers: operand rows of one block, 16 bytes per lane and step ----------------
+      // lane = (row of eight, one of four 16-byte pieces); each warp takes half of a row's codes, the first one the split sums
+      // too and the second one the scales
+      const int half = warp - kWarpProd0 - 1, r8 = lane & 7, pc = lane >> 3;
       constexpr int kGroups = kGemmTok / 8, kGroups32 = (kGemmTok + 31) / 32;
       const size_t xrow_bytes = static_cast<size_t>(a.nb) * kOpBlk;
-      const uint32_t lane_dst = smem_u32(smem + kOffB) + (pc >> 1) * kBTile + tile_at(r8, pc & 1);
+      const uint32_t lane_dst = smem_u32(smem + kOffB) + (pc >> 1) * kBTile + tile_at(r8, pc & 1);      // (of the first half)
       const uint32_t xd_dst = smem_u32(smem + kOffXd) + lane * 4;
       unsigned fill = 0;
       while (wk.next<DUAL>(a, u)) {
@@ -524,12 +567,12 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
             if (g * 8 < u.n_mma) {
               const unsigned char* xb = src + __shfl_sync(0xFFFFFFFFu, row[g / 4], (g & 3) * 8 + r8) * xrow_bytes + pc * 16;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) cp_async16(dst + g * 256 + q * 2 * kBTile, xb + q * 64);
-              if (pc < 2) cp_async16(dst + g * 256 + 16 * kBTile, xb + 512);
+              for (int q = 0; q < 4; ++q) cp_async16(dst + half * 8 * kBTile + g * 256 + q * 2 * kBTile, xb + half * 256 + q * 64);
+              if (half == 0 && pc < 2) cp_async16(dst + g * 256 + 16 * kBTile, xb + 512);
             }
 #pragma unroll
           for (int g = 0; g < kGroups32; ++g)
-            if (g * 32 + lane < u.n_mma)
+            if (half == 1 && g * 32 + lane < u.n_mma)
               asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(xd_dst + ((fill & 3) * kGemmTok + g * 32) * 4),
                            "l"(src + row[g] * xrow_bytes + 544)
                            : "memory");
@@ -662,18 +705,25 @@ int launch_gemm(GemmArgs a, cudaStream_t stream) {
 
 // Rows of fp16 values - or SwiGLU of two rows, rounded to fp16 as silu_mul_f16 does - -> operand rows
 // (api_util.cuh): the Q8_K quantiser of quantize_block_f16 with the codes, the split sums and the scale in
-// the form the GEMM copies. Two slabs in one launch, the first bounded by *d_rows on the device. One warp
-// per block.
+// the form the GEMM copies. Two slabs in one launch, the first bounded by *d_rows on the device; and, in map_ctas CTAs of
+// their own, the experts' descriptors. One warp per block or expert.
 constexpr int kQuantWarps = 4;
 __global__ void __launch_bounds__(kQuantWarps * 32)
 quantize_operand_kernel(const uint16_t* __restrict__ x0, const uint16_t* __restrict__ u0,
                         unsigned char* __restrict__ out0, long long n0, const int* __restrict__ d_rows,
                         const uint16_t* __restrict__ x1, const uint16_t* __restrict__ u1,
-                        unsigned char* __restrict__ out1, long long n1, int nb) {
+                        unsigned char* __restrict__ out1, long long n1, int nb, unsigned map_ctas,
+                        const __grid_constant__ MapArgs m) {
+  __shared__ __align__(128) unsigned char patch[kQuantWarps][384];
   pdl_wait();
   pdl_launch_dependents();
-  long long b = static_cast<long long>(blockIdx.x) * kQuantWarps + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x < map_ctas) {
+    const int e = blockIdx.x * kQuantWarps + warp;
+    if (e <= m.n_expert) make_maps(m, e, patch[warp], lane);
+    return;
+  }
+  long long b = static_cast<long long>(blockIdx.x - map_ctas) * kQuantWarps + warp;
   const uint16_t *x = x0, *u = u0;
   unsigned char* out = out0;
   if (b >= n0) {
@@ -717,6 +767,7 @@ GemmArgs args_of(const ExpertGemm& g) {
   a.n_rows = g.n_rows; a.nb = g.k / kQK; a.n_expert = g.n_expert;
   a.sw0 = a.sw1 = static_cast<const unsigned char*>(g.shared_w);
   a.sxq = g.shared_xq; a.sy = g.shared_y; a.s_rows = g.shared_rows;
+  a.maps = static_cast<const unsigned char*>(g.maps);
   return a;
 }
 
@@ -730,16 +781,23 @@ int gemm_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, uint16
   return g.operand_rows ? launch_gemm<true, false>(a, stream) : launch_gemm<true, true>(a, stream);
 }
 int gemm_grouped(const ExpertGemm& g, cudaStream_t stream) {
-  return g.operand_rows ? launch_gemm<false, false>(args_of(g), stream) : launch_gemm<false, true>(args_of(g), stream);
+  GemmArgs a = args_of(g);
+  a.map0 = 2;
+  return g.operand_rows ? launch_gemm<false, false>(a, stream) : launch_gemm<false, true>(a, stream);
 }
 int quantize_operand(const uint16_t* x0, const uint16_t* u0, void* out0, long long rows0, const int* d_rows,
-                     const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, cudaStream_t stream) {
+                     const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, const ExpertMaps& em, bool make_maps,
+                     cudaStream_t stream) {
   const int nb = k / kQK;
-  const long long blocks = (rows0 + rows1) * nb;
-  if (blocks <= 0) return kOk;
-  return launch_pdl(quantize_operand_kernel, dim3(static_cast<unsigned>((blocks + kQuantWarps - 1) / kQuantWarps)),
-                    kQuantWarps * 32, 0, stream, x0, u0, static_cast<unsigned char*>(out0), rows0 * nb, d_rows, x1, u1,
-                    static_cast<unsigned char*>(out1), rows1 * nb, nb);
+  const long long ctas = ((rows0 + rows1) * nb + kQuantWarps - 1) / kQuantWarps;
+  MapArgs m{};
+  if (!map_args(em, make_maps, &m)) return kErrUnsupported;
+  const unsigned map_ctas = make_maps ? static_cast<unsigned>(em.n_expert / kQuantWarps + 1) : 0;
+  if (ctas + map_ctas > 0x7FFFFFFF) return kErrUnsupported;
+  if (ctas + map_ctas == 0) return kOk;
+  return launch_pdl(quantize_operand_kernel, dim3(static_cast<unsigned>(ctas + map_ctas)), kQuantWarps * 32, 0, stream, x0, u0,
+                    static_cast<unsigned char*>(out0), rows0 * nb, d_rows, x1, u1, static_cast<unsigned char*>(out1), rows1 * nb, nb,
+                    map_ctas, m);
 }
 
 }  // namespace sgr

@@ -377,41 +377,18 @@ int launch_rows(RowsArgs a, cudaStream_t stream) {
 // in one launch, the first bounded by *d_rows on the device; and, in CTAs of their own (map_ctas of them), the descriptors of every
 // expert's three matrices. One warp per block or expert.
 constexpr int kQuantWarps = 4;
-struct MapArgs {
-  unsigned* counters;                  // of the GEMM launches, cleared
-  const unsigned char* const* tab;     // [3][stride]
-  long long stride;
-  unsigned char* maps;
-  const unsigned char* shared[3];
-  int n_expert;
-  alignas(16) uint32_t up[32], down[32];
-};
 __global__ void __launch_bounds__(kQuantWarps * 32)
 quantize_rows_kernel(const uint16_t* __restrict__ x0, unsigned char* __restrict__ out0, long long n0, const int* __restrict__ d_rows,
                      const uint16_t* __restrict__ x1, unsigned char* __restrict__ out1, long long n1, int nb, unsigned map_ctas,
                      const __grid_constant__ MapArgs m) {
-  __shared__ __align__(128) unsigned char patch[kQuantWarps][3][128];
+  __shared__ __align__(128) unsigned char patch[kQuantWarps][384];
   pdl_wait();
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (blockIdx.x == 0 && threadIdx.x < 4) m.counters[threadIdx.x] = 0u;
   if (blockIdx.x < map_ctas) {
     const int e = blockIdx.x * kQuantWarps + warp;
-    if (e > m.n_expert) return;
-    const unsigned char* w[3];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      w[i] = e == m.n_expert ? m.shared[i] : m.tab[i * m.stride + e];
-      reinterpret_cast<uint32_t*>(patch[warp][i])[lane] = i < 2 ? m.up[lane] : m.down[lane];
-    }
-    __syncwarp();
-    // (a base that is absent or off a 16-byte boundary keeps the placeholder: its descriptor is not used)
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-      if (lane == i && w[i] != nullptr && (reinterpret_cast<uintptr_t>(w[i]) & 15u) == 0) tmap_replace_addr(patch[warp][i], w[i]);
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 3; ++i) tmap_publish(m.maps + (static_cast<size_t>(e) * 3 + i) * 128, patch[warp][i]);
+    if (e <= m.n_expert) make_maps(m, e, patch[warp], lane);
     return;
   }
   long long b = static_cast<long long>(blockIdx.x - map_ctas) * kQuantWarps + warp;
@@ -442,13 +419,10 @@ quantize_rows_kernel(const uint16_t* __restrict__ x0, unsigned char* __restrict_
   }
 }
 
-unsigned* counters_of(const void* maps, int n_expert) {
-  return reinterpret_cast<unsigned*>(static_cast<unsigned char*>(const_cast<void*>(maps)) + (n_expert + 1LL) * 384);
-}
 RowsArgs args_of(const ExpertGemm& g, const void* maps, int map0) {
   RowsArgs a{};
   a.maps = static_cast<const unsigned char*>(maps);
-  a.next = counters_of(maps, g.n_expert) + map0;
+  a.next = map_counters(maps, g.n_expert) + map0;
   a.tab0 = g.tab; a.map0 = map0; a.off = g.off; a.rows = g.rows; a.xq = g.xq; a.y = g.y;
   a.n_rows = g.n_rows; a.nb = g.k / kQK; a.n_expert = g.n_expert;
   a.sw0 = a.sw1 = static_cast<const unsigned char*>(g.shared_w);
@@ -471,15 +445,8 @@ int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_
   const int nb = k / kQK;
   const long long ctas = ((rows0 + rows1) * nb + kQuantWarps - 1) / kQuantWarps;
   MapArgs m{};
-  unsigned map_ctas = 0;
-  m.counters = counters_of(em.maps, em.n_expert);
-  if (make_maps) {
-    m.tab = em.tab; m.stride = em.stride; m.maps = static_cast<unsigned char*>(em.maps); m.n_expert = em.n_expert;
-    for (int i = 0; i < 3; ++i) m.shared[i] = static_cast<const unsigned char*>(em.shared[i]);
-    if (!matrix_tmap(em.hidden / kQK * kW4, em.n_ff, em.maps, m.up) || !matrix_tmap(em.n_ff / kQK * kW4, em.hidden, em.maps, m.down))
-      return kErrUnsupported;
-    map_ctas = static_cast<unsigned>(em.n_expert / kQuantWarps + 1);
-  }
+  if (!map_args(em, make_maps, &m)) return kErrUnsupported;
+  const unsigned map_ctas = make_maps ? static_cast<unsigned>(em.n_expert / kQuantWarps + 1) : 0;
   if (ctas + map_ctas > 0x7FFFFFFF) return kErrUnsupported;
   if (ctas + map_ctas == 0) return kOk;
   return launch_pdl(quantize_rows_kernel, dim3(static_cast<unsigned>(ctas + map_ctas)), kQuantWarps * 32, 0, stream, x0,

@@ -93,8 +93,8 @@ __global__ void combine_grouped_kernel(uint16_t* __restrict__ x, const uint16_t*
 
 inline bool has_shared(const sgr_moe_prefill* a) { return a->shared_gate && a->shared_up && a->shared_down; }
 
-// The rows the GEMMs read lie in the combine slab's memory when they fit there: Q8_K rows in padded blocks and the expert
-// descriptors for the kernel of few token rows per expert, ready operands for the tcgen05 one (FFN up to about 0.8 x hidden
+// The rows the GEMMs read lie in the combine slab's memory, behind the experts' descriptors, when they fit there: Q8_K rows in
+// padded blocks for the kernel of few token rows per expert, ready operands for the tcgen05 one (FFN up to about 0.8 x hidden
 // at top-8); otherwise Q8_K rows from which the tcgen05 GEMMs make their operands themselves.
 enum class Rows { kPadded, kOperands, kPacked };
 struct OperandRows {
@@ -111,14 +111,15 @@ OperandRows operand_rows(const sgr_moe_prefill* a) {
     unsigned char* base = slab + front;
     return OperandRows{front + x + h + s <= room ? form : Rows::kPacked, base, base + x, base + x + h, slab + (-at & 127u)};
   };
+  const long long maps = (-at & 127u) + (a->n_expert + 1LL) * 384 + 16;      // in front: the descriptors
   const uintptr_t outs = reinterpret_cast<uintptr_t>(a->g) | reinterpret_cast<uintptr_t>(a->y_grouped) |
                          reinterpret_cast<uintptr_t>(a->sh_g) | reinterpret_cast<uintptr_t>(a->sh_y);
   if ((at & 15u) == 0 && (outs & 3u) == 0 && static_cast<long long>(a->n) * a->n_used <= static_cast<long long>(kFewRows) * a->n_expert) {
-    const OperandRows r = laid(Rows::kPadded, kRowBlk, (-at & 127u) + (a->n_expert + 1LL) * 384 + 16);
+    const OperandRows r = laid(Rows::kPadded, kRowBlk, maps);
     if (r.form == Rows::kPadded) return r;
   }
   if ((at & 15u) == 0) {
-    const OperandRows r = laid(Rows::kOperands, kOpBlk, 0);
+    const OperandRows r = laid(Rows::kOperands, kOpBlk, maps);
     if (r.form == Rows::kOperands) return r;
   }
   return {Rows::kPacked, static_cast<unsigned char*>(a->xq), static_cast<unsigned char*>(a->hq), static_cast<unsigned char*>(a->sh_q), nullptr};
@@ -147,6 +148,7 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   up.y = a->g; up.n_rows = F; up.k = H; up.n_expert = E;
   ExpertGemm down{};
   down.tab = tab(2); down.off = a->off; down.xq = op.h; down.operand_rows = up.operand_rows;
+  up.maps = down.maps = op.maps;
   down.y = a->y_grouped; down.n_rows = H; down.k = F; down.n_expert = E;
   if (shared) {
     up.shared_w = a->shared_gate; up.shared_xq = op.x; up.shared_y = a->sh_g; up.shared_rows = n;
@@ -162,7 +164,8 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   rc = gemm_gate_up(up, tab(1), a->u, a->shared_up, a->sh_u, stream);
   if (rc != kOk) return rc;
   if (op.form == Rows::kOperands) {
-    rc = quantize_operand(a->g, a->u, op.h, static_cast<long long>(n) * K, a->meta, a->sh_g, a->sh_u, op.s, shared ? n : 0, F, stream);
+    rc = quantize_operand(a->g, a->u, op.h, static_cast<long long>(n) * K, a->meta, a->sh_g, a->sh_u, op.s, shared ? n : 0, F, expert_maps(a, op), false,
+                          stream);
   } else {
     rc = sgr_silu_mul_f16_n(a->g, a->g, a->u, a->meta, static_cast<int>(R), F, stream);
     if (rc == kOk) rc = sgr_quantize_q8_k_n(a->g, a->hq, a->meta, F, static_cast<int>(R * (F / kQK)), stream);
@@ -208,7 +211,7 @@ SGR_API int sgr_moe_layer_prefill(const sgr_moe_prefill* a, void* stream) {
   const OperandRows op = operand_rows(a);
   if (op.form == Rows::kPadded) {
     SGR_STEP(quantize_rows(a->xn, op.x, n, nullptr, nullptr, nullptr, 0, H, expert_maps(a, op), true, as_stream(stream)));
-  } else if (op.form == Rows::kOperands) SGR_STEP(quantize_operand(a->xn, nullptr, op.x, n, nullptr, nullptr, nullptr, nullptr, 0, H, as_stream(stream)));
+  } else if (op.form == Rows::kOperands) SGR_STEP(quantize_operand(a->xn, nullptr, op.x, n, nullptr, nullptr, nullptr, nullptr, 0, H, expert_maps(a, op), true, as_stream(stream)));
   else SGR_STEP(sgr_quantize_q8_k(a->xn, a->xq, static_cast<long long>(n) * H, stream));
   const float* logits = a->logits_in;
   if (logits == nullptr) {

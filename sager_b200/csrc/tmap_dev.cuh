@@ -3,6 +3,7 @@
 // encoded on the host for a placeholder address and gets its base there.
 #pragma once
 
+#include "api_util.cuh"
 #include "q4k_common.cuh"
 
 namespace sgr {
@@ -26,6 +27,46 @@ __device__ __forceinline__ void tmap_acquire(const void* gmem_map) {
 __device__ __forceinline__ void tma_load_box(void* dst, const void* gmem_map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
+}
+
+// The descriptors of a layer's experts (ExpertMaps, api_util.cuh), made by CTAs of a launch before the GEMMs; and the counters
+// that lie behind them, cleared.
+struct MapArgs {
+  unsigned* counters;
+  const unsigned char* const* tab;     // [3][stride]
+  long long stride;
+  unsigned char* maps;
+  const unsigned char* shared[3];
+  int n_expert;
+  alignas(16) uint32_t up[32], down[32];
+};
+inline unsigned* map_counters(const void* maps, int n_expert) {
+  return reinterpret_cast<unsigned*>(static_cast<unsigned char*>(const_cast<void*>(maps)) + (n_expert + 1LL) * 384);
+}
+// false: the driver has no encoder
+inline bool map_args(const ExpertMaps& em, bool make, MapArgs* m) {
+  m->counters = map_counters(em.maps, em.n_expert);
+  if (!make) return true;
+  m->tab = em.tab; m->stride = em.stride; m->maps = static_cast<unsigned char*>(em.maps); m->n_expert = em.n_expert;
+  for (int i = 0; i < 3; ++i) m->shared[i] = static_cast<const unsigned char*>(em.shared[i]);
+  return matrix_tmap(em.hidden / kQK * kW4, em.n_ff, em.maps, m->up) && matrix_tmap(em.n_ff / kQK * kW4, em.hidden, em.maps, m->down);
+}
+// One warp: the three descriptors of expert e (n_expert: the shared one); `patch` is 384 bytes of shared memory, 128-byte aligned.
+// A base that is absent or off a 16-byte boundary keeps the placeholder: its descriptor is not used.
+__device__ __forceinline__ void make_maps(const MapArgs& m, int e, unsigned char* patch, int lane) {
+  const unsigned char* w[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    w[i] = e == m.n_expert ? m.shared[i] : m.tab[i * m.stride + e];
+    reinterpret_cast<uint32_t*>(patch + 128 * i)[lane] = i < 2 ? m.up[lane] : m.down[lane];
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (lane == i && w[i] != nullptr && (reinterpret_cast<uintptr_t>(w[i]) & 15u) == 0) tmap_replace_addr(patch + 128 * i, w[i]);
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 3; ++i) tmap_publish(m.maps + (static_cast<size_t>(e) * 3 + i) * 128, patch + 128 * i);
 }
 
 }  // namespace sgr
