@@ -46,9 +46,8 @@ __global__ void router_logits_kernel(const float* __restrict__ w, const uint16_t
 // 16, 8, 4, 2, 1 a lane adds the partner's half of the outputs to its own, which is the pairing
 // of the reference's shuffle-down tree (addition commutes), in 31/32 of a shuffle per output
 // instead of five. Bound by the fp32 pipes and the issue slots around them (1.07 G FMAs for 2048
-// tokens x 256 rows x 2048: 29 us at 128 per clock and SM). Measured for 2048 / 777 / 96 tokens:
-// 81 / 41 / 10 us; a warp per (row, eight tokens) with the fp16 values converted at every use
-// took 534 / 212 / 33 us.
+// tokens x 256 rows x 2048: 29 us at 128 per clock and SM). (A warp per (row, eight tokens)
+// with the fp16 values converted at every use took 534 / 212 / 33 us for 2048 / 777 / 96 tokens.)
 __device__ __forceinline__ void fma2(unsigned long long& acc, float w, unsigned long long x) {
   unsigned long long ww;
   asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w));
@@ -69,6 +68,160 @@ __device__ __forceinline__ void fold_lanes(float* f, int lane) {
   }
 }
 
+// Fold the 32 lanes and store: output o = r * TT + t; after the five exchanges lane l holds the outputs whose bits above
+// log2(TR * TT / 32) spell l's bits from bit 4 down.
+template <int TR, int TT>
+__device__ __forceinline__ void store_folded(const unsigned long long (&acc)[TR][TT / 2], float* __restrict__ y, int row0, int tok0,
+                                             int n_rows, int n_tokens, int lane) {
+  float f[TR * TT];
+#pragma unroll
+  for (int r = 0; r < TR; ++r)
+#pragma unroll
+    for (int p = 0; p < TT / 2; ++p)
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(f[r * TT + 2 * p]), "=f"(f[r * TT + 2 * p + 1]) : "l"(acc[r][p]));
+  fold_lanes<TR * TT, 16>(f, lane);
+  constexpr int kLeft = TR * TT / 32;
+#pragma unroll
+  for (int i = 0; i < kLeft; ++i) {
+    const int o = i + kLeft * lane;           // step s split on output bit log2(TR*TT) - 1 - s and lane bit 4 - s
+    const int row = row0 + o / TT, tok = tok0 + o % TT;
+    if (row < n_rows && tok < n_tokens) y[static_cast<size_t>(tok) * n_rows + row] = f[i];
+  }
+}
+
+// The product for rows of whole 16-byte pieces: the raw columns of W and x arrive by cp.async three stages of 128 columns
+// ahead, x is turned into fp32 token pairs stage by stage - ldmatrix.trans hands a lane two tokens' values of one k, so
+// eight tokens x 32 columns are one load, eight conversions and four stores -, W is used as it lies. Against the kernel below,
+// which converts from registers after 2-byte loads: 2048 / 1024 / 592 / 96 tokens 70.6 / 38.0 / 23.3 / 7.9 us, 76.9 / 44.7 /
+// 35.0 / 9.2 before. Bound by the FMA pipe (2 cycles a packed FMA: 30 us at 2048 tokens) and the shared-memory operands (36 us),
+// which two warps per scheduler do not overlap further: volatile loads, other tiles and more warps changed nothing.
+// block: WR x WT warps; grid (row tiles, token tiles).
+template <int TR, int TT, int WR, int WT>
+struct Logits {
+  static constexpr int kWarps = WR * WT, kRows = TR * WR, kToks = TT * WT, kPairs = kToks / 2, kCols = 128, kSlots = 4;
+  static constexpr int kXPitch = (kCols + 8) * 2;            // bytes of a raw x row: eight rows' 16 bytes in different banks
+  static constexpr int kPairPitch = kCols * 8 + 32;          // bytes of a pair: [column][two tokens]
+  static constexpr int kWBytes = kRows * kCols * 4, kXBytes = kToks * kXPitch, kPairBytes = kPairs * kPairPitch;
+  static constexpr int kSmem = kSlots * (kWBytes + kXBytes) + 2 * kPairBytes;
+  static_assert(kToks % 8 == 0 && kWBytes % 16 == 0 && kXBytes % 16 == 0 && kPairBytes % 16 == 0, "tile");
+};
+template <int TR, int TT, int WR, int WT>
+__global__ void __launch_bounds__(WR* WT * 32, (TR * TT >= 128 ? 8 : TR * TT >= 64 ? 16 : 20) / (WR * WT))
+router_logits_staged_kernel(const float* __restrict__ w, const uint16_t* __restrict__ x, float* __restrict__ y,
+                            int n_rows, int k, int n_tokens) {
+  using T = Logits<TR, TT, WR, WT>;
+  constexpr int kThreads = T::kWarps * 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  unsigned char* const w_raw = smem;                                           // [kSlots][kRows][128] fp32
+  unsigned char* const x_raw = smem + T::kSlots * T::kWBytes;                  // [kSlots][kToks][kXPitch]
+  unsigned char* const x_f32 = x_raw + T::kSlots * T::kXBytes;                 // [2][kPairs][kPairPitch]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row0 = blockIdx.x * T::kRows, tok0 = blockIdx.y * T::kToks;
+  const int wr = warp % WR, wt = warp / WR;
+  // rows and tokens past the end repeat the last one (never stored), columns past k are zero (add nothing)
+  auto piece = [](uint32_t dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+  };
+  constexpr int kWPieces = T::kRows * 32 / kThreads, kXPieces = T::kToks * 16 / kThreads;
+  static_assert(T::kRows * 32 % kThreads == 0 && T::kToks * 16 % kThreads == 0, "pieces");
+  const int w_col = (tid & 31) * 4, x_col = (tid & 15) * 8;      // a thread's pieces lie in one column of pieces
+  const float* w_at[kWPieces];
+  const uint16_t* x_at[kXPieces];
+#pragma unroll
+  for (int i = 0; i < kWPieces; ++i) w_at[i] = w + static_cast<size_t>(min(row0 + (tid >> 5) + i * (kThreads / 32), n_rows - 1)) * k + w_col;
+#pragma unroll
+  for (int i = 0; i < kXPieces; ++i) x_at[i] = x + static_cast<size_t>(min(tok0 + (tid >> 4) + i * (kThreads / 16), n_tokens - 1)) * k + x_col;
+  auto fill_w = [&](int c) {
+    const int k0 = c * T::kCols;
+    if (k0 >= k) return;
+    const bool in = k0 + w_col < k;
+    const uint32_t dst = smem_u32(w_raw + (c % T::kSlots) * T::kWBytes + tid * 16);
+#pragma unroll
+    for (int i = 0; i < kWPieces; ++i) piece(dst + i * kThreads * 16, in ? w_at[i] + k0 : w, in);
+  };
+  auto fill_x = [&](int c) {
+    const int k0 = c * T::kCols;
+    if (k0 < k) {
+      const bool in = k0 + x_col < k;
+      const uint32_t dst = smem_u32(x_raw + (c % T::kSlots) * T::kXBytes + (tid >> 4) * T::kXPitch + (tid & 15) * 16);
+#pragma unroll
+      for (int i = 0; i < kXPieces; ++i) piece(dst + i * (kThreads / 16) * T::kXPitch, in ? x_at[i] + k0 : x, in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // unit: eight tokens x 32 columns; lane i receives tokens 2 (i % 4), + 1 of columns i / 4 + 0, 8, 16, 24
+  auto convert = [&](int c) {
+    const unsigned char* raw = x_raw + (c % T::kSlots) * T::kXBytes;
+    unsigned char* out = x_f32 + (c & 1) * T::kPairBytes;
+    auto load = [&](uint32_t (&v)[4], int g, int j) {
+      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                   : "r"(smem_u32(raw + (g * 8 + (lane & 7)) * T::kXPitch + (j * 32 + (lane >> 3) * 8) * 2)) : "memory");
+    };
+    auto f = [](uint32_t h, int hi) { return __half2float(__ushort_as_half(static_cast<unsigned short>(hi ? h >> 16 : h & 0xFFFFu))); };
+    constexpr int kUnits = T::kToks / 8 * 4;
+    static_assert(kUnits % T::kWarps == 0, "units");
+#pragma unroll
+    for (int u = warp; u < kUnits; u += T::kWarps) {
+      const int g = u >> 2, j = u & 3;
+      uint32_t a[4];
+      load(a, g, j);
+      unsigned char* o = out + (g * 4 + (lane & 3)) * T::kPairPitch + j * 256 + (lane >> 2) * 8;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) *reinterpret_cast<float2*>(o + m * 64) = make_float2(f(a[m], 0), f(a[m], 1));
+    }
+  };
+
+  const int chunks = (k + T::kCols - 1) / T::kCols;
+#pragma unroll
+  for (int c = 0; c < T::kSlots - 1; ++c) fill_w(c);             // (W does not depend on the kernel before)
+  pdl_wait();
+  pdl_launch_dependents();
+#pragma unroll
+  for (int c = 0; c < T::kSlots - 1; ++c) fill_x(c);
+  asm volatile("cp.async.wait_group %0;" ::"n"(T::kSlots - 2) : "memory");
+  __syncthreads();
+  convert(0);
+  unsigned long long acc[TR][TT / 2];           // two packed fp32 sums each
+#pragma unroll
+  for (int r = 0; r < TR; ++r)
+#pragma unroll
+    for (int p = 0; p < TT / 2; ++p) acc[r][p] = 0ull;
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(T::kSlots - 3) : "memory");     // chunk c + 1 has landed
+    __syncthreads();                            // ... everybody's part of it; chunk c is converted, chunk c - 1 no longer read
+    fill_w(c + T::kSlots - 1);
+    fill_x(c + T::kSlots - 1);
+    const float* wp = reinterpret_cast<const float*>(w_raw + (c % T::kSlots) * T::kWBytes) + wr * TR * T::kCols + lane;
+    const unsigned char* xp = x_f32 + (c & 1) * T::kPairBytes + wt * (TT / 2) * T::kPairPitch + lane * 8;
+    // operands of 32 columns (one per lane); the next ones are loaded under this one's products
+    float wv[2][TR];
+    unsigned long long xv[2][TT / 2];
+    auto load = [&](int j) {
+#pragma unroll
+      for (int r = 0; r < TR; ++r)
+        wv[j & 1][r] = wp[r * T::kCols + j * 32];
+#pragma unroll
+      for (int p = 0; p < TT / 2; ++p)
+        xv[j & 1][p] = *reinterpret_cast<const unsigned long long*>(xp + p * T::kPairPitch + j * 256);
+
+    };
+    load(0);
+#pragma unroll
+    for (int j = 0; j < T::kCols / 32; ++j) {
+      if (j + 1 < T::kCols / 32) load(j + 1);
+      if (j == 0 && c + 1 < chunks) convert(c + 1);
+#pragma unroll
+      for (int r = 0; r < TR; ++r)
+#pragma unroll
+        for (int p = 0; p < TT / 2; ++p) fma2(acc[r][p], wv[j & 1][r], xv[j & 1][p]);
+    }
+  }
+  store_folded<TR, TT>(acc, y, row0 + wr * TR, tok0 + wt * TT, n_rows, n_tokens, lane);
+}
+
+// The same for rows off a 16-byte boundary.
 // block: WR x WT warps; grid (row tiles, token tiles). KC columns per shared-memory stage, two
 // stages: the next one is on its way to registers while this one is used, so a stage has to last a
 // round trip to L2 (with 64 columns the trip showed: 124 us for 2048 tokens, 14 us for eight).
@@ -177,22 +330,7 @@ router_logits_tiled_kernel(const float* __restrict__ w, const uint16_t* __restri
     __syncthreads();
   }
 
-  // fold the 32 lanes: output o = r * TT + t; after the five exchanges lane l holds the outputs
-  // whose bits above log2(TR * TT / 32) spell l's bits from bit 4 down
-  float f[TR * TT];
-#pragma unroll
-  for (int r = 0; r < TR; ++r)
-#pragma unroll
-    for (int p = 0; p < TT / 2; ++p)
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(f[r * TT + 2 * p]), "=f"(f[r * TT + 2 * p + 1]) : "l"(acc[r][p]));
-  fold_lanes<TR * TT, 16>(f, lane);
-  constexpr int kLeft = TR * TT / 32;
-#pragma unroll
-  for (int i = 0; i < kLeft; ++i) {
-    const int o = i + kLeft * lane;           // step s split on output bit log2(TR*TT) - 1 - s and lane bit 4 - s
-    const int row = row0 + wr * TR + o / TT, tok = tok0 + wt * TT + o % TT;
-    if (row < n_rows && tok < n_tokens) y[static_cast<size_t>(tok) * n_rows + row] = f[i];
-  }
+  store_folded<TR, TT>(acc, y, row0 + wr * TR, tok0 + wt * TT, n_rows, n_tokens, lane);
 }
 
 template <int TR, int TT, int WR, int WT, int KC>
@@ -201,6 +339,14 @@ int launch_tiled(const float* w, const uint16_t* x, float* y, int n_rows, int k,
   if (kSmem > 48 * 1024 && !opt_in_smem<router_logits_tiled_kernel<TR, TT, WR, WT, KC>>(kSmem)) return kErrLaunch;
   const dim3 grid((n_rows + TR * WR - 1) / (TR * WR), (n_tokens + TT * WT - 1) / (TT * WT));
   return launch_pdl(router_logits_tiled_kernel<TR, TT, WR, WT, KC>, grid, WR * WT * 32, kSmem, stream, w, x, y, n_rows, k, n_tokens);
+}
+
+template <int TR, int TT, int WR, int WT>
+int launch_staged(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens, cudaStream_t stream) {
+  using T = Logits<TR, TT, WR, WT>;
+  if (!opt_in_smem<router_logits_staged_kernel<TR, TT, WR, WT>>(T::kSmem)) return kErrLaunch;
+  const dim3 grid((n_rows + T::kRows - 1) / T::kRows, (n_tokens + T::kToks - 1) / T::kToks);
+  return launch_pdl(router_logits_staged_kernel<TR, TT, WR, WT>, grid, T::kWarps * 32, T::kSmem, stream, w, x, y, n_rows, k, n_tokens);
 }
 
 int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens,
@@ -212,6 +358,15 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
     const size_t smem = static_cast<size_t>(k) * 2;
     if (smem > 48 * 1024) return kErrUnsupported;
     router_logits_kernel<<<(n_rows + warps - 1) / warps, warps * 32, smem, stream>>>(w, x, y, n_rows, k);
+  } else if ((k & 7) == 0 && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0 &&
+             (n_tokens + 15) / 16 <= 65535) {
+    // A warp's outputs: more of them need fewer shared-memory operands per FMA, fewer of them give more warps to spread. 256 rows
+    // x 128 / 300 / 400 / 900 / 1200 / 1400 / 2048 tokens, us: 4 x 8 outputs 8.1 / 16.6 / 19.3 / 39.0 / 50.3 / 56.5 / 81.7,
+    // 8 x 8 8.6 / 17.3 / 17.5 / 37.6 / 47.4 / 52.9 / 73.2, 8 x 16 13.3 / 22.1 / 21.7 / 42.4 / 50.9 / 51.6 / 70.6.
+    const long long outputs = static_cast<long long>(n_rows) * n_tokens;
+    if (outputs >= 256LL * 1300) return launch_staged<8, 16, 2, 2>(w, x, y, n_rows, k, n_tokens, stream);
+    if (outputs >= 256LL * 320) return launch_staged<8, 8, 2, 2>(w, x, y, n_rows, k, n_tokens, stream);
+    return launch_staged<4, 8, 4, 1>(w, x, y, n_rows, k, n_tokens, stream);
   } else if (static_cast<long long>(n_rows) * n_tokens >= 256LL * 592) {
     // 8 x 16 outputs per warp keep the FMA pipes fullest; below one such CTA per SM the smaller tile has more
     // warps to spread (at 256 x 592 the two take 41 and 38 us, and from there the larger one wins)

@@ -59,6 +59,34 @@ def test_logits_tile_edges_bit_exact(oracle, rows, k, n_tok):
     assert torch.all(y[n_tok] == 7.0)
 
 
+@pytest.mark.parametrize("rows,k,n_tok", [(256, 2048, 319), (256, 2048, 320), (250, 1000, 327), (256, 512, 1300), (256, 512, 1299),
+                                          (250, 1000, 1333), (31, 8, 70), (256, 136, 600)])
+def test_logits_staged_tiles_bit_exact(oracle, rows, k, n_tok):
+    """The three tiles for rows of whole 16-byte pieces (lines at rows x tokens = 256 x 320 and 256 x 1300), ragged rows, tokens
+    and columns, fewer columns than a stage."""
+    w_np, w_dev = router_w(7, e=rows, h=k)
+    x_np, x_dev = make_x16(n_tok, k, 8)
+    y = torch.full((n_tok + 1, rows), 7.0, dtype=torch.float32, device=DEV)
+    ops.gemv_f32_out_f16x_mtok(w_dev, x_dev, y, rows, k, n_tok)
+    want = np.stack([oracle.router_logits(w_np, x_np[t]) for t in range(n_tok)])
+    assert np.array_equal(y.cpu().numpy()[:n_tok].view(np.uint32), want.view(np.uint32))
+    assert torch.all(y[n_tok] == 7.0)
+
+
+@pytest.mark.parametrize("shift_w,shift_x,k", [(1, 0, 512), (0, 1, 512), (0, 0, 500)])
+def test_logits_off_a_16_byte_boundary(oracle, shift_w, shift_x, k):
+    w_np, w_dev = router_w(9, e=40, h=k)
+    x_np, x_dev = make_x16(21, k, 10)
+    big_w = torch.zeros(40 * k + 4, dtype=torch.float32, device=DEV)
+    big_x = torch.zeros(21 * k + 4, dtype=torch.float16, device=DEV)
+    big_w[shift_w:shift_w + 40 * k] = w_dev.reshape(-1)
+    big_x[shift_x:shift_x + 21 * k] = x_dev.reshape(-1)
+    y = torch.zeros(21, 40, dtype=torch.float32, device=DEV)
+    ops.gemv_f32_out_f16x_mtok(big_w[shift_w:], big_x[shift_x:], y, 40, k, 21)
+    want = np.stack([oracle.router_logits(w_np, x_np[t]) for t in range(21)])
+    assert np.array_equal(y.cpu().numpy().view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("seed", range(8))
 def test_topk_selection_exact(oracle, seed):
     rng = np.random.default_rng(seed)
