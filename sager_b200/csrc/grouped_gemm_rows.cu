@@ -36,7 +36,7 @@ constexpr int kHalfBytes = 128 * kW4, kWBytes = 2 * kHalfBytes;
 constexpr int kXRow = 304, kXCodes = 16, kXSums = 272, kXBytes = kTok * kXRow;
 static_assert(kRowBlk <= kXRow && kXSums + 16 == kRowBlk, "block layout");
 constexpr int kStageBytes = (kWBytes + kXBytes + 127) & ~127;
-constexpr int kHdr = 1024;
+constexpr int kHdr = 1024;                                    // the last 256 bytes are zeros
 constexpr int kSmem = kHdr + kStages * kStageBytes;
 static_assert(kSmem <= 227 * 1024, "shared memory");
 
@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
   Desc* desc = reinterpret_cast<Desc*>(smem + 256);
   Unit* list = reinterpret_cast<Unit*>(smem + 512);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned char* const zeros = smem + kHdr - 256;
+  if (tid < 64) reinterpret_cast<uint32_t*>(zeros)[tid] = 0u;
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1 + kXWarps);
@@ -315,8 +317,20 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
         __syncwarp();
         if (lane == 0) mbar_arrive_one(&wempty[s]);
       };
-      if (d.flags >> 10 & 1) loaded();
-      else if (nt <= 8) rows_block<1>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
+      if (d.flags >> 10 & 1) {
+        loaded();
+      } else if (nt <= 4) {
+        const unsigned char* xs = st + kWBytes;
+        const uint4 h0 = *reinterpret_cast<const uint4*>(st + own_lo), h1 = *reinterpret_cast<const uint4*>(st + own_hi);
+        warp_mma_block4(st + w_off, h0, h1, b_row4(xs + kXCodes, kXRow, zeros, lane), 0, lane, loaded,
+                        [&] { return *reinterpret_cast<const uint32_t*>(xs + (gid >> 1) * kXRow + kXSums + (tig & 1) * 8 + (gid & 1) * 4); },
+                        [&](int r, int isum, int msum) {
+                          const uint32_t dm = r ? h1.x : h0.x;
+                          const float s = __fmul_rn(0.0625f * h2f(static_cast<uint16_t>(dm & 0xFFFFu)), static_cast<float>(isum));
+                          const float v = __fmaf_rn(-h2f(static_cast<uint16_t>(dm >> 16)), static_cast<float>(msum), s);
+                          acc[0][r] = __fmaf_rn(*reinterpret_cast<const float*>(xs + tig * kXRow), v, acc[0][r]);
+                        });
+      } else if (nt <= 8) rows_block<1>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
       else if (nt <= 16) rows_block<2>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
       else if (nt <= 24) rows_block<3>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
       else rows_block<4>(st + w_off, st + own_lo, st + own_hi, st + kWBytes, acc, lane, loaded);
@@ -326,6 +340,21 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
       // ---- the unit is complete for this warp's rows: the lanes of two neighbouring rows trade halves, so that a
       // store is two rows of one token ----
       uint16_t* y = (d.flags >> 11 & 1) ? a.sy : a.y;
+      if (nt <= 4) {                                 // token tig; row pairs by the even lanes
+        const __half2 v = __floats2half2_rn(acc[0][0], acc[0][1]);
+        uint32_t mine = *reinterpret_cast<const uint32_t*>(&v);
+        if (DUAL) {
+          const __half h = __float2half(silu_mul(__low2float(v), __high2float(v)));
+          mine = *reinterpret_cast<const uint16_t*>(&h);
+        }
+        const uint32_t other = __shfl_xor_sync(0xFFFFFFFFu, mine, 4);
+        if (tig < nt && (gid & 1) == 0) {
+          uint16_t* o = y + static_cast<size_t>(d.slot0 + tig) * a.n_rows + d.group * (DUAL ? 128 : 256) + (DUAL ? 8 : 16) * warp + gid;
+          *reinterpret_cast<uint32_t*>(o) = __byte_perm(mine, other, 0x5410);
+          if (!DUAL) *reinterpret_cast<uint32_t*>(o + 8) = __byte_perm(mine, other, 0x7632);
+        }
+        continue;
+      }
       const int odd = gid & 1;
       const uint32_t sel = odd ? 0x3276u : 0x5410u;
       const int row = d.group * (DUAL ? 128 : 256) + (DUAL ? 8 : 16) * warp + gid - odd;

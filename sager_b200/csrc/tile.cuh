@@ -384,6 +384,57 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
   }
 }
 
+// The same for at most four token rows, with two of the MMA's eight columns to a token: the even sub-blocks' dots land in
+// column 2t, the odd ones' in 2t + 1 (each MMA's activation operand is zero in the other columns), so one set of results holds
+// both, and a lane scales the results of one token - half the multiply-adds, conversions and fp32 steps, which for eight
+// columns are spent on tokens that are not there (us per layer of 2048 / 512 / 256 experts at 64 skewed, 32 skewed, 8 rows: 92.2 /
+// 73.5 / 50.2 with eight columns, 90.1 / 72.5 / 49.5). Results: rows gid and gid + 8, token tig.
+//   b_ptr   this lane's ldmatrix row (b_row4), advanced by 64 bytes per pair of sub-blocks, + mid_pad after two
+//   min_b   sub-block sums 4 (tig & 1) .. + 3 of token gid / 2: their low parts in even gid, high parts (bsum = 128 hi + lo) in odd
+//   fold(row, isum, msum): the fp32 steps; isum is sixteen-fold
+template <typename Loaded, typename MinB, typename Fold>
+__device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, const uint4& h0, const uint4& h1, const unsigned char* b_ptr,
+                                                int mid_pad, int lane, Loaded loaded, MinB min_b, Fold fold) {
+  const int tig = lane & 3;
+  uint32_t raw[4][4];
+#pragma unroll
+  for (int g = 0; g < 4; ++g) ldmatrix_x4(raw[g], a_ptr + g * 32);
+  loaded();
+  const Scales6 s_lo = unpack_scales6(h0.y, h0.z, h0.w), s_hi = unpack_scales6(h1.y, h1.z, h1.w);
+  const int zero[4] = {0, 0, 0, 0};
+  int is[2] = {0, 0}, hs[2] = {0, 0};            // even sub-blocks; odd ones, sixteen-fold
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    uint32_t b[4], lo[4], hi[4];
+    ldmatrix_x4(b, b_ptr + g * 64 + (g >> 1) * mid_pad);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      lo[j] = raw[g][j] & 0x0F0F0F0Fu;
+      hi[j] = raw[g][j] & 0xF0F0F0F0u;
+    }
+    int c[4];
+    mma_u8s8(c, lo, b[0], b[1], zero);
+    mma_u8s8(c, hi, b[2], b[3], c);
+    const int sh = 2 * (g & 1);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint32_t sc = r ? s_hi.sc[g >> 1] : s_lo.sc[g >> 1];
+      is[r] += static_cast<int>(__byte_perm(sc, 0, 0x4440 + sh)) * c[2 * r];
+      hs[r] += static_cast<int>(__byte_perm(sc, 0, 0x4441 + sh)) * c[2 * r + 1];
+    }
+  }
+  const uint32_t ma[4] = {tig == 0 ? s_lo.mn[0] : (tig == 1 ? s_lo.mn[1] : 0u), tig == 0 ? s_hi.mn[0] : (tig == 1 ? s_hi.mn[1] : 0u), 0u, 0u};
+  int m[4];
+  mma_u8s8(m, ma, min_b(), 0u, zero);
+#pragma unroll
+  for (int r = 0; r < 2; ++r) fold(r, 16 * is[r] + hs[r], m[2 * r] + 128 * m[2 * r + 1]);
+}
+// This lane's ldmatrix row for warp_mma_block4: lanes 0-7 / 8-15 name the columns' first / second sixteen codes of an even
+// sub-block, 16-31 those of the odd one after it; `codes` is token 0's row, `zeros` 256 + mid_pad bytes of zeros.
+__device__ __forceinline__ const unsigned char* b_row4(const unsigned char* codes, int tok_stride, const unsigned char* zeros, int lane) {
+  return ((lane & 1) == (lane >> 4) ? codes + ((lane & 7) >> 1) * tok_stride : zeros) + (lane >> 3) * 16;
+}
+
 // Four warps cover the tile: with at least four 16-row groups each warp takes
 // groups w, w+4, ...; with fewer, the warps of a group split the super-blocks and
 // their partial sums meet in shared memory (fixed order, so results are

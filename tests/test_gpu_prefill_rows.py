@@ -43,8 +43,8 @@ def chosen_logits(counts, n, seed):
     return dev(logits)
 
 
-# rows per expert at the edges of the token groups (8, 16, 24, 32), of the passes, none at all
-EDGES = [1, 8, 9, 16, 17, 24, 25, 32, 33, 40, 0, 65, 2, 3, 0, 31]
+# rows per expert at the edges of the token groups (4, 8, 16, 24, 32), of the passes, none at all
+EDGES = [1, 8, 9, 16, 17, 24, 25, 32, 33, 40, 0, 65, 2, 3, 4, 31, 5]
 
 
 @pytest.mark.parametrize("H,F", [(512, 256), (256, 512), (2048, 512), (512, 768)])
