@@ -1195,6 +1195,19 @@ int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const
   return launch_pdl(K, grid, threads, smem, stream, L);
 }
 
+int launch_token_layer(const tk::Geom& g, cudaStream_t s, const LayerDev& L) {
+  const dim3 grid(L.grid);
+  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false>>(grid, tk::kThreads, g.total, s, L);
+  // sharing by cost: two rows seldom meet in a tile (22.9 us a layer either way), and where a pass of both groups takes a CTA's
+  // pairs there is nothing to share out
+  const bool by_cost = L.n > 2 && static_cast<long long>(L.n) * L.K * L.FF > 2LL * L.grid * g.stage_pairs;
+  if (L.n < kRowsKernelMinRows)
+    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true>>(grid, tk::kThreads, g.total, s, L)
+                   : launch_layer<tk::token_layer_kernel<false, false, false>>(grid, tk::kThreads, g.total, s, L);
+  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true>>(grid, tk::kThreads, g.total, s, L)
+                 : launch_layer<tk::token_layer_kernel<true, false, false>>(grid, tk::kThreads, g.total, s, L);
+}
+
 }  // namespace
 
 // (tmap_dev.cuh; cuTensorMapEncodeTiled is reached through the runtime's driver entry point)
@@ -1443,8 +1456,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       a->workspace_bytes >= lay.items_total) {
     const tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid);
     if (g.total <= 227 * 1024 && g.down_tiles > 0 && g.rows_per_cta <= tk::kGroupWarps)
-      return a->n < kRowsKernelMinRows ? launch_layer<tk::token_layer_kernel<false>>(dim3(L.grid), tk::kThreads, g.total, s, L)
-                                       : launch_layer<tk::token_layer_kernel<true>>(dim3(L.grid), tk::kThreads, g.total, s, L);
+      return launch_token_layer(g, s, L);
   }
 
   int rc = kOk;

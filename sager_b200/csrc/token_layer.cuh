@@ -29,10 +29,10 @@
 // What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 15.7 us per
 // layer, of which 3.5 to the first barrier, 2 for picks and tables, 1.5 for the first bytes, 2 for
 // gate / up, 2 for the second barrier, 1 + 1 for h and the down rows; 26.6 with eight warps on whole
-// blocks and the selection in sequence). A further row costs 7 us - 22.1 / 29.7 / 36.4 us at 2 / 3 / 4 rows -,
-// where its bytes cost 2.2.
+// blocks and the selection in sequence). A further row costs 6 us - 22.6 / 29.2 / 33.6 us at 2 / 3 / 4 rows -,
+// where its bytes cost 2.2: the dots' instructions of a tile grow with its rows.
 //
-// Work split: gate / up by pairs (a flat range of (tile, pair) per CTA), down by output
+// Work split: gate / up by pairs (a flat range of (tile, pair) per CTA, of equal cost), down by output
 // rows. Contracts are those of the two-launch path: null table entry = absent expert
 // (zero contribution, id mailed), weight pointers may be only 2-byte aligned (then the
 // producer copies with plain loads), routing written to route_idx / route_w.
@@ -369,11 +369,12 @@ __device__ __forceinline__ void plain_done() {
   fence_proxy_async();
 }
 
-// CHAIN: layers of four token rows (see half_dots)
-template <bool CHAIN>
+// CHAIN: layers of four token rows (see half_dots). ONE: layers of one, which are a chain of short steps: what only more rows
+// need is neither executed nor fetched. BY_COST: layers whose CTAs take more pairs than a pass of both groups (see routed_share).
+template <bool CHAIN, bool ONE, bool BY_COST>
 __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const Geom G = geom(L.n, L.K, L.H, L.FF, L.E, gridDim.x);
+  const Geom G = geom(ONE ? 1 : L.n, L.K, L.H, L.FF, L.E, gridDim.x);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);              // [kRing]
   uint64_t* empty = full + kRing;                                  // [kRing]
   uint64_t* sh_full = empty + kRing;                               // shared expert's gate / up pairs
@@ -396,18 +397,46 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   float* ysm = reinterpret_cast<float*>(smem + G.off_y);           // [hrow][nr_max]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cta = blockIdx.x, grid = gridDim.x;
-  const int n = L.n, H = L.H, FF = L.FF, E = L.E, K = L.K;
+  const int n = ONE ? 1 : L.n, H = L.H, FF = L.FF, E = L.E, K = L.K;
   const bool has_shared = L.sh[0] != nullptr;
   unsigned long long* gctr = reinterpret_cast<unsigned long long*>(L.cnt + 12);
 
   // this CTA's shares: shared-expert pairs [sp0, sp1), output rows [r0, r1)
-  // (products stay below 2^31: at most 33 tiles x 8192 pairs x 192 CTAs)
+  // (products stay below 2^31: at most 33 tiles x 8192 pairs x a cost of 21 x 192 CTAs)
   const unsigned grid_inv = 0xFFFFFFFFu / static_cast<unsigned>(grid);
   auto share = [&](int total, int part) {        // total * part / grid: the estimate is at most one short
     const unsigned x = static_cast<unsigned>(total) * static_cast<unsigned>(part), q = __umulhi(x, grid_inv);
     return static_cast<int>(q + (x - q * static_cast<unsigned>(grid) >= static_cast<unsigned>(grid) ? 1u : 0u));
   };
   const int sp0 = share(FF, cta), sp1 = share(FF, cta + 1), r0 = share(H, cta), r1 = share(H, cta + 1);
+  // This CTA's share [pos, end) of the flat (tile, pair) range of the routed tiles; whole warps, after the tables. A pair costs
+  // about 0.25 + 1.2 per row of its tile (us per 16 pairs): in equal numbers of pairs the CTAs whose tile four rows share
+  // finished gate / up 8 us after the median one. Us per layer at 4 rows skewed / uniform and 3 rows: 39.0 / 37.0 and 31.1 with
+  // equal numbers, 33.6 / 34.4 and 29.2 by cost. As long as the two groups take a CTA's pairs in one pass each the
+  // numbers do not matter (and the code alone costs layers of hidden 512 a hundredth: they have a kernel without it).
+  auto routed_share = [&](int t_first, int tiles, int& pos, int& end) {
+    if (!BY_COST || tiles * FF <= grid * 2 * G.stage_pairs) {
+      pos = share(tiles * FF, cta);
+      end = share(tiles * FF, cta + 1);
+      return;
+    }
+    const int rows = lane < tiles ? __popc(tb.tile_mask[t_first + lane]) : 0, cost = lane < tiles ? 1 + 5 * rows : 0;
+    int sum = cost;                              // a pair of every tile up to this one
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int v = __shfl_up_sync(0xFFFFFFFFu, sum, off);
+      if (lane >= off) sum += v;
+    }
+    auto reciprocal = [](unsigned c) { return 0xFFFFFFFFu / c + 1; };      // (quotients below are exact: dividends stay below 2^27)
+    const unsigned inv = rows <= 1 ? reciprocal(6) : (rows == 2 ? reciprocal(11) : (rows == 3 ? reciprocal(16) : reciprocal(21)));
+    const int all = __shfl_sync(0xFFFFFFFFu, sum, 31) * FF, before = lane < tiles ? (sum - cost) * FF : 0x7FFFFFFF;
+    auto from = [&](int x) {
+      const int j = __popc(__ballot_sync(0xFFFFFFFFu, before <= x)) - 1;
+      return j * FF + static_cast<int>(__umulhi(static_cast<unsigned>(x - __shfl_sync(0xFFFFFFFFu, before, j)), __shfl_sync(0xFFFFFFFFu, inv, j)));
+    };
+    pos = from(share(all, cta));
+    end = from(share(all, cta + 1));
+  };
   const int nr = r1 - r0;
 
   const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
@@ -493,8 +522,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int T = tb.n_tiles;
     const int t_first = has_shared ? 1 : 0;
     // routed gate / up pairs: a flat range of (tile, pair) per CTA
-    const int P = (T - t_first) * FF, pb = share(P, cta + 1);
-    int pos = share(P, cta);
+    int pos, pb;
+    routed_share(t_first, T - t_first, pos, pb);
     const int cut = min(G.stage_pairs, (pb - pos + 1) / 2);          // both groups get work
     int tile = t_first + pos / FF, pair0 = pos - (tile - t_first) * FF;
     int issued = 0;
@@ -809,9 +838,10 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
 
   // ---- phase 3: gate / up of the routed tiles, SwiGLU; the groups take stages in turn ----
   {
-    const int P = (T - t_first) * FF, pb = share(P, cta + 1);
+    int pos, pb;
+    routed_share(t_first, T - t_first, pos, pb);
     const int group = warp / kGroupWarps;
-    int pos = share(P, cta), pair0 = pos % FF;
+    int pair0 = pos % FF;
     const int cut = min(G.stage_pairs, (pb - pos + 1) / 2);
     for (int i = 0; pos < pb && ok; ++i) {
       const int s = i % kRing, np = min(cut, min(FF - pair0, pb - pos));    // as the producer cuts the range

@@ -671,3 +671,31 @@ def test_fused_exchange_entry_points_with_one_rank(full_w, tokens, own_plan):
     assert torch.equal(recv, send)
     assert rel(x.float().cpu().numpy(), x_full.float().cpu().numpy()) <= 2.0 ** -10      # fp16 store after another add order
     assert lib().raw("sgr_status")(0) == 0
+
+
+@pytest.mark.parametrize("n", [3, 4])
+@pytest.mark.parametrize("meet", ["all", "pair", "none", "absent"])
+def test_token_layer_shares_by_cost(oracle, n, meet):
+    """Layers of three and four rows whose CTAs take more pairs than a pass of both groups: tiles of one to four rows in one
+    layer, every tile with all rows, no two rows in a tile, an absent expert among them. Every (tile, pair) has to be in exactly
+    one CTA's share: a pair left out or taken by a neighbour shows in h. Bias by row is not possible, so the rows' inputs choose."""
+    H, F, E, K = 2048, 256, 40, 8
+    w = synth.MoeWeights(H, F, E, DEV, seed=91, std=0.05)
+    x16 = synth.normal_fp16((n, H), 92 + n, DEV)
+    if meet == "all":
+        x16[1:] = x16[0]
+    elif meet != "none":
+        x16[1] = x16[0]
+    x_np = x16.cpu().numpy()
+    want = oracle_layer(oracle, w, x_np, x_np.astype(np.float32), K)
+    absent = (int(want["idx"][0, 2]),) if meet == "absent" else ()
+    if absent:
+        want = oracle_layer(oracle, w, x_np, x_np.astype(np.float32), K, absent=absent)
+    for rep in range(2):                         # (the second call finds the first one's h rows)
+        runner, x_out, out32 = run_layer(w, n, K, x16, absent=absent)
+        assert np.array_equal(runner.route_idx.cpu().numpy()[:n, :K], want["idx"][:, :K])
+        assert rel(out32.cpu().numpy(), want["out"]) < LAYER_TOL
+    # the row-streaming kernel adds a row's blocks in the same order from four rows on
+    if n == 4:
+        other = run_layer(w, n, K, x16, absent=absent, kernel="rows")[2]
+        assert torch.equal(out32, other)
