@@ -164,8 +164,7 @@ struct alignas(16) GEntry {
   volatile int there;           // down groups: the tile's h has been seen complete
 };
 static_assert(kListSlots > kAhead + kStageCount + 1 + 2, "a reader could be overtaken");
-constexpr int kZeroBytes = 272, kZeros = kHdr - kZeroBytes;     // zeros for b_row4: a block of codes with its padding
-static_assert(sizeof(GEntry) * kListSlots + 2048 <= kZeros, "group list exceeds the header");
+static_assert(sizeof(GEntry) * kListSlots + 2048 <= kHdr, "group list exceeds the header");
 
 // One warp: Q8_K-quantise block `hb` of h, rows `src` in shared memory, into the padded rows
 // [hrow0, hrow0 + ntok) of L.hq (arithmetic of src/kernels/cpu/q4_avx2.cpp:77-94 in the reference,
@@ -371,8 +370,6 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
     for (int e = tid; e < kPlanExperts; e += kThreads) reinterpret_cast<unsigned long long*>(plan_s + kPlanOffMask)[e] = 0ull;
     if (tid == 0) reinterpret_cast<int*>(plan_s + kPlanOffScan)[120] = 0;
   }
-  const unsigned char* const zeros = smem + kZeros;
-  if (tid < kZeroBytes / 4) reinterpret_cast<uint32_t*>(smem + kZeros)[tid] = 0u;
   unsigned char* smaps = smem + 1024;                                 // three 128-byte descriptors being patched
   uint32_t* tmpl = reinterpret_cast<uint32_t*>(smem + 1408);          // the two host-made descriptors
   if (tid == kPrepWarp * 32) {
@@ -841,24 +838,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         if (lane == 0) mbar_arrive(&wempty[s]);
       };
       w_released = true;
-      if (d_ntok <= 4) {
-        const unsigned char* x = st + kWBytes;
-        const uint4 h0 = *reinterpret_cast<const uint4*>(st + own_lo), h1 = *reinterpret_cast<const uint4*>(st + own_hi);
-        const int tig = lane & 3, gid = lane >> 2;
-        const float xd = *reinterpret_cast<const float*>(x + kXCodes + kTok * 16 + tig * 16);
-        warp_mma_block4(st + w_off, h0, h1, b_row4(x, kXqStride, zeros, lane), 16, lane, loaded,
-                        [&] {
-                          const uint2 sv = *reinterpret_cast<const uint2*>(x + kXCodes + (gid >> 1) * 16 + 8 * (tig & 1));
-                          const uint32_t lo = __byte_perm(sv.x & 0x007F007Fu, sv.y & 0x007F007Fu, 0x6420);
-                          const uint32_t hi = __byte_perm((sv.x >> 7) & 0x00FF00FFu, (sv.y >> 7) & 0x00FF00FFu, 0x6420);
-                          return gid & 1 ? hi : lo;
-                        },
-                        [&](int r, int isum, int msum) {
-                          const uint32_t dm = r ? h1.x : h0.x;
-                          const float dd = 0.0625f * h2f(static_cast<uint16_t>(dm & 0xFFFFu)), mm = h2f(static_cast<uint16_t>(dm >> 16));
-                          acc[0][r] += xd * (dd * static_cast<float>(isum) - mm * static_cast<float>(msum));
-                        });
-      } else if (d_ntok <= 8) warp_mma_block<1>(st + w_off, st + own_lo, st + own_hi, xt, acc, loaded);
+      if (d_ntok <= 8) warp_mma_block<1>(st + w_off, st + own_lo, st + own_hi, xt, acc, loaded);
       else warp_mma_block<2>(st + w_off, st + own_lo, st + own_hi, xt, acc, loaded);
     }
     __syncwarp();
@@ -889,9 +869,6 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
         if (d_ntok == 1) {
           const float g = acc[0][0], u = __shfl_down_sync(0xFFFFFFFFu, g, 16);
           if (lane < 16 && (lane & 1) == 0) hb[lane >> 1] = g / (1.f + expf(-g)) * u;
-        } else if (d_ntok <= 4) {
-          const float g = acc[0][0], u = acc[0][1];
-          if (tig < d_ntok) hb[tig * kHRow + gid] = g / (1.f + expf(-g)) * u;
         } else {
 #pragma unroll
           for (int n = 0; n < 2; ++n) {
@@ -917,12 +894,6 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
       }
       if (d_ntok == 1) {
         if ((lane & 1) == 0) L.ybuf[static_cast<size_t>(d.hrow0) * L.H + d.row0 + 16 * warp + (lane >> 1)] = acc[0][0];
-      } else if (d_ntok <= 4) {
-        if (tig < d_ntok) {
-          float* o = L.ybuf + static_cast<size_t>(d.hrow0 + tig) * L.H + d.row0 + 16 * warp + gid;
-          o[0] = acc[0][0];
-          o[8] = acc[0][1];
-        }
       } else {
         const int col = d.row0 + 16 * warp + gid;
 #pragma unroll

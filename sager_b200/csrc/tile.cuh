@@ -387,8 +387,8 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
 // The same for at most four token rows, with two of the MMA's eight columns to a token: the even sub-blocks' dots land in
 // column 2t, the odd ones' in 2t + 1 (each MMA's activation operand is zero in the other columns), so one set of results holds
 // both, and a lane scales the results of one token - half the multiply-adds, conversions and fp32 steps, which for eight
-// columns are spent on tokens that are not there (us per layer of 2048 / 512 / 256 experts at 64 skewed, 32 skewed, 8 rows: 92.2 /
-// 73.5 / 50.2 with eight columns, 90.1 / 72.5 / 49.5). Results: rows gid and gid + 8, token tig.
+// columns are spent on tokens that are not there (prefill of 96 rows over 256 experts, four layers: 512 -> 504 us; in the decode
+// layer's row-streaming kernel the tiles gain as much, but the larger kernel costs every layer 0.8 to 1.2 us more). Results: rows gid and gid + 8, token tig.
 //   b_ptr   this lane's ldmatrix row (b_row4), advanced by 64 bytes per pair of sub-blocks, + mid_pad after two
 //   min_b   sub-block sums 4 (tig & 1) .. + 3 of token gid / 2: their low parts in even gid, high parts (bsum = 128 hi + lo) in odd
 //   fold(row, isum, msum): the fp32 steps; isum is sixteen-fold
