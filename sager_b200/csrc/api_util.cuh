@@ -52,6 +52,15 @@ int launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cuda
   return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? 0 : 4 /* kErrLaunch */;
 }
 
+// Whether a layer's weights are read under the policy that makes them the first to leave L2. As ordinary lines they push out what
+// every layer needs again: 2048 / 512 / 256 experts at 64 / 8 / 4 / 1 rows 88.9 / 48.7 / 33.4 / 15.7 us a layer, 81.5 / 44.1 / 32.8 /
+// 15.4 as the first to leave; prefill of 96 / 777 / 2048 rows, two layers, 257 / 556 / 864 -> 248 / 546 / 853. What a model keeps in
+// L2 between two uses of a layer is not known here: a layer of more than an eighth of it (126 MB) is taken for one of
+// many. Small layers (512 / 256 / 16 experts, 4 MB, twelve of them) lose by it: 11.5 -> 11.8 us at one row.
+inline bool streams_weights(int hidden, int n_ff, int n_expert) {
+  return static_cast<long long>(hidden) * n_ff / 256 * 144 * 3 * n_expert > (16LL << 20);
+}
+
 // ---- tensor-core GEMM of Q4_K experts over their routed rows (grouped_gemm_i8.cu) ----
 // Operand rows: the quantised activations as the GEMM's fp16 tiles want them, kOpBlk bytes per 256 values -
 // 256 codes in K order (0, 2, 1, 3 of every four), eight low and eight high parts of the sub-block sums
@@ -77,6 +86,7 @@ struct ExpertGemm {
   uint16_t* y;
   int n_rows, k, n_expert;
   bool operand_rows;
+  bool stream;                  // the weights' L2 policy (streams_weights)
   const void* maps;             // with operand rows: the descriptors; n_rows is then a multiple of 128
   const void* shared_w;
   const unsigned char* shared_xq;

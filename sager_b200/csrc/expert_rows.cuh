@@ -338,6 +338,8 @@ __device__ __forceinline__ int build_plan_shared(const LayerDev& L, unsigned cha
   return tiles_total + sh_tiles;
 }
 
+// STREAM: weights first to leave L2 (streams_weights)
+template <bool STREAM>
 __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
@@ -602,11 +604,11 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           if (lane == 0) {
             mbar_expect_tx(&full[s], kWBytes);      // this lane's arrival, with the bytes to come
             if (wk.kind == 0) {
-              tma_load_box(st, maps, blk * kW4, row0, &full[s]);
-              tma_load_box(st + kHalfBytes, maps + 128, blk * kW4, row0, &full[s]);
+              tma_load_box<STREAM>(st, maps, blk * kW4, row0, &full[s]);
+              tma_load_box<STREAM>(st + kHalfBytes, maps + 128, blk * kW4, row0, &full[s]);
             } else {
-              tma_load_box(st, maps, blk * kW4, row0, &full[s]);
-              tma_load_box(st + kHalfBytes, maps, blk * kW4, row0 + kHalfRows, &full[s]);
+              tma_load_box<STREAM>(st, maps, blk * kW4, row0, &full[s]);
+              tma_load_box<STREAM>(st + kHalfBytes, maps, blk * kW4, row0 + kHalfRows, &full[s]);
             }
           }
         } else {
@@ -633,6 +635,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           __syncwarp();                            // every lane's part of the stage (and of its descriptor) is written
           if (lane == 0) mbar_arrive(&full[s]);
         }
+        __syncwarp();                              // (the copies' operands pass through uniform registers: no lane runs ahead)
         ++q;
         if (lane == 0) *issued = static_cast<unsigned>(q);
         if (++s == kStageCount) { s = 0; ph ^= 1u; }

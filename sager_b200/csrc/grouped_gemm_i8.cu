@@ -190,7 +190,8 @@ __device__ __forceinline__ bool for_jobs(const GemmArgs& a, const Unit& u, F f) 
 }
 __device__ __forceinline__ int fills_of(const GemmArgs& a, const Unit& u) { return a.nb <= 2 ? a.nb : u.n_tiles * a.nb; }
 
-template <bool DUAL, bool RAW>
+// STREAM: weights first to leave L2 (streams_weights)
+template <bool DUAL, bool RAW, bool STREAM>
 __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(const GemmArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
           if (align == 0) {
             if (lane == 0) {
               mbar_expect_tx(&bar[kBarWFull + s], kStageBytes);
-              tma_load_box(stage, map + 128 * m, b * kW4, row0, &bar[kBarWFull + s]);
+              tma_load_box<STREAM>(stage, map + 128 * m, b * kW4, row0, &bar[kBarWFull + s]);
             }
           } else {                                               // a base off a 16-byte boundary
             const unsigned char* src = (m == 0 ? u.w0 : u.w1) + static_cast<size_t>(row0) * row_bytes + b * kW4;
@@ -676,7 +677,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
   }
 }
 
-template <bool DUAL, bool RAW>
+template <bool DUAL, bool RAW, bool STREAM>
 int launch_gemm(GemmArgs a, cudaStream_t stream) {
   a.status = status_word();
   const int sms = device_sms();
@@ -699,8 +700,8 @@ int launch_gemm(GemmArgs a, cudaStream_t stream) {
   const long long n_items = static_cast<long long>(a.groups) * a.n_expert + a.s_items;
   if (n_items > 0x7FFFFFFF - 1024) return kErrUnsupported;
   a.n_items = static_cast<int>(n_items);
-  if (!opt_in_smem<grouped_gemm_kernel<DUAL, RAW>>(kGemmSmem)) return kErrLaunch;
-  return launch_pdl(grouped_gemm_kernel<DUAL, RAW>, dim3(std::min(a.n_items, sms)), Cfg<RAW>::kThreads, kGemmSmem, stream, a);
+  if (!opt_in_smem<grouped_gemm_kernel<DUAL, RAW, STREAM>>(kGemmSmem)) return kErrLaunch;
+  return launch_pdl(grouped_gemm_kernel<DUAL, RAW, STREAM>, dim3(std::min(a.n_items, sms)), Cfg<RAW>::kThreads, kGemmSmem, stream, a);
 }
 
 // Rows of fp16 values - or SwiGLU of two rows, rounded to fp16 as silu_mul_f16 does - -> operand rows
@@ -778,12 +779,14 @@ int gemm_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, uint16
   GemmArgs a = args_of(g);
   a.tab1 = tab_up; a.y1 = y_up;
   a.sw1 = static_cast<const unsigned char*>(shared_up); a.sy1 = shared_y_up;
-  return g.operand_rows ? launch_gemm<true, false>(a, stream) : launch_gemm<true, true>(a, stream);
+  if (!g.operand_rows) return launch_gemm<true, true, false>(a, stream);
+  return g.stream ? launch_gemm<true, false, true>(a, stream) : launch_gemm<true, false, false>(a, stream);
 }
 int gemm_grouped(const ExpertGemm& g, cudaStream_t stream) {
   GemmArgs a = args_of(g);
   a.map0 = 2;
-  return g.operand_rows ? launch_gemm<false, false>(a, stream) : launch_gemm<false, true>(a, stream);
+  if (!g.operand_rows) return launch_gemm<false, true, false>(a, stream);
+  return g.stream ? launch_gemm<false, false, true>(a, stream) : launch_gemm<false, false, false>(a, stream);
 }
 int quantize_operand(const uint16_t* x0, const uint16_t* u0, void* out0, long long rows0, const int* d_rows,
                      const uint16_t* x1, const uint16_t* u1, void* out1, long long rows1, int k, const ExpertMaps& em, bool make_maps,

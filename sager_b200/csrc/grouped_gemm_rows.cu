@@ -142,7 +142,8 @@ __device__ __forceinline__ void rows_block(const unsigned char* a_ptr, const uns
   }
 }
 
-template <bool DUAL>
+// STREAM: weights first to leave L2 (streams_weights)
+template <bool DUAL, bool STREAM>
 __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const RowsArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);            // [kStages] copies landed
@@ -230,8 +231,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
           if (!absent && align == 0) {
             if (lane == 0) {
               mbar_expect_tx(&full[s], kWBytes);
-              tma_load_box(st, map0, b * kW4, row0, &full[s]);
-              tma_load_box(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
+              tma_load_box<STREAM>(st, map0, b * kW4, row0, &full[s]);
+              tma_load_box<STREAM>(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
             }
           } else {
             if (!absent) {                           // a base off a 16-byte boundary: plain copies
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
   }
 }
 
-template <bool DUAL>
+template <bool DUAL, bool STREAM>
 int launch_rows(RowsArgs a, cudaStream_t stream) {
   a.status = status_word();
   const int sms = device_sms();
@@ -398,8 +399,8 @@ int launch_rows(RowsArgs a, cudaStream_t stream) {
   const long long n_items = static_cast<long long>(a.groups) * a.n_expert + a.s_items;
   if (n_items > 0x7FFFFFFF) return kErrUnsupported;
   a.n_items = static_cast<int>(n_items);
-  if (!opt_in_smem<grouped_gemm_rows_kernel<DUAL>>(kSmem)) return kErrLaunch;
-  return launch_pdl(grouped_gemm_rows_kernel<DUAL>, dim3(std::min(a.n_items, sms)), kThreads, kSmem, stream, a);
+  if (!opt_in_smem<grouped_gemm_rows_kernel<DUAL, STREAM>>(kSmem)) return kErrLaunch;
+  return launch_pdl(grouped_gemm_rows_kernel<DUAL, STREAM>, dim3(std::min(a.n_items, sms)), kThreads, kSmem, stream, a);
 }
 
 // Rows of fp16 values -> Q8_K rows in blocks of kRowBlk bytes, two slabs
@@ -465,9 +466,12 @@ int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, c
   RowsArgs a = args_of(g, maps, 0);
   a.tab1 = tab_up;
   a.sw1 = static_cast<const unsigned char*>(shared_up);
-  return launch_rows<true>(a, stream);
+  return g.stream ? launch_rows<true, true>(a, stream) : launch_rows<true, false>(a, stream);
 }
-int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream) { return launch_rows<false>(args_of(g, maps, 2), stream); }
+int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream) { 
+  const RowsArgs a = args_of(g, maps, 2);
+  return g.stream ? launch_rows<false, true>(a, stream) : launch_rows<false, false>(a, stream);
+}
 
 int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_rows, const uint16_t* x1, void* out1, long long rows1,
                   int k, const ExpertMaps& em, bool make_maps, cudaStream_t stream) {

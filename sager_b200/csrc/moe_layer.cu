@@ -1195,17 +1195,18 @@ int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const
   return launch_pdl(K, grid, threads, smem, stream, L);
 }
 
+template <bool STREAM>
 int launch_token_layer(const tk::Geom& g, cudaStream_t s, const LayerDev& L) {
   const dim3 grid(L.grid);
-  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false>>(grid, tk::kThreads, g.total, s, L);
+  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
   // sharing by cost: two rows seldom meet in a tile (22.9 us a layer either way), and where a pass of both groups takes a CTA's
   // pairs there is nothing to share out
   const bool by_cost = L.n > 2 && static_cast<long long>(L.n) * L.K * L.FF > 2LL * L.grid * g.stage_pairs;
   if (L.n < kRowsKernelMinRows)
-    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true>>(grid, tk::kThreads, g.total, s, L)
-                   : launch_layer<tk::token_layer_kernel<false, false, false>>(grid, tk::kThreads, g.total, s, L);
-  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true>>(grid, tk::kThreads, g.total, s, L)
-                 : launch_layer<tk::token_layer_kernel<true, false, false>>(grid, tk::kThreads, g.total, s, L);
+    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                   : launch_layer<tk::token_layer_kernel<false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                 : launch_layer<tk::token_layer_kernel<true, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
 }
 
 }  // namespace
@@ -1359,6 +1360,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
   L.hbuf = reinterpret_cast<float*>(ws + lay.hbuf);
   L.ybuf = reinterpret_cast<float*>(ws + lay.ybuf);
   L.n_max = a->n_max;
+  const bool stream_weights = streams_weights(a->hidden, a->n_ff, a->n_expert);
   // (null: the address lookup failed - a first call on this device made inside stream capture, or a
   // device ordinal beyond the table; the kernels write through this pointer when a wait gives up)
   L.status = status_word();
@@ -1456,7 +1458,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       a->workspace_bytes >= lay.items_total) {
     const tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid);
     if (g.total <= 227 * 1024 && g.down_tiles > 0 && g.rows_per_cta <= tk::kGroupWarps)
-      return launch_token_layer(g, s, L);
+      return stream_weights ? launch_token_layer<true>(g, s, L) : launch_token_layer<false>(g, s, L);
   }
 
   int rc = kOk;
@@ -1486,7 +1488,8 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       rc = launch_layer<rearm_kernel>(dim3(1), 256, 0, s, L);
       if (rc != kOk) return rc;
     }
-    rc = launch_layer<rs::expert_rows_kernel>(dim3(sms), rs::kThreads, rs::kSmem, s, L);
+    rc = stream_weights ? launch_layer<rs::expert_rows_kernel<true>>(dim3(sms), rs::kThreads, rs::kSmem, s, L)
+                        : launch_layer<rs::expert_rows_kernel<false>>(dim3(sms), rs::kThreads, rs::kSmem, s, L);
   } else if (stages & 6) {
     // geometry the consumer mapping was written for: a tile of rows is one 16-row
     // group, or at most eight (group, super-block) units

@@ -91,6 +91,24 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
+// L2 policy of weights that are read once: first to leave, so that they do not push out what the kernels after this one need -
+// their code, router rows, activations (streams_weights, api_util.cuh, has the line and the figures). A constant where it is used:
+// a policy chosen at run time and kept in a register across the weight warp's loop left copies that did not complete - waits ran
+// out -, most likely because the copies' operands pass through uniform registers and the warp's other lanes ran ahead.
+__device__ __forceinline__ uint64_t evict_first_policy() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+// bulk_g2s, under that policy if STREAM (a parameter of the kernel: both kinds of copies in one cost small layers a hundredth)
+template <bool STREAM>
+__device__ __forceinline__ void bulk_g2s_weights(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  if constexpr (!STREAM) bulk_g2s(dst, src, bytes, bar);
+  else asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+      ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(evict_first_policy())
+      : "memory");
+}
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }

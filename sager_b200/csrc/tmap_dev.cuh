@@ -23,10 +23,15 @@ __device__ __forceinline__ void tmap_publish(void* gmem_map, void* smem_map) {
 __device__ __forceinline__ void tmap_acquire(const void* gmem_map) {
   asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(gmem_map) : "memory");
 }
-// box (144 bytes x 128 rows) at byte column x, row y; dst 128-byte aligned, x a multiple of 16
+// box (144 bytes x 128 rows) at byte column x, row y; dst 128-byte aligned, x a multiple of 16; STREAM: evict_first_policy
+template <bool STREAM>
 __device__ __forceinline__ void tma_load_box(void* dst, const void* gmem_map, int x, int y, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-               ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
+  if constexpr (STREAM)
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+                 ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(evict_first_policy()) : "memory");
+  else
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
 
 // The descriptors of a layer's experts (ExpertMaps, api_util.cuh), made by CTAs of a launch before the GEMMs; and the counters

@@ -371,7 +371,8 @@ __device__ __forceinline__ void plain_done() {
 
 // CHAIN: layers of four token rows (see half_dots). ONE: layers of one, which are a chain of short steps: what only more rows
 // need is neither executed nor fetched. BY_COST: layers whose CTAs take more pairs than a pass of both groups (see routed_share).
-template <bool CHAIN, bool ONE, bool BY_COST>
+// STREAM: weights first to leave L2 (streams_weights).
+template <bool CHAIN, bool ONE, bool BY_COST, bool STREAM>
 __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
   const Geom G = geom(ONE ? 1 : L.n, L.K, L.H, L.FF, L.E, gridDim.x);
@@ -471,15 +472,15 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         if (lane == 0) {
           if (np > 0) {
             mbar_expect_tx(sh_full, static_cast<uint32_t>(2 * np * G.rb_h));
-            bulk_g2s(sh_stage, L.sh[0] + static_cast<size_t>(sp0) * G.rb_h, static_cast<uint32_t>(np * G.rb_h), sh_full);
-            bulk_g2s(sh_stage + static_cast<size_t>(np) * G.rb_h, L.sh[1] + static_cast<size_t>(sp0) * G.rb_h,
+            bulk_g2s_weights<STREAM>(sh_stage, L.sh[0] + static_cast<size_t>(sp0) * G.rb_h, static_cast<uint32_t>(np * G.rb_h), sh_full);
+            bulk_g2s_weights<STREAM>(sh_stage + static_cast<size_t>(np) * G.rb_h, L.sh[1] + static_cast<size_t>(sp0) * G.rb_h,
                      static_cast<uint32_t>(np * G.rb_h), sh_full);
           } else {
             mbar_arrive_one(sh_full);
           }
           if (nr > 0) {
             mbar_expect_tx(shdn_full, static_cast<uint32_t>(nr * G.rb_f));
-            bulk_g2s(dn, L.sh[2] + static_cast<size_t>(r0) * G.rb_f, static_cast<uint32_t>(nr * G.rb_f), shdn_full);
+            bulk_g2s_weights<STREAM>(dn, L.sh[2] + static_cast<size_t>(r0) * G.rb_f, static_cast<uint32_t>(nr * G.rb_f), shdn_full);
           } else {
             mbar_arrive_one(shdn_full);
           }
@@ -553,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       __syncwarp();
       const int jl = j0 + lane;                     // a lane per tile
       if (bytes > 0 && md == 0)
-        bulk_g2s(to + static_cast<size_t>(lane) * G.slot_bytes, tb.w[2][jl] + static_cast<size_t>(r0) * G.rb_f,
+        bulk_g2s_weights<STREAM>(to + static_cast<size_t>(lane) * G.slot_bytes, tb.w[2][jl] + static_cast<size_t>(r0) * G.rb_f,
                  static_cast<uint32_t>(nr * G.rb_f), full_bar);
       __syncwarp();
     };
@@ -586,8 +587,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       if (lane == 0) {
         if (mode == 0) {
           mbar_expect_tx(&full[s], static_cast<uint32_t>(2 * np * G.rb_h));
-          bulk_g2s(st, tb.w[0][tile] + static_cast<size_t>(pair0) * G.rb_h, static_cast<uint32_t>(np * G.rb_h), &full[s]);
-          bulk_g2s(st + static_cast<size_t>(np) * G.rb_h, tb.w[1][tile] + static_cast<size_t>(pair0) * G.rb_h,
+          bulk_g2s_weights<STREAM>(st, tb.w[0][tile] + static_cast<size_t>(pair0) * G.rb_h, static_cast<uint32_t>(np * G.rb_h), &full[s]);
+          bulk_g2s_weights<STREAM>(st + static_cast<size_t>(np) * G.rb_h, tb.w[1][tile] + static_cast<size_t>(pair0) * G.rb_h,
                    static_cast<uint32_t>(np * G.rb_h), &full[s]);
         } else {
           mbar_arrive_one(&full[s]);
