@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemv_stream_kernel(const Ge
         const long long nblk = total_blocks - b0 < kStreamBlocks ? total_blocks - b0 : kStreamBlocks;
         const uint32_t bytes = static_cast<uint32_t>(nblk) * kW4;
         mbar_expect_tx(full + s, bytes);
-        bulk_g2s(ring + s * kStreamStageBytes, a.w[0] + b0 * kW4, bytes, full + s);
+        bulk_g2s_weights<true>(ring + s * kStreamStageBytes, a.w[0] + b0 * kW4, bytes, full + s);
       }
     }
   } else {
@@ -405,6 +405,8 @@ __device__ __forceinline__ void direct_blocks(const DirectArgs& a, const uint4 (
   }
 }
 
+// (Weights as the first to leave L2: 24 layers at 2 / 4 / 8 rows 15.2 / 15.8 / 17.3 us a layer as ordinary lines, 13.0 / 13.5 / 15.4;
+// 8 layers that L2 can hold 14.5 and 14.1.)
 // NI: block columns per warp (1 for rows of up to eight blocks); LONG: rows of more than 32 blocks, 32 at a time
 template <int NI, bool F16, bool LONG = false>
 __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const DirectArgs a) {
@@ -425,9 +427,9 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
                                 (static_cast<size_t>(row - a.first_row(m)) * nb + blk0 + c0) * kW4;
 #pragma unroll
       for (int i = 0; i < NI; ++i) {
-        hdr[h][i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+        hdr[h][i] = load_weights<true>(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
 #pragma unroll
-        for (int g = 0; g < 4; ++g) q[h][i][g] = __ldg(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
+        for (int g = 0; g < 4; ++g) q[h][i][g] = load_weights<true>(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
       }
     }
   };
@@ -480,7 +482,8 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
 // exactly by shuffle over its four lanes, the blocks' terms in the tile kernels' shuffle tree.
 constexpr int kDirectGroup = 80, kDirectBlock = 4 * kDirectGroup;
 
-template <int NI, bool F16>
+// STREAM: weights first to leave L2 (launch_direct)
+template <int NI, bool F16, bool STREAM>
 __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct1_kernel(const DirectArgs a) {
   __shared__ __align__(16) unsigned char xs[32 * kDirectBlock];
   const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -493,9 +496,9 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct1_kernel(const D
   uint4 hdr[NI], q0[NI], q1[NI];
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
-    hdr[i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
-    q0[i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 16 + 32 * g));
-    q1[i] = __ldg(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 32 + 32 * g));
+    hdr[i] = load_weights<STREAM>(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+    q0[i] = load_weights<STREAM>(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 16 + 32 * g));
+    q1[i] = load_weights<STREAM>(reinterpret_cast<const uint4*>(wb + i * 8 * kW4 + 32 + 32 * g));
   }
   pdl_wait();
   pdl_launch_dependents();
@@ -564,9 +567,14 @@ int launch_direct(const DirectArgs& a, cudaStream_t stream) {
   if (a.n_tokens == 1) {
     const int rows_cta = kDirectWarps * std::max(1, 8 / a.nb);
     const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
-    if (a.nb <= 8) return launch_pdl(gemv_direct1_kernel<1, F16>, grid, threads, 0, stream, a);
-    if (a.nb == 16) return launch_pdl(gemv_direct1_kernel<2, F16>, grid, threads, 0, stream, a);
-    return launch_pdl(gemv_direct1_kernel<4, F16>, grid, threads, 0, stream, a);
+    // Matrices of four megabytes and more are taken for those of a model that L2 does not hold between two tokens: as the first to
+    // leave, its weights no longer push out the kernels' code and activations. 40 / 24 layers of 4096 + 2 x 512 from 2048 and 2048
+    // from 4096: 11.0 / 10.5 us a layer, 10.3 / 9.7; where L2 could hold all of it (8 layers) 9.9 against 10.7, and
+    // smaller matrices (2048 + 2 x 256 from 1024, 12 layers) 6.9 against 7.2.
+    const bool first = static_cast<long long>(a.rows_cum[2]) * a.nb * kW4 >= 4 << 20;
+    if (a.nb <= 8) return launch_pdl(first ? gemv_direct1_kernel<1, F16, true> : gemv_direct1_kernel<1, F16, false>, grid, threads, 0, stream, a);
+    if (a.nb == 16) return launch_pdl(first ? gemv_direct1_kernel<2, F16, true> : gemv_direct1_kernel<2, F16, false>, grid, threads, 0, stream, a);
+    return launch_pdl(first ? gemv_direct1_kernel<4, F16, true> : gemv_direct1_kernel<4, F16, false>, grid, threads, 0, stream, a);
   }
   const int rows_cta = 16 * std::max(1, kDirectWarps / a.nb);
   const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
         const int nr = min(a.rows_per_stage, a.n_rows - r0);
         const uint32_t bytes = static_cast<uint32_t>(nr) * row_bytes;
         mbar_expect_tx(full + s, bytes);
-        bulk_g2s(ring + static_cast<size_t>(s) * stage_bytes, a.w + static_cast<size_t>(r0) * row_bytes, bytes, full + s);
+        bulk_g2s_weights<true>(ring + static_cast<size_t>(s) * stage_bytes, a.w + static_cast<size_t>(r0) * row_bytes, bytes, full + s);
       }
     }
   } else {

@@ -109,6 +109,21 @@ __device__ __forceinline__ void bulk_g2s_weights(void* dst, const void* src, uin
       ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(evict_first_policy())
       : "memory");
 }
+// the same for weights that go straight into registers
+template <bool STREAM>
+__device__ __forceinline__ uint4 load_weights(const uint4* p) {
+  if constexpr (!STREAM) return __ldg(p);
+  uint4 v;
+  asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(evict_first_policy()));
+  return v;
+}
+template <bool STREAM>
+__device__ __forceinline__ uint2 load_weights(const uint2* p) {
+  if constexpr (!STREAM) return __ldg(p);
+  uint2 v;
+  asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(evict_first_policy()));
+  return v;
+}
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
