@@ -25,9 +25,10 @@ using namespace sgr;
 
 namespace {
 // Up to this many routed rows per expert on average the row-streaming GEMM takes the expert stage: its work grows with the rows,
-// the tcgen05 form's with the weights. Two layers of 2048 / 512 / 256 experts, us: 3 rows per expert 255 against 405 for the
-// tcgen05 form, 8 314 / 464, 16 423 / 532, 24 553 / 579, 28 625 / 611; of 1024 / 512 / 128: 16 170 / 190, 24 200 / 204.
-constexpr int kFewRows = 24;
+// the tcgen05 form's with the weights. Two layers of 2048 / 512 / 256 experts, us, against the tcgen05 form: 16 rows per expert
+// 382 / 502, 24 497 / 546, 28 558 / 575, 31 608 / 587; of 1024 / 512 / 128: 24 183 / 193, 26 192 / 198, 30 212 / 206; of 2048 / 256 /
+// 64: 20 132 / 150, 24 148 / 144, 29 153 / 151.
+constexpr int kFewRows = 26;
 // x[row] += sum_k w[row][k] * y_grouped[gslot[row][k]] (k = 0 .. K-1, in this order; a route that was
 // not computed, gslot < 0, adds nothing) + w[row][K] * sh_y[row] (when there is a shared expert):
 // scatter_routed_f16 + the strided copy + moe_combine_batched_f16 of the reference's sequence
