@@ -173,12 +173,13 @@ router_logits_staged_kernel(const float* __restrict__ w, const uint16_t* __restr
   };
 
   const int chunks = (k + T::kCols - 1) / T::kCols;
-#pragma unroll
-  for (int c = 0; c < T::kSlots - 1; ++c) fill_w(c);             // (W does not depend on the kernel before)
-  pdl_wait();
+  pdl_wait();                                   // (a caller's kernel may have written W as well as x)
   pdl_launch_dependents();
 #pragma unroll
-  for (int c = 0; c < T::kSlots - 1; ++c) fill_x(c);
+  for (int c = 0; c < T::kSlots - 1; ++c) {
+    fill_w(c);
+    fill_x(c);
+  }
   asm volatile("cp.async.wait_group %0;" ::"n"(T::kSlots - 2) : "memory");
   __syncthreads();
   convert(0);
