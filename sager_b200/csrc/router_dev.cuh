@@ -63,9 +63,10 @@ __device__ __forceinline__ void router_row_dot(const float* __restrict__ wrow,
 // number l / (32 / (R * T)), row-major.
 template <int R, int T>
 __device__ __forceinline__ float router_tile_dot(const float* ws, const uint16_t* xs, int k, int lane) {
-  float v[R * T];
+  // two tokens share a packed fp32 FMA (each component rounds as the scalar instruction): 64 rows, 81.9 -> 81.4 us per layer
+  unsigned long long sum[R * T / 2];
 #pragma unroll
-  for (int i = 0; i < R * T; ++i) v[i] = 0.f;
+  for (int i = 0; i < R * T / 2; ++i) sum[i] = 0ull;
   // the loads of S steps are issued ahead of the FMAs of the S steps before (k is a multiple of 256: S divides the steps)
   constexpr int S = T == 2 ? 8 : 4;
   uint32_t raw[2][S][T / 2];
@@ -91,10 +92,14 @@ __device__ __forceinline__ float router_tile_dot(const float* ws, const uint16_t
 #pragma unroll
     for (int j = 0; j < S; ++j)
 #pragma unroll
-      for (int t = 0; t < T; ++t) {
-        const float x = h2f(static_cast<uint16_t>(raw[b][j][t / 2] >> (16 * (t & 1))));
+      for (int t = 0; t < T / 2; ++t) {
+        unsigned long long x, ww;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(h2f(static_cast<uint16_t>(raw[b][j][t] & 0xFFFFu))), "f"(h2f(static_cast<uint16_t>(raw[b][j][t] >> 16))));
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r * T + t] = fmaf(w[b][j][r], x, v[r * T + t]);
+        for (int r = 0; r < R; ++r) {
+          asm("mov.b64 %0, {%1, %1};" : "=l"(ww) : "f"(w[b][j][r]));
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[r * T / 2 + t]) : "l"(ww), "l"(x));
+        }
       }
   };
   load(0, lane);
@@ -105,6 +110,9 @@ __device__ __forceinline__ float router_tile_dot(const float* ws, const uint16_t
     if (kk + 2 * S * 32 < k) load(0, kk + 2 * S * 32);
     if (kk + S * 32 < k) add(1);
   }
+  float v[R * T];
+#pragma unroll
+  for (int i = 0; i < R * T / 2; ++i) asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2 * i]), "=f"(v[2 * i + 1]) : "l"(sum[i]));
   int off = 16;
 #pragma unroll
   for (int m = R * T / 2; m > 0; m >>= 1, off >>= 1) {
