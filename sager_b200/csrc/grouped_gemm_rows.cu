@@ -238,10 +238,12 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
             if (!absent) {                           // a base off a 16-byte boundary: plain copies
               const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
               const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
-              warp_copy_unaligned(st, kWBytes / 16, lane, align, [&](int p) {
-                const int r = p / 9, h = r >> 7;
-                return (h ? b1 : b0) + static_cast<size_t>(r & 127) * row_bytes + (p - r * 9) * 16;
-              });
+#pragma unroll 1
+              for (int h = 0; h < 2; ++h)
+                warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
+                  const int r = p / 9;
+                  return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
+                });
               asm volatile("cp.async.wait_all;" ::: "memory");
               fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
             }
