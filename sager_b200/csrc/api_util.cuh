@@ -88,6 +88,7 @@ struct ExpertGemm {
   bool operand_rows;
   bool stream;                  // the weights' L2 policy (streams_weights)
   const void* maps;             // with operand rows: the descriptors; n_rows is then a multiple of 128
+  long long routes;             // routed rows at most (gemm_rows_*)
   const void* shared_w;
   const unsigned char* shared_xq;
   uint16_t* shared_y;

@@ -11,7 +11,7 @@
 // are applied to the int32 results.
 //
 // Persistent, one CTA per SM. A unit is 128 (gate, up) row pairs, or 256 rows, of one expert and at most 32 of its
-// token rows; its block columns stream through a ring of four stages (256 blocks of 144 bytes by two TMA copies, and
+// token rows, and is handed out by itself, so that the passes of a hot expert spread over the SMs; its block columns stream through a ring of four stages (256 blocks of 144 bytes by two TMA copies, and
 // that block of the token rows by one bulk copy each). Sixteen consumer warps, one weight warp, two activation warps; a
 // consumer returns its share of the weight bytes as soon as they are in registers. Gate and up rows of the same index meet
 // in a warp, so SwiGLU happens on the accumulators (rounded to fp16 first, as the reference's staged rows are). Waits are
@@ -51,7 +51,7 @@ struct RowsArgs {
   uint16_t *y, *sy;                    // [slots][n_rows]
   const unsigned char *sw0, *sw1;      // the shared expert (null: none)
   int n_rows, nb, n_expert, groups;    // row groups per matrix
-  int s_rows, s_step, s_items, n_items;
+  int s_rows, s_step, s_items;
   unsigned* next;                      // items handed out beyond the first of every CTA
   int* status;
 };
@@ -178,8 +178,14 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
 
   if (warp == kWeightWarp) {
     // ---------------- weights ----------------
-    // Items are handed out as CTAs come to want them: with rounds of fixed length the slowest CTA had 293,000 cycles of
-    // 241,000 on average (777 rows over 256 experts). The three round trips of a new item hide behind four full stages.
+    // Items are units: one pass of an expert's token rows over one row group, handed out as CTAs come to want them. (With rounds of
+    // fixed length the slowest CTA had 293,000 cycles of 241,000 on average, 777 rows over 256 experts. With all passes of an
+    // expert in one item a chunk waited for its hot experts: two layers, 832 rows over 256 experts, 439 us evenly spread, 804
+    // with a fifth of the experts in 70 % of the routes, 1409 with one in almost all of them; 439 / 469 / 421 by passes.)
+    // The passes of a row group follow one another, so that the CTAs that read the same weights do so together. Where an item
+    // lies is looked up in a window of 32 experts that only moves on, a lane per expert, while the item before it streams; the
+    // next window's loads are under way before it is needed. (96 rows, two layers: 228 us with loads and look-up
+    // between two items, 220 with the loads ahead, 214 like this.)
     const int row_bytes = a.nb * kW4;
     unsigned k = 0;                                  // units published
     auto publish = [&](int slot0, int nt, int flags) {
@@ -191,69 +197,133 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
       }
       ++k;
     };
-    unsigned item = blockIdx.x;
-    while (item < static_cast<unsigned>(a.n_items)) {
+    int e0 = 0, w_slot, w_rows, w_end = 0;           // the window: this lane's expert's first slot and rows, items up to and with it
+    const unsigned char *w_0, *w_1;                  // ... and its matrices
+    int n_slot = 0, n_to = 0;                        // the same of the window after it, on its way
+    const unsigned char *n_0 = nullptr, *n_1 = nullptr;
+    auto passes_of = [](int rows) { return (rows + kTok - 1) / kTok; };
+    auto request = [&](int e) {
+      n_slot = n_to = 0;
+      if (e < a.n_expert) {
+        n_slot = __ldg(a.off + e);
+        n_to = __ldg(a.off + e + 1);
+        n_0 = a.tab0[e];
+        n_1 = DUAL ? a.tab1[e] : n_0;
+      }
+    };
+    auto window = [&](int before) {                  // the window at e0 becomes the present one
+      const int to = n_to;
+      w_slot = n_slot;
+      w_0 = n_0;
+      w_1 = n_1;
+      request(e0 + 32 + lane);
+      w_rows = to - w_slot;
+      if (!__any_sync(0xFFFFFFFFu, w_rows > kTok)) {           // (a scan costs a launch of short items 0.6 us at its start)
+        w_end = __popc(__ballot_sync(0xFFFFFFFFu, w_rows > 0) & ((2u << lane) - 1)) * a.groups;
+      } else {
+        w_end = passes_of(w_rows) * a.groups;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const int v = __shfl_up_sync(0xFFFFFFFFu, w_end, off);
+          if (lane >= off) w_end += v;
+        }
+      }
+      w_end += before;
+    };
+    auto lane_ptr = [](const unsigned char* p, int from) {
+      return reinterpret_cast<const unsigned char*>(__shfl_sync(0xFFFFFFFFu, reinterpret_cast<unsigned long long>(p), from));
+    };
+    request(lane);
+    window(0);
+    struct Item { int e, group, slot, nt; const unsigned char *w0, *w1; };
+    auto find = [&](unsigned item) {
+      Item f;
+      if (item < static_cast<unsigned>(a.s_items)) {
+        const int pass = static_cast<int>(item) / a.groups;
+        f.e = a.n_expert;
+        f.group = static_cast<int>(item) - pass * a.groups;
+        f.slot = pass * a.s_step;
+        f.nt = min(a.s_step, a.s_rows - f.slot);
+        f.w0 = a.sw0;
+        f.w1 = a.sw1;
+        return f;
+      }
+      const int i = static_cast<int>(item) - a.s_items;
+      for (int before; i >= (before = __shfl_sync(0xFFFFFFFFu, w_end, 31)) && e0 < a.n_expert;) {
+        e0 += 32;
+        window(before);
+      }
+      f.e = f.group = f.slot = f.nt = 0;             // no rows: the list is at its end
+      f.w0 = f.w1 = nullptr;
+      if (e0 >= a.n_expert) return f;
+      const int at = __popc(__ballot_sync(0xFFFFFFFFu, w_end <= i)), rows = __shfl_sync(0xFFFFFFFFu, w_rows, at);
+      const int passes = passes_of(rows), r = i - (__shfl_sync(0xFFFFFFFFu, w_end, at) - passes * a.groups);
+      f.slot = __shfl_sync(0xFFFFFFFFu, w_slot, at);
+      f.group = r;
+      f.nt = rows;
+      if (passes > 1) {
+        const int step = ((rows + passes - 1) / passes + 7) & ~7;
+        f.group = r / passes;
+        const int t0 = (r - f.group * passes) * step;
+        f.slot += t0;
+        f.nt = min(step, rows - t0);
+      }
+      f.e = e0 + at;
+      f.w0 = lane_ptr(w_0, at);
+      f.w1 = DUAL ? lane_ptr(w_1, at) : f.w0;
+      return f;
+    };
+    const int look = (a.nb - 1) / 2;                 // the column under which the next item is looked up
+    for (Item it = find(blockIdx.x), after; it.nt > 0; it = after) {
       unsigned later = 0;
       if (lane == 0) later = atomicAdd(a.next, 1u);
-      const bool shared = item < static_cast<unsigned>(a.s_items);
-      const int i = static_cast<int>(shared ? item : item - a.s_items), e = i / a.groups, group = i - e * a.groups;
-      int slot = e * a.s_step, m = min(a.s_step, a.s_rows - slot);
-      const unsigned char *w0 = a.sw0, *w1 = a.sw1;
-      if (!shared) {
-        slot = __ldg(a.off + e);
-        m = __ldg(a.off + e + 1) - slot;
-        w0 = a.tab0[e];
-        w1 = DUAL ? a.tab1[e] : w0;
-      }
+      const int e = it.e, group = it.group, slot = it.slot, nt = it.nt;
+      const unsigned char *w0 = it.w0, *w1 = it.w1;
+      const bool shared = e == a.n_expert;
       const uintptr_t align = (reinterpret_cast<uintptr_t>(w0) | reinterpret_cast<uintptr_t>(w1)) & 15u;
       const bool absent = w0 == nullptr || w1 == nullptr;
-      const unsigned char* map0 = a.maps + (static_cast<size_t>(shared ? a.n_expert : e) * 3 + a.map0) * 128;
+      const unsigned char* map0 = a.maps + (static_cast<size_t>(e) * 3 + a.map0) * 128;
       const int row0 = group * (DUAL ? 128 : 256);
-      if (m > 0 && !absent && align == 0 && lane == 0) {
+      if (!absent && align == 0 && lane == 0) {
         tmap_acquire(map0);
         if (DUAL) tmap_acquire(map0 + 128);
       }
-      const int passes = (m + kTok - 1) / kTok, step = m > kTok ? ((m + passes - 1) / passes + 7) & ~7 : kTok;
+      publish(slot, nt, (shared ? 1 : 0) | (absent ? 2 : 0));
 #pragma unroll 1
-      for (; m > 0; m -= step, slot += step) {
-        const int nt = min(step, m);
-        publish(slot, nt, (shared ? 1 : 0) | (absent ? 2 : 0));
-#pragma unroll 1
-        for (int b = 0; b < a.nb; ++b) {
-          if (!wait(&wempty[s], ph ^ 1u)) return;
-          unsigned char* st = smem + kHdr + s * kStageBytes;
-          if (lane == 0) {
-            Desc d;
-            d.flags = nt | (b == 0 ? 1 << 8 : 0) | (b + 1 == a.nb ? 1 << 9 : 0) | (absent ? 1 << 10 : 0) | (shared ? 1 << 11 : 0);
-            d.slot0 = slot; d.group = group; d.pad = 0;
-            desc[s] = d;
-          }
-          if (!absent && align == 0) {
-            if (lane == 0) {
-              mbar_expect_tx(&full[s], kWBytes);
-              tma_load_box<STREAM>(st, map0, b * kW4, row0, &full[s]);
-              tma_load_box<STREAM>(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
-            }
-          } else {
-            if (!absent) {                           // a base off a 16-byte boundary: plain copies
-              const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
-              const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
-#pragma unroll 1
-              for (int h = 0; h < 2; ++h)
-                warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
-                  const int r = p / 9;
-                  return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
-                });
-              asm volatile("cp.async.wait_all;" ::: "memory");
-              fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive_one(&full[s]);
-          }
-          advance();
+      for (int b = 0; b < a.nb; ++b) {
+        if (!wait(&wempty[s], ph ^ 1u)) return;
+        unsigned char* st = smem + kHdr + s * kStageBytes;
+        if (lane == 0) {
+          Desc d;
+          d.flags = nt | (b == 0 ? 1 << 8 : 0) | (b + 1 == a.nb ? 1 << 9 : 0) | (absent ? 1 << 10 : 0) | (shared ? 1 << 11 : 0);
+          d.slot0 = slot; d.group = group; d.pad = 0;
+          desc[s] = d;
         }
+        if (!absent && align == 0) {
+          if (lane == 0) {
+            mbar_expect_tx(&full[s], kWBytes);
+            tma_load_box<STREAM>(st, map0, b * kW4, row0, &full[s]);
+            tma_load_box<STREAM>(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
+          }
+        } else {
+          if (!absent) {                             // a base off a 16-byte boundary: plain copies
+            const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
+            const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h)
+              warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
+                const int r = p / 9;
+                return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
+              });
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            fence_proxy_async();                     // the next fill of this stage may come from the TMA unit
+          }
+          __syncwarp();
+          if (lane == 0) mbar_arrive_one(&full[s]);
+        }
+        if (b == look) after = find(__shfl_sync(0xFFFFFFFFu, later, 0) + gridDim.x);
+        advance();
       }
-      item = __shfl_sync(0xFFFFFFFFu, later, 0) + gridDim.x;
     }
     publish(0, 0, 0);
     if (!wait(&wempty[s], ph ^ 1u)) return;
@@ -387,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
 }
 
 template <bool DUAL, bool STREAM>
-int launch_rows(RowsArgs a, cudaStream_t stream) {
+int launch_rows(RowsArgs a, long long routes, cudaStream_t stream) {
   a.status = status_word();
   const int sms = device_sms();
   if (a.status == nullptr || sms <= 0) return kErrLaunch;
@@ -398,11 +468,11 @@ int launch_rows(RowsArgs a, cudaStream_t stream) {
     a.s_step = ((a.s_rows + passes - 1) / passes + 7) & ~7;
     a.s_items = a.groups * ((a.s_rows + a.s_step - 1) / a.s_step);
   }
-  const long long n_items = static_cast<long long>(a.groups) * a.n_expert + a.s_items;
-  if (n_items > 0x7FFFFFFF) return kErrUnsupported;
-  a.n_items = static_cast<int>(n_items);
+  // (the routed items' number is known on the device alone: passes of kTok rows are at most one more per expert than the rows make)
+  const long long n_items = static_cast<long long>(a.groups) * (a.n_expert + routes / kTok) + a.s_items;
+  if (n_items > 0x7FFFFFFF - 1024) return kErrUnsupported;
   if (!opt_in_smem<grouped_gemm_rows_kernel<DUAL, STREAM>>(kSmem)) return kErrLaunch;
-  return launch_pdl(grouped_gemm_rows_kernel<DUAL, STREAM>, dim3(std::min(a.n_items, sms)), kThreads, kSmem, stream, a);
+  return launch_pdl(grouped_gemm_rows_kernel<DUAL, STREAM>, dim3(static_cast<unsigned>(std::min<long long>(n_items, sms))), kThreads, kSmem, stream, a);
 }
 
 // Rows of fp16 values -> Q8_K rows in blocks of kRowBlk bytes, two slabs
@@ -468,11 +538,11 @@ int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, c
   RowsArgs a = args_of(g, maps, 0);
   a.tab1 = tab_up;
   a.sw1 = static_cast<const unsigned char*>(shared_up);
-  return g.stream ? launch_rows<true, true>(a, stream) : launch_rows<true, false>(a, stream);
+  return g.stream ? launch_rows<true, true>(a, g.routes, stream) : launch_rows<true, false>(a, g.routes, stream);
 }
 int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream) { 
   const RowsArgs a = args_of(g, maps, 2);
-  return g.stream ? launch_rows<false, true>(a, stream) : launch_rows<false, false>(a, stream);
+  return g.stream ? launch_rows<false, true>(a, g.routes, stream) : launch_rows<false, false>(a, g.routes, stream);
 }
 
 int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_rows, const uint16_t* x1, void* out1, long long rows1,

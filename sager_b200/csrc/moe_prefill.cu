@@ -151,6 +151,7 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   down.tab = tab(2); down.off = a->off; down.xq = op.h; down.operand_rows = up.operand_rows;
   up.maps = down.maps = op.maps;
   up.stream = down.stream = streams_weights(H, F, E);
+  up.routes = down.routes = static_cast<long long>(n) * K;
   down.y = a->y_grouped; down.n_rows = H; down.k = F; down.n_expert = E;
   if (shared) {
     up.shared_w = a->shared_gate; up.shared_xq = op.x; up.shared_y = a->sh_g; up.shared_rows = n;

@@ -116,3 +116,48 @@ def test_saturated_codes():
     got = L.g[:n].double().cpu().numpy()[np.argsort(L.grows[:n].cpu().numpy())]
     # g to fp16 (2^-11), h = silu(g) g: its relative error is at most (2 + |g|) times that of g, and rounded itself
     assert (np.abs(got - h[:, None]) <= (np.abs(h) * (3 + np.abs(g)) * 2.0 ** -11 + 1e-6)[:, None]).all()
+
+
+@pytest.mark.parametrize("E,hot", [(70, {66: 301}), (70, {0: 130, 31: 97, 32: 65, 69: 33}), (300, {5: 1, 299: 260}), (33, {32: 400})])
+def test_hot_experts(E, hot):
+    """Passes of one expert are handed out one by one: hot experts at the edges of the 32-expert windows in which an item is
+    looked up, windows without a row in between."""
+    H, F = 512, 256
+    counts = [hot.get(e, 0) for e in range(E)]
+    n = sum(counts)
+    w = synth.MoeWeights(H, F, E, DEV, seed=87, std=0.05, distinct=7)
+    x16 = synth.normal_fp16((n, H), 88, DEV)
+    L = PrefillLayer(4 * n, H, F, E, 1, DEV)
+    t = w.table()
+    L.run(n, x16, x16.clone(), w, t, logits=chosen_logits(counts, n, 9))
+    assert np.array_equal(np.diff(L.off.cpu().numpy()), counts)
+    y = launchers([t[m].contiguous() for m in range(3)], L.off, L.grows, x16, n, H, F, E)
+    assert torch.equal(L.yg[:n].view(torch.int16), y.view(torch.int16))
+    assert lib().raw("sgr_status")(0) == 0
+
+
+def test_a_hot_expert_is_shared_out():
+    """The same routes with one expert in all of them: as many dots and fewer weights than spread evenly, and so no slower as
+    long as every SM gets its share (one CTA for an expert's passes took three times as long)."""
+    H, F, E, K, n = 2048, 512, 256, 2, 1024
+    w = synth.MoeWeights(H, F, E, DEV, seed=89, std=0.05, distinct=7)
+    x16 = synth.normal_fp16((n, H), 90, DEV)
+    L = PrefillLayer(2 * n, H, F, E, K, DEV)
+    t = w.table()
+    spread = torch.randn(n, E, generator=torch.Generator(device=DEV).manual_seed(1), device=DEV)
+    hot = spread.clone()
+    hot[:, 100:102] += 20.0
+    us = []
+    for logits in (spread, hot):
+        x = torch.zeros_like(x16)
+        best = []
+        for rep in range(8):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            L.run(n, x16, x, w, t, logits=logits)
+            b.record()
+            b.synchronize()
+            best.append(a.elapsed_time(b) * 1e3)
+        us.append(min(best))
+    assert L.off.cpu().numpy()[102] == 2 * n and L.off.cpu().numpy()[100] == 0
+    assert us[1] < 1.2 * us[0], us
