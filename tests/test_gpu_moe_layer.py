@@ -673,24 +673,44 @@ def test_fused_exchange_entry_points_with_one_rank(full_w, tokens, own_plan):
     assert lib().raw("sgr_status")(0) == 0
 
 
+def picks_of(meet, n):
+    """Experts of each row, eight apiece, so that tiles of the wanted numbers of rows arise."""
+    if meet == "all":
+        return [list(range(8)) for _ in range(n)]
+    own = [list(range(8 + 8 * t, 16 + 8 * t)) for t in range(n)]          # experts no other row has
+    if meet == "none":
+        return own
+    if meet == "pair":
+        return [list(range(8)) if t < 2 else own[t] for t in range(n)]
+    # tiles of one to four rows beside one another
+    common = {0: range(4), 1: range(4), 2: (0, 1, 2), 3: (1, 2, 3), 4: (0, 1), 5: (2, 3), 6: (0, 2)}
+    return [([e for e, rows in common.items() if t in rows] + own[t])[:8] for t in range(n)]
+
+
 @pytest.mark.parametrize("n", [3, 4])
-@pytest.mark.parametrize("meet", ["all", "pair", "none", "absent"])
+@pytest.mark.parametrize("meet", ["all", "pair", "none", "mixed", "absent"])
 def test_token_layer_shares_by_cost(oracle, n, meet):
     """Layers of three and four rows whose CTAs take more pairs than a pass of both groups: tiles of one to four rows in one
     layer, every tile with all rows, no two rows in a tile, an absent expert among them. Every (tile, pair) has to be in exactly
-    one CTA's share: a pair left out or taken by a neighbour shows in h. Bias by row is not possible, so the rows' inputs choose."""
-    H, F, E, K = 2048, 256, 40, 8
+    one CTA's share: a pair left out or taken by a neighbour shows in h. The router's first columns hold the logits wanted, the
+    rows' first values name the column."""
+    H, F, E, K = 2048, 768, 40, 8
     w = synth.MoeWeights(H, F, E, DEV, seed=91, std=0.05)
     x16 = synth.normal_fp16((n, H), 92 + n, DEV)
-    if meet == "all":
-        x16[1:] = x16[0]
-    elif meet != "none":
-        x16[1] = x16[0]
+    x16[:, :n] = torch.eye(n, dtype=torch.float16, device=DEV)
+    picks = picks_of(meet, n)
+    w.router.zero_()
+    for t, chosen in enumerate(picks):
+        w.router[chosen, t] = 3.0 - 0.125 * torch.arange(K, dtype=torch.float32, device=DEV)
+    distinct = {e for chosen in picks for e in chosen}
+    # (the line of the kernel's rule: a pass of both groups is 2 x 16 pairs at hidden 2048)
+    assert len(distinct) * F > 2 * 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    if meet in ("mixed", "absent"):
+        assert {sum(e in chosen for chosen in picks) for e in distinct} == set(range(1, n + 1))
     x_np = x16.cpu().numpy()
-    want = oracle_layer(oracle, w, x_np, x_np.astype(np.float32), K)
-    absent = (int(want["idx"][0, 2]),) if meet == "absent" else ()
-    if absent:
-        want = oracle_layer(oracle, w, x_np, x_np.astype(np.float32), K, absent=absent)
+    absent = (0, 3) if meet == "absent" else ()
+    want = oracle_layer(oracle, w, x_np, x_np.astype(np.float32), K, absent=absent)
+    assert [sorted(r) for r in want["idx"][:, :K].tolist()] == [sorted(chosen) for chosen in picks]
     for rep in range(2):                         # (the second call finds the first one's h rows)
         runner, x_out, out32 = run_layer(w, n, K, x16, absent=absent)
         assert np.array_equal(runner.route_idx.cpu().numpy()[:n, :K], want["idx"][:, :K])
