@@ -46,10 +46,11 @@ def test_logits_odd_shapes(oracle):
 
 
 @pytest.mark.parametrize("rows,k,n_tok", [(256, 2048, 592), (250, 736, 611), (256, 2048, 591), (13, 96, 9), (1, 2048, 33),
-                                          (17, 32, 2)])
+                                          (17, 32, 2), (256, 516, 592), (250, 500, 611), (256, 516, 591), (255, 90, 593), (13, 100, 9),
+                                          (1, 2044, 33), (17, 33, 2)])
 def test_logits_tile_edges_bit_exact(oracle, rows, k, n_tok):
-    """Both tilings of the many-token kernel (the rule's line is rows x tokens = 256 x 592): ragged rows,
-    tokens and columns."""
+    """Ragged rows, tokens and columns; with k off a multiple of eight, both tilings of the kernel for rows off a 16-byte boundary
+    (the rule's line is rows x tokens = 256 x 592)."""
     w_np, w_dev = router_w(5, e=rows, h=k)
     x_np, x_dev = make_x16(n_tok, k, 6)
     y = torch.full((n_tok + 1, rows), 7.0, dtype=torch.float32, device=DEV)
