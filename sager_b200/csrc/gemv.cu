@@ -405,10 +405,9 @@ __device__ __forceinline__ void direct_blocks(const DirectArgs& a, const uint4 (
   }
 }
 
-// (Weights as the first to leave L2: 24 layers at 2 / 4 / 8 rows 15.2 / 15.8 / 17.3 us a layer as ordinary lines, 13.0 / 13.5 / 15.4;
-// 8 layers that L2 can hold 14.5 and 14.1.)
+// STREAM: weights first to leave L2 (launch_direct)
 // NI: block columns per warp (1 for rows of up to eight blocks); LONG: rows of more than 32 blocks, 32 at a time
-template <int NI, bool F16, bool LONG = false>
+template <int NI, bool F16, bool STREAM, bool LONG = false>
 __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const DirectArgs a) {
   __shared__ float red[kDirectWarps][8][16];                // [warp][token][row]
   const int nb = a.nb, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -427,9 +426,9 @@ __global__ void __launch_bounds__(kDirectWarps * 32) gemv_direct_kernel(const Di
                                 (static_cast<size_t>(row - a.first_row(m)) * nb + blk0 + c0) * kW4;
 #pragma unroll
       for (int i = 0; i < NI; ++i) {
-        hdr[h][i] = load_weights<true>(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
+        hdr[h][i] = load_weights<STREAM>(reinterpret_cast<const uint4*>(wb + i * 8 * kW4));
 #pragma unroll
-        for (int g = 0; g < 4; ++g) q[h][i][g] = load_weights<true>(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
+        for (int g = 0; g < 4; ++g) q[h][i][g] = load_weights<STREAM>(reinterpret_cast<const uint2*>(wb + i * 8 * kW4 + 16 + 32 * g + 8 * tig));
       }
     }
   };
@@ -564,24 +563,34 @@ inline bool direct_fits(const DirectArgs& a) {
 template <bool F16>
 int launch_direct(const DirectArgs& a, cudaStream_t stream) {
   const int threads = kDirectWarps * 32;
-  if (a.n_tokens == 1) {
-    const int rows_cta = kDirectWarps * std::max(1, 8 / a.nb);
+  // Launches of four megabytes of weights and more are taken for those of a model that L2 does not hold between two steps: as the
+  // first to leave, its weights no longer push out the kernels' code and activations. What decides is whether the weights are
+  // still in L2 at their next use, which a launch cannot know; both sides, in us per step from a graph, ordinary lines / first to leave:
+  //   projections of 4096 + 2 x 512 from 2048 and 2048 from 4096 with nothing in between, one row: 4 / 6 / 8 / 10 / 24 / 40 layers
+  //   39.5 / 55.8 / 77 / 107 / 259 / 424 and 40.0 / 60.5 / 82 / 101 / 240 / 407 - six or eight such layers, which just fit, lose -,
+  //   four rows: 4 / 8 / 24 layers 56 / 119 / 375 and 54 / 110 / 332;
+  //   with a layer's experts in between, as a model has them (256 experts, 2048 / 512), one row: 2 / 4 / 8 / 12 layers
+  //   49 / 108 / 215 / 319 and 49 / 100 / 198 / 302.
+  // Below, where a model of many layers may stay in L2 (2048 + 2 x 256 from 1024, 24 layers, 4 rows: 222 as ordinary lines, 233 as
+  // the first to leave), the lines keep their place: 214.
+  const bool first = static_cast<long long>(a.rows_cum[2]) * a.nb * kW4 >= 4 << 20;
+  auto launch = [&](auto stream_weights) {
+    constexpr bool S = decltype(stream_weights)::value;
+    if (a.n_tokens == 1) {
+      const int rows_cta = kDirectWarps * std::max(1, 8 / a.nb);
+      const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
+      if (a.nb <= 8) return launch_pdl(gemv_direct1_kernel<1, F16, S>, grid, threads, 0, stream, a);
+      if (a.nb == 16) return launch_pdl(gemv_direct1_kernel<2, F16, S>, grid, threads, 0, stream, a);
+      return launch_pdl(gemv_direct1_kernel<4, F16, S>, grid, threads, 0, stream, a);
+    }
+    const int rows_cta = 16 * std::max(1, kDirectWarps / a.nb);
     const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
-    // Matrices of four megabytes and more are taken for those of a model that L2 does not hold between two tokens: as the first to
-    // leave, its weights no longer push out the kernels' code and activations. 40 / 24 layers of 4096 + 2 x 512 from 2048 and 2048
-    // from 4096: 11.0 / 10.5 us a layer, 10.3 / 9.7; where L2 could hold all of it (8 layers) 9.9 against 10.7, and
-    // smaller matrices (2048 + 2 x 256 from 1024, 12 layers) 6.9 against 7.2.
-    const bool first = static_cast<long long>(a.rows_cum[2]) * a.nb * kW4 >= 4 << 20;
-    if (a.nb <= 8) return launch_pdl(first ? gemv_direct1_kernel<1, F16, true> : gemv_direct1_kernel<1, F16, false>, grid, threads, 0, stream, a);
-    if (a.nb == 16) return launch_pdl(first ? gemv_direct1_kernel<2, F16, true> : gemv_direct1_kernel<2, F16, false>, grid, threads, 0, stream, a);
-    return launch_pdl(first ? gemv_direct1_kernel<4, F16, true> : gemv_direct1_kernel<4, F16, false>, grid, threads, 0, stream, a);
-  }
-  const int rows_cta = 16 * std::max(1, kDirectWarps / a.nb);
-  const dim3 grid((a.rows_cum[2] + rows_cta - 1) / rows_cta);
-  if (a.nb <= 8) return launch_pdl(gemv_direct_kernel<1, F16>, grid, threads, 0, stream, a);
-  if (a.nb == 16) return launch_pdl(gemv_direct_kernel<2, F16>, grid, threads, 0, stream, a);
-  if (a.nb == 32) return launch_pdl(gemv_direct_kernel<4, F16>, grid, threads, 0, stream, a);
-  return launch_pdl(gemv_direct_kernel<4, F16, true>, grid, threads, 0, stream, a);
+    if (a.nb <= 8) return launch_pdl(gemv_direct_kernel<1, F16, S>, grid, threads, 0, stream, a);
+    if (a.nb == 16) return launch_pdl(gemv_direct_kernel<2, F16, S>, grid, threads, 0, stream, a);
+    if (a.nb == 32) return launch_pdl(gemv_direct_kernel<4, F16, S>, grid, threads, 0, stream, a);
+    return launch_pdl(gemv_direct_kernel<4, F16, S, true>, grid, threads, 0, stream, a);
+  };
+  return first ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 // Where the tile kernel's CTAs, which copy their rows by one bulk copy each, are faster than the direct ones (us, direct / tile):

@@ -109,19 +109,24 @@ __device__ __forceinline__ void bulk_g2s_weights(void* dst, const void* src, uin
       ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(evict_first_policy())
       : "memory");
 }
-// the same for weights that go straight into registers
+// the same for weights that go straight into registers; if not STREAM, lines keep the place in L2's order that they have
+template <bool STREAM>
+__device__ __forceinline__ uint64_t weights_policy() {
+  if constexpr (STREAM) return evict_first_policy();
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_unchanged.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
 template <bool STREAM>
 __device__ __forceinline__ uint4 load_weights(const uint4* p) {
-  if constexpr (!STREAM) return __ldg(p);
   uint4 v;
-  asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(evict_first_policy()));
+  asm("ld.global.nc.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "l"(weights_policy<STREAM>()));
   return v;
 }
 template <bool STREAM>
 __device__ __forceinline__ uint2 load_weights(const uint2* p) {
-  if constexpr (!STREAM) return __ldg(p);
   uint2 v;
-  asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(evict_first_policy()));
+  asm("ld.global.nc.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(v.x), "=r"(v.y) : "l"(p), "l"(weights_policy<STREAM>()));
   return v;
 }
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
