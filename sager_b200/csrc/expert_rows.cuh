@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
           __syncwarp();                            // every lane's part of the stage (and of its descriptor) is written
           if (lane == 0) mbar_arrive(&full[s]);
         }
-        __syncwarp();                              // (the copies' operands pass through uniform registers: no lane runs ahead)
+        __syncwarp();
         ++q;
         if (lane == 0) *issued = static_cast<unsigned>(q);
         if (++s == kStageCount) { s = 0; ph ^= 1u; }

@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
           __syncwarp();
           if (lane == 0) mbar_arrive_one(&full[s]);
         }
+        __syncwarp();
         if (b == look) after = find(__shfl_sync(0xFFFFFFFFu, later, 0) + gridDim.x);
         advance();
       }

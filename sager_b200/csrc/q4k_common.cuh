@@ -92,9 +92,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       : "memory");
 }
 // L2 policy of weights that are read once: first to leave, so that they do not push out what the kernels after this one need -
-// their code, router rows, activations (streams_weights, api_util.cuh, has the line and the figures). A constant where it is used:
-// a policy chosen at run time and kept in a register across the weight warp's loop left copies that did not complete - waits ran
-// out -, most likely because the copies' operands pass through uniform registers and the warp's other lanes ran ahead.
+// their code, router rows, activations (streams_weights, api_util.cuh, has the line and the figures). A copy that carries a policy
+// is a kernel of its own, and the policy is made by createpolicy right at the copy: PTX leaves any other 64-bit operand undefined.
+// (A form with the choice at run time, one operand for both kinds of layers, left copies that did not complete - waits ran out -;
+// its cause was not established, and it is not to be run again.)
 __device__ __forceinline__ uint64_t evict_first_policy() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));

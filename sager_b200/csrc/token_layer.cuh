@@ -594,6 +594,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
           mbar_arrive_one(&full[s]);
         }
       }
+      __syncwarp();
       pos += np;
       pair0 += np;
       if (pair0 == FF) { pair0 = 0; ++tile; }
