@@ -68,7 +68,11 @@ inline bool streams_weights(int hidden, int n_ff, int n_expert) {
 constexpr int kOpBlk = 560;
 
 // TMA descriptors of a layer's experts, which quantize_operand or quantize_rows makes: [n_expert + 1][3] of 128 bytes (gate, up,
-// down; the shared expert's last), then 16 bytes of counters.
+// down; the shared expert's last), then the addresses they were made from, [3][n_expert + 1], then 16 bytes of counters.
+constexpr int kExpertMapBytes = 3 * (128 + 8);
+inline const unsigned char* const* map_addresses(const void* maps, int n_expert, int m) {
+  return reinterpret_cast<const unsigned char* const*>(static_cast<const unsigned char*>(maps) + (n_expert + 1LL) * 384) + m * (n_expert + 1LL);
+}
 struct ExpertMaps {
   const unsigned char* const* tab;     // [3][stride]
   long long stride;

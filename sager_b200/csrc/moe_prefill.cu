@@ -112,7 +112,7 @@ OperandRows operand_rows(const sgr_moe_prefill* a) {
     unsigned char* base = slab + front;
     return OperandRows{front + x + h + s <= room ? form : Rows::kPacked, base, base + x, base + x + h, slab + (-at & 127u)};
   };
-  const long long maps = (-at & 127u) + (a->n_expert + 1LL) * 384 + 16;      // in front: the descriptors
+  const long long maps = (-at & 127u) + (((a->n_expert + 1LL) * kExpertMapBytes + 15) & ~15LL) + 16;      // in front: the descriptors
   const uintptr_t outs = reinterpret_cast<uintptr_t>(a->g) | reinterpret_cast<uintptr_t>(a->y_grouped) |
                          reinterpret_cast<uintptr_t>(a->sh_g) | reinterpret_cast<uintptr_t>(a->sh_y);
   if ((at & 15u) == 0 && (outs & 3u) == 0 && static_cast<long long>(a->n) * a->n_used <= static_cast<long long>(kFewRows) * a->n_expert) {
@@ -143,7 +143,10 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   const int n = a->n, H = a->hidden, F = a->n_ff, E = a->n_expert, K = a->n_used;
   const bool shared = has_shared(a);
   const long long ts = a->tab_stride > 0 ? a->tab_stride : E, R = static_cast<long long>(a->n_max) * K;
-  auto tab = [&](int m) { return reinterpret_cast<const unsigned char* const*>(a->w_tab + m * ts); };
+  // (with descriptors: the addresses that these were made from, not what the table says by now)
+  auto tab = [&](int m) {
+    return op.maps != nullptr ? map_addresses(op.maps, E, m) : reinterpret_cast<const unsigned char* const*>(a->w_tab + m * ts);
+  };
   ExpertGemm up{};
   up.tab = tab(0); up.off = a->off; up.rows = a->grows; up.xq = op.x; up.operand_rows = op.form == Rows::kOperands;
   up.y = a->g; up.n_rows = F; up.k = H; up.n_expert = E;

@@ -1,5 +1,5 @@
-// tmap_dev.cuh - TMA descriptors that are patched on the device, shared by the row-streaming expert kernels
-// (expert_rows.cuh, grouped_gemm_rows.cu): expert addresses live in a pointer table on the device, so a descriptor is
+// tmap_dev.cuh - TMA descriptors that are patched on the device, shared by the row-streaming expert kernels and the tcgen05 GEMM
+// (expert_rows.cuh, grouped_gemm_rows.cu, grouped_gemm_i8.cu): expert addresses live in a pointer table on the device, so a descriptor is
 // encoded on the host for a placeholder address and gets its base there.
 #pragma once
 
@@ -34,8 +34,9 @@ __device__ __forceinline__ void tma_load_box(void* dst, const void* gmem_map, in
                  ::"r"(smem_u32(dst)), "l"(gmem_map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
 
-// The descriptors of a layer's experts (ExpertMaps, api_util.cuh), made by CTAs of a launch before the GEMMs; and the counters
-// that lie behind them, cleared.
+// The descriptors of a layer's experts (ExpertMaps, api_util.cuh), made by CTAs of a launch before the GEMMs, with the addresses
+// that they were made from: the GEMMs take absence, alignment and plain copies' sources from those, since the table may be
+// rewritten in between, and an entry that was null when the descriptors were made has none. And the counters, cleared.
 struct MapArgs {
   unsigned* counters;
   const unsigned char* const* tab;     // [3][stride]
@@ -46,7 +47,7 @@ struct MapArgs {
   alignas(16) uint32_t up[32], down[32];
 };
 inline unsigned* map_counters(const void* maps, int n_expert) {
-  return reinterpret_cast<unsigned*>(static_cast<unsigned char*>(const_cast<void*>(maps)) + (n_expert + 1LL) * 384);
+  return reinterpret_cast<unsigned*>(static_cast<unsigned char*>(const_cast<void*>(maps)) + (n_expert + 1LL) * kExpertMapBytes);
 }
 // false: the driver has no encoder
 inline bool map_args(const ExpertMaps& em, bool make, MapArgs* m) {
@@ -71,7 +72,10 @@ __device__ __forceinline__ void make_maps(const MapArgs& m, int e, unsigned char
     if (lane == i && w[i] != nullptr && (reinterpret_cast<uintptr_t>(w[i]) & 15u) == 0) tmap_replace_addr(patch + 128 * i, w[i]);
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 3; ++i) tmap_publish(m.maps + (static_cast<size_t>(e) * 3 + i) * 128, patch + 128 * i);
+  for (int i = 0; i < 3; ++i) {
+    tmap_publish(m.maps + (static_cast<size_t>(e) * 3 + i) * 128, patch + 128 * i);
+    if (lane == i) reinterpret_cast<const unsigned char**>(m.maps + (m.n_expert + 1LL) * 384)[i * (m.n_expert + 1LL) + e] = w[i];
+  }
 }
 
 }  // namespace sgr

@@ -161,3 +161,56 @@ def test_a_hot_expert_is_shared_out():
         us.append(min(best))
     assert L.off.cpu().numpy()[102] == 2 * n and L.off.cpu().numpy()[100] == 0
     assert us[1] < 1.2 * us[0], us
+
+
+@pytest.mark.parametrize("n", [70, 200])
+def test_the_table_is_read_once(n):
+    """The expert cache may rewrite the table at any time: what counts for a chunk is the table as it was when the descriptors
+    were made, for absent and present experts and for their alignment alike. A graph of the call with a copy of another
+    table between its first kernel (which makes them) and the rest; row-streaming and tcgen05 form."""
+    from cuda.bindings import runtime as rt
+    H, F, E, K = 512, 256, 12, 4
+    w, other = (synth.MoeWeights(H, F, E, DEV, seed=s, std=0.05) for s in (95, 96))
+    before = w.table((2, 9)).clone()
+    odd = torch.empty(other.blob.numel() + 16, dtype=torch.uint8, device=DEV)
+    shifted = other.table() - other.blob.data_ptr() + odd.data_ptr() + 2
+    after = other.table((4, 9)).clone()
+    after[:, 6:8] = shifted[:, 6:8]
+    x16 = synth.normal_fp16((n, H), 97, DEV)
+    L = PrefillLayer(n, H, F, E, K, DEV)
+    x = x16.clone()
+    L.run(n, x16, x, w, before)
+    want = x.clone()
+    want_y = L.yg.clone()
+
+    def ok(r):
+        assert r[0] == rt.cudaError_t.cudaSuccess, r[0]
+        return r[1] if len(r) > 1 else None
+
+    table = before.clone()
+    a = L.args(n, x16, x, w, table)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ok(rt.cudaStreamBeginCapture(s.cuda_stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeRelaxed))
+    lib().call("sgr_moe_layer_prefill", C.byref(a), C.c_void_p(s.cuda_stream))
+    graph = ok(rt.cudaStreamEndCapture(s.cuda_stream))
+    count = rt.cudaGraphGetNodes(graph, 0)[2]
+    nodes = rt.cudaGraphGetNodes(graph, count)[1][:count]
+    firsts = rt.cudaGraphGetRootNodes(graph, 1)[1]
+    rest = [v for v in nodes if int(v) != int(firsts[0])]
+    copy = ok(rt.cudaGraphAddMemcpyNode1D(graph, firsts, 1, table.data_ptr(), after.data_ptr(), table.numel() * 8,
+                                          rt.cudaMemcpyKind.cudaMemcpyDeviceToDevice))
+    for v in rest:
+        ok(rt.cudaGraphAddDependencies(graph, [copy], [v], 1))
+    run = ok(rt.cudaGraphInstantiate(graph, 0))
+    x.copy_(x16)
+    L.yg.zero_()
+    torch.cuda.synchronize()
+    ok(rt.cudaGraphLaunch(run, s.cuda_stream))
+    torch.cuda.synchronize()
+    assert torch.equal(table, after)
+    assert torch.equal(L.yg.view(torch.int16), want_y.view(torch.int16))
+    assert torch.equal(x.view(torch.int16), want.view(torch.int16))
+    assert lib().raw("sgr_status")(0) == 0
+    ok(rt.cudaGraphExecDestroy(run))
+    ok(rt.cudaGraphDestroy(graph))
