@@ -358,7 +358,8 @@ typedef struct sgr_moe_prefill {
   void* hq;                 /* [R][n_ff/256] Q8_K blocks, 16-byte aligned */
   uint16_t* y_grouped;      /* [R][hidden] */
   uint16_t* expert_y;       /* [n_max][n_used+1][hidden] combine slab, 16-byte aligned: scratch for the GEMMs' operand
-                               rows; the combine itself uses it only when x_f16, y_grouped or sh_y is not 16-byte aligned */
+                               rows and, where they fit as well, the experts' TMA descriptors (408 bytes an expert); the
+                               combine itself uses it only when x_f16, y_grouped or sh_y is not 16-byte aligned */
   uint16_t* sh_g;           /* [n_max][n_ff] */
   uint16_t* sh_u;           /* [n_max][n_ff] */
   void* sh_q;               /* [n_max][n_ff/256] Q8_K blocks */

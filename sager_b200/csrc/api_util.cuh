@@ -68,7 +68,7 @@ inline bool streams_weights(int hidden, int n_ff, int n_expert) {
 constexpr int kOpBlk = 560;
 
 // TMA descriptors of a layer's experts, which quantize_operand or quantize_rows makes: [n_expert + 1][3] of 128 bytes (gate, up,
-// down; the shared expert's last), then the addresses they were made from, [3][n_expert + 1], then 16 bytes of counters.
+// down; the shared expert's last), then the addresses they were made from, [3][n_expert + 1].
 constexpr int kExpertMapBytes = 3 * (128 + 8);
 inline const unsigned char* const* map_addresses(const void* maps, int n_expert, int m) {
   return reinterpret_cast<const unsigned char* const*>(static_cast<const unsigned char*>(maps) + (n_expert + 1LL) * 384) + m * (n_expert + 1LL);
@@ -76,7 +76,8 @@ inline const unsigned char* const* map_addresses(const void* maps, int n_expert,
 struct ExpertMaps {
   const unsigned char* const* tab;     // [3][stride]
   long long stride;
-  void* maps;                          // 128-byte aligned
+  void* maps;                          // 128-byte aligned; null: no room for them
+  unsigned* counters;                  // [4], cleared with every launch of quantize_rows
   const void* shared[3];
   int n_expert, hidden, n_ff;
 };
@@ -91,7 +92,8 @@ struct ExpertGemm {
   int n_rows, k, n_expert;
   bool operand_rows;
   bool stream;                  // the weights' L2 policy (streams_weights)
-  const void* maps;             // with operand rows: the descriptors; n_rows is then a multiple of 128
+  const void* maps;             // the descriptors (null: none); for operand rows n_rows is a multiple of 128
+  unsigned* counters;           // gemm_rows_*: ExpertMaps'
   long long routes;             // routed rows at most (gemm_rows_*)
   const void* shared_w;
   const unsigned char* shared_xq;
@@ -105,8 +107,8 @@ int gemm_grouped(const ExpertGemm& g, cudaStream_t stream);
 constexpr int kRowBlk = 288;
 // n_rows and k multiples of 256, outputs 4-byte aligned.
 // gate, up and SwiGLU: y receives h
-int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, const void* maps, cudaStream_t stream);
-int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream);
+int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, cudaStream_t stream);
+int gemm_rows_down(const ExpertGemm& g, cudaStream_t stream);
 // rows of k fp16 values -> such rows; two slabs, the first of at most *d_rows rows when that is given.
 // Clears the counters of the two GEMM launches; with make_maps the descriptors are made as well.
 int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_rows, const uint16_t* x1, void* out1, long long rows1,

@@ -112,7 +112,7 @@ struct GemmArgs {
   uint16_t *sy, *sy1;
   int s_rows, s_step, s_items;         // its rows, rows per unit, units
   int n_items;
-  const unsigned char* maps;           // (operand rows) [n_expert + 1][3] descriptors; the matrix of tab0 is map0
+  const unsigned char* maps;           // (operand rows) [n_expert + 1][3] descriptors, or null; the matrix of tab0 is map0
   int map0;
   int* status;
 };
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
         if (u.w0 == nullptr) continue;
         const uintptr_t align = (reinterpret_cast<uintptr_t>(u.w0) | reinterpret_cast<uintptr_t>(u.w1)) & 15u;
         const unsigned char* map = a.maps + (static_cast<size_t>(u.expert) * 3 + a.map0) * 128;
-        if (align == 0 && lane == 0) {
+        if (a.maps != nullptr && align == 0 && lane == 0) {
           tmap_acquire(map);
           if (DUAL) tmap_acquire(map + 128);
         }
@@ -467,13 +467,17 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
           if (++st == kStages) { st = 0; st_ph ^= 1u; }
           unsigned char* stage = smem + kOffW + s * kStageBytes;
           const int row0 = (u.tile0 + t) * kGemmRows;
+          const unsigned char* src = (m == 0 ? u.w0 : u.w1) + static_cast<size_t>(row0) * row_bytes + b * kW4;
           if (align == 0) {
-            if (lane == 0) {
+            if (a.maps == nullptr) {
+              cp_load_box(stage, src, kGemmRows, row_bytes, &bar[kBarWFull + s], lane);
+              __syncwarp();
+              if (lane == 0) mbar_arrive_one(&bar[kBarWFull + s]);
+            } else if (lane == 0) {
               mbar_expect_tx(&bar[kBarWFull + s], kStageBytes);
               tma_load_box<STREAM>(stage, map + 128 * m, b * kW4, row0, &bar[kBarWFull + s]);
             }
           } else {                                               // a base off a 16-byte boundary
-            const unsigned char* src = (m == 0 ? u.w0 : u.w1) + static_cast<size_t>(row0) * row_bytes + b * kW4;
             warp_copy_unaligned(stage, kStageBytes / 16, lane, src, [&](int p) { return p / 9 * row_bytes + p % 9 * 16; });
             asm volatile("cp.async.wait_all;" ::: "memory");
             fence_proxy_async();                                 // the next fill of the stage may be a TMA copy
@@ -795,7 +799,7 @@ int quantize_operand(const uint16_t* x0, const uint16_t* u0, void* out0, long lo
   const long long ctas = ((rows0 + rows1) * nb + kQuantWarps - 1) / kQuantWarps;
   MapArgs m{};
   if (!map_args(em, make_maps, &m)) return kErrUnsupported;
-  const unsigned map_ctas = make_maps ? static_cast<unsigned>(em.n_expert / kQuantWarps + 1) : 0;
+  const unsigned map_ctas = make_maps && em.maps != nullptr ? static_cast<unsigned>(em.n_expert / kQuantWarps + 1) : 0;
   if (ctas + map_ctas > 0x7FFFFFFF) return kErrUnsupported;
   if (ctas + map_ctas == 0) return kOk;
   return launch_pdl(quantize_operand_kernel, dim3(static_cast<unsigned>(ctas + map_ctas)), kQuantWarps * 32, 0, stream, x0, u0,

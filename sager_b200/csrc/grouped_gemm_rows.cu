@@ -43,7 +43,7 @@ static_assert(kSmem <= 227 * 1024, "shared memory");
 struct RowsArgs {
   const unsigned char* const* tab0;    // [E] gate (or the only matrix)
   const unsigned char* const* tab1;    // [E] up
-  const unsigned char* maps;           // [E + 1][3] descriptors; the matrix of tab0 is map0
+  const unsigned char* maps;           // [E + 1][3] descriptors (null: none); the matrix of tab0 is map0
   int map0;
   const int* off;                      // [E + 1] grouped slots of each expert
   const int* rows;                     // source row of a grouped slot; null: the slot itself
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
       const bool absent = w0 == nullptr || w1 == nullptr;
       const unsigned char* map0 = a.maps + (static_cast<size_t>(e) * 3 + a.map0) * 128;
       const int row0 = group * (DUAL ? 128 : 256);
-      if (!absent && align == 0 && lane == 0) {
+      if (a.maps != nullptr && !absent && align == 0 && lane == 0) {
         tmap_acquire(map0);
         if (DUAL) tmap_acquire(map0 + 128);
       }
@@ -299,25 +299,31 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
           d.slot0 = slot; d.group = group; d.pad = 0;
           desc[s] = d;
         }
-        if (!absent && align == 0) {
-          if (lane == 0) {
+        // the 128 rows of either half (where they are addressed one by one)
+        const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
+        const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
+        if (absent) {
+          if (lane == 0) mbar_arrive_one(&full[s]);
+        } else if (align == 0) {
+          if (a.maps == nullptr) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) cp_load_box(st + h * kHalfBytes, h ? b1 : b0, 128, row_bytes, &full[s], lane);
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(&full[s]);
+          } else if (lane == 0) {
             mbar_expect_tx(&full[s], kWBytes);
             tma_load_box<STREAM>(st, map0, b * kW4, row0, &full[s]);
             tma_load_box<STREAM>(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
           }
-        } else {
-          if (!absent) {                             // a base off a 16-byte boundary: plain copies
-            const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
-            const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
+        } else {                                     // a base off a 16-byte boundary: plain copies
 #pragma unroll 1
-            for (int h = 0; h < 2; ++h)
-              warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
-                const int r = p / 9;
-                return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
-              });
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            fence_proxy_async();                     // the next fill of this stage may come from the TMA unit
-          }
+          for (int h = 0; h < 2; ++h)
+            warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
+              const int r = p / 9;
+              return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
+            });
+          asm volatile("cp.async.wait_all;" ::: "memory");
+          fence_proxy_async();                       // the next fill of this stage may come from the TMA unit
           __syncwarp();
           if (lane == 0) mbar_arrive_one(&full[s]);
         }
@@ -522,10 +528,10 @@ quantize_rows_kernel(const uint16_t* __restrict__ x0, unsigned char* __restrict_
   }
 }
 
-RowsArgs args_of(const ExpertGemm& g, const void* maps, int map0) {
+RowsArgs args_of(const ExpertGemm& g, int map0) {
   RowsArgs a{};
-  a.maps = static_cast<const unsigned char*>(maps);
-  a.next = map_counters(maps, g.n_expert) + map0;
+  a.maps = static_cast<const unsigned char*>(g.maps);
+  a.next = g.counters + map0;
   a.tab0 = g.tab; a.map0 = map0; a.off = g.off; a.rows = g.rows; a.xq = g.xq; a.y = g.y;
   a.n_rows = g.n_rows; a.nb = g.k / kQK; a.n_expert = g.n_expert;
   a.sw0 = a.sw1 = static_cast<const unsigned char*>(g.shared_w);
@@ -535,14 +541,14 @@ RowsArgs args_of(const ExpertGemm& g, const void* maps, int map0) {
 
 }  // namespace
 
-int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, const void* maps, cudaStream_t stream) {
-  RowsArgs a = args_of(g, maps, 0);
+int gemm_rows_gate_up(const ExpertGemm& g, const unsigned char* const* tab_up, const void* shared_up, cudaStream_t stream) {
+  RowsArgs a = args_of(g, 0);
   a.tab1 = tab_up;
   a.sw1 = static_cast<const unsigned char*>(shared_up);
   return g.stream ? launch_rows<true, true>(a, g.routes, stream) : launch_rows<true, false>(a, g.routes, stream);
 }
-int gemm_rows_down(const ExpertGemm& g, const void* maps, cudaStream_t stream) { 
-  const RowsArgs a = args_of(g, maps, 2);
+int gemm_rows_down(const ExpertGemm& g, cudaStream_t stream) {
+  const RowsArgs a = args_of(g, 2);
   return g.stream ? launch_rows<false, true>(a, g.routes, stream) : launch_rows<false, false>(a, g.routes, stream);
 }
 
@@ -552,7 +558,7 @@ int quantize_rows(const uint16_t* x0, void* out0, long long rows0, const int* d_
   const long long ctas = ((rows0 + rows1) * nb + kQuantWarps - 1) / kQuantWarps;
   MapArgs m{};
   if (!map_args(em, make_maps, &m)) return kErrUnsupported;
-  const unsigned map_ctas = make_maps ? static_cast<unsigned>(em.n_expert / kQuantWarps + 1) : 0;
+  const unsigned map_ctas = make_maps && em.maps != nullptr ? static_cast<unsigned>(em.n_expert / kQuantWarps + 1) : 0;
   if (ctas + map_ctas > 0x7FFFFFFF) return kErrUnsupported;
   if (ctas + map_ctas == 0) return kOk;
   return launch_pdl(quantize_rows_kernel, dim3(static_cast<unsigned>(ctas + map_ctas)), kQuantWarps * 32, 0, stream, x0,

@@ -94,36 +94,43 @@ __global__ void combine_grouped_kernel(uint16_t* __restrict__ x, const uint16_t*
 
 inline bool has_shared(const sgr_moe_prefill* a) { return a->shared_gate && a->shared_up && a->shared_down; }
 
-// The rows the GEMMs read lie in the combine slab's memory, behind the experts' descriptors, when they fit there: Q8_K rows in
-// padded blocks for the kernel of few token rows per expert, ready operands for the tcgen05 one (FFN up to about 0.8 x hidden
-// at top-8); otherwise Q8_K rows from which the tcgen05 GEMMs make their operands themselves.
+// The rows the GEMMs read lie in the combine slab's memory when they fit there: Q8_K rows in padded blocks for the kernel of few
+// token rows per expert, ready operands for the tcgen05 one (FFN up to about 0.8 x hidden at top-8); otherwise Q8_K rows from
+// which the tcgen05 GEMMs make their operands themselves. In front of them lie the hand-out counters and, where the slab holds
+// those too (some 400 bytes per expert: buffers of a few rows for many experts have no room), the experts' descriptors.
 enum class Rows { kPadded, kOperands, kPacked };
 struct OperandRows {
   Rows form;
   unsigned char *x, *h, *s;       // layer input, routed h, shared expert's h
-  unsigned char* maps;
+  unsigned char* maps;            // null: none
+  unsigned* counters;
 };
 OperandRows operand_rows(const sgr_moe_prefill* a) {
   const long long nbh = a->hidden / kQK, nbf = a->n_ff / kQK, room = static_cast<long long>(a->n_max) * (a->n_used + 1) * a->hidden * 2;
   unsigned char* slab = reinterpret_cast<unsigned char*>(a->expert_y);
   const uintptr_t at = reinterpret_cast<uintptr_t>(slab);
-  auto laid = [&](Rows form, long long blk, long long front) {
+  const long long pad = -at & 127u, map_bytes = (a->n_expert + 1LL) * kExpertMapBytes;
+  OperandRows r{};
+  auto fits = [&](Rows form, long long blk) {
     const long long x = a->n * nbh * blk, h = static_cast<long long>(a->n) * a->n_used * nbf * blk, s = a->n * nbf * blk;
-    unsigned char* base = slab + front;
-    return OperandRows{front + x + h + s <= room ? form : Rows::kPacked, base, base + x, base + x + h, slab + (-at & 127u)};
+    for (const bool with_maps : {true, false}) {
+      const long long maps_end = with_maps ? pad + ((map_bytes + 15) & ~15LL) : 0;
+      const long long front = maps_end + (with_maps || form == Rows::kPadded ? 16 : 0);
+      if (front + x + h + s > room) continue;
+      unsigned char* base = slab + front;
+      r = {form, base, base + x, base + x + h, with_maps ? slab + pad : nullptr, reinterpret_cast<unsigned*>(slab + maps_end)};
+      return true;
+    }
+    return false;
   };
-  const long long maps = (-at & 127u) + (((a->n_expert + 1LL) * kExpertMapBytes + 15) & ~15LL) + 16;      // in front: the descriptors
   const uintptr_t outs = reinterpret_cast<uintptr_t>(a->g) | reinterpret_cast<uintptr_t>(a->y_grouped) |
                          reinterpret_cast<uintptr_t>(a->sh_g) | reinterpret_cast<uintptr_t>(a->sh_y);
-  if ((at & 15u) == 0 && (outs & 3u) == 0 && static_cast<long long>(a->n) * a->n_used <= static_cast<long long>(kFewRows) * a->n_expert) {
-    const OperandRows r = laid(Rows::kPadded, kRowBlk, maps);
-    if (r.form == Rows::kPadded) return r;
-  }
   if ((at & 15u) == 0) {
-    const OperandRows r = laid(Rows::kOperands, kOpBlk, maps);
-    if (r.form == Rows::kOperands) return r;
+    if ((outs & 3u) == 0 && static_cast<long long>(a->n) * a->n_used <= static_cast<long long>(kFewRows) * a->n_expert && fits(Rows::kPadded, kRowBlk))
+      return r;
+    if (fits(Rows::kOperands, kOpBlk)) return r;
   }
-  return {Rows::kPacked, static_cast<unsigned char*>(a->xq), static_cast<unsigned char*>(a->hq), static_cast<unsigned char*>(a->sh_q), nullptr};
+  return {Rows::kPacked, static_cast<unsigned char*>(a->xq), static_cast<unsigned char*>(a->hq), static_cast<unsigned char*>(a->sh_q), nullptr, nullptr};
 }
 
 // the combine reads the grouped rows in place when every buffer allows 16-byte accesses
@@ -134,7 +141,7 @@ bool combines_in_place(const sgr_moe_prefill* a) {
 }
 
 ExpertMaps expert_maps(const sgr_moe_prefill* a, const OperandRows& op) {
-  return {reinterpret_cast<const unsigned char* const*>(a->w_tab), a->tab_stride > 0 ? a->tab_stride : a->n_expert, op.maps,
+  return {reinterpret_cast<const unsigned char* const*>(a->w_tab), a->tab_stride > 0 ? a->tab_stride : a->n_expert, op.maps, op.counters,
           {a->shared_gate, a->shared_up, a->shared_down}, a->n_expert, a->hidden, a->n_ff};
 }
 
@@ -153,6 +160,7 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   ExpertGemm down{};
   down.tab = tab(2); down.off = a->off; down.xq = op.h; down.operand_rows = up.operand_rows;
   up.maps = down.maps = op.maps;
+  up.counters = down.counters = op.counters;
   up.stream = down.stream = streams_weights(H, F, E);
   up.routes = down.routes = static_cast<long long>(n) * K;
   down.y = a->y_grouped; down.n_rows = H; down.k = F; down.n_expert = E;
@@ -162,10 +170,10 @@ int expert_stage(const sgr_moe_prefill* a, const OperandRows& op, cudaStream_t s
   }
   int rc;
   if (op.form == Rows::kPadded) {              // SwiGLU happens in the GEMM
-    rc = gemm_rows_gate_up(up, tab(1), a->shared_up, op.maps, stream);
+    rc = gemm_rows_gate_up(up, tab(1), a->shared_up, stream);
     if (rc == kOk)
       rc = quantize_rows(a->g, op.h, static_cast<long long>(n) * K, a->meta, a->sh_g, op.s, shared ? n : 0, F, expert_maps(a, op), false, stream);
-    return rc == kOk ? gemm_rows_down(down, op.maps, stream) : rc;
+    return rc == kOk ? gemm_rows_down(down, stream) : rc;
   }
   rc = gemm_gate_up(up, tab(1), a->u, a->shared_up, a->sh_u, stream);
   if (rc != kOk) return rc;

@@ -214,3 +214,28 @@ def test_the_table_is_read_once(n):
     assert lib().raw("sgr_status")(0) == 0
     ok(rt.cudaGraphExecDestroy(run))
     ok(rt.cudaGraphDestroy(graph))
+
+
+# combine slabs with room for the operand rows but not for descriptors: few rows for many experts (row-streaming form), and the
+# tcgen05 form's operands at exactly the slab's size (7 x 512 bytes a row and route against 64 blocks of 560)
+@pytest.mark.parametrize("H,F,E,K,n", [(512, 256, 256, 8, 16), (512, 256, 256, 8, 5), (1024, 512, 256, 8, 9), (3584, 2560, 4, 4, 40)])
+@pytest.mark.parametrize("shift", [0, 2, 8])
+def test_no_room_for_descriptors(H, F, E, K, n, shift):
+    w = synth.MoeWeights(H, F, E, DEV, seed=91, std=0.05, distinct=5)
+    big = torch.empty(w.blob.numel() + 16, dtype=torch.uint8, device=DEV)
+    big[shift:shift + w.blob.numel()] = w.blob.reshape(-1)
+    w.blob = big[shift:shift + w.blob.numel()].view(w.n_slots, -1)
+    x16 = synth.normal_fp16((n, H), 92, DEV)
+    L = PrefillLayer(n, H, F, E, K, DEV)
+    L.xq.fill_(0xA5)
+    absent = (1,)
+    t = w.table(absent)
+    x = x16.clone()
+    L.run(n, x16, x, w, t)
+    assert (L.xq == 0xA5).all()                  # (the form that reads plain Q8_K rows would have written them there)
+    y = launchers([t[m].contiguous() for m in range(3)], L.off, L.grows, x16, n * K, H, F, E)
+    assert torch.equal(L.yg[:n * K].view(torch.int16), y.view(torch.int16))
+    one = [ops.ptr_table([w.matrix(E, m)], DEV) for m in range(3)]
+    sy = launchers(one, dev(np.int32([0, n])), dev(np.arange(n, dtype=np.int32)), x16, n, H, F, 1)
+    assert torch.equal(L.sh_y[:n].view(torch.int16), sy.view(torch.int16))
+    assert lib().raw("sgr_status")(0) == 0
