@@ -25,10 +25,14 @@ using namespace sgr;
 
 namespace {
 // Up to this many routed rows per expert on average the row-streaming GEMM takes the expert stage: its work grows with the rows,
-// the tcgen05 form's with the weights. Two layers of 2048 / 512 / 256 experts, us, against the tcgen05 form: 16 rows per expert
-// 382 / 502, 24 497 / 546, 28 558 / 575, 31 608 / 587; of 1024 / 512 / 128: 24 183 / 193, 26 192 / 198, 30 212 / 206; of 2048 / 256 /
-// 64: 20 132 / 150, 24 148 / 144, 29 153 / 151.
-constexpr int kFewRows = 26;
+// the tcgen05 form's with the weights. Two layers (hidden / FFN / experts / top-k), us, against the tcgen05 form, evenly spread rows:
+//   2048 / 512 / 256 / 8: 12 rows per expert 298 / 433, 20 376 / 469, 25 424 / 481, 28 462 / 485, 31 511 / 496
+//   1024 / 512 / 128 / 8: 12 132 / 163, 20 152 / 173, 25 168 / 176, 28 178 / 180, 31 189 / 184
+//   2048 / 256 / 64 / 8:  12 101 / 111, 20 109 / 122, 25 122 / 123, 26 143 / 123 (passes past 32 rows begin a second wave of items)
+//   1024 / 512 / 16 / 4:  12 69 / 72, 20 74 / 80, 25 76 / 77, 28 79 / 77;  512 / 256 / 128 / 8: 20 86 / 96, 25 93 / 97, 28 99 / 98
+// The mean is what the host knows; hot experts move the line up, since both forms then work in passes, these of 32 rows and
+// those of 80 (a fifth of the experts in 70 % of the routes: 25 rows 464 / 690, 183 / 281, 140 / 159; 31 rows 533 / 764, 198 / 324, 145 / 174).
+constexpr int kFewRows = 25;
 // x[row] += sum_k w[row][k] * y_grouped[gslot[row][k]] (k = 0 .. K-1, in this order; a route that was
 // not computed, gslot < 0, adds nothing) + w[row][K] * sh_y[row] (when there is a shared expert):
 // scatter_routed_f16 + the strided copy + moe_combine_batched_f16 of the reference's sequence
