@@ -28,7 +28,8 @@ long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff, int n_
 int sgr_residency_test_set_inflight(void* handle, int slot, int on);
 
 /* The expert stage (gate, up, SwiGLU, requantise, down) of a finished sgr_moe_layer_prefill call once more, on
- * the plan and the operand rows that call left in its buffers. For timing. SGR_EUNSUPPORTED where the combine
+ * the plan and the operand rows that call left in its buffers, with the weights that args names now (their descriptors are
+ * made anew: one short launch). For timing. SGR_EUNSUPPORTED where the combine
  * has used the slab that held those rows (x_f16, y_grouped or sh_y off a 16-byte boundary). */
 struct sgr_moe_prefill;
 int sgr_moe_prefill_expert_stage(const struct sgr_moe_prefill* args, void* stream);

@@ -199,6 +199,12 @@ SGR_API int sgr_moe_prefill_expert_stage(const sgr_moe_prefill* a, void* stream)
   if (a == nullptr) return kErrArg;
   const OperandRows op = operand_rows(a);
   if (op.form != Rows::kPacked && !combines_in_place(a)) return kErrUnsupported;      // the combine's slab lies where the operand rows were
+  if (op.maps != nullptr) {                    // the weights are those of the table given here
+    const int rc = op.form == Rows::kPadded
+        ? quantize_rows(nullptr, nullptr, 0, nullptr, nullptr, nullptr, 0, a->hidden, expert_maps(a, op), true, as_stream(stream))
+        : quantize_operand(nullptr, nullptr, nullptr, 0, nullptr, nullptr, nullptr, nullptr, 0, a->hidden, expert_maps(a, op), true, as_stream(stream));
+    if (rc != kOk) return rc;
+  }
   return expert_stage(a, op, as_stream(stream));
 }
 

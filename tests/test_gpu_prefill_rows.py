@@ -239,3 +239,18 @@ def test_no_room_for_descriptors(H, F, E, K, n, shift):
     sy = launchers(one, dev(np.int32([0, n])), dev(np.arange(n, dtype=np.int32)), x16, n, H, F, 1)
     assert torch.equal(L.sh_y[:n].view(torch.int16), sy.view(torch.int16))
     assert lib().raw("sgr_status")(0) == 0
+
+
+@pytest.mark.parametrize("n", [70, 200])
+def test_expert_stage_reads_the_table_it_is_given(n):
+    """The stage once more with another layer's weights on the same buffers: row-streaming and tcgen05 form."""
+    H, F, E, K = 512, 256, 12, 4
+    w, other = (synth.MoeWeights(H, F, E, DEV, seed=s, std=0.05) for s in (97, 98))
+    x16 = synth.normal_fp16((n, H), 99, DEV)
+    L = PrefillLayer(n, H, F, E, K, DEV)
+    for absent in ((), (5,)):
+        L.run(n, x16, x16.clone(), w, w.table())
+        t = other.table(absent)
+        L.run(n, x16, x16.clone(), other, t, experts_only=True)
+        y = launchers([t[m].contiguous() for m in range(3)], L.off, L.grows, x16, n * K, H, F, E)
+        assert torch.equal(L.yg[:n * K].view(torch.int16), y.view(torch.int16))
