@@ -389,12 +389,12 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
 // both, and a lane scales the results of one token - half the multiply-adds, conversions and fp32 steps, which for eight
 // columns are spent on tokens that are not there (prefill of 96 rows over 256 experts, four layers: 512 -> 504 us; in the decode
 // layer's row-streaming kernel the tiles gain as much, but the larger kernel costs every layer 0.8 to 1.2 us more). Results: rows gid and gid + 8, token tig.
-//   b_ptr   this lane's ldmatrix row (b_row4), advanced by 64 bytes per pair of sub-blocks, + mid_pad after two
+//   b_ptr   this lane's ldmatrix row (b_row4), advanced by 64 bytes per pair of sub-blocks
 //   min_b   sub-block sums 4 (tig & 1) .. + 3 of token gid / 2: their low parts in even gid, high parts (bsum = 128 hi + lo) in odd
 //   fold(row, isum, msum): the fp32 steps; isum is sixteen-fold
 template <typename Loaded, typename MinB, typename Fold>
 __device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, const uint4& h0, const uint4& h1, const unsigned char* b_ptr,
-                                                int mid_pad, int lane, Loaded loaded, MinB min_b, Fold fold) {
+                                                int lane, Loaded loaded, MinB min_b, Fold fold) {
   const int tig = lane & 3;
   uint32_t raw[4][4];
 #pragma unroll
@@ -406,7 +406,7 @@ __device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, cons
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     uint32_t b[4], lo[4], hi[4];
-    ldmatrix_x4(b, b_ptr + g * 64 + (g >> 1) * mid_pad);
+    ldmatrix_x4(b, b_ptr + g * 64);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       lo[j] = raw[g][j] & 0x0F0F0F0Fu;
@@ -430,7 +430,7 @@ __device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, cons
   for (int r = 0; r < 2; ++r) fold(r, 16 * is[r] + hs[r], m[2 * r] + 128 * m[2 * r + 1]);
 }
 // This lane's ldmatrix row for warp_mma_block4: lanes 0-7 / 8-15 name the columns' first / second sixteen codes of an even
-// sub-block, 16-31 those of the odd one after it; `codes` is token 0's row, `zeros` 256 + mid_pad bytes of zeros.
+// sub-block, 16-31 those of the odd one after it; `codes` is token 0's row, `zeros` 256 bytes of zeros.
 __device__ __forceinline__ const unsigned char* b_row4(const unsigned char* codes, int tok_stride, const unsigned char* zeros, int lane) {
   return ((lane & 1) == (lane >> 4) ? codes + ((lane & 7) >> 1) * tok_stride : zeros) + (lane >> 3) * 16;
 }
