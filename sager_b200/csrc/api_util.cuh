@@ -53,10 +53,17 @@ int launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cuda
 }
 
 // Whether a layer's weights are read under the policy that makes them the first to leave L2. As ordinary lines they push out what
-// every layer needs again: 2048 / 512 / 256 experts at 64 / 8 / 4 / 1 rows 88.9 / 48.7 / 33.4 / 15.7 us a layer, 81.5 / 44.1 / 32.8 /
-// 15.4 as the first to leave; prefill of 96 / 777 / 2048 rows, two layers, 257 / 556 / 864 -> 248 / 546 / 853. What a model keeps in
-// L2 between two uses of a layer is not known here: a layer of more than an eighth of it (126 MB) is taken for one of
-// many. Small layers (512 / 256 / 16 experts, 4 MB, twelve of them) lose by it: 11.5 -> 11.8 us at one row.
+// every layer needs again. What a model keeps in L2 between two uses of a layer is not known here: a layer of more than an eighth
+// of it (126 MB) is taken for one of many. us per step, ordinary lines / first to leave:
+//   453 MB a layer (2048 / 512 / 256 experts), one layer: 64 / 8 / 4 / 1 rows 88.9 / 48.7 / 33.4 / 15.7, 81.5 / 44.1 / 32.8 / 15.4
+//   113 MB (1024 / 512 / 128), 12 layers: 64 / 8 / 4 / 1 rows 669 / 420 / 275 / 162, 595 / 404 / 268 / 159
+//   57 MB (2048 / 256 / 64), 12 layers: 588 / 444 / 264 / 160, 579 / 434 / 256 / 155
+//   28 MB (1024 / 256 / 64), 12 layers: 459 / 363 / 233 / 151, 452 / 357 / 228 / 151; four, which L2 holds: 157 / 114 / 79 / 54, 154 / 118 / 79 / 54
+//   14 MB (1024 / 256 / 32), 24 layers: 799 / 650 / 382 / 284, 788 / 635 / 375 / 284; four 133 / 108 / 64.5 / 51.8, 135 / 109 / 65.5 / 52.2
+//   4 MB (512 / 256 / 16), 12 layers: 338 / 283 / 183 / 140, 345 / 287 / 185 / 142
+// Below the line few layers lose as much as many would gain. In a prefill chunk the shared expert's weights are read once per 32
+// or 80 of its rows, and a hot expert's once per pass, under the same policy: 96 / 777 / 2048 rows of the first geometry, four / two /
+// two layers, 499 / 501 / 857 without the policy, 485 / 491 / 850 with it, 490 / 485 / 854 with the shared expert's copies left out of it.
 inline bool streams_weights(int hidden, int n_ff, int n_expert) {
   return static_cast<long long>(hidden) * n_ff / 256 * 144 * 3 * n_expert > (16LL << 20);
 }

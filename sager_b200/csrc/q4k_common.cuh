@@ -91,7 +91,7 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
       ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
 }
-// L2 policy of weights that are read once: first to leave, so that they do not push out what the kernels after this one need -
+// L2 policy of weights that are read once or in a few passes close together: first to leave, so that they do not push out what the kernels after this one need -
 // their code, router rows, activations (streams_weights, api_util.cuh, has the line and the figures). A copy that carries a policy
 // is a kernel of its own, and the policy is made by createpolicy right at the copy: PTX leaves any other 64-bit operand undefined.
 // (A form with the choice at run time, one operand for both kinds of layers, left copies that did not complete - waits ran out -;
