@@ -142,6 +142,30 @@ __device__ __forceinline__ void rows_block(const unsigned char* a_ptr, const uns
   }
 }
 
+// Weight warp: a stage's two halves of 128 blocks where the TMA unit cannot bring them - no descriptors, or a base off a 16-byte
+// boundary - and the barrier's arrival. (Not inlined: beside the TMA copies its code costs registers and a chunk of 300 to 500 rows
+// a hundredth.)
+static __device__ __noinline__ void copy_blocks(unsigned char* st, const unsigned char* b0, const unsigned char* b1, int row_bytes, bool aligned,
+                                                uint64_t* bar, int lane) {
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    if (aligned) {
+      cp_load_box(st + h * kHalfBytes, h ? b1 : b0, 128, row_bytes, bar, lane);
+    } else {
+      warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
+        const int r = p / 9;
+        return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
+      });
+    }
+  }
+  if (!aligned) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    fence_proxy_async();                             // the next fill of this stage may come from the TMA unit
+  }
+  __syncwarp();
+  if (lane == 0) mbar_arrive_one(bar);
+}
+
 // STREAM: weights first to leave L2 (streams_weights)
 template <bool DUAL, bool STREAM>
 __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const RowsArgs a) {
@@ -203,13 +227,11 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
     const unsigned char *n_0 = nullptr, *n_1 = nullptr;
     auto passes_of = [](int rows) { return (rows + kTok - 1) / kTok; };
     auto request = [&](int e) {
-      n_slot = n_to = 0;
-      if (e < a.n_expert) {
-        n_slot = __ldg(a.off + e);
-        n_to = __ldg(a.off + e + 1);
-        n_0 = a.tab0[e];
-        n_1 = DUAL ? a.tab1[e] : n_0;
-      }
+      const int c = min(e, a.n_expert - 1);
+      n_slot = __ldg(a.off + c);
+      n_to = __ldg(a.off + c + (e < a.n_expert ? 1 : 0));      // (past the end: no rows)
+      n_0 = a.tab0[c];
+      n_1 = DUAL ? a.tab1[c] : n_0;
     };
     auto window = [&](int before) {                  // the window at e0 becomes the present one
       const int to = n_to;
@@ -299,33 +321,18 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
           d.slot0 = slot; d.group = group; d.pad = 0;
           desc[s] = d;
         }
-        // the 128 rows of either half (where they are addressed one by one)
-        const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
-        const unsigned char* b1 = DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes;
         if (absent) {
           if (lane == 0) mbar_arrive_one(&full[s]);
-        } else if (align == 0) {
-          if (a.maps == nullptr) {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) cp_load_box(st + h * kHalfBytes, h ? b1 : b0, 128, row_bytes, &full[s], lane);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_one(&full[s]);
-          } else if (lane == 0) {
+        } else if (align == 0 && a.maps != nullptr) {
+          if (lane == 0) {
             mbar_expect_tx(&full[s], kWBytes);
             tma_load_box<STREAM>(st, map0, b * kW4, row0, &full[s]);
             tma_load_box<STREAM>(st + kHalfBytes, DUAL ? map0 + 128 : map0, b * kW4, DUAL ? row0 : row0 + 128, &full[s]);
           }
-        } else {                                     // a base off a 16-byte boundary: plain copies
-#pragma unroll 1
-          for (int h = 0; h < 2; ++h)
-            warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
-              const int r = p / 9;
-              return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
-            });
-          asm volatile("cp.async.wait_all;" ::: "memory");
-          fence_proxy_async();                       // the next fill of this stage may come from the TMA unit
-          __syncwarp();
-          if (lane == 0) mbar_arrive_one(&full[s]);
+        } else {
+          const unsigned char* b0 = w0 + static_cast<size_t>(row0) * row_bytes + b * kW4;
+          copy_blocks(st, b0, DUAL ? w1 + static_cast<size_t>(row0) * row_bytes + b * kW4 : b0 + static_cast<size_t>(128) * row_bytes,
+                      row_bytes, align == 0, &full[s], lane);
         }
         __syncwarp();
         if (b == look) after = find(__shfl_sync(0xFFFFFFFFu, later, 0) + gridDim.x);
