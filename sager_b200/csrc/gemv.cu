@@ -563,17 +563,20 @@ inline bool direct_fits(const DirectArgs& a) {
 template <bool F16>
 int launch_direct(const DirectArgs& a, cudaStream_t stream) {
   const int threads = kDirectWarps * 32;
-  // Launches of four megabytes of weights and more are taken for those of a model that L2 does not hold between two steps: as the
-  // first to leave, its weights no longer push out the kernels' code and activations. What decides is whether the weights are
-  // still in L2 at their next use, which a launch cannot know; both sides, in us per step from a graph, ordinary lines / first to leave:
+  // Launches of four megabytes of weights and more - two for several rows - are taken for those of a model that L2 does not hold
+  // between two steps: as the first to leave, its weights no longer push out the kernels' code and activations. What decides is
+  // whether the weights are still in L2 at their next use, which a launch cannot know; both sides, in us per step from a
+  // graph, ordinary lines / first to leave:
   //   projections of 4096 + 2 x 512 from 2048 and 2048 from 4096 with nothing in between, one row: 4 / 6 / 8 / 10 / 24 / 40 layers
   //   39.5 / 55.8 / 77 / 107 / 259 / 424 and 40.0 / 60.5 / 82 / 101 / 240 / 407 - six or eight such layers, which just fit, lose -,
   //   four rows: 4 / 8 / 24 layers 56 / 119 / 375 and 54 / 110 / 332;
   //   with a layer's experts in between, as a model has them (256 experts, 2048 / 512), one row: 2 / 4 / 8 / 12 layers
   //   49 / 108 / 215 / 319 and 49 / 100 / 198 / 302.
-  // Below, where a model of many layers may stay in L2 (2048 + 2 x 256 from 1024, 24 layers, 4 rows: 222 as ordinary lines, 233 as
-  // the first to leave), the lines keep their place: 214.
-  const bool first = static_cast<long long>(a.rows_cum[2]) * a.nb * kW4 >= 4 << 20;
+  // Below the line, where a model of many layers may stay in L2, the lines keep their place. 2048 + 2 x 512 from 2048 and 2048 from
+  // 2048 (2.4 MB the largest), 8 / 12 / 16 / 24 layers: one row ordinary 63 / 96 / 138 / 224, first 71 / 105 / 130 / 203; four rows ordinary
+  // 89 / 135 / 202 / 319, first 86 / 128 / 171 / 258, keeping their place 85 / 128 / 191 / 297. 2048 + 2 x 256 from 1024 and 1024 from
+  // 2048 (1.2 MB), 24 layers, four rows: 219, 224, 211.
+  const bool first = static_cast<long long>(a.rows_cum[2]) * a.nb * kW4 >= (a.n_tokens == 1 ? 4 : 2) << 20;
   auto launch = [&](auto stream_weights) {
     constexpr bool S = decltype(stream_weights)::value;
     if (a.n_tokens == 1) {

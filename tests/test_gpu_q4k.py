@@ -325,11 +325,12 @@ def test_line_between_direct_and_tile_kernel(oracle, rows, k, tok):
 
 
 @pytest.mark.parametrize("rows,k", [(1, 256), (37, 256), (67, 512), (129, 1024), (1187, 2048), (2371, 2048), (4737, 2048), (33, 4096),
-                                    (2373, 4096), (19, 8192), (3640, 2048), (3641, 2048), (910, 8192), (911, 8192)])
+                                    (2373, 4096), (19, 8192), (1820, 2048), (1821, 2048), (3640, 2048), (3641, 2048),
+                                    (455, 8192), (456, 8192), (910, 8192), (911, 8192)])
 @pytest.mark.parametrize("tok", [1, 2, 3, 4, 5, 8])
 def test_direct_kernel_edges(oracle, rows, k, tok):
     """Every variant of the small-matrix kernel (lanes per row, rows per warp, groups per lane, token slots; L2 policy from
-    4 MB of weights) at ragged row counts."""
+    4 MB of weights, from 2 MB at several rows) at ragged row counts."""
     w_np, w_dev = make_q4k(rows, k, 5)
     x_np, x_dev = make_x16(tok, k, 6)
     xq = torch.zeros(tok, k // 256 * 276, dtype=torch.uint8, device=DEV)
