@@ -624,12 +624,11 @@ __global__ void __launch_bounds__(kThreads, 1) expert_rows_kernel(const LayerDev
               b0 = ge->w[2] + static_cast<size_t>(row0) * rb_f + blk * kW4;
               b1 = b0 + static_cast<size_t>(kHalfRows) * rb_f;
             }
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h)
-              warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
-                const int r = p / 9;
-                return static_cast<size_t>(r) * rb + (p - r * 9) * 16;
-              });
+            const uintptr_t a0 = reinterpret_cast<uintptr_t>(b0), a1 = reinterpret_cast<uintptr_t>(b1);
+            warp_copy_unaligned(st, 2 * kHalfBytes / 16, lane, a0 | a1, ((a0 ^ a1) & 2u) != 0, [&](int p) {
+              const int r = p / 9, h = r / kHalfRows;
+              return (h ? b1 : b0) + static_cast<size_t>(r - h * kHalfRows) * rb + (p - r * 9) * 16;
+            });
             asm volatile("cp.async.wait_all;" ::: "memory");
             fence_proxy_async();                   // the next fill of this stage may come from the TMA unit
           }

@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
               tma_load_box<STREAM>(stage, map + 128 * m, b * kW4, row0, &bar[kBarWFull + s]);
             }
           } else {                                               // a base off a 16-byte boundary
-            warp_copy_unaligned(stage, kStageBytes / 16, lane, src, [&](int p) { return p / 9 * row_bytes + p % 9 * 16; });
+            warp_copy_unaligned(stage, kStageBytes / 16, lane, reinterpret_cast<uintptr_t>(src), false, [&](int p) { return src + p / 9 * row_bytes + p % 9 * 16; });
             asm volatile("cp.async.wait_all;" ::: "memory");
             fence_proxy_async();                                 // the next fill of the stage may be a TMA copy
             __syncwarp();
@@ -522,12 +522,12 @@ __global__ void __launch_bounds__(Cfg<RAW>::kThreads, 1) grouped_gemm_kernel(con
             cp_async_arrive(&bar[kBarWFull + s]);
           } else {                                               // ragged last tile, or a base off a 16-byte boundary
             const int last = a.n_rows - 1 - row0;                // rows past the matrix (never stored): zero, or its last one
-            auto piece = [&](int p) { return min(p / 9, last) * row_bytes + p % 9 * 16; };
+            auto piece = [&](int p) { return src + min(p / 9, last) * row_bytes + p % 9 * 16; };
             if (align == 0) {
 #pragma unroll 4
-              for (int q = lane; q < kStageBytes / 16; q += 32) cp_async16_or_zero(smem_u32(stage) + q * 16, src + piece(q), q / 9 <= last);
+              for (int q = lane; q < kStageBytes / 16; q += 32) cp_async16_or_zero(smem_u32(stage) + q * 16, piece(q), q / 9 <= last);
               cp_async_arrive(&bar[kBarWFull + s]);
-            } else if (warp_copy_unaligned(stage, kStageBytes / 16, lane, src, piece)) {
+            } else if (warp_copy_unaligned(stage, kStageBytes / 16, lane, align, false, piece)) {
               mbar_arrive_one(&bar[kBarWFull + s]);
             } else {
               cp_async_arrive(&bar[kBarWFull + s]);

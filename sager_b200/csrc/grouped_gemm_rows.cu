@@ -143,22 +143,18 @@ __device__ __forceinline__ void rows_block(const unsigned char* a_ptr, const uns
 }
 
 // Weight warp: a stage's two halves of 128 blocks where the TMA unit cannot bring them - no descriptors, or a base off a 16-byte
-// boundary - and the barrier's arrival. (Not inlined: beside the TMA copies its code costs registers and a chunk of 300 to 500 rows
-// a hundredth.)
-static __device__ __noinline__ void copy_blocks(unsigned char* st, const unsigned char* b0, const unsigned char* b1, int row_bytes, bool aligned,
+// boundary - and the barrier's arrival.
+__device__ __forceinline__ void copy_blocks(unsigned char* st, const unsigned char* b0, const unsigned char* b1, int row_bytes, bool aligned,
                                                 uint64_t* bar, int lane) {
+  if (aligned) {
 #pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
-    if (aligned) {
-      cp_load_box(st + h * kHalfBytes, h ? b1 : b0, 128, row_bytes, bar, lane);
-    } else {
-      warp_copy_unaligned(st + h * kHalfBytes, kHalfBytes / 16, lane, h ? b1 : b0, [&](int p) {
-        const int r = p / 9;
-        return static_cast<size_t>(r) * row_bytes + (p - r * 9) * 16;
-      });
-    }
-  }
-  if (!aligned) {
+    for (int h = 0; h < 2; ++h) cp_load_box(st + h * kHalfBytes, h ? b1 : b0, 128, row_bytes, bar, lane);
+  } else {
+    const uintptr_t a0 = reinterpret_cast<uintptr_t>(b0), a1 = reinterpret_cast<uintptr_t>(b1);
+    warp_copy_unaligned(st, kWBytes / 16, lane, a0 | a1, ((a0 ^ a1) & 2u) != 0, [&](int p) {
+      const int r = p / 9, h = r >> 7;
+      return (h ? b1 : b0) + static_cast<size_t>(r & 127) * row_bytes + (p - r * 9) * 16;
+    });
     asm volatile("cp.async.wait_all;" ::: "memory");
     fence_proxy_async();                             // the next fill of this stage may come from the TMA unit
   }

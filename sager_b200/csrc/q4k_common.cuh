@@ -134,21 +134,20 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 // ---- weights off a 16-byte boundary (a pointer table only promises the block struct's two bytes) ----
-// One warp copies `pieces` pieces of 16 bytes, piece p from base + off(p) to dst + 16 p; off(p) is a multiple of 16, so that the
-// base's low bits are those of every piece: one matrix per call, since gate, up and down may each lie on another boundary. On a
-// 4- or 8-byte boundary the copies are asynchronous (cp.async) and the caller waits for them, or lets a
-// barrier count them, when the function returns false; else words in the middle of a piece and half words at its ends,
-// four pieces' loads in flight, and the stores are done (true). Bound by the loads in flight: a prefill chunk of 1000 rows
-// over 256 experts 8 / 2 bytes off takes 367 / 1230 us, with a piece's half words one piece at a time 2059 / 2060; a
-// three-row layer of the one-launch kernel 40 / 96 us, 178 / 178 before.
-template <typename Off>
-__device__ __forceinline__ bool warp_copy_unaligned(unsigned char* dst, int pieces, int lane, const unsigned char* base, Off off) {
-  const uintptr_t align = reinterpret_cast<uintptr_t>(base);
+// One warp copies `pieces` pieces of 16 bytes, piece p from src_of(p) to dst + 16 p; `align`: the OR of all sources' address bits;
+// `mixed`: some of them lie on a word and some two bytes off one (gate, up and down of an expert may each lie on another
+// boundary). With all of them on a 4- or 8-byte boundary the copies are asynchronous (cp.async) and the caller waits for them, or
+// lets a barrier count them, when the function returns false; else words in the middle of a piece and half words at its ends,
+// four pieces' loads in flight, and the stores are done (true); mixed ones go half word by half word. Bound by the loads in
+// flight: a prefill chunk of 1000 rows over 256 experts 8 / 2 bytes off takes 367 / 1230 us, with a piece's half words one
+// piece at a time 2059 / 2060; a three-row layer of the one-launch kernel 40 / 96 us, 178 / 178 before.
+template <typename Src>
+__device__ __forceinline__ bool warp_copy_unaligned(unsigned char* dst, int pieces, int lane, uintptr_t align, bool mixed, Src src_of) {
   if ((align & 3u) == 0) {
     const bool by8 = (align & 7u) == 0;
 #pragma unroll 4
     for (int p = lane; p < pieces; p += 32) {
-      const unsigned char* src = base + off(p);
+      const unsigned char* src = src_of(p);
       const uint32_t d = smem_u32(dst) + p * 16;
       if (by8) {
 #pragma unroll
@@ -162,13 +161,22 @@ __device__ __forceinline__ bool warp_copy_unaligned(unsigned char* dst, int piec
     }
     return false;
   }
+  if (mixed) {
+#pragma unroll 1
+    for (int p = lane; p < pieces; p += 32) {
+      const uint16_t* src = reinterpret_cast<const uint16_t*>(src_of(p));
+#pragma unroll
+      for (int i = 0; i < 8; ++i) reinterpret_cast<uint16_t*>(dst + p * 16)[i] = __ldg(src + i);
+    }
+    return true;
+  }
 #pragma unroll 1
   for (int p0 = lane; p0 < pieces; p0 += 128) {
     uint32_t w[4][3];
     uint16_t first[4], last[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const unsigned char* src = base + off(min(p0 + 32 * u, pieces - 1));
+      const unsigned char* src = src_of(min(p0 + 32 * u, pieces - 1));
       first[u] = __ldg(reinterpret_cast<const uint16_t*>(src));
 #pragma unroll
       for (int i = 0; i < 3; ++i) w[u][i] = __ldg(reinterpret_cast<const uint32_t*>(src + 2) + i);

@@ -37,8 +37,9 @@ __device__ __forceinline__ void tma_load_box(void* dst, const void* gmem_map, in
 // One warp: what tma_load_box copies, where there is no descriptor - `rows` (a multiple of 32) rows' blocks from src, the first
 // row's, 16-byte aligned - by cp.async. Each lane's copies add an arrival of their own to the barrier's phase, so the caller's
 // arrival counts as with the other form and comes after a __syncwarp. (By a bulk copy per block it is issue-bound:
-// 5 rows, 1024 / 512 / 256 experts, 122 us instead of 45; 30 rows, 3584 / 2560 / 4 198 instead of 74.)
-__device__ __forceinline__ void cp_load_box(unsigned char* dst, const unsigned char* src, int rows, int row_bytes, uint64_t* bar, int lane) {
+// 5 rows, 1024 / 512 / 256 experts, 122 us instead of 45; 30 rows, 3584 / 2560 / 4 198 instead of 75. Not inlined: its registers beside the
+// TMA copies made the copies of unaligned weights spill, 500 rows of 1024 / 512 / 64 two bytes off 277 -> 410 us.)
+static __device__ __noinline__ void cp_load_box(unsigned char* dst, const unsigned char* src, int rows, int row_bytes, uint64_t* bar, int lane) {
   int offs[9];                                   // 16-byte piece q * 32 + lane of 32 rows
 #pragma unroll
   for (int q = 0; q < 9; ++q) offs[q] = (q * 32 + lane) / 9 * row_bytes + (q * 32 + lane) % 9 * 16;

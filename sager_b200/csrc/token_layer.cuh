@@ -362,7 +362,7 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
 // Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned; plain_done() ends a row of them. (Not
 // inlined at its six rarely taken uses: straight-line code beside them is paid for in instruction fetch, 0.4 us a layer.)
 static __device__ __noinline__ void copy_plain(unsigned char* dst, const unsigned char* src, int bytes, int lane) {
-  warp_copy_unaligned(dst, bytes / 16, lane, src, [](int p) { return p * 16; });
+  warp_copy_unaligned(dst, bytes / 16, lane, reinterpret_cast<uintptr_t>(src), false, [&](int p) { return src + static_cast<size_t>(p) * 16; });
 }
 __device__ __forceinline__ void plain_done() {
   asm volatile("cp.async.wait_all;" ::: "memory");
