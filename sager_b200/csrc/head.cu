@@ -15,8 +15,10 @@
 //
 // The head is the largest matrix of a step (151,936 x 2048: 255 MB), so the GEMV is a
 // persistent kernel: one CTA per SM, a producer warp streaming stages of whole rows (1680
-// contiguous bytes each at k = 2048) into a shared-memory ring with bulk copies, eight
-// consumer warps of four rows each. A lane owns a quarter of a block (64 weights, four sub-groups): two
+// contiguous bytes each at k = 2048) into a shared-memory ring with bulk copies, two groups of eight
+// consumer warps of four rows each, which take the stages in turn: what one group waits for - shared-memory loads with two lanes
+// to a bank, chains of dp4a - the other's arithmetic covers (two warps to a scheduler instead of four left its issue slots half
+// empty: 151,936 x 2048 49.7 us, now 44; with norm and top-k 64.4 and 59.0). A lane owns a quarter of a block (64 weights, four sub-groups): two
 // 16-byte runs of ql and one of qh, read as words (blocks start on 2-byte boundaries only: odd
 // blocks are realigned with a funnel shift), each ql word giving two packed words of 6-bit values
 // and each qh word serving four of them, fed to dp4a; a row of k = 2048 is one pass of a warp.
@@ -28,9 +30,11 @@ namespace sgr {
 namespace {
 
 constexpr int kQ6 = 210;                     // bytes per Q6_K super-block
-constexpr int kHeadWarps = 8;
+constexpr int kHeadWarps = 8;                 // warps to a stage
+constexpr int kHeadGroups = 2;                // groups of them, stages in turn
 constexpr int kHeadRows = 4;                  // rows a warp works on at once
-constexpr int kHeadThreads = kHeadWarps * 32 + 32;
+constexpr int kHeadConsumers = kHeadGroups * kHeadWarps;
+constexpr int kHeadThreads = kHeadConsumers * 32 + 32;
 constexpr int kHeadStages = 4;                // at most
 
 struct HeadArgs {
@@ -72,7 +76,7 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
   __syncthreads();
 
   bool ok = true;
-  if (warp == kHeadWarps) {                    // producer: the weights do not depend on the previous kernel
+  if (warp == kHeadConsumers) {                // producer: the weights do not depend on the previous kernel
     if (lane == 0) {
       int it = 0;
       for (int st = blockIdx.x; st < n_stages; st += gridDim.x, ++it) {
@@ -93,15 +97,15 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
     pdl_launch_dependents();
     // stage the activation row: codes, per-16-column sums, block scales
     const int ctid = threadIdx.x;
-    for (int i = ctid; i < nb * 64; i += kHeadWarps * 32) {
+    for (int i = ctid; i < nb * 64; i += kHeadConsumers * 32) {
       const int blk = i >> 6, wi = i & 63;
       reinterpret_cast<uint32_t*>(xs)[blk * 64 + wi] =
           reinterpret_cast<const uint32_t*>(a.xq + static_cast<size_t>(blk) * kX8 + 4)[wi];
     }
-    for (int i = ctid; i < nb; i += kHeadWarps * 32)
+    for (int i = ctid; i < nb; i += kHeadConsumers * 32)
       xd[i] = *reinterpret_cast<const float*>(a.xq + static_cast<size_t>(i) * kX8);
-    asm volatile("bar.sync 1, %0;" ::"n"(kHeadWarps * 32) : "memory");
-    for (int i = ctid; i < nb * 16; i += kHeadWarps * 32) {
+    asm volatile("bar.sync 1, %0;" ::"n"(kHeadConsumers * 32) : "memory");
+    for (int i = ctid; i < nb * 16; i += kHeadConsumers * 32) {
       const uint4 c = *reinterpret_cast<const uint4*>(xs + static_cast<size_t>(i) * 16);
       int s = __dp4a(static_cast<int>(c.x), 0x01010101, 0);
       s = __dp4a(static_cast<int>(c.y), 0x01010101, s);
@@ -109,25 +113,26 @@ __global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const H
       s = __dp4a(static_cast<int>(c.w), 0x01010101, s);
       xsum[i] = s;
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(kHeadWarps * 32) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(kHeadConsumers * 32) : "memory");
 
     // A lane owns a quarter of a block: the sixteen columns (n, is) of all four qslots, i.e. the
     // 16-byte runs ql[n*64 + is*16 ..], ql[n*64 + 32 + is*16 ..] and qh[n*32 + is*16 ..], which hold
     // the sub-groups t = n*8 + 2*qslot + is, qslot = 0..3 (64 weights, four scales). A row of
     // k = 2048 is one pass of the warp. Blocks start on 2-byte boundaries only: the runs are read
     // as five aligned words each and realigned with a funnel shift (by 0 or 16 bits).
-    int it = 0;
-    for (int st = blockIdx.x; st < n_stages && ok; st += gridDim.x, ++it) {
+    const int group = warp / kHeadWarps, gwarp = warp % kHeadWarps;
+    int it = group;
+    for (int st = blockIdx.x + group * gridDim.x; st < n_stages && ok; st += kHeadGroups * gridDim.x, it += kHeadGroups) {
       const int s = it % S;
       ok = mbar_wait(full + s, (it / S) & 1);
       if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
       const int r0 = st * a.rows_per_stage;
       const int nr = min(a.rows_per_stage, a.n_rows - r0);
       const unsigned char* stage = ring + static_cast<size_t>(s) * stage_bytes;
-      // four rows of the stage per warp and pass (rows warp, warp + 8, ...): their loads are in flight
+      // four rows of the stage per warp and pass (rows gwarp, gwarp + 8, ...): their loads are in flight
       // together, the activation words are fetched once for the four, and one transposing reduction
       // (six shuffles) replaces four of five
-      for (int rb = warp; rb < nr; rb += kHeadWarps * kHeadRows * (32 / G)) {
+      for (int rb = gwarp; rb < nr; rb += kHeadWarps * kHeadRows * (32 / G)) {
         const unsigned char* roww[kHeadRows];
 #pragma unroll
         for (int i = 0; i < kHeadRows; ++i)

@@ -53,6 +53,27 @@ def test_q6k_head_gemv(oracle, rows, k):
     assert lib().raw("sgr_status")(0) == 0
 
 
+@pytest.mark.parametrize("k,stages", [(2048, 4), (3072, 3), (4096, 2), (1024, 4)])
+@pytest.mark.parametrize("more", [0, 1, 2])
+def test_q6k_head_stages_go_round_two_groups(oracle, k, stages, more):
+    """Stage counts at which a CTA's two groups of warps have as many stages, or one of them one more or none, for every
+    depth of the ring; the last stage is half of one. Every row, against the oracle: exact integer sums, fp32 terms of a row."""
+    per_stage = 64 if k <= 1024 else 32
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rows = (more * sms + (0 if more else sms // 2)) * per_stage + per_stage // 2
+    rng = np.random.default_rng(rows + k)
+    base = make_q6k(rng, 1024, k)
+    pick = rng.integers(0, 1024, size=rows)
+    w = torch.from_numpy(base).to(DEV)[torch.from_numpy(pick).to(DEV)].contiguous()
+    _, x = make_x16(1, k, 5)
+    xq = _q8(x, k)
+    y = torch.full((rows,), float("nan"), dtype=torch.float32, device=DEV)
+    ops.gemv_q6_k_q8(w, xq, y, rows, k)
+    want = gemv_q6k_q8k(base, xq.cpu().numpy()[0], k)[pick]
+    assert rel(y.cpu().numpy(), want) <= GEMV_TOL
+    assert lib().raw("sgr_status")(0) == 0
+
+
 def test_q6k_head_gemv_unaligned_base_takes_the_plain_path(oracle):
     rows, k = 600, 2048
     rng = np.random.default_rng(9)
