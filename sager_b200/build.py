@@ -2,7 +2,8 @@
 sm_100a. The library is built in-tree (next to this file) so that it travels
 with the source tree; nothing is installed. Every source file is compiled to
 its own object (in parallel, only when it or a header changed) and the objects
-are linked into the shared library."""
+are linked into the shared library. csrc/fastcall.c, the entry points as Python
+callables, becomes an extension module of its own beside it."""
 from __future__ import annotations
 
 import glob
@@ -10,12 +11,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libsager_b200.so")
+FASTCALL = os.path.join(HERE, "_fastcall.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -49,10 +52,54 @@ def _obj(src):
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(FASTCALL):
         return True
-    t = os.path.getmtime(LIB)
-    return any(os.path.getmtime(p) > t for p in sources() + headers())
+    t = min(os.path.getmtime(LIB), os.path.getmtime(FASTCALL))
+    return any(os.path.getmtime(p) > t for p in sources() + headers() + [os.path.join(CSRC, "fastcall.c")])
+
+
+def fastcall_calls() -> str:
+    """The C functions of csrc/fastcall.c: one per parameter list that an int-returning entry point with a trailing
+    stream has in the headers (letters of capi.kinds_of)."""
+    from . import capi
+    kinds = sorted({k for k in map(capi.kinds_of, capi.prototypes().values()) if k})
+    types = {"p": "void*", "i": "int", "q": "long long", "z": "size_t", "f": "float", "d": "double"}
+    take = {"p": "as_pointer(a[{i}], &x{i})", "i": "as_integer(a[{i}], INT_MIN, INT_MAX, &n{i})",
+            "q": "as_integer(a[{i}], LLONG_MIN, LLONG_MAX, &n{i})", "z": "as_integer(a[{i}], 0, LLONG_MAX, &n{i})",
+            "f": "as_double(a[{i}], &n{i})", "d": "as_double(a[{i}], &n{i})"}
+    out = []
+    for ks in kinds:
+        args = ks[:-1]
+        out.append(f"static PyObject* call_{ks}(PyObject* self, PyObject* const* a, size_t nargsf, PyObject* kw) {{\n  Call* c = (Call*)self;\n"
+                   "  void* s;\n  int rc;")
+        for i, k in enumerate(args):
+            out.append(f"  void* x{i};" if k == "p" else f"  {'double' if k in 'fd' else 'long long'} n{i};")
+        out.append(f"  TAKE(kw == NULL && PyVectorcall_NARGS(nargsf) == {len(args)});")
+        out += ["  TAKE(" + take[k].format(i=i) + ");" for i, k in enumerate(args)]
+        out.append("  TAKE(as_stream(&s));\n  Py_BEGIN_ALLOW_THREADS")
+        params = ", ".join(types[k] for k in ks)
+        values = ", ".join([f"x{i}" if k == "p" else f"({types[k]})n{i}" for i, k in enumerate(args)] + ["s"])
+        out.append(f"  rc = ((int (*)({params}))c->fn)({values});\n  Py_END_ALLOW_THREADS\n  return finish(c, rc);\n}}")
+    out.append("static vectorcallfunc call_of(const char* kinds) {")
+    out += [f'  if (strcmp(kinds, "{ks}") == 0) return call_{ks};' for ks in kinds]
+    out.append("  return NULL;\n}\n")
+    return "\n".join(out)
+
+
+def build_fastcall() -> None:
+    os.makedirs(OBJ, exist_ok=True)
+    with open(os.path.join(OBJ, "fastcall_calls.inc"), "w") as f:
+        f.write(fastcall_calls())
+    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
+    if cc is None:
+        raise RuntimeError("no C compiler found")
+    cmd = [cc, "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], "-I", OBJ,
+           "-o", FASTCALL + ".tmp", os.path.join(CSRC, "fastcall.c"), "-lpthread"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("building the extension module failed")
+    os.replace(FASTCALL + ".tmp", FASTCALL)
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
@@ -98,6 +145,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError("link failed")
     os.replace(LIB + ".tmp", LIB)          # a reader never sees a half-written library
+    build_fastcall()
     return LIB
 
 

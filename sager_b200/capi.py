@@ -51,6 +51,22 @@ def parse_header(path: str = HEADER):
     return protos
 
 
+def prototypes():
+    return dict(parse_header(), **parse_header(DIAG_HEADER))
+
+
+_KINDS = {C.c_void_p: "p", C.c_int: "i", C.c_longlong: "q", C.c_size_t: "z", C.c_float: "f", C.c_double: "d"}
+
+
+def kinds_of(proto):
+    """The parameter list of an int-returning entry point that ends with a stream, a letter per parameter; None for others.
+    (size_t and unsigned long are one type here: all that matters is how a value is passed.)"""
+    res, args = proto
+    if res is not C.c_int or not args or args[-1] is not C.c_void_p or any(a not in _KINDS for a in args):
+        return None
+    return "".join(_KINDS[a] for a in args)
+
+
 class Lib:
     def __init__(self, path: str = LIB_PATH):
         if not os.path.exists(path):
@@ -59,7 +75,7 @@ class Lib:
                 "(there is no CPU or PyTorch fallback)")
         self.path = path
         self.cdll = C.CDLL(path)
-        self.protos = dict(parse_header(), **parse_header(DIAG_HEADER))
+        self.protos = prototypes()
         missing = []
         for name, (res, args) in self.protos.items():
             try:

@@ -12,7 +12,7 @@ import sys
 
 import torch
 
-from .capi import SagerError, lib
+from .capi import SagerError, kinds_of, lib
 
 
 _raw_stream = torch._C._cuda_getCurrentRawStream
@@ -30,20 +30,37 @@ def stream_ptr():
     return C.c_void_p(_stream())
 
 
+_fast = None
+
+
+def _fastcall():
+    """The extension module that makes the calls (csrc/fastcall.c)."""
+    global _fast
+    if _fast is None:
+        from . import _fastcall
+        _fastcall.setup(torch.Tensor, torch.nn.Parameter, _stream, _raw_stream, _device)
+        _fast = _fastcall
+    return _fast
+
+
 def _bind(name: str):
-    """The entry point as a Python function: tensors go as device addresses, the current stream last. A decode
-    step issues hundreds of these, so what does not depend on the arguments is looked up once."""
+    """The entry point as a callable: tensors go as device addresses, the current stream last. A decode step issues
+    hundreds of these: the extension module makes the call; `slow` takes the arguments that it does not know."""
     L = lib()
     cfn = getattr(L.cdll, "sgr_" + name)
     tensor, stream = torch.Tensor, _stream
 
-    def fn(*args):
+    def fail(rc):
+        raise SagerError("sgr_" + name, rc)
+
+    def slow(*args):
         rc = cfn(*[a.data_ptr() if isinstance(a, tensor) else a for a in args], stream())
         if rc != 0:
-            raise SagerError("sgr_" + name, rc)
+            fail(rc)
 
-    fn.__name__ = name
-    return fn
+    slow.__name__ = name
+    kinds = kinds_of(L.protos["sgr_" + name])
+    return slow if kinds is None else _fastcall().bind(kinds, C.cast(cfn, C.c_void_p).value, slow, fail, name)
 
 
 def call(name: str, *args):
