@@ -36,19 +36,22 @@ bool opt_in_smem(int bytes) {
 }
 
 // Launch that may start while the kernel before it in the stream drains (programmatic dependent launch);
-// the kernel waits for that one's results itself.
-template <typename... KArgs, typename... Args>
+// the kernel waits for that one's results itself. CLUSTER: CTAs to a cluster, along x.
+template <int CLUSTER = 1, typename... KArgs, typename... Args>
 int launch_pdl(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CLUSTER;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = CLUSTER > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? 0 : 4 /* kErrLaunch */;
 }
 

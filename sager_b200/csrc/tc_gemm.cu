@@ -82,6 +82,11 @@ __device__ __forceinline__ void tc_tma_2d(uint32_t dst, const CUtensorMap* map, 
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
 }
+// into this CTA's shared memory, the bytes counted at a barrier of the CTA pair (an address in the cluster's shared memory)
+__device__ __forceinline__ void tc_tma_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar) : "memory");
+}
 __device__ __forceinline__ void tc_tma_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
                ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)) : "memory");
@@ -243,32 +248,53 @@ __device__ __forceinline__ uint4 dequant_octet(const unsigned char* blk, int lan
 }
 
 // ---- Q4_K weights: the dequantisation inside the GEMM ------------------------------------------
-// A CTA owns 128 weight rows and up to 256 token rows. The 128 rows are the M lanes of tensor memory, so a thread
-// dequantises its row of a block in registers and stores it as the tensor-memory operand (tcgen05.st); only the
-// activations go through shared memory. Against a separate dequantisation and 128 x 128 tiles (7.5 + 64 us for
-// 4096 x 2048 over 2048 rows) that reads 36 bytes of weights per 64 k instead of 128 and half the activations: the
-// tiles' traffic from L2 was the bound. 43.7 us now, the MMAs' own time being 21. `scratch` still receives the dequantised
-// rows: with few tiles by CTAs of their own on the SMs left over (a thread's 16-byte pieces of its row take longer than its
-// block: 1000 x 4096 over 75 rows 33.8 -> 22.6 us, over 64 rows 54.5 -> 22.5), else each token tile writes its share of the blocks.
-//   * warps 0-7: unpack, four to a block, even and odd blocks; then the epilogue
-//   * warp 8: activation tiles (TMA, 128-byte swizzle, 64 k a stage)
-//   * warp 9: block columns of the weights (cp.async), four in flight
-//   * warp 10: tensor memory and MMA issue
-constexpr int kQ4Threads = 352, kQ4WStages = 4, kQ4WBytes = 128 * kW4, kQ4Slots = 3;
+// Persistent: a CTA, or a pair of CTAs (CG = 2, cta_group::2), takes units of 128 weight rows per CTA x up to 256 token rows. The
+// rows are the M lanes of tensor memory, so a thread dequantises its row of a block in registers and stores it as the
+// tensor-memory operand (tcgen05.st); only the activations go through shared memory, of a pair's each CTA half.
+//   * warps 0-7: unpack, four to a block, even and odd blocks, on into the next unit; a block is two of four slots in tensor memory,
+//     so neither four waits for the other's
+//   * warps 8-15: epilogue, a quarter of the lanes and half of the columns each; the accumulators are free once they are in
+//     registers as fp16
+//   * warp 16: activation tiles (TMA, 128-byte swizzle, 64 k a stage)
+//   * warp 17: block columns of the weights (a TMA copy of 128 blocks each), four in flight
+//   * warp 18: tensor memory and (a pair's first CTA) MMA issue
+// 4096 x 2048 over 2048 rows (MMAs 16 us at two units each, 20.8 at the library's rate): 38.5 us with a CTA per unit, whose start and epilogue
+// nothing covered, 32.8 persistent and in pairs, 31.8 with the weights by TMA (one warp's cp.async, 36 to a block with a division
+// each, took longer than the block: 130 x 4096 over 333 rows 28 -> 21), 31.2 with four slots instead of three. Bound now by the hand-overs
+// of a block, about 2,000 cycles where the MMAs of 256 columns need 2,080, and the scratch, 3.5 us.
+// `scratch` receives the dequantised rows: with few units by CTAs of their own on the SMs left over (a thread's 16-byte pieces of
+// its row take longer than its block: 1000 x 4096 over 75 rows 33.8 -> 22.6 us, over 64 rows 54.5 -> 22.5), else each token
+// tile writes its share of the blocks. (Written by the epilogue warps out of the weights' ring, 512 bytes a row: 33.8 us for 31.0.)
+constexpr int kQ4Unpack = 8, kQ4Epi = 8, kQ4WarpX = kQ4Unpack + kQ4Epi, kQ4WarpW = kQ4WarpX + 1, kQ4WarpMma = kQ4WarpW + 1;
+constexpr int kQ4Threads = (kQ4WarpMma + 1) * 32, kQ4WStages = 4, kQ4WBytes = 128 * kW4, kQ4Slots = 4;
 constexpr int kQ4BBytes = 128 * 1024;             // activation ring: 4 stages of 256 rows, 8 of 128 or fewer
 constexpr int kQ4Smem = 1024 + 1024 + kQ4BBytes + kQ4WStages * kQ4WBytes;
-enum { kQ4WFull = 0, kQ4WEmpty = 4, kQ4AFull = 8, kQ4AEmpty = 11, kQ4BFull = 14, kQ4BEmpty = 22, kQ4Acc = 30, kQ4Bars = 31 };
+enum { kQ4WFull = 0, kQ4WEmpty = 4, kQ4AFull = 8, kQ4AEmpty = 12, kQ4BFull = 16, kQ4BEmpty = 24, kQ4AccFull = 32, kQ4AccEmpty = 33, kQ4Drain = 34 };
+
+// The four weights of a word under `mask` (its low or its high nibbles), sd * q + sm rounded to fp16: 2^23 + q by byte insertion,
+// - 2^23 exactly. (Nibbles as 1024 + q in fp16 and an addition in mixed precision, half the integer instructions: no faster.)
+__device__ __forceinline__ void dequant_word(uint32_t raw, uint32_t mask, f32x2 sd, f32x2 sm, uint32_t& v01, uint32_t& v23) {
+  const f32x2 magic = splat2(-8388608.f);
+  const uint32_t nib = raw & mask;
+  const f32x2 q01 = add2(pack2(__byte_perm(nib, 0x4B000000u, 0x7440), __byte_perm(nib, 0x4B000000u, 0x7441)), magic);
+  const f32x2 q23 = add2(pack2(__byte_perm(nib, 0x4B000000u, 0x7442), __byte_perm(nib, 0x4B000000u, 0x7443)), magic);
+  const f32x2 f01 = fma2(sd, q01, sm), f23 = fma2(sd, q23, sm);
+  v01 = h2_bits(__floats2half2_rn(part2(f01, 0), part2(f01, 1)));
+  v23 = h2_bits(__floats2half2_rn(part2(f23, 0), part2(f23, 1)));
+}
 
 struct Q4Args {
   const unsigned char* w;
   uint16_t *y, *scratch;
   int n_rows, k, n_tokens;
-  int bn, stages, tiles;                          // token rows per CTA, activation stages, token tiles (grid.y beyond: scratch)
+  int bn, stages, tiles;                          // token rows per unit, activation stages, token tiles
+  int row_units, units, workers;                  // groups of CG row tiles, units, CTAs that work on them (the others: scratch)
   int tiles_write;                                // the token tiles write the scratch
   int* status;
 };
 
-__global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_constant__ CUtensorMap map_x, const Q4Args a) {
+template <int CG>
+__global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const Q4Args a) {
   extern __shared__ unsigned char tc_smem_raw[];
   const uint32_t base = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
   unsigned char* smem = tc_smem_raw + (base - smem_u32(tc_smem_raw));
@@ -277,13 +303,13 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
   volatile int* fail = reinterpret_cast<volatile int*>(smem + 516);
   unsigned char* w_sm = smem + 1024 + kQ4BBytes;
   const uint32_t b_sm = base + 1024;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row0 = blockIdx.x * 128, tok0 = blockIdx.y * a.bn;
-  const int ntok = min(a.bn, a.n_tokens - tok0), nb = a.k / kQK;
-  if (static_cast<int>(blockIdx.y) >= a.tiles) {  // writes the row tile's dequantised blocks, a warp per block
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = a.k / kQK;
+  if (static_cast<int>(blockIdx.x) >= a.workers) {        // writes a row tile's dequantised blocks, a warp per block
     pdl_wait();
     pdl_launch_dependents();
-    const int blocks = min(128, a.n_rows - row0) * nb, part = blockIdx.y - a.tiles, parts = gridDim.y - a.tiles;
+    const int row_tiles = (a.n_rows + 127) / 128, i = blockIdx.x - a.workers, row0 = i % row_tiles * 128;
+    const int blocks = min(128, a.n_rows - row0) * nb, part = i / row_tiles, parts = (gridDim.x - a.workers) / row_tiles;
+    if (part >= parts) return;
     const unsigned char* w = a.w + static_cast<size_t>(row0) * nb * kW4;
     uint4* out = reinterpret_cast<uint4*>(a.scratch + static_cast<size_t>(row0) * a.k);
     const int stride = parts * (kQ4Threads / 32);
@@ -297,24 +323,27 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     }
     return;
   }
-  const uint32_t b_bytes = static_cast<uint32_t>(a.bn) * 128;
+  const uint32_t rank = CG == 2 ? blockIdx.x & 1u : 0u, b_bytes = static_cast<uint32_t>(a.bn / CG) * 128;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < kQ4WStages; ++i) { mbar_init(&bar[kQ4WFull + i], 32); mbar_init(&bar[kQ4WEmpty + i], 4); }
-    for (int i = 0; i < kQ4Slots; ++i) { mbar_init(&bar[kQ4AFull + i], 4); mbar_init(&bar[kQ4AEmpty + i], 1); }
+    for (int i = 0; i < kQ4WStages; ++i) { mbar_init(&bar[kQ4WFull + i], 1); mbar_init(&bar[kQ4WEmpty + i], 4); }
+    for (int i = 0; i < kQ4Slots; ++i) { mbar_init(&bar[kQ4AFull + i], 4 * CG); mbar_init(&bar[kQ4AEmpty + i], 1); }
     for (int i = 0; i < 8; ++i) { mbar_init(&bar[kQ4BFull + i], 1); mbar_init(&bar[kQ4BEmpty + i], 1); }
-    mbar_init(&bar[kQ4Acc], 1);
+    mbar_init(&bar[kQ4AccFull], 1);
+    mbar_init(&bar[kQ4AccEmpty], kQ4Epi * CG);
+    mbar_init(&bar[kQ4Drain], 1);
     *fail = 0;
     fence_barrier_init();
     fence_proxy_async();
   }
-  if (warp == 10) {
+  if (warp == kQ4WarpMma) {
     __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::%2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512), "n"(CG) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::%0.sync.aligned;" ::"n"(CG) : "memory");
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (CG == 2) cluster_sync();          // the other CTA's barriers are there
   tc_fence_after();
   const uint32_t tmem = *tmem_slot, tmem_a = tmem + 256;
   auto wait_warp = [&](int b, unsigned parity) {
@@ -322,168 +351,201 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     *fail = 1;
     return false;
   };
+  // arrives at a barrier of the CTA that issues the MMAs; `first` is that barrier's address there
+  auto arrive_first = [&](uint64_t* b, uint32_t first) {
+    if constexpr (CG == 1) mbar_arrive_one(b);
+    else mbar_arrive_cluster(first);
+  };
+  // units of this CTA (pair): f(first weight row of this CTA, first token row, token rows, token tile) -> false ends the walk
+  auto for_units = [&](auto f) {
+    for (int u = blockIdx.x / CG; u < a.units; u += a.workers / CG) {
+      const int t = u / a.row_units, tok0 = t * a.bn;
+      if (!f(((u - t * a.row_units) * CG + static_cast<int>(rank)) * 128, tok0, min(a.bn, a.n_tokens - tok0), t)) return;
+    }
+  };
 
-  if (warp < 8) {
+  if (warp < kQ4Unpack) {
     const int grp = warp >> 2, r = (warp & 3) * 32 + lane;
-    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    pdl_wait();                                   // scratch and y may still be read by the kernel before
+    const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16, a_full = cluster_addr(&bar[kQ4AFull], 0);
+    pdl_wait();                                   // scratch may still be read by the kernel before
     pdl_launch_dependents();
-    const f32x2 magic = splat2(-8388608.f);
-    const int share = a.tiles;                    // this token tile writes blocks blockIdx.y, + share, ... to scratch
-    uint16_t* row_out = a.scratch + static_cast<size_t>(min(row0 + r, a.n_rows - 1)) * a.k;
-    bool ok = true;
-    for (int job = grp; job < nb && ok; job += 2) {
-      const int st = job % kQ4WStages;
-      if (!(ok = wait_warp(kQ4WFull + st, (job / kQ4WStages) & 1))) break;
-      const uint4* blk = reinterpret_cast<const uint4*>(w_sm + st * kQ4WBytes + r * kW4);
-      const uint4 hdr = blk[0];
-      const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
-      const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
-      const bool keep = a.tiles_write && job % share == static_cast<int>(blockIdx.y) && row0 + r < a.n_rows;
+    const int share = a.tiles;                    // the units of token tile t write blocks t, t + share, ... to scratch
+    int job0 = 0;                                 // blocks of the units before this one
+    for_units([&](int row0, int, int, int tile) {
+      uint16_t* row_out = a.scratch + static_cast<size_t>(min(row0 + r, a.n_rows - 1)) * a.k;
+      for (int b = (grp ^ job0) & 1; b < nb; b += 2) {
+        const int job = job0 + b, st = job % kQ4WStages;
+        if (!wait_warp(kQ4WFull + st, (job / kQ4WStages) & 1)) return false;
+        const uint4* blk = reinterpret_cast<const uint4*>(w_sm + st * kQ4WBytes + r * kW4);
+        const uint4 hdr = blk[0];
+        const float d = h2f(static_cast<uint16_t>(hdr.x & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(hdr.x >> 16));
+        const Scales6 s6 = unpack_scales6(hdr.y, hdr.z, hdr.w);
+        const bool keep = a.tiles_write && b % share == tile && row0 + r < a.n_rows;
 #pragma unroll 1
-      for (int g = 0; g < 4; ++g) {
-        const int x = 2 * job + (g >> 1), slot = x % kQ4Slots;
-        if ((g & 1) == 0) {
-          if (!(ok = wait_warp(kQ4AEmpty + slot, ((x / kQ4Slots) & 1) ^ 1u))) break;
-          tc_fence_after();
-        }
-        const uint4 q0 = blk[1 + 2 * g], q1 = blk[2 + 2 * g];
-        const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const uint32_t scw = (g < 2 ? s6.sc[0] : s6.sc[1]) >> (16 * (g & 1)), mnw = (g < 2 ? s6.mn[0] : s6.mn[1]) >> (16 * (g & 1));
+        for (int g = 0; g < 4; ++g) {
+          const int x = 2 * job + (g >> 1), slot = x % kQ4Slots;
+          const uint4 q0 = blk[1 + 2 * g], q1 = blk[2 + 2 * g];
+          const uint32_t raw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+          const uint32_t scw = (g < 2 ? s6.sc[0] : s6.sc[1]) >> (16 * (g & 1)), mnw = (g < 2 ? s6.mn[0] : s6.mn[1]) >> (16 * (g & 1));
+          uint32_t v[32];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {             // sub-block 2 g + h: value = fp16(fma(d * sc, q, -(dmin * mn)))
-          const f32x2 sd = splat2(d * static_cast<float>((scw >> (8 * h)) & 0xFFu));
-          const f32x2 sm = splat2(-(dmin * static_cast<float>((mnw >> (8 * h)) & 0xFFu)));
-          const uint32_t dst = tmem_a + lanes + slot * 64 + (g & 1) * 32 + h * 16;
+          for (int h = 0; h < 2; ++h) {
+            // sub-block 2 g + h: value = fp16(fma(d * sc, q, -(dmin * mn))); the odd one's nibbles come sixteen-fold, its scale as a sixteenth (exact)
+            const f32x2 sd = splat2((h ? 0.0625f : 1.f) * (d * static_cast<float>((scw >> (8 * h)) & 0xFFu)));
+            const f32x2 sm = splat2(-(dmin * static_cast<float>((mnw >> (8 * h)) & 0xFFu)));
 #pragma unroll
-          for (int i0 = 0; i0 < 8; i0 += 4) {
-            uint32_t v[8];
+            for (int i = 0; i < 8; ++i) dequant_word(raw[i], h ? 0xF0F0F0F0u : 0x0F0F0F0Fu, sd, sm, v[16 * h + 2 * i], v[16 * h + 2 * i + 1]);
+          }
+          if ((g & 1) == 0) {
+            if (!wait_warp(kQ4AEmpty + slot, ((x / kQ4Slots) & 1) ^ 1u)) return false;
+            tc_fence_after();
+          }
+          tmem_st32(tmem_a + lanes + slot * 64 + (g & 1) * 32, v);
+          if (keep) {
+            uint4* o = reinterpret_cast<uint4*>(row_out + b * kQK + g * 64);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const uint32_t nib = (raw[i0 + i] >> (4 * h)) & 0x0F0F0F0Fu;
-#pragma unroll
-              for (int c = 0; c < 2; ++c) {       // 2^23 + q by byte insertion, - 2^23 exactly
-                const f32x2 q = add2(pack2(__byte_perm(nib, 0x4B000000u, 0x7440 + 2 * c), __byte_perm(nib, 0x4B000000u, 0x7441 + 2 * c)), magic);
-                const f32x2 f = fma2(sd, q, sm);
-                asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(v[2 * i + c]) : "f"(part2(f, 1)), "f"(part2(f, 0)));
-              }
-            }
-            tmem_st8(dst + 2 * i0, v);
-            if (keep) {
-              uint4* o = reinterpret_cast<uint4*>(row_out + job * kQK + (2 * g + h) * 32 + i0 * 4);
-              o[0] = make_uint4(v[0], v[1], v[2], v[3]);
-              o[1] = make_uint4(v[4], v[5], v[6], v[7]);
-            }
+            for (int i = 0; i < 8; ++i) o[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          }
+          if (g & 1) {
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) arrive_first(&bar[kQ4AFull + slot], a_full + 8 * slot);
           }
         }
-        if (g & 1) {
-          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_one(&bar[kQ4AFull + slot]);
-        }
+        if (lane == 0) mbar_arrive_one(&bar[kQ4WEmpty + st]);
       }
-      if (ok && lane == 0) mbar_arrive_one(&bar[kQ4WEmpty + st]);
-    }
-    // epilogue: this thread's weight row, half of the token columns; lane pairs exchange so that a store is two rows
-    ok = ok && wait_warp(kQ4Acc, 0);
-    if (ok && *fail == 0) {
+      job0 += nb;
+      return true;
+    });
+  } else if (warp < kQ4Unpack + kQ4Epi) {
+    // this thread's weight row, half of the token columns; lane pairs trade halves so that a store is two rows of one token
+    const int quarter = warp & 3, half = ((warp - kQ4Unpack) >> 2) * (a.bn >> 1);
+    const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + half, acc_empty = cluster_addr(&bar[kQ4AccEmpty], 0);
+    const bool pairs = (a.n_rows & 1) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 3u) == 0;
+    const int odd = lane & 1;
+    unsigned ph = 0;
+    pdl_wait();                                   // y may still be read by the kernel before
+    for_units([&](int row0, int tok0, int ntok, int) {
+      if (!wait_warp(kQ4AccFull, ph)) return false;
+      ph ^= 1u;
       tc_fence_after();
-      const int row = row0 + r, half = (a.bn >> 1);
-      const int c1 = min((grp + 1) * half, ntok);
-      const bool pairs = (a.n_rows & 1) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 3u) == 0;
-      const bool odd = lane & 1;
-#pragma unroll 1
-      for (int c = grp * half; c < c1; c += 8) {
-        uint32_t v[8];
-        tmem_ld8(tmem + lanes + c, v);
+      const int cols = min(a.bn >> 1, ntok - half), row = row0 + quarter * 32 + lane;
+      uint32_t h[64];                             // tokens 2 i, 2 i + 1 of the half
+#pragma unroll
+      for (int c = 0; c < 128; c += 16) {
+        if (c >= cols) break;
+        uint32_t v[16];
+        tc_ld16(src + c, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (pairs) {
 #pragma unroll
-          for (int q = 0; q < 8; q += 2) {
-            const uint32_t got = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[q] : v[q + 1], 1);
-            const float lo = __uint_as_float(odd ? got : v[q]), hi = __uint_as_float(odd ? v[q + 1] : got);
-            const int t = c + q + (odd ? 1 : 0);
-            if (t < c1 && row < a.n_rows)
-              *reinterpret_cast<uint32_t*>(a.y + static_cast<size_t>(tok0 + t) * a.n_rows + (row & ~1)) = h2_bits(__floats2half2_rn(lo, hi));
-          }
-        } else if (row < a.n_rows) {
+        for (int i = 0; i < 8; ++i) h[c / 2 + i] = h2_bits(__floats2half2_rn(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_first(&bar[kQ4AccEmpty], acc_empty);
+      uint16_t* y = a.y + static_cast<size_t>(tok0 + half) * a.n_rows + row;
+      if (pairs) {
+        const uint32_t sel = odd ? 0x3276u : 0x5410u;
+        const int last = row < a.n_rows ? cols : 0;
+        y += odd ? a.n_rows - 1 : 0;
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            if (c + q < c1) a.y[static_cast<size_t>(tok0 + c + q) * a.n_rows + row] = f2h(__uint_as_float(v[q]));
+        for (int i = 0; i < 64; ++i) {
+          if (2 * i >= cols) break;
+          const uint32_t v = __byte_perm(h[i], __shfl_xor_sync(0xFFFFFFFFu, h[i], 1), sel);
+          if (2 * i + odd < last) *reinterpret_cast<uint32_t*>(y) = v;
+          y += 2 * static_cast<size_t>(a.n_rows);
+        }
+      } else if (row < a.n_rows) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          if (2 * i >= cols) break;
+          y[0] = static_cast<uint16_t>(h[i] & 0xFFFFu);
+          if (2 * i + 1 < cols) y[a.n_rows] = static_cast<uint16_t>(h[i] >> 16);
+          y += 2 * static_cast<size_t>(a.n_rows);
         }
       }
-    }
-  } else if (warp == 8) {
+      return true;
+    });
+  } else if (warp == kQ4WarpX) {
+    const uint32_t b_full = cluster_addr(&bar[kQ4BFull], 0);
+    int s = 0;
+    unsigned ph = 1;
     pdl_wait();
     if (lane == 0) {
-      for (int kb = 0; kb < 4 * nb; ++kb) {
-        const int s = kb % a.stages;
-        if (!mbar_wait_tight(&bar[kQ4BEmpty + s], ((kb / a.stages) & 1) ^ 1u)) {
-          *fail = 1;
-          break;
+      for_units([&](int, int tok0, int ntok, int) {
+        const int from = tok0 + static_cast<int>(rank) * (max(16, (ntok + 15) & ~15) >> 1);
+        for (int kb = 0; kb < 4 * nb; ++kb) {
+          if (!mbar_wait_tight(&bar[kQ4BEmpty + s], ph)) {
+            *fail = 1;
+            return false;
+          }
+          // (of a pair: the first CTA's barrier counts both halves; its phase cannot be over before its own expect)
+          if (rank == 0) mbar_expect_tx(&bar[kQ4BFull + s], CG * b_bytes);
+          if constexpr (CG == 1) tc_tma_2d(b_sm + s * b_bytes, &map_x, kb * kBK, tok0, &bar[kQ4BFull + s]);
+          else tc_tma_2d_pair(b_sm + s * b_bytes, &map_x, kb * kBK, from, b_full + 8 * s);
+          if (++s == a.stages) { s = 0; ph ^= 1u; }
         }
-        mbar_expect_tx(&bar[kQ4BFull + s], b_bytes);
-        tc_tma_2d(b_sm + s * b_bytes, &map_x, kb * kBK, tok0, &bar[kQ4BFull + s]);
-      }
+        return true;
+      });
     }
-  } else if (warp == 9) {
-    // (the weights do not depend on the kernel before) 16-byte piece p = 9 * row + c goes to lane p % 32; nine steps
-    // of 32 pieces are 32 rows. Rows past the matrix are zero: never stored. (Repeating its last row, hundreds of warps
-    // asked for the same lines: 32 rows over 2048 tokens of 2048 columns 32.3 us, now 13.6.)
-    const int row_bytes = nb * kW4, last = a.n_rows - 1 - row0;
-    for (int job = 0; job < nb; ++job) {
-      const int st = job % kQ4WStages;
-      if (!wait_warp(kQ4WEmpty + st, ((job / kQ4WStages) & 1) ^ 1u)) break;
-      const unsigned char* src = a.w + static_cast<size_t>(row0) * row_bytes + job * kW4;
-      const uint32_t dst = smem_u32(w_sm + st * kQ4WBytes) + lane * 16;
-      if (last >= 127) {
-#pragma unroll 9
-        for (int q = 0; q < 36; ++q) {
-          const int piece = q * 32 + lane, row = piece / 9;
-          cp_async16(dst + q * 512, src + static_cast<size_t>(row) * row_bytes + (piece - 9 * row) * 16);
+  } else if (warp == kQ4WarpW) {
+    // (the weights do not depend on the kernel before) Rows past the matrix arrive as zeros and are never stored.
+    int st = 0;
+    unsigned ph = 1;
+    if (lane == 0) {
+      for_units([&](int row0, int, int, int) {
+        for (int b = 0; b < nb; ++b) {
+          if (!mbar_wait_tight(&bar[kQ4WEmpty + st], ph)) {
+            *fail = 1;
+            return false;
+          }
+          mbar_expect_tx(&bar[kQ4WFull + st], kQ4WBytes);
+          tc_tma_2d(smem_u32(w_sm + st * kQ4WBytes), &map_w, b * kW4, row0, &bar[kQ4WFull + st]);
+          if (++st == kQ4WStages) { st = 0; ph ^= 1u; }
         }
-      } else {
-#pragma unroll 1
-        for (int q = 0; q < 36; ++q) {
-          const int piece = q * 32 + lane, row = piece / 9;
-          cp_async16_or_zero(dst + q * 512, src + static_cast<size_t>(min(row, last)) * row_bytes + (piece - 9 * row) * 16, row <= last);
-        }
-      }
-      cp_async_arrive(&bar[kQ4WFull + st]);
+        return true;
+      });
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
-    const uint32_t lead = elect_one();
-    const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc_f16(max(16, (ntok + 15) & ~15)), 0);
-    int slot = 0, s = 0;
-    unsigned slot_ph = 0, s_ph = 0;
-    bool ok = true;
-    for (int x = 0; x < 2 * nb && ok; ++x) {      // half-blocks
-      if (!(ok = wait_warp(kQ4AFull + slot, slot_ph))) break;
+    if (rank == 0) {
+      const uint32_t lead = elect_one();
+      int slot = 0, s = 0;
+      unsigned slot_ph = 0, s_ph = 0, acc_ph = 1;
+      for_units([&](int, int, int ntok, int) {
+        const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc_f16(max(16, (ntok + 15) & ~15), 128 * CG), 0);
+        if (!wait_warp(kQ4AccEmpty, acc_ph)) return false;
+        acc_ph ^= 1u;
+        for (int x = 0; x < 2 * nb; ++x) {        // half-blocks
+          if (!wait_warp(kQ4AFull + slot, slot_ph)) return false;
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        if (!(ok = wait_warp(kQ4BFull + s, s_ph))) break;
-        tc_fence_after();
-        const uint32_t db = umma_desc_swizzled(b_sm + s * b_bytes), ta = tmem_a + slot * 64 + j * 32;
+          for (int j = 0; j < 2; ++j) {
+            if (!wait_warp(kQ4BFull + s, s_ph)) return false;
+            tc_fence_after();
+            const uint32_t db = umma_desc_swizzled(b_sm + s * b_bytes), ta = tmem_a + slot * 64 + j * 32;
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) umma_ts(lead, tmem, ta + kk * 8, db + kk * 2, kDescSwizzled, idesc, (x | j | kk) != 0);
-        if (lead) umma_commit(&bar[kQ4BEmpty + s]);
-        if (++s == a.stages) { s = 0; s_ph ^= 1u; }
-      }
-      if (!ok) break;
-      if (lead) umma_commit(&bar[kQ4AEmpty + slot]);
-      if (++slot == kQ4Slots) { slot = 0; slot_ph ^= 1u; }
+            for (int kk = 0; kk < 4; ++kk) umma_ts<CG>(lead, tmem, ta + kk * 8, db + kk * 2, kDescSwizzled, idesc, (x | j | kk) != 0);
+            if (lead) umma_commit<CG>(&bar[kQ4BEmpty + s]);
+            if (++s == a.stages) { s = 0; s_ph ^= 1u; }
+          }
+          if (lead) umma_commit<CG>(&bar[kQ4AEmpty + slot]);
+          if (++slot == kQ4Slots) { slot = 0; slot_ph ^= 1u; }
+        }
+        if (lead) umma_commit<CG>(&bar[kQ4AccFull]);
+        return true;
+      });
+      if (lead) umma_commit<CG>(&bar[kQ4Drain]);  // everything issued has finished before tensor memory goes back
     }
-    if (lead) umma_commit(&bar[kQ4Acc]);          // arrives when everything issued so far has finished
-    mbar_wait_tight(&bar[kQ4Acc], 0);
+    mbar_wait_tight(&bar[kQ4Drain], 0);
   }
+  __syncwarp();
   tc_fence_before();
   __syncthreads();
-  if (warp == 10) {
+  if constexpr (CG == 2) cluster_sync();          // neither CTA goes while the other may still arrive at its barriers
+  if (warp == kQ4WarpMma) {
     __syncwarp();
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::%2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512), "n"(CG) : "memory");
   }
   if (threadIdx.x == 0 && *fail != 0 && a.status != nullptr) atomicExch(a.status, 1);
 }
@@ -582,6 +644,18 @@ bool operand_map(CUtensorMap* tm, const void* base, int rows, int k, int layout,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A [rows][k] Q4_K matrix as tiles of one block column of 128 rows.
+bool weight_map(CUtensorMap* tm, const void* base, int rows, int k) {
+  EncodeFn enc = tc_encoder();
+  if (enc == nullptr) return false;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k / kQK) * kW4, static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k / kQK) * kW4};
+  const cuuint32_t box[2] = {kW4, 128};
+  const cuuint32_t estr[2] = {1u, 1u};
+  return enc(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <bool F32OUT>
 int launch_tc_gemm(const void* w16, const void* x16, void* y, int n_rows, int k, int n_tokens, cudaStream_t s) {
   if (n_rows <= 0 || n_tokens <= 0) return kOk;
@@ -619,39 +693,67 @@ int launch_dequant(const void* w, void* out16, long long n_blocks, cudaStream_t 
 
 int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratch, int n_rows, int k, int n_tokens, cudaStream_t s) {
   if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(y) & 1u)) return kErrAlign;
-  const int sms = device_sms(), row_tiles = (n_rows + 127) / 128;
+  const int sms = device_sms(), row_tiles = (n_rows + 127) / 128, nb = k / kQK;
   if (sms <= 0) return kErrLaunch;
-  // Token rows per CTA: the fewest estimated cycles - waves of CTAs, each its blocks at the MMAs' rate (130 cycles
-  // per 256 columns and K = 16) or the unpacking's (about 1100 a block), and start-up and epilogue.
-  int bn = 64;
-  long long best = 0;
-  for (const int cand : {256, 128, 64}) {
-    const long long waves = (static_cast<long long>(row_tiles) * ((n_tokens + cand - 1) / cand) + sms - 1) / sms;
-    const long long cycles = waves * (static_cast<long long>(k / kQK) * std::max(2080 * cand / 256, 1100) + 4000 + 12 * cand);
-    if (best == 0 || cycles < best) {
-      best = cycles;
-      bn = cand;
+  // Token rows per unit, CTAs that share a unit, and who writes the scratch: what takes the least by estimates in us, fitted to
+  // 17 shapes (4096 x 2048 over 2048 tokens: 31 measured / 31 estimated with units of a pair's 256 rows x 240 tokens, 45 / 44 with 128
+  // tokens, 33 / 34 by single CTAs; 1000 x 2048 over 777: 12.2 / 13.3 with 64 tokens, 14.1 / 14.2 with 208).
+  //   a block column of a unit: 1.0 and, with the square of its tokens, up to 0.35 more, a fifth more when every SM works; a pair
+  //     brings half of the activations per CTA and gains a twentieth past 128 tokens, but costs 0.3 to set up
+  //   the scratch, per block of a row tile: SMs that the units leave idle, in whole columns of row tiles, 3.2 / spare beside
+  //     the units' 1.3; the units of a row tile themselves, 2 / token tiles on top of it; or the dequantisation kernel ahead of the
+  //     GEMM, 2.5 us and the bytes at 5 TB/s (8192 x 4096 over 64 tokens: 53 us by one spare column, 41 by the kernel ahead).
+  struct Plan { int cg, bn, tiles, units, workers, spare; bool ahead; double us; } p{};
+  for (int cg = 1; cg <= (row_tiles > 1 ? 2 : 1); ++cg) {
+    for (int most = 256, last = 0; most >= 32; most -= 16) {
+      const int t = (n_tokens - 1) / most + 1, bn = ((n_tokens - 1) / t + 16) & ~15;      // tiles of nearly equal length
+      if (bn == last) continue;
+      last = bn;
+      Plan c{cg, bn, (n_tokens + bn - 1) / bn, 0, 0, 0, false, 0.};
+      const long long units = static_cast<long long>((row_tiles + cg - 1) / cg) * c.tiles;
+      if (units > 0x3FFFFFFF) continue;
+      c.units = static_cast<int>(units);
+      c.workers = std::min(c.units, sms / cg) * cg;
+      const int waves = (c.units * cg + c.workers - 1) / c.workers;
+      const double wide = bn / 256.;
+      c.us = 4 + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.05 : 1.);
+      const int spare = std::min(nb, (sms - c.workers) / row_tiles);
+      const double by_spare = spare > 0 ? nb * std::max(0., 3.2 / spare - 1.3) : 1e30, by_tiles = 2. * nb / c.tiles;
+      const double by_kernel = 2.5 + static_cast<double>(n_rows) * k * 2.5625 / 5e6;
+      c.spare = by_spare < by_tiles ? spare : 0;
+      if (by_kernel < std::min(by_spare, by_tiles)) {
+        c.spare = 0;
+        c.ahead = true;
+      }
+      c.us += std::min(by_kernel, std::min(by_spare, by_tiles));
+      if (p.cg == 0 || c.us < p.us) p = c;
     }
   }
-  CUtensorMap mx;
-  if (!operand_map(&mx, x, n_tokens, k, kLayoutSwizzled, bn)) return kErrUnsupported;
-  if (!opt_in_smem<tc_gemm_q4_kernel>(kQ4Smem)) return kErrLaunch;
-  Q4Args a{static_cast<const unsigned char*>(w), y, scratch, n_rows, k, n_tokens, bn, std::min(8, kQ4BBytes / (bn * 128)), (n_tokens + bn - 1) / bn, 0, status_word()};
-  // Who writes the scratch, by us per block of a row tile (measured): SMs that the tiles leave idle, in whole columns of row
-  // tiles, 3.2 / spare beside the tiles' 1.3; the tiles themselves, 2 / tiles on top of it; or the dequantisation kernel
-  // ahead of the GEMM, 2.5 us and the bytes at 5 TB/s. Few tokens over many rows leave few SMs and few tiles: 8192 x 4096
-  // over 64 tokens takes 53 us by one spare column, 43 by the kernel ahead.
-  int spare = std::max(0, std::min(k / kQK, sms / row_tiles - a.tiles));
-  if (32 * a.tiles >= spare * (13 * a.tiles + 20)) spare = 0;
-  const double added = k / kQK * (spare > 0 ? std::max(0.0, 3.2 / spare - 1.3) : 2.0 / a.tiles);
-  const bool ahead = added > 2.5 + static_cast<double>(n_rows) * k * 2.5625 / 5e6;
-  if (ahead) {
-    const int rc = launch_dequant(w, scratch, static_cast<long long>(n_rows) * (k / kQK), s);
+  if (p.cg == 0) return kErrUnsupported;
+  CUtensorMap mx, mw;
+  if (!weight_map(&mw, w, n_rows, k) || !operand_map(&mx, x, n_tokens, k, kLayoutSwizzled, p.bn / p.cg)) return kErrUnsupported;
+  Q4Args a{};
+  a.scratch = scratch; a.y = y;
+  a.n_rows = n_rows; a.k = k; a.n_tokens = n_tokens; a.w = static_cast<const unsigned char*>(w);
+  a.bn = p.bn;
+  a.stages = std::min(8, kQ4BBytes * p.cg / (p.bn * 128));
+  a.tiles = p.tiles;
+  a.row_units = (row_tiles + p.cg - 1) / p.cg;
+  a.units = p.units;
+  a.workers = p.workers;
+  a.tiles_write = p.spare == 0 && !p.ahead;
+  a.status = status_word();
+  if (p.ahead) {
+    const int rc = launch_dequant(w, scratch, static_cast<long long>(n_rows) * nb, s);
     if (rc != kOk) return rc;
-    spare = 0;
   }
-  a.tiles_write = spare == 0 && !ahead;
-  return launch_pdl(tc_gemm_q4_kernel, dim3(row_tiles, a.tiles + spare), kQ4Threads, kQ4Smem, s, mx, a);
+  const dim3 grid(p.workers + (p.spare * row_tiles + p.cg - 1) / p.cg * p.cg);
+  if (p.cg == 1) {
+    if (!opt_in_smem<tc_gemm_q4_kernel<1>>(kQ4Smem)) return kErrLaunch;
+    return launch_pdl(tc_gemm_q4_kernel<1>, grid, kQ4Threads, kQ4Smem, s, mx, mw, a);
+  }
+  if (!opt_in_smem<tc_gemm_q4_kernel<2>>(kQ4Smem)) return kErrLaunch;
+  return launch_pdl<2>(tc_gemm_q4_kernel<2>, grid, kQ4Threads, kQ4Smem, s, mx, mw, a);
 }
 
 }  // namespace

@@ -189,6 +189,30 @@ def test_q4k_gemm_few_rows_past_a_tile(rows):
     assert rel(y[:tok].float().cpu().numpy(), gemm_want(w16, x_dev).cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
 
 
+@pytest.mark.parametrize("rows,k,tok", [
+    (4224, 1024, 2040),      # CTA pairs over an odd number of row tiles, two units each, a ragged last token tile
+    (2176, 4096, 1000),      # pairs, one unit each, the scratch by CTAs of their own
+    (3201, 1024, 2048),      # pairs, odd rows: no paired stores
+    (4224, 256, 1555),       # single CTAs, two units each, one block to a row
+    (4096, 512, 2047),       # the units of a CTA start on even and odd blocks of the rings alike
+])
+def test_q4k_gemm_units(rows, k, tok):
+    """Several units to a CTA, units of CTA pairs, and what lies past the matrix in them."""
+    w_np, w_dev = make_q4k(rows, k, 33)
+    x_np, x_dev = make_x16(tok, k, 34)
+    scratch = torch.zeros(rows * k + 8, dtype=torch.float16, device=DEV)
+    y = torch.full((tok + 1, rows), 9.0, dtype=torch.float16, device=DEV)
+    w16 = torch.zeros(rows, k, dtype=torch.float16, device=DEV)
+    ops.dequant_q4_k_f16(w_dev, w16, rows, k)
+    want = gemm_want(w16, x_dev)
+    for _ in range(2):       # (the second launch may start while the first one drains)
+        ops.tc_gemm_q4_k_f16(w_dev, x_dev, y, scratch, rows, k, tok)
+    assert torch.equal(scratch[:rows * k].view(torch.int16), w16.view(-1).view(torch.int16)) and torch.all(scratch[rows * k:] == 0)
+    # fp32 accumulation in another order, one rounding to fp16
+    assert rel(y[:tok].float().cpu().numpy(), want.cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
+    assert lib().raw("sgr_status")(0) == 0
+
+
 @pytest.mark.parametrize("rows,k,tok", [(8192, 4096, 64), (8200, 4096, 3), (12288, 4096, 17)])
 def test_q4k_gemm_dequantised_ahead(rows, k, tok):
     """Few tokens over many rows: the scratch is written by the dequantisation kernel ahead of the GEMM."""
