@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) expert_stream_kernel(const 
 
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
-      mbar_init(&full[s], 1);
+      mbar_init(&full[s], kProducerWarps);
       mbar_init(&empty[s], kTeamWarps);
     }
     fence_barrier_init();
@@ -946,6 +946,10 @@ __global__ void __launch_bounds__(kStreamThreads, 1) expert_stream_kernel(const 
           }
         }
       }
+      // (every producer warp counts in, also one that had nothing to copy: otherwise the stages could go round twice while it waits for its
+      // item's pointers, and the phase that it waits for next would not come)
+      __syncwarp();
+      if (lane == 0 && pw > 0) mbar_arrive_one(&full[s]);
     }
     return;
   }
