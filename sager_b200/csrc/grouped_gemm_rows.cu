@@ -405,7 +405,8 @@ __global__ void __launch_bounds__(kThreads, 1) grouped_gemm_rows_kernel(const Ro
       } else if (nt <= 4) {
         const unsigned char* xs = st + kWBytes;
         const uint4 h0 = *reinterpret_cast<const uint4*>(st + own_lo), h1 = *reinterpret_cast<const uint4*>(st + own_hi);
-        warp_mma_block4(st + w_off, h0, h1, b_row4(xs + kXCodes, kXRow, zeros, lane), lane, loaded,
+        const unsigned char* b_row = b_row4(xs + kXCodes, kXRow, zeros, lane);
+        warp_mma_block4(st + w_off, h0, h1, [&](int g) { return b_row + g * 64; }, lane, loaded,
                         [&] { return *reinterpret_cast<const uint32_t*>(xs + (gid >> 1) * kXRow + kXSums + (tig & 1) * 8 + (gid & 1) * 4); },
                         [&](int r, int isum, int msum) {
                           const uint32_t dm = r ? h1.x : h0.x;

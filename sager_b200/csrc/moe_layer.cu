@@ -50,8 +50,8 @@ constexpr int kMaxGrid = 160;            // most CTAs the expert kernels are lau
 constexpr int kAheadStages = 3;          // stages of published groups that the row-streaming kernel's weight warp is kept ahead with
 constexpr int kTmapSlots = kAheadStages + 7;      // patched TMA descriptor pairs per CTA of that kernel
 // Layers of up to this many token rows run as one persistent launch: all that its row sets hold (us per layer at 1 / 2 /
-// 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 15.7 / 22.1 / 29.7 / 36.4, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
-// 128 experts, hidden 1024: 13.6 / 17.9 / 20.3 / 22.6 against 23.6 / 25.7 / 31.3 / 29.6).
+// 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 13.8 / 20.8 / 24.4 / 27.2, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
+// 128 experts, hidden 1024: 12.3 / 17.6 / 19.9 / 22.1 against 23.6 / 25.7 / 31.3 / 29.6).
 constexpr int kTokenKernelMaxRows = 4;
 // Layers of at least this many token rows have the row-streaming kernel's order of the sums (block after block), and of the
 // two expert kernels run that one (us per layer with the route kernel, 256 experts: 37.7 against 46.5 for the item kernel at
@@ -1202,15 +1202,16 @@ int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const
 template <bool STREAM>
 int launch_token_layer(const tk::Geom& g, cudaStream_t s, const LayerDev& L) {
   const dim3 grid(L.grid);
-  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  if (g.part_bytes > 0) return launch_layer<tk::token_layer_kernel<true, false, false, true, STREAM>>(grid, tk::kThreads, g.total, s, L);
   // sharing by cost: two rows seldom meet in a tile (22.9 us a layer either way), and where a pass of both groups takes a CTA's
   // pairs there is nothing to share out
   const bool by_cost = L.n > 2 && static_cast<long long>(L.n) * L.K * L.FF > 2LL * L.grid * g.stage_pairs;
   if (L.n < kRowsKernelMinRows)
-    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true, STREAM>>(grid, tk::kThreads, g.total, s, L)
-                   : launch_layer<tk::token_layer_kernel<false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
-  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true, STREAM>>(grid, tk::kThreads, g.total, s, L)
-                 : launch_layer<tk::token_layer_kernel<true, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                   : launch_layer<tk::token_layer_kernel<false, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                 : launch_layer<tk::token_layer_kernel<true, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
 }
 
 }  // namespace
@@ -1460,7 +1461,9 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
       a->ep_dst == nullptr && a->ep_out == nullptr &&
       L.e_lo == 0 && L.e_hi == L.E && L.sh_lo == 0 && L.sh_hi == L.n && L.nbh <= 16 && L.nbf <= 16 &&
       a->workspace_bytes >= lay.items_total) {
-    const tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid);
+    // the MMA kernel where its shared memory fits too
+    tk::Geom g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid, tk::use_mma(L.n, L.K, L.H, L.FF, L.grid));
+    if (g.total > 227 * 1024) g = tk::geom(L.n, L.K, L.H, L.FF, L.E, L.grid, false);
     if (g.total <= 227 * 1024 && g.down_tiles > 0 && g.rows_per_cta <= tk::kGroupWarps)
       return stream_weights ? launch_token_layer<true>(g, s, L) : launch_token_layer<false>(g, s, L);
   }

@@ -389,11 +389,11 @@ __device__ __forceinline__ void warp_mma_block(const unsigned char* a_ptr, const
 // both, and a lane scales the results of one token - half the multiply-adds, conversions and fp32 steps, which for eight
 // columns are spent on tokens that are not there (prefill of 96 rows over 256 experts, four layers: 512 -> 504 us; in the decode
 // layer's row-streaming kernel the tiles gain as much, but the larger kernel costs every layer 0.8 to 1.2 us more). Results: rows gid and gid + 8, token tig.
-//   b_ptr   this lane's ldmatrix row (b_row4), advanced by 64 bytes per pair of sub-blocks
+//   b_at(g) this lane's ldmatrix row of sub-blocks 2g and 2g + 1 (b_row4 + 64 g where a row's codes follow one another)
 //   min_b   sub-block sums 4 (tig & 1) .. + 3 of token gid / 2: their low parts in even gid, high parts (bsum = 128 hi + lo) in odd
 //   fold(row, isum, msum): the fp32 steps; isum is sixteen-fold
-template <typename Loaded, typename MinB, typename Fold>
-__device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, const uint4& h0, const uint4& h1, const unsigned char* b_ptr,
+template <typename BAt, typename Loaded, typename MinB, typename Fold>
+__device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, const uint4& h0, const uint4& h1, BAt b_at,
                                                 int lane, Loaded loaded, MinB min_b, Fold fold) {
   const int tig = lane & 3;
   uint32_t raw[4][4];
@@ -406,7 +406,7 @@ __device__ __forceinline__ void warp_mma_block4(const unsigned char* a_ptr, cons
 #pragma unroll
   for (int g = 0; g < 4; ++g) {
     uint32_t b[4], lo[4], hi[4];
-    ldmatrix_x4(b, b_ptr + g * 64);
+    ldmatrix_x4(b, b_at(g));
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       lo[j] = raw[g][j] & 0x0F0F0F0Fu;

@@ -19,18 +19,19 @@
 //            then issues the weight copies (TMA): the CTA's pairs of the routed gate / up
 //            rows through a ring AND its rows of the down matrices, so the down weights
 //            arrive while gate / up computes
-//   phase 3  gate / up dots (dp4a, integer sub-block dots exact), SwiGLU, fp32 h rows to
-//            global memory, grid barrier; the first down weights go into registers meanwhile
+//   phase 3  gate / up dots (dp4a or the int8 MMA, integer sub-block dots exact), SwiGLU, fp32 h rows to
+//            global memory, grid barrier; with dp4a the first down weights go into registers meanwhile
 //   phase 4  every CTA quantises the h rows it needs (all of them: a few KB from L2),
 //            runs the down dots for its H / grid output rows of EVERY tile, and - since
 //            all of a row's expert contributions are then in this CTA - adds
 //            residual + sum_k w_k * y_k + shared in place. No third barrier.
 //
-// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 15.7 us per
+// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 13.8 us per
 // layer, of which 3.5 to the first barrier, 2 for picks and tables, 1.5 for the first bytes, 2 for
-// gate / up, 2 for the second barrier, 1 + 1 for h and the down rows; 26.6 with eight warps on whole
-// blocks and the selection in sequence). A further row costs 6 us - 22.6 / 29.2 / 33.6 us at 2 / 3 / 4 rows -,
-// where its bytes cost 2.2: the dots' instructions of a tile grow with its rows.
+// gate / up, 2 for the second barrier, 1 + 1 for h and the down rows; 15.1 with the loops over rows of larger layers, whose live
+// values were spilled, 26.6 with eight warps on whole
+// blocks and the selection in sequence). A further row costs 3 to 6 us - 20.8 / 24.4 / 27.2 us at 2 / 3 / 4 rows, by dp4a
+// 21.7 / 28.3 / 32.7 -, where its bytes cost 2.2: of the 27.2, gate / up terms take 2.9, down terms 3.3, h in every CTA 2.3.
 //
 // Work split: gate / up by pairs (a flat range of (tile, pair) per CTA, of equal cost), down by output
 // rows. Contracts are those of the two-launch path: null table entry = absent expert
@@ -63,6 +64,30 @@ struct HTile {
   __device__ __forceinline__ unsigned char* blk(int row, int b) const { return p + static_cast<size_t>(row * nb + b) * kHBlk; }
 };
 
+// One super-block of sixteen weight rows against up to four of the rows above (warp_mma_block4): term(r, v) with the block term of
+// fragment row gid (r = 0) and gid + 8 and of token tig, before the token's scale. `row` and `row_m` are the blocks of tokens
+// (lane & 7) / 2 and gid / 2 (any where there is no such token).
+template <typename Loaded, typename Term>
+__device__ __forceinline__ void mma_terms(const unsigned char* a_ptr, const unsigned char* own0, const unsigned char* own1, const unsigned char* row,
+                                          const unsigned char* row_m, const unsigned char* zeros, int lane, Loaded loaded, Term term) {
+  const uint4 h0 = *reinterpret_cast<const uint4*>(own0), h1 = *reinterpret_cast<const uint4*>(own1);
+  const bool codes = (lane & 1) == (lane >> 4);
+  const unsigned char* b0 = codes ? row + (lane >> 3) * 16 : zeros;
+  const int step = codes ? 64 : 0, half = codes ? kHalf : 0;
+  warp_mma_block4(a_ptr, h0, h1, [&](int g) { return b0 + (g >> 1) * half + (g & 1) * step; }, lane, loaded,
+                  [&] {
+                    const uint2 sv = *reinterpret_cast<const uint2*>(row_m + (lane & 1) * kHalf + 128);
+                    const int high = (lane >> 2) & 1;                 // bsum = 128 * high + low
+                    const uint32_t mask = high ? 0x00FF00FFu : 0x007F007Fu;
+                    return __byte_perm((sv.x >> (7 * high)) & mask, (sv.y >> (7 * high)) & mask, 0x6420);
+                  },
+                  [&](int r, int isum, int msum) {
+                    const uint32_t dm = r ? h1.x : h0.x;
+                    const float d = 0.0625f * h2f(static_cast<uint16_t>(dm & 0xFFFFu)), dmin = h2f(static_cast<uint16_t>(dm >> 16));
+                    term(r, d * static_cast<float>(isum) - dmin * static_cast<float>(msum));
+                  });
+}
+
 struct Tables {                            // built after the selection, the same in every CTA
   int n_tiles;
   int n_hrows;
@@ -82,6 +107,17 @@ struct StageDesc {
   int tile, pair0, np, mode;
 };
 
+// Kernels on the MMA stage each matrix of a stage of `np` pairs as eight chunks of whole rows, 16 bytes apart, so that ldmatrix
+// finds its eight rows - one of every chunk - in different banks. (Each row by itself, 16 bytes apart: 32 to 128 copies a stage, which
+// cost the narrow rows of hidden 1024 3 us a layer.)
+constexpr int kChunkPad = 8 * 16;
+struct Chunks {
+  int rows, step;        // rows to a chunk; bytes from one to the next
+  __device__ __forceinline__ Chunks(int np, int rb) : rows((np + 7) >> 3), step(rows * rb + 16) {}
+  __device__ __forceinline__ int matrix() const { return 8 * step; }                                        // bytes from gate to up
+  __device__ __forceinline__ int rows_of(int chunk, int np) const { return max(0, min(rows, np - chunk * rows)); }
+};
+
 struct Geom {
   int rows_per_cta;      // router rows per CTA
   int nr_max;            // output rows per CTA (down split)
@@ -89,8 +125,9 @@ struct Geom {
   int rb_h, rb_f;        // bytes per gate/up row, per down row
   size_t off_prob, off_ptab, off_xh, off_rw, off_xt, off_sh, off_ring, off_dn, off_y, total;
   int stage_pairs, stage_bytes, slot_bytes, down_tiles;
+  int part_bytes;        // a stage's block terms: [block][pair][token][gate, up] floats
 };
-__host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int grid) {
+__host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int grid, bool mma) {
   Geom g;
   g.rows_per_cta = (E + grid - 1) / grid;
   g.nr_max = (H + grid - 1) / grid;
@@ -98,22 +135,24 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
   g.rb_h = (H / kQK) * kW4;
   g.rb_f = (FF / kQK) * kW4;
   const int hrows = n * (K + 1);                            // (tile, row) pairs at most
+  // as many pairs as a group of warps takes at once (narrow rows take few lanes each)
+  const int nbh = H / kQK;
+  const int lanes = nbh <= 1 ? 2 : (nbh <= 2 ? 4 : (nbh <= 4 ? 8 : (nbh <= 8 ? 16 : 32)));
+  g.stage_pairs = kGroupThreads / lanes > kPairsStage ? kGroupThreads / lanes : kPairsStage;
+  g.part_bytes = mma ? nbh * g.stage_pairs * 2 * kMaxTok * 4 : 0;
   size_t p = kHdr + kTables;
   auto take = [&](size_t bytes) { const size_t at = p; p = (p + bytes + 127) & ~static_cast<size_t>(127); return at; };
   g.off_prob = take(static_cast<size_t>(n) * ((E + 3) & ~3) * 4);                // rows at 16-byte steps
   g.off_ptab = take(static_cast<size_t>(3) * E * 8);        // the layer's pointer table, read once per CTA
   // x rows as fp16 and the router rows; later the same bytes hold the quantised h rows
   const size_t a = static_cast<size_t>(n) * H * 2 + 128 + static_cast<size_t>(g.rows_per_cta) * H * 4;
-  const size_t b = static_cast<size_t>(hrows) * (FF / kQK) * kHBlk;
-  g.off_xh = take(a > b ? a : b);
+  // (on the MMA: and in between the block terms of gate / up, of two stages of each group)
+  const size_t b = static_cast<size_t>(hrows) * (FF / kQK) * kHBlk, c = static_cast<size_t>(4) * g.part_bytes;
+  g.off_xh = take(a > b ? (a > c ? a : c) : (b > c ? b : c));
   g.off_rw = g.off_xh + ((static_cast<size_t>(n) * H * 2 + 127) & ~static_cast<size_t>(127));
   g.off_xt = take(static_cast<size_t>(n) * (H / kQK) * kHBlk);
   g.off_sh = take(static_cast<size_t>(2) * g.sp_max * g.rb_h);
-  // as many pairs as a group of warps takes at once (narrow rows take few lanes each)
-  const int nbh = H / kQK;
-  const int lanes = nbh <= 1 ? 2 : (nbh <= 2 ? 4 : (nbh <= 4 ? 8 : (nbh <= 8 ? 16 : 32)));
-  g.stage_pairs = kGroupThreads / lanes > kPairsStage ? kGroupThreads / lanes : kPairsStage;
-  g.stage_bytes = 2 * g.stage_pairs * g.rb_h;
+  g.stage_bytes = 2 * (g.stage_pairs * g.rb_h + (mma ? kChunkPad : 0));
   g.off_ring = take(static_cast<size_t>(kRing) * g.stage_bytes);
   g.slot_bytes = g.nr_max * g.rb_f;
   const int in_ring = kRing * g.stage_bytes / (g.slot_bytes > 0 ? g.slot_bytes : 1);
@@ -124,9 +163,19 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
   return g;
 }
 
+// Whether a layer of several rows runs its routed tiles on the int8 MMA. It costs a barrier and a sum per stage, which pay when a CTA's
+// pairs take more than one pass of both groups, and a row of few blocks leaves little to gain: us per layer, dp4a / MMA,
+//   2048 / 512 / 256 experts / top-8 at 2 / 3 / 4 rows (1.7 / 2.6 / 3.5 passes) 21.8 / 28.3 / 32.7, 20.8 / 24.4 / 27.2
+//   2048 / 256 / 64 / 8 (0.9 / 1.3 / 1.7) 16.5 / 18.9 / 21.0, 17.2 / 18.7 / 19.8
+//   1024 / 512 / 128 / 8 (0.9 / 1.3 / 1.7) 17.8 / 20.0 / 22.1, 19.0 / 21.1 / 22.7
+//   512 / 256 / 16 / 4 (0.1 / 0.2 / 0.2) 13.2 / 14.0 / 15.1, 13.6 / 14.0 / 14.7.
+inline bool use_mma(int n, int K, int H, int FF, int grid) {
+  return n > 1 && H / kQK > 4 && static_cast<long long>(n) * K * FF > 2LL * grid * kPairsStage;
+}
+
 // Named barriers of the consumers: 6 all of them, 7 the warps with router rows, 5 the warps that quantise, 8 .. 11 the
 // two warps that select for a token row, 12 the warps that pick,
-// 13 the warp that picks the only row and the second group.
+// 13 the warp that picks the only row and the second group, 14 and 15 each group.
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void consumers_sync() {
   asm volatile("bar.sync 6, %0;" ::"n"(kConsumers) : "memory");
@@ -187,25 +236,30 @@ __device__ __forceinline__ void quantize_to_tile(unsigned char* blk, const float
   if ((lane & 15) == 0) *reinterpret_cast<float*>(half + 136) = d;
 }
 
-// `rows` fp32 rows of h (global memory, FF values each) into a tile, a warp per 256-value block, two blocks' loads
-// in flight per warp.
+// `rows` fp32 rows of h (global memory, FF values each) into a tile, a warp per 256-value block, D blocks' loads
+// in flight per warp: every round of them is a trip to L2 (four rows have 72 blocks, 4.5 a warp: two at a time took 3.2 us, all at
+// once 2.3).
+// (every CTA reads the same few KB: a load too many is 148 more requests to the same L2 lines)
+template <int D>
 __device__ __forceinline__ void quantize_h_rows(const HTile& xt, int rows, const float* src, int warp, int lane) {
-  // (every CTA reads the same few KB: a load too many is 148 more requests to the same L2 lines)
   const int jobs = rows * xt.nb;                   // blocks lie one after another in both places
-  for (int j0 = warp; j0 < jobs; j0 += 2 * kWarps) {
+  for (int j0 = warp; j0 < jobs; j0 += D * kWarps) {
     const float4* p = reinterpret_cast<const float4*>(src + static_cast<size_t>(j0) * kQK) + lane * 2;
-    float4 x = __ldcg(p), y = __ldcg(p + 1), x2, y2;
-    const bool two = j0 + kWarps < jobs;           // warp-uniform
-    if (two) {
-      x2 = __ldcg(p + kWarps * (kQK / 4));
-      y2 = __ldcg(p + kWarps * (kQK / 4) + 1);
-    }
-    const float v[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-    quantize_to_tile(xt.blk(0, j0), v, lane);
-    if (two) {
-      const float v2[8] = {x2.x, x2.y, x2.z, x2.w, y2.x, y2.y, y2.z, y2.w};
-      quantize_to_tile(xt.blk(0, j0 + kWarps), v2, lane);
-    }
+    float4 x[D][2];
+    x[0][0] = __ldcg(p);
+    x[0][1] = __ldcg(p + 1);
+#pragma unroll
+    for (int d = 1; d < D; ++d)
+      if (j0 + d * kWarps < jobs) {                // warp-uniform
+        x[d][0] = __ldcg(p + d * kWarps * (kQK / 4));
+        x[d][1] = __ldcg(p + d * kWarps * (kQK / 4) + 1);
+      }
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+      if (d == 0 || j0 + d * kWarps < jobs) {
+        const float v[8] = {x[d][0].x, x[d][0].y, x[d][0].z, x[d][0].w, x[d][1].x, x[d][1].y, x[d][1].z, x[d][1].w};
+        quantize_to_tile(xt.blk(0, j0 + d * kWarps), v, lane);
+      }
   }
 }
 
@@ -324,12 +378,12 @@ __device__ __forceinline__ float reduce_pairs(float v, int lpr) {
 // (Inlined at both of its uses: as a function it saved and restored 2,400 warp registers per CTA through local memory.)
 // A warp arrives at `empty` (if given) as soon as its weight bytes are in registers: the stage's refill, a DRAM round
 // trip, then runs under the arithmetic. Warps without a pair only arrive.
-template <bool CHAIN>
+template <bool CHAIN, bool ONE>
 __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, int mask, int hrow0, int pair0,
                                            const HTile& xt, float* hbuf, int FF, int nbh, int rb_h, int row_lanes, uint64_t* empty) {
   const int tid = threadIdx.x & (kGroupThreads - 1), lane = tid & 31;
   const int lpr = 1 << (row_lanes - 1);
-  const RowSet rs = rows_of(mask, 0, true);
+  const RowSet rs = ONE ? RowSet{0, 0, 0, 0, 1} : rows_of(mask, 0, true);
   const int tasks = np << row_lanes;
   if ((tid & ~31) >= tasks) {
     if (empty != nullptr && lane == 0) mbar_arrive_one(empty);
@@ -359,6 +413,54 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
   }
 }
 
+// The same for layers of several rows, on the int8 MMA: a warp takes eight pairs and one block column at a time - gate rows and the
+// up rows of the same indices are the sixteen rows of a fragment -, the terms of a row's blocks meet in `part` and are added
+// block after block. A tile of four rows costs what a tile of one does; by dp4a 16 pairs took 0.25 us and 1.2 more per row of
+// the tile, and the CTAs whose tile four rows share finished 8 us after the median one, or took fewer pairs.
+// `st` holds chunks of rows of `rb` bytes; a barrier of the group lies between the two functions.
+__device__ __forceinline__ void gate_up_terms(const unsigned char* st, int np, const RowSet& rs, const HTile& xt, int nbh, int rb, float* part,
+                                              int part_pairs, const unsigned char* zeros, uint64_t* empty) {
+  const int tid = threadIdx.x & (kGroupThreads - 1), lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+  const int row = rs.at(min((lane & 7) >> 1, rs.n - 1)), row_m = rs.at(min(gid >> 1, rs.n - 1));
+  const Chunks ch(np, rb);
+  const int tasks = ch.rows * nbh;
+  int task = tid >> 5;
+  if (task >= tasks && lane == 0) mbar_arrive_one(empty);
+#pragma unroll 1
+  for (; task < tasks; task += kGroupWarps) {
+    const int q = task / nbh, b = task - q * nbh;          // row q of every chunk, block column b
+    const unsigned char* col = st + b * kW4 + q * rb;
+    auto chunk = [&](int i) { return (i * ch.rows + q < np ? i : 0) * ch.step; };
+    // matrices of a weight load: gate rows, up rows of k 0-15, then of k 16-31 of a sub-block
+    const unsigned char* a_ptr = col + chunk(lane & 7) + ((lane >> 3) & 1) * ch.matrix() + 16 + (lane >> 4) * 16;
+    const unsigned char* own = col + chunk(gid);
+    float v[2];
+    mma_terms(a_ptr, own, own + ch.matrix(), xt.blk(row, b), xt.blk(row_m, b), zeros, lane,
+              [&] {
+                if (task + kGroupWarps >= tasks) {                     // this warp's last weight bytes are in registers
+                  __syncwarp();
+                  if (lane == 0) mbar_arrive_one(empty);
+                }
+              },
+              [&](int r, float t) { v[r] = t; });
+    *reinterpret_cast<float2*>(part + ((b * part_pairs + gid * ch.rows + q) * kMaxTok + tig) * 2) = make_float2(v[0], v[1]);
+  }
+}
+__device__ __forceinline__ void gate_up_sums(const float* part, int part_pairs, int np, const RowSet& rs, int hrow0, int pair0, const HTile& xt,
+                                             float* hbuf, int FF, int nbh) {
+  const int tid = threadIdx.x & (kGroupThreads - 1);
+#pragma unroll 1
+  for (int i = tid; (i & ~31) < np * 2 * kMaxTok; i += kGroupThreads) {        // (pair, token, matrix)
+    const int t = (i >> 1) & (kMaxTok - 1), pair = i >> 3;
+    const unsigned char* x = xt.blk(rs.at(min(t, rs.n - 1)), 0) + 136;
+    float v = 0.f;
+#pragma unroll 4
+    for (int b = 0; b < nbh; ++b) v = fmaf(*reinterpret_cast<const float*>(x + b * kHBlk), part[(b * part_pairs) * 2 * kMaxTok + i], v);
+    const float u = __shfl_down_sync(0xFFFFFFFFu, v, 1);
+    if ((i & 1) == 0 && pair < np && t < rs.n) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(v, u);
+  }
+}
+
 // Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned; plain_done() ends a row of them. (Not
 // inlined at its six rarely taken uses: straight-line code beside them is paid for in instruction fetch, 0.4 us a layer.)
 static __device__ __noinline__ void copy_plain(unsigned char* dst, const unsigned char* src, int bytes, int lane) {
@@ -371,11 +473,12 @@ __device__ __forceinline__ void plain_done() {
 
 // CHAIN: layers of four token rows (see half_dots). ONE: layers of one, which are a chain of short steps: what only more rows
 // need is neither executed nor fetched. BY_COST: layers whose CTAs take more pairs than a pass of both groups (see routed_share).
-// STREAM: weights first to leave L2 (streams_weights).
-template <bool CHAIN, bool ONE, bool BY_COST, bool STREAM>
+// MMA: routed tiles on the int8 MMA (see use_mma). STREAM: weights first to leave L2 (streams_weights).
+template <bool CHAIN, bool ONE, bool BY_COST, bool MMA, bool STREAM>
 __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
-  const Geom G = geom(ONE ? 1 : L.n, L.K, L.H, L.FF, L.E, gridDim.x);
+  static_assert(!MMA || (CHAIN && !ONE && !BY_COST), "tiles on the MMA cost the same whatever their rows");
+  const Geom G = geom(ONE ? 1 : L.n, L.K, L.H, L.FF, L.E, gridDim.x, MMA);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);              // [kRing]
   uint64_t* empty = full + kRing;                                  // [kRing]
   uint64_t* sh_full = empty + kRing;                               // shared expert's gate / up pairs
@@ -387,6 +490,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   uint64_t* passed = based + 1;                                    // grid barrier passed (or given up), one phase each
   StageDesc* desc = reinterpret_cast<StageDesc*>(smem + 128);      // [kRing]
   int* flag = reinterpret_cast<int*>(smem + 256);
+  unsigned char* zeros = smem + 512;                               // (MMA) sixteen bytes
   Tables& tb = *reinterpret_cast<Tables*>(smem + kHdr);
   float* prob = reinterpret_cast<float*>(smem + G.off_prob);
   const unsigned char** ptab = reinterpret_cast<const unsigned char**>(smem + G.off_ptab);   // [3][E]
@@ -441,6 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   const int nr = r1 - r0;
 
   const bool by_pairs = E <= 256 && K < 32;      // warps t and t + 4 select for row t, otherwise warp t
+  if (MMA && tid >= 32 && tid < 36) reinterpret_cast<uint32_t*>(zeros)[tid - 32] = 0u;
   if (tid == 0) {
     for (int s = 0; s < kRing; ++s) {
       mbar_init(&full[s], 1);
@@ -579,12 +684,29 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         desc[s] = d;
       }
       if (mode == 2) {
-        copy_plain(st, tb.w[0][tile] + static_cast<size_t>(pair0) * G.rb_h, np * G.rb_h, lane);
-        copy_plain(st + static_cast<size_t>(np) * G.rb_h, tb.w[1][tile] + static_cast<size_t>(pair0) * G.rb_h, np * G.rb_h, lane);
+        if (!MMA) {
+          copy_plain(st, tb.w[0][tile] + static_cast<size_t>(pair0) * G.rb_h, np * G.rb_h, lane);
+          copy_plain(st + static_cast<size_t>(np) * G.rb_h, tb.w[1][tile] + static_cast<size_t>(pair0) * G.rb_h, np * G.rb_h, lane);
+        } else {
+          const Chunks ch(np, G.rb_h);
+          for (int i = 0; i < 16; ++i)
+            copy_plain(st + i * ch.step, tb.w[i >> 3][tile] + static_cast<size_t>(pair0 + (i & 7) * ch.rows) * G.rb_h, ch.rows_of(i & 7, np) * G.rb_h, lane);
+        }
         plain_done();
       }
       __syncwarp();
-      if (lane == 0) {
+      if (MMA) {                                    // a lane per chunk
+        if (lane == 0) {
+          if (mode == 0) mbar_expect_tx(&full[s], static_cast<uint32_t>(2 * np * G.rb_h));
+          else mbar_arrive_one(&full[s]);
+        }
+        __syncwarp();
+        const Chunks ch(np, G.rb_h);
+        const int rows = ch.rows_of(lane & 7, np);
+        if (mode == 0 && lane < 16 && rows > 0)
+          bulk_g2s_weights<STREAM>(st + lane * ch.step, tb.w[lane >> 3][tile] + static_cast<size_t>(pair0 + (lane & 7) * ch.rows) * G.rb_h,
+                                   static_cast<uint32_t>(rows * G.rb_h), &full[s]);
+      } else if (lane == 0) {
         if (mode == 0) {
           mbar_expect_tx(&full[s], static_cast<uint32_t>(2 * np * G.rb_h));
           bulk_g2s_weights<STREAM>(st, tb.w[0][tile] + static_cast<size_t>(pair0) * G.rb_h, static_cast<uint32_t>(np * G.rb_h), &full[s]);
@@ -707,7 +829,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     if (warp >= kGroupWarps && has_shared && sp1 > sp0) {
       if (!mbar_wait(sh_full, 0)) ok = false;
       if (__all_sync(0xFFFFFFFFu, ok))
-        gate_up_stage<CHAIN>(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, nullptr);
+        gate_up_stage<CHAIN, ONE>(sh_stage, sp1 - sp0, (1 << n) - 1, 0, sp0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, nullptr);
     }
   }
 
@@ -845,18 +967,34 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     const int group = warp / kGroupWarps;
     int pair0 = pos % FF;
     const int cut = min(G.stage_pairs, (pb - pos + 1) / 2);
-    for (int i = 0; pos < pb && ok; ++i) {
+    // (where x and the router rows were; two stages' terms per group, so that one barrier a stage is enough)
+    float* part = reinterpret_cast<float*>(smem + G.off_xh) + group * (G.part_bytes / 2);
+    for (int i = 0; pos < pb && (MMA || ok); ++i) {
       const int s = i % kRing, np = min(cut, min(FF - pair0, pb - pos));    // as the producer cuts the range
       pos += np;
       pair0 = pair0 + np == FF ? 0 : pair0 + np;
       if ((i & 1) != group) continue;
-      ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], (i / kRing) & 1)) != 0;
-      if (!ok) break;
-      const StageDesc d = desc[s];
-      if (d.mode != 1)
-        gate_up_stage<CHAIN>(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
-                      d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, &empty[s]);
-      else if (lane == 0) mbar_arrive_one(&empty[s]);
+      if constexpr (!MMA) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], (i / kRing) & 1)) != 0;
+        if (!ok) break;
+        const StageDesc d = desc[s];
+        if (d.mode != 1)
+          gate_up_stage<CHAIN, ONE>(ring + static_cast<size_t>(s) * G.stage_bytes, d.np, tb.tile_mask[d.tile], tb.tile_hrow0[d.tile],
+                        d.pair0, xt, L.hbuf, FF, L.nbh, G.rb_h, row_lanes, &empty[s]);
+        else if (lane == 0) mbar_arrive_one(&empty[s]);
+      } else {
+        // (whole groups: a warp whose wait ran out goes on to the barriers)
+        if (ok) ok = __all_sync(0xFFFFFFFFu, mbar_wait(&full[s], (i / kRing) & 1)) != 0;
+        const StageDesc d = desc[s];
+        const bool work = ok && d.mode != 1;
+        if (ok && !work && lane == 0) mbar_arrive_one(&empty[s]);
+        const unsigned char* st = ring + static_cast<size_t>(s) * G.stage_bytes;
+        float* terms = part + ((i >> 1) & 1) * (G.part_bytes / 4);
+        const RowSet rs = rows_of(work ? tb.tile_mask[d.tile] : 1, 0, true);
+        if (work) gate_up_terms(st, d.np, rs, xt, L.nbh, G.rb_h, terms, G.stage_pairs, zeros, &empty[s]);
+        named_sync(14 + group, kGroupThreads);
+        if (work) gate_up_sums(terms, G.stage_pairs, d.np, rs, tb.tile_hrow0[d.tile], d.pair0, xt, L.hbuf, FF, L.nbh);
+      }
     }
   }
   ok = consumers_all(ok);                                   // (a wait that ran out in any thread ends the CTA's work)
@@ -880,42 +1018,76 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     if (rd == 0 && has_shared && !mbar_wait(shdn_full, 0)) ok = false;
     if (ok && !mbar_wait(&dn_full[rd & 1], (rd >> 1) & 1)) ok = false;
     ok = __all_sync(0xFFFFFFFFu, ok) != 0;
-    const int tasks = (j1 - j0) * nr << f_lanes;
-    int base = 0;
-#pragma unroll 1
-    do {
-      // a task's weights go into registers first, at the first task while the other CTAs finish their gate / up
-      const int q = base + tid;
-      const int jr = q >> f_lanes;
-      const int js = jr / max(nr, 1), r = jr - js * nr;
-      const int tile = min(j0 + js, T - 1);
-      const bool live = q < tasks && tb.tile_mode[tile] != 1;
-      const int hrow0 = tb.tile_hrow0[tile];
-      const RowSet rs = rows_of(live ? tb.tile_mask[tile] : 0, live ? hrow0 : 0, false);   // h rows are stored per tile
-      const int rows = __reduce_max_sync(0xFFFFFFFFu, rs.n);
-      const unsigned char* const w[1] = {from + (live ? js * G.slot_bytes + r * G.rb_f + f_blk * kW4 : 0)};
-      HalfW<1> W;
-      load_half<1>(W, w, f_half);
-      if (first) {
-        first = false;
+    if constexpr (MMA) {
+      if (rd == 0) {
         const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
-        quantize_h_rows(hq, tb.n_hrows, L.hbuf, warp, lane);
+        quantize_h_rows<5>(hq, tb.n_hrows, L.hbuf, warp, lane);
         if (!consumers_all(met && ok)) {
           if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
           return;
         }
       }
-      float v[kMaxTok];
-      half_dots<1, CHAIN>(W, f_half, hq, f_blk, f_lr, L.nbf, rs, rows, v);
-      const int at = CHAIN ? L.nbf - 1 : 0;
-#pragma unroll
-      for (int t = 0; t < kMaxTok; ++t) {
-        if (t >= rows) break;                    // warp-uniform
-        const float y = CHAIN ? v[t] : reduce_pairs(f_lr < L.nbf ? v[t] : 0.f, lpf);
-        if (live && f_half == 0 && f_lr == at && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
+      const int gid = lane >> 2, tig = lane & 3;
+#pragma unroll 1
+      for (int j = ok ? j0 + warp : j1; j < j1; j += kWarps) {         // a warp per tile, sixteen output rows at a time
+        if (tb.tile_mode[j] == 1) continue;
+        const int hrow0 = tb.tile_hrow0[j], rows = __popc(tb.tile_mask[j]);
+        const int row = hrow0 + min((lane & 7) >> 1, rows - 1), row_m = hrow0 + min(gid >> 1, rows - 1), row_t = hrow0 + min(tig, rows - 1);
+#pragma unroll 1
+        for (int m0 = 0; m0 < nr; m0 += 16) {
+          const unsigned char* w = from + static_cast<size_t>(j - j0) * G.slot_bytes;
+          const int ra = min(m0 + (lane & 15), nr - 1), q0 = m0 + gid, q1 = q0 + 8;
+          float acc[2] = {0.f, 0.f};
+#pragma unroll 1
+          for (int b = 0; b < L.nbf; ++b, w += kW4) {
+            const float xd = *reinterpret_cast<const float*>(hq.blk(row_t, b) + 136);
+            mma_terms(w + ra * G.rb_f + 16 + (lane >> 4) * 16, w + min(q0, nr - 1) * G.rb_f, w + min(q1, nr - 1) * G.rb_f, hq.blk(row, b), hq.blk(row_m, b),
+                      zeros, lane, [] {}, [&](int r, float v) { acc[r] = fmaf(xd, v, acc[r]); });
+          }
+          if (tig < rows) {
+            if (q0 < nr) ysm[(hrow0 + tig) * G.nr_max + q0] = acc[0];
+            if (q1 < nr) ysm[(hrow0 + tig) * G.nr_max + q1] = acc[1];
+          }
+        }
       }
-      base += kConsumers;
-    } while (base < tasks && ok);
+    } else {
+      const int tasks = (j1 - j0) * nr << f_lanes;
+      int base = 0;
+#pragma unroll 1
+      do {
+        // a task's weights go into registers first, at the first task while the other CTAs finish their gate / up
+        const int q = base + tid;
+        const int jr = q >> f_lanes;
+        const int js = jr / max(nr, 1), r = jr - js * nr;
+        const int tile = min(j0 + js, T - 1);
+        const bool live = q < tasks && tb.tile_mode[tile] != 1;
+        const int hrow0 = tb.tile_hrow0[tile];
+        const RowSet rs = ONE ? RowSet{live ? hrow0 : 0, 0, 0, 0, 1} : rows_of(live ? tb.tile_mask[tile] : 0, live ? hrow0 : 0, false);   // h rows are stored per tile
+        const int rows = ONE ? 1 : __reduce_max_sync(0xFFFFFFFFu, rs.n);
+        const unsigned char* const w[1] = {from + (live ? js * G.slot_bytes + r * G.rb_f + f_blk * kW4 : 0)};
+        HalfW<1> W;
+        load_half<1>(W, w, f_half);
+        if (first) {
+          first = false;
+          const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
+          quantize_h_rows<2>(hq, tb.n_hrows, L.hbuf, warp, lane);
+          if (!consumers_all(met && ok)) {
+            if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
+            return;
+          }
+        }
+        float v[kMaxTok];
+        half_dots<1, CHAIN>(W, f_half, hq, f_blk, f_lr, L.nbf, rs, rows, v);
+        const int at = CHAIN ? L.nbf - 1 : 0;
+#pragma unroll
+        for (int t = 0; t < kMaxTok; ++t) {
+          if (t >= rows) break;                    // warp-uniform
+          const float y = CHAIN ? v[t] : reduce_pairs(f_lr < L.nbf ? v[t] : 0.f, lpf);
+          if (live && f_half == 0 && f_lr == at && t < rs.n) ysm[(hrow0 + t) * G.nr_max + r] = y;
+        }
+        base += kConsumers;
+      } while (base < tasks && ok);
+    }
     __syncwarp();
     if (lane == 0 && rd + 2 < rounds) mbar_arrive_one(&dn_empty[rd & 1]);
   }

@@ -574,6 +574,36 @@ def test_one_launch_layers_back_to_back_on_one_workspace(hidden, n_ff, E, k):
     assert lib().raw("sgr_status")(0) == 0
 
 
+@pytest.mark.parametrize("hidden,n_ff,E,k", [
+    (2048, 512, 256, 8),     # two rows of a stage to a chunk, the last stage of a CTA one or none
+    (1280, 1024, 48, 8),     # five block columns, eight tiles' down rows at a time, four blocks to a down row
+    (1536, 768, 40, 7),      # six and three
+    (2048, 256, 64, 8),      # two rows: the dp4a kernel and its order, three and four: the MMA's
+])
+def test_several_rows_on_the_mma(hidden, n_ff, E, k):
+    """Routed tiles on the int8 MMA: exact integer sums, the fp32 terms of a row's blocks one after the other, as in the
+    row-streaming kernel - the same bits. Tiles of one row to all, null experts, no shared one, weights off a 16-byte boundary."""
+    for shift in (0, 4):
+        w = synth.MoeWeights(hidden, n_ff, E, DEV, seed=95, std=0.05)
+        if shift:
+            big = torch.zeros(w.blob.numel() + 16, dtype=torch.uint8, device=DEV)
+            moved = big[shift:shift + w.blob.numel()]
+            moved.copy_(w.blob.view(-1))
+            w.blob = moved.view(w.blob.shape)
+        for n in (2, 3, 4):
+            on_mma = n * k * n_ff > 2 * 16 * torch.cuda.get_device_properties(0).multi_processor_count
+            for i, (absent, use_shared) in enumerate((((), True), ((0, E - 1), False))):
+                x16 = synth.normal_fp16((n, hidden), 960 + 10 * n + i, DEV)
+                x16[1:] = x16[0] + (0.05 if i else 0.4) * x16[1:]          # rows that pick much the same experts
+                r0, x0, o0 = run_layer(w, n, k, x16, absent=absent, use_shared=use_shared)
+                r1, x1, o1 = run_layer(w, n, k, x16, absent=absent, use_shared=use_shared, kernel="rows")
+                assert torch.equal(r0.route_idx, r1.route_idx)
+                if on_mma or n == 4:
+                    assert torch.equal(o0.view(torch.int32), o1.view(torch.int32)) and torch.equal(x0.view(torch.int16), x1.view(torch.int16))
+                else:
+                    assert rel(o0.cpu().numpy(), o1.cpu().numpy()) < 1e-5        # another order of the same fp32 terms
+
+
 def test_four_rows_on_a_workspace_for_the_item_kernel(full_w):
     """A workspace too small for the row-streaming kernel keeps four rows on the item kernel and its order of the sums."""
     x16 = synth.normal_fp16((4, full_w.hidden), 870, DEV)
