@@ -50,9 +50,10 @@ constexpr int kMaxGrid = 160;            // most CTAs the expert kernels are lau
 constexpr int kAheadStages = 3;          // stages of published groups that the row-streaming kernel's weight warp is kept ahead with
 constexpr int kTmapSlots = kAheadStages + 7;      // patched TMA descriptor pairs per CTA of that kernel
 // Layers of up to this many token rows run as one persistent launch: all that its row sets hold (us per layer at 1 / 2 /
-// 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 13.8 / 20.8 / 24.4 / 27.2, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
-// 128 experts, hidden 1024: 12.3 / 17.6 / 19.9 / 22.1 against 23.6 / 25.7 / 31.3 / 29.6).
+// 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 13.2 / 20.7 / 24.0 / 27.2, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
+// 128 experts, hidden 1024: 12.0 / 17.6 / 19.9 / 22.1 against 23.6 / 25.7 / 31.3 / 29.6).
 constexpr int kTokenKernelMaxRows = 4;
+constexpr int kXchgCopies = 16;        // of the logits that a one-launch layer's CTAs exchange (token_layer.cuh)
 // Layers of at least this many token rows have the row-streaming kernel's order of the sums (block after block), and of the
 // two expert kernels run that one (us per layer with the route kernel, 256 experts: 37.7 against 46.5 for the item kernel at
 // 4 rows, 50.3 against 66.7 at 8; at 1 row 29.4 against 26.9).
@@ -107,6 +108,7 @@ struct LayerDev {
   unsigned* tile_cnt;  // [2][max_tiles] item kernel: finished gate/up items per tile; row-streaming kernel: [tile][finisher
                        // warp] a bit per block of h whose first half is in global memory
   unsigned* ready;     // [max_tiles] row-streaming kernel: finisher warps done with a quantised block of h
+  unsigned long long* xchg;   // [kXchgCopies][n][E] one-launch layer: logits with the launch's number above them
   unsigned char* hq;   // [(n_max*K + n_max)][nbf] Q8_K rows of h, 288-byte blocks (row-streaming kernel)
   int tok_tile;        // token rows per tile: 8 (item kernel) or 16 (row-streaming kernel)
   unsigned char* xq16; // the quantised rows once more in 288-byte blocks (row-streaming kernel)
@@ -145,7 +147,7 @@ struct LayerDev {
 __host__ __device__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct WsLayout {
-  size_t xq, logits, off, rec, meta, gslot, grows, cnt, tile_cnt, ready, hbuf, ybuf, hq, xq16, tmaps, total;
+  size_t xq, logits, off, rec, meta, gslot, grows, cnt, tile_cnt, ready, xchg, hbuf, ybuf, hq, xq16, tmaps, total;
   size_t items_total;   // what the item kernel needs: everything up to and including ybuf
 };
 inline WsLayout ws_layout(int n_max, int H, int FF, int E, int K) {
@@ -164,6 +166,7 @@ inline WsLayout ws_layout(int n_max, int H, int FF, int E, int K) {
   l.cnt = take((16 + static_cast<size_t>(H) / 16 + 1) * 4);
   l.tile_cnt = take(tiles * 2 * 4);
   l.ready = take(tiles * 4);
+  l.xchg = take(static_cast<size_t>(kXchgCopies) * std::min(n_max, kTokenKernelMaxRows) * E * 8);
   l.hbuf = take(rows * FF * 4);
   l.ybuf = take(rows * H * 4);
   l.items_total = p;
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(kRouteWarps * 32) route_kernel(const LayerDev 
     int* idx = L.idx + static_cast<size_t>(tok0 + t) * L.rstride;
     float* w = L.w + static_cast<size_t>(tok0 + t) * L.rstride;
     if (t < nt && L.E <= 256 && L.K < 32) {
-      router_select_pair(lg, prob, pick_e[t], idx, w, 1 + t, warp >= kRouteTok, L.E, L.K, L.shared_w, lane, [] {});
+      router_select_pair([&](int j) { return __ldcg(lg + lane + 32 * j); }, prob, pick_e[t], idx, w, 1 + t, warp >= kRouteTok, L.E, L.K, L.shared_w, lane, [] {});
     } else if (t < nt && warp < kRouteTok) {
       for (int i = lane; i < L.E; i += 32) prob[i] = __ldcg(lg + i);
       __syncwarp();
@@ -1101,8 +1104,9 @@ __global__ void __launch_bounds__(kStreamThreads, 1) expert_stream_kernel(const 
 // Scratch of the allocation-free entry point (sgr_moe_layer_decode_static): the
 // same layout a caller-provided workspace has, held by every device that loads
 // the library until the process exits.
-constexpr size_t kStaticWsBytes = 2u << 20;
-static __device__ __align__(256) unsigned char g_static_ws[kStaticWsBytes];
+constexpr size_t kStaticWsBytes = 2u << 20;                      // beside the logits that a one-launch layer exchanges
+constexpr size_t kStaticXchgBytes = kXchgCopies * kTokenKernelMaxRows * 1024 * 8;
+static __device__ __align__(256) unsigned char g_static_ws[kStaticWsBytes + kStaticXchgBytes];
 constexpr int kStaticMaxDevices = 64;
 unsigned char* g_static_ws_addr[kStaticMaxDevices];     // per-device address of g_static_ws
 
@@ -1353,6 +1357,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
   L.rec = reinterpret_cast<int4*>(ws + lay.rec);
   L.tile_cnt = reinterpret_cast<unsigned*>(ws + lay.tile_cnt);
   L.ready = reinterpret_cast<unsigned*>(ws + lay.ready);
+  L.xchg = reinterpret_cast<unsigned long long*>(ws + lay.xchg);
   L.hq = ws + lay.hq;
   L.xq16 = ws + lay.xq16;
   L.xq16_stride = L.nbh * 288;
@@ -1606,7 +1611,7 @@ SGR_API int sgr_moe_layer_decode_static(const sgr_moe_layer* a, void* stream) {
   const WsLayout lay = ws_layout(a->n_max, a->hidden, a->n_ff, a->n_expert, a->n_used);
   // The whole layout must fit, so that the call picks its expert kernel exactly as a call on a
   // caller's workspace of sgr_moe_layer_workspace_bytes() does.
-  if (lay.total > kStaticWsBytes) return kErrStaticLimit;
+  if (lay.total - (lay.hbuf - lay.xchg) > kStaticWsBytes || lay.hbuf - lay.xchg > kStaticXchgBytes) return kErrStaticLimit;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kStaticMaxDevices) return kErrLaunch;
   if (g_static_ws_addr[dev] == nullptr) {
@@ -1616,11 +1621,12 @@ SGR_API int sgr_moe_layer_decode_static(const sgr_moe_layer* a, void* stream) {
   }
   unsigned char* ws = g_static_ws_addr[dev];
   // what must start at zero: the counters of the route and expert kernels, [cnt, hbuf) of the layout
-  // (cnt, tile_cnt, ready are adjacent)
-  if (cudaMemsetAsync(ws + lay.cnt, 0, lay.hbuf - lay.cnt, as_stream(stream)) != cudaSuccess)
+  // (cnt, tile_cnt, ready are adjacent), and the words by which a one-launch layer knows its own logits (xchg, after them)
+  const size_t words = a->n <= kTokenKernelMaxRows ? static_cast<size_t>(kXchgCopies) * a->n * a->n_expert * 8 : 0;
+  if (cudaMemsetAsync(ws + lay.cnt, 0, lay.xchg + words - lay.cnt, as_stream(stream)) != cudaSuccess)
     return kErrLaunch;
   sgr_moe_layer b = *a;
   b.workspace = ws;
-  b.workspace_bytes = kStaticWsBytes;
+  b.workspace_bytes = sizeof(g_static_ws);
   return sgr_moe_layer_decode_stages(&b, 7, stream);
 }

@@ -293,13 +293,13 @@ static __device__ __noinline__ void router_select_general(float* prob, int E, in
 // what follows from them (`picked()`) while the other adds and makes the weights. Dividing by the sum keeps
 // the order; only if it makes two of them equal, or something is not finite, the order of the quotients could be another
 // one, and the adding warp runs the general selection on the quotients: it returns true, and the picks do not stand.
-// `logits` in global memory, `prob` (E) and `pick_e` (K + 1) in shared memory, `bar` a barrier of the two warps.
-template <typename Picked>
-__device__ __forceinline__ bool router_select_pair(const float* logits, float* prob, float* pick_e, int* idx, float* w, int bar, bool adds, int E,
+// logit(j) is the row's logit lane + 32 j; `prob` (E) and `pick_e` (K + 1) in shared memory, `bar` a barrier of the two warps.
+template <typename Logit, typename Picked>
+__device__ __forceinline__ bool router_select_pair(Logit logit, float* prob, float* pick_e, int* idx, float* w, int bar, bool adds, int E,
                                             int K, float shared_w, int lane, Picked picked) {
   float e[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) e[j] = lane + 32 * j < E ? __ldcg(logits + lane + 32 * j) : -1e30f;
+  for (int j = 0; j < 8; ++j) e[j] = lane + 32 * j < E ? logit(j) : -1e30f;
   float mx = -1e30f;
 #pragma unroll
   for (int j = 0; j < 8; ++j) mx = fmaxf(mx, e[j]);
@@ -374,7 +374,9 @@ __device__ __forceinline__ bool router_select_pair(const float* logits, float* p
     if (lane == 0) w[K] = shared_w;
   } else {
     __syncwarp();
-    for (int m = lane; m < E; m += 32) prob[m] = __ldcg(logits + m);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (lane + 32 * j < E) prob[lane + 32 * j] = logit(j);
     __syncwarp();
     router_select_general(prob, E, K, idx, w, shared_w, lane);
   }

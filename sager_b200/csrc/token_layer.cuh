@@ -11,8 +11,8 @@
 //     are already on their way into shared memory - none of them depends on routing
 //   phase 1  Q8_K-quantise the rows (every CTA, redundantly: 4 KB per row), logits of the
 //            CTA's experts (a warp per expert row and token, the reference kernel's FMA order,
-//            so logits are bit-identical); arrive at the grid barrier; the shared expert's
-//            gate / up share while the others arrive
+//            so logits are bit-identical), published for the other CTAs; the shared expert's
+//            gate / up share while theirs arrive
 //   phase 2  every CTA selects redundantly from the n x E logits: for each row one warp picks
 //            and one adds up the softmax; from the picks warp 0 builds the list of tiles
 //            (distinct experts, each with the set of rows routed to it). The producer warp
@@ -24,14 +24,14 @@
 //   phase 4  every CTA quantises the h rows it needs (all of them: a few KB from L2),
 //            runs the down dots for its H / grid output rows of EVERY tile, and - since
 //            all of a row's expert contributions are then in this CTA - adds
-//            residual + sum_k w_k * y_k + shared in place. No third barrier.
+//            residual + sum_k w_k * y_k + shared in place. No second barrier.
 //
-// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 13.8 us per
-// layer, of which 3.5 to the first barrier, 2 for picks and tables, 1.5 for the first bytes, 2 for
-// gate / up, 2 for the second barrier, 1 + 1 for h and the down rows; 15.1 with the loops over rows of larger layers, whose live
-// values were spilled, 26.6 with eight warps on whole
-// blocks and the selection in sequence). A further row costs 3 to 6 us - 20.8 / 24.4 / 27.2 us at 2 / 3 / 4 rows, by dp4a
-// 21.7 / 28.3 / 32.7 -, where its bytes cost 2.2: of the 27.2, gate / up terms take 2.9, down terms 3.3, h in every CTA 2.3.
+// What it is bound by: at one row the chain (hidden 2048, n_ff 512, 256 experts, 8 used: 13.2 us per
+// layer, 2.3 to the logits, 1 until a CTA has all of them, 2 for picks and tables, 1.5 for the first bytes, 2 for
+// gate / up, 2 for the barrier, 1 + 1 for h and the down rows; 13.8 with a barrier between logits and selection, 15.1 with the loops over rows
+// of larger layers, whose live values were spilled, 26.6 with eight warps on whole blocks and the selection in sequence). A further
+// row costs 3 to 7 us - 20.7 / 23.9 / 27.1 us at 2 / 3 / 4 rows, by dp4a 21.7 / 28.3 / 32.7 -, where its bytes cost 2.2: of the 27.1, gate / up
+// terms take 2.9, down terms 3.3, h in every CTA 2.3.
 //
 // Work split: gate / up by pairs (a flat range of (tile, pair) per CTA, of equal cost), down by output
 // rows. Contracts are those of the two-launch path: null table entry = absent expert
@@ -173,8 +173,9 @@ inline bool use_mma(int n, int K, int H, int FF, int grid) {
   return n > 1 && H / kQK > 4 && static_cast<long long>(n) * K * FF > 2LL * grid * kPairsStage;
 }
 
-// Named barriers of the consumers: 6 all of them, 7 the warps with router rows, 5 the warps that quantise, 8 .. 11 the
-// two warps that select for a token row, 12 the warps that pick,
+// Named barriers of the consumers: 6 all of them, 5 the warps that quantise, 1 .. 4 and 8 .. 11 the
+// two warps that select for a token row (the logits are there; the picks are: the picking warp only arrives at both, so they cannot be
+// one barrier, at which its second arrival could stand for the other warp's), 12 the warps that pick,
 // 13 the warp that picks the only row and the second group, 14 and 15 each group.
 __device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 __device__ __forceinline__ void consumers_sync() {
@@ -198,17 +199,54 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
   asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-// Grid-wide barrier on a 64-bit arrival counter that only ever grows: the k-th barrier of the
-// grid (over all launches on this workspace) completes when the counter reaches k * G. Waits are
-// bounded: false when the others did not arrive in time.
+// Grid-wide barrier on a 64-bit arrival counter that only ever grows: that of the k-th launch on this
+// workspace completes when the counter reaches k * G. Waits are bounded: false when the others did not arrive in time.
 // The counter is read by the producer warp when the kernels before this one have finished - some multiple of
-// the grid size plus the arrivals of this launch's CTAs that are already further on, none of which can have passed
-// the first barrier - so barrier k of this launch completes at base + k * grid. (Read at kernel start, it could lie
-// between the barriers of a launch before on the same workspace, wherever two CTAs fit on one SM.) An arrival is a fire-and-forget releasing
-// add by the thread whose warp finishes the work; the producer warp polls and passes the word on
-// through an mbarrier, so no consumer waits for a round trip that it could work through.
-__device__ __forceinline__ unsigned long long grid_base(const unsigned long long* ctr, unsigned grid) {
-  return ld_acquire_u64(ctr) / grid * grid;
+// the grid size plus the arrivals of this launch's CTAs that are already further on, of which one at least is missing, this
+// CTA's own -, so the barrier completes at base + grid. (Read at kernel start, it could lie among the arrivals of a launch before on the
+// same workspace, wherever two CTAs fit on one SM.) An arrival is a fire-and-forget releasing add by the thread whose warp
+// finishes the work; the producer warp polls and passes the word on through an mbarrier, so no consumer waits for a round trip
+// that it could work through.
+//
+// The logits go from CTA to CTA without a barrier. A word holds a logit and, above it, base / grid + 1, which no launch before on the
+// workspace had; a warp of each CTA reads a row's words until all have it. Behind a barrier they took two more trips: an
+// arrival waits for the stores before it, and the reads begin when the poll returns. There are kXchgCopies of the words, written by
+// as many lanes, and a CTA reads one: 148 readers of the same lines are in the writers' way. us per layer at one row, behind the
+// barrier, then with 1 / 2 / 4 / 8 / 16 copies: hidden 2048, 256 experts 13.8, 14.3 / 13.6 / 13.4 / 13.2 / 13.2; 1024, 128 12.3, 13.8 / 12.7 / 12.7 /
+// 12.3 / 12.0; 2048, 64 12.0, 12.7 / 12.4 / 12.2 / 12.1 / 11.9; 512, 16 10.8, 11.1 / 11.2 / 11.0 / 10.9 / 10.8; two to four rows of the first 21.0 / 24.5 /
+// 27.2 and 20.7 / 23.9 / 27.1 with 16. Two warps per CTA that read, or words that are there read again: 16.5. (Copies of the
+// barrier's counter as well: no gain.)
+__device__ __forceinline__ void put_logit(unsigned long long* p, unsigned tag, float v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(static_cast<unsigned long long>(tag) << 32 | __float_as_uint(v)) : "memory");
+}
+__device__ __forceinline__ unsigned long long poll_word(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+// Logits first + lane, + 32, ... (at most N) of the row; false when they did not all arrive. Only what is missing is read again.
+template <int N>
+__device__ __forceinline__ bool get_logits(const unsigned long long* row, unsigned tag, int first, int E, int lane, float (&v)[N]) {
+  unsigned missing = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    v[j] = 0.f;
+    if (first + lane + 32 * j < E) missing |= 1u << j;
+  }
+  for (unsigned it = 0; it < kSpinLimit; ++it) {
+    unsigned long long w[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (missing >> j & 1) w[j] = poll_word(row + first + lane + 32 * j);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if ((missing >> j & 1) && static_cast<unsigned>(w[j] >> 32) == tag) {
+        v[j] = __uint_as_float(static_cast<unsigned>(w[j]));
+        missing &= ~(1u << j);
+      }
+    if (__all_sync(0xFFFFFFFFu, missing == 0)) return true;
+  }
+  return false;
 }
 __device__ __forceinline__ void grid_arrive(unsigned long long* ctr) {
   asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(ctr) : "memory");
@@ -486,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   uint64_t* dn_full = shdn_full + 1;                               // [2] routed tiles' down rows, rounds in turn
   uint64_t* dn_empty = dn_full + 2;                                // [2]
   uint64_t* ready = dn_empty + 2;                                  // tables built
-  uint64_t* based = ready + 1;                                     // the grid counter has been read
+  uint64_t* based = ready + 1;                                     // the grid counter has been read: flag[0] is base / grid + 1
   uint64_t* passed = based + 1;                                    // grid barrier passed (or given up), one phase each
   StageDesc* desc = reinterpret_cast<StageDesc*>(smem + 128);      // [kRing]
   int* flag = reinterpret_cast<int*>(smem + 256);
@@ -606,23 +644,16 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     pdl_wait();
     unsigned long long bar_base = 0;
     if (lane == 0) {
-      bar_base = grid_base(gctr, grid);
+      const unsigned long long k = ld_acquire_u64(gctr) / grid;
+      bar_base = k * grid;
+      flag[0] = static_cast<int>(static_cast<unsigned>(k) + 1u);
+      __threadfence_block();
       mbar_arrive_one(based);
     }
-    // barrier k of the grid: its outcome goes to flag[k - 1]
-    auto grid_poll = [&](int k) {
-      if (lane == 0) {
-        flag[k - 1] = grid_wait(gctr, bar_base + static_cast<unsigned long long>(k) * grid) ? 1 : 0;
-        __threadfence_block();
-        mbar_arrive_one(passed);
-      }
-      __syncwarp();
-    };
-    grid_poll(1);
     bool built = mbar_wait(ready, 0);
     if (built && by_pairs && *reinterpret_cast<volatile int*>(flag + 2) != 0) built = mbar_wait(ready, 1);
     if (!built) {
-      if (lane == 0 && flag[0]) atomicExch(L.status, 7);
+      if (lane == 0) atomicExch(L.status, 7);
       return;
     }
     const int T = tb.n_tiles;
@@ -736,7 +767,12 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       }
       issue_down_round(round++);
     }
-    grid_poll(2);
+    if (lane == 0) {                                // the barrier's outcome goes to flag[1]
+      flag[1] = grid_wait(gctr, bar_base + grid) ? 1 : 0;
+      __threadfence_block();
+      mbar_arrive_one(passed);
+    }
+    __syncwarp();
     for (; round < rounds; ++round) {               // later rounds reuse the regions
       if (!mbar_wait(&dn_empty[round & 1], (round / 2 - 1) & 1)) {
         if (lane == 0) atomicExch(L.status, 2);
@@ -809,12 +845,9 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       for (; k < H; k += 32) acc = fmaf(wr[k], h2f(xr[k]), acc);
 #pragma unroll
       for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xFFFFFFFFu, acc, off);
-      if (lane == 0) L.logits[static_cast<size_t>(t) * E + e] = acc + b;
-    }
-    if (nlw > 1) named_sync(7, nlw * 32);
-    if (tid == 0) {
-      mbar_wait(based, 0);                       // (set when the kernels before this one have finished)
-      grid_arrive(gctr);
+      acc = __shfl_sync(0xFFFFFFFFu, acc, 0);
+      if (lane < kXchgCopies && mbar_wait(based, 0))         // (set when the kernels before this one have finished)
+        put_logit(L.xchg + (lane * n + t) * E + e, static_cast<unsigned>(*reinterpret_cast<volatile int*>(flag)), acc + b);
     }
   } else {
 #pragma unroll 1
@@ -899,12 +932,28 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   };
   if (warp < 2 * kMaxTok && (warp & (kMaxTok - 1)) < n) {
     const int t = warp & (kMaxTok - 1);
-    const bool there = __all_sync(0xFFFFFFFFu, mbar_wait(passed, 0)) && *reinterpret_cast<volatile int*>(flag) != 0;
-    const float* lg = L.logits + static_cast<size_t>(t) * E;
+    const unsigned long long* row = L.xchg + ((cta & (kXchgCopies - 1)) * n + t) * E;
     float* pr = prob + static_cast<size_t>(t) * ((E + 3) & ~3);
+    float v[8] = {};                             // (one row) this lane's logits
+    bool there = true;
+    if (warp < kMaxTok) {
+      there = __all_sync(0xFFFFFFFFu, mbar_wait(based, 0)) &&
+              get_logits<8>(row, static_cast<unsigned>(*reinterpret_cast<volatile int*>(flag)), 0, min(E, 256), lane, v);
+      if (by_pairs) {                            // for the warp that adds
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (lane + 32 * j < E) pr[lane + 32 * j] = v[j];
+        __syncwarp();
+        asm volatile("bar.arrive %0, 64;" ::"r"(1 + t) : "memory");
+      }
+    } else if (by_pairs) {
+      named_sync(1 + t, 64);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = lane + 32 * j < E ? pr[lane + 32 * j] : 0.f;
+    }
     if (!there) ok = false;                      // (the named barriers below need every warp: it goes on with what is there)
     if (by_pairs) {
-      const bool redo = router_select_pair(lg, pr, tb.pick_e[t], tb.sel_idx[t], tb.sel_w[t], 8 + t, warp >= kMaxTok, E, K, L.shared_w, lane, [&] {
+      const bool redo = router_select_pair([&](int j) { return v[j]; }, pr, tb.pick_e[t], tb.sel_idx[t], tb.sel_w[t], 8 + t, warp >= kMaxTok, E, K, L.shared_w, lane, [&] {
         if (n == 1) asm volatile("bar.arrive 13, %0;" ::"n"(32 + kGroupThreads) : "memory");   // the second group fetches
         else named_sync(12, n * 32);             // every row's picks are in the tables
         if (warp == 0) build();
@@ -913,7 +962,12 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       __syncwarp();
       if (there && lane == 0 && (warp == 0 || warp >= kMaxTok)) mbar_arrive_one(ready);
     } else if (warp < kMaxTok && there) {
-      for (int i = lane; i < E; i += 32) pr[i] = __ldcg(lg + i);
+      for (int first = 0; first < E; first += 256) {
+        if (!get_logits<8>(row, static_cast<unsigned>(*reinterpret_cast<volatile int*>(flag)), first, E, lane, v)) ok = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (first + lane + 32 * j < E) pr[first + lane + 32 * j] = v[j];
+      }
       __syncwarp();
       router_select_general(pr, E, K, tb.sel_idx[t], tb.sel_w[t], L.shared_w, lane);
     }
@@ -1020,7 +1074,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     ok = __all_sync(0xFFFFFFFFu, ok) != 0;
     if constexpr (MMA) {
       if (rd == 0) {
-        const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
+        const bool met = mbar_wait(passed, 0) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
         quantize_h_rows<5>(hq, tb.n_hrows, L.hbuf, warp, lane);
         if (!consumers_all(met && ok)) {
           if (tid == 0) atomicExch(L.status, ok ? 5 : 3);
@@ -1069,7 +1123,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         load_half<1>(W, w, f_half);
         if (first) {
           first = false;
-          const bool met = mbar_wait(passed, 1) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
+          const bool met = mbar_wait(passed, 0) && *reinterpret_cast<volatile int*>(flag + 1) != 0;
           quantize_h_rows<2>(hq, tb.n_hrows, L.hbuf, warp, lane);
           if (!consumers_all(met && ok)) {
             if (tid == 0) atomicExch(L.status, ok ? 5 : 3);

@@ -604,6 +604,25 @@ def test_several_rows_on_the_mma(hidden, n_ff, E, k):
                     assert rel(o0.cpu().numpy(), o1.cpu().numpy()) < 1e-5        # another order of the same fp32 terms
 
 
+@pytest.mark.parametrize("hidden,n_ff,E,k", [(512, 256, 16, 4), (512, 256, 300, 4), (2048, 512, 64, 8)])
+def test_one_workspace_through_changing_row_counts(hidden, n_ff, E, k):
+    """The CTAs of a one-launch layer know each other's logits by the launch's number: whatever ran on the workspace before - more
+    rows, fewer, the two-launch path - every layer has the bits that it has on a workspace of its own."""
+    w = synth.MoeWeights(hidden, n_ff, E, DEV, seed=97, std=0.05)
+    runner = MoeLayerRunner(6, hidden, n_ff, E, k, DEV)
+    for step, n in enumerate((1, 4, 1, 6, 1, 2, 3, 5, 4, 2, 1, 1, 3)):
+        x16 = synth.normal_fp16((n, hidden), 970 + step, DEV)
+        if step % 3 == 0:
+            x16.zero_()                                   # logits of zero, equal everywhere
+        outs = []
+        for r in (runner, MoeLayerRunner(6, hidden, n_ff, E, k, DEV)):
+            out = torch.zeros(n, hidden, dtype=torch.float32, device=DEV)
+            r.run(r.args(n, x16, w.router, w.table(), w.shared_ptrs(), x_f16=x16.clone(), out_f32=out))
+            outs.append((out, r.route_idx[:n].clone(), r.route_w[:n].clone()))
+        assert all(torch.equal(a, b) for a, b in zip(*outs)), (step, n)
+    assert lib().raw("sgr_status")(0) == 0
+
+
 def test_four_rows_on_a_workspace_for_the_item_kernel(full_w):
     """A workspace too small for the row-streaming kernel keeps four rows on the item kernel and its order of the sums."""
     x16 = synth.normal_fp16((4, full_w.hidden), 870, DEV)
