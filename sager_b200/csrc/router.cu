@@ -89,32 +89,48 @@ __device__ __forceinline__ void store_folded(const unsigned long long (&acc)[TR]
   }
 }
 
-// The product for rows of whole 16-byte pieces: the raw columns of W and x arrive by cp.async three stages of 128 columns
-// ahead, x is turned into fp32 token pairs stage by stage - ldmatrix.trans hands a lane two tokens' values of one k, so
-// eight tokens x 32 columns are one load, eight conversions and four stores -, W is used as it lies. Against the kernel below,
-// which converts from registers after 2-byte loads: 2048 / 1024 / 592 / 96 tokens 70.6 / 38.0 / 23.3 / 7.9 us, 76.9 / 44.7 /
-// 35.0 / 9.2 before. Bound by the FMA pipe (2 cycles a packed FMA: 30 us at 2048 tokens) and the shared-memory operands (36 us),
-// which two warps per scheduler do not overlap further: volatile loads, other tiles and more warps changed nothing.
+// The product for rows of whole 16-byte pieces: a lane holds two neighbouring chains (columns 2 c, 2 c + 1 of every 32, c = lane % 16)
+// of TR rows x TT tokens, and the packed FMA's two components are these chains, so that W and x are used as they lie: a row's two
+// weights are one 8-byte read that both halves of the warp share, a token's two values one 4-byte read and two conversions.
+// The raw columns arrive by cp.async, 128 to a stage, SLOTS - 1 stages ahead. 2048 / 1200 / 777 tokens x 256 rows of 2048 columns behind a
+// top-k: 66.6 / 40.9 / 28.3 us, where a lane with one chain of two tokens - its weights spread over both components, x turned
+// into token pairs in shared memory first - took 80.9 / 49.0 / 33.8. Neither pipe is full (at 2048 tokens FMA 66 %,
+// shared memory 65 %): a packed FMA takes about three cycles and not two, and leaving out the conversions, either operand's loads or the
+// copies gives 4 to 10 % each. (Scalar FMAs 75.8 for 57.6 back to back; the order of the products, the roles of the operands, W brought
+// into L2 before the wait for the kernel before: nothing.)
 // block: WR x WT warps; grid (row tiles, token tiles).
-template <int TR, int TT, int WR, int WT>
+template <int TR, int TT, int WR, int WT, int SLOTS>
 struct Logits {
-  static constexpr int kWarps = WR * WT, kRows = TR * WR, kToks = TT * WT, kPairs = kToks / 2, kCols = 128, kSlots = 4;
-  static constexpr int kXPitch = (kCols + 8) * 2;            // bytes of a raw x row: eight rows' 16 bytes in different banks
-  static constexpr int kPairPitch = kCols * 8 + 32;          // bytes of a pair: [column][two tokens]
-  static constexpr int kWBytes = kRows * kCols * 4, kXBytes = kToks * kXPitch, kPairBytes = kPairs * kPairPitch;
-  static constexpr int kSmem = kSlots * (kWBytes + kXBytes) + 2 * kPairBytes;
-  static_assert(kToks % 8 == 0 && kWBytes % 16 == 0 && kXBytes % 16 == 0 && kPairBytes % 16 == 0, "tile");
+  static constexpr int kWarps = WR * WT, kRows = TR * WR, kToks = 2 * TT * WT, kCols = 128, kSlots = SLOTS;
+  static constexpr int kXPitch = kCols * 2 + 64;             // bytes of an x row: two tokens' 64 bytes in different banks
+  static constexpr int kWBytes = kRows * kCols * 4, kXBytes = kToks * kXPitch;
+  static constexpr int kSmem = kSlots * (kWBytes + kXBytes);
 };
-template <int TR, int TT, int WR, int WT>
-__global__ void __launch_bounds__(WR* WT * 32, (TR * TT >= 128 ? 8 : TR * TT >= 64 ? 16 : 20) / (WR * WT))
+// One step of the exchange for lanes that hold two chains each: as fold_lanes.
+template <int N, int Bit>
+__device__ __forceinline__ void fold_pairs(float (*f)[2], int lane) {
+  if constexpr (Bit > 0) {
+    const bool up = (lane & Bit) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float keep = up ? f[i + N / 2][h] : f[i][h];
+        const float send = up ? f[i][h] : f[i + N / 2][h];
+        f[i][h] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, Bit);
+      }
+    fold_pairs<N / 2, Bit / 2>(f, lane);
+  }
+}
+template <int TR, int TT, int WR, int WT, int SLOTS>
+__global__ void __launch_bounds__(WR* WT * 32, (TR * TT >= 64 ? 8 : TR * TT >= 32 ? 16 : 20) / (WR * WT))
 router_logits_staged_kernel(const float* __restrict__ w, const uint16_t* __restrict__ x, float* __restrict__ y,
                             int n_rows, int k, int n_tokens) {
-  using T = Logits<TR, TT, WR, WT>;
+  using T = Logits<TR, TT, WR, WT, SLOTS>;
   constexpr int kThreads = T::kWarps * 32;
   extern __shared__ __align__(16) unsigned char smem[];
   unsigned char* const w_raw = smem;                                           // [kSlots][kRows][128] fp32
   unsigned char* const x_raw = smem + T::kSlots * T::kWBytes;                  // [kSlots][kToks][kXPitch]
-  unsigned char* const x_f32 = x_raw + T::kSlots * T::kXBytes;                 // [2][kPairs][kPairPitch]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row0 = blockIdx.x * T::kRows, tok0 = blockIdx.y * T::kToks;
   const int wr = warp % WR, wt = warp / WR;
@@ -131,95 +147,74 @@ router_logits_staged_kernel(const float* __restrict__ w, const uint16_t* __restr
   for (int i = 0; i < kWPieces; ++i) w_at[i] = w + static_cast<size_t>(min(row0 + (tid >> 5) + i * (kThreads / 32), n_rows - 1)) * k + w_col;
 #pragma unroll
   for (int i = 0; i < kXPieces; ++i) x_at[i] = x + static_cast<size_t>(min(tok0 + (tid >> 4) + i * (kThreads / 16), n_tokens - 1)) * k + x_col;
-  auto fill_w = [&](int c) {
-    const int k0 = c * T::kCols;
-    if (k0 >= k) return;
-    const bool in = k0 + w_col < k;
-    const uint32_t dst = smem_u32(w_raw + (c % T::kSlots) * T::kWBytes + tid * 16);
-#pragma unroll
-    for (int i = 0; i < kWPieces; ++i) piece(dst + i * kThreads * 16, in ? w_at[i] + k0 : w, in);
-  };
-  auto fill_x = [&](int c) {
+  auto fill = [&](int c) {
     const int k0 = c * T::kCols;
     if (k0 < k) {
-      const bool in = k0 + x_col < k;
-      const uint32_t dst = smem_u32(x_raw + (c % T::kSlots) * T::kXBytes + (tid >> 4) * T::kXPitch + (tid & 15) * 16);
+      const bool w_in = k0 + w_col < k, x_in = k0 + x_col < k;
+      const uint32_t wd = smem_u32(w_raw + (c % T::kSlots) * T::kWBytes + tid * 16);
+      const uint32_t xd = smem_u32(x_raw + (c % T::kSlots) * T::kXBytes + (tid >> 4) * T::kXPitch + (tid & 15) * 16);
 #pragma unroll
-      for (int i = 0; i < kXPieces; ++i) piece(dst + i * (kThreads / 16) * T::kXPitch, in ? x_at[i] + k0 : x, in);
+      for (int i = 0; i < kWPieces; ++i) piece(wd + i * kThreads * 16, w_in ? w_at[i] + k0 : w, w_in);
+#pragma unroll
+      for (int i = 0; i < kXPieces; ++i) piece(xd + i * (kThreads / 16) * T::kXPitch, x_in ? x_at[i] + k0 : x, x_in);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // unit: eight tokens x 32 columns; lane i receives tokens 2 (i % 4), + 1 of columns i / 4 + 0, 8, 16, 24
-  auto convert = [&](int c) {
-    const unsigned char* raw = x_raw + (c % T::kSlots) * T::kXBytes;
-    unsigned char* out = x_f32 + (c & 1) * T::kPairBytes;
-    auto load = [&](uint32_t (&v)[4], int g, int j) {
-      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                   : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
-                   : "r"(smem_u32(raw + (g * 8 + (lane & 7)) * T::kXPitch + (j * 32 + (lane >> 3) * 8) * 2)) : "memory");
-    };
-    auto f = [](uint32_t h, int hi) { return __half2float(__ushort_as_half(static_cast<unsigned short>(hi ? h >> 16 : h & 0xFFFFu))); };
-    constexpr int kUnits = T::kToks / 8 * 4;
-    static_assert(kUnits % T::kWarps == 0, "units");
-#pragma unroll
-    for (int u = warp; u < kUnits; u += T::kWarps) {
-      const int g = u >> 2, j = u & 3;
-      uint32_t a[4];
-      load(a, g, j);
-      unsigned char* o = out + (g * 4 + (lane & 3)) * T::kPairPitch + j * 256 + (lane >> 2) * 8;
-#pragma unroll
-      for (int m = 0; m < 4; ++m) *reinterpret_cast<float2*>(o + m * 64) = make_float2(f(a[m], 0), f(a[m], 1));
-    }
   };
 
   const int chunks = (k + T::kCols - 1) / T::kCols;
   pdl_wait();                                   // (a caller's kernel may have written W as well as x)
   pdl_launch_dependents();
 #pragma unroll
-  for (int c = 0; c < T::kSlots - 1; ++c) {
-    fill_w(c);
-    fill_x(c);
-  }
-  asm volatile("cp.async.wait_group %0;" ::"n"(T::kSlots - 2) : "memory");
-  __syncthreads();
-  convert(0);
-  unsigned long long acc[TR][TT / 2];           // two packed fp32 sums each
+  for (int c = 0; c < T::kSlots - 1; ++c) fill(c);
+  unsigned long long acc[TT][TR];               // two chains' fp32 sums each
 #pragma unroll
-  for (int r = 0; r < TR; ++r)
+  for (int t = 0; t < TT; ++t)
 #pragma unroll
-    for (int p = 0; p < TT / 2; ++p) acc[r][p] = 0ull;
+    for (int r = 0; r < TR; ++r) acc[t][r] = 0ull;
 #pragma unroll 1
   for (int c = 0; c < chunks; ++c) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(T::kSlots - 3) : "memory");     // chunk c + 1 has landed
-    __syncthreads();                            // ... everybody's part of it; chunk c is converted, chunk c - 1 no longer read
-    fill_w(c + T::kSlots - 1);
-    fill_x(c + T::kSlots - 1);
-    const float* wp = reinterpret_cast<const float*>(w_raw + (c % T::kSlots) * T::kWBytes) + wr * TR * T::kCols + lane;
-    const unsigned char* xp = x_f32 + (c & 1) * T::kPairBytes + wt * (TT / 2) * T::kPairPitch + lane * 8;
-    // operands of 32 columns (one per lane); the next ones are loaded under this one's products
-    float wv[2][TR];
-    unsigned long long xv[2][TT / 2];
+    asm volatile("cp.async.wait_group %0;" ::"n"(T::kSlots - 2) : "memory");     // chunk c has landed
+    __syncthreads();                            // ... everybody's part of it; chunk c - 1 is no longer read
+    fill(c + T::kSlots - 1);
+    const unsigned char* wp = w_raw + (c % T::kSlots) * T::kWBytes + wr * TR * T::kCols * 4 + (lane & 15) * 8;
+    const unsigned char* xp = x_raw + (c % T::kSlots) * T::kXBytes + (wt * 2 * TT + (lane >> 4)) * T::kXPitch + (lane & 15) * 4;
+    // operands of 32 columns; the next ones are loaded under this one's products
+    unsigned long long wv[2][TR];
+    uint32_t xv[2][TT];
     auto load = [&](int j) {
 #pragma unroll
-      for (int r = 0; r < TR; ++r)
-        wv[j & 1][r] = wp[r * T::kCols + j * 32];
+      for (int r = 0; r < TR; ++r) wv[j & 1][r] = *reinterpret_cast<const unsigned long long*>(wp + (r * T::kCols + j * 32) * 4);
 #pragma unroll
-      for (int p = 0; p < TT / 2; ++p)
-        xv[j & 1][p] = *reinterpret_cast<const unsigned long long*>(xp + p * T::kPairPitch + j * 256);
-
+      for (int t = 0; t < TT; ++t) xv[j & 1][t] = *reinterpret_cast<const uint32_t*>(xp + 2 * t * T::kXPitch + j * 64);
     };
     load(0);
 #pragma unroll
     for (int j = 0; j < T::kCols / 32; ++j) {
       if (j + 1 < T::kCols / 32) load(j + 1);
-      if (j == 0 && c + 1 < chunks) convert(c + 1);
 #pragma unroll
-      for (int r = 0; r < TR; ++r)
+      for (int t = 0; t < TT; ++t) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&xv[j & 1][t]));
+        unsigned long long xx;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(xx) : "f"(v.x), "f"(v.y));
 #pragma unroll
-        for (int p = 0; p < TT / 2; ++p) fma2(acc[r][p], wv[j & 1][r], xv[j & 1][p]);
+        for (int r = 0; r < TR; ++r) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[t][r]) : "l"(wv[j & 1][r]), "l"(xx));
+      }
     }
   }
-  store_folded<TR, TT>(acc, y, row0 + wr * TR, tok0 + wt * TT, n_rows, n_tokens, lane);
+  // fold: chains 16, 8, 4 and 2 apart are in lanes 8, 4, 2 and 1 apart, the last two in one lane
+  float f[TT * TR][2];
+#pragma unroll
+  for (int t = 0; t < TT; ++t)
+#pragma unroll
+    for (int r = 0; r < TR; ++r) asm("mov.b64 {%0, %1}, %2;" : "=f"(f[t * TR + r][0]), "=f"(f[t * TR + r][1]) : "l"(acc[t][r]));
+  fold_pairs<TT * TR, 8>(f, lane);
+  constexpr int kLeft = TT * TR / 16;
+#pragma unroll
+  for (int i = 0; i < kLeft; ++i) {
+    const int o = i + kLeft * (lane & 15);
+    const int row = row0 + wr * TR + o % TR, tok = tok0 + wt * 2 * TT + 2 * (o / TR) + (lane >> 4);
+    if (row < n_rows && tok < n_tokens) y[static_cast<size_t>(tok) * n_rows + row] = f[i][0] + f[i][1];
+  }
 }
 
 // The same for rows off a 16-byte boundary.
@@ -342,12 +337,12 @@ int launch_tiled(const float* w, const uint16_t* x, float* y, int n_rows, int k,
   return launch_pdl(router_logits_tiled_kernel<TR, TT, WR, WT, KC>, grid, WR * WT * 32, kSmem, stream, w, x, y, n_rows, k, n_tokens);
 }
 
-template <int TR, int TT, int WR, int WT>
+template <int TR, int TT, int WR, int WT, int SLOTS>
 int launch_staged(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens, cudaStream_t stream) {
-  using T = Logits<TR, TT, WR, WT>;
-  if (!opt_in_smem<router_logits_staged_kernel<TR, TT, WR, WT>>(T::kSmem)) return kErrLaunch;
+  using T = Logits<TR, TT, WR, WT, SLOTS>;
+  if (!opt_in_smem<router_logits_staged_kernel<TR, TT, WR, WT, SLOTS>>(T::kSmem)) return kErrLaunch;
   const dim3 grid((n_rows + T::kRows - 1) / T::kRows, (n_tokens + T::kToks - 1) / T::kToks);
-  return launch_pdl(router_logits_staged_kernel<TR, TT, WR, WT>, grid, T::kWarps * 32, T::kSmem, stream, w, x, y, n_rows, k, n_tokens);
+  return launch_pdl(router_logits_staged_kernel<TR, TT, WR, WT, SLOTS>, grid, T::kWarps * 32, T::kSmem, stream, w, x, y, n_rows, k, n_tokens);
 }
 
 int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k, int n_tokens,
@@ -361,13 +356,17 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
     router_logits_kernel<<<(n_rows + warps - 1) / warps, warps * 32, smem, stream>>>(w, x, y, n_rows, k);
   } else if ((k & 7) == 0 && ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x)) & 15u) == 0 &&
              (n_tokens + 15) / 16 <= 65535) {
-    // A warp's outputs: more of them need fewer shared-memory operands per FMA, fewer of them give more warps to spread. 256 rows
-    // x 128 / 300 / 400 / 900 / 1200 / 1400 / 2048 tokens, us: 4 x 8 outputs 8.1 / 16.6 / 19.3 / 39.0 / 50.3 / 56.5 / 81.7,
-    // 8 x 8 8.6 / 17.3 / 17.5 / 37.6 / 47.4 / 52.9 / 73.2, 8 x 16 13.3 / 22.1 / 21.7 / 42.4 / 50.9 / 51.6 / 70.6.
+    // Larger tiles read fewer operands per FMA, smaller ones spread over more warps; and with few outputs W's way out of DRAM is most
+    // of the time, so a ring of eight stages or more asks for half of a CTA's rows at once. us of a prefill chunk with its experts (256 x
+    // 2048; four layers of 65 / 96 / 130 / 200 / 300 / 500 rows, two of 777 / 1200 / 2048): 4 x 4 outputs a lane, two warps, eight stages 444 / 467 /
+    // 494 / - / 615 / - / 493 / - / -; 8 x 4, four warps, eight 456 / 479 / 508 / 542 / 612 / 741 / 478 / 612 / 835 (with four stages 484 /
+    // 505 / 540 / 576 / 629 / 747 / 476 / 608 / 826, with twelve 442 / 464 / 505 / 547 / 621 / 758 / 490 / 634 / 864); 16 x 4, four warps, four 483 /
+    // 504 / 533 / 568 / 622 / 743 / 472 / 605 / 818; one chain to a lane 466 / 488 / 516 / 552 / 616 / 755 / 487 / 623 / 851. 64 experts, 300 rows:
+    // 141.6, 148.3, 147.9 and 147.3. (592 rows, back to back and L2-hot: 8 x 4 21.3, 16 x 4 25.7 - three CTAs on an SM for little more than two.)
     const long long outputs = static_cast<long long>(n_rows) * n_tokens;
-    if (outputs >= 256LL * 1300) return launch_staged<8, 16, 2, 2>(w, x, y, n_rows, k, n_tokens, stream);
-    if (outputs >= 256LL * 320) return launch_staged<8, 8, 2, 2>(w, x, y, n_rows, k, n_tokens, stream);
-    return launch_staged<4, 8, 4, 1>(w, x, y, n_rows, k, n_tokens, stream);
+    if (outputs >= 256LL * 620) return launch_staged<16, 4, 1, 4, 4>(w, x, y, n_rows, k, n_tokens, stream);
+    if (outputs >= 256LL * 180) return launch_staged<8, 4, 2, 2, 8>(w, x, y, n_rows, k, n_tokens, stream);
+    return launch_staged<4, 4, 2, 1, 8>(w, x, y, n_rows, k, n_tokens, stream);
   } else if (static_cast<long long>(n_rows) * n_tokens >= 256LL * 592) {
     // 8 x 16 outputs per warp keep the FMA pipes fullest; below one such CTA per SM the smaller tile has more
     // warps to spread (at 256 x 592 the two take 41 and 38 us, and from there the larger one wins)

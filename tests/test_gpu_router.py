@@ -74,6 +74,19 @@ def test_logits_staged_tiles_bit_exact(oracle, rows, k, n_tok):
     assert torch.all(y[n_tok] == 7.0)
 
 
+@pytest.mark.parametrize("rows,k,n_tok", [(256, 1032, 179), (256, 1024, 180), (250, 520, 619), (256, 136, 620), (256, 72, 619),
+                                          (7, 40, 17), (9, 1160, 31), (3, 2048, 2)])
+def test_logits_of_chain_pairs_bit_exact(oracle, rows, k, n_tok):
+    """Both sides of the lines between the tiles of two chains to a lane (rows x tokens = 256 x 180 and 256 x 620), with rows, tokens and columns that fill no tile."""
+    w_np, w_dev = router_w(11, e=rows, h=k)
+    x_np, x_dev = make_x16(n_tok, k, 12)
+    y = torch.full((n_tok + 1, rows), 7.0, dtype=torch.float32, device=DEV)
+    ops.gemv_f32_out_f16x_mtok(w_dev, x_dev, y, rows, k, n_tok)
+    want = np.stack([oracle.router_logits(w_np, x_np[t]) for t in range(n_tok)])
+    assert np.array_equal(y.cpu().numpy()[:n_tok].view(np.uint32), want.view(np.uint32))
+    assert torch.all(y[n_tok] == 7.0)
+
+
 @pytest.mark.parametrize("shift_w,shift_x,k", [(1, 0, 512), (0, 1, 512), (0, 0, 500)])
 def test_logits_off_a_16_byte_boundary(oracle, shift_w, shift_x, k):
     w_np, w_dev = router_w(9, e=40, h=k)
