@@ -366,7 +366,10 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
     const long long outputs = static_cast<long long>(n_rows) * n_tokens;
     if (outputs >= 256LL * 620) return launch_staged<16, 4, 1, 4, 4>(w, x, y, n_rows, k, n_tokens, stream);
     if (outputs >= 256LL * 180) return launch_staged<8, 4, 2, 2, 8>(w, x, y, n_rows, k, n_tokens, stream);
-    return launch_staged<4, 4, 2, 1, 8>(w, x, y, n_rows, k, n_tokens, stream);
+    if (outputs > 64LL * 2 * 148) return launch_staged<4, 4, 2, 1, 8>(w, x, y, n_rows, k, n_tokens, stream);
+    // (all CTAs fit on the SMs at once with twelve stages as well: 80 rows x 64 experts 112.5 for 115.6, 100 x 128 123.7 for 125.6, 65 x 256 440
+    // for 444; 96 x 256, where they do not, 474 for 467)
+    return launch_staged<4, 4, 2, 1, 12>(w, x, y, n_rows, k, n_tokens, stream);
   } else if (static_cast<long long>(n_rows) * n_tokens >= 256LL * 592) {
     // 8 x 16 outputs per warp keep the FMA pipes fullest; below one such CTA per SM the smaller tile has more
     // warps to spread (at 256 x 592 the two take 41 and 38 us, and from there the larger one wins)

@@ -74,10 +74,10 @@ def test_logits_staged_tiles_bit_exact(oracle, rows, k, n_tok):
     assert torch.all(y[n_tok] == 7.0)
 
 
-@pytest.mark.parametrize("rows,k,n_tok", [(256, 1032, 179), (256, 1024, 180), (250, 520, 619), (256, 136, 620), (256, 72, 619),
+@pytest.mark.parametrize("rows,k,n_tok", [(256, 1032, 74), (256, 1672, 75), (256, 1032, 179), (256, 1024, 180), (250, 520, 619), (256, 136, 620), (256, 72, 619),
                                           (7, 40, 17), (9, 1160, 31), (3, 2048, 2)])
 def test_logits_of_chain_pairs_bit_exact(oracle, rows, k, n_tok):
-    """Both sides of the lines between the tiles of two chains to a lane (rows x tokens = 256 x 180 and 256 x 620), with rows, tokens and columns that fill no tile."""
+    """Both sides of the lines between the tiles of two chains to a lane (rows x tokens = 256 x 74, 256 x 180 and 256 x 620), with rows, tokens and columns that fill no tile."""
     w_np, w_dev = router_w(11, e=rows, h=k)
     x_np, x_dev = make_x16(n_tok, k, 12)
     y = torch.full((n_tok + 1, rows), 7.0, dtype=torch.float32, device=DEV)
