@@ -696,12 +696,16 @@ int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratc
   const int sms = device_sms(), row_tiles = (n_rows + 127) / 128, nb = k / kQK;
   if (sms <= 0) return kErrLaunch;
   // Token rows per unit, CTAs that share a unit, and who writes the scratch: what takes the least by estimates in us, fitted to
-  // 17 shapes (4096 x 2048 over 2048 tokens: 31 measured / 31 estimated with units of a pair's 256 rows x 240 tokens, 45 / 44 with 128
-  // tokens, 33 / 34 by single CTAs; 1000 x 2048 over 777: 12.2 / 13.3 with 64 tokens, 14.1 / 14.2 with 208).
+  // 27 shapes (4096 x 2048 over 2048 tokens: units of a pair's 256 rows x 240 tokens 31 us, 45 with 128
+  // tokens, 33 by single CTAs; 1000 x 2048 over 777: 12.0). Against a CTA per unit only short rows come near: 2048 x 512 over 1457 / 700
+  // tokens 8.9 / 6.5 us for 8.7 / 6.4.
+  //   the start, 4, and the last unit's epilogue, 3 for 256 tokens (without it, and with a row tile's scratch in equal parts and not in whole
+  //     blocks, 512 x 512 over 400 / 1457 tokens 6.6 / 7.1 us for 5.0 / 5.5, 2048 x 2048 over 512 12.9 for 12.5)
   //   a block column of a unit: 1.0 and, with the square of its tokens, up to 0.35 more, a fifth more when every SM works; a pair
   //     brings half of the activations per CTA and gains a twentieth past 128 tokens, but costs 0.3 to set up
   //   the scratch, per block of a row tile: SMs that the units leave idle, in whole columns of row tiles, 3.2 / spare beside
-  //     the units' 1.3; the units of a row tile themselves, 2 / token tiles on top of it; or the dequantisation kernel ahead of the
+  //     the units' 1.3 and epilogue (2048 x 512 over 2048 tokens 10.9 -> 9.7); the units of a row tile themselves, 2 for each block that one
+  //     of its token tiles writes on top of it; or the dequantisation kernel ahead of the
   //     GEMM, 2.5 us and the bytes at 5 TB/s (8192 x 4096 over 64 tokens: 53 us by one spare column, 41 by the kernel ahead).
   struct Plan { int cg, bn, tiles, units, workers, spare; bool ahead; double us; } p{};
   for (int cg = 1; cg <= (row_tiles > 1 ? 2 : 1); ++cg) {
@@ -716,9 +720,9 @@ int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratc
       c.workers = std::min(c.units, sms / cg) * cg;
       const int waves = (c.units * cg + c.workers - 1) / c.workers;
       const double wide = bn / 256.;
-      c.us = 4 + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.05 : 1.);
+      c.us = 4 + 3 * wide + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.05 : 1.);
       const int spare = std::min(nb, (sms - c.workers) / row_tiles);
-      const double by_spare = spare > 0 ? nb * std::max(0., 3.2 / spare - 1.3) : 1e30, by_tiles = 2. * nb / c.tiles;
+      const double by_spare = spare > 0 ? std::max(0., nb * (3.2 / spare - 1.3) - 3 * wide) : 1e30, by_tiles = 2. * ((nb + c.tiles - 1) / c.tiles);
       const double by_kernel = 2.5 + static_cast<double>(n_rows) * k * 2.5625 / 5e6;
       c.spare = by_spare < by_tiles ? spare : 0;
       if (by_kernel < std::min(by_spare, by_tiles)) {
