@@ -18,7 +18,7 @@
 // contiguous bytes each at k = 2048) into a shared-memory ring with bulk copies, two groups of eight
 // consumer warps of four rows each, which take the stages in turn: what one group waits for - shared-memory loads with two lanes
 // to a bank, chains of dp4a - the other's arithmetic covers (two warps to a scheduler instead of four left its issue slots half
-// empty: 151,936 x 2048 49.7 us, now 44; with norm and top-k 64.4 and 59.0). A lane owns a quarter of a block (64 weights, four sub-groups): two
+// empty: 151,936 x 2048 49.2 us, now 42.3; with norm and top-k 64.4 and 58.3). A lane owns a quarter of a block (64 weights, four sub-groups): two
 // 16-byte runs of ql and one of qh, read as words (blocks start on 2-byte boundaries only: odd
 // blocks are realigned with a funnel shift), each ql word giving two packed words of 6-bit values
 // and each qh word serving four of them, fed to dp4a; a row of k = 2048 is one pass of a warp.
