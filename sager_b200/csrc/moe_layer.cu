@@ -1206,16 +1206,21 @@ int launch_layer(dim3 grid, int threads, size_t smem, cudaStream_t stream, const
 template <bool STREAM>
 int launch_token_layer(const tk::Geom& g, cudaStream_t s, const LayerDev& L) {
   const dim3 grid(L.grid);
-  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
-  if (g.part_bytes > 0) return launch_layer<tk::token_layer_kernel<true, false, false, true, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  if (L.n == 1) return launch_layer<tk::token_layer_kernel<false, true, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  static_assert(kRowsKernelMinRows == tk::kMaxTok, "geom has the blocks' terms of fewer rows apart");
+  if (g.part_bytes > 0) {
+    if (L.n >= kRowsKernelMinRows) return launch_layer<tk::token_layer_kernel<true, false, false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+    return tk::terms_apart(L.n, L.nbf) ? launch_layer<tk::token_layer_kernel<false, false, false, true, true, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                                       : launch_layer<tk::token_layer_kernel<false, false, false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  }
   // sharing by cost: two rows seldom meet in a tile (22.9 us a layer either way), and where a pass of both groups takes a CTA's
   // pairs there is nothing to share out
   const bool by_cost = L.n > 2 && static_cast<long long>(L.n) * L.K * L.FF > 2LL * L.grid * g.stage_pairs;
   if (L.n < kRowsKernelMinRows)
-    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L)
-                   : launch_layer<tk::token_layer_kernel<false, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
-  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true, false, STREAM>>(grid, tk::kThreads, g.total, s, L)
-                 : launch_layer<tk::token_layer_kernel<true, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+    return by_cost ? launch_layer<tk::token_layer_kernel<false, false, true, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                   : launch_layer<tk::token_layer_kernel<false, false, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
+  return by_cost ? launch_layer<tk::token_layer_kernel<true, false, true, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L)
+                 : launch_layer<tk::token_layer_kernel<true, false, false, false, false, STREAM>>(grid, tk::kThreads, g.total, s, L);
 }
 
 }  // namespace

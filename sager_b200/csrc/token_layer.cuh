@@ -127,6 +127,9 @@ struct Geom {
   int stage_pairs, stage_bytes, slot_bytes, down_tiles;
   int part_bytes;        // a stage's block terms: [block][pair][token][gate, up] floats
 };
+// Whether the MMA kernel keeps the terms of a down row's blocks until all are there: two and three rows add them as reduce_pairs does, which
+// for up to two blocks is one after the other.
+__host__ __device__ constexpr bool terms_apart(int n, int nbf) { return n < kMaxTok && nbf > 2; }
 __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int grid, bool mma) {
   Geom g;
   g.rows_per_cta = (E + grid - 1) / grid;
@@ -158,7 +161,7 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
   const int in_ring = kRing * g.stage_bytes / (g.slot_bytes > 0 ? g.slot_bytes : 1);
   g.down_tiles = in_ring < kDownTiles ? in_ring : kDownTiles;      // (none: the caller takes another path)
   g.off_dn = take(static_cast<size_t>(hrows < g.down_tiles ? hrows : g.down_tiles) * g.slot_bytes);
-  g.off_y = take(static_cast<size_t>(hrows) * g.nr_max * 4);
+  g.off_y = take(static_cast<size_t>(hrows) * g.nr_max * 4 * (mma && terms_apart(n, FF / kQK) ? FF / kQK : 1));
   g.total = p;
   return g;
 }
@@ -453,9 +456,16 @@ __device__ __forceinline__ void gate_up_stage(const unsigned char* st, int np, i
   }
 }
 
+// The sum of p(0), .. p(L - 1) in the order of reduce_pairs: i and i + L / 2 first.
+template <int L, int STEP = 1, typename Term>
+__device__ __forceinline__ float tree_sum(Term p, int i = 0) {
+  if constexpr (STEP == L) return p(i);
+  else return __fadd_rn(tree_sum<L, 2 * STEP>(p, i), tree_sum<L, 2 * STEP>(p, i + STEP));
+}
+
 // The same for layers of several rows, on the int8 MMA: a warp takes eight pairs and one block column at a time - gate rows and the
-// up rows of the same indices are the sixteen rows of a fragment -, the terms of a row's blocks meet in `part` and are added
-// block after block. A tile of four rows costs what a tile of one does; by dp4a 16 pairs took 0.25 us and 1.2 more per row of
+// up rows of the same indices are the sixteen rows of a fragment -, the terms of a row's blocks meet in `part` and are added in
+// gate_up_stage's order, so that a row's bits do not depend on which of the two took it. A tile of four rows costs what a tile of one does; by dp4a 16 pairs took 0.25 us and 1.2 more per row of
 // the tile, and the CTAs whose tile four rows share finished 8 us after the median one, or took fewer pairs.
 // `st` holds chunks of rows of `rb` bytes; a barrier of the group lies between the two functions.
 __device__ __forceinline__ void gate_up_terms(const unsigned char* st, int np, const RowSet& rs, const HTile& xt, int nbh, int rb, float* part,
@@ -486,6 +496,7 @@ __device__ __forceinline__ void gate_up_terms(const unsigned char* st, int np, c
     *reinterpret_cast<float2*>(part + ((b * part_pairs + gid * ch.rows + q) * kMaxTok + tig) * 2) = make_float2(v[0], v[1]);
   }
 }
+template <bool CHAIN>
 __device__ __forceinline__ void gate_up_sums(const float* part, int part_pairs, int np, const RowSet& rs, int hrow0, int pair0, const HTile& xt,
                                              float* hbuf, int FF, int nbh) {
   const int tid = threadIdx.x & (kGroupThreads - 1);
@@ -494,11 +505,27 @@ __device__ __forceinline__ void gate_up_sums(const float* part, int part_pairs, 
     const int t = (i >> 1) & (kMaxTok - 1), pair = i >> 3;
     const unsigned char* x = xt.blk(rs.at(min(t, rs.n - 1)), 0) + 136;
     float v = 0.f;
+    if constexpr (CHAIN) {
 #pragma unroll 4
-    for (int b = 0; b < nbh; ++b) v = fmaf(*reinterpret_cast<const float*>(x + b * kHBlk), part[(b * part_pairs) * 2 * kMaxTok + i], v);
+      for (int b = 0; b < nbh; ++b) v = fmaf(*reinterpret_cast<const float*>(x + b * kHBlk), part[(b * part_pairs) * 2 * kMaxTok + i], v);
+    } else {                                     // (five to sixteen blocks: use_mma)
+      auto term = [&](int b) {
+        return b < nbh ? __fmul_rn(*reinterpret_cast<const float*>(x + b * kHBlk), part[(b * part_pairs) * 2 * kMaxTok + i]) : 0.f;
+      };
+      v = nbh <= 8 ? tree_sum<8>(term) : tree_sum<16>(term);
+    }
     const float u = __shfl_down_sync(0xFFFFFFFFu, v, 1);
     if ((i & 1) == 0 && pair < np && t < rs.n) hbuf[static_cast<size_t>(hrow0 + t) * FF + pair0 + pair] = silu_mul(v, u);
   }
+}
+
+// The sum of the terms of `nb` blocks, `step` apart from p on and this thread's own, in the order of reduce_pairs.
+__device__ __forceinline__ float blocks_tree(float* p, int step, int nb) {
+#pragma unroll 1
+  for (int off = next_pow2_cap32(nb) >> 1; off > 0; off >>= 1)
+#pragma unroll 1
+    for (int i = 0; i < min(off, nb); ++i) p[i * step] = __fadd_rn(p[i * step], i + off < nb ? p[(i + off) * step] : 0.f);
+  return p[0];
 }
 
 // Producer: `bytes` (a multiple of 16) from a source that may be only 2-byte aligned; plain_done() ends a row of them. (Not
@@ -511,13 +538,15 @@ __device__ __forceinline__ void plain_done() {
   fence_proxy_async();
 }
 
-// CHAIN: layers of four token rows (see half_dots). ONE: layers of one, which are a chain of short steps: what only more rows
+// CHAIN: layers of four token rows (see half_dots); one to three have the bits of each row by itself. ONE: layers of one, which are a chain of short steps: what only more rows
 // need is neither executed nor fetched. BY_COST: layers whose CTAs take more pairs than a pass of both groups (see routed_share).
 // MMA: routed tiles on the int8 MMA (see use_mma). STREAM: weights first to leave L2 (streams_weights).
-template <bool CHAIN, bool ONE, bool BY_COST, bool MMA, bool STREAM>
+// APART: with terms_apart (a kernel of its own: its code in the other one cost layers of two blocks to a down row 0.8 us).
+template <bool CHAIN, bool ONE, bool BY_COST, bool MMA, bool APART, bool STREAM>
 __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev L) {
   extern __shared__ __align__(128) unsigned char smem[];
-  static_assert(!MMA || (CHAIN && !ONE && !BY_COST), "tiles on the MMA cost the same whatever their rows");
+  static_assert(!MMA || (!ONE && !BY_COST), "tiles on the MMA cost the same whatever their rows");
+  static_assert(!APART || (MMA && !CHAIN), "only a tree needs the terms apart");
   const Geom G = geom(ONE ? 1 : L.n, L.K, L.H, L.FF, L.E, gridDim.x, MMA);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);              // [kRing]
   uint64_t* empty = full + kRing;                                  // [kRing]
@@ -539,7 +568,8 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   unsigned char* sh_stage = smem + G.off_sh;
   unsigned char* ring = smem + G.off_ring;
   unsigned char* dn = smem + G.off_dn;
-  float* ysm = reinterpret_cast<float*>(smem + G.off_y);           // [hrow][nr_max]
+  float* ysm = reinterpret_cast<float*>(smem + G.off_y);           // [hrow][nr_max], terms apart: [block of h][hrow][nr_max]
+  const int y_plane = L.n * (L.K + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cta = blockIdx.x, grid = gridDim.x;
   const int n = ONE ? 1 : L.n, H = L.H, FF = L.FF, E = L.E, K = L.K;
@@ -1056,7 +1086,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         const RowSet rs = rows_of(work ? tb.tile_mask[d.tile] : 1, 0, true);
         if (work) gate_up_terms(st, d.np, rs, xt, L.nbh, G.rb_h, terms, G.stage_pairs, zeros, &empty[s]);
         named_sync(14 + group, kGroupThreads);
-        if (work) gate_up_sums(terms, G.stage_pairs, d.np, rs, tb.tile_hrow0[d.tile], d.pair0, xt, L.hbuf, FF, L.nbh);
+        if (work) gate_up_sums<CHAIN>(terms, G.stage_pairs, d.np, rs, tb.tile_hrow0[d.tile], d.pair0, xt, L.hbuf, FF, L.nbh);
       }
     }
   }
@@ -1090,26 +1120,29 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
           return;
         }
       }
-      const int gid = lane >> 2, tig = lane & 3;
+      // A warp per tile, or per tile and block where the blocks' terms are added as a tree of more than two; sixteen output rows at a time
+      const int gid = lane >> 2, tig = lane & 3, tasks = ok ? (j1 - j0) * (APART ? L.nbf : 1) : 0;
 #pragma unroll 1
-      for (int j = ok ? j0 + warp : j1; j < j1; j += kWarps) {         // a warp per tile, sixteen output rows at a time
+      for (int q = warp; q < tasks; q += kWarps) {
+        const int j = j0 + (APART ? q / L.nbf : q), b0 = APART ? q % L.nbf : 0, b1 = APART ? b0 + 1 : L.nbf;
         if (tb.tile_mode[j] == 1) continue;
         const int hrow0 = tb.tile_hrow0[j], rows = __popc(tb.tile_mask[j]);
         const int row = hrow0 + min((lane & 7) >> 1, rows - 1), row_m = hrow0 + min(gid >> 1, rows - 1), row_t = hrow0 + min(tig, rows - 1);
+        float* y = ysm + (b0 * y_plane + hrow0 + tig) * G.nr_max;
 #pragma unroll 1
         for (int m0 = 0; m0 < nr; m0 += 16) {
-          const unsigned char* w = from + static_cast<size_t>(j - j0) * G.slot_bytes;
+          const unsigned char* w = from + static_cast<size_t>(j - j0) * G.slot_bytes + b0 * kW4;
           const int ra = min(m0 + (lane & 15), nr - 1), q0 = m0 + gid, q1 = q0 + 8;
-          float acc[2] = {0.f, 0.f};
+          float acc[2] = {CHAIN ? 0.f : -0.f, CHAIN ? 0.f : -0.f};       // (-0 + v is v)
 #pragma unroll 1
-          for (int b = 0; b < L.nbf; ++b, w += kW4) {
+          for (int b = b0; b < b1; ++b, w += kW4) {
             const float xd = *reinterpret_cast<const float*>(hq.blk(row_t, b) + 136);
             mma_terms(w + ra * G.rb_f + 16 + (lane >> 4) * 16, w + min(q0, nr - 1) * G.rb_f, w + min(q1, nr - 1) * G.rb_f, hq.blk(row, b), hq.blk(row_m, b),
-                      zeros, lane, [] {}, [&](int r, float v) { acc[r] = fmaf(xd, v, acc[r]); });
+                      zeros, lane, [] {}, [&](int r, float v) { acc[r] = CHAIN ? fmaf(xd, v, acc[r]) : __fadd_rn(acc[r], __fmul_rn(xd, v)); });
           }
           if (tig < rows) {
-            if (q0 < nr) ysm[(hrow0 + tig) * G.nr_max + q0] = acc[0];
-            if (q1 < nr) ysm[(hrow0 + tig) * G.nr_max + q1] = acc[1];
+            if (q0 < nr) y[q0] = acc[0];
+            if (q1 < nr) y[q1] = acc[1];
           }
         }
       }
@@ -1157,6 +1190,14 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   if (!consumers_all(ok)) {
     if (tid == 0) atomicExch(L.status, 3);
     return;
+  }
+  if constexpr (APART) {
+    for (int i = tid; i < tb.n_hrows * nr; i += kConsumers) {
+      const int hr = i / nr;
+      float* p = ysm + hr * G.nr_max + (i - hr * nr);
+      p[0] = blocks_tree(p, y_plane * G.nr_max, L.nbf);
+    }
+    consumers_sync();
   }
   for (int i = tid; i < n * nr; i += kConsumers) {
     const int t = i / nr, rr = i - t * nr;

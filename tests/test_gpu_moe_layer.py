@@ -578,11 +578,17 @@ def test_one_launch_layers_back_to_back_on_one_workspace(hidden, n_ff, E, k):
     (2048, 512, 256, 8),     # two rows of a stage to a chunk, the last stage of a CTA one or none
     (1280, 1024, 48, 8),     # five block columns, eight tiles' down rows at a time, four blocks to a down row
     (1536, 768, 40, 7),      # six and three
-    (2048, 256, 64, 8),      # two rows: the dp4a kernel and its order, three and four: the MMA's
+    (2048, 256, 64, 8),      # two rows: the dp4a kernel
+    (3072, 256, 24, 10),     # twelve, and one
+    (1280, 2048, 24, 8),     # five, and eight
 ])
 def test_several_rows_on_the_mma(hidden, n_ff, E, k):
-    """Routed tiles on the int8 MMA: exact integer sums, the fp32 terms of a row's blocks one after the other, as in the
-    row-streaming kernel - the same bits. Tiles of one row to all, null experts, no shared one, weights off a 16-byte boundary."""
+    """Routed tiles on the int8 MMA: exact integer sums, and the fp32 terms of a row's blocks in the order of the kernels without it.
+    Two and three rows have the bits that each row has by itself, four those of the row-streaming kernel, whichever form a
+    geometry takes. Tiles of one row to all, null experts, no shared one, weights off a 16-byte boundary."""
+    def same(a, b):
+        return torch.equal(a.view(torch.int32 if a.dtype == torch.float32 else torch.int16), b.view(torch.int32 if b.dtype == torch.float32 else torch.int16))
+
     for shift in (0, 4):
         w = synth.MoeWeights(hidden, n_ff, E, DEV, seed=95, std=0.05)
         if shift:
@@ -591,17 +597,17 @@ def test_several_rows_on_the_mma(hidden, n_ff, E, k):
             moved.copy_(w.blob.view(-1))
             w.blob = moved.view(w.blob.shape)
         for n in (2, 3, 4):
-            on_mma = n * k * n_ff > 2 * 16 * torch.cuda.get_device_properties(0).multi_processor_count
             for i, (absent, use_shared) in enumerate((((), True), ((0, E - 1), False))):
                 x16 = synth.normal_fp16((n, hidden), 960 + 10 * n + i, DEV)
                 x16[1:] = x16[0] + (0.05 if i else 0.4) * x16[1:]          # rows that pick much the same experts
                 r0, x0, o0 = run_layer(w, n, k, x16, absent=absent, use_shared=use_shared)
-                r1, x1, o1 = run_layer(w, n, k, x16, absent=absent, use_shared=use_shared, kernel="rows")
-                assert torch.equal(r0.route_idx, r1.route_idx)
-                if on_mma or n == 4:
-                    assert torch.equal(o0.view(torch.int32), o1.view(torch.int32)) and torch.equal(x0.view(torch.int16), x1.view(torch.int16))
-                else:
-                    assert rel(o0.cpu().numpy(), o1.cpu().numpy()) < 1e-5        # another order of the same fp32 terms
+                if n == 4:
+                    r1, x1, o1 = run_layer(w, n, k, x16, absent=absent, use_shared=use_shared, kernel="rows")
+                    assert torch.equal(r0.route_idx, r1.route_idx) and same(o0, o1) and same(x0, x1)
+                    continue
+                for t in range(n):
+                    r1, x1, o1 = run_layer(w, 1, k, x16[t:t + 1], absent=absent, use_shared=use_shared)
+                    assert torch.equal(r0.route_idx[t], r1.route_idx[0]) and same(o0[t], o1[0]) and same(x0[t], x1[0]), (n, i, t)
 
 
 @pytest.mark.parametrize("hidden,n_ff,E,k", [(512, 256, 16, 4), (512, 256, 300, 4), (2048, 512, 64, 8)])
