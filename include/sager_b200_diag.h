@@ -22,6 +22,10 @@ int sgr_tc_set_operand_layout(int layout);
 long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff, int n_expert, int n_used,
                                          int which);
 
+/* How sgr_gemv_q6_k_q8 streams a matrix of k columns (host arithmetic, no device): plan[0] = rows to a stage, plan[1] =
+ * stages of the ring (fewer than 2: always the plain kernel), plan[2] = groups of warps that take the stages in turn. */
+int sgr_gemv_q6_k_plan(int* plan, int k);
+
 /* Residency handle in host-only mode: mark an arena slot as "its copy is still in flight" (what an
  * unfinished event says on the device), so that the rule "an in-flight slot is never evicted" can be
  * exercised without a GPU. */

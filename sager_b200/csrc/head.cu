@@ -15,7 +15,7 @@
 //
 // The head is the largest matrix of a step (151,936 x 2048: 255 MB), so the GEMV is a
 // persistent kernel: one CTA per SM, a producer warp streaming stages of whole rows (1680
-// contiguous bytes each at k = 2048) into a shared-memory ring with bulk copies, two groups of eight
+// contiguous bytes each at k = 2048) into a shared-memory ring with bulk copies, one or, for a ring of four stages, two groups of eight
 // consumer warps of four rows each, which take the stages in turn: what one group waits for - shared-memory loads with two lanes
 // to a bank, chains of dp4a - the other's arithmetic covers (two warps to a scheduler instead of four left its issue slots half
 // empty: 151,936 x 2048 49.2 us, now 42.3; with norm and top-k 64.4 and 58.3). A lane owns a quarter of a block (64 weights, four sub-groups): two
@@ -31,11 +31,13 @@ namespace {
 
 constexpr int kQ6 = 210;                     // bytes per Q6_K super-block
 constexpr int kHeadWarps = 8;                 // warps to a stage
-constexpr int kHeadGroups = 2;                // groups of them, stages in turn
 constexpr int kHeadRows = 4;                  // rows a warp works on at once
-constexpr int kHeadConsumers = kHeadGroups * kHeadWarps;
-constexpr int kHeadThreads = kHeadConsumers * 32 + 32;
 constexpr int kHeadStages = 4;                // at most
+// Groups of kHeadWarps that take the stages in turn. Rings of two or three stages have one: with a stage to a group (and of three stages
+// none a group's own, see the kernel) nothing is on its way to a group while it computes. us of 151,936 rows by one group / by two of two stages: k =
+// 2304 83.2 / 89.8, 2560 85.0 / 92.7, 2816 85.2 / 95.0, 3072 85.2 / 97.2; 2048, four stages, 54.3 / 49.0.
+constexpr int head_groups(int stages) { return stages == kHeadStages ? 2 : 1; }
+constexpr int head_threads(int stages) { return (head_groups(stages) * kHeadWarps + 1) * 32; }
 
 struct HeadArgs {
   const unsigned char* w;
@@ -49,9 +51,12 @@ struct HeadArgs {
 // staged activations: codes [nb][256] int8, 16-column sums [nb][16] int32, scales [nb] fp32
 __host__ __device__ constexpr size_t head_x_bytes(int nb) { return static_cast<size_t>(nb) * (256 + 64 + 4); }
 
-// G lanes to a row: 32, or 16 for rows of up to four blocks; S stages
+// G lanes to a row: 32, or 16 for rows of up to four blocks; S stages. A slot of the ring belongs to one group: a wait by parity tells
+// the phase it is for from the one before only if that one has been waited for, which a group does for its own stages.
 template <int G, int S>
-__global__ void __launch_bounds__(kHeadThreads, 1) gemv_q6_stream_kernel(const HeadArgs a) {
+__global__ void __launch_bounds__(head_threads(S), 1) gemv_q6_stream_kernel(const HeadArgs a) {
+  constexpr int kHeadGroups = head_groups(S), kHeadConsumers = kHeadGroups * kHeadWarps;
+  static_assert(S % kHeadGroups == 0, "no slot passes from one group to the other");
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);
   uint64_t* empty = full + kHeadStages;
@@ -243,7 +248,25 @@ __global__ void gemv_q6_direct_kernel(const HeadArgs a) {
 template <int G, int S>
 int launch_stream(const HeadArgs& a, int sms, size_t smem, cudaStream_t stream) {
   if (!opt_in_smem<gemv_q6_stream_kernel<G, S>>(static_cast<int>(smem))) return kErrLaunch;
-  return launch_pdl(gemv_q6_stream_kernel<G, S>, dim3(sms), kHeadThreads, smem, stream, a);
+  return launch_pdl(gemv_q6_stream_kernel<G, S>, dim3(sms), head_threads(S), smem, stream, a);
+}
+
+struct Q6Plan {
+  int rows, stages;            // rows to a stage, stages of the ring
+  size_t stage_bytes;
+};
+// A stage is what a pass of a group's eight warps takes - 32 rows, or 64 of up to four blocks, which two half-warps share (k =
+// 1024: a lane in two had nothing to do) - as long as two fit; half a pass costs as much as a whole one (k = 4096 with
+// 54 KB stages, 248,320 rows: 261 us with norm and top-k, now 150; k = 1024, by the plain kernel before: 194, now 63). Bulk copies need
+// 16-byte multiples: all stages are, and the last one has to be.
+Q6Plan q6_plan(int nb) {
+  const size_t fixed = 128 + head_x_bytes(nb), room = fixed < 227 * 1024 ? 227 * 1024 - fixed : 0;
+  const int row_bytes = nb * kQ6, fit = static_cast<int>((room / 2 < 128 ? 0 : room / 2 - 127) / row_bytes);
+  Q6Plan p{kHeadWarps * kHeadRows * (nb <= 4 ? 2 : 1), 0, 0};
+  if (fit < p.rows) p.rows = fit >= 8 ? fit & ~7 : fit;
+  p.stage_bytes = (static_cast<size_t>(p.rows) * row_bytes + 127) & ~size_t(127);
+  if (p.rows > 0) p.stages = static_cast<int>(std::min<size_t>(kHeadStages, room / p.stage_bytes));
+  return p;
 }
 
 int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStream_t stream) {
@@ -262,29 +285,22 @@ int gemv_q6(const void* w, const void* xq, float* y, int n_rows, int k, cudaStre
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
     return kErrLaunch;
-  // A stage is what a pass of the eight warps takes - 32 rows, or 64 of up to four blocks, which two half-warps share (k =
-  // 1024: a lane in two had nothing to do) - as long as two fit; half a pass costs as much as a whole one (k = 4096 with
-  // 54 KB stages, 248,320 rows: 261 us with norm and top-k, now 150; k = 1024, by the plain kernel before: 194, now 63). Bulk copies need 16-byte multiples: all stages are, and the last one has to be.
   const bool narrow = a.nb <= 4;
-  const size_t fixed = 128 + head_x_bytes(a.nb), room = fixed < 227 * 1024 ? 227 * 1024 - fixed : 0;
-  a.rows_per_stage = kHeadWarps * kHeadRows * (narrow ? 2 : 1);
-  const int fit = static_cast<int>((room / 2 < 128 ? 0 : room / 2 - 127) / row_bytes);
-  if (fit < a.rows_per_stage) a.rows_per_stage = fit >= 8 ? fit & ~7 : fit;
-  const size_t stage_bytes = (static_cast<size_t>(a.rows_per_stage) * row_bytes + 127) & ~size_t(127);
-  const int stages = a.rows_per_stage > 0 ? static_cast<int>(std::min<size_t>(kHeadStages, room / stage_bytes)) : 0;
+  const Q6Plan p = q6_plan(a.nb);
+  a.rows_per_stage = p.rows;
   // Rows per SM from which the ring pays (us, plain kernel / ring: one block 2,500 rows 2.8 / 2.8, 1,000 rows 2.3 / 2.9; two
   // blocks 2,500 rows 2.8 / 3.1, 3,000 rows 3.4 / 3.2; four blocks 1,000 rows 3.1 / 3.4, 1,500 rows 3.5 / 3.4).
   const int least = a.nb <= 2 ? 18 : (narrow ? 8 : 4);
-  const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && stages >= 2 && n_rows >= least * sms &&
+  const bool streamable = (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && p.stages >= 2 && n_rows >= least * sms &&
                           static_cast<long long>(a.rows_per_stage) * row_bytes % 16 == 0 &&
                           static_cast<long long>(n_rows % a.rows_per_stage) * row_bytes % 16 == 0;
   if (!streamable) return launch_pdl(gemv_q6_direct_kernel, dim3((n_rows + 7) / 8), 256, 0, stream, a);
-  const size_t smem = fixed + stages * stage_bytes;
+  const size_t smem = 128 + head_x_bytes(a.nb) + p.stages * p.stage_bytes;
   static_assert(kHeadStages == 4 && 128 + head_x_bytes(4) + 4 * ((kHeadWarps * kHeadRows * 2 * 4 * kQ6 + 127) / 128 * 128) <= 227 * 1024,
                 "four stages of narrow rows fit, and so do those of fewer blocks");
   if (narrow) return launch_stream<16, 4>(a, sms, smem, stream);
-  if (stages == 4) return launch_stream<32, 4>(a, sms, smem, stream);
-  return stages == 3 ? launch_stream<32, 3>(a, sms, smem, stream) : launch_stream<32, 2>(a, sms, smem, stream);
+  if (p.stages == 4) return launch_stream<32, 4>(a, sms, smem, stream);
+  return p.stages == 3 ? launch_stream<32, 3>(a, sms, smem, stream) : launch_stream<32, 2>(a, sms, smem, stream);
 }
 
 // ---- two-phase top-k ---------------------------------------------------------------------
@@ -751,6 +767,15 @@ SGR_API int sgr_gemv_q6_k_q8(const void* w_q6, const void* x_q8, float* y, int n
 
 // cuda_ops.hpp:181-182 of the reference: the variant with the activations staged in shared memory.
 // Here every path stages them; the two entry points are the same kernel and agree to the bit.
+SGR_API int sgr_gemv_q6_k_plan(int* plan, int k) {
+  if (!plan || k <= 0 || k % kQK != 0) return kErrArg;
+  const Q6Plan p = q6_plan(k / kQK);
+  plan[0] = p.rows;
+  plan[1] = p.stages;
+  plan[2] = head_groups(p.stages);
+  return kOk;
+}
+
 SGR_API int sgr_gemv_q6_k_q8_smx(const void* w_q6, const void* x_q8, float* y, int n_rows, int k, void* stream) {
   return gemv_q6(w_q6, x_q8, y, n_rows, k, as_stream(stream));
 }

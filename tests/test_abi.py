@@ -38,6 +38,21 @@ def test_argument_validation_needs_no_gpu():
     assert lib.raw("sgr_tc_scratch_elems")(512, 2048) == 512 * 2048
 
 
+def test_head_ring_slots_belong_to_one_group_of_warps():
+    """A wait by parity tells a phase from the one before only if that one was waited for: the ring's stages are a multiple of the
+    groups that take them in turn, for every row length."""
+    lib, plan, depths = capi.lib(), (C.c_int * 3)(), set()
+    for k in range(256, 1 << 17, 256):
+        assert lib.raw("sgr_gemv_q6_k_plan")(plan, k) == 0
+        rows, stages, groups = plan
+        assert stages % groups == 0
+        if stages >= 2:
+            depths.add((stages, groups))
+            assert rows > 0 and stages * ((rows * (k // 256) * 210 + 127) // 128 * 128) + 128 + k // 256 * 324 <= 227 * 1024
+    assert depths == {(2, 1), (3, 1), (4, 2)}
+    assert lib.raw("sgr_gemv_q6_k_plan")(plan, 100) == 1
+
+
 def test_prefill_chunk_refuses_unaligned_buffers():
     """What the launchers of the sequence refuse, the one call refuses, and before anything is launched."""
     lib = capi.lib()

@@ -2,6 +2,8 @@
 topk_select_f32_2p of the reference: src/kernels/cuda/q4_k.cu:1564-1658, src/kernels/cuda/mmq.cu:890-986,
 src/kernels/cuda/sampling.cu:162-289). The GEMV is held to the oracle's exact-integer restatement and
 to the reference's own kernels to fp32 rounding; the selection is index work and must be exact."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -53,24 +55,31 @@ def test_q6k_head_gemv(oracle, rows, k):
     assert lib().raw("sgr_status")(0) == 0
 
 
-@pytest.mark.parametrize("k,stages", [(2048, 4), (3072, 3), (4096, 2), (1024, 4)])
-@pytest.mark.parametrize("more", [0, 1, 2])
-def test_q6k_head_stages_go_round_two_groups(oracle, k, stages, more):
-    """Stage counts at which a CTA's two groups of warps have as many stages, or one of them one more or none, for every
-    depth of the ring; the last stage is half of one. Every row, against the oracle: exact integer sums, fp32 terms of a row."""
-    per_stage = 64 if k <= 1024 else 32
+@pytest.mark.parametrize("k,stages,groups", [(2048, 4, 2), (1024, 4, 2), (2304, 3, 1), (2560, 3, 1), (2816, 3, 1), (3072, 2, 1), (4096, 2, 1)])
+@pytest.mark.parametrize("per_cta", [0, 1, 2, 9])
+def test_q6k_head_stages_go_round(oracle, k, stages, groups, per_cta):
+    """Stage counts at which a CTA's two groups of warps have as many stages, or one of them one more or none, and at which every
+    slot of the ring is filled three times at least; the last stage is half of one. Every row, against the oracle: exact
+    integer sums, fp32 terms of a row."""
+    plan = (C.c_int * 3)()
+    lib().call("sgr_gemv_q6_k_plan", plan, k)
+    per_stage = plan[0]
+    assert plan[1] == stages and plan[2] == groups
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    rows = (more * sms + (0 if more else sms // 2)) * per_stage + per_stage // 2
+    rows = (per_cta * sms + (0 if per_cta else sms // 2)) * per_stage + per_stage // 2
+    if per_cta == 9:
+        assert per_cta >= 2 * stages + 1
     rng = np.random.default_rng(rows + k)
     base = make_q6k(rng, 1024, k)
     pick = rng.integers(0, 1024, size=rows)
     w = torch.from_numpy(base).to(DEV)[torch.from_numpy(pick).to(DEV)].contiguous()
     _, x = make_x16(1, k, 5)
     xq = _q8(x, k)
-    y = torch.full((rows,), float("nan"), dtype=torch.float32, device=DEV)
-    ops.gemv_q6_k_q8(w, xq, y, rows, k)
     want = gemv_q6k_q8k(base, xq.cpu().numpy()[0], k)[pick]
-    assert rel(y.cpu().numpy(), want) <= GEMV_TOL
+    for _ in range(3):       # (the next launch's copies start while the last one drains)
+        y = torch.full((rows,), float("nan"), dtype=torch.float32, device=DEV)
+        ops.gemv_q6_k_q8(w, xq, y, rows, k)
+        assert rel(y.cpu().numpy(), want) <= GEMV_TOL
     assert lib().raw("sgr_status")(0) == 0
 
 
