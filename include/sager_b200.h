@@ -45,7 +45,8 @@ extern "C" {
 
 int sgr_abi_version(void);
 /* Device status word of the current device: non-zero after a bounded device-side
- * wait gave up. Synchronises; diagnostics only. clear != 0 resets it. */
+ * wait gave up; the outputs of the call that did are undefined. Synchronises; diagnostics
+ * only. clear != 0 resets it. */
 int sgr_status(int clear);
 
 /* ---- activation quantiser ------------------------------------------------------ */
@@ -228,8 +229,9 @@ int sgr_moe_combine_add_slots_f16(uint16_t* out, const uint16_t* expert_y, const
  * no_residual != 0 out_f32 receives the weighted expert sum alone.
  *
  * The workspace (size from sgr_moe_layer_workspace_bytes, 256-byte aligned) must be
- * cleared once with sgr_moe_layer_workspace_init before its first use; one layer call
- * may be in flight per workspace. */
+ * cleared once with sgr_moe_layer_workspace_init before its first use, and again after a
+ * call on it that raised the status word (its counters stay as that call left them); one
+ * layer call may be in flight per workspace. */
 typedef struct sgr_moe_layer {
   int n;                 /* token rows this call, 1..n_max */
   int n_max;             /* rows the workspace was sized for, <= 64 */

@@ -18,7 +18,9 @@ int sgr_tc_set_operand_layout(int layout);
  * sgr_moe_layer_workspace_bytes), so that a test can read the intermediate rows a finished call
  * left there. which: 0 = fp32 h rows [n_max*K + n_max][n_ff] (routed rows in grouped order, then
  * the shared expert's), 1 = fp32 y rows [..][hidden], 2 = gslot [n_max*K] (route -> grouped row,
- * -1 = not computed), 3 = grows, 4 = plan records, 5 = meta. -1 for a refused geometry. */
+ * -1 = not computed), 3 = grows, 4 = plan records, 5 = meta, 6 = counters (uint32; words 12 and 13 are the 64-bit arrival
+ * counter of the one-launch layers, CTAs that gave up counted in its top byte), 7 = the logits that these exchange
+ * [16 copies][n][n_expert], the launch's number in a word's upper half. -1 for a refused geometry. */
 long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff, int n_expert, int n_used,
                                          int which);
 

@@ -1282,7 +1282,7 @@ SGR_API size_t sgr_moe_layer_workspace_bytes(int n_max, int hidden, int n_ff, in
 
 // Diagnostics (sager_b200_diag.h): where a region of the workspace starts, so that a test can read
 // the intermediate rows a finished call left there. which: 0 fp32 h rows, 1 fp32 y rows, 2 gslot,
-// 3 grows, 4 plan records, 5 meta.
+// 3 grows, 4 plan records, 5 meta, 6 counters, 7 exchanged logits.
 SGR_API long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff, int n_expert, int n_used,
                                                  int which) {
   if (sgr_moe_layer_workspace_bytes(n_max, hidden, n_ff, n_expert, n_used) == 0) return -1;
@@ -1294,6 +1294,8 @@ SGR_API long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff
     case 3: return static_cast<long long>(l.grows);
     case 4: return static_cast<long long>(l.rec);
     case 5: return static_cast<long long>(l.meta);
+    case 6: return static_cast<long long>(l.cnt);
+    case 7: return static_cast<long long>(l.xchg);
     default: return -1;
   }
 }

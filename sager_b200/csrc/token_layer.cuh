@@ -203,16 +203,18 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
   return v;
 }
 // Grid-wide barrier on a 64-bit arrival counter that only ever grows: that of the k-th launch on this
-// workspace completes when the counter reaches k * G. Waits are bounded: false when the others did not arrive in time.
+// workspace completes when the counter reaches k * G. Waits are bounded: false when the others did not arrive in time. A CTA that
+// gives up before the barrier arrives all the same, and counts itself in the word's top byte: the others learn of it when the barrier
+// completes and give up too, and the next launch finds a multiple of the grid, a number of its own and so no logits that it could take for its own.
 // The counter is read by the producer warp when the kernels before this one have finished - some multiple of
 // the grid size plus the arrivals of this launch's CTAs that are already further on, of which one at least is missing, this
-// CTA's own -, so the barrier completes at base + grid. (Read at kernel start, it could lie among the arrivals of a launch before on the
+// CTA's own -, so the barrier completes at the next multiple. (Read at kernel start, it could lie among the arrivals of a launch before on the
 // same workspace, wherever two CTAs fit on one SM.) An arrival is a fire-and-forget releasing add by the thread whose warp
 // finishes the work; the producer warp polls and passes the word on through an mbarrier, so no consumer waits for a round trip
 // that it could work through.
 //
-// The logits go from CTA to CTA without a barrier. A word holds a logit and, above it, base / grid + 1, which no launch before on the
-// workspace had; a warp of each CTA reads a row's words until all have it. Behind a barrier they took two more trips: an
+// The logits go from CTA to CTA without a barrier. A word holds a logit and, above it, the launch's number, which no launch before on the
+// workspace had (in 32 bits: a word would have to be 2^32 launches old); a warp of each CTA reads a row's words until all have it. Behind a barrier they took two more trips: an
 // arrival waits for the stores before it, and the reads begin when the poll returns. There are kXchgCopies of the words, written by
 // as many lanes, and a CTA reads one: 148 readers of the same lines are in the writers' way. us per layer at one row, behind the
 // barrier, then with 1 / 2 / 4 / 8 / 16 copies: hidden 2048, 256 experts 13.8, 14.3 / 13.6 / 13.4 / 13.2 / 13.2; 1024, 128 12.3, 13.8 / 12.7 / 12.7 /
@@ -252,14 +254,19 @@ __device__ __forceinline__ bool get_logits(const unsigned long long* row, unsign
   }
   return false;
 }
-__device__ __forceinline__ void grid_arrive(unsigned long long* ctr) {
-  asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(ctr) : "memory");
+constexpr unsigned long long kGaveUp = 1ull << 56, kArrivals = kGaveUp - 1;       // (a grid has fewer than 256 CTAs)
+static_assert(kMaxGrid < 256, "the top byte counts the CTAs of a launch that gave up");
+__device__ __forceinline__ void grid_arrive(unsigned long long* ctr, bool ok) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(ctr), "l"(ok ? 1ull : kGaveUp + 1) : "memory");
 }
-__device__ __forceinline__ bool grid_wait(const unsigned long long* ctr, unsigned long long target) {
+// Launch k + 1's barrier; `gave_up` is the top byte as it was at the launch's start.
+__device__ __forceinline__ bool grid_wait(const unsigned long long* ctr, unsigned long long k, unsigned grid, unsigned gave_up) {
+  const unsigned long long target = (k + 1) * grid;
   unsigned it = 0;
-  while (ld_acquire_u64(ctr) < target && ++it < kSpinLimit) {
+  unsigned long long v;
+  while (((v = ld_acquire_u64(ctr)) & kArrivals) < target && ++it < kSpinLimit) {
   }
-  return it < kSpinLimit;
+  return it < kSpinLimit && static_cast<unsigned>(v >> 56) == gave_up;
 }
 
 // One warp: eight values per lane of a 256-value block -> Q8_K codes, sums and scale in a tile
@@ -555,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
   uint64_t* dn_full = shdn_full + 1;                               // [2] routed tiles' down rows, rounds in turn
   uint64_t* dn_empty = dn_full + 2;                                // [2]
   uint64_t* ready = dn_empty + 2;                                  // tables built
-  uint64_t* based = ready + 1;                                     // the grid counter has been read: flag[0] is base / grid + 1
+  uint64_t* based = ready + 1;                                     // the grid counter has been read: flag[0] is the launch's number
   uint64_t* passed = based + 1;                                    // grid barrier passed (or given up), one phase each
   StageDesc* desc = reinterpret_cast<StageDesc*>(smem + 128);      // [kRing]
   int* flag = reinterpret_cast<int*>(smem + 256);
@@ -672,12 +679,14 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
         }
       }
     }
-    // (an earlier launch on this workspace may still be between its two barriers until now)
+    // (an earlier launch on this workspace may still be at its barrier until now)
     pdl_wait();
-    unsigned long long bar_base = 0;
+    unsigned long long k = 0;                    // launches before this one
+    unsigned gave_up = 0;
     if (lane == 0) {
-      const unsigned long long k = ld_acquire_u64(gctr) / grid;
-      bar_base = k * grid;
+      const unsigned long long word = ld_acquire_u64(gctr);
+      k = (word & kArrivals) / grid;
+      gave_up = static_cast<unsigned>(word >> 56);
       flag[0] = static_cast<int>(static_cast<unsigned>(k) + 1u);
       __threadfence_block();
       mbar_arrive_one(based);
@@ -800,7 +809,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
       issue_down_round(round++);
     }
     if (lane == 0) {                                // the barrier's outcome goes to flag[1]
-      flag[1] = grid_wait(gctr, bar_base + grid) ? 1 : 0;
+      flag[1] = grid_wait(gctr, k, grid, gave_up) ? 1 : 0;
       __threadfence_block();
       mbar_arrive_one(passed);
     }
@@ -1031,7 +1040,10 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     }
   }
   if (!consumers_all(ok)) {
-    if (tid == 0) atomicExch(L.status, 5);
+    if (tid == 0) {
+      atomicExch(L.status, 5);
+      grid_arrive(gctr, false);
+    }
     return;
   }
   if (!by_pairs || *reinterpret_cast<volatile int*>(flag + 2) != 0) {
@@ -1091,7 +1103,7 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     }
   }
   ok = consumers_all(ok);                                   // (a wait that ran out in any thread ends the CTA's work)
-  if (tid == 0) grid_arrive(gctr);
+  if (tid == 0) grid_arrive(gctr, ok);
 
   // ---- phase 4: quantise h (all rows, from L2), down rows of this CTA, combine in place ----
   const HTile hq = {smem + G.off_xh, L.nbf};

@@ -38,12 +38,16 @@ class MoeLayerRunner:
             raise ValueError("geometry refused by sgr_moe_layer_workspace_bytes")
         self.ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
         assert self.ws.data_ptr() % 256 == 0
-        with torch.cuda.device(device):
-            L.call("sgr_moe_layer_workspace_init", _p(self.ws), nbytes, stream_ptr())
+        self.clear_workspace()
         self.route_idx = torch.zeros(n_max, n_used + 1, dtype=torch.int32, device=device)
         self.route_w = torch.zeros(n_max, n_used + 1, dtype=torch.float32, device=device)
         self.mail = torch.zeros(n_expert, dtype=torch.int32, device=device)
         self.mail_n = torch.zeros(1, dtype=torch.int32, device=device)
+
+    def clear_workspace(self):
+        """Before the first call, and after one that raised the status word."""
+        with torch.cuda.device(self.device):
+            lib().call("sgr_moe_layer_workspace_init", _p(self.ws), self.ws.numel(), stream_ptr())
 
     def args(self, n, xn, router_w, w_tab, shared_ptrs, x_f16=None, out_f32=None, bias=None,
              shared_w=1.0, xq_in=None, routing_given=False, no_residual=False, shared_lo=0,

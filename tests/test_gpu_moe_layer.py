@@ -629,6 +629,35 @@ def test_one_workspace_through_changing_row_counts(hidden, n_ff, E, k):
     assert lib().raw("sgr_status")(0) == 0
 
 
+@pytest.mark.parametrize("hidden,n_ff,E,k", [(512, 256, 16, 4), (512, 256, 300, 4), (2048, 512, 64, 8)])
+def test_one_launch_layer_after_one_that_gave_up(hidden, n_ff, E, k):
+    """A launch whose waits ran out leaves logits with its number behind and the arrival counter at a multiple of the grid, the
+    CTAs that gave up counted in the top byte (written here by the host). The next launch has a number of its own: it
+    takes none of those logits, and what was counted before is not its own failure."""
+    w = synth.MoeWeights(hidden, n_ff, E, DEV, seed=98, std=0.05)
+    grid = min(torch.cuda.get_device_properties(0).multi_processor_count, 160)
+    offset = lib().raw("sgr_moe_layer_workspace_offset")
+    for n in (1, 3):
+        runner = MoeLayerRunner(4, hidden, n_ff, E, k, DEV)
+        at, words = offset(4, hidden, n_ff, E, k, 6) + 48, offset(4, hidden, n_ff, E, k, 7)
+        counter = runner.ws[at:at + 8].view(torch.int64)
+        logits = runner.ws[words:words + 16 * n * E * 8].view(torch.int32).view(-1, 2)     # value, number
+        x16 = synth.normal_fp16((n, hidden), 980 + n, DEV)
+        outs = []
+        for launch in range(3):
+            out = torch.zeros(n, hidden, dtype=torch.float32, device=DEV)
+            runner.run(runner.args(n, x16, w.router, w.table(), w.shared_ptrs(), x_f16=x16.clone(), out_f32=out))
+            torch.cuda.synchronize()
+            gave_up = 0 if launch == 0 else 3 * launch << 56
+            assert counter.item() == (2 * launch + 1) * grid + gave_up and torch.all(logits[:, 1] == 2 * launch + 1)
+            outs.append((out, runner.route_idx[:n].clone(), runner.route_w[:n].clone()))
+            counter += grid + (3 << 56)                              # the launch that gives up: three of its CTAs
+            logits[:, 0] = torch.randperm(logits.shape[0], device=DEV).to(torch.float32).view(torch.int32)
+            logits[:, 1] += 1
+        assert all(torch.equal(a, b) for o in outs[1:] for a, b in zip(outs[0], o)), n
+    assert lib().raw("sgr_status")(0) == 0
+
+
 def test_four_rows_on_a_workspace_for_the_item_kernel(full_w):
     """A workspace too small for the row-streaming kernel keeps four rows on the item kernel and its order of the sums."""
     x16 = synth.normal_fp16((4, full_w.hidden), 870, DEV)
