@@ -28,6 +28,11 @@ long long sgr_moe_layer_workspace_offset(int n_max, int hidden, int n_ff, int n_
  * stages of the ring (fewer than 2: always the plain kernel), plan[2] = groups of warps that take the stages in turn. */
 int sgr_gemv_q6_k_plan(int* plan, int k);
 
+/* How sgr_tc_gemm_q4_k_f16 splits a product over `sms` SMs (host arithmetic, no device): plan[0] = CTAs that share a unit (1, or 2 of a
+ * cluster), [1] = token rows of a unit, [2] = token tiles, [3] = units, [4] = CTAs that work on them, [5] = CTAs per row tile that only
+ * write the scratch, [6] = the scratch is written by the dequantisation kernel ahead. */
+int sgr_tc_gemm_q4_k_plan(int* plan, int sms, int n_rows, int k, int n_tokens);
+
 /* Residency handle in host-only mode: mark an arena slot as "its copy is still in flight" (what an
  * unfinished event says on the device), so that the rule "an in-flight slot is never evicted" can be
  * exercised without a GPU. */

@@ -260,7 +260,8 @@ __device__ __forceinline__ uint4 dequant_octet(const unsigned char* blk, int lan
 //   * warp 18: tensor memory and (a pair's first CTA) MMA issue
 // 4096 x 2048 over 2048 rows (MMAs 16 us at two units each, 20.8 at the library's rate): 38.5 us with a CTA per unit, whose start and epilogue
 // nothing covered, 32.8 persistent and in pairs, 31.8 with the weights by TMA (one warp's cp.async, 36 to a block with a division
-// each, took longer than the block: 130 x 4096 over 333 rows 28 -> 21), 31.2 with four slots instead of three. Bound now by the hand-overs
+// each, took longer than the block: 130 x 4096 over 333 rows 28 -> 21), 31.2 with four slots instead of three (those with pairs of N = 240; inputs from HBM
+// 37.9, and 38.4 with the N = 256 that mma_columns asks for). Bound now by the hand-overs
 // of a block, about 2,000 cycles where the MMAs of 256 columns need 2,080, and the scratch, 3.5 us.
 // `scratch` receives the dequantised rows: with few units by CTAs of their own on the SMs left over (a thread's 16-byte pieces of
 // its row take longer than its block: 1000 x 4096 over 75 rows 33.8 -> 22.6 us, over 64 rows 54.5 -> 22.5), else each token
@@ -282,6 +283,12 @@ __device__ __forceinline__ void dequant_word(uint32_t raw, uint32_t mask, f32x2 
   v01 = h2_bits(__floats2half2_rn(part2(f01, 0), part2(f01, 1)));
   v23 = h2_bits(__floats2half2_rn(part2(f23, 0), part2(f23, 1)));
 }
+
+// Columns of an MMA over n tokens: M = 128 of one CTA takes any multiple of 16, a pair's M = 256 with A in tensor memory multiples of 32 (what
+// CUTLASS's SM100_MMA_F16BF16_2x1SM_TS asserts). The tokens past a tile's end are the next tile's or, past the matrix, zeros; their sums are
+// not stored.
+template <int CG>
+__host__ __device__ constexpr int mma_columns(int n) { return (n + 16 * CG - 1) / (16 * CG) * (16 * CG); }
 
 struct Q4Args {
   const unsigned char* w;
@@ -474,7 +481,7 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     pdl_wait();
     if (lane == 0) {
       for_units([&](int, int tok0, int ntok, int) {
-        const int from = tok0 + static_cast<int>(rank) * (max(16, (ntok + 15) & ~15) >> 1);
+        const int from = tok0 + static_cast<int>(rank) * (mma_columns<CG>(ntok) >> 1);
         for (int kb = 0; kb < 4 * nb; ++kb) {
           if (!mbar_wait_tight(&bar[kQ4BEmpty + s], ph)) {
             *fail = 1;
@@ -513,7 +520,7 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
       int slot = 0, s = 0;
       unsigned slot_ph = 0, s_ph = 0, acc_ph = 1;
       for_units([&](int, int, int ntok, int) {
-        const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc_f16(max(16, (ntok + 15) & ~15), 128 * CG), 0);
+        const uint32_t idesc = __shfl_sync(0xFFFFFFFFu, umma_idesc_f16(mma_columns<CG>(ntok), 128 * CG), 0);
         if (!wait_warp(kQ4AccEmpty, acc_ph)) return false;
         acc_ph ^= 1u;
         for (int x = 0; x < 2 * nb; ++x) {        // half-blocks
@@ -691,36 +698,39 @@ int launch_dequant(const void* w, void* out16, long long n_blocks, cudaStream_t 
   return cudaPeekAtLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
-int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratch, int n_rows, int k, int n_tokens, cudaStream_t s) {
-  if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(y) & 1u)) return kErrAlign;
-  const int sms = device_sms(), row_tiles = (n_rows + 127) / 128, nb = k / kQK;
-  if (sms <= 0) return kErrLaunch;
-  // Token rows per unit, CTAs that share a unit, and who writes the scratch: what takes the least by estimates in us, fitted to
-  // 27 shapes (4096 x 2048 over 2048 tokens: units of a pair's 256 rows x 240 tokens 31 us, 45 with 128
-  // tokens, 33 by single CTAs; 1000 x 2048 over 777: 12.0). Against a CTA per unit only short rows come near: 2048 x 512 over 1457 / 700
-  // tokens 8.9 / 6.5 us for 8.7 / 6.4.
-  //   the start, 4, and the last unit's epilogue, 3 for 256 tokens (without it, and with a row tile's scratch in equal parts and not in whole
-  //     blocks, 512 x 512 over 400 / 1457 tokens 6.6 / 7.1 us for 5.0 / 5.5, 2048 x 2048 over 512 12.9 for 12.5)
-  //   a block column of a unit: 1.0 and, with the square of its tokens, up to 0.35 more, a fifth more when every SM works; a pair
-  //     brings half of the activations per CTA and gains a twentieth past 128 tokens, but costs 0.3 to set up
-  //   the scratch, per block of a row tile: SMs that the units leave idle, in whole columns of row tiles, 3.2 / spare beside
-  //     the units' 1.3 and epilogue (2048 x 512 over 2048 tokens 10.9 -> 9.7); the units of a row tile themselves, 2 for each block that one
-  //     of its token tiles writes on top of it; or the dequantisation kernel ahead of the
-  //     GEMM, 2.5 us and the bytes at 5 TB/s (8192 x 4096 over 64 tokens: 53 us by one spare column, 41 by the kernel ahead).
-  struct Plan { int cg, bn, tiles, units, workers, spare; bool ahead; double us; } p{};
+struct Q4Plan {
+  int cg, bn, tiles, units, workers, spare;      // CTAs to a unit, its token rows, token tiles, units, CTAs that work on them, CTAs per row tile for the scratch
+  bool ahead;                                    // the scratch is written by the dequantisation kernel
+  double us;
+};
+// Token rows per unit, CTAs that share a unit, and who writes the scratch: what takes the least by estimates in us, fitted to
+// 27 shapes (4096 x 2048 over 2048 tokens, inputs from HBM: units of a pair's 256 rows x 256 tokens 38.9 us, 224 tokens 45.0, a single CTA's 128 rows
+// x 240 / 256 tokens 39.7 / 41.0; 4096 x 4096 63.2, 64.2 and 66.9).
+//   the start, 4, and the last unit's epilogue, 3 for 256 tokens (without it, and with a row tile's scratch in equal parts and not in whole
+//     blocks, 512 x 512 over 400 / 1457 tokens 6.6 / 7.1 us for 5.0 / 5.5, 2048 x 2048 over 512 12.9 for 12.5)
+//   a block column of a unit: 1.0 and, with the square of its tokens, up to 0.35 more, a fifth more when every SM works; a pair
+//     brings half of the activations per CTA and gains 6 % past 128 tokens, but costs 0.3 to set up
+//   the scratch, per block of a row tile: SMs that the units leave idle, in whole columns of row tiles, 3.2 / spare beside
+//     the units' 1.3 and epilogue (2048 x 512 over 2048 tokens 10.9 -> 9.7); the units of a row tile themselves, 2 for each block that one
+//     of its token tiles writes on top of it; or the dequantisation kernel ahead of the
+//     GEMM, 2.5 us and the bytes at 5 TB/s (8192 x 4096 over 64 tokens: 53 us by one spare column, 41 by the kernel ahead).
+Q4Plan q4_plan(int sms, int n_rows, int k, int n_tokens) {
+  const int row_tiles = (n_rows + 127) / 128, nb = k / kQK;
+  Q4Plan p{};
   for (int cg = 1; cg <= (row_tiles > 1 ? 2 : 1); ++cg) {
     for (int most = 256, last = 0; most >= 32; most -= 16) {
-      const int t = (n_tokens - 1) / most + 1, bn = ((n_tokens - 1) / t + 16) & ~15;      // tiles of nearly equal length
+      const int t = (n_tokens - 1) / most + 1, each = (n_tokens - 1) / t + 1;            // tiles of nearly equal length
+      const int bn = cg == 1 ? mma_columns<1>(each) : mma_columns<2>(each);
       if (bn == last) continue;
       last = bn;
-      Plan c{cg, bn, (n_tokens + bn - 1) / bn, 0, 0, 0, false, 0.};
+      Q4Plan c{cg, bn, (n_tokens + bn - 1) / bn, 0, 0, 0, false, 0.};
       const long long units = static_cast<long long>((row_tiles + cg - 1) / cg) * c.tiles;
       if (units > 0x3FFFFFFF) continue;
       c.units = static_cast<int>(units);
       c.workers = std::min(c.units, sms / cg) * cg;
       const int waves = (c.units * cg + c.workers - 1) / c.workers;
       const double wide = bn / 256.;
-      c.us = 4 + 3 * wide + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.05 : 1.);
+      c.us = 4 + 3 * wide + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.06 : 1.);
       const int spare = std::min(nb, (sms - c.workers) / row_tiles);
       const double by_spare = spare > 0 ? std::max(0., nb * (3.2 / spare - 1.3) - 3 * wide) : 1e30, by_tiles = 2. * ((nb + c.tiles - 1) / c.tiles);
       const double by_kernel = 2.5 + static_cast<double>(n_rows) * k * 2.5625 / 5e6;
@@ -733,6 +743,14 @@ int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratc
       if (p.cg == 0 || c.us < p.us) p = c;
     }
   }
+  return p;
+}
+
+int launch_tc_q4(const void* w, const uint16_t* x, uint16_t* y, uint16_t* scratch, int n_rows, int k, int n_tokens, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) || (reinterpret_cast<uintptr_t>(y) & 1u)) return kErrAlign;
+  const int sms = device_sms(), row_tiles = (n_rows + 127) / 128, nb = k / kQK;
+  if (sms <= 0) return kErrLaunch;
+  const Q4Plan p = q4_plan(sms, n_rows, k, n_tokens);
   if (p.cg == 0) return kErrUnsupported;
   CUtensorMap mx, mw;
   if (!weight_map(&mw, w, n_rows, k) || !operand_map(&mx, x, n_tokens, k, kLayoutSwizzled, p.bn / p.cg)) return kErrUnsupported;
@@ -804,6 +822,15 @@ SGR_API int sgr_tc_gemm_q4_k_f16(const void* w, const uint16_t* x, uint16_t* y, 
   if (reinterpret_cast<uintptr_t>(w) & 15u) return kErrAlign;
   if (reinterpret_cast<uintptr_t>(scratch) & 15u) return kErrAlign;
   return launch_tc_q4(w, x, y, scratch, n_rows, k, n_tokens, as_stream(stream));
+}
+
+SGR_API int sgr_tc_gemm_q4_k_plan(int* plan, int sms, int n_rows, int k, int n_tokens) {
+  if (!plan || sms <= 0 || n_rows <= 0 || n_tokens <= 0 || k < kQK || k % kQK != 0) return kErrArg;
+  const Q4Plan p = q4_plan(sms, n_rows, k, n_tokens);
+  if (p.cg == 0) return kErrUnsupported;
+  const int v[7] = {p.cg, p.bn, p.tiles, p.units, p.workers, p.spare, p.ahead};
+  std::memcpy(plan, v, sizeof(v));
+  return kOk;
 }
 
 SGR_API int sgr_dequant_experts_q4_k_f16(const void* const* tab_a, const void* const* tab_b, const int* off,

@@ -53,6 +53,24 @@ def test_head_ring_slots_belong_to_one_group_of_warps():
     assert lib.raw("sgr_gemv_q6_k_plan")(plan, 100) == 1
 
 
+def test_projection_plans_are_shapes_that_the_tensor_cores_take():
+    """M = 128 with N a multiple of 16 for one CTA, M = 256 with N a multiple of 32 for a pair; every token in one tile; whole pairs."""
+    lib, plan, seen = capi.lib(), (C.c_int * 7)(), set()
+    for sms in (148, 132, 7):
+        for rows in (1, 128, 129, 1000, 2048, 3201, 4096, 8192, 100000):
+            for k in (256, 512, 2048, 8192):
+                for tok in (*range(1, 100, 9), 255, 256, 257, 300, 512, 777, 1154, 1457, 2047, 2048, 2049, 5000, 70001):
+                    assert lib.raw("sgr_tc_gemm_q4_k_plan")(plan, sms, rows, k, tok) == 0
+                    cg, bn, tiles, units, workers, spare, ahead = plan
+                    row_tiles = (rows + 127) // 128
+                    assert cg in (1, 2) and bn % (16 * cg) == 0 and 16 * cg <= bn <= 256
+                    assert (tiles - 1) * bn < tok <= tiles * bn and units == (row_tiles + cg - 1) // cg * tiles
+                    assert workers % cg == 0 and cg <= workers <= min(sms // cg * cg, units * cg)
+                    assert workers + spare * row_tiles <= sms and not (ahead and spare)
+                    seen.add(cg)
+    assert seen == {1, 2}
+
+
 def test_prefill_chunk_refuses_unaligned_buffers():
     """What the launchers of the sequence refuse, the one call refuses, and before anything is launched."""
     lib = capi.lib()

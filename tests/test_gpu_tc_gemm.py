@@ -189,15 +189,27 @@ def test_q4k_gemm_few_rows_past_a_tile(rows):
     assert rel(y[:tok].float().cpu().numpy(), gemm_want(w16, x_dev).cpu().numpy()) < 1e-3 and torch.all(y[tok] == 9.0)
 
 
-@pytest.mark.parametrize("rows,k,tok", [
-    (4224, 1024, 2040),      # CTA pairs over an odd number of row tiles, two units each, a ragged last token tile
-    (2176, 4096, 1000),      # pairs, one unit each, the scratch by CTAs of their own
-    (3201, 1024, 2048),      # pairs, odd rows: no paired stores
-    (4224, 256, 1555),       # single CTAs, two units each, one block to a row
-    (4096, 512, 2047),       # the units of a CTA start on even and odd blocks of the rings alike
+@pytest.mark.parametrize("rows,k,tok,cg,says", [
+    (4224, 1024, 2040, 2, "waves odd_row_tiles ragged"),
+    (2176, 4096, 1000, 2, "odd_row_tiles spare ragged"),
+    (3201, 1024, 2048, 2, "waves odd_rows"),             # no paired stores
+    (4096, 4096, 1282, 2, "short_tail"),                 # a pair's last units have 2 tokens,
+    (1000, 4096, 1926, 2, "short_tail spare"),           # ... 6, beside CTAs for the scratch
+    (4096, 4096, 1296, 2, "short_tail"),                 # ... 16
+    (4096, 2048, 2048, 2, "waves"),
+    (4096, 2048, 1027, 1, "waves short_tail"),
+    (4224, 256, 1555, 1, "waves"),                       # one block to a row
+    (4096, 512, 2047, 1, "waves"),                       # the units of a CTA start on even and odd blocks of the rings alike
 ])
-def test_q4k_gemm_units(rows, k, tok):
+def test_q4k_gemm_units(rows, k, tok, cg, says):
     """Several units to a CTA, units of CTA pairs, and what lies past the matrix in them."""
+    plan = (C.c_int * 7)()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    lib().call("sgr_tc_gemm_q4_k_plan", plan, sms, rows, k, tok)
+    bn, tiles, units, workers, spare, row_tiles = *plan[1:6], (rows + 127) // 128
+    tail = tok - (tiles - 1) * bn
+    is_so = dict(waves=units * cg > workers, odd_row_tiles=row_tiles % 2 == 1, odd_rows=rows % 2 == 1, ragged=tail < bn, spare=spare > 0, short_tail=tail <= 16)
+    assert plan[0] == cg and all(is_so[s] for s in says.split())
     w_np, w_dev = make_q4k(rows, k, 33)
     x_np, x_dev = make_x16(tok, k, 34)
     scratch = torch.zeros(rows * k + 8, dtype=torch.float16, device=DEV)
