@@ -18,7 +18,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libsager_b200.so")
-FASTCALL = os.path.join(HERE, "_fastcall.so")
+FASTCALL = os.path.join(HERE, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))      # (another interpreter does not load it)
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -52,10 +52,16 @@ def _obj(src):
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(FASTCALL):
-        return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(FASTCALL))
-    return any(os.path.getmtime(p) > t for p in sources() + headers() + [os.path.join(CSRC, "fastcall.c")])
+    return _older(LIB, sources() + headers())
+
+
+def _older(path, than) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(p) > os.path.getmtime(path) for p in than)
+
+
+def needs_fastcall() -> bool:
+    """The module's functions come from the headers by way of capi.py and this file."""
+    return _older(FASTCALL, headers() + [os.path.join(CSRC, "fastcall.c"), os.path.join(HERE, "capi.py")])
 
 
 def fastcall_calls() -> str:
@@ -87,13 +93,16 @@ def fastcall_calls() -> str:
 
 
 def build_fastcall() -> None:
+    """Without a C compiler or Python's headers there is no module, and ops.py makes its calls through ctypes."""
+    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
+    include = sysconfig.get_paths()["include"]
+    if cc is None or not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write("sager_b200: no C compiler or no Python.h; calls from Python go through ctypes\n")
+        return
     os.makedirs(OBJ, exist_ok=True)
     with open(os.path.join(OBJ, "fastcall_calls.inc"), "w") as f:
         f.write(fastcall_calls())
-    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
-    if cc is None:
-        raise RuntimeError("no C compiler found")
-    cmd = [cc, "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I", sysconfig.get_paths()["include"], "-I", OBJ,
+    cmd = [cc, "-O2", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I", include, "-I", OBJ,
            "-o", FASTCALL + ".tmp", os.path.join(CSRC, "fastcall.c"), "-lpthread"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
@@ -103,8 +112,14 @@ def build_fastcall() -> None:
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB
+    if force or needs_build():
+        build_lib(force, verbose, ptxas_info)
+    if force or needs_fastcall():
+        build_fastcall()
+    return LIB
+
+
+def build_lib(force: bool, verbose: bool, ptxas_info: bool) -> None:
     os.makedirs(OBJ, exist_ok=True)
     nvcc = nvcc_path()
     hdr_t = max(os.path.getmtime(p) for p in headers())
@@ -145,8 +160,6 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError("link failed")
     os.replace(LIB + ".tmp", LIB)          # a reader never sees a half-written library
-    build_fastcall()
-    return LIB
 
 
 if __name__ == "__main__":

@@ -34,18 +34,23 @@ _fast = None
 
 
 def _fastcall():
-    """The extension module that makes the calls (csrc/fastcall.c)."""
+    """The extension module that makes the calls (csrc/fastcall.c); False where it was not built for this interpreter."""
     global _fast
     if _fast is None:
-        from . import _fastcall
-        _fastcall.setup(torch.Tensor, torch.nn.Parameter, _stream, _raw_stream, _device)
-        _fast = _fastcall
+        try:
+            from . import _fastcall
+        except ImportError:
+            _fast = False
+        else:
+            _fastcall.setup(torch.Tensor, torch.nn.Parameter, _stream, _raw_stream, _device)
+            _fast = _fastcall
     return _fast
 
 
 def _bind(name: str):
     """The entry point as a callable: tensors go as device addresses, the current stream last. A decode step issues
-    hundreds of these: the extension module makes the call; `slow` takes the arguments that it does not know."""
+    hundreds of these: the extension module makes the call; `slow` takes the arguments that it does not know, and parameter
+    lists that it was not built with."""
     L = lib()
     cfn = getattr(L.cdll, "sgr_" + name)
     tensor, stream = torch.Tensor, _stream
@@ -60,7 +65,9 @@ def _bind(name: str):
 
     slow.__name__ = name
     kinds = kinds_of(L.protos["sgr_" + name])
-    return slow if kinds is None else _fastcall().bind(kinds, C.cast(cfn, C.c_void_p).value, slow, fail, name)
+    fast = None if kinds is None else _fastcall()
+    fn = fast.bind(kinds, C.cast(cfn, C.c_void_p).value, slow, fail, name) if fast else None
+    return slow if fn is None else fn
 
 
 def call(name: str, *args):

@@ -1,10 +1,14 @@
 """The extension module that makes the launch calls: what it takes, it passes as the Python function does; the
 rest it hands to that function. A host callback stands in for the entry point."""
 import ctypes as C
+import os
+import sys
+import sysconfig
 
 import pytest
 import torch
 
+import sager_b200
 from sager_b200 import _fastcall, build, capi, ops
 
 KINDS = "pipfiqzdp"                   # (not a list of the header's: every kind of parameter once, generated below)
@@ -77,6 +81,41 @@ def test_a_return_code_raises(bound):
     with pytest.raises(capi.SagerError) as e:
         fn(0, 0, 0, 0, 1, 0.5, 1)
     assert e.value.code == 2 and len(seen) == 1
+
+
+@pytest.mark.parametrize("module", ["missing", "older"])
+def test_without_the_module_or_its_function_the_python_function_is_the_launcher(monkeypatch, module):
+    class Older:
+        setup, bind = staticmethod(_fastcall.setup), staticmethod(lambda *a: None)      # (what bind says to a list it does not have)
+
+    monkeypatch.setattr(ops, "_fast", None)
+    monkeypatch.delattr(sager_b200, "_fastcall")
+    monkeypatch.setitem(sys.modules, "sager_b200._fastcall", None if module == "missing" else Older)
+    if module == "older":
+        monkeypatch.setattr(sager_b200, "_fastcall", Older, raising=False)
+    fn = ops._bind("gemv_q4_k_q8")
+    assert type(fn) is type(ops.call) and fn.__name__ == "gemv_q4_k_q8"
+    monkeypatch.setattr(ops, "_raw_stream", lambda dev: 0)
+    monkeypatch.setattr(ops, "_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "is_initialized", lambda: True)
+    assert fn(16, 16, 16, 0, 2048) is None                             # empty: nothing to do
+    with pytest.raises(capi.SagerError) as e:
+        fn(None, None, None, 8, 2048)
+    assert e.value.code == 1
+
+
+def test_the_module_is_this_interpreters_and_follows_its_sources(monkeypatch, tmp_path):
+    assert build.FASTCALL.endswith(sysconfig.get_config_var("EXT_SUFFIX")) and os.path.samefile(_fastcall.__file__, build.FASTCALL)
+    copy = tmp_path / "module"
+    copy.write_bytes(b"")
+    monkeypatch.setattr(build, "FASTCALL", str(copy))
+    newest = max(os.path.getmtime(p) for p in build.headers() + [os.path.join(build.CSRC, "fastcall.c"), os.path.join(build.HERE, "capi.py")])
+    os.utime(copy, (newest, newest))
+    assert not build.needs_fastcall()
+    os.utime(copy, (newest, os.path.getmtime(os.path.join(build.HERE, "capi.py")) - 1))
+    assert build.needs_fastcall()
+    os.remove(copy)
+    assert build.needs_fastcall()
 
 
 def test_every_launcher_has_one():
