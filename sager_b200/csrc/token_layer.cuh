@@ -985,6 +985,11 @@ __global__ void __launch_bounds__(kThreads, 1) token_layer_kernel(const LayerDev
     float v[8] = {};                             // (one row) this lane's logits
     bool there = true;
     if (warp < kMaxTok) {
+      // A CTA without a router row would read from here on, before there can be a logit, and its reads of the lines that a few
+      // CTAs are about to write slow those down. us per layer at 1 / 2 / 3 / 4 rows of 512 / 256 / 16, weights in L2: behind a barrier 11.35 / 13.3 /
+      // 14.2 / 15.05, words 11.1 / 13.1 / 14.2 / 15.4, with the pause 10.7 / 12.9 / 13.9 / 14.8 (300 to 800 ns within 0.1, launches one by one gain
+      // 0.15 more from 600 on; 256 / 256 / 8, one row: 11.3, 10.1, and 10.2 at 500, 10.5 at 800 ns).
+      if (cta >= E) __nanosleep(600);
       there = __all_sync(0xFFFFFFFFu, mbar_wait(based, 0)) &&
               get_logits<8>(row, static_cast<unsigned>(*reinterpret_cast<volatile int*>(flag)), 0, min(E, 256), lane, v);
       if (by_pairs) {                            // for the warp that adds
