@@ -494,9 +494,11 @@ const void* const* sgr_residency_host_table(const void* handle, int which);
  * allocate device memory - an engine whose whole VRAM budget was handed out at
  * start-up (KV cache, expert slab) and that treats any later cudaMalloc as a bug,
  * a host binding with no way to own CUDA buffers, code that only ever runs inside a
- * captured region. The scratch is a file-scope device array inside the library,
- * sgr_moe_layer_static_limit() bytes (2 MiB: at hidden 2048, expert FFN 512, 256 experts,
- * top-8 that is up to n_max = 16 token rows; n_max = 8 needs 1.3 MB); `workspace` / `workspace_bytes` of the
+ * captured region. The scratch is a file-scope device array inside the library:
+ * sgr_moe_layer_static_limit() bytes (2 MiB), and 512 KiB for the logits that layers of up to four rows exchange.
+ * A shape is taken when its sgr_moe_layer_workspace_bytes, less 128 * min(n_max, 4) * n_expert bytes of these
+ * (rounded up to 256), is at most the limit: at hidden 2048, expert FFN 512, 256 experts, top-8 up to
+ * n_max = 16 token rows. `workspace` / `workspace_bytes` of the
  * argument block are ignored, inputs and outputs are still the caller's. A shape
  * whose scratch would not fit returns SGR_ESTATICLIMIT and launches nothing. The first
  * call on each device looks up the array's device address and must be made outside

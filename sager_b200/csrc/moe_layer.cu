@@ -53,6 +53,7 @@ constexpr int kTmapSlots = kAheadStages + 7;      // patched TMA descriptor pair
 // 3 / 4 rows, 256 experts, hidden 2048, n_ff 512: 13.2 / 20.7 / 24.0 / 27.2, route + expert kernel 27.0 / 35.4 / 40.7 / 37.7;
 // 128 experts, hidden 1024: 12.0 / 17.6 / 19.9 / 22.1 against 23.6 / 25.7 / 31.3 / 29.6).
 constexpr int kTokenKernelMaxRows = 4;
+constexpr int kMaxExperts = 1024;
 constexpr int kXchgCopies = 16;        // of the logits that a one-launch layer's CTAs exchange (token_layer.cuh)
 // Layers of at least this many token rows have the row-streaming kernel's order of the sums (block after block), and of the
 // two expert kernels run that one (us per layer with the route kernel, 256 experts: 37.7 against 46.5 for the item kernel at
@@ -1105,7 +1106,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) expert_stream_kernel(const 
 // same layout a caller-provided workspace has, held by every device that loads
 // the library until the process exits.
 constexpr size_t kStaticWsBytes = 2u << 20;                      // beside the logits that a one-launch layer exchanges
-constexpr size_t kStaticXchgBytes = kXchgCopies * kTokenKernelMaxRows * 1024 * 8;
+constexpr size_t kStaticXchgBytes = kXchgCopies * kTokenKernelMaxRows * kMaxExperts * 8;
 static __device__ __align__(256) unsigned char g_static_ws[kStaticWsBytes + kStaticXchgBytes];
 constexpr int kStaticMaxDevices = 64;
 unsigned char* g_static_ws_addr[kStaticMaxDevices];     // per-device address of g_static_ws
@@ -1311,7 +1312,7 @@ SGR_API int sgr_moe_layer_decode_stages(const sgr_moe_layer* a, int stages, void
   if (a->hidden <= 0 || a->hidden % kQK || a->n_ff <= 0 || a->n_ff % kQK || a->n_expert <= 0 ||
       a->n_used <= 0 || a->n_used > a->n_expert || a->n_max < a->n || a->n_max > kMaxRows)
     return kErrGeometry;
-  if (a->n_expert > 1024 || a->hidden > 8192 || a->n_ff > 8192) return kErrUnsupported;
+  if (a->n_expert > kMaxExperts || a->hidden > 8192 || a->n_ff > 8192) return kErrUnsupported;
   if (!a->w_tab || !a->route_idx || !a->route_w || !a->workspace || (!a->x_f16 && !a->out_f32 && !a->ep_out))
     return kErrArg;
   if (!a->routing_given && (!a->xn || !a->router_w)) return kErrArg;
@@ -1617,8 +1618,10 @@ SGR_API int sgr_moe_layer_decode_static(const sgr_moe_layer* a, void* stream) {
     return kErrGeometry;
   const WsLayout lay = ws_layout(a->n_max, a->hidden, a->n_ff, a->n_expert, a->n_used);
   // The whole layout must fit, so that the call picks its expert kernel exactly as a call on a
-  // caller's workspace of sgr_moe_layer_workspace_bytes() does.
-  if (lay.total - (lay.hbuf - lay.xchg) > kStaticWsBytes || lay.hbuf - lay.xchg > kStaticXchgBytes) return kErrStaticLimit;
+  // caller's workspace of sgr_moe_layer_workspace_bytes() does. (The exchanged logits have a place of their own, for as many experts as the
+  // layer takes.)
+  if (lay.total - (lay.hbuf - lay.xchg) > kStaticWsBytes) return kErrStaticLimit;
+  if (a->n_expert > kMaxExperts) return kErrUnsupported;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kStaticMaxDevices) return kErrLaunch;
   if (g_static_ws_addr[dev] == nullptr) {

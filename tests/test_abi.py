@@ -38,6 +38,23 @@ def test_argument_validation_needs_no_gpu():
     assert lib.raw("sgr_tc_scratch_elems")(512, 2048) == 512 * 2048
 
 
+def test_static_scratch_takes_and_refuses_the_shapes_of_its_rule():
+    lib = capi.lib()
+    size, limit = lib.raw("sgr_moe_layer_workspace_bytes"), lib.raw("sgr_moe_layer_static_limit")()
+
+    def call(n_max, hidden, n_ff, E, k):
+        a = capi.MoeLayerArgs()
+        a.n, a.n_max, a.hidden, a.n_ff, a.n_expert, a.n_used = 1, n_max, hidden, n_ff, E, k        # (no buffers: refused further on)
+        return lib.raw("sgr_moe_layer_decode_static")(C.byref(a), None)
+
+    for n_max in (1, 3, 4, 15, 16, 17, 24):
+        for shape in ((2048, 512, 256, 8), (512, 256, 16, 4), (1024, 256, 1024, 2)):
+            logits = (128 * min(n_max, 4) * shape[2] + 255) // 256 * 256
+            assert (call(n_max, *shape) == 6) == (size(n_max, *shape) - logits > limit), (n_max, shape)
+    assert call(16, 2048, 512, 256, 8) != 6 and call(17, 2048, 512, 256, 8) == 6
+    assert call(1, 256, 256, 1025, 2) == 3                   # more experts than the layer takes
+
+
 def test_head_ring_slots_belong_to_one_group_of_warps():
     """A wait by parity tells a phase from the one before only if that one was waited for: the ring's stages are a multiple of the
     groups that take them in turn, for every row length."""
