@@ -363,10 +363,12 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
     // 505 / 540 / 576 / 629 / 747 / 476 / 608 / 826, with twelve 442 / 464 / 505 / 547 / 621 / 758 / 490 / 634 / 864); 16 x 4, four warps, four 483 /
     // 504 / 533 / 568 / 622 / 743 / 472 / 605 / 818; one chain to a lane 466 / 488 / 516 / 552 / 616 / 755 / 487 / 623 / 851. 64 experts, 300 rows:
     // 141.6, 148.3, 147.9 and 147.3. (592 rows, back to back and L2-hot: 8 x 4 21.3, 16 x 4 25.7 - three CTAs on an SM for little more than two.)
+    // The lines are from 2048 columns. At 512 to 4096 columns, 16 to 256 rows and 2 to 4096 tokens the rule is ahead of the kernel with one chain to a
+    // lane and its lines throughout: back to back by 4 to 110 %, 200 tokens x 256 rows of 4096 columns 25.4 -> 20.8, 4096 tokens x 128 of 512 21.5 -> 17.7.
     const long long outputs = static_cast<long long>(n_rows) * n_tokens;
     if (outputs >= 256LL * 620) return launch_staged<16, 4, 1, 4, 4>(w, x, y, n_rows, k, n_tokens, stream);
     if (outputs >= 256LL * 180) return launch_staged<8, 4, 2, 2, 8>(w, x, y, n_rows, k, n_tokens, stream);
-    if (outputs > 64LL * 2 * 148) return launch_staged<4, 4, 2, 1, 8>(w, x, y, n_rows, k, n_tokens, stream);
+    if (outputs > 64LL * 2 * device_sms()) return launch_staged<4, 4, 2, 1, 8>(w, x, y, n_rows, k, n_tokens, stream);
     // (all CTAs fit on the SMs at once with twelve stages as well: 80 rows x 64 experts 112.5 for 115.6, 100 x 128 123.7 for 125.6, 65 x 256 440
     // for 444; 96 x 256, where they do not, 474 for 467)
     return launch_staged<4, 4, 2, 1, 12>(w, x, y, n_rows, k, n_tokens, stream);
