@@ -364,7 +364,7 @@ int launch_logits(const float* w, const uint16_t* x, float* y, int n_rows, int k
     // 504 / 533 / 568 / 622 / 743 / 472 / 605 / 818; one chain to a lane 466 / 488 / 516 / 552 / 616 / 755 / 487 / 623 / 851. 64 experts, 300 rows:
     // 141.6, 148.3, 147.9 and 147.3. (592 rows, back to back and L2-hot: 8 x 4 21.3, 16 x 4 25.7 - three CTAs on an SM for little more than two.)
     // The lines are from 2048 columns. At 512 to 4096 columns, 16 to 256 rows and 2 to 4096 tokens the rule is ahead of the kernel with one chain to a
-    // lane and its lines throughout: back to back by 4 to 110 %, 200 tokens x 256 rows of 4096 columns 25.4 -> 20.8, 4096 tokens x 128 of 512 21.5 -> 17.7.
+    // lane and its lines throughout: back to back by 1 to 110 %, 200 tokens x 256 rows of 4096 columns 25.4 -> 20.8, 4096 tokens x 128 of 512 21.5 -> 17.7.
     const long long outputs = static_cast<long long>(n_rows) * n_tokens;
     if (outputs >= 256LL * 620) return launch_staged<16, 4, 1, 4, 4>(w, x, y, n_rows, k, n_tokens, stream);
     if (outputs >= 256LL * 180) return launch_staged<8, 4, 2, 2, 8>(w, x, y, n_rows, k, n_tokens, stream);

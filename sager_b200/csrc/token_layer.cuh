@@ -30,8 +30,8 @@
 // layer, 2.3 to the logits, 1 until a CTA has all of them, 2 for picks and tables, 1.5 for the first bytes, 2 for
 // gate / up, 2 for the barrier, 1 + 1 for h and the down rows; 13.8 with a barrier between logits and selection, 15.1 with the loops over rows
 // of larger layers, whose live values were spilled, 26.6 with eight warps on whole blocks and the selection in sequence). A further
-// row costs 3 to 7 us - 20.7 / 23.9 / 27.1 us at 2 / 3 / 4 rows, by dp4a 21.7 / 28.3 / 32.7 -, where its bytes cost 2.2: of the 27.1, gate / up
-// terms take 2.9, down terms 3.3, h in every CTA 2.3.
+// row costs 3 to 7 us - 20.7 / 23.9 / 27.1 us at 2 / 3 / 4 rows, by dp4a 21.7 / 28.3 / 32.7 -, where its bytes cost 2.2: at four rows, without
+// the terms of gate / up 2.3 us less, without those of the down rows 2.9, with four of the 36 h rows in every CTA 1.6 (at two rows 1.7, 2.2 and 0.7).
 //
 // Work split: gate / up by pairs (a flat range of (tile, pair) per CTA, of equal cost), down by output
 // rows. Contracts are those of the two-launch path: null table entry = absent expert
@@ -170,6 +170,7 @@ __host__ __device__ inline Geom geom(int n, int K, int H, int FF, int E, int gri
 // pairs take more than one pass of both groups, and a row of few blocks leaves little to gain: us per layer, dp4a / MMA,
 //   2048 / 512 / 256 experts / top-8 at 2 / 3 / 4 rows (1.7 / 2.6 / 3.5 passes) 21.8 / 28.3 / 32.7, 20.8 / 24.4 / 27.2
 //   2048 / 256 / 64 / 8 (0.9 / 1.3 / 1.7) 16.5 / 18.9 / 21.0, 17.2 / 18.7 / 19.8
+//   2048 / 768 / 128 / 8 (2.6 / 3.9 / 5.2) 26.1 / 37.7 / 44.4, 25.2 / 32.3 / 35.0
 //   1024 / 512 / 128 / 8 (0.9 / 1.3 / 1.7) 17.8 / 20.0 / 22.1, 19.0 / 21.1 / 22.7
 //   512 / 256 / 16 / 4 (0.1 / 0.2 / 0.2) 13.2 / 14.0 / 15.1, 13.6 / 14.0 / 14.7.
 inline bool use_mma(int n, int K, int H, int FF, int grid) {
@@ -214,8 +215,8 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 // that it could work through.
 //
 // The logits go from CTA to CTA without a barrier. A word holds a logit and, above it, the launch's number, which no launch before on the
-// workspace had (in 32 bits: a word would have to be 2^32 launches old); a warp of each CTA reads a row's words until all have it. Behind a barrier they took two more trips: an
-// arrival waits for the stores before it, and the reads begin when the poll returns. There are kXchgCopies of the words, written by
+// workspace had (in 32 bits: a word would have to be 2^32 launches old); a warp of each CTA reads a row's words until all have it. Behind
+// a barrier they took two more trips: an arrival waits for the stores before it, and the reads begin when the poll returns. There are kXchgCopies of the words, written by
 // as many lanes, and a CTA reads one: 148 readers of the same lines are in the writers' way. us per layer at one row, behind the
 // barrier, then with 1 / 2 / 4 / 8 / 16 copies: hidden 2048, 256 experts 13.8, 14.3 / 13.6 / 13.4 / 13.2 / 13.2; 1024, 128 12.3, 13.8 / 12.7 / 12.7 /
 // 12.3 / 12.0; 2048, 64 12.0, 12.7 / 12.4 / 12.2 / 12.1 / 11.9; 512, 16 10.8, 11.1 / 11.2 / 11.0 / 10.9 / 10.8; two to four rows of the first 21.0 / 24.5 /
