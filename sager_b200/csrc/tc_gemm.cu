@@ -253,8 +253,9 @@ __device__ __forceinline__ uint4 dequant_octet(const unsigned char* blk, int lan
 // tensor-memory operand (tcgen05.st); only the activations go through shared memory, of a pair's each CTA half.
 //   * warps 0-7: unpack, four to a block, even and odd blocks, on into the next unit; a block is two of four slots in tensor memory,
 //     so neither four waits for the other's
-//   * warps 8-15: epilogue, a quarter of the lanes and half of the columns each; the accumulators are free once they are in
-//     registers as fp16
+//   * warps 8-15: epilogue, a quarter of the lanes and half of the columns each, sixteen columns at a time (all of them into registers
+//     first, so that the accumulators are free earlier, is straight-line code and lost more: 2048 x 512 over 1457 tokens 8.55 us, now 6.5, 4096 x 512
+//     over 1000 10.9 and 8.6, 4096 x 2048 over 2048 29.8 and 29.3)
 //   * warp 16: activation tiles (TMA, 128-byte swizzle, 64 k a stage)
 //   * warp 17: block columns of the weights (a TMA copy of 128 blocks each), four in flight
 //   * warp 18: tensor memory and (a pair's first CTA) MMA issue
@@ -431,47 +432,38 @@ __global__ void __launch_bounds__(kQ4Threads, 1) tc_gemm_q4_kernel(const __grid_
     const uint32_t src = tmem + (static_cast<uint32_t>(quarter * 32) << 16) + half, acc_empty = cluster_addr(&bar[kQ4AccEmpty], 0);
     const bool pairs = (a.n_rows & 1) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 3u) == 0;
     const int odd = lane & 1;
+    const uint32_t sel = odd ? 0x3276u : 0x5410u;
     unsigned ph = 0;
     pdl_wait();                                   // y may still be read by the kernel before
     for_units([&](int row0, int tok0, int ntok, int) {
       if (!wait_warp(kQ4AccFull, ph)) return false;
       ph ^= 1u;
       tc_fence_after();
-      const int cols = min(a.bn >> 1, ntok - half), row = row0 + quarter * 32 + lane;
-      uint32_t h[64];                             // tokens 2 i, 2 i + 1 of the half
-#pragma unroll
-      for (int c = 0; c < 128; c += 16) {
-        if (c >= cols) break;
+      const int cols = min(a.bn >> 1, ntok - half), row = row0 + quarter * 32 + lane, last = row < a.n_rows ? cols : 0;
+      uint16_t* y = a.y + static_cast<size_t>(tok0 + half) * a.n_rows + row;
+      if (pairs) y += odd ? a.n_rows - 1 : 0;
+#pragma unroll 2
+      for (int c = 0; c < cols; c += 16) {
         uint32_t v[16];
         tc_ld16(src + c, v);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int i = 0; i < 8; ++i) h[c / 2 + i] = h2_bits(__floats2half2_rn(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t h = h2_bits(__floats2half2_rn(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])));      // tokens t, t + 1
+          const int t = c + 2 * i;
+          if (pairs) {
+            const uint32_t w = __byte_perm(h, __shfl_xor_sync(0xFFFFFFFFu, h, 1), sel);
+            if (t + odd < last) *reinterpret_cast<uint32_t*>(y) = w;
+          } else {
+            if (t < last) y[0] = static_cast<uint16_t>(h & 0xFFFFu);
+            if (t + 1 < last) y[a.n_rows] = static_cast<uint16_t>(h >> 16);
+          }
+          y += 2 * static_cast<size_t>(a.n_rows);
+        }
       }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) arrive_first(&bar[kQ4AccEmpty], acc_empty);
-      uint16_t* y = a.y + static_cast<size_t>(tok0 + half) * a.n_rows + row;
-      if (pairs) {
-        const uint32_t sel = odd ? 0x3276u : 0x5410u;
-        const int last = row < a.n_rows ? cols : 0;
-        y += odd ? a.n_rows - 1 : 0;
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          if (2 * i >= cols) break;
-          const uint32_t v = __byte_perm(h[i], __shfl_xor_sync(0xFFFFFFFFu, h[i], 1), sel);
-          if (2 * i + odd < last) *reinterpret_cast<uint32_t*>(y) = v;
-          y += 2 * static_cast<size_t>(a.n_rows);
-        }
-      } else if (row < a.n_rows) {
-#pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          if (2 * i >= cols) break;
-          y[0] = static_cast<uint16_t>(h[i] & 0xFFFFu);
-          if (2 * i + 1 < cols) y[a.n_rows] = static_cast<uint16_t>(h[i] >> 16);
-          y += 2 * static_cast<size_t>(a.n_rows);
-        }
-      }
       return true;
     });
   } else if (warp == kQ4WarpX) {
@@ -704,14 +696,14 @@ struct Q4Plan {
   double us;
 };
 // Token rows per unit, CTAs that share a unit, and who writes the scratch: what takes the least by estimates in us, fitted to
-// 27 shapes (4096 x 2048 over 2048 tokens, inputs from HBM: units of a pair's 256 rows x 256 tokens 38.9 us, 224 tokens 45.0, a single CTA's 128 rows
-// x 240 / 256 tokens 39.7 / 41.0; 4096 x 4096 63.2, 64.2 and 66.9).
-//   the start, 4, and the last unit's epilogue, 3 for 256 tokens (without it, and with a row tile's scratch in equal parts and not in whole
-//     blocks, 512 x 512 over 400 / 1457 tokens 6.6 / 7.1 us for 5.0 / 5.5, 2048 x 2048 over 512 12.9 for 12.5)
+// 47 shapes of 512 to 8192 rows, 512 to 4096 columns and 64 to 2048 tokens. us of a pair's units / of a single CTA's, each at their best, inputs
+// from HBM: 4096 x 2048 over 2048 tokens 38.5 / 39.5, 4096 x 4096 70.5 / 73.5, 4096 x 4096 over 1000 40.5 / 42.3, 2048 x 2048 20.1 / 20.2, 4096 x 1024 22.5 / 22.5.
+// (Back to back, all of them in L2, rows of up to eight blocks are 3 to 5 % faster by single CTAs.)
+//   the start, 4, and the last unit's epilogue, 1.5 for 256 tokens
 //   a block column of a unit: 1.0 and, with the square of its tokens, up to 0.35 more, a fifth more when every SM works; a pair
 //     brings half of the activations per CTA and gains 6 % past 128 tokens, but costs 0.3 to set up
 //   the scratch, per block of a row tile: SMs that the units leave idle, in whole columns of row tiles, 3.2 / spare beside
-//     the units' 1.3 and epilogue (2048 x 512 over 2048 tokens 10.9 -> 9.7); the units of a row tile themselves, 2 for each block that one
+//     the units' 1.3 and epilogue; the units of a row tile themselves, 2 for each block that one
 //     of its token tiles writes on top of it; or the dequantisation kernel ahead of the
 //     GEMM, 2.5 us and the bytes at 5 TB/s (8192 x 4096 over 64 tokens: 53 us by one spare column, 41 by the kernel ahead).
 Q4Plan q4_plan(int sms, int n_rows, int k, int n_tokens) {
@@ -730,9 +722,9 @@ Q4Plan q4_plan(int sms, int n_rows, int k, int n_tokens) {
       c.workers = std::min(c.units, sms / cg) * cg;
       const int waves = (c.units * cg + c.workers - 1) / c.workers;
       const double wide = bn / 256.;
-      c.us = 4 + 3 * wide + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.06 : 1.);
+      c.us = 4 + 1.5 * wide + 0.3 * (cg - 1) + waves * nb * (1 + 0.35 * wide * wide) * (1 + 0.2 * c.workers / sms) * (cg == 1 && bn > 128 ? 1.06 : 1.);
       const int spare = std::min(nb, (sms - c.workers) / row_tiles);
-      const double by_spare = spare > 0 ? std::max(0., nb * (3.2 / spare - 1.3) - 3 * wide) : 1e30, by_tiles = 2. * ((nb + c.tiles - 1) / c.tiles);
+      const double by_spare = spare > 0 ? std::max(0., nb * (3.2 / spare - 1.3) - 1.5 * wide) : 1e30, by_tiles = 2. * ((nb + c.tiles - 1) / c.tiles);
       const double by_kernel = 2.5 + static_cast<double>(n_rows) * k * 2.5625 / 5e6;
       c.spare = by_spare < by_tiles ? spare : 0;
       if (by_kernel < std::min(by_spare, by_tiles)) {

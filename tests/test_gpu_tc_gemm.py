@@ -190,13 +190,15 @@ def test_q4k_gemm_few_rows_past_a_tile(rows):
 
 
 @pytest.mark.parametrize("rows,k,tok,cg,says", [
-    (4224, 1024, 2040, 2, "waves odd_row_tiles ragged"),
-    (2176, 4096, 1000, 2, "odd_row_tiles spare ragged"),
-    (3201, 1024, 2048, 2, "waves odd_rows"),             # no paired stores
+    (4224, 4096, 1828, 2, "waves odd_row_tiles ragged"),
+    (2176, 4096, 1103, 2, "odd_row_tiles spare ragged"),
+    (3201, 2048, 1682, 2, "waves odd_rows"),             # no paired stores
     (4096, 4096, 1282, 2, "short_tail"),                 # a pair's last units have 2 tokens,
+    (3201, 2048, 1605, 2, "short_tail odd_rows"),        # ... 5, no paired stores
     (1000, 4096, 1926, 2, "short_tail spare"),           # ... 6, beside CTAs for the scratch
     (4096, 4096, 1296, 2, "short_tail"),                 # ... 16
-    (4096, 2048, 2048, 2, "waves"),
+    (4096, 4096, 2048, 2, "waves"),
+    (4224, 1024, 2040, 2, "waves odd_row_tiles"),
     (4096, 2048, 1027, 1, "waves short_tail"),
     (4224, 256, 1555, 1, "waves"),                       # one block to a row
     (4096, 512, 2047, 1, "waves"),                       # the units of a CTA start on even and odd blocks of the rings alike
