@@ -262,8 +262,8 @@ __device__ __forceinline__ uint4 dequant_octet(const unsigned char* blk, int lan
 // 4096 x 2048 over 2048 rows (MMAs 16 us at two units each, 20.8 at the library's rate): 38.5 us with a CTA per unit, whose start and epilogue
 // nothing covered, 32.8 persistent and in pairs, 31.8 with the weights by TMA (one warp's cp.async, 36 to a block with a division
 // each, took longer than the block: 130 x 4096 over 333 rows 28 -> 21), 31.2 with four slots instead of three (those with pairs of N = 240;
-// inputs from HBM 37.9, and 38.4 with the N = 256 that mma_columns asks for). The tensor pipe of an SM with two units is busy for 66 % of its
-// cycles, about 2,100 to a block; the rest is the start, the last epilogue, the scratch (by the estimate below 2 us) and hand-overs.
+// inputs from HBM 37.9, and 38.4 with the N = 256 that mma_columns asks for). The tensor pipe of an SM with two units is busy for 67 % of its
+// cycles, about 2,050 to a block; the rest is the start, the last epilogue, the scratch (by the estimate below 2 us) and hand-overs.
 // `scratch` receives the dequantised rows: with few units by CTAs of their own on the SMs left over (a thread's 16-byte pieces of
 // its row take longer than its block: 1000 x 4096 over 75 rows 33.8 -> 22.6 us, over 64 rows 54.5 -> 22.5), else each token
 // tile writes its share of the blocks. (Written by the epilogue warps out of the weights' ring, 512 bytes a row: 33.8 us for 31.0.)
